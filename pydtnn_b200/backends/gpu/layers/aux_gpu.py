@@ -7,15 +7,14 @@ import numpy as np
 from .... import _lib
 from ....layers import (AdditionBlock, AveragePool2D, BatchNormalization, Dropout, Flatten, Input, MaxPool2D, Relu,
                         Softmax)
-from ....tensor_gpu import TensorGPU, empty, to_gpu, zeros
-from ....utils import EVALUATE_MODE, PYDTNN_TENSOR_FORMAT_NCHW, TRAIN_MODE
+from ....tensor_gpu import ChannelLastTensor, TensorGPU, empty, to_gpu
+from ....utils import EVALUATE_MODE, TRAIN_MODE
 from .. import memory_allocation as wsp
 from .layer_gpu import LayerGPU
 
 
-def _layout(model):
-    return _lib.LAYOUT_NCHW if model.tensor_format == PYDTNN_TENSOR_FORMAT_NCHW else _lib.LAYOUT_NHWC
-
+# Activations are channel-last in either tensor format (ChannelLastTensor), so the library is always called with that
+# layout; a (batch, features) tensor is the case h = w = 1.
 
 class InputGPU(LayerGPU, Input):
     """pydtnn/backends/gpu/layers/input_gpu.py:28-40"""
@@ -49,9 +48,10 @@ class BatchNormalizationGPU(LayerGPU, BatchNormalization):
         self.save_inv_var = TensorGPU(empty((c,), m.dtype), m.tensor_format)
         self._inv_std = empty((c,), m.dtype)
         wsp.require_reduction_scratch(c)
-        self.y = TensorGPU(empty(x.ary.shape, m.dtype), m.tensor_format)
+        self.y = self._activation(x.dims)
         if self.need_dx:
-            self.dx = TensorGPU(empty(x.ary.shape, m.dtype), m.tensor_format)
+            self.dx = self._activation(x.dims)
+        self._x_ptr = None
         self.fuse_relu = False           # set by the model's fusion pass (BN followed by ReLU)
         self.prestats = None             # (buffer, bytes) left by the preceding convolution's forward pass of this step
         self.residual = None             # (other branch, output) while an addition block folds its sum + ReLU in here
@@ -63,42 +63,46 @@ class BatchNormalizationGPU(LayerGPU, BatchNormalization):
         m = self.model
         L = _lib.lib()
         self.x = x
+        x_ptr = self._x_ptr = self._in(x, "x")
         if m.mode == TRAIN_MODE and self.prestats is not None:
             # the convolution that wrote x already summed it per channel: statistics from those sums, one pass over x
             st, nbytes = self.prestats
             self.prestats = None
             addend, out, relu = (self.residual[0], self.residual[1], 1) if self.residual is not None else (None, self.y, int(self.fuse_relu))
             _lib.check(L.b2c_bn_train_forward_prestats(
-                m.batch_size, self.ci, self._hw, x.ptr, st.data_ptr(), nbytes, self.gamma.ptr, self.beta.ptr,
+                m.batch_size, self.ci, self._hw, x_ptr, st.data_ptr(), nbytes, self.gamma.ptr, self.beta.ptr,
                 self.running_mean.ptr, self.running_var.ptr, float(self.momentum), float(self.epsilon), relu,
-                addend.ptr if addend is not None else None, out.ptr, self.save_mean.ptr, self.save_inv_var.ptr,
+                self._in(addend, "addend") if addend is not None else None, out.out, self.save_mean.ptr, self.save_inv_var.ptr,
                 wsp.reduction_scratch().data_ptr(), wsp.reduction_scratch().numel() * 8, m.stream_handle))
+            out.written()
             self.updated_running_var = True
             return out
         if m.mode == TRAIN_MODE and self.residual is not None:
             # last batch norm of a residual branch: out = relu(bn(x) + other branch), written to the block's ReLU
             addend, out = self.residual
             _lib.check(L.b2c_bn_train_forward_residual(
-                self._dt, _layout(m), m.batch_size, self.ci, self._hw, x.ptr, self.gamma.ptr, self.beta.ptr,
-                self.running_mean.ptr, self.running_var.ptr, float(self.momentum), float(self.epsilon), addend.ptr, 1,
-                out.ptr, self.save_mean.ptr, self.save_inv_var.ptr, wsp.reduction_scratch().data_ptr(),
+                self._dt, _lib.LAYOUT_NHWC, m.batch_size, self.ci, self._hw, x_ptr, self.gamma.ptr, self.beta.ptr,
+                self.running_mean.ptr, self.running_var.ptr, float(self.momentum), float(self.epsilon), self._in(addend, "addend"), 1,
+                out.out, self.save_mean.ptr, self.save_inv_var.ptr, wsp.reduction_scratch().data_ptr(),
                 wsp.reduction_scratch().numel() * 8, m.stream_handle))
+            out.written()
             self.updated_running_var = True
             return out
         if m.mode == TRAIN_MODE:
-            _lib.check(L.b2c_bn_train_forward(self._dt, _layout(m), m.batch_size, self.ci, self._hw, x.ptr,
+            _lib.check(L.b2c_bn_train_forward(self._dt, _lib.LAYOUT_NHWC, m.batch_size, self.ci, self._hw, x_ptr,
                                               self.gamma.ptr, self.beta.ptr, self.running_mean.ptr,
                                               self.running_var.ptr, float(self.momentum), float(self.epsilon),
-                                              int(self.fuse_relu), self.y.ptr, self.save_mean.ptr,
+                                              int(self.fuse_relu), self.y.out, self.save_mean.ptr,
                                               self.save_inv_var.ptr, wsp.reduction_scratch().data_ptr(),
                                               wsp.reduction_scratch().numel() * 8, m.stream_handle))
             self.updated_running_var = True
         elif m.mode == EVALUATE_MODE:
-            _lib.check(L.b2c_bn_inference(self._dt, _layout(m), m.batch_size, self.ci, self._hw, x.ptr,
+            _lib.check(L.b2c_bn_inference(self._dt, _lib.LAYOUT_NHWC, m.batch_size, self.ci, self._hw, x_ptr,
                                           self.running_mean.ptr, self.inference_inv_std().gpudata, self.gamma.ptr,
-                                          self.beta.ptr, int(self.fuse_relu), self.y.ptr, m.stream_handle))
+                                          self.beta.ptr, int(self.fuse_relu), self.y.out, m.stream_handle))
         else:
             raise ValueError("Unexpected model mode")
+        self.y.written()
         return self.y
 
     def inference_inv_std(self):
@@ -114,12 +118,14 @@ class BatchNormalizationGPU(LayerGPU, BatchNormalization):
     def backward(self, dy):
         m = self.model
         _lib.check(_lib.lib().b2c_bn_train_backward(
-            self._dt, _layout(m), m.batch_size, self.ci, self._hw, self.x.ptr, dy.ptr,
-            self.y.ptr if self.fuse_relu else None, self.beta.ptr if self.fuse_relu else None, self.gamma.ptr,
+            self._dt, _lib.LAYOUT_NHWC, m.batch_size, self.ci, self._hw,
+            self._x_ptr if self._x_ptr is not None else self._in(self.x, "x"), self._in(dy, "dy"),
+            self._in(self.y, "y") if self.fuse_relu else None, self.beta.ptr if self.fuse_relu else None, self.gamma.ptr,
             self.save_mean.ptr, self.save_inv_var.ptr,
-            self.dgamma.ptr, self.dbeta.ptr, self.dx.ptr if self.need_dx else None,
+            self.dgamma.ptr, self.dbeta.ptr, self.dx.out if self.need_dx else None,
             wsp.reduction_scratch().data_ptr(), wsp.reduction_scratch().numel() * 8, m.stream_handle))
         if self.need_dx:
+            self.dx.written()
             return self.dx
 
 
@@ -129,9 +135,9 @@ class ReluGPU(LayerGPU, Relu):
     def initialize(self, prev_shape, need_dx, x):
         super().initialize(prev_shape, need_dx, x)
         m = self.model
-        self.y = TensorGPU(empty(x.ary.shape, m.dtype), m.tensor_format)
+        self.y = self._activation(x.dims)
         if self.need_dx:
-            self.dx = TensorGPU(empty(x.ary.shape, m.dtype), m.tensor_format)
+            self.dx = self._activation(x.dims)
         self._dt = _lib.dtype_code(m.dtype)
         self.absorbed = False            # True when the preceding BatchNormalization applies the ReLU itself
         self.fed_by_block = False        # True when the preceding AdditionBlock writes max(sum, 0) into self.y
@@ -142,7 +148,8 @@ class ReluGPU(LayerGPU, Relu):
             return x
         if self.fed_by_block:
             return self.y
-        _lib.check(_lib.lib().b2c_relu_forward(self._dt, self.y.size, x.ptr, self.y.ptr, self.model.stream_handle))
+        _lib.check(_lib.lib().b2c_relu_forward(self._dt, self.y.size, self._in(x, "x"), self.y.out, self.model.stream_handle))
+        self.y.written()
         return self.y
 
     def backward(self, dy):
@@ -151,8 +158,9 @@ class ReluGPU(LayerGPU, Relu):
         if self.bwd_by_block and self.model.mode == TRAIN_MODE:
             return self.dx
         if self.need_dx:
-            _lib.check(_lib.lib().b2c_relu_backward(self._dt, self.y.size, dy.ptr, self.y.ptr, self.dx.ptr,
+            _lib.check(_lib.lib().b2c_relu_backward(self._dt, self.y.size, self._in(dy, "dy"), self._in(self.y, "y"), self.dx.out,
                                                     self.model.stream_handle))
+            self.dx.written()
             return self.dx
 
 
@@ -162,11 +170,11 @@ class SoftmaxGPU(LayerGPU, Softmax):
     def initialize(self, prev_shape, need_dx, x):
         super().initialize(prev_shape, need_dx, x)
         m = self.model
-        self.y = TensorGPU(empty(x.ary.shape, m.dtype), m.tensor_format)
+        self.y = TensorGPU(empty(x.dims, m.dtype), m.tensor_format)
         if self.need_dx:
-            self.dx = TensorGPU(empty(x.ary.shape, m.dtype), m.tensor_format)
+            self.dx = TensorGPU(empty(x.dims, m.dtype), m.tensor_format)
         self._dt = _lib.dtype_code(m.dtype)
-        self._rows, self._cols = int(x.ary.shape[0]), int(np.prod(x.ary.shape[1:]))
+        self._rows, self._cols = int(x.dims[0]), int(np.prod(x.dims[1:]))
 
     def forward(self, x):
         _lib.check(_lib.lib().b2c_softmax_forward(self._dt, self._rows, self._cols, x.ptr, self.y.ptr,
@@ -197,19 +205,44 @@ class DropoutGPU(LayerGPU, Dropout):
 
 
 class FlattenGPU(LayerGPU, Flatten):
-    """pydtnn/backends/gpu/layers/flatten_gpu.py:33-52 -- views, no copies."""
+    """pydtnn/backends/gpu/layers/flatten_gpu.py:33-52 -- views, no copies, where the flattened order is the stored one;
+    the (c, h, w) order of an NCHW model's features is copied out of the channel-last activation otherwise."""
 
     def initialize(self, prev_shape, need_dx, x):
         super().initialize(prev_shape, need_dx, x)
-        self.y = TensorGPU(x.ary.reshape((self.model.batch_size, *self.shape)), self.model.tensor_format)
+        m = self.model
+        self._copied = isinstance(x, ChannelLastTensor) and not x.same_order
+        if self._copied:
+            self.y = TensorGPU(empty((m.batch_size, *self.shape), m.dtype), m.tensor_format)
+            if self.need_dx:
+                self.dx = self._activation(x.dims)
+        else:
+            self.y = TensorGPU(x.ary.reshape((m.batch_size, *self.shape)), m.tensor_format)
+
+    def _chw(self):
+        c, h, w = self.prev_shape
+        return c, h * w
 
     def forward(self, x):
-        self.y = TensorGPU(x.ary.reshape((self.model.batch_size, *self.shape)), self.model.tensor_format)
+        m = self.model
+        if self._copied:
+            c, hw = self._chw()
+            _lib.check(_lib.lib().b2c_transpose(_lib.dtype_code(m.dtype), m.batch_size, hw, c, self._in(x, "x"), self.y.ptr,
+                                                m.stream_handle))
+            return self.y
+        self.y = TensorGPU(x.ary.reshape((m.batch_size, *self.shape)), m.tensor_format)
         return self.y
 
     def backward(self, dy):
+        m = self.model
         if self.need_dx:
-            self.dx = TensorGPU(dy.ary.reshape((self.model.batch_size, *self.prev_shape)), self.model.tensor_format)
+            if self._copied:
+                c, hw = self._chw()
+                _lib.check(_lib.lib().b2c_transpose(_lib.dtype_code(m.dtype), m.batch_size, c, hw, dy.ptr, self.dx.out,
+                                                    m.stream_handle))
+                self.dx.written()
+            else:
+                self.dx = TensorGPU(dy.ary.reshape((m.batch_size, *self.prev_shape)), m.tensor_format)
             return self.dx
 
 
@@ -220,11 +253,11 @@ class _Pool2DGPU(LayerGPU):
     def initialize(self, prev_shape, need_dx, x):
         super().initialize(prev_shape, need_dx, x)
         m = self.model
-        self.y = TensorGPU(empty((m.batch_size, *self.shape), m.dtype), m.tensor_format)
+        self.y = self._activation((m.batch_size, *self.shape))
         if self._is_max:
-            self.idx_max = empty((m.batch_size, *self.shape), np.int32)
+            self.idx_max = empty((m.batch_size, self.ho, self.wo, self.co), np.int32)
         if self.need_dx:
-            self.dx = TensorGPU(empty(x.ary.shape, m.dtype), m.tensor_format)
+            self.dx = self._activation(x.dims)
         self._dt = _lib.dtype_code(m.dtype)
 
     def _geom(self):
@@ -233,16 +266,19 @@ class _Pool2DGPU(LayerGPU):
 
     def forward(self, x):
         m = self.model
-        _lib.check(_lib.lib().b2c_pool_forward(self._dt, _layout(m), self._is_max, *self._geom(), x.ptr, self.y.ptr,
-                                               self.idx_max.gpudata if self._is_max else None, m.stream_handle))
+        _lib.check(_lib.lib().b2c_pool_forward(self._dt, _lib.LAYOUT_NHWC, self._is_max, *self._geom(),
+                                               self._in(x, "x"), self.y.out, self.idx_max.gpudata if self._is_max else None,
+                                               m.stream_handle))
+        self.y.written()
         return self.y
 
     def backward(self, dy):
         if self.need_dx:
             m = self.model
-            _lib.check(_lib.lib().b2c_pool_backward(self._dt, _layout(m), self._is_max, *self._geom(), dy.ptr,
-                                                    self.idx_max.gpudata if self._is_max else None, self.dx.ptr,
-                                                    m.stream_handle))
+            _lib.check(_lib.lib().b2c_pool_backward(self._dt, _lib.LAYOUT_NHWC, self._is_max, *self._geom(),
+                                                    self._in(dy, "dy"), self.idx_max.gpudata if self._is_max else None,
+                                                    self.dx.out, m.stream_handle))
+            self.dx.written()
             return self.dx
 
 
@@ -294,6 +330,14 @@ class AdditionBlockGPU(LayerGPU, AdditionBlock):
             return None
         return bn
 
+    def _add(self, acc, other):
+        """acc += other, in the buffer ``acc`` is kept in."""
+        if acc.channel_last() is not None:
+            _lib.check(_lib.lib().b2c_add_inplace(self._dt, acc.size, acc.out, self._in(other, "other"), self.model.stream_handle))
+            acc.written()
+        else:
+            _lib.check(_lib.lib().b2c_add_inplace(self._dt, acc.size, acc.ptr, other.ptr, self.model.stream_handle))
+
     def forward(self, x):
         L = _lib.lib()
         bn = self._fold_sum_into_last_bn()
@@ -317,10 +361,11 @@ class AdditionBlockGPU(LayerGPU, AdditionBlock):
                 self.y = y_i
             elif i == last and self.relu_after is not None:
                 # residual sum and the ReLU that follows in one pass: relu.y = max(y + y_i, 0)
-                _lib.check(L.b2c_add_relu(self._dt, self.y.size, self.y.ptr, y_i.ptr, self.relu_after.y.ptr,
-                                          self.model.stream_handle))
+                _lib.check(L.b2c_add_relu(self._dt, self.y.size, self._in(self.y, "y"), self._in(y_i, "other"),
+                                          self.relu_after.y.out, self.model.stream_handle))
+                self.relu_after.y.written()
             else:
-                _lib.check(L.b2c_add_inplace(self._dt, self.y.size, self.y.ptr, y_i.ptr, self.model.stream_handle))
+                self._add(self.y, y_i)
         return self.y
 
     def backward(self, dy):
@@ -335,10 +380,11 @@ class AdditionBlockGPU(LayerGPU, AdditionBlock):
             elif i == len(self.paths) - 1 and self.relu_before is not None:
                 # the sum of the branch gradients and the backward of the ReLU that feeds this block in one pass
                 r = self.relu_before
-                _lib.check(L.b2c_add_relu_backward(self._dt, dx0.size, dx0.ptr, dx_i.ptr, r.y.ptr, r.dx.ptr,
-                                                   self.model.stream_handle))
+                _lib.check(L.b2c_add_relu_backward(self._dt, dx0.size, self._in(dx0, "dx0"), self._in(dx_i, "other"),
+                                                   self._in(r.y, "relu"), r.dx.out, self.model.stream_handle))
+                r.dx.written()
             else:
-                _lib.check(L.b2c_add_inplace(self._dt, dx0.size, dx0.ptr, dx_i.ptr, self.model.stream_handle))
+                self._add(dx0, dx_i)
         self.dx = dx0
         return dx0
 

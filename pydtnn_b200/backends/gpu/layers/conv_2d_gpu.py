@@ -7,7 +7,7 @@ import numpy as np
 
 from .... import _lib, tracer
 from ....layers import Conv2D, Conv2DBatchNormalization, Conv2DBatchNormalizationRelu, Conv2DRelu
-from ....tensor_gpu import TensorGPU, empty
+from ....tensor_gpu import TensorGPU
 from ....utils import PYDTNN_TENSOR_FORMAT_NCHW, PYDTNN_TENSOR_FORMAT_NHWC, TRAIN_MODE
 from .. import memory_allocation as wsp
 from .layer_gpu import LayerGPU
@@ -21,12 +21,14 @@ class Conv2DGPU(LayerGPU, Conv2D):
         self.engine = _lib.ENGINE_AUTO
         self.stats_for_bn = None         # set by the model's fusion pass: the BatchNormalization this layer feeds
         self.stats_bytes = 0
+        self._x_ptr = None
 
     def _make_desc(self):
         m = self.model
         nchw = m.tensor_format == PYDTNN_TENSOR_FORMAT_NCHW
+        # activations are channel-last in either format (ChannelLastTensor); the filters keep the format's layout
         return _lib.ConvDesc(
-            layout=_lib.LAYOUT_NCHW if nchw else _lib.LAYOUT_NHWC, dtype=_lib.dtype_code(m.dtype),
+            layout=_lib.LAYOUT_NHWC, dtype=_lib.dtype_code(m.dtype),
             w_layout=_lib.W_KCRS if nchw else _lib.W_KRSC, engine=getattr(m, "conv_engine", self.engine),
             n=m.batch_size, h=self.hi, w=self.wi, ci=self.ci, co=self.co, kh=self.kh, kw=self.kw,
             vpad=self.vpadding, hpad=self.hpadding, vstr=self.vstride, hstr=self.hstride,
@@ -48,9 +50,9 @@ class Conv2DGPU(LayerGPU, Conv2D):
             b_arr, db_arr = m.arena.alloc_param(self.biases_cpu)
             self.biases = TensorGPU(b_arr, m.tensor_format)
             self.db = TensorGPU(db_arr, m.tensor_format)
-        self.y = TensorGPU(empty((m.batch_size, *self.shape), m.dtype), m.tensor_format)
+        self.y = self._activation((m.batch_size, *self.shape))
         if self.need_dx:
-            self.dx = TensorGPU(empty(self.x.ary.shape, m.dtype), m.tensor_format)
+            self.dx = self._activation(self.x.dims)
         self.desc = self._make_desc()
         L = _lib.lib()
         need = max(L.b2c_conv_workspace_bytes(ctypes.byref(self.desc), p) for p in
@@ -64,7 +66,7 @@ class Conv2DGPU(LayerGPU, Conv2D):
         self._lowered_valid = False
         if L.b2c_conv_keeps_lowered_input(ctypes.byref(self.desc)):
             import torch
-            self._own_ws = torch.empty(int(need), dtype=torch.uint8, device=self.y.ary.t.device)
+            self._own_ws = torch.empty(int(need), dtype=torch.uint8, device=m.device)
         # can this layer's forward pass leave the batch sums of its output for a following batch norm?
         self.stats_bytes = int(L.b2c_conv_stats_bytes(ctypes.byref(self.desc)))
 
@@ -94,6 +96,7 @@ class Conv2DGPU(LayerGPU, Conv2D):
 
     def forward(self, x):
         L = _lib.lib()
+        x_ptr = self._x_ptr = self._in(x, "x")
         self.x = x          # backward reads the tensor this call saw (a fused predecessor may hand over its own buffer)
         bn = self.stats_for_bn
         ws_ptr, ws_size = (self._own_ws.data_ptr(), self._own_ws.numel()) if self._own_ws is not None else (wsp.ptr(), wsp.size())
@@ -102,36 +105,42 @@ class Conv2DGPU(LayerGPU, Conv2D):
             # training step, a batch norm follows: the same pass also sums y and y^2 per channel while the tiles leave
             st = wsp.conv_stats()
             self._timed("fprop", lambda: L.b2c_conv_fprop_stats(
-                ctypes.byref(self.desc), x.ptr, self.weights.ptr, self.biases.ptr if self.use_bias else None,
-                self.y.ptr, st.data_ptr(), self.stats_bytes, ws_ptr, ws_size, self.model.stream_handle))
+                ctypes.byref(self.desc), x_ptr, self.weights.ptr, self.biases.ptr if self.use_bias else None,
+                self.y.out, st.data_ptr(), self.stats_bytes, ws_ptr, ws_size, self.model.stream_handle))
+            self.y.written()
             bn.prestats = (st, self.stats_bytes)
             return self.y
         self._timed("fprop", lambda: L.b2c_conv_fprop(
-            ctypes.byref(self.desc), x.ptr, self.weights.ptr, self.biases.ptr if self.use_bias else None, None, 0,
-            self.y.ptr, ws_ptr, ws_size, self.model.stream_handle))
+            ctypes.byref(self.desc), x_ptr, self.weights.ptr, self.biases.ptr if self.use_bias else None, None, 0,
+            self.y.out, ws_ptr, ws_size, self.model.stream_handle))
+        self.y.written()
         return self.y
 
-    def _wgrad_call(self, dy, ws_ptr, ws_size, stream):
+    def _wgrad_call(self, dy_ptr, ws_ptr, ws_size, stream):
         """The weight-gradient call on ``stream``; a layer that still holds its forward pass's lowered input in its own
         workspace uses that instead of lowering x again."""
         L = _lib.lib()
         db = self.db.ptr if self.use_bias else None
+        if self._x_ptr is None:
+            self._x_ptr = self._in(self.x, "x")
         if self._lowered_valid:
             self._lowered_valid = False
             own = self._own_ws
-            return lambda: L.b2c_conv_wgrad_lowered(ctypes.byref(self.desc), self.x.ptr, dy.ptr, self.dw.ptr, db, own.data_ptr(),
+            return lambda: L.b2c_conv_wgrad_lowered(ctypes.byref(self.desc), self._x_ptr, dy_ptr, self.dw.ptr, db, own.data_ptr(),
                                                     own.numel(), stream)
-        return lambda: L.b2c_conv_wgrad(ctypes.byref(self.desc), self.x.ptr, dy.ptr, self.dw.ptr, db, ws_ptr, ws_size, stream)
+        return lambda: L.b2c_conv_wgrad(ctypes.byref(self.desc), self._x_ptr, dy_ptr, self.dw.ptr, db, ws_ptr, ws_size, stream)
 
     def backward(self, dy):
         L = _lib.lib()
         m = self.model
+        dy_ptr = self._in(dy, "dy")
         side = m.side_stream_for_wgrad()
         if side is None:
-            self._timed("wgrad", self._wgrad_call(dy, wsp.ptr(), wsp.size(), m.stream_handle))
+            self._timed("wgrad", self._wgrad_call(dy_ptr, wsp.ptr(), wsp.size(), m.stream_handle))
             if self.need_dx:
                 self._timed("dgrad", lambda: L.b2c_conv_dgrad(
-                    ctypes.byref(self.desc), dy.ptr, self.weights.ptr, self.dx.ptr, wsp.ptr(), wsp.size(), m.stream_handle))
+                    ctypes.byref(self.desc), dy_ptr, self.weights.ptr, self.dx.out, wsp.ptr(), wsp.size(), m.stream_handle))
+                self.dx.written()
                 return self.dx
             return None
         # The weight gradient only has to be there when the gradients are exchanged or applied, so it runs on a side
@@ -144,11 +153,12 @@ class Conv2DGPU(LayerGPU, Conv2D):
             self._dy_ready, self._wgrad_done = torch.cuda.Event(), torch.cuda.Event()
         self._dy_ready.record()
         if self.need_dx:
-            _lib.check(L.b2c_conv_dgrad(ctypes.byref(self.desc), dy.ptr, self.weights.ptr, self.dx.ptr, wsp.ptr(), wsp.size(),
+            _lib.check(L.b2c_conv_dgrad(ctypes.byref(self.desc), dy_ptr, self.weights.ptr, self.dx.out, wsp.ptr(), wsp.size(),
                                         m.stream_handle))
+            self.dx.written()
         side.wait_event(self._dy_ready)
         sw = wsp.side()
-        _lib.check(self._wgrad_call(dy, sw.data_ptr(), sw.numel(), side.cuda_stream)())
+        _lib.check(self._wgrad_call(dy_ptr, sw.data_ptr(), sw.numel(), side.cuda_stream)())
         self._wgrad_done.record(side)
         m.note_side_work(self._wgrad_done)
         return self.dx if self.need_dx else None
@@ -189,10 +199,12 @@ class _FusedConvInference(Conv2DGPU):
         if self._with_bn:
             self._refresh_bn()
         L = _lib.lib()
+        x_ptr = self._in(x, "x")
         self._timed("fprop", lambda: L.b2c_conv_fprop(
-            ctypes.byref(self.desc), x.ptr, self.weights.ptr, self.biases.ptr if self.use_bias else None,
+            ctypes.byref(self.desc), x_ptr, self.weights.ptr, self.biases.ptr if self.use_bias else None,
             ctypes.byref(self._bn) if self._with_bn else None, int(self._relu_flag()),
-            self.y.ptr, wsp.ptr(), wsp.size(), self.model.stream_handle))
+            self.y.out, wsp.ptr(), wsp.size(), self.model.stream_handle))
+        self.y.written()
         return self.y
 
     def backward(self, dy):

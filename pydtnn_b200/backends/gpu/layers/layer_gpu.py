@@ -9,6 +9,7 @@ from abc import ABC
 
 from .... import tracer
 from ....layers.base import Layer
+from ....tensor_gpu import ChannelLastTensor, TensorGPU, empty, transpose_inner
 
 
 class LayerGPU(Layer, ABC):
@@ -22,10 +23,32 @@ class LayerGPU(Layer, ABC):
         self.dx = None
         self.dw = None
         self.db = None
+        self._copies = {}
 
     def initialize(self, prev_shape, need_dx, x):
         self.x = x  # must be set before super().initialize()
         super().initialize(prev_shape, need_dx)
+
+    # -- activations ---------------------------------------------------------------------
+    def _activation(self, dims):
+        """A buffer for an activation or its gradient (``dims`` in the model's tensor format)."""
+        m = self.model
+        if m.channels_last and len(dims) == 4:
+            return ChannelLastTensor(dims, m.dtype, m.tensor_format)
+        return TensorGPU(empty(dims, m.dtype), m.tensor_format)
+
+    def _in(self, t, slot):
+        """Address of a tensor's values in the order this layer's kernels read (channel last).  A plain NCHW tensor
+        (the network's input, or one the caller made) is copied into a buffer this layer keeps per ``slot``."""
+        p = t.channel_last()
+        if p is None:
+            n, c, h, w = t.ary.shape
+            buf = self._copies.get(slot)
+            if buf is None or buf.shape != (n, h, w, c):
+                buf = self._copies[slot] = empty((n, h, w, c), t.ary.dtype, t.ary.t.device)
+            transpose_inner(t.ary, buf, n, c, h * w)
+            p = buf.gpudata
+        return p
 
     # -- gradient exchange ---------------------------------------------------------------
     def _grad_tensors(self):

@@ -155,6 +155,13 @@ extern "C" int b2c_conv_index_map(const b2c_conv_desc* desc, int64_t* map, void*
     return fma_index_map(g, map, (cudaStream_t)stream);
 }
 
+extern "C" int b2c_transpose(int dtype, int n, int rows, int cols, const void* src, void* dst, void* stream) {
+    if (dtype < 0 || dtype > 1) return B2C_ERR_BAD_ENUM;
+    if (n <= 0 || rows <= 0 || cols <= 0) return B2C_ERR_BAD_GEOMETRY;
+    if (!src || !dst) return B2C_ERR_NULL_POINTER;
+    return transpose_images(dtype, src, dst, n, rows, cols, (cudaStream_t)stream);
+}
+
 extern "C" size_t b2c_fc_workspace_bytes(int dtype, int batch, int in_f, int out_f, int engine) {
     Geo g; if (fc_geo(dtype, engine, batch, in_f, out_f, g)) return 0;
     size_t m = 0;

@@ -118,6 +118,7 @@ int tc_wgrad(const Geo& g, const void* x, const void* dy, void* dw, void* db, vo
 int tc_read_status(int* out);
 bool tc_keeps_lowered(const Geo& g);
 int tc_wgrad_lowered(const Geo& g, const void* x, const void* dy, void* dw, void* db, void* ws, size_t ws_bytes, cudaStream_t st);
+int transpose_images(int dtype, const void* src, void* dst, int n, int rows, int cols, cudaStream_t st);
 bool tc_fc_small_batch(int dtype, int engine, int batch, int in_f, int out_f);
 size_t tc_fc_small_batch_bytes(int batch, int in_f, int out_f);
 int tc_fc_forward_small_batch(int batch, int in_f, int out_f, const void* x, const void* w, const void* bias, void* y,

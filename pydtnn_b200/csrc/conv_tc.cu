@@ -2138,16 +2138,17 @@ static int tc_wgrad_nhwc(const Geo& g, const void* x, const void* dy, void* dw, 
 // is read through strides).  Taken when the transposes cost less than the FMA engine would lose.
 // ---------------------------------------------------------------------------------------------
 // src [n][rows][cols] -> dst [n][cols][rows]; block (32, 8), grid (cols/32, rows/32, n)
-__global__ void transpose_inner_kernel(const float* __restrict__ src, float* __restrict__ dst, int rows, int cols)
+template <typename T>
+__global__ void transpose_inner_kernel(const T* __restrict__ src, T* __restrict__ dst, int rows, int cols)
 {
     pdl_prologue();
-    __shared__ float tile[32][33];
+    __shared__ T tile[32][33];
     const int64_t plane = (int64_t)rows * cols;
     const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32, tx = threadIdx.x, ty = threadIdx.y;
     {
         const int img = blockIdx.z;
-        const float* s = src + img * plane;
-        float* d = dst + img * plane;
+        const T* s = src + img * plane;
+        T* d = dst + img * plane;
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             const int r = r0 + ty + 8 * j, c = c0 + tx;
@@ -2166,16 +2167,16 @@ __global__ void transpose_inner_kernel(const float* __restrict__ src, float* __r
 // leave nine tenths of its threads idle.  One thread per position of the long axis; ROWS_THIN: src [n][thin][len]
 // -> dst [n][len][thin], else src [n][len][thin] -> dst [n][thin][len].  Loads or stores of a warp cover whole
 // contiguous runs either way.
-template <bool ROWS_THIN>
-__global__ void __launch_bounds__(256) transpose_thin_kernel(const float* __restrict__ src, float* __restrict__ dst, int thin, int len)
+template <typename T, bool ROWS_THIN>
+__global__ void __launch_bounds__(256) transpose_thin_kernel(const T* __restrict__ src, T* __restrict__ dst, int thin, int len)
 {
     pdl_prologue();
     const int l = blockIdx.x * blockDim.x + threadIdx.x;
     if (l >= len) return;
     const int64_t plane = (int64_t)thin * len;
-    const float* s = src + blockIdx.y * plane;
-    float* d = dst + blockIdx.y * plane;
-    float v[8];
+    const T* s = src + blockIdx.y * plane;
+    T* d = dst + blockIdx.y * plane;
+    T v[8];
 #pragma unroll
     for (int r = 0; r < 8; r++)
         if (r < thin) v[r] = ROWS_THIN ? s[(int64_t)r * len + l] : s[(int64_t)l * thin + r];
@@ -2184,20 +2185,35 @@ __global__ void __launch_bounds__(256) transpose_thin_kernel(const float* __rest
         if (r < thin) { if (ROWS_THIN) d[(int64_t)l * thin + r] = v[r]; else d[(int64_t)r * len + l] = v[r]; }
 }
 
-static int transpose_inner(const void* src, void* dst, int n, int rows, int cols, cudaStream_t st)
+template <typename T>
+static int transpose_t(const void* src, void* dst, int n, int rows, int cols, cudaStream_t st)
 {
-    if (n > 65535) return B2C_ERR_TOO_LARGE;
+    if ((rows + 31) / 32 > 65535) return B2C_ERR_TOO_LARGE;
+    if (n > 65535) {                                  // the image index is a grid axis: in parts
+        const size_t part = (size_t)65535 * rows * cols * sizeof(T);
+        const int rc = transpose_t<T>(src, dst, 65535, rows, cols, st);
+        return rc ? rc : transpose_t<T>((const char*)src + part, (char*)dst + part, n - 65535, rows, cols, st);
+    }
     if (rows <= 8 && cols > 8) {
-        launch_pdl(transpose_thin_kernel<true>, dim3((cols + 255) / 256, n), 256, 0, st, (const float*)src, (float*)dst, rows, cols);
+        launch_pdl(transpose_thin_kernel<T, true>, dim3((cols + 255) / 256, n), 256, 0, st, (const T*)src, (T*)dst, rows, cols);
         return check_launch("transpose_thin_kernel");
     }
     if (cols <= 8 && rows > 8) {
-        launch_pdl(transpose_thin_kernel<false>, dim3((rows + 255) / 256, n), 256, 0, st, (const float*)src, (float*)dst, cols, rows);
+        launch_pdl(transpose_thin_kernel<T, false>, dim3((rows + 255) / 256, n), 256, 0, st, (const T*)src, (T*)dst, cols, rows);
         return check_launch("transpose_thin_kernel");
     }
-    launch_pdl(transpose_inner_kernel, dim3((cols + 31) / 32, (rows + 31) / 32, n), dim3(32, 8), 0, st,
-               (const float*)src, (float*)dst, rows, cols);
+    launch_pdl(transpose_inner_kernel<T>, dim3((cols + 31) / 32, (rows + 31) / 32, n), dim3(32, 8), 0, st,
+               (const T*)src, (T*)dst, rows, cols);
     return check_launch("transpose_inner_kernel");
+}
+
+int transpose_images(int dtype, const void* src, void* dst, int n, int rows, int cols, cudaStream_t st)
+{
+    return dtype == B2C_F32 ? transpose_t<float>(src, dst, n, rows, cols, st) : transpose_t<double>(src, dst, n, rows, cols, st);
+}
+static int transpose_inner(const void* src, void* dst, int n, int rows, int cols, cudaStream_t st)
+{
+    return transpose_t<float>(src, dst, n, rows, cols, st);
 }
 
 static Geo as_nhwc(const Geo& g) { Geo q = g; q.layout = B2C_LAYOUT_NHWC; return q; }

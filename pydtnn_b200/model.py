@@ -52,6 +52,7 @@ class Model:
             self.tensor_format = PYDTNN_TENSOR_FORMAT_NCHW
         else:
             self.tensor_format = PYDTNN_TENSOR_FORMAT_NHWC
+        self.channels_last = self.tensor_format == PYDTNN_TENSOR_FORMAT_NCHW     # activations kept as ChannelLastTensor
         self.enable_fused_bn_relu = enable_fused_bn_relu
         self.enable_fused_conv_relu = enable_fused_conv_relu
         self.enable_fused_conv_bn = enable_fused_conv_bn
@@ -152,7 +153,7 @@ class Model:
                 # batch norm skips its own statistics pass over the tensor
                 if self.fuse_conv_bn_stats and type(a).__name__ == "Conv2DGPU" and type(b).__name__ == "BatchNormalizationGPU" \
                         and getattr(a, "stats_bytes", 0) and b.spatial and self.dtype == np.float32 \
-                        and self.tensor_format == PYDTNN_TENSOR_FORMAT_NHWC and _bn_fast_path(b.ci):
+                        and _bn_fast_path(b.ci):
                     a.stats_for_bn = b
                     wsp.require_conv_stats(a.stats_bytes)
                 # an addition block followed by a ReLU: the last residual sum writes max(sum, 0)
@@ -362,6 +363,7 @@ class Model:
         x = self.layers[0].y
         for layer in self._eval_layers[1:]:
             x = layer.forward(x)
+        x.ary          # the answer is the caller's: in the model's tensor format before this call returns
         if y_batch is None:
             return x
         self._ensure_loss()

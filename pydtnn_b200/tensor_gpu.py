@@ -9,6 +9,7 @@ import ctypes
 import numpy as np
 import torch
 
+from . import _lib
 from .utils import PYDTNN_TENSOR_FORMAT_NCHW
 
 _TORCH_DTYPE = {np.dtype(np.float32): torch.float32, np.dtype(np.float64): torch.float64,
@@ -94,3 +95,84 @@ class TensorGPU:
     def reshape(self, shape):
         self.ary = self.ary.reshape(shape)
         return self
+
+    # -- what the layers' kernels read and write (see ChannelLastTensor) --------------------------------------
+    @property
+    def dims(self):
+        """Shape without the promotion to 4-D."""
+        return self.ary.shape
+
+    def channel_last(self):
+        """Address of the values with the channel axis last, or None where they are stored otherwise."""
+        s = self.ary.shape
+        if self.tensor_format != PYDTNN_TENSOR_FORMAT_NCHW or len(s) != 4 or s[1] == 1 or s[2] * s[3] == 1:
+            return self.ary.gpudata
+        return None
+
+    @property
+    def out(self):
+        """Address a layer's kernel writes to; ``written()`` follows the call."""
+        return self.ary.gpudata
+
+    def written(self):
+        pass
+
+
+def transpose_inner(src, dst, n, rows, cols):
+    """dst[n][cols][rows] = src[n][rows][cols] (device arrays), on the current stream."""
+    _lib.check(_lib.lib().b2c_transpose(_lib.dtype_code(src.dtype), n, rows, cols, src.gpudata, dst.gpudata,
+                                        torch.cuda.current_stream(src.t.device).cuda_stream))
+
+
+class ChannelLastTensor(TensorGPU):
+    """An (n, c, h, w) activation of an NCHW model whose values are kept channel-last between the layers: every kernel
+    of this package runs channel-last, and in a network all neighbours of an activation are such kernels, so copying
+    each tensor to NCHW and back around every layer would be most of the step (measured on a ResNet-50 step, batch 32:
+    27.8 ms with NCHW storage).
+
+    Whoever looks at the tensor (``ary``, ``ptr``) gets a real NCHW buffer: it is made at the first look and from then
+    on the tensor is an NCHW buffer to everyone -- a layer that writes it brings the buffer up to date in the same call,
+    a layer that reads it takes what the buffer holds, so the caller may also write to it."""
+
+    def __init__(self, dims, dtype, tensor_format, tensor_type="tensor"):
+        n, c, h, w = dims
+        self._dims = self.shape = tuple(int(d) for d in dims)
+        self.size = n * c * h * w
+        self.tensor_format, self.tensor_type, self.desc = tensor_format, tensor_type, None
+        self._cl = empty((n, h, w, c), dtype)
+        self.same_order = c == 1 or h * w == 1              # both orders are the same bytes
+        self._nchw = DeviceArray(self._cl.t.view(self._dims)) if self.same_order else None
+
+    @property
+    def ary(self):
+        if self._nchw is None:
+            n, c, h, w = self._dims
+            self._nchw = empty(self._dims, self._cl.dtype, self._cl.t.device)
+            ChannelLastTensor.looks += 1
+            transpose_inner(self._cl, self._nchw, n, h * w, c)
+        return self._nchw
+
+    #: counts first looks in the process: a recorded sequence of launches is only valid while it has not moved
+    looks = 0
+
+    @property
+    def dims(self):
+        return self._dims
+
+    def channel_last(self):
+        if self._nchw is not None and not self.same_order:
+            n, c, h, w = self._dims
+            transpose_inner(self._nchw, self._cl, n, c, h * w)
+        return self._cl.gpudata
+
+    @property
+    def out(self):
+        return self._cl.gpudata
+
+    def written(self):
+        if self._nchw is not None and not self.same_order:
+            n, c, h, w = self._dims
+            transpose_inner(self._cl, self._nchw, n, h * w, c)
+
+    def reshape(self, shape):
+        return TensorGPU(self.ary.reshape(shape), self.tensor_format, tensor_type=self.tensor_type)
