@@ -31,6 +31,23 @@ static int pick_engine(const Geo& g, int pass, int& engine) {
     return B2C_OK;
 }
 
+// The engine of a call: the shape's, except that channel counts which are no whole blocks on 16-byte pixels also run
+// with pointers on any alignment, which only the FMA engine takes.
+static int call_engine(const Geo& g, int pass, const void* a, const void* b, int& engine) {
+    int rc = pick_engine(g, pass, engine);
+    if (!rc && engine == B2C_ENGINE_TENSOR && g.engine == B2C_ENGINE_AUTO && (((uintptr_t)a | (uintptr_t)b) & 15) && !tc_any_alignment(g, pass))
+        engine = B2C_ENGINE_FMA;
+    return rc;
+}
+static size_t pass_workspace_bytes(const Geo& g, int pass) {
+    int e; if (pick_engine(g, pass, e)) return 0;
+    if (e == B2C_ENGINE_FMA) return fma_workspace_bytes(g, pass);
+    const size_t t = tc_workspace_bytes(g, pass);
+    if (g.engine != B2C_ENGINE_AUTO || tc_any_alignment(g, pass)) return t;
+    const size_t f = fma_workspace_bytes(g, pass);
+    return t > f ? t : f;
+}
+
 // An FC layer is a 1x1 convolution over a (batch, 1, 1, in) NHWC tensor with a (in,1,1,out) filter.
 static int fc_geo(int dtype, int engine, int batch, int in_f, int out_f, Geo& g) {
     b2c_conv_desc d{};
@@ -84,8 +101,7 @@ extern "C" int b2c_conv_engine_for(const b2c_conv_desc* desc, int pass) {
 extern "C" size_t b2c_conv_workspace_bytes(const b2c_conv_desc* desc, int pass) {
     Geo g; if (make_geo(desc, g)) return 0;
     if (pass < 0 || pass > 2) return 0;
-    int e; if (pick_engine(g, pass, e)) return 0;
-    return e == B2C_ENGINE_TENSOR ? tc_workspace_bytes(g, pass) : fma_workspace_bytes(g, pass);
+    return pass_workspace_bytes(g, pass);
 }
 
 extern "C" int b2c_conv_fprop(const b2c_conv_desc* desc, const void* x, const void* w, const void* bias,
@@ -93,7 +109,7 @@ extern "C" int b2c_conv_fprop(const b2c_conv_desc* desc, const void* x, const vo
     Geo g; int rc = make_geo(desc, g); if (rc) return rc;
     if (!x || !w || !y) return B2C_ERR_NULL_POINTER;
     if (bn && (!bn->mean || !bn->inv_std || !bn->gamma || !bn->beta)) return B2C_ERR_NULL_POINTER;
-    int e; rc = pick_engine(g, B2C_PASS_FPROP, e); if (rc) return rc;
+    int e; rc = call_engine(g, B2C_PASS_FPROP, x, y, e); if (rc) return rc;
     if (e == B2C_ENGINE_TENSOR) return tc_fprop(g, x, w, bias, bn, relu, y, ws, ws_bytes, (cudaStream_t)stream);
     return fma_fprop(g, x, w, bias, bn, relu, y, ws, ws_bytes, (cudaStream_t)stream);
 }
@@ -110,7 +126,7 @@ extern "C" int b2c_conv_fprop_stats(const b2c_conv_desc* desc, const void* x, co
     Geo g; int rc = make_geo(desc, g); if (rc) return rc;
     if (!x || !w || !y || !stats) return B2C_ERR_NULL_POINTER;
     if (g.dtype != B2C_F32) return B2C_ERR_UNSUPPORTED;
-    int e; rc = pick_engine(g, B2C_PASS_FPROP, e); if (rc) return rc;
+    int e; rc = call_engine(g, B2C_PASS_FPROP, x, y, e); if (rc) return rc;
     if (e != B2C_ENGINE_TENSOR) return B2C_ERR_UNSUPPORTED;
     return tc_fprop_stats(g, x, w, bias, y, stats, stats_bytes, ws, ws_bytes, (cudaStream_t)stream);
 }
@@ -119,7 +135,7 @@ extern "C" int b2c_conv_dgrad(const b2c_conv_desc* desc, const void* dy, const v
                               void* ws, size_t ws_bytes, void* stream) {
     Geo g; int rc = make_geo(desc, g); if (rc) return rc;
     if (!dy || !w || !dx) return B2C_ERR_NULL_POINTER;
-    int e; rc = pick_engine(g, B2C_PASS_DGRAD, e); if (rc) return rc;
+    int e; rc = call_engine(g, B2C_PASS_DGRAD, dy, dx, e); if (rc) return rc;
     if (e == B2C_ENGINE_TENSOR) return tc_dgrad(g, dy, w, dx, ws, ws_bytes, (cudaStream_t)stream);
     return fma_dgrad(g, dy, w, dx, ws, ws_bytes, (cudaStream_t)stream);
 }
@@ -135,7 +151,7 @@ extern "C" int b2c_conv_wgrad_lowered(const b2c_conv_desc* desc, const void* x, 
                                       void* ws, size_t ws_bytes, void* stream) {
     Geo g; int rc = make_geo(desc, g); if (rc) return rc;
     if (!x || !dy || !dw) return B2C_ERR_NULL_POINTER;
-    int e; rc = pick_engine(g, B2C_PASS_WGRAD, e); if (rc) return rc;
+    int e; rc = call_engine(g, B2C_PASS_WGRAD, x, dy, e); if (rc) return rc;
     if (e != B2C_ENGINE_TENSOR) return B2C_ERR_UNSUPPORTED;
     return tc_wgrad_lowered(g, x, dy, dw, db, ws, ws_bytes, (cudaStream_t)stream);
 }
@@ -144,7 +160,7 @@ extern "C" int b2c_conv_wgrad(const b2c_conv_desc* desc, const void* x, const vo
                               void* ws, size_t ws_bytes, void* stream) {
     Geo g; int rc = make_geo(desc, g); if (rc) return rc;
     if (!x || !dy || !dw) return B2C_ERR_NULL_POINTER;
-    int e; rc = pick_engine(g, B2C_PASS_WGRAD, e); if (rc) return rc;
+    int e; rc = call_engine(g, B2C_PASS_WGRAD, x, dy, e); if (rc) return rc;
     if (e == B2C_ENGINE_TENSOR) return tc_wgrad(g, x, dy, dw, db, ws, ws_bytes, (cudaStream_t)stream);
     return fma_wgrad(g, x, dy, dw, db, ws, ws_bytes, (cudaStream_t)stream);
 }
@@ -166,8 +182,7 @@ extern "C" size_t b2c_fc_workspace_bytes(int dtype, int batch, int in_f, int out
     Geo g; if (fc_geo(dtype, engine, batch, in_f, out_f, g)) return 0;
     size_t m = 0;
     for (int pass = 0; pass < 3; pass++) {
-        int e; if (pick_engine(g, pass, e)) return 0;
-        size_t b = e == B2C_ENGINE_TENSOR ? tc_workspace_bytes(g, pass) : fma_workspace_bytes(g, pass);
+        size_t b = pass_workspace_bytes(g, pass);
         if (b > m) m = b;
     }
     if (tc_fc_small_batch(dtype, engine, batch, in_f, out_f)) {
@@ -183,7 +198,7 @@ extern "C" int b2c_fc_forward(int dtype, int engine, int batch, int in_f, int ou
     if (!x || !w || !y) return B2C_ERR_NULL_POINTER;
     if (tc_fc_small_batch(dtype, engine, batch, in_f, out_f))
         return tc_fc_forward_small_batch(batch, in_f, out_f, x, w, bias, y, ws, ws_bytes, (cudaStream_t)stream);
-    int e; rc = pick_engine(g, B2C_PASS_FPROP, e); if (rc) return rc;
+    int e; rc = call_engine(g, B2C_PASS_FPROP, x, y, e); if (rc) return rc;
     if (e == B2C_ENGINE_TENSOR) return tc_fprop(g, x, w, bias, nullptr, 0, y, ws, ws_bytes, (cudaStream_t)stream);
     return fma_fprop(g, x, w, bias, nullptr, 0, y, ws, ws_bytes, (cudaStream_t)stream);
 }
@@ -209,7 +224,7 @@ extern "C" int b2c_fc_backward(int dtype, int engine, int batch, int in_f, int o
     }
     if (dw) {
         if (!x) return B2C_ERR_NULL_POINTER;
-        int e; rc = pick_engine(g, B2C_PASS_WGRAD, e); if (rc) return rc;
+        int e; rc = call_engine(g, B2C_PASS_WGRAD, x, dy, e); if (rc) return rc;
         rc = e == B2C_ENGINE_TENSOR ? tc_wgrad(g, x, dy, dw, db, ws, ws_bytes, st) : fma_wgrad(g, x, dy, dw, db, ws, ws_bytes, st);
         if (rc) return rc;
     } else if (db) {
@@ -219,7 +234,7 @@ extern "C" int b2c_fc_backward(int dtype, int engine, int batch, int in_f, int o
     }
     if (dx) {
         if (!w) return B2C_ERR_NULL_POINTER;
-        int e; rc = pick_engine(g, B2C_PASS_DGRAD, e); if (rc) return rc;
+        int e; rc = call_engine(g, B2C_PASS_DGRAD, dy, dx, e); if (rc) return rc;
         rc = e == B2C_ENGINE_TENSOR ? tc_dgrad(g, dy, w, dx, ws, ws_bytes, st) : fma_dgrad(g, dy, w, dx, ws, ws_bytes, st);
     }
     return rc;

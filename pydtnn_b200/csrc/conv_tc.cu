@@ -39,6 +39,7 @@
 #include <cuda.h>
 #include <stdlib.h>
 #include <mutex>
+#include <type_traits>
 
 namespace b2c {
 
@@ -262,10 +263,11 @@ __device__ long long g_tc_prof[32];
 // Filter preparation: hi/lo split into the K-major GEMM layout the fprop/dgrad kernel reads by TMA
 // ---------------------------------------------------------------------------------------------
 struct PrepParams {
-    int rows, C, R, S;               // output is [rows][(r*S+s)*C + c], r < R, s < S (virtual taps)
+    int rows, C, R, S;               // output is [rows][(r*S+s)*Cp + c], r < R, s < S (virtual taps), zero for C <= c < Cp
     int64_t s_row, s_c, s_r, s_s;    // element strides of the source filter by (row, c, r, s)
     int r0, rstep, s0, sstep;        // real tap of virtual tap (r, s): (r0 + rstep*r, s0 + sstep*s)
     int Rreal, Sreal;                // extent of the real filter
+    int Cp;                          // C up to a multiple of 32 (set by run_fwd)
 };
 
 // Also clears `nflags` ints at `flags` (the hand-over flags of the balanced mode of the convolution kernel that
@@ -275,14 +277,14 @@ __global__ void tc_prep_filter_kernel(PrepParams p, const float* __restrict__ w,
 {
     pdl_prologue();
     if (blockIdx.x == 0) for (int i = threadIdx.x; i < nflags; i += blockDim.x) flags[i] = 0;
-    int64_t K = (int64_t)p.R * p.S * p.C;
+    int64_t K = (int64_t)p.R * p.S * p.Cp;
     int64_t total = (int64_t)p.rows * K;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
         int row = (int)(i / K);
         int k = (int)(i - (int64_t)row * K);
-        int c = k % p.C; int rs = k / p.C; int r = rs / p.S; int s = rs - r * p.S;
+        int c = k % p.Cp; int rs = k / p.Cp; int r = rs / p.S; int s = rs - r * p.S;
         r = p.r0 + p.rstep * r; s = p.s0 + p.sstep * s;
-        float v = w[row * p.s_row + c * p.s_c + r * p.s_r + s * p.s_s];
+        float v = c < p.C ? w[row * p.s_row + c * p.s_c + r * p.s_r + s * p.s_s] : 0.f;
         float h = to_tf32_rn(v);
         hi[i] = h;
         lo[i] = v - h;
@@ -295,7 +297,7 @@ __global__ void tc_prep_filter_kernel(PrepParams p, const float* __restrict__ w,
 // 32 columns, and the layer then runs as a 1x1 convolution over it.  With C*R*S small the matrix costs
 // less HBM traffic than the output tensor it produces.
 // ---------------------------------------------------------------------------------------------
-struct LowerParams { int n, h, w, c, ho, wo, kh, kw, vpad, hpad, vstr, hstr, vdil, hdil, K, Kp; };
+struct LowerParams { int n, h, w, c, ho, wo, kh, kw, vpad, hpad, vstr, hstr, vdil, hdil, K, Kp; int64_t sn, sh, sw, sc; };      // s*: strides of x, whose layout is free
 
 // The grid's thread count is a multiple of the float4 count of a row (Kp / 4), so a thread keeps its column
 // group for the whole grid-stride loop: the four (tap, channel) pairs are decoded once into registers and the
@@ -308,13 +310,14 @@ __global__ void tc_lower_kernel(LowerParams p, const float* __restrict__ x, floa
     const int64_t threads = (int64_t)gridDim.x * blockDim.x;          // multiple of kq (see launch_lower)
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int q4 = (int)(i % kq);
-    int dh[4], dwc[4], off[4];
+    int dh[4], dwc[4];
+    int64_t off[4];
 #pragma unroll
     for (int e = 0; e < 4; e++) {
         const int k = q4 * 4 + e;
         if (k < p.K) {
             const int c = k % p.c, rs = k / p.c, r = rs / p.kw, sx = rs - r * p.kw;
-            dh[e] = r * p.vdil; dwc[e] = sx * p.hdil; off[e] = (dh[e] * p.w + dwc[e]) * p.c + c;
+            dh[e] = r * p.vdil; dwc[e] = sx * p.hdil; off[e] = dh[e] * p.sh + dwc[e] * p.sw + c * p.sc;
         } else { dh[e] = 1 << 28; dwc[e] = 0; off[e] = 0; }          // padding column: always out of range
     }
     int64_t m = i / kq;
@@ -325,7 +328,7 @@ __global__ void tc_lower_kernel(LowerParams p, const float* __restrict__ x, floa
     const int s_h = (int)(step % p.ho); const int s_n = (int)(step / p.ho);
     for (; i < total; i += threads) {
         const int h0 = oh * p.vstr - p.vpad, w0 = ow * p.hstr - p.hpad;
-        const float* base = x + (((int64_t)nn * p.h + h0) * p.w + w0) * p.c;
+        const float* base = x + nn * p.sn + h0 * p.sh + w0 * p.sw;
         float v[4];
 #pragma unroll
         for (int e = 0; e < 4; e++)
@@ -351,12 +354,12 @@ __global__ void tc_lower_rows_kernel(LowerParams p, const float* __restrict__ x,
     for (int r = 0; r < p.kh; r++) {
         const int ih = oh * p.vstr - p.vpad + r * p.vdil;
         const bool row_in = (unsigned)ih < (unsigned)p.h;
-        const float* src = x + ((int64_t)nn * p.h + ih) * p.w * p.c;
+        const float* src = x + nn * p.sn + ih * p.sh;
         for (int j = threadIdx.x; j < wp; j += blockDim.x) {
             const int iw = j - p.hpad;
             const bool in = row_in && (unsigned)iw < (unsigned)p.w;
             float* dst = patch + r * rowlen + j * p.c;
-            for (int c = 0; c < p.c; c++) dst[c] = in ? __ldg(src + (int64_t)iw * p.c + c) : 0.f;
+            for (int c = 0; c < p.c; c++) dst[c] = in ? __ldg(src + iw * p.sw + c * p.sc) : 0.f;
         }
     }
     __syncthreads();
@@ -417,7 +420,9 @@ struct TcParams {
     int P, Q;                  // pixel grid per image the pixel index runs over
     int kblocks;               // FWD: taps * cblocks.  WGRAD: 32-pixel blocks per split
     int cblocks, S;            // channel blocks of 32 per tap, filter width
-    int C;                     // gathered channels per tap
+    int C;                     // WGRAD: rows per tap, the channels up to a multiple of 32
+    int ktail;                 // FWD: MMA steps (of 8 channels) that the last channel block of a tap holds values for
+    int Np;                    // WGRAD: row pitch of the partial tiles and of db_partial, N up to a multiple of 4
     int str_h, str_w, dil_h, dil_w;
     int low_h, low_w;          // lower corner of the im2col window (= -padding for a plain convolution)
     int Mpix;                  // WGRAD: total pixels
@@ -811,7 +816,6 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         // Converged warp, one elected lane issues (see elect_one_sync).
         {
             constexpr bool B_MN = MODE == TCM_WGRAD || BSRC == TCB_RAW_MN;
-            constexpr uint32_t idesc = make_idesc_tf32(128, BN, 0, B_MN);
             // B tiles, K-major (FWD): rows of 128 B, 8-row groups 1024 B apart, K advances 32 B inside the row.
             // B tiles, MN-major (WGRAD): 32-row (K) boxes of 4096 B per 32 N elements, 4-row swizzle atoms of
             // 512 B, K advances by 8 rows = 1024 B.  A comes from tensor memory, K advances 8 columns.
@@ -824,7 +828,16 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             TileWalk w;
             w.init(total_tiles, p.kblocks);
             while (ok && w.template next<SK>()) {
-                if (MULTI) w.kb_e = tile_geo(w.tile).kblocks;
+                const TileGeo tg = tile_geo(w.tile);
+                if (MULTI) w.kb_e = tg.kblocks;
+                // columns past the last channel are not computed (N of an MMA is a multiple of 16)
+                const int left = p.N - (tg.ltile % nt) * BN;
+                // and neither are the steps of a last channel block that hold only the zeros past the last channel
+                const uint32_t idesc = make_idesc_tf32(128, left >= BN ? BN : (left + 15) & ~15, 0, B_MN);
+                // The k-blocks of one tile.  WHOLE has operand shape and step count in constants: with them in registers
+                // (or a branch between the two forms per k-block) a long launch lost 3 to 6 % (2 %).
+                auto issue_tile = [&](auto whole_c) {
+                constexpr bool WHOLE = decltype(whole_c)::value;
                 for (int kb = w.kb_b; kb < w.kb_e && ok; kb++, it++) {
                     const int s = it % TSLOTS, use = it / TSLOTS;        // A slot in tensor memory (= the stage, unless the filters are resident)
                     const int b = gc & 1;
@@ -848,18 +861,24 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                     const uint32_t d = tmem_base + (uint32_t)(b * BN);
                     if (elect_one_sync()) {
                         // small terms first: lo*hi, hi*lo, then hi*hi
-#pragma unroll
-                        for (int k = 0; k < 4; k++) {
+                        auto step = [&](int k, uint32_t id) {
                             const uint64_t adv = (uint64_t)k * KADV;
 #ifdef B2C_TC_DEV
-                            if (p.dbg & 32) continue;
+                            if (p.dbg & 32) return;
 #endif
-                            umma_tf32_ts(d, a_lo + k * 8, b_hi + adv, idesc, (!chunk_start || k > 0) ? 1u : 0u);
+                            umma_tf32_ts(d, a_lo + k * 8, b_hi + adv, id, (!chunk_start || k > 0) ? 1u : 0u);
 #ifdef B2C_TC_DEV
-                            if (p.dbg & 2) continue;
+                            if (p.dbg & 2) return;
 #endif
-                            umma_tf32_ts(d, a_hi + k * 8, b_lo + adv, idesc, 1u);
-                            umma_tf32_ts(d, a_hi + k * 8, b_hi + adv, idesc, 1u);
+                            umma_tf32_ts(d, a_hi + k * 8, b_lo + adv, id, 1u);
+                            umma_tf32_ts(d, a_hi + k * 8, b_hi + adv, id, 1u);
+                        };
+                        if constexpr (WHOLE) {
+#pragma unroll
+                            for (int k = 0; k < 4; k++) step(k, make_idesc_tf32(128, BN, 0, B_MN));
+                        } else {
+                            const int ks = MODE == TCM_FWD && kb % p.cblocks == p.cblocks - 1 ? p.ktail : 4;
+                            for (int k = 0; k < ks; k++) step(k, idesc);
                         }
                         umma_commit(&empty_bar[s]);
                         if (chunk_end) umma_commit(&tfull_bar[b]);
@@ -868,6 +887,9 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                     if (chunk_end) gc++;
                     if (lane == 0) TC_PROF_ADD(4);    // MMA: issue
                 }
+                };
+                if (left > BN - 16 && (MODE == TCM_WGRAD || p.ktail == 4)) issue_tile(std::true_type{});
+                else issue_tile(std::false_type{});
             }
         }
     } else if (warp < 6) {
@@ -995,8 +1017,8 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                         v.z += __shfl_xor_sync(0xffffffffu, v.z, mask); v.w += __shfl_xor_sync(0xffffffffu, v.w, mask);
                     }
                     const int n = ni * BN + bx * 32;
-                    if (lane < 8 && n < p.N)
-                        *reinterpret_cast<float4*>(p.db_partial + ((size_t)z * 4 + (warp - 2)) * p.N + n + lane * 4) = v;
+                    if (lane < 8 && n + lane * 4 < p.N)
+                        *reinterpret_cast<float4*>(p.db_partial + ((size_t)z * 4 + (warp - 2)) * p.Np + n + lane * 4) = v;
                 }
             }
         }
@@ -1219,7 +1241,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                     my_off = tg.out_off + img * p.o_sn + pi * p.o_sh + qi * p.o_sw;
                     if (p.zfill) zmask = (2 * qi + 1 < p.z_W ? 1 : 0) | (2 * pi + 1 < p.z_H ? 2 : 0);
                 } else {
-                    my_off = ((int64_t)z * p.M + m) * p.N;
+                    my_off = ((int64_t)z * p.M + m) * p.Np;
                 }
             }
             if (ok && p.tma_store) {
@@ -1280,7 +1302,8 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
 
 // Second stage of the weight gradient: fixed-order sum of the per-split partial tiles, written in the
 // caller's filter layout.
-struct WgradReduceParams { int M, N, C, S, splits; int64_t sk, sc, sr, ss; int Mreal; };
+// C rows per tap of which the first Creal are channels, Np floats per row.
+struct WgradReduceParams { int M, N, C, S, splits; int64_t sk, sc, sr, ss; int Mreal, Creal, Np; };
 
 template <int ROWS>
 __global__ void __launch_bounds__(256) tc_wgrad_reduce_kernel(WgradReduceParams p, const float* __restrict__ partial, float* __restrict__ dw,
@@ -1292,7 +1315,7 @@ __global__ void __launch_bounds__(256) tc_wgrad_reduce_kernel(WgradReduceParams 
         const int n = blockIdx.x * 32 + threadIdx.x;
         if (threadIdx.y == 0 && n < p.N) {
             float v = 0.f;
-            for (int i = 0; i < p.splits * 4; i++) v += __ldcg(db_partial + (size_t)i * p.N + n);
+            for (int i = 0; i < p.splits * 4; i++) v += __ldcg(db_partial + (size_t)i * p.Np + n);
             db[n] = v;
         }
     }
@@ -1305,13 +1328,13 @@ __global__ void __launch_bounds__(256) tc_wgrad_reduce_kernel(WgradReduceParams 
     constexpr int TR = 8 * ROWS, U = 16 / ROWS;
     __shared__ float tile[TR][33];
     const int m0 = blockIdx.y * TR, n0 = blockIdx.x * 32;
-    const int64_t plane = (int64_t)p.M * p.N;
+    const int64_t plane = (int64_t)p.M * p.Np;
     const int n = n0 + threadIdx.x;
     float v[ROWS];
 #pragma unroll
     for (int r = 0; r < ROWS; r++) v[r] = 0.f;
     if (n < p.N) {
-        const float* src = partial + (int64_t)(m0 + threadIdx.y) * p.N + n;
+        const float* src = partial + (int64_t)(m0 + threadIdx.y) * p.Np + n;
         bool in[ROWS];
 #pragma unroll
         for (int r = 0; r < ROWS; r++) in[r] = m0 + threadIdx.y + 8 * r < p.M;
@@ -1321,7 +1344,7 @@ __global__ void __launch_bounds__(256) tc_wgrad_reduce_kernel(WgradReduceParams 
 #pragma unroll
             for (int u = 0; u < U; u++)
 #pragma unroll
-                for (int r = 0; r < ROWS; r++) q[u][r] = in[r] ? __ldcg(src + (int64_t)(z + u) * plane + (int64_t)(8 * r) * p.N) : 0.f;
+                for (int r = 0; r < ROWS; r++) q[u][r] = in[r] ? __ldcg(src + (int64_t)(z + u) * plane + (int64_t)(8 * r) * p.Np) : 0.f;
 #pragma unroll
             for (int u = 0; u < U; u++)
 #pragma unroll
@@ -1329,7 +1352,7 @@ __global__ void __launch_bounds__(256) tc_wgrad_reduce_kernel(WgradReduceParams 
         }
         for (; z < p.splits; z++)
 #pragma unroll
-            for (int r = 0; r < ROWS; r++) v[r] += in[r] ? __ldcg(src + (int64_t)z * plane + (int64_t)(8 * r) * p.N) : 0.f;
+            for (int r = 0; r < ROWS; r++) v[r] += in[r] ? __ldcg(src + (int64_t)z * plane + (int64_t)(8 * r) * p.Np) : 0.f;
     }
     if (p.sk == 1) {
         // output channels contiguous: store the row segments as they are
@@ -1338,7 +1361,7 @@ __global__ void __launch_bounds__(256) tc_wgrad_reduce_kernel(WgradReduceParams 
             const int m = m0 + threadIdx.y + 8 * r;
             if (m < p.Mreal && n < p.N) {            // rows >= Mreal: zero padding of a lowered few-channel layer
                 const int tap = m / p.C, c = m - tap * p.C, rr = tap / p.S, s = tap - rr * p.S;
-                dw[c * p.sc + rr * p.sr + s * p.ss + n] = v[r];
+                if (c < p.Creal) dw[c * p.sc + rr * p.sr + s * p.ss + n] = v[r];
             }
         }
         return;
@@ -1350,6 +1373,7 @@ __global__ void __launch_bounds__(256) tc_wgrad_reduce_kernel(WgradReduceParams 
     const int m = m0 + threadIdx.x;
     if (threadIdx.x >= TR || m >= p.Mreal) return;
     const int tap = m / p.C, c = m - tap * p.C, rr = tap / p.S, s = tap - rr * p.S;
+    if (c >= p.Creal) return;
     float* d = dw + c * p.sc + rr * p.sr + s * p.ss;
 #pragma unroll
     for (int j = 0; j < 4; j++) {
@@ -1370,7 +1394,7 @@ __global__ void __launch_bounds__(256) tc_wgrad_reduce_deep_kernel(WgradReducePa
     if (db && blockIdx.y == 0) {
         // bias gradient: [splits * 4] row sums per channel, shared among the thread rows the same way
         float v = 0.f;
-        if (n < p.N) for (int i = threadIdx.y; i < p.splits * 4; i += 8) v += __ldcg(db_partial + (size_t)i * p.N + n);
+        if (n < p.N) for (int i = threadIdx.y; i < p.splits * 4; i += 8) v += __ldcg(db_partial + (size_t)i * p.Np + n);
         part[threadIdx.y][threadIdx.x] = v;
         __syncthreads();
         if (threadIdx.y == 0 && n < p.N) {
@@ -1381,10 +1405,10 @@ __global__ void __launch_bounds__(256) tc_wgrad_reduce_deep_kernel(WgradReducePa
         }
         __syncthreads();
     }
-    const int64_t plane = (int64_t)p.M * p.N;
+    const int64_t plane = (int64_t)p.M * p.Np;
     float v = 0.f;
     if (n < p.N) {
-        const float* src = partial + (int64_t)m * p.N + n;
+        const float* src = partial + (int64_t)m * p.Np + n;
         int z = threadIdx.y;
         for (; z + 56 < p.splits; z += 64) {
             float q[8];
@@ -1402,7 +1426,7 @@ __global__ void __launch_bounds__(256) tc_wgrad_reduce_deep_kernel(WgradReducePa
 #pragma unroll
     for (int y = 0; y < 8; y++) t += part[y][threadIdx.x];
     const int tap = m / p.C, c = m - tap * p.C, rr = tap / p.S, s = tap - rr * p.S;
-    dw[(int64_t)n * p.sk + c * p.sc + rr * p.sr + s * p.ss] = t;
+    if (c < p.Creal) dw[(int64_t)n * p.sk + c * p.sc + rr * p.sr + s * p.ss] = t;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1430,12 +1454,12 @@ static bool load_driver_entry_points()
     return true;
 }
 
-// 2-D row-major float matrix [rows][cols], box = 32 columns x box_rows rows, 128B swizzle.
-static bool make_map_2d(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows,
+// 2-D row-major float matrix [rows][cols], rows `pitch` floats apart, box = 32 columns x box_rows rows, 128B swizzle.
+static bool make_map_2d(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t pitch, uint32_t box_rows,
                         CUtensorMapSwizzle swz = CU_TENSOR_MAP_SWIZZLE_128B)
 {
     cuuint64_t dims[2] = {cols, rows};
-    cuuint64_t strides[1] = {cols * sizeof(float)};
+    cuuint64_t strides[1] = {pitch * sizeof(float)};
     cuuint32_t box[2] = {32, box_rows};
     cuuint32_t estr[2] = {1, 1};
     return g_encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims, strides, box, estr,
@@ -1446,12 +1470,13 @@ static bool make_map_2d(CUtensorMap* map, const void* base, uint64_t rows, uint6
 // NHWC activation tensor (n, h, w, c) seen through an im2col window of `pixels` consecutive window
 // positions x 32 channels per load. The window's first position sits at (low_h, low_w); it has
 // `cnt_h` x `cnt_w` positions per image before the traversal stride is applied. Corners in (w, h) order.
-static bool make_map_im2col(CUtensorMap* map, const void* base, int n, int h, int w, int c, int low_h, int low_w,
+// Pixels lie `pitch` floats apart (a multiple of 4); channels from c on read as zeros.
+static bool make_map_im2col(CUtensorMap* map, const void* base, int n, int h, int w, int c, int pitch, int low_h, int low_w,
                             int cnt_h, int cnt_w, int str_h, int str_w, uint32_t pixels,
                             CUtensorMapSwizzle swz = CU_TENSOR_MAP_SWIZZLE_128B, uint32_t channels = 32)
 {
     cuuint64_t dims[4] = {(cuuint64_t)c, (cuuint64_t)w, (cuuint64_t)h, (cuuint64_t)n};
-    cuuint64_t strides[3] = {(cuuint64_t)c * 4, (cuuint64_t)w * c * 4, (cuuint64_t)h * w * c * 4};
+    cuuint64_t strides[3] = {(cuuint64_t)pitch * 4, (cuuint64_t)w * pitch * 4, (cuuint64_t)h * w * pitch * 4};
     int lower[2] = {low_w, low_h};
     int upper[2] = {cnt_w - w + low_w, cnt_h - h + low_h};
     for (int i = 0; i < 2; i++) if (lower[i] < -128 || lower[i] > 127 || upper[i] < -128 || upper[i] > 127) return false;
@@ -1484,25 +1509,34 @@ static AxisClass axis_class(int a, int str, int pad, int k, int in_len)
 
 // Few-channel layers run through the written-out im2row matrix (see tc_lower_kernel).
 static int lowered_kp(const Geo& g) { return (int)((g.K + 31) / 32 * 32); }
+static int round4(int v) { return (v + 3) & ~3; }
+static int round32(int v) { return (v + 31) & ~31; }
 static bool lowered_ok(const Geo& g)
 {
     if (g.ci % 32 == 0 || g.ci > 16) return false;
     if (g.K > 1024) return false;
-    return (int64_t)g.M * lowered_kp(g) * 4 <= (int64_t)3 << 30;
+    if ((int64_t)g.M * lowered_kp(g) * 4 > (int64_t)3 << 30) return false;
+    if (g.ci % 4) return true;          // the gather needs 16-byte pixels: the other way is a padded copy and one k-block per tap
+    // One k-block per tap read in place (its channels past ci cost loads, not products: about 0.4 us of an SM per 128
+    // rows), or K / 32 full ones (0.6 us) and the matrix written and read once (about 4 TB/s).
+    const double tiles = (double)((g.M + 127) / 128) * ((g.co + 127) / 128) / 148.0;
+    const double in_place = tiles * g.kh * g.kw * 0.4e-6;
+    const double lowered = tiles * (lowered_kp(g) / 32) * 0.6e-6 + (double)g.M * lowered_kp(g) * 8.0 / 4e12 + 3e-6;
+    return lowered < in_place;
 }
 
+// Any channel counts: blocks of 32 channels end in zeros past the last channel, pixels that are no multiple of 16 bytes
+// are copied to a pitch that is one (tc_copies).
 static bool tc_supported_nhwc(const Geo& g, int pass)
 {
     if (g.dtype != B2C_F32 || g.layout != B2C_LAYOUT_NHWC || g.engine == B2C_ENGINE_FMA) return false;
     if (g.vstr > 8 || g.hstr > 8) return false;
     if ((g.kh - 1) * g.vdil > 255 || (g.kw - 1) * g.hdil > 255 || g.vpad > 127 || g.hpad > 127) return false;
-    if (pass == B2C_PASS_FPROP) return (g.ci % 32 == 0 || lowered_ok(g)) && g.co % 4 == 0;
     if (pass == B2C_PASS_DGRAD) {
-        if (g.co % 32 || g.ci % 4) return false;
         if (g.vstr == 1 && g.hstr == 1) return (g.kh - 1) * g.vdil - g.vpad >= -127 && (g.kw - 1) * g.hdil - g.hpad >= -127;
         return g.vdil == 1 && g.hdil == 1;             // strided: parity-class decomposition, dilation 1 only
     }
-    return (g.ci % 32 == 0 || lowered_ok(g)) && g.co % 32 == 0;
+    return true;
 }
 
 // Function attributes and the SM count belong to a device, not to the process: both are kept per device ordinal
@@ -1580,8 +1614,11 @@ static size_t filter_split_bytes(const Geo& g, int pass)
 {
     int rows = pass == B2C_PASS_FPROP ? g.co : g.ci;
     int C = pass == B2C_PASS_FPROP ? g.ci : g.co;
-    return align_up((size_t)rows * g.kh * g.kw * C * sizeof(float), 1024);
+    return align_up((size_t)rows * g.kh * g.kw * round32(C) * sizeof(float), 1024);
 }
+
+// GEMM rows of a weight gradient: (tap, channel up to a multiple of 32), or the columns of the lowered matrix.
+static int64_t wgrad_rows(const Geo& g) { return lowered_ok(g) ? lowered_kp(g) : (int64_t)g.kh * g.kw * round32(g.ci); }
 
 struct WgradPlan { int splits, kblocks, bn; };
 // The pixel axis is cut into `splits` ranges of `kblocks` 32-pixel blocks; tiles x splits work items run on one
@@ -1592,7 +1629,7 @@ static WgradPlan wgrad_plan(const Geo& g)
 {
     WgradPlan pl;
     pl.bn = g.co <= 64 ? 64 : 128;
-    const int64_t Krows = g.ci % 32 == 0 ? g.K : lowered_kp(g);
+    const int64_t Krows = wgrad_rows(g);
     const int64_t tiles = ((Krows + 127) / 128) * ((g.co + pl.bn - 1) / pl.bn);
     const int64_t blocks = (g.M + 31) / 32;
     const double reduce_per_split = (double)Krows * g.co * 4.0 / 5e12 / 0.6e-6;   // k-block units (0.6 us each)
@@ -1622,7 +1659,7 @@ static bool wgrad_swap_ok(const Geo& g)
 static Geo wgrad_swapped(const Geo& g)
 {
     Geo q = g;
-    q.ci = g.co; q.co = g.ci; q.K = q.ci;
+    q.ci = g.co; q.co = g.ci; q.xp = g.yp; q.yp = g.xp; q.K = q.ci;
     return q;
 }
 
@@ -1635,14 +1672,14 @@ static size_t tc_workspace_bytes_nhwc(const Geo& g, int pass)
         const size_t b = align_up((size_t)pl.splits * g.K * g.co * sizeof(float), 1024) + 2048 + align_up((size_t)pl.splits * 4 * g.co * sizeof(float), 1024);
         return a > b ? a : b;
     }
-    const bool low = g.ci % 32 != 0;
+    const bool low = lowered_ok(g);
     const size_t lowered = low ? align_up((size_t)g.M * lowered_kp(g) * sizeof(float), 1024) : 0;
     if (pass == B2C_PASS_FPROP && low) return lowered + 2 * align_up((size_t)g.co * lowered_kp(g) * sizeof(float), 1024) + 2048;
-    if (pass == B2C_PASS_FPROP || pass == B2C_PASS_DGRAD) return 2 * filter_split_bytes(g, pass) + 1024 + sk_bytes();
+    if (pass == B2C_PASS_FPROP || pass == B2C_PASS_DGRAD)
+        return (pass == B2C_PASS_DGRAD && (g.vstr > 1 || g.hstr > 1) ? 3 : 2) * filter_split_bytes(g, pass) + 2048 + sk_bytes();
     WgradPlan pl = wgrad_plan(g);
-    const size_t Krows = low ? (size_t)lowered_kp(g) : (size_t)g.K;
-    return lowered + align_up((size_t)pl.splits * Krows * g.co * sizeof(float), 1024) + 2048 +
-           align_up((size_t)pl.splits * 4 * g.co * sizeof(float), 1024);
+    return lowered + align_up((size_t)pl.splits * wgrad_rows(g) * round4(g.co) * sizeof(float), 1024) + 2048 +
+           align_up((size_t)pl.splits * 4 * round4(g.co) * sizeof(float), 1024);
 }
 
 template <int MODE, int BN, int STAGES, bool SK, int SLABS, int BSRC, int STREAM = 0, bool MULTI = false, int RESKB = 0>
@@ -1721,14 +1758,14 @@ static bool make_map_filter(CUtensorMap* map, const void* base, uint64_t d0, uin
                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Output seen as [planes][rows][cols] floats, box = 32 cols x 32 rows (x 1 plane), 128B swizzle.
+// Output seen as [planes][rows][cols] floats, rows `pitch` floats apart, box = 32 cols x 32 rows (x 1 plane), 128B swizzle.
 // planes == 0 asks for the 2-D form (the forward kernel stores with 2-D coordinates, the weight-gradient
 // kernel always with 3-D ones, so the rank must match the kernel, not the data).
-static bool make_map_out(CUtensorMap* map, const void* base, uint64_t planes, uint64_t rows, uint64_t cols)
+static bool make_map_out(CUtensorMap* map, const void* base, uint64_t planes, uint64_t rows, uint64_t cols, uint64_t pitch)
 {
     if (planes == 0) {
         cuuint64_t dims[2] = {cols, rows};
-        cuuint64_t strides[1] = {cols * sizeof(float)};
+        cuuint64_t strides[1] = {pitch * sizeof(float)};
         cuuint32_t box[2] = {32, 32};
         cuuint32_t estr[2] = {1, 1};
         return g_encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims, strides, box, estr,
@@ -1736,13 +1773,16 @@ static bool make_map_out(CUtensorMap* map, const void* base, uint64_t planes, ui
                               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
     }
     cuuint64_t dims[3] = {cols, rows, planes};
-    cuuint64_t strides[2] = {cols * sizeof(float), rows * cols * sizeof(float)};
+    cuuint64_t strides[2] = {pitch * sizeof(float), rows * pitch * sizeof(float)};
     cuuint32_t box[3] = {32, 32, 1};
     cuuint32_t estr[3] = {1, 1, 1};
     return g_encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void*>(base), dims, strides, box, estr,
                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
+
+template <typename T>
+static int transpose_t(const void* src, void* dst, int n, int rows, int cols, int sp, int dp, cudaStream_t st);
 
 // fprop-shaped launch: `act` (n, ah, aw, C) gathered through a window whose first position is
 // (low_h, low_w), with cnt_h x cnt_w positions per image and traversal stride (str_h, str_w); virtual
@@ -1778,17 +1818,38 @@ static int64_t fwd_stats_rows(int64_t M, int N, int64_t kblocks, bool may_balanc
 // Stride-2 data gradient of a 1x1 filter: the launch writes class (0, 0) and the zeros of the other three (TcParams::zfill).
 struct ZeroFill { int W, H; int64_t off_w, off_h; };
 
+// A (co, ci, kh, kw) filter has no contiguous channel axis, so no tensor map can serve it.  Its K-major copy in real tap
+// order, [row][tap][C up to a multiple of 4], is a transpose either way round: (C x taps) per row when the rows are the
+// output channels, (C x rows * taps) when they are the input channels.  Then the strides of `pp` describe the copy.
+// Returns 1 when the filter is laid out otherwise (nothing done).  About 5 us for a 512 x 512 x 3 x 3 filter; the hi/lo copy it
+// spares the kernel's B operand from is twice the bytes and reads the filter across its rows.
+static int kmajor_filter_copy(PrepParams& pp, const void*& w, float* buf, cudaStream_t st)
+{
+    const int taps = pp.Rreal * pp.Sreal, pitch = round4(pp.C);
+    if (taps == 1 || pp.s_s != 1 || pp.s_r != pp.Sreal) return 1;
+    int rc;
+    if (pp.s_c == taps && pp.s_row == (int64_t)pp.C * taps) rc = transpose_t<float>(w, buf, pp.rows, pp.C, taps, taps, pitch, st);
+    else if (pp.s_row == taps && pp.s_c == (int64_t)pp.rows * taps) rc = transpose_t<float>(w, buf, 1, pp.C, pp.rows * taps, pp.rows * taps, pitch, st);
+    else return 1;
+    if (rc) return rc;
+    pp.s_c = 1; pp.s_s = pitch; pp.s_r = (int64_t)pp.Sreal * pitch; pp.s_row = (int64_t)taps * pitch;
+    w = buf;
+    return B2C_OK;
+}
+
 struct FwdLaunch {
-    int n, ah, aw, C, P, Q, N, kh, kw, low_h, low_w, cnt_h, cnt_w, str_h, str_w, dil_h, dil_w;
+    int n, ah, aw, C, ap, P, Q, N, kh, kw, low_h, low_w, cnt_h, cnt_w, str_h, str_w, dil_h, dil_w;     // ap: pixel pitch of act
     int64_t o_sn, o_sh, o_sw;
 };
 
-static int run_fwd(const FwdLaunch& f, const void* act, const void* w, const PrepParams& pp, const void* bias,
+static int run_fwd(const FwdLaunch& f, const void* act, const void* w, PrepParams pp, const void* bias,
                    const b2c_bn_params* bn, int relu, float* out, void* ws, size_t ws_bytes, cudaStream_t st,
                    bool filters_ready = false, const StatsOut* stats = nullptr, const ZeroFill* zf = nullptr)
 {
     if (!load_driver_entry_points()) return B2C_ERR_UNSUPPORTED;
-    const int64_t K = (int64_t)f.kh * f.kw * f.C;
+    const int cblocks = (f.C + 31) / 32;
+    pp.Cp = cblocks * 32;
+    const int64_t K = (int64_t)f.kh * f.kw * pp.Cp;
     const size_t fbytes = align_up((size_t)f.N * K * sizeof(float), 1024);
     uintptr_t base = align_up((uintptr_t)ws, 1024);
     if (!ws || base + 2 * fbytes > (uintptr_t)ws + ws_bytes) return B2C_ERR_WORKSPACE_TOO_SMALL;
@@ -1804,7 +1865,7 @@ static int run_fwd(const FwdLaunch& f, const void* act, const void* w, const Pre
     unsigned int* sk_bank = tc_sm_count() * 4 <= TC_SYNC_FLAGS ? tc_sync_bank(st) : nullptr;
     if (sk_bank) sk_flags = (int*)sk_bank;
     {
-        const int64_t kblocks = (int64_t)f.kh * f.kw * (f.C / 32);
+        const int64_t kblocks = (int64_t)f.kh * f.kw * cblocks;
         const bool room = base + 2 * fbytes + sk_bytes() <= (uintptr_t)ws + ws_bytes;
         if (!filters_ready && room && fwd_prefers_balanced((int64_t)f.n * f.P * f.Q, f.N, kblocks)) sk = 1;
     }
@@ -1814,7 +1875,11 @@ static int run_fwd(const FwdLaunch& f, const void* act, const void* w, const Pre
     // kernel about 5 us: the copies win beyond roughly 125 us of work (0.6 us per k-block on 148 SMs).
     int bsrc = TCB_SPLIT;
     CUtensorMap ma, mbh, mbl;
-    const bool long_launch = (((int64_t)f.n * f.P * f.Q + 127) / 128) * ((f.N + BN - 1) / BN) * f.kh * f.kw * (f.C / 32) > 30000;
+    const bool long_launch = (((int64_t)f.n * f.P * f.Q + 127) / 128) * ((f.N + BN - 1) / BN) * f.kh * f.kw * cblocks > 30000;
+    if (!filters_ready && !long_launch) {
+        const int rc = kmajor_filter_copy(pp, w, w_hi, st);
+        if (rc < 0) return rc;
+    }
     if (!filters_ready && !long_launch && ((uintptr_t)w & 15) == 0 && pp.s_r == (int64_t)pp.Sreal * pp.s_s && (pp.s_s * 4) % 16 == 0) {
         const uint64_t taps = (uint64_t)pp.Rreal * pp.Sreal;
         if (pp.s_c == 1 && (pp.s_row * 4) % 16 == 0 &&
@@ -1835,11 +1900,11 @@ static int run_fwd(const FwdLaunch& f, const void* act, const void* w, const Pre
         cudaError_t e = cudaMemsetAsync(sk_flags, 0, (size_t)tc_sm_count() * 4 * sizeof(int), st);
         if (e != cudaSuccess) { set_cuda_error(e, "cudaMemsetAsync(balanced-mode flags)"); return B2C_ERR_CUDA; }
     }
-    if (!make_map_im2col(&ma, act, f.n, f.ah, f.aw, f.C, f.low_h, f.low_w, f.cnt_h, f.cnt_w, f.str_h, f.str_w, 128)) return B2C_ERR_UNSUPPORTED;
-    if (bsrc == TCB_SPLIT && (!make_map_2d(&mbh, w_hi, f.N, K, BN) || !make_map_2d(&mbl, w_lo, f.N, K, BN))) return B2C_ERR_UNSUPPORTED;
+    if (!make_map_im2col(&ma, act, f.n, f.ah, f.aw, f.C, f.ap, f.low_h, f.low_w, f.cnt_h, f.cnt_w, f.str_h, f.str_w, 128)) return B2C_ERR_UNSUPPORTED;
+    if (bsrc == TCB_SPLIT && (!make_map_2d(&mbh, w_hi, f.N, K, K, BN) || !make_map_2d(&mbl, w_lo, f.N, K, K, BN))) return B2C_ERR_UNSUPPORTED;
     TcParams p{};
     p.M = f.n * f.P * f.Q; p.N = f.N; p.P = f.P; p.Q = f.Q;
-    p.C = f.C; p.cblocks = f.C / 32; p.kblocks = f.kh * f.kw * p.cblocks; p.S = f.kw;
+    p.C = f.C; p.cblocks = cblocks; p.ktail = (f.C - (cblocks - 1) * 32 + 7) / 8; p.kblocks = f.kh * f.kw * p.cblocks; p.S = f.kw;
     p.str_h = f.str_h; p.str_w = f.str_w; p.dil_h = f.dil_h; p.dil_w = f.dil_w; p.low_h = f.low_h; p.low_w = f.low_w;
     p.bias = (const float*)bias;
     if (bn) { p.mean = (const float*)bn->mean; p.inv_std = (const float*)bn->inv_std; p.gamma = (const float*)bn->gamma; p.beta = (const float*)bn->beta; }
@@ -1850,13 +1915,13 @@ static int run_fwd(const FwdLaunch& f, const void* act, const void* w, const Pre
     p.out = out; p.o_sn = f.o_sn; p.o_sh = f.o_sh; p.o_sw = f.o_sw;
     p.tap_r0 = pp.r0; p.tap_rstep = pp.rstep; p.tap_s0 = pp.s0; p.tap_sstep = pp.sstep; p.tap_sreal = pp.Sreal;
     p.sk = sk; p.sk_flags = sk_flags; p.sk_partial = sk_partial; p.sk_selfclean = sk_bank ? 1 : 0;
-    // dense rows (plain fprop / stride-1 dgrad): rows are N floats apart in (n, i, j) order
-    const bool dense = f.o_sw == f.N && f.o_sh == (int64_t)f.Q * f.N && f.o_sn == (int64_t)f.P * f.Q * f.N;
+    // dense rows (plain fprop / stride-1 dgrad): rows are a constant pitch apart in (n, i, j) order
+    const bool dense = f.o_sw % 4 == 0 && f.o_sh == (int64_t)f.Q * f.o_sw && f.o_sn == (int64_t)f.P * f.Q * f.o_sw;
     CUtensorMap mo = mbh;
     p.tma_store = 0;
-    if (dense && make_map_out(&mo, out, 0, (uint64_t)p.M, (uint64_t)f.N)) p.tma_store = 1;
+    if (dense && make_map_out(&mo, out, 0, (uint64_t)p.M, (uint64_t)f.N, (uint64_t)f.o_sw)) p.tma_store = 1;
     if (zf) {
-        if (p.tma_store || (f.N % 4) || ((zf->off_w | zf->off_h) & 3)) return B2C_ERR_UNSUPPORTED;
+        if (p.tma_store || ((zf->off_w | zf->off_h) & 3)) return B2C_ERR_UNSUPPORTED;
         p.zfill = 1; p.z_W = zf->W; p.z_H = zf->H; p.z_w = zf->off_w; p.z_h = zf->off_h;
     }
     if (stats) {
@@ -1874,7 +1939,8 @@ static int run_fwd(const FwdLaunch& f, const void* act, const void* w, const Pre
 
 static LowerParams lower_params(const Geo& g)
 {
-    return LowerParams{g.n, g.h, g.w, g.ci, g.ho, g.wo, g.kh, g.kw, g.vpad, g.hpad, g.vstr, g.hstr, g.vdil, g.hdil, (int)g.K, lowered_kp(g)};
+    const ActStride xs = act_stride(g.x_nchw ? B2C_LAYOUT_NCHW : B2C_LAYOUT_NHWC, g.h, g.w, g.ci);
+    return LowerParams{g.n, g.h, g.w, g.ci, g.ho, g.wo, g.kh, g.kw, g.vpad, g.hpad, g.vstr, g.hstr, g.vdil, g.hdil, (int)g.K, lowered_kp(g), xs.sn, xs.sh, xs.sw, xs.sc};
 }
 static int launch_lower(const Geo& g, const void* x, float* rows, cudaStream_t st)
 {
@@ -1906,7 +1972,8 @@ static int tc_fprop_nhwc(const Geo& g, const void* x, const void* w, const void*
              void* y, void* ws, size_t ws_bytes, cudaStream_t st, const StatsOut* stats = nullptr)
 {
     WStride wsd = w_stride(g.w_layout, g.ci, g.co, g.kh, g.kw);
-    if (g.ci % 32 != 0) {
+    const int64_t yp = g.yp;
+    if (lowered_ok(g)) {
         // few-channel layer: write out the im2row matrix, then a 1x1 convolution over it
         const int Kp = lowered_kp(g);
         const size_t lbytes = align_up((size_t)g.M * Kp * sizeof(float), 1024);
@@ -1924,14 +1991,13 @@ static int tc_fprop_nhwc(const Geo& g, const void* x, const void* w, const void*
         rc = check_launch("tc_prep_filter_lowered_kernel");
         if (rc) return rc;
         PrepParams none{};
-        FwdLaunch f{g.n, g.ho, g.wo, Kp, g.ho, g.wo, g.co, 1, 1, 0, 0, g.ho, g.wo, 1, 1, 1, 1,
-                    (int64_t)g.ho * g.wo * g.co, (int64_t)g.wo * g.co, (int64_t)g.co};
+        FwdLaunch f{g.n, g.ho, g.wo, Kp, Kp, g.ho, g.wo, g.co, 1, 1, 0, 0, g.ho, g.wo, 1, 1, 1, 1, g.ho * g.wo * yp, g.wo * yp, yp};
         return run_fwd(f, rows, nullptr, none, bias, bn, relu, (float*)y, (void*)w_hi, 2 * fbytes + 1024, st, true, stats);
     }
     PrepParams pp{g.co, g.ci, g.kh, g.kw, wsd.sk, wsd.sc, wsd.sr, wsd.ss, 0, 1, 0, 1, g.kh, g.kw};
-    FwdLaunch f{g.n, g.h, g.w, g.ci, g.ho, g.wo, g.co, g.kh, g.kw, -g.vpad, -g.hpad,
+    FwdLaunch f{g.n, g.h, g.w, g.ci, g.xp, g.ho, g.wo, g.co, g.kh, g.kw, -g.vpad, -g.hpad,
                 g.h + 2 * g.vpad - (g.kh - 1) * g.vdil, g.w + 2 * g.hpad - (g.kw - 1) * g.hdil,
-                g.vstr, g.hstr, g.vdil, g.hdil, (int64_t)g.ho * g.wo * g.co, (int64_t)g.wo * g.co, (int64_t)g.co};
+                g.vstr, g.hstr, g.vdil, g.hdil, g.ho * g.wo * yp, g.wo * yp, yp};
     return run_fwd(f, x, w, pp, bias, bn, relu, (float*)y, ws, ws_bytes, st, false, stats);
 }
 
@@ -1976,20 +2042,20 @@ static int tc_dgrad_classes_one_launch(const Geo& g, const WStride& wsd, const v
     TcParams p{};
     CUtensorMap ma[4];
     const int nt = (g.ci + BN - 1) / BN;
-    p.N = g.ci; p.C = g.co; p.cblocks = g.co / 32;
+    p.N = g.ci; p.C = g.co; p.cblocks = (g.co + 31) / 32; p.ktail = (g.co - (p.cblocks - 1) * 32 + 7) / 8;
     p.str_h = 1; p.str_w = 1; p.dil_h = 1; p.dil_w = 1;
-    p.out = (float*)dx; p.o_sn = (int64_t)g.h * g.w * g.ci; p.o_sh = (int64_t)g.vstr * g.w * g.ci; p.o_sw = (int64_t)g.hstr * g.ci;
+    p.out = (float*)dx; p.o_sn = (int64_t)g.h * g.w * g.xp; p.o_sh = (int64_t)g.vstr * g.w * g.xp; p.o_sw = (int64_t)g.hstr * g.xp;
     p.tap_rstep = -g.vstr; p.tap_sstep = -g.hstr; p.tap_sreal = g.kw;
     p.splits = 1; p.ncls = ncls;
     int64_t tiles = 0;
     for (int i = 0; i < ncls; i++) {
         const AxisClass &ca = cls[i].a, &cb = cls[i].b;
-        if (!make_map_im2col(&ma[i], dy, g.n, g.ho, g.wo, g.co, ca.dmin, cb.dmin, ca.out_cnt, cb.out_cnt, 1, 1, 128)) return 1;
+        if (!make_map_im2col(&ma[i], dy, g.n, g.ho, g.wo, g.co, g.yp, ca.dmin, cb.dmin, ca.out_cnt, cb.out_cnt, 1, 1, 128)) return 1;
         p.cls_tile0[i] = (int)tiles;
         p.cls_M[i] = g.n * ca.out_cnt * cb.out_cnt; p.cls_P[i] = ca.out_cnt; p.cls_Q[i] = cb.out_cnt;
         p.cls_kblocks[i] = ca.cnt * cb.cnt * p.cblocks; p.cls_S[i] = cb.cnt;
         p.cls_low_h[i] = ca.dmin; p.cls_low_w[i] = cb.dmin; p.cls_r0[i] = ca.r0; p.cls_s0[i] = cb.r0;
-        p.cls_out[i] = ((int64_t)cls[i].ia * g.w + cls[i].ib) * g.ci;
+        p.cls_out[i] = ((int64_t)cls[i].ia * g.w + cls[i].ib) * g.xp;
         tiles += (int64_t)((p.cls_M[i] + 127) / 128) * nt;
         if (tiles > 0x7fffffffLL) return 1;
     }
@@ -2012,9 +2078,22 @@ static int tc_dgrad_nhwc(const Geo& g, const void* dy, const void* w, void* dx, 
         // dx = convolution of dy with the flipped, transposed filter and padding (k-1)*dil - pad
         const int pv = (g.kh - 1) * g.vdil - g.vpad, ph = (g.kw - 1) * g.hdil - g.hpad;
         PrepParams pp{g.ci, g.co, g.kh, g.kw, wsd.sc, wsd.sk, wsd.sr, wsd.ss, g.kh - 1, -1, g.kw - 1, -1, g.kh, g.kw};
-        FwdLaunch f{g.n, g.ho, g.wo, g.co, g.h, g.w, g.ci, g.kh, g.kw, -pv, -ph, g.h, g.w, 1, 1, g.vdil, g.hdil,
-                    (int64_t)g.h * g.w * g.ci, (int64_t)g.w * g.ci, (int64_t)g.ci};
+        FwdLaunch f{g.n, g.ho, g.wo, g.co, g.yp, g.h, g.w, g.ci, g.kh, g.kw, -pv, -ph, g.h, g.w, 1, 1, g.vdil, g.hdil,
+                    (int64_t)g.h * g.w * g.xp, (int64_t)g.w * g.xp, (int64_t)g.xp};
         return run_fwd(f, dy, w, pp, nullptr, nullptr, 0, (float*)dx, ws, ws_bytes, st);
+    }
+    // the classes share one K-major copy of a filter that needs one
+    PrepParams whole{g.ci, g.co, g.kh, g.kw, wsd.sc, wsd.sk, wsd.sr, wsd.ss, 0, 1, 0, 1, g.kh, g.kw};
+    {
+        const uintptr_t base = align_up((uintptr_t)ws, 1024);
+        const size_t fbytes = filter_split_bytes(g, B2C_PASS_DGRAD);
+        if (!ws || base + fbytes > (uintptr_t)ws + ws_bytes) return B2C_ERR_WORKSPACE_TOO_SMALL;
+        const int rc = kmajor_filter_copy(whole, w, (float*)base, st);
+        if (rc < 0) return rc;
+        if (rc == B2C_OK) {
+            wsd.sc = whole.s_row; wsd.sk = whole.s_c; wsd.sr = whole.s_r; wsd.ss = whole.s_s;
+            ws_bytes -= base + fbytes - (uintptr_t)ws; ws = (void*)(base + fbytes);
+        }
     }
     // Strided: the input positions split into str_h*str_w parity classes; each class is a dense
     // stride-1 convolution of dy with the sub-filter of the taps that reach it, written to its
@@ -2035,18 +2114,18 @@ static int tc_dgrad_nhwc(const Geo& g, const void* dy, const void* w, void* dx, 
         // 2 x 2 stride, only class (0, 0) reached by a tap (a 1x1 filter without padding): the class's launch writes the
         // other classes' zeros next to its own rows, no clearing pass over dx
         AxisClass ca = axis_class(0, g.vstr, g.vpad, g.kh, g.h), cb = axis_class(0, g.hstr, g.hpad, g.kw, g.w);
-        if (g.vstr == 2 && g.hstr == 2 && live == 1 && ca.cnt > 0 && cb.cnt > 0 && g.ci % 4 == 0 && ((uintptr_t)dx & 15) == 0) {
+        if (g.vstr == 2 && g.hstr == 2 && live == 1 && ca.cnt > 0 && cb.cnt > 0 && g.xp % 4 == 0 && ((uintptr_t)dx & 15) == 0) {
             PrepParams pp{g.ci, g.co, ca.cnt, cb.cnt, wsd.sc, wsd.sk, wsd.sr, wsd.ss, ca.r0, -g.vstr, cb.r0, -g.hstr, g.kh, g.kw};
-            FwdLaunch f{g.n, g.ho, g.wo, g.co, ca.out_cnt, cb.out_cnt, g.ci, ca.cnt, cb.cnt, ca.dmin, cb.dmin,
+            FwdLaunch f{g.n, g.ho, g.wo, g.co, g.yp, ca.out_cnt, cb.out_cnt, g.ci, ca.cnt, cb.cnt, ca.dmin, cb.dmin,
                         ca.out_cnt, cb.out_cnt, 1, 1, 1, 1,
-                        (int64_t)g.h * g.w * g.ci, (int64_t)g.vstr * g.w * g.ci, (int64_t)g.hstr * g.ci};
-            ZeroFill zf{g.w, g.h, (int64_t)g.ci, (int64_t)g.w * g.ci};
+                        (int64_t)g.h * g.w * g.xp, (int64_t)g.vstr * g.w * g.xp, (int64_t)g.hstr * g.xp};
+            ZeroFill zf{g.w, g.h, (int64_t)g.xp, (int64_t)g.w * g.xp};
             int rc = run_fwd(f, dy, w, pp, nullptr, nullptr, 0, (float*)dx, ws, ws_bytes, st, false, nullptr, &zf);
             if (rc != B2C_ERR_UNSUPPORTED) return rc;
         }
     }
     if (any_empty) {
-        cudaError_t e = cudaMemsetAsync(dx, 0, (size_t)g.n * g.h * g.w * g.ci * sizeof(float), st);
+        cudaError_t e = cudaMemsetAsync(dx, 0, (size_t)g.n * g.h * g.w * g.xp * sizeof(float), st);
         if (e != cudaSuccess) { set_cuda_error(e, "cudaMemsetAsync(dx)"); return B2C_ERR_CUDA; }
     }
     for (int a = 0; a < g.vstr; a++)
@@ -2054,10 +2133,10 @@ static int tc_dgrad_nhwc(const Geo& g, const void* dy, const void* w, void* dx, 
             AxisClass ca = axis_class(a, g.vstr, g.vpad, g.kh, g.h), cb = axis_class(b, g.hstr, g.hpad, g.kw, g.w);
             if (ca.out_cnt == 0 || cb.out_cnt == 0 || ca.cnt == 0 || cb.cnt == 0) continue;
             PrepParams pp{g.ci, g.co, ca.cnt, cb.cnt, wsd.sc, wsd.sk, wsd.sr, wsd.ss, ca.r0, -g.vstr, cb.r0, -g.hstr, g.kh, g.kw};
-            FwdLaunch f{g.n, g.ho, g.wo, g.co, ca.out_cnt, cb.out_cnt, g.ci, ca.cnt, cb.cnt, ca.dmin, cb.dmin,
+            FwdLaunch f{g.n, g.ho, g.wo, g.co, g.yp, ca.out_cnt, cb.out_cnt, g.ci, ca.cnt, cb.cnt, ca.dmin, cb.dmin,
                         ca.out_cnt, cb.out_cnt, 1, 1, 1, 1,
-                        (int64_t)g.h * g.w * g.ci, (int64_t)g.vstr * g.w * g.ci, (int64_t)g.hstr * g.ci};
-            float* out = (float*)dx + ((int64_t)a * g.w + b) * g.ci;
+                        (int64_t)g.h * g.w * g.xp, (int64_t)g.vstr * g.w * g.xp, (int64_t)g.hstr * g.xp};
+            float* out = (float*)dx + ((int64_t)a * g.w + b) * g.xp;
             int rc = run_fwd(f, dy, w, pp, nullptr, nullptr, 0, out, ws, ws_bytes, st);
             if (rc) return rc;
         }
@@ -2070,15 +2149,15 @@ static int tc_wgrad_nhwc(const Geo& g, const void* x, const void* dy, void* dw, 
     if (!load_driver_entry_points()) return B2C_ERR_UNSUPPORTED;
     if (!exchanged && !db && !lowered_in_ws && wgrad_swap_ok(g))
         return tc_wgrad_nhwc(wgrad_swapped(g), dy, x, dw, nullptr, ws, ws_bytes, st, false, true);
-    const bool low = g.ci % 32 != 0;
-    const int Krows = low ? lowered_kp(g) : (int)g.K;
+    const bool low = lowered_ok(g);
+    const int Krows = (int)wgrad_rows(g), Np = round4(g.co), Cp = round32(g.ci);
     WgradPlan pl = wgrad_plan(g);
     const size_t lbytes = low ? align_up((size_t)g.M * Krows * sizeof(float), 1024) : 0;
-    const size_t pbytes = align_up((size_t)pl.splits * Krows * g.co * sizeof(float), 1024);
+    const size_t pbytes = align_up((size_t)pl.splits * Krows * Np * sizeof(float), 1024);
     uintptr_t base = align_up((uintptr_t)ws, 1024);
-    const size_t cs = align_up((size_t)pl.splits * 4 * g.co * sizeof(float), 1024);
+    const size_t cs = align_up((size_t)pl.splits * 4 * Np * sizeof(float), 1024);
     if (!ws || base + lbytes + pbytes + (db ? cs : 0) > (uintptr_t)ws + ws_bytes) return B2C_ERR_WORKSPACE_TOO_SMALL;
-    if (((uintptr_t)x & 15) || ((uintptr_t)dy & 15)) return B2C_ERR_MISALIGNED;
+    if ((!low && ((uintptr_t)x & 15)) || ((uintptr_t)dy & 15)) return B2C_ERR_MISALIGNED;
     float* partial = (float*)(base + lbytes);
     CUtensorMap ma, mb;
     TcParams p{};
@@ -2090,7 +2169,7 @@ static int tc_wgrad_nhwc(const Geo& g, const void* x, const void* dy, void* dw, 
             if (rc) return rc;
         }
         int lg = Krows % 128 == 0 ? 7 : Krows % 64 == 0 ? 6 : 5;       // widest box first, narrower if the encoder refuses
-        while (lg >= 5 && !make_map_im2col(&ma, rows, g.n, g.ho, g.wo, Krows, 0, 0, g.ho, g.wo, 1, 1, 32, CU_TENSOR_MAP_SWIZZLE_NONE, 1u << lg)) lg--;
+        while (lg >= 5 && !make_map_im2col(&ma, rows, g.n, g.ho, g.wo, Krows, Krows, 0, 0, g.ho, g.wo, 1, 1, 32, CU_TENSOR_MAP_SWIZZLE_NONE, 1u << lg)) lg--;
         if (lg < 5) return B2C_ERR_UNSUPPORTED;
         p.a_box_log2 = lg;
         p.C = Krows; p.cblocks = Krows / 32; p.S = 1;
@@ -2098,21 +2177,21 @@ static int tc_wgrad_nhwc(const Geo& g, const void* x, const void* dy, void* dw, 
     } else {
         // x boxes as wide as the channel count allows (fewer TMA instructions per k-block: the producer's issue
         // time was 36-63 % of the kernel's on the weight gradients of the step)
-        int lg = g.ci % 128 == 0 ? 7 : g.ci % 64 == 0 ? 6 : 5;
-        while (lg >= 5 && !make_map_im2col(&ma, x, g.n, g.h, g.w, g.ci, -g.vpad, -g.hpad, g.h + 2 * g.vpad - (g.kh - 1) * g.vdil,
+        int lg = Cp % 128 == 0 ? 7 : Cp % 64 == 0 ? 6 : 5;
+        while (lg >= 5 && !make_map_im2col(&ma, x, g.n, g.h, g.w, g.ci, g.xp, -g.vpad, -g.hpad, g.h + 2 * g.vpad - (g.kh - 1) * g.vdil,
                                            g.w + 2 * g.hpad - (g.kw - 1) * g.hdil, g.vstr, g.hstr, 32, CU_TENSOR_MAP_SWIZZLE_NONE, 1u << lg)) lg--;
         if (lg < 5) return B2C_ERR_UNSUPPORTED;
         p.a_box_log2 = lg;
-        p.C = g.ci; p.cblocks = g.ci / 32; p.S = g.kw;
+        p.C = Cp; p.cblocks = Cp / 32; p.S = g.kw;
         p.str_h = g.vstr; p.str_w = g.hstr; p.dil_h = g.vdil; p.dil_w = g.hdil; p.low_h = -g.vpad; p.low_w = -g.hpad;
     }
-    if (!make_map_2d(&mb, dy, (uint64_t)g.M, (uint64_t)g.co, 32, CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B)) return B2C_ERR_UNSUPPORTED;
-    p.M = Krows; p.N = g.co; p.P = g.ho; p.Q = g.wo; p.kblocks = pl.kblocks;
+    if (!make_map_2d(&mb, dy, (uint64_t)g.M, (uint64_t)g.co, (uint64_t)g.yp, 32, CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B)) return B2C_ERR_UNSUPPORTED;
+    p.M = Krows; p.N = g.co; p.Np = Np; p.ktail = 4; p.P = g.ho; p.Q = g.wo; p.kblocks = pl.kblocks;
     p.Mpix = (int)g.M;
     p.out = partial;
     p.db_partial = db ? (float*)(base + lbytes + pbytes) : nullptr;
     CUtensorMap mo = mb;
-    p.tma_store = make_map_out(&mo, partial, (uint64_t)pl.splits, (uint64_t)Krows, (uint64_t)g.co) ? 1 : 0;
+    p.tma_store = make_map_out(&mo, partial, (uint64_t)pl.splits, (uint64_t)Krows, (uint64_t)g.co, (uint64_t)Np) ? 1 : 0;
     WStride wsd = w_stride(g.w_layout, g.ci, g.co, g.kh, g.kw);
     if (exchanged) {
         // g is the layer with ci and co exchanged: the caller's filter has g.co input and g.ci output channels
@@ -2121,7 +2200,7 @@ static int tc_wgrad_nhwc(const Geo& g, const void* x, const void* dy, void* dw, 
     }
     int rc = dispatch_wgrad(pl.bn, ma, mb, mo, p, pl.splits, st);
     if (rc) return rc;
-    WgradReduceParams rp{Krows, g.co, g.ci, g.kw, pl.splits, wsd.sk, wsd.sc, wsd.sr, wsd.ss, (int)g.K};
+    WgradReduceParams rp{Krows, g.co, low ? g.ci : Cp, g.kw, pl.splits, wsd.sk, wsd.sc, wsd.sr, wsd.ss, low ? (int)g.K : Krows, g.ci, Np};
     if ((int64_t)((g.co + 31) / 32) * ((Krows + 31) / 32) >= 2 * (int64_t)tc_sm_count())
         launch_pdl(tc_wgrad_reduce_kernel<4>, dim3((g.co + 31) / 32, (Krows + 31) / 32), dim3(32, 8), 0, st, rp, partial, (float*)dw, p.db_partial, (float*)db);
     else if ((int64_t)((g.co + 31) / 32) * ((Krows + 7) / 8) >= 2 * (int64_t)tc_sm_count() || pl.splits < 16)
@@ -2137,28 +2216,27 @@ static int tc_wgrad_nhwc(const Geo& g, const void* x, const void* dy, void* dw, 
 // (pydtnn/backends/cpu/layers/conv_2d_cpu.py:264-291, 447-481); filters stay where they are (every filter layout
 // is read through strides).  Taken when the transposes cost less than the FMA engine would lose.
 // ---------------------------------------------------------------------------------------------
-// src [n][rows][cols] -> dst [n][cols][rows]; block (32, 8), grid (cols/32, rows/32, n)
+// src [n][rows][cols] -> dst [n][cols][rows], rows sp (dst: dp) elements apart; block (32, 8), grid (cols/32, rows/32, n)
 template <typename T>
-__global__ void transpose_inner_kernel(const T* __restrict__ src, T* __restrict__ dst, int rows, int cols)
+__global__ void transpose_inner_kernel(const T* __restrict__ src, T* __restrict__ dst, int rows, int cols, int sp, int dp)
 {
     pdl_prologue();
     __shared__ T tile[32][33];
-    const int64_t plane = (int64_t)rows * cols;
     const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32, tx = threadIdx.x, ty = threadIdx.y;
     {
         const int img = blockIdx.z;
-        const T* s = src + img * plane;
-        T* d = dst + img * plane;
+        const T* s = src + (int64_t)img * rows * sp;
+        T* d = dst + (int64_t)img * cols * dp;
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             const int r = r0 + ty + 8 * j, c = c0 + tx;
-            if (r < rows && c < cols) tile[ty + 8 * j][tx] = s[(int64_t)r * cols + c];
+            if (r < rows && c < cols) tile[ty + 8 * j][tx] = s[(int64_t)r * sp + c];
         }
         __syncthreads();
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             const int c = c0 + ty + 8 * j, r = r0 + tx;
-            if (r < rows && c < cols) d[(int64_t)c * rows + r] = tile[tx][ty + 8 * j];
+            if (r < rows && c < cols) d[(int64_t)c * dp + r] = tile[tx][ty + 8 * j];
         }
     }
 }
@@ -2168,89 +2246,172 @@ __global__ void transpose_inner_kernel(const T* __restrict__ src, T* __restrict_
 // -> dst [n][len][thin], else src [n][len][thin] -> dst [n][thin][len].  Loads or stores of a warp cover whole
 // contiguous runs either way.
 template <typename T, bool ROWS_THIN>
-__global__ void __launch_bounds__(256) transpose_thin_kernel(const T* __restrict__ src, T* __restrict__ dst, int thin, int len)
+__global__ void __launch_bounds__(256) transpose_thin_kernel(const T* __restrict__ src, T* __restrict__ dst, int thin, int len, int tp)
 {
     pdl_prologue();
     const int l = blockIdx.x * blockDim.x + threadIdx.x;
     if (l >= len) return;
-    const int64_t plane = (int64_t)thin * len;
-    const T* s = src + blockIdx.y * plane;
-    T* d = dst + blockIdx.y * plane;
+    const T* s = src + (int64_t)blockIdx.y * len * (ROWS_THIN ? thin : tp);      // tp: pitch of the thin rows
+    T* d = dst + (int64_t)blockIdx.y * len * (ROWS_THIN ? tp : thin);
     T v[8];
 #pragma unroll
     for (int r = 0; r < 8; r++)
-        if (r < thin) v[r] = ROWS_THIN ? s[(int64_t)r * len + l] : s[(int64_t)l * thin + r];
+        if (r < thin) v[r] = ROWS_THIN ? s[(int64_t)r * len + l] : s[(int64_t)l * tp + r];
 #pragma unroll
     for (int r = 0; r < 8; r++)
-        if (r < thin) { if (ROWS_THIN) d[(int64_t)l * thin + r] = v[r]; else d[(int64_t)r * len + l] = v[r]; }
+        if (r < thin) { if (ROWS_THIN) d[(int64_t)l * tp + r] = v[r]; else d[(int64_t)r * len + l] = v[r]; }
 }
 
 template <typename T>
-static int transpose_t(const void* src, void* dst, int n, int rows, int cols, cudaStream_t st)
+static int transpose_t(const void* src, void* dst, int n, int rows, int cols, int sp, int dp, cudaStream_t st)
 {
     if ((rows + 31) / 32 > 65535) return B2C_ERR_TOO_LARGE;
     if (n > 65535) {                                  // the image index is a grid axis: in parts
-        const size_t part = (size_t)65535 * rows * cols * sizeof(T);
-        const int rc = transpose_t<T>(src, dst, 65535, rows, cols, st);
-        return rc ? rc : transpose_t<T>((const char*)src + part, (char*)dst + part, n - 65535, rows, cols, st);
+        const int rc = transpose_t<T>(src, dst, 65535, rows, cols, sp, dp, st);
+        return rc ? rc : transpose_t<T>((const T*)src + (size_t)65535 * rows * sp, (T*)dst + (size_t)65535 * cols * dp, n - 65535, rows, cols, sp, dp, st);
     }
-    if (rows <= 8 && cols > 8) {
-        launch_pdl(transpose_thin_kernel<T, true>, dim3((cols + 255) / 256, n), 256, 0, st, (const T*)src, (T*)dst, rows, cols);
+    if (rows <= 8 && cols > 8 && sp == cols) {
+        launch_pdl(transpose_thin_kernel<T, true>, dim3((cols + 255) / 256, n), 256, 0, st, (const T*)src, (T*)dst, rows, cols, dp);
         return check_launch("transpose_thin_kernel");
     }
-    if (cols <= 8 && rows > 8) {
-        launch_pdl(transpose_thin_kernel<T, false>, dim3((rows + 255) / 256, n), 256, 0, st, (const T*)src, (T*)dst, cols, rows);
+    if (cols <= 8 && rows > 8 && dp == rows) {
+        launch_pdl(transpose_thin_kernel<T, false>, dim3((rows + 255) / 256, n), 256, 0, st, (const T*)src, (T*)dst, cols, rows, sp);
         return check_launch("transpose_thin_kernel");
     }
     launch_pdl(transpose_inner_kernel<T>, dim3((cols + 31) / 32, (rows + 31) / 32, n), dim3(32, 8), 0, st,
-               (const T*)src, (T*)dst, rows, cols);
+               (const T*)src, (T*)dst, rows, cols, sp, dp);
     return check_launch("transpose_inner_kernel");
 }
 
 int transpose_images(int dtype, const void* src, void* dst, int n, int rows, int cols, cudaStream_t st)
 {
-    return dtype == B2C_F32 ? transpose_t<float>(src, dst, n, rows, cols, st) : transpose_t<double>(src, dst, n, rows, cols, st);
+    return dtype == B2C_F32 ? transpose_t<float>(src, dst, n, rows, cols, cols, rows, st) : transpose_t<double>(src, dst, n, rows, cols, cols, rows, st);
 }
 static int transpose_inner(const void* src, void* dst, int n, int rows, int cols, cudaStream_t st)
 {
-    return transpose_t<float>(src, dst, n, rows, cols, st);
+    return transpose_t<float>(src, dst, n, rows, cols, cols, rows, st);
+}
+
+// Rows of c floats between a dense matrix and one with rows `pitch` (a multiple of 4) floats apart, one float4 of the
+// pitched side per thread.  Bound by the copy's bytes; the dense side's rows start on any 4 bytes.
+template <bool TO_PITCH>
+__global__ void __launch_bounds__(256) pitch_copy_kernel(const float* __restrict__ src, float* __restrict__ dst, int64_t rows, int c, int pitch)
+{
+    pdl_prologue();
+    const int q = pitch / 4;
+    const int64_t total = rows * q;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t r = i / q;
+        const int c0 = (int)(i - r * q) * 4;
+        if (TO_PITCH) {
+            const float* s = src + r * c + c0;
+            float4 v;
+            v.x = __ldg(s); v.y = c0 + 1 < c ? __ldg(s + 1) : 0.f; v.z = c0 + 2 < c ? __ldg(s + 2) : 0.f; v.w = c0 + 3 < c ? __ldg(s + 3) : 0.f;
+            *reinterpret_cast<float4*>(dst + r * pitch + c0) = v;
+        } else {
+            const float4 v = __ldg(reinterpret_cast<const float4*>(src + r * pitch + c0));
+            float* d = dst + r * c + c0;
+            d[0] = v.x; if (c0 + 1 < c) d[1] = v.y; if (c0 + 2 < c) d[2] = v.z; if (c0 + 3 < c) d[3] = v.w;
+        }
+    }
 }
 
 static Geo as_nhwc(const Geo& g) { Geo q = g; q.layout = B2C_LAYOUT_NHWC; return q; }
 static size_t act_bytes(int64_t n, int64_t h, int64_t w, int64_t c) { return align_up((size_t)(n * h * w * c) * sizeof(float), 1024); }
 
+// Which activations a pass runs on copies of: NCHW ones, and those whose pixels are no multiple of 16 bytes (a few-channel
+// layer that lowers x reads it as it is, in either layout).  The copies lie at the start of the workspace, channel-last, pixels
+// round4(channels) floats apart; a forward pass and the weight gradient of a layer agree on the place.
+struct Copies { bool x, y; size_t xb, yb; };
+static Copies tc_copies(const Geo& g, int pass)
+{
+    Copies c;
+    const bool nchw = g.layout == B2C_LAYOUT_NCHW;
+    c.x = (nchw || g.ci % 4) && (pass == B2C_PASS_DGRAD || !lowered_ok(g));
+    c.y = nchw || g.co % 4;
+    c.xb = c.x ? act_bytes(g.n, g.h, g.w, round4(g.ci)) : 0;
+    c.yb = c.y ? act_bytes(g.n, g.ho, g.wo, round4(g.co)) : 0;
+    return c;
+}
+static Geo copied_geo(const Geo& g, const Copies& c)
+{
+    Geo q = as_nhwc(g);
+    if (c.x) q.xp = round4(g.ci);
+    else q.x_nchw = g.layout == B2C_LAYOUT_NCHW;
+    if (c.y) q.yp = round4(g.co);
+    return q;
+}
+static int copy_in(const Geo& g, const void* src, void* dst, int hw, int c, cudaStream_t st)
+{
+    if (g.layout == B2C_LAYOUT_NCHW) return transpose_t<float>(src, dst, g.n, c, hw, hw, round4(c), st);
+    const int64_t quads = (int64_t)g.n * hw * (round4(c) / 4);
+    launch_pdl(pitch_copy_kernel<true>, (unsigned)((quads + 255) / 256 < tc_sm_count() * 16 ? (quads + 255) / 256 : tc_sm_count() * 16), 256, 0, st,
+               (const float*)src, (float*)dst, (int64_t)g.n * hw, c, round4(c));
+    return check_launch("pitch_copy_kernel");
+}
+static int copy_out(const Geo& g, const void* src, void* dst, int hw, int c, cudaStream_t st)
+{
+    if (g.layout == B2C_LAYOUT_NCHW) return transpose_t<float>(src, dst, g.n, hw, c, round4(c), hw, st);
+    const int64_t quads = (int64_t)g.n * hw * (round4(c) / 4);
+    launch_pdl(pitch_copy_kernel<false>, (unsigned)((quads + 255) / 256 < tc_sm_count() * 16 ? (quads + 255) / 256 : tc_sm_count() * 16), 256, 0, st,
+               (const float*)src, (float*)dst, (int64_t)g.n * hw, c, round4(c));
+    return check_launch("pitch_copy_kernel");
+}
+
 bool tc_supported(const Geo& g, int pass)
 {
     if (g.layout == B2C_LAYOUT_NHWC) return tc_supported_nhwc(g, pass);
-    if (g.dtype != B2C_F32 || g.engine == B2C_ENGINE_FMA || g.n > 65535) return false;
-    const Geo q = as_nhwc(g);
-    if (!tc_supported_nhwc(q, pass)) return false;
+    if (g.dtype != B2C_F32 || g.engine == B2C_ENGINE_FMA) return false;
+    if (!tc_supported_nhwc(as_nhwc(g), pass)) return false;
     if (g.engine == B2C_ENGINE_TENSOR) return true;
     // two tensors are copied there and/or back (read + write each) at about 2.5 TB/s; the FMA engine runs the
-    // pass at about 26 TFLOP/s, this engine at about 130
+    // pass at about 20 TFLOP/s, this engine at about 130
     const double flops = 2.0 * (double)g.M * (double)g.K * g.co;
     const double xb = 4.0 * g.n * g.h * g.w * g.ci, yb = 4.0 * (double)g.M * g.co;
     const double moved = 2.0 * (xb + yb);
-    return flops / 130e12 + moved / 2.5e12 < flops / 26e12;
+    return flops / 130e12 + moved / 2.5e12 < flops / 20e12;
+}
+
+// Shapes whose channel counts keep every activation on 16-byte pixels and whole blocks, whatever the pointers: for the
+// others a pointer that is not 16-byte aligned sends the call to the FMA engine (b2c_conv_* with engine AUTO).
+bool tc_any_alignment(const Geo& g, int pass)
+{
+    const Copies c = tc_copies(g, pass);
+    if (pass == B2C_PASS_FPROP) return g.ci % 32 == 0 && g.co % 4 == 0;
+    if (pass == B2C_PASS_DGRAD) return g.co % 32 == 0 && g.ci % 4 == 0;
+    return (c.x || g.ci % 32 == 0 || lowered_ok(g)) && g.co % 32 == 0;
 }
 
 size_t tc_workspace_bytes(const Geo& g, int pass)
 {
-    if (g.layout == B2C_LAYOUT_NHWC) return tc_workspace_bytes_nhwc(g, pass);
-    return act_bytes(g.n, g.h, g.w, g.ci) + act_bytes(g.n, g.ho, g.wo, g.co) + 1024 + tc_workspace_bytes_nhwc(as_nhwc(g), pass);
+    const Copies c = tc_copies(g, pass);
+    if (!c.x && !c.y) return tc_workspace_bytes_nhwc(g, pass);
+    return c.xb + c.yb + 1024 + tc_workspace_bytes_nhwc(copied_geo(g, c), pass);
 }
 
-// workspace of an NCHW call: [x or dx, channel-last][y or dy, channel-last][workspace of the channel-last pass]
-struct NchwWs { float *a, *b; void* inner; size_t inner_bytes; };
-static bool nchw_ws(const Geo& g, void* ws, size_t ws_bytes, NchwWs& o)
+// workspace of a call with copies: [x or dx, channel-last][y or dy, channel-last][workspace of the channel-last pass]
+struct CopyWs { void *x, *y, *inner; size_t inner_bytes; };
+static bool copy_ws(const Copies& c, void* ws, size_t ws_bytes, CopyWs& o)
 {
+    if (!c.x && !c.y) { o.x = o.y = nullptr; o.inner = ws; o.inner_bytes = ws_bytes; return true; }
     if (!ws) return false;
     const uintptr_t base = align_up((uintptr_t)ws, 1024);
-    const size_t xa = act_bytes(g.n, g.h, g.w, g.ci), ya = act_bytes(g.n, g.ho, g.wo, g.co);
-    if (base + xa + ya > (uintptr_t)ws + ws_bytes) return false;
-    o.a = (float*)base; o.b = (float*)(base + xa); o.inner = (void*)(base + xa + ya);
-    o.inner_bytes = (uintptr_t)ws + ws_bytes - (base + xa + ya);
+    if (base + c.xb + c.yb > (uintptr_t)ws + ws_bytes) return false;
+    o.x = (void*)base; o.y = (void*)(base + c.xb); o.inner = (void*)(base + c.xb + c.yb);
+    o.inner_bytes = (uintptr_t)ws + ws_bytes - (base + c.xb + c.yb);
     return true;
+}
+
+static int tc_fprop_any(const Geo& g, const void* x, const void* w, const void* bias, const b2c_bn_params* bn, int relu,
+                        void* y, void* ws, size_t ws_bytes, cudaStream_t st, const StatsOut* stats)
+{
+    const Copies c = tc_copies(g, B2C_PASS_FPROP);
+    CopyWs t;
+    if (!copy_ws(c, ws, ws_bytes, t)) return B2C_ERR_WORKSPACE_TOO_SMALL;
+    if (c.x) { const int rc = copy_in(g, x, t.x, g.h * g.w, g.ci, st); if (rc) return rc; }
+    const int rc = tc_fprop_nhwc(copied_geo(g, c), c.x ? t.x : x, w, bias, bn, relu, c.y ? t.y : y, t.inner, t.inner_bytes, st, stats);
+    if (rc || !c.y) return rc;
+    return copy_out(g, t.y, y, g.ho * g.wo, g.co, st);
 }
 
 // Forward pass that also leaves the per-channel sums of its output for a training-mode batch norm (NHWC float32 on this
@@ -2258,8 +2419,8 @@ static bool nchw_ws(const Geo& g, void* ws, size_t ws_bytes, NchwWs& o)
 size_t tc_stats_bytes(const Geo& g)
 {
     if (g.layout != B2C_LAYOUT_NHWC || !tc_supported_nhwc(g, B2C_PASS_FPROP) || g.co % 4) return 0;
-    const bool lowered = g.ci % 32 != 0;        // few-channel layers run as a 1x1 convolution over the lowered matrix
-    const int64_t kblocks = lowered ? lowered_kp(g) / 32 : (int64_t)g.kh * g.kw * (g.ci / 32);
+    const bool lowered = lowered_ok(g);         // few-channel layers run as a 1x1 convolution over the lowered matrix
+    const int64_t kblocks = lowered ? lowered_kp(g) / 32 : (int64_t)g.kh * g.kw * (round32(g.ci) / 32);
     return (size_t)fwd_stats_rows(g.M, g.co, kblocks, !lowered, nullptr) * 2 * g.co * sizeof(float);
 }
 
@@ -2271,54 +2432,50 @@ int tc_fprop_stats(const Geo& g, const void* x, const void* w, const void* bias,
     if (stats_bytes < need) return B2C_ERR_WORKSPACE_TOO_SMALL;
     if ((uintptr_t)stats & 15) return B2C_ERR_MISALIGNED;
     StatsOut so{(float*)stats};
-    return tc_fprop_nhwc(g, x, w, bias, nullptr, 0, y, ws, ws_bytes, st, &so);
+    return tc_fprop_any(g, x, w, bias, nullptr, 0, y, ws, ws_bytes, st, &so);
 }
 
 int tc_fprop(const Geo& g, const void* x, const void* w, const void* bias, const b2c_bn_params* bn, int relu,
              void* y, void* ws, size_t ws_bytes, cudaStream_t st)
 {
-    if (g.layout == B2C_LAYOUT_NHWC) return tc_fprop_nhwc(g, x, w, bias, bn, relu, y, ws, ws_bytes, st);
-    NchwWs t;
-    if (!nchw_ws(g, ws, ws_bytes, t)) return B2C_ERR_WORKSPACE_TOO_SMALL;
-    int rc = transpose_inner(x, t.a, g.n, g.ci, g.h * g.w, st);                 // (c, hw) -> (hw, c)
-    if (rc) return rc;
-    rc = tc_fprop_nhwc(as_nhwc(g), t.a, w, bias, bn, relu, t.b, t.inner, t.inner_bytes, st);
-    if (rc) return rc;
-    return transpose_inner(t.b, y, g.n, g.ho * g.wo, g.co, st);                 // (hw, c) -> (c, hw)
+    return tc_fprop_any(g, x, w, bias, bn, relu, y, ws, ws_bytes, st, nullptr);
 }
 
 int tc_dgrad(const Geo& g, const void* dy, const void* w, void* dx, void* ws, size_t ws_bytes, cudaStream_t st)
 {
-    if (g.layout == B2C_LAYOUT_NHWC) return tc_dgrad_nhwc(g, dy, w, dx, ws, ws_bytes, st);
-    NchwWs t;
-    if (!nchw_ws(g, ws, ws_bytes, t)) return B2C_ERR_WORKSPACE_TOO_SMALL;
-    int rc = transpose_inner(dy, t.b, g.n, g.co, g.ho * g.wo, st);
-    if (rc) return rc;
-    rc = tc_dgrad_nhwc(as_nhwc(g), t.b, w, t.a, t.inner, t.inner_bytes, st);
-    if (rc) return rc;
-    return transpose_inner(t.a, dx, g.n, g.h * g.w, g.ci, st);
+    const Copies c = tc_copies(g, B2C_PASS_DGRAD);
+    CopyWs t;
+    if (!copy_ws(c, ws, ws_bytes, t)) return B2C_ERR_WORKSPACE_TOO_SMALL;
+    if (c.y) { const int rc = copy_in(g, dy, t.y, g.ho * g.wo, g.co, st); if (rc) return rc; }
+    const int rc = tc_dgrad_nhwc(copied_geo(g, c), c.y ? t.y : dy, w, c.x ? t.x : dx, t.inner, t.inner_bytes, st);
+    if (rc || !c.x) return rc;
+    return copy_out(g, t.x, dx, g.h * g.w, g.ci, st);
 }
 
-// Few-channel NHWC layers write the im2row matrix of x at the start of the workspace in their forward pass and again
-// in their weight gradient.  A caller that gives the layer a workspace of its own can say that the forward pass's
-// matrix is still there.
-bool tc_keeps_lowered(const Geo& g) { return g.layout == B2C_LAYOUT_NHWC && g.ci % 32 != 0 && tc_supported_nhwc(g, B2C_PASS_WGRAD) && tc_supported_nhwc(g, B2C_PASS_FPROP); }
+// Few-channel NHWC layers write the im2row matrix of x at the start of the workspace (behind the copies) in their forward
+// pass and again in their weight gradient.  A caller that gives the layer a workspace of its own can say that the forward
+// pass's matrix is still there.
+bool tc_keeps_lowered(const Geo& g) { return g.layout == B2C_LAYOUT_NHWC && lowered_ok(g) && tc_supported_nhwc(g, B2C_PASS_WGRAD) && tc_supported_nhwc(g, B2C_PASS_FPROP); }
+
+static int tc_wgrad_any(const Geo& g, const void* x, const void* dy, void* dw, void* db, void* ws, size_t ws_bytes, cudaStream_t st, bool lowered_in_ws)
+{
+    const Copies c = tc_copies(g, B2C_PASS_WGRAD);
+    CopyWs t;
+    if (!copy_ws(c, ws, ws_bytes, t)) return B2C_ERR_WORKSPACE_TOO_SMALL;
+    if (c.x) { const int rc = copy_in(g, x, t.x, g.h * g.w, g.ci, st); if (rc) return rc; }
+    if (c.y) { const int rc = copy_in(g, dy, t.y, g.ho * g.wo, g.co, st); if (rc) return rc; }
+    return tc_wgrad_nhwc(copied_geo(g, c), c.x ? t.x : x, c.y ? t.y : dy, dw, db, t.inner, t.inner_bytes, st, lowered_in_ws);
+}
+
 int tc_wgrad_lowered(const Geo& g, const void* x, const void* dy, void* dw, void* db, void* ws, size_t ws_bytes, cudaStream_t st)
 {
     if (!tc_keeps_lowered(g)) return B2C_ERR_UNSUPPORTED;
-    return tc_wgrad_nhwc(g, x, dy, dw, db, ws, ws_bytes, st, true);
+    return tc_wgrad_any(g, x, dy, dw, db, ws, ws_bytes, st, true);
 }
 
 int tc_wgrad(const Geo& g, const void* x, const void* dy, void* dw, void* db, void* ws, size_t ws_bytes, cudaStream_t st)
 {
-    if (g.layout == B2C_LAYOUT_NHWC) return tc_wgrad_nhwc(g, x, dy, dw, db, ws, ws_bytes, st);
-    NchwWs t;
-    if (!nchw_ws(g, ws, ws_bytes, t)) return B2C_ERR_WORKSPACE_TOO_SMALL;
-    int rc = transpose_inner(x, t.a, g.n, g.ci, g.h * g.w, st);
-    if (rc) return rc;
-    rc = transpose_inner(dy, t.b, g.n, g.co, g.ho * g.wo, st);
-    if (rc) return rc;
-    return tc_wgrad_nhwc(as_nhwc(g), t.a, t.b, dw, db, t.inner, t.inner_bytes, st);
+    return tc_wgrad_any(g, x, dy, dw, db, ws, ws_bytes, st, false);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -2340,7 +2497,7 @@ static Geo fc_pixels_view(int pixels, int ci, int co, int w_layout)
     q.layout = B2C_LAYOUT_NHWC; q.dtype = B2C_F32; q.w_layout = w_layout; q.engine = B2C_ENGINE_TENSOR;
     q.n = 1; q.h = pixels; q.w = 1; q.ci = ci; q.co = co; q.kh = q.kw = 1;
     q.vstr = q.hstr = q.vdil = q.hdil = 1;
-    q.ho = pixels; q.wo = 1; q.M = pixels; q.K = ci;
+    q.ho = pixels; q.wo = 1; q.M = pixels; q.K = ci; q.xp = ci; q.yp = co;
     return q;
 }
 
