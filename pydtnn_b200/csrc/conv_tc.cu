@@ -461,6 +461,9 @@ struct TcParams {
     int cls_tile0[5];
     int cls_M[4], cls_P[4], cls_Q[4], cls_kblocks[4], cls_S[4], cls_low_h[4], cls_low_w[4], cls_r0[4], cls_s0[4];
     int64_t cls_out[4];
+    // FWD with the K loop split over CTAs (a launch with few tiles): CTA (tile, z) takes k-blocks [z * kper, (z + 1) * kper)
+    // and stores its partial tile to row block z of [splits][row tiles * 128][N]; tc_split_finish_kernel adds them.  0: off.
+    int kper;
     // FWD with batch statistics: for every block of 32 output rows, row (m / 32) of `stats` ([ceil(M/32)][2][N] floats)
     // receives the per-channel sum and sum of squares of the stored values (rows past M left out).  Null: off.
     // stats_cta: the grid is a multiple of the column-tile count nt, so a CTA keeps one column tile; it adds the sums
@@ -551,11 +554,11 @@ struct TcSmem {
 // [total * b / G, total * (b + 1) / G) of CTA b, unit = tile * kblocks + kb.
 struct TileWalk {
     int tile, kb_b, kb_e;
-    int next_tile, total_tiles, kblocks;
+    int next_tile, total_tiles, kblocks, kper, plane;
     long long u, u_end;
     __device__ __forceinline__ static long long range_begin(long long total, int cta, int ctas) { return total * cta / ctas; }
-    __device__ __forceinline__ void init(int total_tiles_, int kblocks_) {
-        total_tiles = total_tiles_; kblocks = kblocks_; next_tile = blockIdx.x;
+    __device__ __forceinline__ void init(int total_tiles_, int kblocks_, int kper_, int plane_) {
+        total_tiles = total_tiles_; kblocks = kblocks_; kper = kper_; plane = plane_; next_tile = blockIdx.x;
         const long long total = (long long)total_tiles_ * kblocks_;
         u = range_begin(total, blockIdx.x, gridDim.x); u_end = range_begin(total, blockIdx.x + 1, gridDim.x);
     }
@@ -563,6 +566,7 @@ struct TileWalk {
         if (!BALANCED) {
             if (next_tile >= total_tiles) return false;
             tile = next_tile; next_tile += gridDim.x; kb_b = 0; kb_e = kblocks;
+            if (kper) { kb_b = tile / plane * kper; if (kb_b + kper < kblocks) kb_e = kb_b + kper; }
             return true;
         }
         if (u >= u_end) return false;
@@ -707,7 +711,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             __syncwarp();
         }
         TileWalk w;
-        w.init(total_tiles, p.kblocks);
+        w.init(total_tiles, p.kblocks, MODE == TCM_FWD && !SK && !MULTI && RESKB == 0 ? p.kper : 0, mt * nt);
         while (ok && w.template next<SK>()) {
             const TileGeo tg = tile_geo(w.tile);
             if (MULTI) w.kb_e = tg.kblocks;
@@ -826,7 +830,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             bool ok = true;
             int it = 0, gc = 0;
             TileWalk w;
-            w.init(total_tiles, p.kblocks);
+            w.init(total_tiles, p.kblocks, MODE == TCM_FWD && !SK && !MULTI && RESKB == 0 ? p.kper : 0, mt * nt);
             while (ok && w.template next<SK>()) {
                 const TileGeo tg = tile_geo(w.tile);
                 if (MULTI) w.kb_e = tg.kblocks;
@@ -928,7 +932,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             }
         }
         TileWalk w;
-        w.init(total_tiles, p.kblocks);
+        w.init(total_tiles, p.kblocks, MODE == TCM_FWD && !SK && !MULTI && RESKB == 0 ? p.kper : 0, mt * nt);
         while (ok && w.template next<SK>()) {
             if (MULTI) w.kb_e = tile_geo(w.tile).kblocks;
             // WGRAD: the tiles of the first row block also sum their dy tile over the pixels (the bias gradient);
@@ -1037,7 +1041,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
 #pragma unroll
         for (int i = 0; i < NSLAB; i++) cs0[i] = cs1[i] = 0.f;
         TileWalk w;
-        w.init(total_tiles, p.kblocks);
+        w.init(total_tiles, p.kblocks, MODE == TCM_FWD && !SK && !MULTI && RESKB == 0 ? p.kper : 0, mt * nt);
         while (ok && w.template next<SK>()) {
             const TileGeo tg = tile_geo(w.tile);
             if (MULTI) w.kb_e = tg.kblocks;
@@ -1064,7 +1068,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 fence_proxy_async();
                 __syncwarp();
                 if (lane == 0) {
-                    if (MODE == TCM_FWD) tma_store_2d(&tmap_out, buf, n0 + cc * 32, m0 + quad * 32);
+                    if (MODE == TCM_FWD) tma_store_2d(&tmap_out, buf, n0 + cc * 32, (p.kper ? z * mt * 128 : 0) + m0 + quad * 32);
                     else tma_store_3d(&tmap_out, buf, n0 + cc * 32, m0 + quad * 32, z);
                     tma_store_commit();
                 }
@@ -1298,6 +1302,81 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     tc_fence_before();
     __syncthreads();
     if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem_base, L::TMEM_COLS); }
+}
+
+// Second stage of a forward launch with a split K loop: the partial tiles of a row added in split order, the epilogue
+// steps, the store (row m = (n, i, j) at out + n * o_sn + i * o_sh + j * o_sw) and, when asked for, one row of batch sums
+// per 32 output rows.  A thread takes four channels of ROWS rows; its loads over the splits are independent, so the kernel
+// costs about one trip to L2 (the partials were just written) behind the launch: 2 to 3 us for the 2 to 10 MB it meets.
+struct FinishParams {
+    int M, N, P, Q, splits, pitch;          // pitch: floats per partial row
+    int64_t plane;                          // floats per split
+    const float* partial;
+    float* out;
+    int64_t o_sn, o_sh, o_sw;
+    const float *bias, *mean, *inv_std, *gamma, *beta;
+    int relu;
+    float* stats;
+};
+template <int ROWS>
+__global__ void __launch_bounds__(256) tc_split_finish_kernel(FinishParams p)
+{
+    pdl_prologue();
+    const int lane = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const int n0 = blockIdx.x * 128 + lane * 4;
+    float4 t0 = make_float4(0.f, 0.f, 0.f, 0.f), t1 = t0;
+    if (n0 < p.N) {
+        const bool vec = n0 + 4 <= p.N && p.N % 4 == 0 && p.o_sw % 4 == 0;
+        const int cnt = p.N - n0 < 4 ? p.N - n0 : 4;
+#pragma unroll
+        for (int r = 0; r < ROWS; r++) {
+            const int m = (blockIdx.y * ROWS + r) * 8 + ty;
+            if (m >= p.M) continue;
+            const float* src = p.partial + (int64_t)m * p.pitch + n0;
+            float4 v = __ldcg(reinterpret_cast<const float4*>(src));
+            int z = 1;
+            for (; z + 8 <= p.splits; z += 8) {
+                float4 q[8];
+#pragma unroll
+                for (int u = 0; u < 8; u++) q[u] = __ldcg(reinterpret_cast<const float4*>(src + (z + u) * p.plane));
+#pragma unroll
+                for (int u = 0; u < 8; u++) { v.x += q[u].x; v.y += q[u].y; v.z += q[u].z; v.w += q[u].w; }
+            }
+            for (; z < p.splits; z++) {
+                const float4 q = __ldcg(reinterpret_cast<const float4*>(src + z * p.plane));
+                v.x += q.x; v.y += q.y; v.z += q.z; v.w += q.w;
+            }
+            float a[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int e = 0; e < 4; e++)
+                if (e < cnt) {
+                    if (p.bias) a[e] += __ldg(p.bias + n0 + e);
+                    if (p.mean) { const float t = (a[e] - __ldg(p.mean + n0 + e)) * __ldg(p.inv_std + n0 + e); a[e] = t * __ldg(p.gamma + n0 + e) + __ldg(p.beta + n0 + e); }
+                    if (p.relu) a[e] = fmaxf(a[e], 0.f);
+                }
+            const int img = m / (p.P * p.Q), rem = m - img * (p.P * p.Q), pi = rem / p.Q, qi = rem - pi * p.Q;
+            float* d = p.out + img * p.o_sn + pi * p.o_sh + qi * p.o_sw + n0;
+            if (vec) *reinterpret_cast<float4*>(d) = make_float4(a[0], a[1], a[2], a[3]);
+            else for (int e = 0; e < cnt; e++) d[e] = a[e];
+            t0.x += a[0]; t0.y += a[1]; t0.z += a[2]; t0.w += a[3];
+            t1.x = fmaf(a[0], a[0], t1.x); t1.y = fmaf(a[1], a[1], t1.y); t1.z = fmaf(a[2], a[2], t1.z); t1.w = fmaf(a[3], a[3], t1.w);
+        }
+    }
+    if (ROWS == 4 && p.stats) {              // the block's 32 rows: one row of [2][N] sums (N is a multiple of 4 here)
+        __shared__ float4 s0[8][32], s1[8][32];
+        s0[ty][lane] = t0; s1[ty][lane] = t1;
+        __syncthreads();
+        if (ty == 0 && n0 < p.N) {
+#pragma unroll
+            for (int y = 1; y < 8; y++) {
+                const float4 u = s0[y][lane], w = s1[y][lane];
+                t0.x += u.x; t0.y += u.y; t0.z += u.z; t0.w += u.w; t1.x += w.x; t1.y += w.y; t1.z += w.z; t1.w += w.w;
+            }
+            float* row = p.stats + (size_t)blockIdx.y * 2 * p.N + n0;
+            *reinterpret_cast<float4*>(row) = t0;
+            *reinterpret_cast<float4*>(row + p.N) = t1;
+        }
+    }
 }
 
 // Second stage of the weight gradient: fixed-order sum of the per-split partial tiles, written in the
@@ -1713,6 +1792,15 @@ static int dispatch_fwd(int bn, const CUtensorMap& ma, const CUtensorMap& mb0, c
         if (bn == 64) return launch_tc<TCM_FWD, 64, 6, true, 2, BSRC>(ma, mb0, mb1, mo, p, 1, st);
         return launch_tc<TCM_FWD, 128, 4, true, 2, BSRC>(ma, mb0, mb1, mo, p, 1, st);
     }
+    if (p.kper) {
+        const int splits = (p.kblocks + p.kper - 1) / p.kper;
+        if (p.kper <= TC_CHUNK) {
+            if (bn == 64) return launch_tc<TCM_FWD, 64, 6, false, 2, BSRC, 1>(ma, mb0, mb1, mo, p, splits, st);
+            return launch_tc<TCM_FWD, 128, 4, false, 2, BSRC, 1>(ma, mb0, mb1, mo, p, splits, st);
+        }
+        if (bn == 64) return launch_tc<TCM_FWD, 64, 6, false, 2, BSRC>(ma, mb0, mb1, mo, p, splits, st);
+        return launch_tc<TCM_FWD, 128, 4, false, 2, BSRC>(ma, mb0, mb1, mo, p, splits, st);
+    }
     // Short K loops are bound by the epilogue.  Tiles of one tensor-memory chunk (at most TC_CHUNK k-blocks) take the
     // streaming epilogue (32 columns at a time straight from tensor memory); up to four k-blocks per tile a shallower
     // operand pipeline also leaves room for four output slabs per drain warp, so a whole tile's stores are in flight.
@@ -1790,17 +1878,32 @@ static int transpose_t(const void* src, void* dst, int n, int rows, int cols, in
 // Where a forward pass leaves the batch statistics of its output (see TcParams::stats), or null.
 struct StatsOut { float* sums; };
 
-// Whole tiles or balanced k-block ranges for a forward launch (cost in k-block units: whole tiles take
-// rounds x kblocks; balanced ranges take units / G plus the hand-over of one partial tile: store, flag, load, add,
-// about four k-blocks).
-static bool fwd_prefers_balanced(int64_t M, int N, int64_t kblocks)
+// How a forward launch is cut: whole tiles, balanced k-block ranges (sk), or the K loop of every tile split over several
+// CTAs (kper k-blocks each).  Costs in k-block units (0.6 us): whole tiles take rounds x kblocks; balanced ranges take
+// units / G plus the hand-over of partial tiles, one after the other in the CTA that owns the tile (about four units for
+// the first, ten for each further CTA on the same tile: 57 us on 32 tiles of 144 k-blocks that are 20 us of products); a split
+// takes its k-blocks, the partials' way through L2 and the second stage's launch (about five units).  The partials of
+// a split fit the balanced mode's scratch because tiles x splits is at most one CTA per SM.
+struct FwdPlan { bool sk; int kper; };
+static FwdPlan fwd_plan(int64_t M, int N, int64_t kblocks)
 {
     const int G = tc_sm_count();
     const int BN = N <= 64 ? 64 : 128;
     const int64_t tiles = ((M + 127) / 128) * ((N + BN - 1) / BN);
     const int64_t rounds = (tiles + G - 1) / G;
-    const double plain = (double)rounds * (double)kblocks, balanced = (double)(tiles * kblocks) / G + 4.0;
-    return tiles * kblocks >= 4 * (int64_t)G && balanced < tc_balance_threshold() * plain;
+    const double plain = (double)rounds * (double)kblocks;
+    const double shared = (double)G / (double)tiles;         // CTAs on one tile
+    const double balanced = (double)(tiles * kblocks) / G + 4.0 + (shared > 2.0 ? 10.0 * (shared - 2.0) : 0.0);
+    FwdPlan best{false, 0};
+    double cost = plain;
+    if (tiles * kblocks >= 4 * (int64_t)G && balanced < tc_balance_threshold() * plain) { best.sk = true; cost = balanced; }
+    for (int64_t s = 2; s * tiles <= G && s <= kblocks; s++) {
+        const int64_t kper = (kblocks + s - 1) / s;
+        if ((kblocks + kper - 1) / kper != s) continue;
+        const double split = (double)kper + 5.0 + (double)s * (double)M * N * 8.0 / 4e12 / 0.6e-6;
+        if (split < 0.9 * cost) { best.sk = false; best.kper = (int)kper; cost = split / 0.9; }
+    }
+    return best;
 }
 
 // Rows of the statistics buffer a forward launch with batch sums writes: one per CTA group and row quadrant when the
@@ -1811,7 +1914,8 @@ static int64_t fwd_stats_rows(int64_t M, int N, int64_t kblocks, bool may_balanc
     const int BN = N <= 64 ? 64 : 128;
     const int64_t nt = (N + BN - 1) / BN, tiles = ((M + 127) / 128) * nt;
     const int64_t grid = tiles < G ? tiles : G;
-    const bool cta = nt <= grid && !(may_balance && fwd_prefers_balanced(M, N, kblocks));
+    const FwdPlan plan = may_balance ? fwd_plan(M, N, kblocks) : FwdPlan{false, 0};
+    const bool cta = nt <= grid && !plan.sk && !plan.kper;
     if (by_cta) *by_cta = cta;
     return cta ? (grid / nt) * 4 : (M + 31) / 32;
 }
@@ -1857,8 +1961,7 @@ static int run_fwd(const FwdLaunch& f, const void* act, const void* w, PrepParam
     float* w_hi = (float*)base;
     float* w_lo = (float*)(base + fbytes);
     const int BN = f.N <= 64 ? 64 : 128;
-    // Balanced mode when whole tiles would leave a large part of the last round of the CTA grid idle.
-    int sk = 0;
+    int sk = 0, kper = 0;
     int* sk_flags = (int*)(base + 2 * fbytes);
     float* sk_partial = (float*)((uintptr_t)sk_flags + sk_flag_bytes());
     // hand-over flags: in the library's self-cleaning bank when this stream has one, else cleared in the workspace
@@ -1867,7 +1970,10 @@ static int run_fwd(const FwdLaunch& f, const void* act, const void* w, PrepParam
     {
         const int64_t kblocks = (int64_t)f.kh * f.kw * cblocks;
         const bool room = base + 2 * fbytes + sk_bytes() <= (uintptr_t)ws + ws_bytes;
-        if (!filters_ready && room && fwd_prefers_balanced((int64_t)f.n * f.P * f.Q, f.N, kblocks)) sk = 1;
+        if (!filters_ready && room && !zf) {
+            const FwdPlan plan = fwd_plan((int64_t)f.n * f.P * f.Q, f.N, kblocks);
+            sk = plan.sk; kper = plan.kper;
+        }
     }
     // The filter itself serves as the B operand when its layout allows a tensor map over it (the channel axis
     // that is contiguous decides K-major or MN-major); otherwise hi/lo copies in the GEMM layout are written first.
@@ -1919,22 +2025,34 @@ static int run_fwd(const FwdLaunch& f, const void* act, const void* w, PrepParam
     const bool dense = f.o_sw % 4 == 0 && f.o_sh == (int64_t)f.Q * f.o_sw && f.o_sn == (int64_t)f.P * f.Q * f.o_sw;
     CUtensorMap mo = mbh;
     p.tma_store = 0;
-    if (dense && make_map_out(&mo, out, 0, (uint64_t)p.M, (uint64_t)f.N, (uint64_t)f.o_sw)) p.tma_store = 1;
+    const int splits = kper ? (p.kblocks + kper - 1) / kper : 1;
+    const int64_t mrows = (int64_t)((p.M + 127) / 128) * 128;
+    if (kper) {
+        if (!make_map_out(&mo, sk_partial, 0, (uint64_t)(splits * mrows), (uint64_t)round4(f.N), (uint64_t)round4(f.N))) return B2C_ERR_UNSUPPORTED;
+        p.tma_store = 1; p.kper = kper; p.epi = 0;
+    } else if (dense && make_map_out(&mo, out, 0, (uint64_t)p.M, (uint64_t)f.N, (uint64_t)f.o_sw)) p.tma_store = 1;
     if (zf) {
         if (p.tma_store || ((zf->off_w | zf->off_h) & 3)) return B2C_ERR_UNSUPPORTED;
         p.zfill = 1; p.z_W = zf->W; p.z_H = zf->H; p.z_w = zf->off_w; p.z_h = zf->off_h;
     }
     if (stats) {
-        // the statistics are taken from the staging slabs of the TMA-store epilogue
+        // the statistics are taken from the staging slabs of the TMA-store epilogue, or by the second stage of a split
         if (!p.tma_store) return B2C_ERR_UNSUPPORTED;
-        p.stats = stats->sums;
+        p.stats = kper ? nullptr : stats->sums;
         bool by_cta = false;
         fwd_stats_rows(p.M, p.N, p.kblocks, !filters_ready, &by_cta);
-        p.stats_cta = by_cta ? 1 : 0;       // by_cta implies sk == 0: balanced ranges are only taken when preferred
+        p.stats_cta = by_cta ? 1 : 0;       // by_cta implies whole tiles
     }
-    if (bsrc == TCB_RAW_K) return dispatch_fwd<TCB_RAW_K>(BN, ma, mbh, mbl, mo, p, st);
-    if (bsrc == TCB_RAW_MN) return dispatch_fwd<TCB_RAW_MN>(BN, ma, mbh, mbl, mo, p, st);
-    return dispatch_fwd<TCB_SPLIT>(BN, ma, mbh, mbl, mo, p, st);
+    const int rc = bsrc == TCB_RAW_K ? dispatch_fwd<TCB_RAW_K>(BN, ma, mbh, mbl, mo, p, st)
+                 : bsrc == TCB_RAW_MN ? dispatch_fwd<TCB_RAW_MN>(BN, ma, mbh, mbl, mo, p, st)
+                 : dispatch_fwd<TCB_SPLIT>(BN, ma, mbh, mbl, mo, p, st);
+    if (rc || !kper) return rc;
+    FinishParams fp{p.M, p.N, p.P, p.Q, splits, round4(f.N), mrows * round4(f.N), sk_partial, out, f.o_sn, f.o_sh, f.o_sw,
+                    p.bias, p.mean, p.inv_std, p.gamma, p.beta, relu, stats ? stats->sums : nullptr};
+    const dim3 fgrid((p.N + 127) / 128, stats ? (p.M + 31) / 32 : (p.M + 7) / 8);
+    if (stats) launch_pdl(tc_split_finish_kernel<4>, fgrid, 256, 0, st, fp);
+    else launch_pdl(tc_split_finish_kernel<1>, fgrid, 256, 0, st, fp);
+    return check_launch("tc_split_finish_kernel");
 }
 
 static LowerParams lower_params(const Geo& g)
