@@ -72,6 +72,8 @@ int b2c_version(void);
 /* Number of kernels this library has launched in the process so far (diagnostic; lets a caller
  * state how many of its launches fall inside a timed region). No counterpart in the reference. */
 uint64_t b2c_launch_count(void);
+/* Adds n to that number: for a caller that replays a captured graph of n of this library's launches. */
+void b2c_note_launches(uint64_t n);
 
 /* Reads and clears the status word the tensor-core kernels set when one of their bounded in-kernel
  * waits runs out (the kernel then skips its remaining work and returns; the context stays usable).

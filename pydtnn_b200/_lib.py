@@ -39,6 +39,7 @@ PROTOTYPES = {
     "b2c_last_cuda_error": (c_char_p, []),
     "b2c_version": (c_int, []),
     "b2c_launch_count": (ctypes.c_uint64, []),
+    "b2c_note_launches": (None, [ctypes.c_uint64]),
     "b2c_check_device_status": (c_int, [POINTER(c_int)]),
     "b2c_conv_workspace_bytes": (c_size_t, [POINTER(ConvDesc), c_int]),
     "b2c_conv_engine_for": (c_int, [POINTER(ConvDesc), c_int]),

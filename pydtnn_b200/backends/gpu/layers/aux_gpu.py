@@ -58,6 +58,7 @@ class BatchNormalizationGPU(LayerGPU, BatchNormalization):
         self._dt = _lib.dtype_code(m.dtype)
         self._hw = self.hi * self.wi if self.spatial else 1
         self.updated_running_var = True
+        self._inv_std_step = 0           # replayed training steps of the model when _inv_std was computed
 
     def forward(self, x):
         m = self.model
@@ -109,10 +110,11 @@ class BatchNormalizationGPU(LayerGPU, BatchNormalization):
         """1 / sqrt(running_var + eps) on the device, recomputed (one small kernel, no host round trip) only after
         the running variance changed: a training step or a checkpoint load
         (pydtnn/backends/cpu/layers/batch_normalization_cpu.py:92-94 refreshes it under the same flag)."""
-        if self.updated_running_var:
+        if self.updated_running_var or self._inv_std_step != self.model.replayed_steps:
             _lib.check(_lib.lib().b2c_bn_inv_std(self._dt, self.ci, self.running_var.ptr, float(self.epsilon),
                                                  self._inv_std.gpudata, self.model.stream_handle))
             self.updated_running_var = False
+            self._inv_std_step = self.model.replayed_steps
         return self._inv_std
 
     def backward(self, dy):
@@ -230,8 +232,16 @@ class FlattenGPU(LayerGPU, Flatten):
             _lib.check(_lib.lib().b2c_transpose(_lib.dtype_code(m.dtype), m.batch_size, hw, c, self._in(x, "x"), self.y.ptr,
                                                 m.stream_handle))
             return self.y
-        self.y = TensorGPU(x.ary.reshape((m.batch_size, *self.shape)), m.tensor_format)
+        self.y = self._view(self.y, x, (m.batch_size, *self.shape))
         return self.y
+
+    @staticmethod
+    def _view(last, t, dims):
+        """``t`` with other dimensions; the handle of the last call where that still is the same memory."""
+        a = t.ary
+        if last is not None and last.ary.gpudata == a.gpudata and last.ary.shape == dims:
+            return last
+        return TensorGPU(a.reshape(dims), t.tensor_format)
 
     def backward(self, dy):
         m = self.model
@@ -242,7 +252,7 @@ class FlattenGPU(LayerGPU, Flatten):
                                                     m.stream_handle))
                 self.dx.written()
             else:
-                self.dx = TensorGPU(dy.ary.reshape((m.batch_size, *self.prev_shape)), m.tensor_format)
+                self.dx = self._view(self.dx, dy, (m.batch_size, *self.prev_shape))
             return self.dx
 
 

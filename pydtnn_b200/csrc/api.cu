@@ -76,6 +76,8 @@ extern "C" const char* b2c_last_cuda_error(void) { return g_cuda_err; }
 extern "C" int b2c_version(void) { return 100; }
 extern "C" uint64_t b2c_launch_count(void) { return (uint64_t)__atomic_load_n(&b2c::g_launches, __ATOMIC_RELAXED); }
 
+extern "C" void b2c_note_launches(uint64_t n) { __atomic_add_fetch(&b2c::g_launches, (unsigned long long)n, __ATOMIC_RELAXED); }
+
 extern "C" int b2c_check_device_status(int* detail) {
     int v = 0;
     int rc = tc_read_status(&v);

@@ -59,6 +59,17 @@ class LayerAndActivationBase(ABC):
         self.reqs_allred = {}
         self.stream_2 = None
 
+    #: attributes a hook hands to the next one; everything else that changes on a layer may change its launches
+    _PASSED_ON = frozenset(("x", "_x_ptr", "prestats", "residual", "updated_running_var", "_inv_std_step", "_lowered_valid"))
+
+    def __setattr__(self, name, value):
+        d = self.__dict__
+        if name not in self._PASSED_ON and d.get(name, d) is not value:
+            m = d.get("model")
+            if m is not None:
+                m.layer_edits += 1
+        object.__setattr__(self, name, value)
+
     def set_model(self, parent_model):
         self.model = parent_model
         self.id = next(parent_model.layer_id)

@@ -21,7 +21,8 @@ from .layers import (BatchNormalization, Conv2D, Conv2DBatchNormalization, Conv2
                      Relu)
 from .losses import CategoricalCrossEntropy
 from .performance_counter import PerformanceCounter
-from .tensor_gpu import empty
+from .recorder import Recorder
+from .tensor_gpu import Storage, empty
 from .utils import (EVALUATE_MODE, PYDTNN_TENSOR_FORMAT_NCHW, PYDTNN_TENSOR_FORMAT_NHWC, TRAIN_MODE,
                     UNSPECIFIED_MODE, np_dtype)
 
@@ -68,6 +69,10 @@ class Model:
             if dist.is_initialized() and dist.get_world_size() > 1:
                 self.comm = dist.group.WORLD if comm is True else comm
                 self.rank, self.nprocs = dist.get_rank(), dist.get_world_size()
+        self.layer_edits = 0             # counts attribute changes on this model's layers (see recorder.py)
+        self.record_passes = True        # replay training and evaluation passes as CUDA graphs once they repeat
+        self._train_recorder, self._eval_recorder = Recorder(self), Recorder(self)
+        self.replayed_steps = 0
         self.layers = []
         self.layer_id = itertools.count()
         self.nparams = 0
@@ -127,6 +132,7 @@ class Model:
         layer.initialize(prev_shape, need_dx, y)
         self.nparams += layer.nparams
         self.layers.append(layer)
+        self.layer_edits += 1
         if layer.act:
             self.add(layer.act())
 
@@ -203,6 +209,19 @@ class Model:
             out.append(cur); i += 1
         return out
 
+    # -- recorded passes -----------------------------------------------------------------------------
+    def _recordable(self):
+        """Whether a pass may be recorded: no ranks to meet, nothing timed from the host (what the layers themselves
+        do is looked at when a recording is made)."""
+        return self.record_passes and self.comm is None and not self.tracer.enabled \
+            and getattr(self, "conv_profile", None) is None
+
+    def _pass_key(self, *more):
+        """Everything on the host that the launches of a pass depend on, and the shared buffers they use."""
+        keep = (wsp._buf, wsp._side, wsp._red, wsp._stats)
+        return (self.layer_edits, Storage.moves, len(self.layers), self.overlap_wgrad, self.blocking_mpi, *map(id, keep),
+                *more), keep
+
     # -- steps ---------------------------------------------------------------------------------------
     def _ensure_loss(self):
         if self.loss_func is None:
@@ -237,6 +256,17 @@ class Model:
         self._fuse_training()
         if global_batch_size is None:
             global_batch_size = self.batch_size * self.nprocs
+        if not self._recordable():
+            return self._forward_backward(global_batch_size)
+        key, keep = self._pass_key(global_batch_size, id(self.loss_func), getattr(self.loss_func, "eps", None),
+                                   id(self.y_batch))
+        keep += (self.loss_func, self.y_batch)
+        recorder = self._train_recorder
+        if recorder.graph is not None:
+            self.replayed_steps += 1     # the batch norms' running variances change without their hooks being called
+        return recorder.run(key, keep, lambda: self._forward_backward(global_batch_size))
+
+    def _forward_backward(self, global_batch_size):
         tr = self.tracer
         x = self.layers[0].y
         for layer in self.layers[1:]:
@@ -351,6 +381,8 @@ class Model:
         if self._eval_layers is None:
             self._fuse_training()          # the flags it sets (absorbed ReLUs, folded sums) are read in evaluation too
             self._eval_layers = self._fuse_inference(self.layers)
+            self.layer_edits += 1
+            self._norms = [l for l in self.get_all_layers() if isinstance(l, BatchNormalization)]
         if x_batch is not None:
             xin = self.layers[0].y.ary
             if isinstance(x_batch, torch.Tensor):
@@ -360,9 +392,12 @@ class Model:
                 xin.set(x_batch)
         if isinstance(next_batch, torch.Tensor):
             self._stage_next(next_batch, None)
-        x = self.layers[0].y
-        for layer in self._eval_layers[1:]:
-            x = layer.forward(x)
+        if self._recordable():
+            for bn in self._norms:       # refreshed outside the recording: only after a step or a load
+                bn.inference_inv_std()
+            x = self._eval_recorder.run(*self._pass_key(id(self._eval_layers)), self._forward)
+        else:
+            x = self._forward()
         x.ary          # the answer is the caller's: in the model's tensor format before this call returns
         if y_batch is None:
             return x
@@ -371,6 +406,12 @@ class Model:
         self.y_batch.set(lab.astype(np.int32) if not isinstance(lab, torch.Tensor) else lab.cpu().numpy().astype(np.int32))
         loss, _ = self.loss_func(x, self.y_batch, self.batch_size * self.nprocs)
         return x, loss
+
+    def _forward(self):
+        x = self.layers[0].y
+        for layer in self._eval_layers[1:]:
+            x = layer.forward(x)
+        return x
 
     def store_weights_and_bias(self, filename, layout="cpu"):
         """Write the reference's NPZ checkpoint (pydtnn/model.py:380-384); see ``checkpoint.py`` for layouts."""

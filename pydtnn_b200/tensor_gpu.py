@@ -16,12 +16,23 @@ _TORCH_DTYPE = {np.dtype(np.float32): torch.float32, np.dtype(np.float64): torch
                 np.dtype(np.int32): torch.int32, np.dtype(np.int64): torch.int64}
 
 
+class Storage:
+    #: counts, over the process, the times a tensor handle came to stand for other memory: recorded launches are only
+    #: valid while this has not moved
+    moves = 0
+
+
 class DeviceArray:
     """Stands in for ``pycuda.gpuarray.GPUArray`` for the members the layer code touches."""
 
     def __init__(self, tensor: torch.Tensor):
         assert tensor.is_contiguous()
         self.t = tensor
+
+    def __setattr__(self, name, value):
+        if name in self.__dict__:
+            Storage.moves += 1
+        object.__setattr__(self, name, value)
 
     @property
     def shape(self):
@@ -88,6 +99,11 @@ class TensorGPU:
         self.tensor_type = tensor_type
         self.desc = desc
 
+    def __setattr__(self, name, value):
+        if name == "ary" and "ary" in self.__dict__:
+            Storage.moves += 1
+        object.__setattr__(self, name, value)
+
     @property
     def ptr(self):
         return ctypes.c_void_p(self.ary.gpudata)
@@ -148,12 +164,9 @@ class ChannelLastTensor(TensorGPU):
         if self._nchw is None:
             n, c, h, w = self._dims
             self._nchw = empty(self._dims, self._cl.dtype, self._cl.t.device)
-            ChannelLastTensor.looks += 1
+            Storage.moves += 1
             transpose_inner(self._cl, self._nchw, n, h * w, c)
         return self._nchw
-
-    #: counts first looks in the process: a recorded sequence of launches is only valid while it has not moved
-    looks = 0
 
     @property
     def dims(self):
