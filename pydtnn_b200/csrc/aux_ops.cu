@@ -90,25 +90,6 @@ template <typename T> struct StatF {
 };
 
 template <typename T>
-__global__ void bn_stats_final_kernel(const double* __restrict__ partial, int chunks, int c, double count,
-                                      double momentum, double eps, T* running_mean, T* running_var,
-                                      T* save_mean, T* save_inv_std)
-{
-    pdl_prologue();
-    int ch = blockIdx.x * blockDim.x + threadIdx.x;
-    if (ch >= c) return;
-    double s = 0.0, ss = 0.0;
-    for (int i = 0; i < chunks; i++) { s += partial[((int64_t)i * 2) * c + ch]; ss += partial[((int64_t)i * 2 + 1) * c + ch]; }
-    double mean = s / count;
-    double var = ss / count - mean * mean;
-    if (var < 0.0) var = 0.0;
-    save_mean[ch] = (T)mean;
-    save_inv_std[ch] = (T)(1.0 / sqrt(var + eps));
-    running_mean[ch] = (T)(momentum * (double)running_mean[ch] + (1.0 - momentum) * mean);
-    running_var[ch] = (T)(momentum * (double)running_var[ch] + (1.0 - momentum) * var);
-}
-
-template <typename T>
 __global__ void bn_apply_kernel(const T* __restrict__ x, T* __restrict__ y, const T* __restrict__ mean,
                                 const T* __restrict__ inv_std, const T* __restrict__ gamma, const T* __restrict__ beta,
                                 int64_t total, int c, int hw, int nchw, int relu, int ref_order, const T* __restrict__ addend)
@@ -134,17 +115,6 @@ template <typename T> struct BnBwdF {
         v0 = (double)g * (double)xn; v1 = (double)g;
     }
 };
-
-template <typename T>
-__global__ void bn_bwd_final_kernel(const double* __restrict__ partial, int chunks, int c, T* dgamma, T* dbeta)
-{
-    pdl_prologue();
-    int ch = blockIdx.x * blockDim.x + threadIdx.x;
-    if (ch >= c) return;
-    double s0 = 0.0, s1 = 0.0;
-    for (int i = 0; i < chunks; i++) { s0 += partial[((int64_t)i * 2) * c + ch]; s1 += partial[((int64_t)i * 2 + 1) * c + ch]; }
-    dgamma[ch] = (T)s0; dbeta[ch] = (T)s1;
-}
 
 // dx = (gamma / (std*n)) * (n*dy - xn*dgamma - dbeta)   (pydtnn/cython_modules/bn_training_cython.pyx:227)
 template <typename T>
@@ -298,8 +268,9 @@ struct BnBwdV4 {
 // With a few hundred chunks a thread has a handful of independent loads, so the kernel costs one memory round trip.
 // mode 0: batch statistics -> save_mean, save_inv_std, running averages. mode 1: (dgamma, dbeta).
 // mode 2: single sum -> out0.
+template <typename T>
 __global__ void __launch_bounds__(256) reduce2_final_warp_kernel(const double* __restrict__ partial, int chunks, int c, int mode, double count,
-                                                                 double momentum, double eps, float* out0, float* out1, float* run0, float* run1)
+                                                                 double momentum, double eps, T* out0, T* out1, T* run0, T* run1)
 {
     pdl_prologue();
     __shared__ double w0[2][4], w1[2][4];
@@ -330,11 +301,11 @@ __global__ void __launch_bounds__(256) reduce2_final_warp_kernel(const double* _
     if (mode == 0) {
         double mean = s0 / count, var = s1 / count - mean * mean;
         if (var < 0.0) var = 0.0;
-        out0[ch] = (float)mean; out1[ch] = (float)(1.0 / sqrt(var + eps));
-        run0[ch] = (float)(momentum * (double)run0[ch] + (1.0 - momentum) * mean);
-        run1[ch] = (float)(momentum * (double)run1[ch] + (1.0 - momentum) * var);
-    } else if (mode == 1) { out0[ch] = (float)s0; out1[ch] = (float)s1; }
-    else out0[ch] = (float)s0;
+        out0[ch] = (T)mean; out1[ch] = (T)(1.0 / sqrt(var + eps));
+        run0[ch] = (T)(momentum * (double)run0[ch] + (1.0 - momentum) * mean);
+        run1[ch] = (T)(momentum * (double)run1[ch] + (1.0 - momentum) * var);
+    } else if (mode == 1) { out0[ch] = (T)s0; out1[ch] = (T)s1; }
+    else out0[ch] = (T)s0;
 }
 
 __global__ void __launch_bounds__(256) bn_apply_v4_kernel(const float4* __restrict__ x, float4* __restrict__ y, const float* __restrict__ mean,
@@ -505,10 +476,11 @@ static V4Geo v4_apply_geo(int64_t rows, int c)
     return g;
 }
 
+template <typename T>
 static int final_warp(const double* partial, int chunks, int c, int mode, double count, double momentum, double eps,
-                      float* o0, float* o1, float* r0, float* r1, cudaStream_t st)
+                      T* o0, T* o1, T* r0, T* r1, cudaStream_t st)
 {
-    launch_pdl(reduce2_final_warp_kernel, (c + 1) / 2, 256, 0, st, partial, chunks, c, mode, count, momentum, eps, o0, o1, r0, r1);
+    launch_pdl(reduce2_final_warp_kernel<T>, (c + 1) / 2, 256, 0, st, partial, chunks, c, mode, count, momentum, eps, o0, o1, r0, r1);
     return check_launch("reduce2_final_warp");
 }
 
@@ -522,7 +494,7 @@ int channel_sum_v4(int n, int c, int hw, const void* src, void* dst, void* ws, s
     SumV4 f{(const float4*)src};
     launch_pdl(reduce2_v4_kernel<SumV4>, dim3(g.gx, g.chunks), 256, 0, st, f, (double*)ws, g);
     int rc = check_launch("reduce2_v4(sum)"); if (rc) return rc;
-    return final_warp((const double*)ws, g.chunks, c, 2, 1.0, 0.0, 0.0, (float*)dst, nullptr, nullptr, nullptr, st);
+    return final_warp((const double*)ws, g.chunks, c, 2, 1.0, 0.0, 0.0, (float*)dst, (float*)nullptr, (float*)nullptr, (float*)nullptr, st);
 }
 
 static unsigned ew_blocks(int64_t total) { int64_t b = (total + 255) / 256; return (unsigned)(b > 148 * 16 ? 148 * 16 : (b < 1 ? 1 : b)); }
@@ -549,8 +521,7 @@ static int bn_train_forward_t(int layout, int n, int c, int hw, const T* x, cons
     StatF<T> f{x};
     int rc = launch_reduce2(f, scratch, layout, n, c, hw, chunks, st);
     if (rc) return rc;
-    launch_pdl(bn_stats_final_kernel<T>, (c + 127) / 128, 128, 0, st, scratch, chunks, c, (double)n * hw, momentum, eps, rm, rv, sm, si);
-    rc = check_launch("bn_stats_final"); if (rc) return rc;
+    rc = final_warp<T>(scratch, chunks, c, 0, (double)n * hw, momentum, eps, sm, si, rm, rv, st); if (rc) return rc;
     int64_t total = (int64_t)n * c * hw;
     launch_pdl(bn_apply_kernel<T>, ew_blocks(total), 256, 0, st, x, y, sm, si, gamma, beta, total, c, hw, layout == B2C_LAYOUT_NCHW, relu, 0, addend);
     return check_launch("bn_apply");
@@ -570,7 +541,7 @@ static int bn_train_backward_t(int layout, int n, int c, int hw, const T* x, con
                   (const float*)beta, relu};
         launch_pdl(reduce2_v4_kernel<BnBwdV4>, dim3(g.gx, g.chunks), 256, 0, st, f, scratch, g);
         int rc = check_launch("reduce2_v4(bn_bwd)"); if (rc) return rc;
-        rc = final_warp(scratch, g.chunks, c, 1, 1.0, 0.0, 0.0, (float*)dgamma, (float*)dbeta, nullptr, nullptr, st);
+        rc = final_warp(scratch, g.chunks, c, 1, 1.0, 0.0, 0.0, (float*)dgamma, (float*)dbeta, (float*)nullptr, (float*)nullptr, st);
         if (rc || !dx) return rc;
         V4Geo ga = v4_apply_geo((int64_t)n * hw, c);
         launch_pdl(bn_bwd_dx_v4_kernel, dim3(ga.gx, ga.chunks), 256, 0, st, (const float4*)x, (const float4*)dy, (const float4*)y, (const float*)gamma,
@@ -582,8 +553,7 @@ static int bn_train_backward_t(int layout, int n, int c, int hw, const T* x, con
     BnBwdF<T> f{x, dy, y, sm, si, relu};
     int rc = launch_reduce2(f, scratch, layout, n, c, hw, chunks, st);
     if (rc) return rc;
-    launch_pdl(bn_bwd_final_kernel<T>, (c + 127) / 128, 128, 0, st, scratch, chunks, c, dgamma, dbeta);
-    rc = check_launch("bn_bwd_final"); if (rc) return rc;
+    rc = final_warp<T>(scratch, chunks, c, 1, 1.0, 0.0, 0.0, dgamma, dbeta, (T*)nullptr, (T*)nullptr, st); if (rc) return rc;
     if (!dx) return B2C_OK;
     int64_t total = (int64_t)n * c * hw;
     launch_pdl(bn_bwd_dx_kernel<T>, ew_blocks(total), 256, 0, st, x, dy, y, gamma, sm, si, dgamma, dbeta, dx, total, c, hw,

@@ -10,6 +10,8 @@
 // float32 uses FP32 FMA, float64 uses FP64 FMA.  This engine is the one every shape can run on;
 // the tensor-core engine (conv_tc.cu) takes over the shapes it supports.
 #include "b2c_common.cuh"
+#include <atomic>
+#include <type_traits>
 
 namespace b2c {
 
@@ -41,6 +43,8 @@ struct IgemmParams {
     // tap (r, s) of the (R, S) grid is filter tap (tap_r0 + r*tap_rs, tap_s0 + s*tap_ss).  Identity elsewhere.
     int pix_h0, pix_hs, pix_w0, pix_ws;
     int tap_r0, tap_rs, tap_s0, tap_ss;
+    bool small;                   // x (dx), y (dy) with a window's overhang and the filter have fewer than 2^31 elements each
+    int lin_h, lin_w;             // dgrad: how far one tap of the (R, S) grid moves the gathered row and column
 };
 
 template <typename T> struct Epilogue { const T *bias, *mean, *inv_std, *gamma, *beta; int relu; };
@@ -90,13 +94,8 @@ __device__ __forceinline__ bool gather_off(const IgemmParams& p, const Info& pix
     return true;
 }
 
-template <typename T> __device__ __forceinline__ void lds4(const T* p, T (&o)[4]);
-template <> __device__ __forceinline__ void lds4<float>(const float* p, float (&o)[4]) {
+__device__ __forceinline__ void lds4(const float* p, float (&o)[4]) {
     float4 v = *reinterpret_cast<const float4*>(p); o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
-}
-template <> __device__ __forceinline__ void lds4<double>(const double* p, double (&o)[4]) {
-    double2 a = *reinterpret_cast<const double2*>(p), b = *reinterpret_cast<const double2*>(p + 2);
-    o[0] = a.x; o[1] = a.y; o[2] = b.x; o[3] = b.y;
 }
 
 template <typename T> __device__ __forceinline__ T apply_epilogue(T v, int n, const Epilogue<T>& ep) {
@@ -106,17 +105,16 @@ template <typename T> __device__ __forceinline__ T apply_epilogue(T v, int n, co
     return v;
 }
 
-template <typename T> struct TileCfg;
-template <> struct TileCfg<float> { static constexpr int BK = 16; };
-template <> struct TileCfg<double> { static constexpr int BK = 8; };
+constexpr int FMA_BK = 16;
 
-template <typename T, int MODE, int BN, int TN>
+template <int MODE, int BN, int TN>
 __global__ void __launch_bounds__(256)
-igemm_kernel(IgemmParams p, const T* __restrict__ A, const T* __restrict__ B, T* __restrict__ C,
-             T* __restrict__ partial, Epilogue<T> ep)
+igemm_kernel(IgemmParams p, const float* __restrict__ A, const float* __restrict__ B, float* __restrict__ C,
+             float* __restrict__ partial, Epilogue<float> ep)
 {
+    using T = float;
     pdl_prologue();
-    constexpr int BM = 128, NT = 256, BK = TileCfg<T>::BK;
+    constexpr int BM = 128, NT = 256, BK = FMA_BK;
     constexpr int A_PER = BM * BK / NT, B_PER = BN * BK / NT;
     constexpr int PADW = 16 / sizeof(T);
     __shared__ __align__(16) T As[2][BK][BM + PADW];
@@ -203,27 +201,18 @@ igemm_kernel(IgemmParams p, const T* __restrict__ A, const T* __restrict__ B, T*
         for (int k = 0; k < BK; k++) {
             T a[8], b[TN];
             T t4[4];
-            lds4<T>(&As[cur][k][ty * 4], t4);
+            lds4(&As[cur][k][ty * 4], t4);
 #pragma unroll
             for (int i = 0; i < 4; i++) a[i] = t4[i];
-            lds4<T>(&As[cur][k][BM / 2 + ty * 4], t4);
+            lds4(&As[cur][k][BM / 2 + ty * 4], t4);
 #pragma unroll
             for (int i = 0; i < 4; i++) a[4 + i] = t4[i];
-            if (sizeof(T) == 8) {
-                // doubles: two columns per 16-byte load, column pairs 32 apart, so that the 16 lanes of a row of the
-                // thread grid read consecutive 16-byte words (four columns per thread would stride them 32 bytes
-                // apart: a 4-way bank conflict)
-#pragma unroll
-                for (int g = 0; g < TN / 2; g++) {
-                    const double2 v = *reinterpret_cast<const double2*>(&Bs[cur][k][g * 32 + tx * 2]);
-                    b[2 * g] = (T)v.x; b[2 * g + 1] = (T)v.y;
-                }
-            } else {
-                lds4<T>(&Bs[cur][k][tx * 4], t4);
+            {
+                lds4(&Bs[cur][k][tx * 4], t4);
 #pragma unroll
                 for (int j = 0; j < 4; j++) b[j] = t4[j];
                 if (TN == 8) {
-                    lds4<T>(&Bs[cur][k][BN / 2 + tx * 4], t4);
+                    lds4(&Bs[cur][k][BN / 2 + tx * 4], t4);
 #pragma unroll
                     for (int j = 0; j < 4; j++) b[(TN == 8 ? 4 : 0) + j] = t4[j];
                 }
@@ -252,7 +241,7 @@ igemm_kernel(IgemmParams p, const T* __restrict__ A, const T* __restrict__ B, T*
         const int64_t row_off = rowinfo[rl].b_off;
 #pragma unroll
         for (int j = 0; j < TN; j++) {
-            int cl = sizeof(T) == 8 ? ((j >> 1) * 32 + tx * 2 + (j & 1)) : ((j < 4) ? (tx * 4 + j) : (BN / 2 + tx * 4 + j - 4));
+            int cl = (j < 4) ? (tx * 4 + j) : (BN / 2 + tx * 4 + j - 4);
             int n = n0 + cl;
             if (n >= p.N) continue;
             if (p.splits > 1) partial[((int64_t)blockIdx.z * p.M + m) * p.N + n] = acc[i][j];
@@ -261,18 +250,257 @@ igemm_kernel(IgemmParams p, const T* __restrict__ A, const T* __restrict__ B, T*
     }
 }
 
-// Second stage of split-K: fixed-order sum over the splits, epilogue, scatter to the output.
-template <typename T, int MODE>
-__global__ void splitk_reduce_kernel(IgemmParams p, const T* __restrict__ partial, T* __restrict__ C, Epilogue<T> ep)
+// ---- float64: the same implicit GEMM on the double-precision tensor pipe ----------------------------
+// mma.m16n8k8 keeps the full FP64 rate (measured 37.0 TFLOP/s on register-resident chains, 35 with the fragment reads of
+// this kernel; the FMA pipe reaches 33) with a sixteenth of the operand reads of 8 x 8 register blocks, which is what held
+// the FMA form of this kernel to 14 TFLOP/s.  One CTA per SM = a 128 x BN tile: eight warps of 64 x 32 (BN = 128) or
+// 32 x 32 (BN = 64) only read fragments and multiply, four more gather k-slices of 16 into a ring of three stages with cp.async,
+// zero-filled where a tap or an index is out of range.  The roles are separate because a warp issues in order: with the
+// gather's address arithmetic between the products of the same warps the pipe stood idle 30 to 40 % of the time.
+// An address is the sum of a row's and a k's offset, a bound check the sum of their coordinates (DInfo), and pairs of
+// doubles go as one 16-byte copy where the channel count and the pointers allow: a slice of a 128-column tile is 16 copies
+// a thread under 4096 cycles of products.
+// Tiles in shared memory are [index][k] with rows of 20 or [k][index] with rows of 132 or 68 doubles, whichever way the
+// source is contiguous: a row pitch of 4 modulo 16 doubles makes the fragments' (8 x 4) reads conflict-free either way.
+// Consecutive warps lie along M so that a narrow N (whose unused 8-column steps are skipped) still feeds all four
+// sub-partitions.
+constexpr int DG_BK = 16, DG_STAGES = 3, DG_KP = DG_BK + 4, DG_MMA = 256, DG_GATHER = 128, DG_THREADS = DG_MMA + DG_GATHER;
+
+// A GEMM row or a k index: element (row, k) of A lies at off + off and is inside the tensor when the summed coordinates
+// are; boff is a k's offset in B or a row's in C.  With 32-bit offsets it is one 16-byte read.
+template <typename OFF> struct __align__(16) DInfo { OFF off; int d0, d1; OFF boff; };
+
+template <int BN> constexpr int dg_tile_doubles() {
+    return (128 * DG_KP > DG_BK * 132 ? 128 * DG_KP : DG_BK * 132) + (BN * DG_KP > DG_BK * (BN + 4) ? BN * DG_KP : DG_BK * (BN + 4));
+}
+template <int BN, typename OFF> constexpr size_t dg_smem_bytes() {
+    return DG_STAGES * (dg_tile_doubles<BN>() * sizeof(double) + DG_BK * sizeof(DInfo<OFF>)) + 128 * sizeof(DInfo<OFF>);
+}
+template <int N> __device__ __forceinline__ void cp_async_doubles(uint32_t d, const double* src, bool ok) {
+    if (N == 2) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(ok ? 16 : 0) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(ok ? 8 : 0) : "memory");
+}
+__device__ __forceinline__ void dmma_16x8x8(double (&c)[4], const double (&a)[4], const double (&b)[2]) {
+    asm volatile("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3]) : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
+}
+
+// A strided input gradient runs per residue class (dgrad_class_params), inside which the division by the stride is exact:
+// the row takes the quotient at the class's first tap and every further tap lowers it by lin_h.
+template <typename OFF>
+__device__ __forceinline__ DInfo<OFF> dinfo_pix(const IgemmParams& p, int mode, int idx, int limit) {
+    DInfo<OFF> f{0, -B2C_SENTINEL, 0, 0};
+    if (idx >= limit) return f;
+    const int n = idx / p.PQ, rem = idx - n * p.PQ;
+    int pp = rem / p.Q, qq = rem - pp * p.Q;
+    pp = p.pix_h0 + pp * p.pix_hs; qq = p.pix_w0 + qq * p.pix_ws;
+    if (mode == MODE_DGRAD) { f.d0 = (pp + p.vpad - p.tap_r0 * p.vdil) / p.vstr; f.d1 = (qq + p.hpad - p.tap_s0 * p.hdil) / p.hstr; }
+    else { f.d0 = pp * p.vstr - p.vpad; f.d1 = qq * p.hstr - p.hpad; }
+    f.off = (OFF)(n * p.a_sn + f.d0 * p.a_sh + f.d1 * p.a_sw);
+    f.boff = (OFF)(n * p.pb_sn + pp * p.pb_sh + qq * p.pb_sw);
+    return f;
+}
+template <typename OFF>
+__device__ __forceinline__ DInfo<OFF> dinfo_tap(const IgemmParams& p, int mode, int idx, int limit) {
+    DInfo<OFF> f{0, -B2C_SENTINEL, 0, 0};
+    if (idx >= limit) return f;
+    int c, r, s;
+    if (p.tap_c_fast) { c = idx % p.C; const int rs = idx / p.C; r = rs / p.S; s = rs - r * p.S; }
+    else { const int RS = p.R * p.S; c = idx / RS; const int rs = idx - c * RS; r = rs / p.S; s = rs - r * p.S; }
+    if (mode == MODE_DGRAD) { f.d0 = -r * p.lin_h; f.d1 = -s * p.lin_w; }
+    else { f.d0 = r * p.vdil; f.d1 = s * p.hdil; }
+    f.off = (OFF)(c * p.a_sc + f.d0 * p.a_sh + f.d1 * p.a_sw);
+    f.boff = (OFF)(c * p.tb_sc + (p.tap_r0 + r * p.tap_rs) * p.tb_sr + (p.tap_s0 + s * p.tap_ss) * p.tb_ss);
+    return f;
+}
+
+// Named barriers: DG_FULL + stage (slice landed), DG_EMPTY + stage (slice read), DG_KS (among the gathering warps).  The
+// gathering warps wait for DG_EMPTY of slice s - 3 before they refill its stage and report slice s - 1 only after that;
+// the multiplying warps need slices up to s - 3 for it, all of them reported one round before: no cycle.
+enum { DG_FULL = 1, DG_EMPTY = 4, DG_KS = 7 };
+__device__ __forceinline__ void bar_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+// what this thread wrote or read before it is done when the barrier completes
+__device__ __forceinline__ void bar_arrive(int id, int n) {
+    __threadfence_block();
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory");
+}
+
+// AK, BK_: the tile of A (B) is contiguous along k, else along its other index.  V doubles per copy.  OFF: offsets in A, B, C.
+template <int BN, bool AK, bool BK_, int V, typename OFF>
+__global__ void __launch_bounds__(DG_THREADS, 1)
+dgemm_kernel(IgemmParams p, int mode, const double* __restrict__ A, const double* __restrict__ B,
+             double* __restrict__ C, double* __restrict__ partial, Epilogue<double> ep)
 {
     pdl_prologue();
-    int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    int64_t total = (int64_t)p.M * p.N;
-    if (idx >= total) return;
-    int m = (int)(idx / p.N), n = (int)(idx - (int64_t)m * p.N);
+    constexpr int BM = 128, BK = DG_BK, KP = DG_KP, NP = DG_GATHER;
+    constexpr int A_SIZE = 128 * KP > BK * 132 ? 128 * KP : BK * 132, TILE = dg_tile_doubles<BN>();
+    constexpr int WM = BN == 128 ? 64 : 32, MI = WM / 16, WARPS_M = BM / WM;     // warp tile WM x 32
+    constexpr int A_SI = AK ? KP : 1, A_SK = AK ? 1 : 132, B_SI = BK_ ? KP : 1, B_SK = BK_ ? 1 : BN + 4;   // strides of (index, k)
+    extern __shared__ __align__(16) uint8_t dg_smem[];
+    double* tiles = reinterpret_cast<double*>(dg_smem);
+    DInfo<OFF>* kinfo = reinterpret_cast<DInfo<OFF>*>(dg_smem + DG_STAGES * TILE * sizeof(double));
+    DInfo<OFF>* rowinfo = kinfo + DG_STAGES * BK;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
+    const int kbeg = blockIdx.z * p.k_chunk, kend = min(p.K, kbeg + p.k_chunk);
+    const int nslice = (kend - kbeg + BK - 1) / BK;
+    if (tid < BM) rowinfo[tid] = mode == MODE_WGRAD ? dinfo_tap<OFF>(p, mode, m0 + tid, p.M) : dinfo_pix<OFF>(p, mode, m0 + tid, p.M);
+    __syncthreads();
+
+    if (warp >= DG_MMA / 32) {
+        // ---------------- gather ----------------
+        const int t = tid - DG_MMA;
+        const int H = p.H, W = p.W, N = p.N;
+        auto decode_k = [&](int slice, int st) {           // by threads 0 .. BK-1
+            const int k = kbeg + slice * BK + t;
+            kinfo[st * BK + t] = mode == MODE_WGRAD ? dinfo_pix<OFF>(p, mode, k, kend) : dinfo_tap<OFF>(p, mode, k, kend);
+        };
+        // copy e of a tile: V doubles from index (e % FAST) * V along memory, at index e / FAST of the other axis
+        constexpr int A_FAST = (AK ? BK : BM) / V, A_CNT = BM * BK / V / NP, B_FAST = (BK_ ? BK : BN) / V, B_CNT = BN * BK / V / NP;
+        const uint32_t tiles_s = (uint32_t)__cvta_generic_to_shared(tiles);
+        if (t < BK) decode_k(0, 0);
+        int st = 0;
+#pragma unroll 1
+        for (int s = 0; s < nslice; s++) {
+            if (s >= DG_STAGES) bar_sync(DG_EMPTY + st, DG_THREADS);
+            bar_sync(DG_KS, NP);                          // the k's of slice s are decoded
+            const DInfo<OFF>* kis = kinfo + st * BK;
+            const uint32_t as = tiles_s + st * TILE * 8, bs = as + A_SIZE * 8;
+#pragma unroll 8
+            for (int i = 0; i < A_CNT; i++) {
+                const int e = t + i * NP, f = e % A_FAST * V, x = e / A_FAST;
+                const DInfo<OFF> &u = AK ? kis[f] : rowinfo[f], &w = AK ? rowinfo[x] : kis[x];
+                const bool ok = (unsigned)(u.d0 + w.d0) < (unsigned)H && (unsigned)(u.d1 + w.d1) < (unsigned)W;
+                cp_async_doubles<V>(as + 8 * (x * (AK ? KP : 132) + f), A + (ok ? u.off + w.off : 0), ok);
+            }
+#pragma unroll 8
+            for (int i = 0; i < B_CNT; i++) {
+                const int e = t + i * NP, f = e % B_FAST * V, x = e / B_FAST, n = n0 + (BK_ ? x : f);
+                const DInfo<OFF>& ki = kis[BK_ ? f : x];
+                const bool ok = ki.d0 > -(B2C_SENTINEL >> 1) && n < N;
+                cp_async_doubles<V>(bs + 8 * (x * (BK_ ? KP : BN + 4) + f), B + (ok ? ki.boff + n * (OFF)p.b_sn : 0), ok);
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            const int nxt = st + 1 == DG_STAGES ? 0 : st + 1, prev = st == 0 ? DG_STAGES - 1 : st - 1;
+            // the k's of slice s + 1 go where those of slice s - 2 were read: every gathering thread is past them (DG_KS)
+            if (t < BK) decode_k(s + 1, nxt);
+            if (s > 0) {
+                asm volatile("cp.async.wait_group 1;" ::: "memory");
+                bar_arrive(DG_FULL + prev, DG_THREADS);
+            }
+            st = nxt;
+        }
+        if (nslice > 0) {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            bar_arrive(DG_FULL + (st == 0 ? DG_STAGES - 1 : st - 1), DG_THREADS);
+        }
+        return;
+    }
+
+    // ---------------- products ----------------
+    const int wm = (warp % WARPS_M) * WM, wn = (warp / WARPS_M) * 32;
+    const int g = lane >> 2, t = lane & 3;
+    int nj = (p.N - n0 - wn + 7) / 8;            // 8-column steps of this warp that hold columns of the output
+    nj = nj < 0 ? 0 : nj > 4 ? 4 : nj;
+    double acc[MI][4][4];
+#pragma unroll
+    for (int i = 0; i < MI; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) acc[i][j][e] = 0.0;
+    // k of a thread's two operand slots in an 8-step: t and t + 4, or with both tiles along k the pair 2t, 2t + 1 (one
+    // 16-byte read; any assignment serves as long as A and B agree)
+    constexpr bool PAIR = AK && BK_;
+    const double* a_src = tiles + (wm + g) * A_SI + (PAIR ? 2 * t : t) * A_SK;
+    const double* b_src = tiles + A_SIZE + (wn + g) * B_SI + (PAIR ? 2 * t : t) * B_SK;
+    int st = 0;
+#pragma unroll 1
+    for (int s = 0; s < nslice; s++) {
+        bar_sync(DG_FULL + st, DG_THREADS);
+        const double *as = a_src + st * TILE, *bs = b_src + st * TILE;
+        if (nj > 0) {
+#pragma unroll
+            for (int kk = 0; kk < BK; kk += 8) {
+                double a[MI][4], b[4][2];
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const double* q = bs + j * 8 * B_SI + kk * B_SK;
+                    if (PAIR) { const double2 u = *reinterpret_cast<const double2*>(q); b[j][0] = u.x; b[j][1] = u.y; }
+                    else { b[j][0] = q[0]; b[j][1] = q[4 * B_SK]; }
+                }
+#pragma unroll
+                for (int i = 0; i < MI; i++) {
+                    const double *q = as + i * 16 * A_SI + kk * A_SK, *q8 = q + 8 * A_SI;
+                    if (PAIR) {
+                        const double2 u = *reinterpret_cast<const double2*>(q), w = *reinterpret_cast<const double2*>(q8);
+                        a[i][0] = u.x; a[i][2] = u.y; a[i][1] = w.x; a[i][3] = w.y;
+                    } else { a[i][0] = q[0]; a[i][1] = q8[0]; a[i][2] = q[4 * A_SK]; a[i][3] = q8[4 * A_SK]; }
+                }
+#pragma unroll
+                for (int i = 0; i < MI; i++)
+#pragma unroll
+                    for (int j = 0; j < 4; j++)
+                        if (j < nj) dmma_16x8x8(acc[i][j], a[i], b[j]);
+            }
+        }
+        // the last DG_STAGES slices are not refilled: nobody waits for their stages
+        if (s + DG_STAGES < nslice) bar_arrive(DG_EMPTY + st, DG_THREADS);
+        st = st + 1 == DG_STAGES ? 0 : st + 1;
+    }
+
+#pragma unroll
+    for (int i = 0; i < MI; i++)
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int rl = wm + i * 16 + h * 8 + g, m = m0 + rl;
+            if (m >= p.M) continue;
+            const OFF row_off = rowinfo[rl].boff;
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+#pragma unroll
+                for (int e = 0; e < 2; e++) {
+                    const int n = n0 + wn + j * 8 + 2 * t + e;
+                    if (n >= p.N) continue;
+                    const double v = acc[i][j][2 * h + e];
+                    if (p.splits > 1) partial[((int64_t)blockIdx.z * p.M + m) * p.N + n] = v;
+                    else C[row_off + (int64_t)n * p.c_sn] = apply_epilogue<double>(v, n, ep);
+                }
+        }
+}
+
+// Second stage of split-K: fixed-order sum over the splits, epilogue, scatter to the output.  Block (32, ROWS): the thread
+// rows share the splits (row y adds splits y, y + ROWS, .. in order, then the rows are added in order).  ROWS = 8 for many
+// splits: a thread's chain of loads is one L2 round trip instead of eight (11 -> 4 us on a 144 x 16 filter cut 128 times).
+template <typename T, int MODE, int ROWS>
+__global__ void __launch_bounds__(256) splitk_reduce_kernel(IgemmParams p, const T* __restrict__ partial, T* __restrict__ C, Epilogue<T> ep)
+{
+    pdl_prologue();
+    constexpr int COLS = 256 / ROWS;
+    __shared__ T part[ROWS][COLS];
+    const int64_t idx = (int64_t)blockIdx.x * COLS + threadIdx.x, total = (int64_t)p.M * p.N;
     T v = T(0);
-    for (int z = 0; z < p.splits; z++) v += partial[(int64_t)z * total + idx];
-    Info ri = (MODE == MODE_WGRAD) ? decode_tap<MODE>(p, m, p.M) : decode_pix<MODE>(p, m, p.M);
+    if (idx < total) {
+        int z = threadIdx.y;
+        for (; z + 7 * ROWS < p.splits; z += 8 * ROWS) {          // eight independent loads
+            T q[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) q[u] = partial[(int64_t)(z + u * ROWS) * total + idx];
+#pragma unroll
+            for (int u = 0; u < 8; u++) v += q[u];
+        }
+        for (; z < p.splits; z += ROWS) v += partial[(int64_t)z * total + idx];
+    }
+    if (ROWS > 1) {
+        part[threadIdx.y][threadIdx.x] = v;
+        __syncthreads();
+        if (threadIdx.y != 0) return;
+#pragma unroll
+        for (int y = 1; y < ROWS; y++) v += part[y][threadIdx.x];
+    }
+    if (idx >= total) return;
+    const int m = (int)(idx / p.N), n = (int)(idx - (int64_t)m * p.N);
+    const Info ri = (MODE == MODE_WGRAD) ? decode_tap<MODE>(p, m, p.M) : decode_pix<MODE>(p, m, p.M);
     C[ri.b_off + (int64_t)n * p.c_sn] = apply_epilogue<T>(v, n, ep);
 }
 
@@ -298,28 +526,19 @@ __global__ void index_map_kernel(IgemmParams p, int64_t* __restrict__ map, int n
 // row-major weight matrix (pydtnn/backends/cpu/layers/fc_cpu.py:66-71).  The sum is over the batch only (32-64
 // terms), so the pass is bound by writing dw; the general kernel above spends its time on gather arithmetic that a
 // dense matrix does not need.  One CTA = one 128 x 128 tile of dw, all of the batch, 8 x 8 outputs per thread.
-template <typename T> __device__ __forceinline__ void ldg4(const T* p, T (&o)[4]);
-template <> __device__ __forceinline__ void ldg4<float>(const float* p, float (&o)[4]) {
+__device__ __forceinline__ void ldg4(const float* p, float (&o)[4]) {
     float4 v = __ldg(reinterpret_cast<const float4*>(p)); o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
 }
-template <> __device__ __forceinline__ void ldg4<double>(const double* p, double (&o)[4]) {
-    double2 a = __ldg(reinterpret_cast<const double2*>(p)), b = __ldg(reinterpret_cast<const double2*>(p) + 1);
-    o[0] = a.x; o[1] = a.y; o[2] = b.x; o[3] = b.y;
-}
-template <typename T> __device__ __forceinline__ void sts4(T* p, const T (&v)[4]);
-template <> __device__ __forceinline__ void sts4<float>(float* p, const float (&v)[4]) {
+__device__ __forceinline__ void sts4(float* p, const float (&v)[4]) {
     *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
 }
-template <> __device__ __forceinline__ void sts4<double>(double* p, const double (&v)[4]) {
-    *reinterpret_cast<double2*>(p) = make_double2(v[0], v[1]); *reinterpret_cast<double2*>(p + 2) = make_double2(v[2], v[3]);
-}
 
-template <typename T>
 __global__ void __launch_bounds__(256)
-fc_wgrad_kernel(const T* __restrict__ x, const T* __restrict__ dy, T* __restrict__ dw, int batch, int in_f, int out_f)
+fc_wgrad_kernel(const float* __restrict__ x, const float* __restrict__ dy, float* __restrict__ dw, int batch, int in_f, int out_f)
 {
+    using T = float;
     pdl_prologue();
-    constexpr int BT = 128, KC = TileCfg<T>::BK, PER = KC * BT / 4 / 256;     // 4-element vectors per thread per tile
+    constexpr int BT = 128, KC = FMA_BK, PER = KC * BT / 4 / 256;     // 4-element vectors per thread per tile
     __shared__ __align__(16) T xs[2][KC][BT];
     __shared__ __align__(16) T ds[2][KC][BT];
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
@@ -330,9 +549,9 @@ fc_wgrad_kernel(const T* __restrict__ x, const T* __restrict__ dy, T* __restrict
         for (int j = 0; j < PER; j++) {
             const int v = tid + j * 256, k = v / (BT / 4), col = (v % (BT / 4)) * 4;
             const bool row_ok = b0 + k < batch;
-            if (row_ok && i0 + col < in_f) ldg4<T>(x + (int64_t)(b0 + k) * in_f + i0 + col, rx[j]);
+            if (row_ok && i0 + col < in_f) ldg4(x + (int64_t)(b0 + k) * in_f + i0 + col, rx[j]);
             else { rx[j][0] = rx[j][1] = rx[j][2] = rx[j][3] = T(0); }
-            if (row_ok && o0 + col < out_f) ldg4<T>(dy + (int64_t)(b0 + k) * out_f + o0 + col, rd[j]);
+            if (row_ok && o0 + col < out_f) ldg4(dy + (int64_t)(b0 + k) * out_f + o0 + col, rd[j]);
             else { rd[j][0] = rd[j][1] = rd[j][2] = rd[j][3] = T(0); }
         }
     };
@@ -340,8 +559,8 @@ fc_wgrad_kernel(const T* __restrict__ x, const T* __restrict__ dy, T* __restrict
 #pragma unroll
         for (int j = 0; j < PER; j++) {
             const int v = tid + j * 256, k = v / (BT / 4), col = (v % (BT / 4)) * 4;
-            sts4<T>(&xs[buf][k][col], rx[j]);
-            sts4<T>(&ds[buf][k][col], rd[j]);
+            sts4(&xs[buf][k][col], rx[j]);
+            sts4(&ds[buf][k][col], rd[j]);
         }
     };
     T acc[8][8];
@@ -359,16 +578,16 @@ fc_wgrad_kernel(const T* __restrict__ x, const T* __restrict__ dy, T* __restrict
 #pragma unroll
         for (int k = 0; k < KC; k++) {
             T a[8], b[8], t4[4];
-            lds4<T>(&xs[cur][k][ty * 4], t4);
+            lds4(&xs[cur][k][ty * 4], t4);
 #pragma unroll
             for (int i = 0; i < 4; i++) a[i] = t4[i];
-            lds4<T>(&xs[cur][k][BT / 2 + ty * 4], t4);
+            lds4(&xs[cur][k][BT / 2 + ty * 4], t4);
 #pragma unroll
             for (int i = 0; i < 4; i++) a[4 + i] = t4[i];
-            lds4<T>(&ds[cur][k][tx * 4], t4);
+            lds4(&ds[cur][k][tx * 4], t4);
 #pragma unroll
             for (int j = 0; j < 4; j++) b[j] = t4[j];
-            lds4<T>(&ds[cur][k][BT / 2 + tx * 4], t4);
+            lds4(&ds[cur][k][BT / 2 + tx * 4], t4);
 #pragma unroll
             for (int j = 0; j < 4; j++) b[4 + j] = t4[j];
 #pragma unroll
@@ -388,7 +607,7 @@ fc_wgrad_kernel(const T* __restrict__ x, const T* __restrict__ dy, T* __restrict
             const int col = o0 + h * (BT / 2) + tx * 4;
             if (col >= out_f) continue;
             const T v[4] = {acc[i][4 * h], acc[i][4 * h + 1], acc[i][4 * h + 2], acc[i][4 * h + 3]};
-            sts4<T>(dw + (int64_t)row * out_f + col, v);
+            sts4(dw + (int64_t)row * out_f + col, v);
         }
     }
 }
@@ -396,7 +615,7 @@ fc_wgrad_kernel(const T* __restrict__ x, const T* __restrict__ dy, T* __restrict
 static bool is_dense_fc(const Geo& g)
 {
     return g.layout == B2C_LAYOUT_NHWC && g.w_layout == B2C_W_CRSK && g.h == 1 && g.w == 1 && g.kh == 1 && g.kw == 1 &&
-           g.vpad == 0 && g.hpad == 0 && g.ci % 4 == 0 && g.co % 4 == 0;
+           g.vpad == 0 && g.hpad == 0 && g.ci % 4 == 0 && g.co % 4 == 0 && g.dtype == B2C_F32;
 }
 
 // ---- host side ----------------------------------------------------------------------------
@@ -412,7 +631,7 @@ static IgemmParams make_params(const Geo& g, int mode)
     p.vstr = g.vstr; p.hstr = g.hstr; p.vpad = g.vpad; p.hpad = g.hpad; p.vdil = g.vdil; p.hdil = g.hdil;
     p.relu = 0; p.splits = 1;
     p.pix_h0 = 0; p.pix_hs = 1; p.pix_w0 = 0; p.pix_ws = 1;
-    p.tap_r0 = 0; p.tap_rs = 1; p.tap_s0 = 0; p.tap_ss = 1;
+    p.tap_r0 = 0; p.tap_rs = 1; p.tap_s0 = 0; p.tap_ss = 1; p.lin_h = g.vdil; p.lin_w = g.hdil;
     if (mode == MODE_FPROP) {
         p.M = (int)g.M; p.N = g.co; p.K = (int)g.K;
         p.P = g.ho; p.Q = g.wo; p.C = g.ci; p.H = g.h; p.W = g.w;
@@ -440,6 +659,10 @@ static IgemmParams make_params(const Geo& g, int mode)
         p.b_lanes_k = !nhwc;
     }
     p.PQ = p.P * p.Q;
+    // a row's offset alone may lie a window outside the tensor
+    const int64_t over_h = (int64_t)g.kh * g.vdil + g.vpad, over_w = (int64_t)g.kw * g.hdil + g.hpad;
+    p.small = (int64_t)g.n * (g.h + 2 * over_h) * (g.w + 2 * over_w) * g.ci < (1LL << 31) && (int64_t)g.n * (g.ho + 2 * over_h) * (g.wo + 2 * over_w) * g.co < (1LL << 31) &&
+              g.K * g.co < (1LL << 31);
     return p;
 }
 
@@ -458,21 +681,47 @@ static int choose_splits(const IgemmParams& p, int bk)
     return (int)s;
 }
 
+// The float64 tensor kernel holds one CTA per SM: the split count that needs the fewest rounds of the chip x (slices of a
+// split + about six for its start, its drain and its share of the second stage).
+static int choose_splits_f64(const IgemmParams& p, int bk)
+{
+    const int64_t ctas = (int64_t)((p.M + 127) / 128) * ((p.N + tile_bn(p.N) - 1) / tile_bn(p.N));
+    const int64_t room = 148, slices = (p.K + bk - 1) / bk;
+    int64_t best = 1, cost = 0;
+    for (int64_t s = 1; s <= 128 && s <= slices && (s == 1 || ctas * s <= 2 * room); s++) {
+        const int64_t c = (ctas * s + room - 1) / room * ((slices + s - 1) / s + (s > 1 ? 6 : 3));
+        if (s == 1 || c < cost) { best = s; cost = c; }
+    }
+    return (int)best;
+}
+
 static void finish_params(IgemmParams& p, int dtype)
 {
-    int bk = dtype == B2C_F32 ? 16 : 8;
+    const int bk = 16;
+    static_assert(FMA_BK == 16 && DG_BK == 16, "k-chunks are whole slices of either kernel");
     if (p.K <= 0) { p.splits = 1; p.k_chunk = bk; return; }        // no taps reach these pixels: the launch writes zeros
-    p.splits = choose_splits(p, bk);
+    p.splits = dtype == B2C_F32 ? choose_splits(p, bk) : choose_splits_f64(p, bk);
     int chunk = (p.K + p.splits - 1) / p.splits;
     chunk = (chunk + bk - 1) / bk * bk;
     p.k_chunk = chunk;
     p.splits = (p.K + chunk - 1) / chunk;
 }
 
-// Strided dgrad, dilation 1: input pixel (h, w) only receives taps with r = (h + vpad) mod vstr, s = (w + hpad) mod hstr
-// (mod the strides).  Class (a, b) of those residues is a dense problem over its own pixels and taps; gathering all
-// taps for all pixels instead would spend (vstr*hstr - 1) / (vstr*hstr) of the inner loop on zeros.
-static bool dgrad_by_class(const Geo& g) { return (g.vstr > 1 || g.hstr > 1) && g.vdil == 1 && g.hdil == 1; }
+// Strided dgrad: input pixel (h, w) only receives taps with r * vdil = h + vpad, s * hdil = w + hpad (mod the strides).
+// Class (a, b) of those residues is a dense problem over its own pixels and taps; gathering all taps for all pixels instead
+// would spend (vstr*hstr - 1) / (vstr*hstr) of the inner loop on zeros.
+static bool dgrad_by_class(const Geo& g) { return g.vstr > 1 || g.hstr > 1; }
+
+// The taps r < k with r * dil = a (mod str): first, step and count; one step moves the gathered position by lin.
+static void class_taps(int a, int str, int dil, int k, int& first, int& step, int& count, int& lin)
+{
+    int x = dil, y = str;
+    while (y) { const int t = x % y; x = y; y = t; }
+    step = str / x; lin = dil / x;
+    first = 0; count = 0;
+    for (int r = 0; r < k && r < str; r++)
+        if ((int64_t)r * dil % str == a) { first = r; count = (k - r + step - 1) / step; break; }
+}
 
 static IgemmParams dgrad_class_params(const Geo& g, int a, int b)
 {
@@ -483,9 +732,8 @@ static IgemmParams dgrad_class_params(const Geo& g, int a, int b)
     p.Q = w0 < g.w ? (g.w - w0 + g.hstr - 1) / g.hstr : 0;
     p.PQ = p.P * p.Q;
     p.M = g.n * p.PQ;
-    p.tap_r0 = a; p.tap_rs = g.vstr; p.tap_s0 = b; p.tap_ss = g.hstr;
-    p.R = a < g.kh ? (g.kh - a + g.vstr - 1) / g.vstr : 0;
-    p.S = b < g.kw ? (g.kw - b + g.hstr - 1) / g.hstr : 0;
+    class_taps(a, g.vstr, g.vdil, g.kh, p.tap_r0, p.tap_rs, p.R, p.lin_h);
+    class_taps(b, g.hstr, g.hdil, g.kw, p.tap_s0, p.tap_ss, p.S, p.lin_w);
     p.K = g.co * p.R * p.S;
     return p;
 }
@@ -512,6 +760,42 @@ size_t fma_workspace_bytes(const Geo& g, int pass)
     return bytes;
 }
 
+template <int BN, bool AK, bool BK_, int V, typename OFF>
+static int launch_dgemm_v(const IgemmParams& p, int mode, dim3 grid, const double* A, const double* B, double* C, double* ws, const Epilogue<double>& ep, cudaStream_t st)
+{
+    // once per device: the attribute belongs to the device's copy of the kernel
+    static std::atomic<uint64_t> done{0};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev > 63) dev = 63;
+    if (dev == 63 || !(done.load() >> dev & 1)) {
+        const cudaError_t e = cudaFuncSetAttribute(dgemm_kernel<BN, AK, BK_, V, OFF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dg_smem_bytes<BN, OFF>());
+        if (e != cudaSuccess) { set_cuda_error(e, "cudaFuncSetAttribute(dgemm_kernel)"); return B2C_ERR_CUDA; }
+        done.fetch_or(1ull << dev);
+    }
+    launch_pdl(dgemm_kernel<BN, AK, BK_, V, OFF>, grid, DG_THREADS, dg_smem_bytes<BN, OFF>(), st, p, mode, A, B, C, ws, ep);
+    return B2C_OK;          // the caller checks the launch
+}
+
+template <int BN>
+static int launch_dgemm(const IgemmParams& p, int mode, dim3 grid, const double* A, const double* B, double* C, double* ws, const Epilogue<double>& ep, cudaStream_t st)
+{
+    // Pairs of doubles per copy: the index that runs along memory must step by one element, keep a pair inside one tap and
+    // one bound (an even channel count), and every other stride and the pointer must be even.
+    const bool a_pair = p.a_sc == 1 && p.tap_c_fast && p.C % 2 == 0 && ((p.a_sn | p.a_sh | p.a_sw) & 1) == 0 && ((uintptr_t)A & 15) == 0;
+    // B(k, n): along k it is a filter's channel axis, along n the output channels of a filter or of dy
+    bool b_pair = ((uintptr_t)B & 15) == 0;
+    if (p.b_lanes_k) b_pair = b_pair && mode != MODE_WGRAD && p.tap_c_fast && p.tb_sc == 1 && p.C % 2 == 0 && ((p.tb_sr | p.tb_ss | p.b_sn) & 1) == 0;
+    else b_pair = b_pair && p.b_sn == 1 && p.N % 2 == 0 &&
+                  ((mode == MODE_WGRAD ? (p.pb_sn | p.pb_sh | p.pb_sw) : (p.tb_sc | p.tb_sr | p.tb_ss)) & 1) == 0;
+    const bool pairs = a_pair && b_pair && p.small;         // small: every offset fits 31 bits
+#define B2C_DG(AK, BK_) (pairs ? launch_dgemm_v<BN, AK, BK_, 2, int>(p, mode, grid, A, B, C, ws, ep, st) : launch_dgemm_v<BN, AK, BK_, 1, int64_t>(p, mode, grid, A, B, C, ws, ep, st))
+    if (p.a_lanes_k && p.b_lanes_k) return B2C_DG(true, true);
+    if (p.a_lanes_k) return B2C_DG(true, false);
+    if (!p.b_lanes_k) return B2C_DG(false, false);
+#undef B2C_DG
+    return launch_dgemm_v<BN, false, true, 1, int64_t>(p, mode, grid, A, B, C, ws, ep, st);
+}
+
 template <typename T, int MODE>
 static int launch_igemm(IgemmParams& p, const void* A, const void* B, void* C, void* ws, size_t ws_bytes,
                         Epilogue<T> ep, cudaStream_t st)
@@ -522,15 +806,20 @@ static int launch_igemm(IgemmParams& p, const void* A, const void* B, void* C, v
     const int bn = tile_bn(p.N);
     dim3 grid((p.M + 127) / 128, (p.N + bn - 1) / bn, p.splits);
     if (grid.y > 65535 || grid.z > 65535) return B2C_ERR_TOO_LARGE;
-    if (bn == 64)
-        launch_pdl(igemm_kernel<T, MODE, 64, 4>, grid, 256, 0, st, p, (const T*)A, (const T*)B, (T*)C, (T*)ws, ep);
+    if constexpr (sizeof(T) == 8) {
+        const int rc = bn == 64 ? launch_dgemm<64>(p, MODE, grid, (const double*)A, (const double*)B, (double*)C, (double*)ws, ep, st)
+                                : launch_dgemm<128>(p, MODE, grid, (const double*)A, (const double*)B, (double*)C, (double*)ws, ep, st);
+        if (rc) return rc;
+    } else if (bn == 64)
+        launch_pdl(igemm_kernel<MODE, 64, 4>, grid, 256, 0, st, p, (const float*)A, (const float*)B, (float*)C, (float*)ws, ep);
     else
-        launch_pdl(igemm_kernel<T, MODE, 128, 8>, grid, 256, 0, st, p, (const T*)A, (const T*)B, (T*)C, (T*)ws, ep);
+        launch_pdl(igemm_kernel<MODE, 128, 8>, grid, 256, 0, st, p, (const float*)A, (const float*)B, (float*)C, (float*)ws, ep);
     int rc = check_launch("igemm_kernel");
     if (rc) return rc;
     if (p.splits > 1) {
         int64_t total = (int64_t)p.M * p.N;
-        launch_pdl(splitk_reduce_kernel<T, MODE>, (unsigned)((total + 255) / 256), 256, 0, st, p, (const T*)ws, (T*)C, ep);
+        if (p.splits >= 16) launch_pdl(splitk_reduce_kernel<T, MODE, 8>, (unsigned)((total + 31) / 32), dim3(32, 8), 0, st, p, (const T*)ws, (T*)C, ep);
+        else launch_pdl(splitk_reduce_kernel<T, MODE, 1>, (unsigned)((total + 255) / 256), dim3(256, 1), 0, st, p, (const T*)ws, (T*)C, ep);
         rc = check_launch("splitk_reduce_kernel");
     }
     return rc;
@@ -576,12 +865,10 @@ int fma_dgrad(const Geo& g, const void* dy, const void* w, void* dx, void* ws, s
 int fma_wgrad(const Geo& g, const void* x, const void* dy, void* dw, void* db, void* ws, size_t ws_bytes,
               cudaStream_t st)
 {
-    const size_t align = g.dtype == B2C_F32 ? 15 : 31;
-    if (is_dense_fc(g) && !(((uintptr_t)x | (uintptr_t)dy | (uintptr_t)dw) & align)) {
+    if (is_dense_fc(g) && !(((uintptr_t)x | (uintptr_t)dy | (uintptr_t)dw) & 15)) {
         dim3 grid((g.co + 127) / 128, (g.ci + 127) / 128);
         if (grid.y > 65535) return B2C_ERR_TOO_LARGE;
-        if (g.dtype == B2C_F32) launch_pdl(fc_wgrad_kernel<float>, grid, 256, 0, st, (const float*)x, (const float*)dy, (float*)dw, g.n, g.ci, g.co);
-        else launch_pdl(fc_wgrad_kernel<double>, grid, 256, 0, st, (const double*)x, (const double*)dy, (double*)dw, g.n, g.ci, g.co);
+        launch_pdl(fc_wgrad_kernel, grid, 256, 0, st, (const float*)x, (const float*)dy, (float*)dw, g.n, g.ci, g.co);
         int rc = check_launch("fc_wgrad_kernel");
         if (rc || !db) return rc;
         size_t cs = channel_sum_workspace_bytes(g.n, g.co, 1);
@@ -658,15 +945,16 @@ __global__ void channel_sum_nchw_kernel(const T* __restrict__ src, double* __res
     if (threadIdx.x == 0) partial[(int64_t)blockIdx.y * c + ch] = sm[0];
 }
 
+// A warp per channel: every lane adds its chunks (32 apart) in index order, a shuffle tree adds the lanes.
 template <typename T>
-__global__ void channel_sum_final_kernel(const double* __restrict__ partial, T* __restrict__ dst, int c, int chunks)
+__global__ void __launch_bounds__(256) channel_sum_final_kernel(const double* __restrict__ partial, T* __restrict__ dst, int c, int chunks)
 {
     pdl_prologue();
-    int ch = blockIdx.x * blockDim.x + threadIdx.x;
-    if (ch >= c) return;
+    const int ch = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     double s = 0.0;
-    for (int i = 0; i < chunks; i++) s += partial[(int64_t)i * c + ch];
-    dst[ch] = (T)s;
+    if (ch < c) for (int i = lane; i < chunks; i += 32) s += partial[(int64_t)i * c + ch];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (ch < c && lane == 0) dst[ch] = (T)s;
 }
 
 // Enough for the float4 fast path to spread over about four CTAs per SM: two doubles per channel and chunk.
@@ -704,8 +992,8 @@ int channel_sum(int dtype, int layout, int n, int c, int hw, const void* src, vo
     }
     int rc = check_launch("channel_sum");
     if (rc) return rc;
-    if (dtype == B2C_F32) launch_pdl(channel_sum_final_kernel<float>, (c + 255) / 256, 256, 0, st, partial, (float*)dst, c, chunks);
-    else launch_pdl(channel_sum_final_kernel<double>, (c + 255) / 256, 256, 0, st, partial, (double*)dst, c, chunks);
+    if (dtype == B2C_F32) launch_pdl(channel_sum_final_kernel<float>, (c + 7) / 8, 256, 0, st, partial, (float*)dst, c, chunks);
+    else launch_pdl(channel_sum_final_kernel<double>, (c + 7) / 8, 256, 0, st, partial, (double*)dst, c, chunks);
     return check_launch("channel_sum_final");
 }
 

@@ -1,0 +1,54 @@
+"""The generic engine at the edges of its tiles: rows, columns and k-slices that end inside a tile, split sums, every layout,
+strided and dilated classes, fully connected layers and unaligned (8-byte) pointers, against the CPU oracle. GPU."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import conv_oracle as co
+from pydtnn_b200 import _lib
+from tests.gpu_util import DEV, assert_parity, run_conv, stream
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [(1, 3, 3, 1, 1, 1, 0, 1), (2, 9, 7, 3, 5, 3, 1, 1), (1, 16, 8, 16, 64, 1, 0, 1), (2, 13, 11, 15, 65, 3, 1, 2),
+          (1, 12, 12, 17, 130, 5, 2, 1), (3, 6, 6, 128, 24, 3, 1, 1), (2, 14, 14, 33, 129, 1, 0, 2), (4, 5, 5, 96, 9, 3, 0, 1)]
+# strides with dilations that share and do not share a factor with them, and taps that reach only some residues
+GEOMS = [co.Geom(n, h, w, ci, cout, k, k, pad, pad, st, st) for n, h, w, ci, cout, k, pad, st in SHAPES] + [
+    co.Geom(2, 13, 12, 4, 6, 3, 3, 2, 1, 2, 3, 2, 1), co.Geom(1, 17, 16, 6, 4, 3, 4, 1, 2, 4, 2, 2, 3), co.Geom(1, 11, 9, 5, 8, 2, 2, 0, 0, 3, 3, 1, 2)]
+
+
+@pytest.mark.parametrize("layout,w_layout", [("NHWC", "KRSC"), ("NHWC", "CRSK"), ("NCHW", "KCRS")])
+@pytest.mark.parametrize("dtype", ["float64", "float32"])
+@pytest.mark.parametrize("g", GEOMS, ids=lambda g: "x".join(map(str, (g.n, g.h, g.w, g.ci, g.co, g.kh, g.vstr, g.vdil))))
+def test_generic_engine(g, layout, w_layout, dtype):
+    n, h, w, ci, cout, k = g.n, g.h, g.w, g.ci, g.co, g.kh
+    rng = np.random.Generator(np.random.PCG64(ci + 7 * cout))
+    nchw = layout == "NCHW"
+    x = rng.standard_normal((n, ci, h, w) if nchw else (n, h, w, ci))
+    wt = rng.standard_normal((cout, ci, k, g.kw) if nchw else (ci, k, g.kw, cout)) * np.sqrt(2.0 / (ci * k * k))
+    b = rng.standard_normal(cout)
+    dy = rng.standard_normal((n, cout, g.ho, g.wo) if nchw else (n, g.ho, g.wo, cout))
+    y = co.conv2d_forward(x, wt, b, g, layout)
+    dw, db, dx = co.conv2d_backward(x, dy, wt, g, layout)
+    out = run_conv(g, layout, np.dtype(dtype), x, wt, b, dy, w_layout=w_layout, engine=_lib.ENGINE_FMA)
+    for name, ref in (("y", y), ("dw", dw), ("db", db), ("dx", dx)):
+        assert_parity(out[name].reshape(ref.shape), ref, dtype, f"{name} {layout} {w_layout}")
+
+
+@pytest.mark.parametrize("n,i,o", [(1, 64, 10), (3, 129, 65), (200, 300, 257)])
+def test_float64_fc_on_8_byte_pointers(n, i, o):
+    L = _lib.lib()
+
+    def odd(*shape):                              # a tensor that starts 8 bytes past a 16-byte boundary
+        count = int(np.prod(shape))
+        return torch.randn(count + 1, dtype=torch.float64, device=DEV)[1:].view(*shape)
+    x, w, b, dy = odd(n, i), odd(i, o), odd(o), odd(n, o)
+    y, dw, db, dx = odd(n, o), odd(i, o), odd(o), odd(n, i)
+    ws = torch.empty(max(256, L.b2c_fc_workspace_bytes(_lib.F64, n, i, o, 0)), dtype=torch.uint8, device=DEV)
+    a = (_lib.F64, 0, n, i, o)
+    _lib.check(L.b2c_fc_forward(*a, x.data_ptr(), w.data_ptr(), b.data_ptr(), y.data_ptr(), ws.data_ptr(), ws.numel(), stream()))
+    _lib.check(L.b2c_fc_backward(*a, x.data_ptr(), dy.data_ptr(), w.data_ptr(), dw.data_ptr(), db.data_ptr(), dx.data_ptr(), ws.data_ptr(),
+                                 ws.numel(), stream()))
+    xs, wn, bn, dn = (t.cpu().numpy() for t in (x, w, b, dy))
+    for got, ref in ((y, xs @ wn + bn), (dw, xs.T @ dn), (db, dn.sum(0)), (dx, dn @ wn.T)):
+        assert_parity(got.cpu().numpy(), ref, np.float64)
