@@ -11,11 +11,10 @@ void set_cuda_error(cudaError_t e, const char* where) {
 }
 
 // Shapes the tensor-core kernels accept but the FMA engine runs faster (measured on fully connected layers at
-// batch 32-64): a weight gradient summed over a handful of pixels is an outer product bound by writing dw, which the
-// FMA engine's dense kernel does at HBM speed.
+// batch 32-64): a weight gradient summed over a handful of pixels whose tiles cannot go straight to dw.
 static bool fma_is_faster(const Geo& g, int pass) {
     const bool one_pixel_images = g.h == 1 && g.w == 1 && g.kh == 1 && g.kw == 1 && g.vpad == 0 && g.hpad == 0;
-    return one_pixel_images && g.n <= 128 && pass == B2C_PASS_WGRAD;
+    return one_pixel_images && g.n <= 128 && pass == B2C_PASS_WGRAD && (g.w_layout != B2C_W_CRSK || g.co % 4);
 }
 
 // FMA for everything unless the tensor-core engine takes the shape (AUTO) or is forced.
@@ -195,6 +194,7 @@ extern "C" int b2c_fc_forward(int dtype, int engine, int batch, int in_f, int ou
                               const void* bias, void* y, void* ws, size_t ws_bytes, void* stream) {
     Geo g; int rc = fc_geo(dtype, engine, batch, in_f, out_f, g); if (rc) return rc;
     if (!x || !w || !y) return B2C_ERR_NULL_POINTER;
+    if (engine == B2C_ENGINE_AUTO && fc_tiny(batch, in_f, out_f)) return fc_tiny_forward(dtype, batch, in_f, out_f, x, w, bias, y, (cudaStream_t)stream);
     if (tc_fc_small_batch(dtype, engine, batch, in_f, out_f))
         return tc_fc_forward_small_batch(batch, in_f, out_f, x, w, bias, y, ws, ws_bytes, (cudaStream_t)stream);
     int e; rc = call_engine(g, B2C_PASS_FPROP, x, y, e); if (rc) return rc;
@@ -207,6 +207,10 @@ extern "C" int b2c_fc_backward(int dtype, int engine, int batch, int in_f, int o
     Geo g; int rc = fc_geo(dtype, engine, batch, in_f, out_f, g); if (rc) return rc;
     if (!dy) return B2C_ERR_NULL_POINTER;
     cudaStream_t st = (cudaStream_t)stream;
+    if (engine == B2C_ENGINE_AUTO && fc_tiny(batch, in_f, out_f) && (dw || !db)) {
+        if ((dw && !x) || (dx && !w)) return B2C_ERR_NULL_POINTER;
+        return fc_tiny_backward(dtype, batch, in_f, out_f, x, dy, w, dw, db, dx, st);
+    }
     if (tc_fc_small_batch(dtype, engine, batch, in_f, out_f)) {
         if (dw) {
             if (!x) return B2C_ERR_NULL_POINTER;

@@ -612,6 +612,100 @@ fc_wgrad_kernel(const float* __restrict__ x, const float* __restrict__ dy, float
     }
 }
 
+// ---- fully connected layers with a small weight matrix ------------------------------------------------
+// The last layer of a small classifier (128 x 10 and the like): a GEMM kernel's start-up, its second stage and the separate
+// bias sum are all there is to such a layer, so each direction is one launch of plain dot products whose operands stay in L1.
+// Weights up to 16 K elements; with more, re-reading them per batch row costs more than the launches saved.
+bool fc_tiny(int batch, int in_f, int out_f) { return batch <= 512 && (int64_t)in_f * out_f <= (1 << 14); }
+
+// y[b][o]: block = 32 outputs x 8 parts of the sum over the inputs, one batch row.
+template <typename T>
+__global__ void __launch_bounds__(256) fc_tiny_forward_kernel(const T* __restrict__ x, const T* __restrict__ w, const T* __restrict__ bias,
+                                                              T* __restrict__ y, int in_f, int out_f)
+{
+    pdl_prologue();
+    __shared__ T part[8][33];
+    const int o = blockIdx.x * 32 + threadIdx.x;
+    const T* xr = x + (int64_t)blockIdx.y * in_f;
+    T v = T(0);
+    if (o < out_f) {
+#pragma unroll 8
+        for (int i = threadIdx.y; i < in_f; i += 8) v = fma(__ldg(xr + i), __ldg(w + (int64_t)i * out_f + o), v);
+    }
+    part[threadIdx.y][threadIdx.x] = v;
+    __syncthreads();
+    if (threadIdx.y != 0 || o >= out_f) return;
+#pragma unroll
+    for (int k = 1; k < 8; k++) v += part[k][threadIdx.x];
+    y[(int64_t)blockIdx.y * out_f + o] = bias ? v + bias[o] : v;
+}
+
+// The first dw_blocks blocks: dw[i][o] and db[o] (the row i = in_f), 32 outputs x 8 parts of the sum over the batch; the
+// rest: dx[b][i], a thread each.
+template <typename T>
+__global__ void __launch_bounds__(256) fc_tiny_backward_kernel(const T* __restrict__ x, const T* __restrict__ dy, const T* __restrict__ w,
+                                                               T* __restrict__ dw, T* __restrict__ db, T* __restrict__ dx, int batch, int in_f, int out_f,
+                                                               int dw_blocks)
+{
+    pdl_prologue();
+    __shared__ T part[8][33];
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    if ((int)blockIdx.x < dw_blocks) {
+        const int nt = (out_f + 31) / 32, i = blockIdx.x / nt, o = (blockIdx.x - i * nt) * 32 + tx;
+        T v = T(0);
+        if (o < out_f) {
+            if (i < in_f) {
+#pragma unroll 8
+                for (int b = ty; b < batch; b += 8) v = fma(__ldg(x + (int64_t)b * in_f + i), __ldg(dy + (int64_t)b * out_f + o), v);
+            } else {
+#pragma unroll 8
+                for (int b = ty; b < batch; b += 8) v += __ldg(dy + (int64_t)b * out_f + o);
+            }
+        }
+        part[ty][tx] = v;
+        __syncthreads();
+        if (ty != 0 || o >= out_f) return;
+#pragma unroll
+        for (int k = 1; k < 8; k++) v += part[k][tx];
+        if (i < in_f) { if (dw) dw[(int64_t)i * out_f + o] = v; }
+        else if (db) db[o] = v;
+        return;
+    }
+    const int64_t e = (int64_t)(blockIdx.x - dw_blocks) * 256 + threadIdx.x;
+    if (e >= (int64_t)batch * in_f) return;
+    const int b = (int)(e / in_f), i = (int)(e - (int64_t)b * in_f);
+    const T *d = dy + (int64_t)b * out_f, *wr = w + (int64_t)i * out_f;
+    T v = T(0);
+#pragma unroll 8
+    for (int o = 0; o < out_f; o++) v = fma(__ldg(d + o), __ldg(wr + o), v);
+    dx[e] = v;
+}
+
+template <typename T>
+static int fc_tiny_forward_t(int batch, int in_f, int out_f, const void* x, const void* w, const void* bias, void* y, cudaStream_t st)
+{
+    launch_pdl(fc_tiny_forward_kernel<T>, dim3((out_f + 31) / 32, batch), dim3(32, 8), 0, st, (const T*)x, (const T*)w, (const T*)bias, (T*)y, in_f, out_f);
+    return check_launch("fc_tiny_forward_kernel");
+}
+int fc_tiny_forward(int dtype, int batch, int in_f, int out_f, const void* x, const void* w, const void* bias, void* y, cudaStream_t st)
+{
+    return dtype == B2C_F32 ? fc_tiny_forward_t<float>(batch, in_f, out_f, x, w, bias, y, st) : fc_tiny_forward_t<double>(batch, in_f, out_f, x, w, bias, y, st);
+}
+template <typename T>
+static int fc_tiny_backward_t(int batch, int in_f, int out_f, const void* x, const void* dy, const void* w, void* dw, void* db, void* dx, cudaStream_t st)
+{
+    const int dw_blocks = dw ? (in_f + (db ? 1 : 0)) * ((out_f + 31) / 32) : 0;
+    const int dx_blocks = dx ? (int)(((int64_t)batch * in_f + 255) / 256) : 0;
+    if (dw_blocks + dx_blocks == 0) return B2C_OK;
+    launch_pdl(fc_tiny_backward_kernel<T>, dw_blocks + dx_blocks, 256, 0, st, (const T*)x, (const T*)dy, (const T*)w, (T*)dw, (T*)db, (T*)dx, batch, in_f, out_f, dw_blocks);
+    return check_launch("fc_tiny_backward_kernel");
+}
+int fc_tiny_backward(int dtype, int batch, int in_f, int out_f, const void* x, const void* dy, const void* w, void* dw, void* db, void* dx, cudaStream_t st)
+{
+    return dtype == B2C_F32 ? fc_tiny_backward_t<float>(batch, in_f, out_f, x, dy, w, dw, db, dx, st)
+                            : fc_tiny_backward_t<double>(batch, in_f, out_f, x, dy, w, dw, db, dx, st);
+}
+
 static bool is_dense_fc(const Geo& g)
 {
     return g.layout == B2C_LAYOUT_NHWC && g.w_layout == B2C_W_CRSK && g.h == 1 && g.w == 1 && g.kh == 1 && g.kw == 1 &&
@@ -957,6 +1051,41 @@ __global__ void __launch_bounds__(256) channel_sum_final_kernel(const double* __
     if (ch < c && lane == 0) dst[ch] = (T)s;
 }
 
+// Few rows (a fully connected layer's batch): one launch, block (32 channels, 32 row lanes), a thread adds its rows 32 apart in
+// order, the lanes are added in order.  Rows `pitch` elements apart.
+constexpr int CS_FEW_ROWS = 1024;
+template <typename T>
+__global__ void __launch_bounds__(1024) channel_sum_few_kernel(const T* __restrict__ src, T* __restrict__ dst, int rows, int c, int pitch)
+{
+    pdl_prologue();
+    __shared__ double sm[32][33];
+    const int ch = blockIdx.x * 32 + threadIdx.x;
+    double acc = 0.0;
+    if (ch < c) {
+#pragma unroll 4
+        for (int r = threadIdx.y; r < rows; r += 32) acc += (double)src[(int64_t)r * pitch + ch];
+    }
+    sm[threadIdx.y][threadIdx.x] = acc;
+    __syncthreads();
+    if (threadIdx.y == 0 && ch < c) {
+        double s = 0.0;
+#pragma unroll
+        for (int i = 0; i < 32; i++) s += sm[i][threadIdx.x];
+        dst[ch] = (T)s;
+    }
+}
+
+// NHWC float32 rows on any pitch (the few-rows kernel up to its limit, else dense rows only through channel_sum).
+int channel_sum_pitched(int64_t rows, int c, int pitch, const float* src, float* dst, void* ws, size_t ws_bytes, cudaStream_t st)
+{
+    if (rows <= CS_FEW_ROWS) {
+        launch_pdl(channel_sum_few_kernel<float>, (c + 31) / 32, dim3(32, 32), 0, st, src, dst, (int)rows, c, pitch);
+        return check_launch("channel_sum_few_kernel");
+    }
+    if (pitch != c) return B2C_ERR_UNSUPPORTED;
+    return channel_sum(B2C_F32, B2C_LAYOUT_NHWC, (int)rows, c, 1, src, dst, ws, ws_bytes, st);
+}
+
 // Enough for the float4 fast path to spread over about four CTAs per SM: two doubles per channel and chunk.
 size_t channel_sum_workspace_bytes(int n, int c, int hw)
 {
@@ -972,6 +1101,11 @@ int channel_sum(int dtype, int layout, int n, int c, int hw, const void* src, vo
 {
     if (!src || !dst || !ws) return B2C_ERR_NULL_POINTER;
     if (ws_bytes < (size_t)CS_CHUNKS * c * sizeof(double)) return B2C_ERR_WORKSPACE_TOO_SMALL;
+    if ((layout == B2C_LAYOUT_NHWC || hw == 1) && (int64_t)n * hw <= CS_FEW_ROWS) {
+        if (dtype == B2C_F32) launch_pdl(channel_sum_few_kernel<float>, (c + 31) / 32, dim3(32, 32), 0, st, (const float*)src, (float*)dst, n * hw, c, c);
+        else launch_pdl(channel_sum_few_kernel<double>, (c + 31) / 32, dim3(32, 32), 0, st, (const double*)src, (double*)dst, n * hw, c, c);
+        return check_launch("channel_sum_few_kernel");
+    }
     if (dtype == B2C_F32 && layout == B2C_LAYOUT_NHWC) {
         int r = channel_sum_v4(n, c, hw, src, dst, ws, ws_bytes, st);
         if (r != 1) return r;     // 1 = fast path not applicable

@@ -63,6 +63,13 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
                  : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
     return ok != 0;
 }
+// The same question without the suspension: for a look ahead between instructions that must not be held up.
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    return ok != 0;
+}
 
 // One lane of the (converged) warp is chosen; the compiler knows that exactly one thread runs the guarded
 // code, which lets it keep descriptors, coordinates and barrier addresses in uniform registers, the form
@@ -99,6 +106,23 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
         }
     }
 }
+
+// The wait of a converged warp: one vote when the phase is already complete, which is the usual case in a running pipeline.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status, code));
+}
+
+// Position in a ring of N stages.  `phase` is the parity of the current round: a consumer waits with it, a producer with the
+// other one (which a barrier nothing has completed yet reports as done, so the first round does not wait).  The warp
+// roles step through k-blocks with counters like this one and not with divisions: a role's bookkeeping per k-block is
+// instructions of a single warp, and with the divisions it cost 300 to 600 cycles of the 384 (64 columns) or 768 that
+// the products of a k-block take.
+template <int N> struct Ring {
+    int s = 0;
+    uint32_t phase = 0;
+    __device__ __forceinline__ void next() { if (++s == N) { s = 0; phase ^= 1; } }
+};
 
 __device__ __forceinline__ void fence_barrier_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
@@ -686,7 +710,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         // ---------------- TMA producer ----------------
         // The warp stays converged (every lane waits and computes the same coordinates); one elected lane arms
         // the barrier and issues the boxes of the k-block.
-        int it = 0;
+        Ring<STAGES> ring;
         bool ok = true;
         if (RESKB) {
             // The grid is a multiple of the column-tile count: this CTA only meets column tile blockIdx.x % nt, whose
@@ -745,21 +769,34 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
 #pragma unroll
                 for (int j = 0; j < BN / 32; j++) if (n0 + 32 * j < p.N) tx_bytes += 4096u;
             }
-            const int pix_begin = (MODE == TCM_WGRAD) ? z * p.kblocks * 32 : 0;
-            for (int kb = w.kb_b; kb < w.kb_e; kb++, it++) {
-                const int s = it % STAGES, use = it / STAGES;
+            // FWD: channel block and tap of the k-block, the tap's pixel offset and its place in the caller's filter.
+            // WGRAD: the first pixel of the k-block (32 pixels further each time: im_step images, p_step rows, q_step columns).
+            int cb = 0, sx = 0, off_w = 0, off_h = 0, tap_real = 0, tap_row = 0, im = 0, p0 = 0, q0 = 0, pix0 = 0;
+            int im_step = 0, p_step = 0, q_step = 0;
+            if (MODE == TCM_FWD) {
+                const int tap = w.kb_b / p.cblocks;
+                cb = w.kb_b - tap * p.cblocks;
+                const int r = tap / tg.S;
+                sx = tap - r * tg.S;
+                off_w = sx * p.dil_w; off_h = r * p.dil_h;
+                tap_row = (tg.r0 + p.tap_rstep * r) * p.tap_sreal + tg.s0; tap_real = tap_row + p.tap_sstep * sx;
+            } else {
+                pix0 = (z * p.kblocks + w.kb_b) * 32;
+                im = pix0 / (p.P * p.Q);
+                int rem = pix0 - im * (p.P * p.Q);
+                p0 = rem / p.Q; q0 = rem - p0 * p.Q;
+                im_step = 32 / (p.P * p.Q); rem = 32 - im_step * (p.P * p.Q); p_step = rem / p.Q; q_step = rem - p_step * p.Q;
+            }
+            for (int kb = w.kb_b; kb < w.kb_e; kb++) {
+                const int s = ring.s;
                 TC_PROF_T0();
-                bool good = true;
                 // a stage is free when the MMAs that read it have completed; with resident filters, as soon as the
                 // transform warps have copied its A tile to tensor memory
-                if (use > 0) good = mbar_wait(RESKB ? &afree_bar[s] : &empty_bar[s], (use - 1) & 1, abort_flag, &g_tc_status, TC_ERR_EMPTY);
-                good = __all_sync(0xffffffffu, good);
+                const bool good = mbar_wait_warp(RESKB ? &afree_bar[s] : &empty_bar[s], ring.phase ^ 1, abort_flag, &g_tc_status, TC_ERR_EMPTY);
                 if (lane == 0) TC_PROF_ADD(0);    // producer: waiting for a free stage
                 if (!good) { ok = false; break; }
                 uint8_t* st = smem + s * L::STAGE_BYTES;
                 if (MODE == TCM_FWD) {
-                    const int tap = kb / p.cblocks, cb = kb - tap * p.cblocks;
-                    const int r = tap / tg.S, sx = tap - r * tg.S;
                     if (elect_one_sync()) {
 #ifdef B2C_TC_DEV
                         if (p.dbg & 64) mbar_arrive(&full_bar[s]);
@@ -768,14 +805,13 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                         {
                             mbar_expect_tx(&full_bar[s], (uint32_t)(RESKB ? L::A_BYTES : BSRC == TCB_SPLIT ? L::STAGE_BYTES : L::A_BYTES + L::B_BYTES));
                             tma_load_im2col_4d(st, tg.ma, &full_bar[s], cb * 32, base_w, base_h, img,
-                                               (uint16_t)(sx * p.dil_w), (uint16_t)(r * p.dil_h));
+                                               (uint16_t)off_w, (uint16_t)off_h);
                             if (RESKB) {
                                 // the filter tiles are resident
                             } else if (BSRC == TCB_SPLIT) {
                                 tma_load_2d(st + L::A_BYTES, &tmap_b0, &full_bar[s], kb * 32, n0);
                                 tma_load_2d(st + L::A_BYTES + L::B_BYTES, &tmap_b1, &full_bar[s], kb * 32, n0);
                             } else {
-                                const int tap_real = (tg.r0 + p.tap_rstep * r) * p.tap_sreal + tg.s0 + p.tap_sstep * sx;
                                 if (BSRC == TCB_RAW_K) {
                                     tma_load_3d(st + L::A_BYTES, &tmap_b0, &full_bar[s], cb * 32, tap_real, n0);
                                 } else {
@@ -786,11 +822,11 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                             }
                         }
                     }
+                    if (++cb == p.cblocks) {
+                        cb = 0; off_w += p.dil_w; tap_real += p.tap_sstep;
+                        if (++sx == tg.S) { sx = 0; off_w = 0; off_h += p.dil_h; tap_row += p.tap_rstep * p.tap_sreal; tap_real = tap_row; }
+                    }
                 } else {
-                    const int pix0 = pix_begin + kb * 32;
-                    const int im = pix0 / (p.P * p.Q);
-                    const int rem = pix0 - im * (p.P * p.Q);
-                    const int p0 = rem / p.Q, q0 = rem - p0 * p.Q;
                     const int cw = q0 * p.str_w + p.low_w, chh = p0 * p.str_h + p.low_h;
                     if (elect_one_sync()) {
 #ifdef B2C_TC_DEV
@@ -810,15 +846,23 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                                 tma_load_2d(st + L::A_BYTES + j * 4096, &tmap_b0, &full_bar[s], n0 + 32 * j, pix0);
                         }
                     }
+                    pix0 += 32;
+                    q0 += q_step; if (q0 >= p.Q) { q0 -= p.Q; p0++; }
+                    p0 += p_step; if (p0 >= p.P) { p0 -= p.P; im++; }
+                    im += im_step;
                 }
+                ring.next();
                 __syncwarp();
                 if (lane == 0) TC_PROF_ADD(14);   // producer: TMA issue
             }
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        // Converged warp, one elected lane issues (see elect_one_sync).
-        {
+        // One elected lane runs the whole loop.  The tensor core takes about two MMAs ahead of the one it executes (measured:
+        // 100 cycles between groups of twelve are free with 128 columns, 400 cost 330), so whatever this lane does between
+        // the last MMA of a k-block and the first of the next is time the pipe stands still: the next k-block's barrier is
+        // looked at under the last MMAs, and votes, elections and divisions are out of the loop.
+        if (elect_one_sync()) {
             constexpr bool B_MN = MODE == TCM_WGRAD || BSRC == TCB_RAW_MN;
             // B tiles, K-major (FWD): rows of 128 B, 8-row groups 1024 B apart, K advances 32 B inside the row.
             // B tiles, MN-major (WGRAD): 32-row (K) boxes of 4096 B per 32 N elements, 4-row swizzle atoms of
@@ -828,7 +872,10 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             constexpr uint32_t LAYOUT = B_MN ? 1 : 2;
             constexpr uint64_t KADV = B_MN ? (1024 >> 4) : (32 >> 4);
             bool ok = true;
-            int it = 0, gc = 0;
+            Ring<TSLOTS> ring;                       // A slots in tensor memory (= the stages, unless the filters are resident)
+            int gc = 0;
+            bool ahead = false;                      // the next k-block was seen to be ready
+            const uint64_t b_desc0 = make_smem_desc(smem_u32(smem) + (RESKB ? L::RES_OFFSET : L::A_BYTES), LBO, SBO, LAYOUT);
             TileWalk w;
             w.init(total_tiles, p.kblocks, MODE == TCM_FWD && !SK && !MULTI && RESKB == 0 ? p.kper : 0, mt * nt);
             while (ok && w.template next<SK>()) {
@@ -842,54 +889,54 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 // (or a branch between the two forms per k-block) a long launch lost 3 to 6 % (2 %).
                 auto issue_tile = [&](auto whole_c) {
                 constexpr bool WHOLE = decltype(whole_c)::value;
-                for (int kb = w.kb_b; kb < w.kb_e && ok; kb++, it++) {
-                    const int s = it % TSLOTS, use = it / TSLOTS;        // A slot in tensor memory (= the stage, unless the filters are resident)
+                int ck = 0, cb = WHOLE || MODE == TCM_WGRAD ? 0 : w.kb_b % p.cblocks;
+                for (int kb = w.kb_b; kb < w.kb_e; kb++) {
+                    const int s = ring.s;
                     const int b = gc & 1;
-                    const bool chunk_start = ((kb - w.kb_b) % TC_CHUNK) == 0;
-                    const bool chunk_end = ((kb - w.kb_b) % TC_CHUNK) == TC_CHUNK - 1 || kb == w.kb_e - 1;
+                    const bool chunk_start = ck == 0;
+                    const bool chunk_end = ++ck == TC_CHUNK || kb == w.kb_e - 1;
                     TC_PROF_T0();
-                    if (chunk_start && gc >= 2)
-                        ok = mbar_wait(&tempty_bar[b], ((gc >> 1) - 1) & 1, abort_flag, &g_tc_status, TC_ERR_TEMPTY);
-                    if (lane == 0) TC_PROF_ADD(1);    // MMA: waiting for a drained TMEM buffer
+                    // a drained tensor-memory buffer (the first two chunks find theirs free)
+                    if (chunk_start) ok = mbar_wait(&tempty_bar[b], ((gc >> 1) & 1) ^ 1, abort_flag, &g_tc_status, TC_ERR_TEMPTY);
+                    TC_PROF_ADD(1);    // MMA: waiting for a drained TMEM buffer
                     // the transform warps arrive only after they have seen the stage's TMA data land
-                    if (ok) ok = mbar_wait(&xform_bar[s], use & 1, abort_flag, &g_tc_status, TC_ERR_XFORM);
-                    ok = __all_sync(0xffffffffu, ok);
-                    if (lane == 0) TC_PROF_ADD(3);    // MMA: waiting for the transform
+                    if (ok && !ahead) ok = mbar_wait(&xform_bar[s], ring.phase, abort_flag, &g_tc_status, TC_ERR_XFORM);
+                    TC_PROF_ADD(3);    // MMA: waiting for the transform
                     if (!ok) break;
                     tc_fence_after();
-                    const uint32_t sb = RESKB ? smem_u32(smem + L::RES_OFFSET + kb * 2 * L::B_BYTES) : smem_u32(smem + s * L::STAGE_BYTES) + L::A_BYTES;
-                    const uint64_t b_hi = make_smem_desc(sb, LBO, SBO, LAYOUT);
-                    const uint64_t b_lo = make_smem_desc(sb + L::B_BYTES, LBO, SBO, LAYOUT);
+                    const uint64_t b_hi = b_desc0 + (uint64_t)(RESKB ? kb * (2 * L::B_BYTES >> 4) : s * (L::STAGE_BYTES >> 4));
+                    const uint64_t b_lo = b_hi + (L::B_BYTES >> 4);
                     const uint32_t a_hi = tmem_base + (uint32_t)(L::TMEM_A_COL + s * 64);
                     const uint32_t a_lo = a_hi + 32;
                     const uint32_t d = tmem_base + (uint32_t)(b * BN);
-                    if (elect_one_sync()) {
-                        // small terms first: lo*hi, hi*lo, then hi*hi
-                        auto step = [&](int k, uint32_t id) {
-                            const uint64_t adv = (uint64_t)k * KADV;
+                    ring.next();
+                    // small terms first: lo*hi, hi*lo, then hi*hi
+                    auto step = [&](int k, uint32_t id) {
+                        const uint64_t adv = (uint64_t)k * KADV;
 #ifdef B2C_TC_DEV
-                            if (p.dbg & 32) return;
+                        if (p.dbg & 32) return;
 #endif
-                            umma_tf32_ts(d, a_lo + k * 8, b_hi + adv, id, (!chunk_start || k > 0) ? 1u : 0u);
+                        umma_tf32_ts(d, a_lo + k * 8, b_hi + adv, id, (!chunk_start || k > 0) ? 1u : 0u);
 #ifdef B2C_TC_DEV
-                            if (p.dbg & 2) return;
+                        if (p.dbg & 2) return;
 #endif
-                            umma_tf32_ts(d, a_hi + k * 8, b_lo + adv, id, 1u);
-                            umma_tf32_ts(d, a_hi + k * 8, b_hi + adv, id, 1u);
-                        };
-                        if constexpr (WHOLE) {
-#pragma unroll
-                            for (int k = 0; k < 4; k++) step(k, make_idesc_tf32(128, BN, 0, B_MN));
-                        } else {
-                            const int ks = MODE == TCM_FWD && kb % p.cblocks == p.cblocks - 1 ? p.ktail : 4;
-                            for (int k = 0; k < ks; k++) step(k, idesc);
-                        }
-                        umma_commit(&empty_bar[s]);
-                        if (chunk_end) umma_commit(&tfull_bar[b]);
+                        umma_tf32_ts(d, a_hi + k * 8, b_lo + adv, id, 1u);
+                        umma_tf32_ts(d, a_hi + k * 8, b_hi + adv, id, 1u);
+                    };
+                    if constexpr (WHOLE) {
+                        constexpr uint32_t id = make_idesc_tf32(128, BN, 0, B_MN);
+                        step(0, id); step(1, id); step(2, id);
+                        ahead = mbar_test(&xform_bar[ring.s], ring.phase);
+                        step(3, id);
+                    } else {
+                        const int ks = MODE == TCM_FWD && cb == p.cblocks - 1 ? p.ktail : 4;
+                        for (int k = 0; k < ks; k++) step(k, idesc);
+                        ahead = mbar_test(&xform_bar[ring.s], ring.phase);
                     }
-                    __syncwarp();
-                    if (chunk_end) gc++;
-                    if (lane == 0) TC_PROF_ADD(4);    // MMA: issue
+                    umma_commit(&empty_bar[s]);
+                    if (chunk_end) { umma_commit(&tfull_bar[b]); gc++; ck = 0; }
+                    if (!WHOLE && ++cb == p.cblocks) cb = 0;
+                    TC_PROF_ADD(4);    // MMA: issue
                 }
                 };
                 if (left > BN - 16 && (MODE == TCM_WGRAD || p.ktail == 4)) issue_tile(std::true_type{});
@@ -908,7 +955,8 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         constexpr bool SPLIT_B = MODE == TCM_WGRAD || BSRC != TCB_SPLIT;    // the lo half of B is made here
         constexpr int B_VEC = SPLIT_B ? L::B_BYTES / 16 / 128 : 0;
         const int t = threadIdx.x - 64;              // 0..127
-        int it = 0;
+        Ring<STAGES> ring;
+        Ring<TSLOTS> slots;                          // the stages' own A slots, or (resident filters) a separate ring
         bool ok = true;
         if (RESKB) {
             // the lo halves of the resident filter tiles, once per launch
@@ -941,20 +989,18 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             const bool do_db = MODE == TCM_WGRAD && p.db_partial != nullptr && (w.tile / nt) % mt == 0;
 #pragma unroll
             for (int i = 0; i < B_VEC / 2; i++) dbacc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int kb = w.kb_b; kb < w.kb_e; kb++, it++) {
-                const int s = it % STAGES, use = it / STAGES;
+            for (int kb = w.kb_b; kb < w.kb_e; kb++, ring.next(), slots.next()) {
+                const int s = ring.s, ts = slots.s;
                 TC_PROF_T0();
-                if (!mbar_wait(&full_bar[s], use & 1, abort_flag, &g_tc_status, TC_ERR_FULL)) { ok = false; break; }
+                if (!mbar_wait(&full_bar[s], ring.phase, abort_flag, &g_tc_status, TC_ERR_FULL)) { ok = false; break; }
                 if (t == 0) TC_PROF_ADD(5);    // transform: waiting for TMA data
                 const uint8_t* st = smem + s * L::STAGE_BYTES;
-                // the A slot in tensor memory: the stage's own, or (resident filters) the next of a separate ring that
-                // is free once the MMAs that read it have completed
-                const int ts = it % TSLOTS, tuse = it / TSLOTS;
-                if (RESKB && tuse > 0 && !mbar_wait(&empty_bar[ts], (tuse - 1) & 1, abort_flag, &g_tc_status, TC_ERR_EMPTY)) { ok = false; break; }
+                // a slot of a separate ring is free once the MMAs that read it have completed
+                if (RESKB && !mbar_wait(&empty_bar[ts], slots.phase ^ 1, abort_flag, &g_tc_status, TC_ERR_EMPTY)) { ok = false; break; }
 #ifdef B2C_TC_DEV
                 if (p.dbg & 4) { tc_fence_before(); __syncwarp(); if (lane == 0) { if (RESKB) mbar_arrive(&afree_bar[s]); mbar_arrive(&xform_bar[ts]); } continue; }
 #endif
-                uint32_t v[32], h[32];
+                uint32_t v[32];
                 if (MODE == TCM_FWD) {
                     // K-major 128B-swizzled tile: row r is 128 B, its 16-byte chunk c sits at chunk c ^ (r & 7)
                     const uint8_t* a_row = st + row * 128;
@@ -965,29 +1011,38 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                     }
                 } else {
                     // unswizzled boxes of [32 pixels][a_box rows]: this thread's row is a column of its box
-                    const int a_box = 1 << p.a_box_log2;
-                    const uint32_t* a_col = reinterpret_cast<const uint32_t*>(st + (row >> p.a_box_log2) * (a_box * 128)) + (row & (a_box - 1));
+                    auto column = [&](auto box_c) {
+                        constexpr int a_box = decltype(box_c)::value;
+                        const uint32_t* a_col = reinterpret_cast<const uint32_t*>(st + (row / a_box) * (a_box * 128)) + (row & (a_box - 1));
 #pragma unroll
-                    for (int k = 0; k < 32; k++) v[k] = a_col[k * a_box];
+                        for (int k = 0; k < 32; k++) v[k] = a_col[k * a_box];
+                    };
+                    if (p.a_box_log2 == 7) column(std::integral_constant<int, 128>{});
+                    else if (p.a_box_log2 == 6) column(std::integral_constant<int, 64>{});
+                    else column(std::integral_constant<int, 32>{});
+                }
+                // all reads of the stage first, so that the B tile's latency is under the A tile's
+                float4 bq[SPLIT_B && RESKB == 0 ? B_VEC : 1];
+                if (SPLIT_B && RESKB == 0) {
+                    const float4* b_hi = (const float4*)(st + L::A_BYTES);
+#pragma unroll
+                    for (int i = 0; i < B_VEC; i++) bq[i] = b_hi[t + i * 128];
                 }
                 if (RESKB) {
                     // the A tile is in registers: the producer may refill the stage
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&afree_bar[s]);
                 }
-#pragma unroll
-                for (int j = 0; j < 32; j++) h[j] = v[j] & 0xFFFFE000u;
                 const uint32_t slot = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(L::TMEM_A_COL + ts * 64);
-                tmem_st_32x32(slot, h);
+                tmem_st_32x32(slot, v);              // hi: the tensor core reads the upper 19 bits
 #pragma unroll
-                for (int j = 0; j < 32; j++) v[j] = __float_as_uint(__uint_as_float(v[j]) - __uint_as_float(h[j]));
+                for (int j = 0; j < 32; j++) v[j] = __float_as_uint(__uint_as_float(v[j]) - __uint_as_float(v[j] & 0xFFFFE000u));
                 tmem_st_32x32(slot + 32, v);
                 if (SPLIT_B && RESKB == 0) {
-                    const float4* b_hi = (const float4*)(st + L::A_BYTES);
                     float4* b_lo = (float4*)(smem + s * L::STAGE_BYTES + L::A_BYTES + L::B_BYTES);
 #pragma unroll
                     for (int i = 0; i < B_VEC; i++) {
-                        const float4 q = b_hi[t + i * 128];
+                        const float4 q = bq[i];
                         if (do_db) { dbacc[i >> 1].x += q.x; dbacc[i >> 1].y += q.y; dbacc[i >> 1].z += q.z; dbacc[i >> 1].w += q.w; }
                         float4 l;
                         l.x = q.x - __uint_as_float(__float_as_uint(q.x) & 0xFFFFE000u);
@@ -1681,7 +1736,7 @@ static unsigned int* tc_sync_bank(cudaStream_t st)
 static double tc_balance_threshold()
 {
     static double v = -1.0;
-    if (v < 0.0) { const char* e = getenv("B2C_TC_BALANCE"); v = e ? atof(e) : 0.85; }
+    if (v < 0.0) { const char* e = getenv("B2C_TC_BALANCE"); v = e ? atof(e) : 1.0; }
     return v;
 }
 
@@ -1880,9 +1935,9 @@ struct StatsOut { float* sums; };
 
 // How a forward launch is cut: whole tiles, balanced k-block ranges (sk), or the K loop of every tile split over several
 // CTAs (kper k-blocks each).  Costs in k-block units (0.6 us): whole tiles take rounds x kblocks; balanced ranges take
-// units / G plus the hand-over of partial tiles, one after the other in the CTA that owns the tile (about four units for
-// the first, ten for each further CTA on the same tile: 57 us on 32 tiles of 144 k-blocks that are 20 us of products); a split
-// takes its k-blocks, the partials' way through L2 and the second stage's launch (about five units).  The partials of
+// units / G plus the hand-over of partial tiles, one after the other in the CTA that owns the tile (24 units for
+// the first -- 4 and a threshold of 0.85 before splits existed: 9.44 -> 9.25 ms on an NCHW ResNet-50 step of 32 images -- and ten
+// for each further CTA on the same tile: 57 us on 32 tiles of 144 k-blocks that are 20 us of products); a split takes its k-blocks, the partials' way through L2 and the second stage's launch (about five units).  The partials of
 // a split fit the balanced mode's scratch because tiles x splits is at most one CTA per SM.
 struct FwdPlan { bool sk; int kper; };
 static FwdPlan fwd_plan(int64_t M, int N, int64_t kblocks)
@@ -1893,7 +1948,7 @@ static FwdPlan fwd_plan(int64_t M, int N, int64_t kblocks)
     const int64_t rounds = (tiles + G - 1) / G;
     const double plain = (double)rounds * (double)kblocks;
     const double shared = (double)G / (double)tiles;         // CTAs on one tile
-    const double balanced = (double)(tiles * kblocks) / G + 4.0 + (shared > 2.0 ? 10.0 * (shared - 2.0) : 0.0);
+    const double balanced = (double)(tiles * kblocks) / G + 24.0 + (shared > 2.0 ? 10.0 * (shared - 2.0) : 0.0);
     FwdPlan best{false, 0};
     double cost = plain;
     if (tiles * kblocks >= 4 * (int64_t)G && balanced < tc_balance_threshold() * plain) { best.sk = true; cost = balanced; }
@@ -2316,6 +2371,15 @@ static int tc_wgrad_nhwc(const Geo& g, const void* x, const void* dy, void* dw, 
         wsd = w_stride(g.w_layout, g.co, g.ci, 1, 1);
         const int64_t t = wsd.sk; wsd.sk = wsd.sc; wsd.sc = t;
     }
+    // One pixel range and a filter layout that is the GEMM's own (rows = input channels, output channels contiguous): the
+    // tiles go straight to dw and only the bias gradient is left for a kernel of its own.
+    if (pl.splits == 1 && !low && !exchanged && g.kh * g.kw == 1 && wsd.sk == 1 && wsd.sc % 4 == 0 && ((uintptr_t)dw & 15) == 0 && p.tma_store &&
+        make_map_out(&mo, dw, 1, (uint64_t)g.ci, (uint64_t)g.co, (uint64_t)wsd.sc)) {
+        p.db_partial = nullptr;
+        const int rc = dispatch_wgrad(pl.bn, ma, mb, mo, p, 1, st);
+        if (rc || !db) return rc;
+        return channel_sum_pitched(g.M, g.co, g.yp, (const float*)dy, (float*)db, partial, pbytes + cs, st);
+    }
     int rc = dispatch_wgrad(pl.bn, ma, mb, mo, p, pl.splits, st);
     if (rc) return rc;
     WgradReduceParams rp{Krows, g.co, low ? g.ci : Cp, g.kw, pl.splits, wsd.sk, wsd.sc, wsd.sr, wsd.ss, low ? (int)g.K : Krows, g.ci, Np};
@@ -2380,6 +2444,51 @@ __global__ void __launch_bounds__(256) transpose_thin_kernel(const T* __restrict
         if (r < thin) { if (ROWS_THIN) d[(int64_t)l * tp + r] = v[r]; else d[(int64_t)r * len + l] = v[r]; }
 }
 
+// The same transpose in 64 x 64 tiles with 16-byte accesses on the sides that allow them (VL: loads, VS: stores): a thread
+// has 64 bytes in flight instead of 16.  32 images of 3136 x 128 floats: 20.7 us (2.5 TB/s) with the 32 x 32 tiles.  Taken
+// when its tiles fill the chip and are not mostly outside the matrix.
+template <typename T, bool VL, bool VS>
+__global__ void __launch_bounds__(256) transpose_wide_kernel(const T* __restrict__ src, T* __restrict__ dst, int rows, int cols, int sp, int dp)
+{
+    pdl_prologue();
+    constexpr int V = 16 / sizeof(T), LV = VL ? V : 1, SV = VS ? V : 1;
+    struct __align__(16) Vec { T v[V]; };
+    __shared__ T tile[64][65];
+    const int c0 = blockIdx.x * 64, r0 = blockIdx.y * 64;
+    const T* s = src + (int64_t)blockIdx.z * rows * sp;
+    T* d = dst + (int64_t)blockIdx.z * cols * dp;
+    constexpr int LX = 64 / LV, LN = 64 * LX / 256, SX = 64 / SV, SN = 64 * SX / 256;
+    const int lc = threadIdx.x % LX * LV, lr = threadIdx.x / LX;
+    T q[LN][LV];
+#pragma unroll
+    for (int i = 0; i < LN; i++) {
+        const int r = r0 + lr + i * (256 / LX), c = c0 + lc;
+        if (r < rows && c < cols) {
+            if constexpr (VL) { const Vec v = *reinterpret_cast<const Vec*>(s + (int64_t)r * sp + c);
+#pragma unroll
+                for (int e = 0; e < LV; e++) q[i][e] = v.v[e]; }
+            else q[i][0] = s[(int64_t)r * sp + c];
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < LN; i++)
+#pragma unroll
+        for (int e = 0; e < LV; e++) tile[lr + i * (256 / LX)][lc + e] = q[i][e];
+    __syncthreads();
+    const int sr = threadIdx.x % SX * SV, sc = threadIdx.x / SX;        // rows of src are columns of dst
+#pragma unroll
+    for (int i = 0; i < SN; i++) {
+        const int cl = sc + i * (256 / SX), c = c0 + cl, r = r0 + sr;
+        if (c < cols && r < rows) {
+            if constexpr (VS) { Vec v;
+#pragma unroll
+                for (int e = 0; e < SV; e++) v.v[e] = tile[sr + e][cl];
+                *reinterpret_cast<Vec*>(d + (int64_t)c * dp + r) = v; }
+            else d[(int64_t)c * dp + r] = tile[sr][cl];
+        }
+    }
+}
+
 template <typename T>
 static int transpose_t(const void* src, void* dst, int n, int rows, int cols, int sp, int dp, cudaStream_t st)
 {
@@ -2395,6 +2504,16 @@ static int transpose_t(const void* src, void* dst, int n, int rows, int cols, in
     if (cols <= 8 && rows > 8 && dp == rows) {
         launch_pdl(transpose_thin_kernel<T, false>, dim3((rows + 255) / 256, n), 256, 0, st, (const T*)src, (T*)dst, cols, rows, sp);
         return check_launch("transpose_thin_kernel");
+    }
+    const int64_t wide = (int64_t)((cols + 63) / 64) * ((rows + 63) / 64) * n;
+    if (rows > 32 && cols > 32 && wide >= tc_sm_count()) {
+        constexpr int V = 16 / (int)sizeof(T);
+        const bool vl = sp % V == 0 && cols % V == 0 && ((uintptr_t)src & 15) == 0, vs = dp % V == 0 && rows % V == 0 && ((uintptr_t)dst & 15) == 0;
+        const dim3 grid((cols + 63) / 64, (rows + 63) / 64, n);
+        auto* kernel = vl ? (vs ? transpose_wide_kernel<T, true, true> : transpose_wide_kernel<T, true, false>)
+                          : (vs ? transpose_wide_kernel<T, false, true> : transpose_wide_kernel<T, false, false>);
+        launch_pdl(kernel, grid, 256, 0, st, (const T*)src, (T*)dst, rows, cols, sp, dp);
+        return check_launch("transpose_wide_kernel");
     }
     launch_pdl(transpose_inner_kernel<T>, dim3((cols + 31) / 32, (rows + 31) / 32, n), dim3(32, 8), 0, st,
                (const T*)src, (T*)dst, rows, cols, sp, dp);

@@ -11,7 +11,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("dtype", ["float32", "float64"])
-@pytest.mark.parametrize("n,rows,cols", [(1, 1, 1), (3, 3, 49), (2, 49, 3), (2, 33, 31), (2, 8, 9), (1, 257, 64), (66000, 3, 4)])
+@pytest.mark.parametrize("n,rows,cols", [(1, 1, 1), (3, 3, 49), (2, 49, 3), (2, 33, 31), (2, 8, 9), (1, 257, 64), (66000, 3, 4),
+                                         (40, 68, 130), (40, 65, 132), (40, 67, 129), (80, 33, 64), (1, 1000, 901)])
 def test_transpose(dtype, n, rows, cols):
     x = torch.randn(n, rows, cols, dtype=getattr(torch, dtype), device=DEV)
     y = torch.full((n, cols, rows), float("nan"), dtype=x.dtype, device=DEV)

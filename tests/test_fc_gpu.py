@@ -1,0 +1,39 @@
+"""FC layers over the range of their routes (dot products, dense tiles written straight to dw, split sums, small batch with a
+large matrix, generic): forward and backward against NumPy in float64, with and without each output. GPU."""
+import numpy as np
+import pytest
+import torch
+
+from pydtnn_b200 import _lib
+from tests.gpu_util import DEV, assert_parity, dev, stream
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", ["float32", "float64"])
+@pytest.mark.parametrize("n,i,o", [(1, 1, 1), (64, 128, 10), (9, 33, 31), (512, 16, 1000), (513, 16, 1000), (5, 129, 127), (1, 4096, 1000), (64, 1568, 128),
+                                   (128, 300, 100), (33, 2048, 1004), (64, 257, 130), (130, 640, 72), (32, 4096, 1024), (97, 520, 1001)])
+def test_fc_routes(n, i, o, dtype):
+    L, dt = _lib.lib(), _lib.dtype_code(np.dtype(dtype))
+    rng = np.random.Generator(np.random.PCG64(n + i + o))
+    x, w, b, dy = (rng.standard_normal(s).astype(dtype) for s in ((n, i), (i, o), (o,), (n, o)))
+    X, W, B, D = (a.astype(np.float64) for a in (x, w, b, dy))
+    xd, wd, bd, dyd = (dev(a) for a in (x, w, b, dy))
+    ws = torch.empty(max(256, L.b2c_fc_workspace_bytes(dt, n, i, o, 0)), dtype=torch.uint8, device=DEV)
+
+    def out(*shape):
+        return torch.full(shape, float("nan"), dtype=xd.dtype, device=DEV)
+    for bias in (bd, None):
+        y = out(n, o)
+        _lib.check(L.b2c_fc_forward(dt, 0, n, i, o, xd.data_ptr(), wd.data_ptr(), bias.data_ptr() if bias is not None else None, y.data_ptr(),
+                                    ws.data_ptr(), ws.numel(), stream()))
+        assert_parity(y.cpu().numpy(), X @ W + (B if bias is not None else 0), dtype, "y")
+    for which in ((1, 1, 1), (1, 0, 0), (0, 1, 0), (0, 0, 1), (1, 0, 1)):
+        t = (out(i, o), out(o), out(n, i))
+        _lib.check(L.b2c_fc_backward(dt, 0, n, i, o, xd.data_ptr(), dyd.data_ptr(), wd.data_ptr(),
+                                     *(u.data_ptr() if k else None for u, k in zip(t, which)), ws.data_ptr(), ws.numel(), stream()))
+        for u, k, ref in zip(t, which, (X.T @ D, D.sum(0), D @ W.T)):
+            if k:
+                assert_parity(u.cpu().numpy(), ref, dtype, str(which))
+            else:
+                assert bool(torch.isnan(u).all())
