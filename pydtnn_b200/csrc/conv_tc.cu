@@ -469,7 +469,7 @@ struct TcParams {
     int sk;
     float* sk_partial;
     int* sk_flags;
-    float* db_partial;         // WGRAD: per-(split, transform warp) channel sums of dy, [splits][4][N], or null
+    float* db_partial;         // WGRAD: per-(split, transform warp) channel sums of dy, [splits][4][Np], or null
     int tma_store;             // output rows are dense [M][N] (or [split][M][N]): store tiles through the output tensor map
     int sk_selfclean;          // balanced mode: the owner returns a consumed flag to zero (flags in the library's bank)
     // FWD writing one parity class of a stride-2 data gradient whose other three classes are zeros (a 1x1 filter): with
@@ -1388,19 +1388,21 @@ __global__ void __launch_bounds__(256) tc_split_finish_kernel(FinishParams p)
             const int m = (blockIdx.y * ROWS + r) * 8 + ty;
             if (m >= p.M) continue;
             const float* src = p.partial + (int64_t)m * p.pitch + n0;
-            float4 v = __ldcg(reinterpret_cast<const float4*>(src));
-            int z = 1;
-            for (; z + 8 <= p.splits; z += 8) {
-                float4 q[8];
+            // eight sums over every eighth split, then those in order: the order of tc_split_finish_deep_kernel
+            float4 s[8];
 #pragma unroll
-                for (int u = 0; u < 8; u++) q[u] = __ldcg(reinterpret_cast<const float4*>(src + (z + u) * p.plane));
+            for (int u = 0; u < 8; u++) s[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int z = 0; z < p.splits; z += 8) {
 #pragma unroll
-                for (int u = 0; u < 8; u++) { v.x += q[u].x; v.y += q[u].y; v.z += q[u].z; v.w += q[u].w; }
+                for (int u = 0; u < 8; u++)
+                    if (z + u < p.splits) {
+                        const float4 q = __ldcg(reinterpret_cast<const float4*>(src + (z + u) * p.plane));
+                        s[u].x += q.x; s[u].y += q.y; s[u].z += q.z; s[u].w += q.w;
+                    }
             }
-            for (; z < p.splits; z++) {
-                const float4 q = __ldcg(reinterpret_cast<const float4*>(src + z * p.plane));
-                v.x += q.x; v.y += q.y; v.z += q.z; v.w += q.w;
-            }
+            float4 v = s[0];
+#pragma unroll
+            for (int u = 1; u < 8; u++) { v.x += s[u].x; v.y += s[u].y; v.z += s[u].z; v.w += s[u].w; }
             float a[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
             for (int e = 0; e < 4; e++)
@@ -1434,25 +1436,71 @@ __global__ void __launch_bounds__(256) tc_split_finish_kernel(FinishParams p)
     }
 }
 
+// The same for few rows cut many times (a single image's late layers, a fully connected layer): a block owns 128 channels of
+// one row and its eight thread rows share the splits (row y adds splits y, y + 8, .. in order, then the rows are added in
+// order), so no thread has more than a few loads one after the other: 14 -> 5 us for 64 rows cut 49 times.
+__global__ void __launch_bounds__(256) tc_split_finish_deep_kernel(FinishParams p)
+{
+    pdl_prologue();
+    __shared__ float4 part[8][32];
+    const int lane = threadIdx.x & 31, ty = threadIdx.x >> 5, n0 = blockIdx.x * 128 + lane * 4, m = blockIdx.y;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (n0 < p.N) {
+        const float* src = p.partial + (int64_t)m * p.pitch + n0;
+#pragma unroll 4
+        for (int z = ty; z < p.splits; z += 8) {
+            const float4 q = __ldcg(reinterpret_cast<const float4*>(src + z * p.plane));
+            v.x += q.x; v.y += q.y; v.z += q.z; v.w += q.w;
+        }
+    }
+    part[ty][lane] = v;
+    __syncthreads();
+    if (ty != 0 || n0 >= p.N) return;
+#pragma unroll
+    for (int y = 1; y < 8; y++) { const float4 q = part[y][lane]; v.x += q.x; v.y += q.y; v.z += q.z; v.w += q.w; }
+    float a[4] = {v.x, v.y, v.z, v.w};
+    const int cnt = p.N - n0 < 4 ? p.N - n0 : 4;
+    const int img = m / (p.P * p.Q), rem = m - img * (p.P * p.Q), pi = rem / p.Q, qi = rem - pi * p.Q;
+    float* d = p.out + img * p.o_sn + pi * p.o_sh + qi * p.o_sw + n0;
+#pragma unroll
+    for (int e = 0; e < 4; e++)
+        if (e < cnt) {
+            if (p.bias) a[e] += __ldg(p.bias + n0 + e);
+            if (p.mean) { const float t = (a[e] - __ldg(p.mean + n0 + e)) * __ldg(p.inv_std + n0 + e); a[e] = t * __ldg(p.gamma + n0 + e) + __ldg(p.beta + n0 + e); }
+            if (p.relu) a[e] = fmaxf(a[e], 0.f);
+            d[e] = a[e];
+        }
+}
+
 // Second stage of the weight gradient: fixed-order sum of the per-split partial tiles, written in the
 // caller's filter layout.
+// db_rows: rows of partial bias sums.
 // C rows per tap of which the first Creal are channels, Np floats per row.
-struct WgradReduceParams { int M, N, C, S, splits; int64_t sk, sc, sr, ss; int Mreal, Creal, Np; };
+struct WgradReduceParams { int M, N, C, S, splits; int64_t sk, sc, sr, ss; int Mreal, Creal, Np, db_rows; };
+
+// The bias gradient of 32 channels, by the blocks of a last block row of their own (in the first row it was the longest chain
+// of the launch): thread row y adds rows y, y + 8, .. of the partial sums, the thread rows are added in order.
+__device__ __forceinline__ void tc_wgrad_bias_sums(const WgradReduceParams& p, const float* __restrict__ db_partial, float* __restrict__ db, float (*part)[33])
+{
+    const int n = blockIdx.x * 32 + threadIdx.x;
+    float v = 0.f;
+    if (n < p.N) {
+#pragma unroll 8
+        for (int i = threadIdx.y; i < p.db_rows; i += 8) v += __ldcg(db_partial + (size_t)i * p.Np + n);
+    }
+    part[threadIdx.y][threadIdx.x] = v;
+    __syncthreads();
+    if (threadIdx.y != 0 || n >= p.N) return;
+#pragma unroll
+    for (int y = 1; y < 8; y++) v += part[y][threadIdx.x];
+    db[n] = v;
+}
 
 template <int ROWS>
 __global__ void __launch_bounds__(256) tc_wgrad_reduce_kernel(WgradReduceParams p, const float* __restrict__ partial, float* __restrict__ dw,
                                                               const float* __restrict__ db_partial, float* __restrict__ db)
 {
     pdl_prologue();
-    // bias gradient: the [splits][4] per-channel sums, added in a fixed order (first block row only)
-    if (db && blockIdx.y == 0) {
-        const int n = blockIdx.x * 32 + threadIdx.x;
-        if (threadIdx.y == 0 && n < p.N) {
-            float v = 0.f;
-            for (int i = 0; i < p.splits * 4; i++) v += __ldcg(db_partial + (size_t)i * p.Np + n);
-            db[n] = v;
-        }
-    }
     // A block owns 8 * ROWS rows (tap, ci) x 32 output channels.  Thread (x, y) adds, in split order, the partials of
     // column n0 + x for rows y, y + 8, ... (loads of a warp cover 128 contiguous bytes; ROWS rows x 16 / ROWS splits
     // at a time are independent loads).  ROWS = 4 for large filters; ROWS = 1 makes four times the blocks when the
@@ -1461,6 +1509,7 @@ __global__ void __launch_bounds__(256) tc_wgrad_reduce_kernel(WgradReduceParams 
     // a transposing shared-memory tile.
     constexpr int TR = 8 * ROWS, U = 16 / ROWS;
     __shared__ float tile[TR][33];
+    if (db && blockIdx.y == gridDim.y - 1) { tc_wgrad_bias_sums(p, db_partial, db, tile); return; }
     const int m0 = blockIdx.y * TR, n0 = blockIdx.x * 32;
     const int64_t plane = (int64_t)p.M * p.Np;
     const int n = n0 + threadIdx.x;
@@ -1524,21 +1573,8 @@ __global__ void __launch_bounds__(256) tc_wgrad_reduce_deep_kernel(WgradReducePa
 {
     pdl_prologue();
     __shared__ float part[8][33];
+    if (db && blockIdx.y == gridDim.y - 1) { tc_wgrad_bias_sums(p, db_partial, db, part); return; }
     const int n = blockIdx.x * 32 + threadIdx.x, m = blockIdx.y;
-    if (db && blockIdx.y == 0) {
-        // bias gradient: [splits * 4] row sums per channel, shared among the thread rows the same way
-        float v = 0.f;
-        if (n < p.N) for (int i = threadIdx.y; i < p.splits * 4; i += 8) v += __ldcg(db_partial + (size_t)i * p.Np + n);
-        part[threadIdx.y][threadIdx.x] = v;
-        __syncthreads();
-        if (threadIdx.y == 0 && n < p.N) {
-            float t = 0.f;
-#pragma unroll
-            for (int y = 0; y < 8; y++) t += part[y][threadIdx.x];
-            db[n] = t;
-        }
-        __syncthreads();
-    }
     const int64_t plane = (int64_t)p.M * p.Np;
     float v = 0.f;
     if (n < p.N) {
@@ -1933,30 +1969,33 @@ static int transpose_t(const void* src, void* dst, int n, int rows, int cols, in
 // Where a forward pass leaves the batch statistics of its output (see TcParams::stats), or null.
 struct StatsOut { float* sums; };
 
-// How a forward launch is cut: whole tiles, balanced k-block ranges (sk), or the K loop of every tile split over several
-// CTAs (kper k-blocks each).  Costs in k-block units (0.6 us): whole tiles take rounds x kblocks; balanced ranges take
-// units / G plus the hand-over of partial tiles, one after the other in the CTA that owns the tile (24 units for
-// the first -- 4 and a threshold of 0.85 before splits existed: 9.44 -> 9.25 ms on an NCHW ResNet-50 step of 32 images -- and ten
-// for each further CTA on the same tile: 57 us on 32 tiles of 144 k-blocks that are 20 us of products); a split takes its k-blocks, the partials' way through L2 and the second stage's launch (about five units).  The partials of
-// a split fit the balanced mode's scratch because tiles x splits is at most one CTA per SM.
-struct FwdPlan { bool sk; int kper; };
-static FwdPlan fwd_plan(int64_t M, int N, int64_t kblocks)
+// How a forward launch is cut: column tiles of 128 or 64, whole tiles, balanced k-block ranges (sk), or the K loop of every
+// tile split over several CTAs (kper k-blocks each).  Costs in microseconds, measured: a k-block takes 0.45 (0.33 with 64
+// columns: half the products, the same hand-offs), the last tile's way out 2 (1); whole tiles take rounds x k-blocks.
+// Balanced ranges take units / G plus the hand-over of partial tiles, one after the other in the CTA that owns the tile (11 for
+// the first, 4.5 for each further CTA on the same tile: 57 us on 32 tiles of 144 k-blocks that are 20 us of products).  A split
+// takes its k-blocks, the second stage's launch (3) and the partials' way through L2; they fit the balanced mode's scratch
+// because tiles x splits is at most one CTA per SM.  Narrow tiles only pay where the wide ones leave the chip idle (single
+// images, late layers of small batches).
+struct FwdPlan { int bn; bool sk; int kper; };
+static FwdPlan fwd_plan(int64_t M, int N, int64_t kblocks, bool may_share)
 {
     const int G = tc_sm_count();
-    const int BN = N <= 64 ? 64 : 128;
-    const int64_t tiles = ((M + 127) / 128) * ((N + BN - 1) / BN);
-    const int64_t rounds = (tiles + G - 1) / G;
-    const double plain = (double)rounds * (double)kblocks;
-    const double shared = (double)G / (double)tiles;         // CTAs on one tile
-    const double balanced = (double)(tiles * kblocks) / G + 24.0 + (shared > 2.0 ? 10.0 * (shared - 2.0) : 0.0);
-    FwdPlan best{false, 0};
-    double cost = plain;
-    if (tiles * kblocks >= 4 * (int64_t)G && balanced < tc_balance_threshold() * plain) { best.sk = true; cost = balanced; }
-    for (int64_t s = 2; s * tiles <= G && s <= kblocks; s++) {
-        const int64_t kper = (kblocks + s - 1) / s;
-        if ((kblocks + kper - 1) / kper != s) continue;
-        const double split = (double)kper + 5.0 + (double)s * (double)M * N * 8.0 / 4e12 / 0.6e-6;
-        if (split < 0.9 * cost) { best.sk = false; best.kper = (int)kper; cost = split / 0.9; }
+    FwdPlan best{128, false, 0};
+    double cost = 1e30;
+    for (int bn = N <= 64 ? 64 : 128; bn >= 64; bn -= 64) {
+        const double kb = bn == 128 ? 0.45 : 0.33, drain = bn == 128 ? 2.0 : 1.0;
+        const int64_t tiles = ((M + 127) / 128) * ((N + bn - 1) / bn), rounds = (tiles + G - 1) / G;
+        auto offer = [&](double c, bool sk, int kper) { if (c < 0.95 * cost) { best = FwdPlan{bn, sk, kper}; cost = c; } };
+        offer((double)(rounds * kblocks) * kb + drain, false, 0);
+        if (!may_share) continue;
+        const double shared = (double)G / (double)tiles;         // CTAs on one tile
+        if (tiles * kblocks >= 4 * (int64_t)G)
+            offer(((double)(tiles * kblocks) / G * kb + 11.0 + (shared > 2.0 ? 4.5 * (shared - 2.0) : 0.0) + drain) / tc_balance_threshold(), true, 0);
+        for (int64_t s = 2; s * tiles <= G && s <= kblocks; s++) {
+            const int64_t kper = (kblocks + s - 1) / s;
+            if ((kblocks + kper - 1) / kper == s) offer((double)kper * kb + drain + 3.0 + (double)s * (double)M * N * 8.0 / 4e6, false, (int)kper);
+        }
     }
     return best;
 }
@@ -1966,10 +2005,9 @@ static FwdPlan fwd_plan(int64_t M, int N, int64_t kblocks)
 static int64_t fwd_stats_rows(int64_t M, int N, int64_t kblocks, bool may_balance, bool* by_cta)
 {
     const int G = tc_sm_count();
-    const int BN = N <= 64 ? 64 : 128;
-    const int64_t nt = (N + BN - 1) / BN, tiles = ((M + 127) / 128) * nt;
+    const FwdPlan plan = fwd_plan(M, N, kblocks, may_balance);
+    const int64_t nt = (N + plan.bn - 1) / plan.bn, tiles = ((M + 127) / 128) * nt;
     const int64_t grid = tiles < G ? tiles : G;
-    const FwdPlan plan = may_balance ? fwd_plan(M, N, kblocks) : FwdPlan{false, 0};
     const bool cta = nt <= grid && !plan.sk && !plan.kper;
     if (by_cta) *by_cta = cta;
     return cta ? (grid / nt) * 4 : (M + 31) / 32;
@@ -2015,21 +2053,14 @@ static int run_fwd(const FwdLaunch& f, const void* act, const void* w, PrepParam
     if (((uintptr_t)act & 15) || ((uintptr_t)out & 15)) return B2C_ERR_MISALIGNED;
     float* w_hi = (float*)base;
     float* w_lo = (float*)(base + fbytes);
-    const int BN = f.N <= 64 ? 64 : 128;
-    int sk = 0, kper = 0;
     int* sk_flags = (int*)(base + 2 * fbytes);
     float* sk_partial = (float*)((uintptr_t)sk_flags + sk_flag_bytes());
     // hand-over flags: in the library's self-cleaning bank when this stream has one, else cleared in the workspace
     unsigned int* sk_bank = tc_sm_count() * 4 <= TC_SYNC_FLAGS ? tc_sync_bank(st) : nullptr;
     if (sk_bank) sk_flags = (int*)sk_bank;
-    {
-        const int64_t kblocks = (int64_t)f.kh * f.kw * cblocks;
-        const bool room = base + 2 * fbytes + sk_bytes() <= (uintptr_t)ws + ws_bytes;
-        if (!filters_ready && room && !zf) {
-            const FwdPlan plan = fwd_plan((int64_t)f.n * f.P * f.Q, f.N, kblocks);
-            sk = plan.sk; kper = plan.kper;
-        }
-    }
+    const bool room = base + 2 * fbytes + sk_bytes() <= (uintptr_t)ws + ws_bytes;
+    const FwdPlan plan = fwd_plan((int64_t)f.n * f.P * f.Q, f.N, (int64_t)f.kh * f.kw * cblocks, !filters_ready && room && !zf);
+    const int BN = plan.bn, sk = plan.sk, kper = plan.kper;
     // The filter itself serves as the B operand when its layout allows a tensor map over it (the channel axis
     // that is contiguous decides K-major or MN-major); otherwise hi/lo copies in the GEMM layout are written first.
     // Splitting the B tile in shared memory costs a long launch about 4 % (measured on a 0.9 ms layer), the split
@@ -2106,6 +2137,8 @@ static int run_fwd(const FwdLaunch& f, const void* act, const void* w, PrepParam
                     p.bias, p.mean, p.inv_std, p.gamma, p.beta, relu, stats ? stats->sums : nullptr};
     const dim3 fgrid((p.N + 127) / 128, stats ? (p.M + 31) / 32 : (p.M + 7) / 8);
     if (stats) launch_pdl(tc_split_finish_kernel<4>, fgrid, 256, 0, st, fp);
+    else if (splits >= 8 && (int64_t)p.M * ((p.N + 127) / 128) <= 8 * (int64_t)tc_sm_count())      // the other kernel would not fill the chip
+        launch_pdl(tc_split_finish_deep_kernel, dim3((p.N + 127) / 128, p.M), 256, 0, st, fp);
     else launch_pdl(tc_split_finish_kernel<1>, fgrid, 256, 0, st, fp);
     return check_launch("tc_split_finish_kernel");
 }
@@ -2201,7 +2234,8 @@ static int tc_dgrad_classes_one_launch(const Geo& g, const WStride& wsd, const v
     // the filter as the B operand, in place (see run_fwd): rows = ci (GEMM N), contraction channel = co
     const int64_t s_row = wsd.sc, s_c = wsd.sk, s_r = wsd.sr, s_s = wsd.ss;
     if (s_r != (int64_t)g.kw * s_s || (s_s * 4) % 16) return 1;
-    const int BN = g.ci <= 64 ? 64 : 128;
+    // narrow tiles where the wide ones would leave half of the chip idle (see fwd_plan)
+    const int BN = g.ci <= 64 || ((int64_t)g.n * g.h * g.w + 127) / 128 * ((g.ci + 127) / 128) * 2 <= tc_sm_count() ? 64 : 128;
     const uint64_t taps = (uint64_t)g.kh * g.kw;
     CUtensorMap mb;
     int bsrc;
@@ -2382,13 +2416,14 @@ static int tc_wgrad_nhwc(const Geo& g, const void* x, const void* dy, void* dw, 
     }
     int rc = dispatch_wgrad(pl.bn, ma, mb, mo, p, pl.splits, st);
     if (rc) return rc;
-    WgradReduceParams rp{Krows, g.co, low ? g.ci : Cp, g.kw, pl.splits, wsd.sk, wsd.sc, wsd.sr, wsd.ss, low ? (int)g.K : Krows, g.ci, Np};
+    WgradReduceParams rp{Krows, g.co, low ? g.ci : Cp, g.kw, pl.splits, wsd.sk, wsd.sc, wsd.sr, wsd.ss, low ? (int)g.K : Krows, g.ci, Np, pl.splits * 4};
+    const int db_row = db ? 1 : 0;
     if ((int64_t)((g.co + 31) / 32) * ((Krows + 31) / 32) >= 2 * (int64_t)tc_sm_count())
-        launch_pdl(tc_wgrad_reduce_kernel<4>, dim3((g.co + 31) / 32, (Krows + 31) / 32), dim3(32, 8), 0, st, rp, partial, (float*)dw, p.db_partial, (float*)db);
+        launch_pdl(tc_wgrad_reduce_kernel<4>, dim3((g.co + 31) / 32, (Krows + 31) / 32 + db_row), dim3(32, 8), 0, st, rp, partial, (float*)dw, p.db_partial, (float*)db);
     else if ((int64_t)((g.co + 31) / 32) * ((Krows + 7) / 8) >= 2 * (int64_t)tc_sm_count() || pl.splits < 16)
-        launch_pdl(tc_wgrad_reduce_kernel<1>, dim3((g.co + 31) / 32, (Krows + 7) / 8), dim3(32, 8), 0, st, rp, partial, (float*)dw, p.db_partial, (float*)db);
+        launch_pdl(tc_wgrad_reduce_kernel<1>, dim3((g.co + 31) / 32, (Krows + 7) / 8 + db_row), dim3(32, 8), 0, st, rp, partial, (float*)dw, p.db_partial, (float*)db);
     else
-        launch_pdl(tc_wgrad_reduce_deep_kernel, dim3((g.co + 31) / 32, Krows), dim3(32, 8), 0, st, rp, partial, (float*)dw, p.db_partial, (float*)db);
+        launch_pdl(tc_wgrad_reduce_deep_kernel, dim3((g.co + 31) / 32, Krows + db_row), dim3(32, 8), 0, st, rp, partial, (float*)dw, p.db_partial, (float*)db);
     return check_launch("tc_wgrad_reduce_kernel");
 }
 
