@@ -107,12 +107,6 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
     }
 }
 
-// The wait of a converged warp: one vote when the phase is already complete, which is the usual case in a running pipeline.
-__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
-    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
-    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status, code));
-}
-
 // Position in a ring of N stages.  `phase` is the parity of the current round: a consumer waits with it, a producer with the
 // other one (which a barrier nothing has completed yet reports as done, so the first round does not wait).  The warp
 // roles step through k-blocks with counters like this one and not with divisions: a role's bookkeeping per k-block is
@@ -454,6 +448,7 @@ struct TcParams {
     int splits;                // WGRAD: pixel ranges (1 for FWD)
     // FWD epilogue
     const float *bias, *mean, *inv_std, *gamma, *beta;
+    const float* addend;       // FWD, dense rows: added to the batch-normalised value before the ReLU (a residual sum), or null
     int relu;
     float* out;                // FWD: row m=(n,i,j) at out + n*o_sn + i*o_sh + j*o_sw.  WGRAD: partial [split][M][N]
     int64_t o_sn, o_sh, o_sw;
@@ -498,12 +493,12 @@ struct TcParams {
 
 // Per-channel epilogue steps of the forward pass, decided once on the host so the drain warps branch on
 // one register instead of testing three pointers per element.
-enum { TC_EPI_BIAS = 1, TC_EPI_BN = 2, TC_EPI_RELU = 4, TC_EPI_VEC = 8 };
+enum { TC_EPI_BIAS = 1, TC_EPI_BN = 2, TC_EPI_RELU = 4, TC_EPI_VEC = 8, TC_EPI_ADD = 16 };
 
 // bias / BN-scale / ReLU on the 32 accumulators a[0..31] of one output row, channels nbase..nbase+31.
 // The per-channel vectors are read at warp-uniform addresses (every lane owns a different row of the
 // same channels); with TC_EPI_VEC (all vectors 16-byte aligned, N a multiple of 4) four channels per load.
-__device__ __forceinline__ void tc_epilogue_math(const TcParams& p, int nbase, float* a)
+__device__ __forceinline__ void tc_epilogue_math(const TcParams& p, int nbase, float* a, int m)
 {
     if (p.epi & TC_EPI_VEC) {
         if (p.epi & TC_EPI_BIAS) {
@@ -542,6 +537,17 @@ __device__ __forceinline__ void tc_epilogue_math(const TcParams& p, int nbase, f
                     const float t = (a[j] - __ldg(p.mean + nbase + j)) * __ldg(p.inv_std + nbase + j);
                     a[j] = t * __ldg(p.gamma + nbase + j) + __ldg(p.beta + nbase + j);
                 }
+        }
+    }
+    if ((p.epi & TC_EPI_ADD) && m < p.M) {
+        const float* src = p.addend + (int64_t)m * p.o_sw + nbase;       // 16-byte aligned: o_sw and the channel count are multiples of 4
+        float4 q[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) q[j] = nbase + 4 * j < p.N ? __ldg(reinterpret_cast<const float4*>(src) + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            a[4 * j] = __fadd_rn(a[4 * j], q[j].x); a[4 * j + 1] = __fadd_rn(a[4 * j + 1], q[j].y);
+            a[4 * j + 2] = __fadd_rn(a[4 * j + 2], q[j].z); a[4 * j + 3] = __fadd_rn(a[4 * j + 3], q[j].w);
         }
     }
     if (p.epi & TC_EPI_RELU) {
@@ -708,15 +714,15 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
 
     if (warp == 0) {
         // ---------------- TMA producer ----------------
-        // The warp stays converged (every lane waits and computes the same coordinates); one elected lane arms
-        // the barrier and issues the boxes of the k-block.
+        // One elected lane runs the whole loop: it arms the barrier and issues the boxes of each k-block.
+        if (elect_one_sync()) {
         Ring<STAGES> ring;
         bool ok = true;
         if (RESKB) {
             // The grid is a multiple of the column-tile count: this CTA only meets column tile blockIdx.x % nt, whose
             // filter tiles (all k-blocks) are fetched once.
             const int n0r = (int)(blockIdx.x % nt) * BN;
-            if (elect_one_sync()) {
+            {
                 mbar_expect_tx(bres_bar, (uint32_t)(p.kblocks * L::B_BYTES));
                 for (int kb = 0; kb < p.kblocks; kb++) {
                     const int tap = kb / p.cblocks, cb = kb - tap * p.cblocks;
@@ -732,7 +738,6 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                     }
                 }
             }
-            __syncwarp();
         }
         TileWalk w;
         w.init(total_tiles, p.kblocks, MODE == TCM_FWD && !SK && !MULTI && RESKB == 0 ? p.kper : 0, mt * nt);
@@ -792,12 +797,12 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 TC_PROF_T0();
                 // a stage is free when the MMAs that read it have completed; with resident filters, as soon as the
                 // transform warps have copied its A tile to tensor memory
-                const bool good = mbar_wait_warp(RESKB ? &afree_bar[s] : &empty_bar[s], ring.phase ^ 1, abort_flag, &g_tc_status, TC_ERR_EMPTY);
-                if (lane == 0) TC_PROF_ADD(0);    // producer: waiting for a free stage
+                const bool good = mbar_wait(RESKB ? &afree_bar[s] : &empty_bar[s], ring.phase ^ 1, abort_flag, &g_tc_status, TC_ERR_EMPTY);
+                TC_PROF_ADD(0);    // producer: waiting for a free stage
                 if (!good) { ok = false; break; }
                 uint8_t* st = smem + s * L::STAGE_BYTES;
                 if (MODE == TCM_FWD) {
-                    if (elect_one_sync()) {
+                    {
 #ifdef B2C_TC_DEV
                         if (p.dbg & 64) mbar_arrive(&full_bar[s]);
                         else
@@ -828,7 +833,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                     }
                 } else {
                     const int cw = q0 * p.str_w + p.low_w, chh = p0 * p.str_h + p.low_h;
-                    if (elect_one_sync()) {
+                    {
 #ifdef B2C_TC_DEV
                         if (p.dbg & 64) mbar_arrive(&full_bar[s]);
                         else
@@ -852,10 +857,11 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                     im += im_step;
                 }
                 ring.next();
-                __syncwarp();
-                if (lane == 0) TC_PROF_ADD(14);   // producer: TMA issue
+                TC_PROF_ADD(14);   // producer: TMA issue
             }
         }
+        }
+        __syncwarp();
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
         // One elected lane runs the whole loop.  The tensor core takes about two MMAs ahead of the one it executes (measured:
@@ -943,6 +949,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 else issue_tile(std::false_type{});
             }
         }
+        __syncwarp();
     } else if (warp < 6) {
         // ---------------- operand transform: a = hi + lo ----------------
         // hi = a with the low 13 mantissa bits cleared (what the tensor core reads of a float32 anyway),
@@ -1028,13 +1035,14 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
 #pragma unroll
                     for (int i = 0; i < B_VEC; i++) bq[i] = b_hi[t + i * 128];
                 }
+                const uint32_t slot = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(L::TMEM_A_COL + ts * 64);
+                tmem_st_32x32(slot, v);              // hi: the tensor core reads the upper 19 bits
                 if (RESKB) {
-                    // the A tile is in registers: the producer may refill the stage
+                    // The store above took every lane's values from its registers, so the reads of the stage are done (a load
+                    // that is merely issued is not: a fast producer overwrote rows of the tile) and the producer may refill it.
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&afree_bar[s]);
                 }
-                const uint32_t slot = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(L::TMEM_A_COL + ts * 64);
-                tmem_st_32x32(slot, v);              // hi: the tensor core reads the upper 19 bits
 #pragma unroll
                 for (int j = 0; j < 32; j++) v[j] = __float_as_uint(__uint_as_float(v[j]) - __uint_as_float(v[j] & 0xFFFFE000u));
                 tmem_st_32x32(slot + 32, v);
@@ -1112,7 +1120,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             TC_PROF_T0();
             auto emit_slab = [&](float* a, int cc, int i) {      // slab cc of the tile, number i of this warp's slabs
                 uint8_t* buf = ebuf + (ecount % SLABS) * 4096;
-                if (MODE == TCM_FWD && p.epi) tc_epilogue_math(p, n0 + cc * 32, a);
+                if (MODE == TCM_FWD && p.epi) tc_epilogue_math(p, n0 + cc * 32, a, m0 + quad * 32 + lane);
                 if (threadIdx.x == 192) TC_PROF_ADD(8);     // drain: tensor-memory loads, adds, epilogue arithmetic
                 if (lane == 0) tma_store_wait_read<SLABS - 1>();     // the store that last read this slab is done
                 __syncwarp();
@@ -1313,7 +1321,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
 #pragma unroll
                 for (int cc = 0; cc < BN / 32; cc++) {
                     if (n0 + cc * 32 < p.N) {
-                        if (MODE == TCM_FWD && p.epi) tc_epilogue_math(p, n0 + cc * 32, &acc[cc * 32]);
+                        if (MODE == TCM_FWD && p.epi) tc_epilogue_math(p, n0 + cc * 32, &acc[cc * 32], m);
 #pragma unroll
                         for (int j = 0; j < 32; j += 4)
                             *reinterpret_cast<float4*>(stage + lane * 36 + j) =
@@ -1369,7 +1377,7 @@ struct FinishParams {
     const float* partial;
     float* out;
     int64_t o_sn, o_sh, o_sw;
-    const float *bias, *mean, *inv_std, *gamma, *beta;
+    const float *bias, *mean, *inv_std, *gamma, *beta, *addend;
     int relu;
     float* stats;
 };
@@ -1409,8 +1417,14 @@ __global__ void __launch_bounds__(256) tc_split_finish_kernel(FinishParams p)
                 if (e < cnt) {
                     if (p.bias) a[e] += __ldg(p.bias + n0 + e);
                     if (p.mean) { const float t = (a[e] - __ldg(p.mean + n0 + e)) * __ldg(p.inv_std + n0 + e); a[e] = t * __ldg(p.gamma + n0 + e) + __ldg(p.beta + n0 + e); }
-                    if (p.relu) a[e] = fmaxf(a[e], 0.f);
                 }
+            if (p.addend) {                    // dense rows, a multiple of four channels
+                const float4 q = __ldg(reinterpret_cast<const float4*>(p.addend + (int64_t)m * p.o_sw + n0));
+                a[0] = __fadd_rn(a[0], q.x); a[1] = __fadd_rn(a[1], q.y); a[2] = __fadd_rn(a[2], q.z); a[3] = __fadd_rn(a[3], q.w);
+            }
+            if (p.relu)
+#pragma unroll
+                for (int e = 0; e < 4; e++) a[e] = fmaxf(a[e], 0.f);
             const int img = m / (p.P * p.Q), rem = m - img * (p.P * p.Q), pi = rem / p.Q, qi = rem - pi * p.Q;
             float* d = p.out + img * p.o_sn + pi * p.o_sh + qi * p.o_sw + n0;
             if (vec) *reinterpret_cast<float4*>(d) = make_float4(a[0], a[1], a[2], a[3]);
@@ -1467,6 +1481,7 @@ __global__ void __launch_bounds__(256) tc_split_finish_deep_kernel(FinishParams 
         if (e < cnt) {
             if (p.bias) a[e] += __ldg(p.bias + n0 + e);
             if (p.mean) { const float t = (a[e] - __ldg(p.mean + n0 + e)) * __ldg(p.inv_std + n0 + e); a[e] = t * __ldg(p.gamma + n0 + e) + __ldg(p.beta + n0 + e); }
+            if (p.addend) a[e] = __fadd_rn(a[e], __ldg(p.addend + (int64_t)m * p.o_sw + n0 + e));
             if (p.relu) a[e] = fmaxf(a[e], 0.f);
             d[e] = a[e];
         }
@@ -2041,11 +2056,13 @@ struct FwdLaunch {
 
 static int run_fwd(const FwdLaunch& f, const void* act, const void* w, PrepParams pp, const void* bias,
                    const b2c_bn_params* bn, int relu, float* out, void* ws, size_t ws_bytes, cudaStream_t st,
-                   bool filters_ready = false, const StatsOut* stats = nullptr, const ZeroFill* zf = nullptr)
+                   bool filters_ready = false, const StatsOut* stats = nullptr, const ZeroFill* zf = nullptr, const float* addend = nullptr)
 {
     if (!load_driver_entry_points()) return B2C_ERR_UNSUPPORTED;
     const int cblocks = (f.C + 31) / 32;
     pp.Cp = cblocks * 32;
+    // the tap strides of a filter with one tap mean nothing: a (co, ci, 1, 1) filter is a (co, 1, 1, ci) one
+    if (pp.Rreal * pp.Sreal == 1) pp.s_s = pp.s_r = pp.s_row > pp.s_c ? pp.s_row : pp.s_c;
     const int64_t K = (int64_t)f.kh * f.kw * pp.Cp;
     const size_t fbytes = align_up((size_t)f.N * K * sizeof(float), 1024);
     uintptr_t base = align_up((uintptr_t)ws, 1024);
@@ -2101,7 +2118,8 @@ static int run_fwd(const FwdLaunch& f, const void* act, const void* w, PrepParam
     p.bias = (const float*)bias;
     if (bn) { p.mean = (const float*)bn->mean; p.inv_std = (const float*)bn->inv_std; p.gamma = (const float*)bn->gamma; p.beta = (const float*)bn->beta; }
     p.relu = relu;
-    p.epi = (p.bias ? TC_EPI_BIAS : 0) | (p.mean ? TC_EPI_BN : 0) | (relu ? TC_EPI_RELU : 0);
+    p.addend = addend;
+    p.epi = (addend ? TC_EPI_ADD : 0) | (p.bias ? TC_EPI_BIAS : 0) | (p.mean ? TC_EPI_BN : 0) | (relu ? TC_EPI_RELU : 0);
     if (f.N % 4 == 0 && !(((uintptr_t)p.bias | (uintptr_t)p.mean | (uintptr_t)p.inv_std | (uintptr_t)p.gamma | (uintptr_t)p.beta) & 15))
         p.epi |= TC_EPI_VEC;
     p.out = out; p.o_sn = f.o_sn; p.o_sh = f.o_sh; p.o_sw = f.o_sw;
@@ -2117,6 +2135,7 @@ static int run_fwd(const FwdLaunch& f, const void* act, const void* w, PrepParam
         if (!make_map_out(&mo, sk_partial, 0, (uint64_t)(splits * mrows), (uint64_t)round4(f.N), (uint64_t)round4(f.N))) return B2C_ERR_UNSUPPORTED;
         p.tma_store = 1; p.kper = kper; p.epi = 0;
     } else if (dense && make_map_out(&mo, out, 0, (uint64_t)p.M, (uint64_t)f.N, (uint64_t)f.o_sw)) p.tma_store = 1;
+    if (addend && (!dense || f.N % 4 || ((uintptr_t)addend & 15))) return B2C_ERR_UNSUPPORTED;
     if (zf) {
         if (p.tma_store || ((zf->off_w | zf->off_h) & 3)) return B2C_ERR_UNSUPPORTED;
         p.zfill = 1; p.z_W = zf->W; p.z_H = zf->H; p.z_w = zf->off_w; p.z_h = zf->off_h;
@@ -2134,7 +2153,7 @@ static int run_fwd(const FwdLaunch& f, const void* act, const void* w, PrepParam
                  : dispatch_fwd<TCB_SPLIT>(BN, ma, mbh, mbl, mo, p, st);
     if (rc || !kper) return rc;
     FinishParams fp{p.M, p.N, p.P, p.Q, splits, round4(f.N), mrows * round4(f.N), sk_partial, out, f.o_sn, f.o_sh, f.o_sw,
-                    p.bias, p.mean, p.inv_std, p.gamma, p.beta, relu, stats ? stats->sums : nullptr};
+                    p.bias, p.mean, p.inv_std, p.gamma, p.beta, addend, relu, stats ? stats->sums : nullptr};
     const dim3 fgrid((p.N + 127) / 128, stats ? (p.M + 31) / 32 : (p.M + 7) / 8);
     if (stats) launch_pdl(tc_split_finish_kernel<4>, fgrid, 256, 0, st, fp);
     else if (splits >= 8 && (int64_t)p.M * ((p.N + 127) / 128) <= 8 * (int64_t)tc_sm_count())      // the other kernel would not fill the chip
@@ -2175,7 +2194,7 @@ static int launch_lower(const Geo& g, const void* x, float* rows, cudaStream_t s
 }
 
 static int tc_fprop_nhwc(const Geo& g, const void* x, const void* w, const void* bias, const b2c_bn_params* bn, int relu,
-             void* y, void* ws, size_t ws_bytes, cudaStream_t st, const StatsOut* stats = nullptr)
+             void* y, void* ws, size_t ws_bytes, cudaStream_t st, const StatsOut* stats = nullptr, const float* addend = nullptr)
 {
     WStride wsd = w_stride(g.w_layout, g.ci, g.co, g.kh, g.kw);
     const int64_t yp = g.yp;
@@ -2198,13 +2217,13 @@ static int tc_fprop_nhwc(const Geo& g, const void* x, const void* w, const void*
         if (rc) return rc;
         PrepParams none{};
         FwdLaunch f{g.n, g.ho, g.wo, Kp, Kp, g.ho, g.wo, g.co, 1, 1, 0, 0, g.ho, g.wo, 1, 1, 1, 1, g.ho * g.wo * yp, g.wo * yp, yp};
-        return run_fwd(f, rows, nullptr, none, bias, bn, relu, (float*)y, (void*)w_hi, 2 * fbytes + 1024, st, true, stats);
+        return run_fwd(f, rows, nullptr, none, bias, bn, relu, (float*)y, (void*)w_hi, 2 * fbytes + 1024, st, true, stats, nullptr, addend);
     }
     PrepParams pp{g.co, g.ci, g.kh, g.kw, wsd.sk, wsd.sc, wsd.sr, wsd.ss, 0, 1, 0, 1, g.kh, g.kw};
     FwdLaunch f{g.n, g.h, g.w, g.ci, g.xp, g.ho, g.wo, g.co, g.kh, g.kw, -g.vpad, -g.hpad,
                 g.h + 2 * g.vpad - (g.kh - 1) * g.vdil, g.w + 2 * g.hpad - (g.kw - 1) * g.hdil,
                 g.vstr, g.hstr, g.vdil, g.hdil, g.ho * g.wo * yp, g.wo * yp, yp};
-    return run_fwd(f, x, w, pp, bias, bn, relu, (float*)y, ws, ws_bytes, st, false, stats);
+    return run_fwd(f, x, w, pp, bias, bn, relu, (float*)y, ws, ws_bytes, st, false, stats, nullptr, addend);
 }
 
 // Strided data gradient, all parity classes in one launch (MULTI kernel variants): up to four classes, every class
@@ -2711,6 +2730,18 @@ int tc_fprop(const Geo& g, const void* x, const void* w, const void* bias, const
              void* y, void* ws, size_t ws_bytes, cudaStream_t st)
 {
     return tc_fprop_any(g, x, w, bias, bn, relu, y, ws, ws_bytes, st, nullptr);
+}
+
+// y = relu?(bn?(conv + bias) + addend) where the kernels write y itself (no copies) in whole 16-byte pixels.
+bool tc_takes_addend(const Geo& g)
+{
+    const Copies c = tc_copies(g, B2C_PASS_FPROP);
+    return g.layout == B2C_LAYOUT_NHWC && !c.x && !c.y && g.co % 4 == 0;
+}
+int tc_fprop_residual(const Geo& g, const void* x, const void* w, const void* bias, const b2c_bn_params* bn, const void* addend, int relu,
+                      void* y, void* ws, size_t ws_bytes, cudaStream_t st)
+{
+    return tc_fprop_nhwc(g, x, w, bias, bn, relu, y, ws, ws_bytes, st, nullptr, (const float*)addend);
 }
 
 int tc_dgrad(const Geo& g, const void* dy, const void* w, void* dx, void* ws, size_t ws_bytes, cudaStream_t st)
