@@ -100,15 +100,6 @@ int b2c_conv_fprop(const b2c_conv_desc *desc, const void *x, const void *w, cons
                    const b2c_bn_params *bn, int relu, void *y,
                    void *workspace, size_t workspace_bytes, void *stream);
 
-/* The same with a residual sum: y = relu?( bn?(conv(x, w) + bias) + addend ), addend and y of the same shape (and not the
- * same buffer), the sum taken on the rounded batch-norm output exactly as a separate add kernel would take it.  For the
- * convolution that ends a residual branch in evaluation (pydtnn/backends/gpu/layers/addition_block_gpu.py:49-66).
- * b2c_conv_takes_addend(desc) says whether the layer's path can (1) or not (0; the call then returns B2C_ERR_UNSUPPORTED). */
-int b2c_conv_takes_addend(const b2c_conv_desc *desc);
-int b2c_conv_fprop_residual(const b2c_conv_desc *desc, const void *x, const void *w, const void *bias,
-                            const b2c_bn_params *bn, const void *addend, int relu, void *y,
-                            void *workspace, size_t workspace_bytes, void *stream);
-
 /* The forward pass for a convolution that feeds a training-mode batch norm (the Conv2D -> BatchNormalization pairs the
  * reference's fusion flags name, pydtnn/parser.py:74-77; the statistics are those of
  * pydtnn/backends/cpu/layers/batch_normalization_cpu.py:65-70): y = conv(x, w) + bias as b2c_conv_fprop writes it, and

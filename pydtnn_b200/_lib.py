@@ -45,9 +45,6 @@ PROTOTYPES = {
     "b2c_conv_engine_for": (c_int, [POINTER(ConvDesc), c_int]),
     "b2c_conv_fprop": (c_int, [POINTER(ConvDesc), c_void_p, c_void_p, c_void_p, POINTER(BnParams), c_int, c_void_p,
                                c_void_p, c_size_t, c_void_p]),
-    "b2c_conv_takes_addend": (c_int, [POINTER(ConvDesc)]),
-    "b2c_conv_fprop_residual": (c_int, [POINTER(ConvDesc), c_void_p, c_void_p, c_void_p, POINTER(BnParams), c_void_p, c_int, c_void_p,
-                                        c_void_p, c_size_t, c_void_p]),
     "b2c_conv_stats_bytes": (c_size_t, [POINTER(ConvDesc)]),
     "b2c_conv_fprop_stats": (c_int, [POINTER(ConvDesc), c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_size_t,
                                      c_void_p, c_size_t, c_void_p]),

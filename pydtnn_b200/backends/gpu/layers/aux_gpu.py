@@ -2,8 +2,6 @@
 AdditionBlock, Flatten, Dropout(identity in evaluation).  Each mirrors the attributes and hook
 behaviour of its reference counterpart under pydtnn/backends/gpu/{layers,activations}/ with the
 cuDNN call replaced by a call through the C ABI."""
-import ctypes
-
 import numpy as np
 
 from .... import _lib
@@ -332,17 +330,12 @@ class AdditionBlockGPU(LayerGPU, AdditionBlock):
         self.relu_before = None          # set by the model: the Relu layer whose output is this block's input
 
     def _fold_sum_into_last_bn(self):
-        """Two branches, the block feeds a ReLU and the first branch ends in a plain batch norm (evaluation: a fused
-        convolution + batch norm): that layer can add the other branch and apply the ReLU while it writes (one pass less over the block's
+        """Training step, two branches, the block feeds a ReLU and the first branch ends in a plain batch norm:
+        that batch norm can add the other branch and apply the ReLU while it writes (one pass less over the block's
         largest tensors, and the batch-norm output itself is never stored)."""
-        if self.relu_after is None or len(self.paths) != 2 or not self.fold_sum:
+        if self.model.mode != TRAIN_MODE or self.relu_after is None or len(self.paths) != 2 or not self.fold_sum:
             return None
         bn = self.paths[0][-1]
-        if self.model.mode != TRAIN_MODE:
-            # evaluation: a convolution with the batch norm folded in and no ReLU of its own takes the sum the same way
-            conv = type(bn).__name__ == "Conv2DBatchNormalizationGPU" and not bn._relu_flag() \
-                and _lib.lib().b2c_conv_takes_addend(ctypes.byref(bn.desc))
-            return bn if conv else None
         if type(bn).__name__ != "BatchNormalizationGPU" or bn.fuse_relu:
             return None
         return bn

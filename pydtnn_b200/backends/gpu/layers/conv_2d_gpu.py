@@ -170,7 +170,6 @@ class _FusedConvInference(Conv2DGPU):
     (pydtnn/backends/cpu/layers/conv_2d_batch_normalization_relu_cpu.py:47-48, 96-97)."""
     _with_bn = False
     _with_relu = False
-    residual = None                      # (other branch, output) while an addition block folds its sum + ReLU in here
 
     def __init__(self, *args, from_parent=None, from_parent_2=None, **kwargs):
         if from_parent is None:
@@ -201,15 +200,6 @@ class _FusedConvInference(Conv2DGPU):
             self._refresh_bn()
         L = _lib.lib()
         x_ptr = self._in(x, "x")
-        if self.residual is not None:
-            # last layer of a residual branch: the block's sum and the ReLU after it, written to that ReLU's output
-            addend, out = self.residual
-            self._timed("fprop", lambda: L.b2c_conv_fprop_residual(
-                ctypes.byref(self.desc), x_ptr, self.weights.ptr, self.biases.ptr if self.use_bias else None,
-                ctypes.byref(self._bn) if self._with_bn else None, self._in(addend, "addend"), 1,
-                out.out, wsp.ptr(), wsp.size(), self.model.stream_handle))
-            out.written()
-            return out
         self._timed("fprop", lambda: L.b2c_conv_fprop(
             ctypes.byref(self.desc), x_ptr, self.weights.ptr, self.biases.ptr if self.use_bias else None,
             ctypes.byref(self._bn) if self._with_bn else None, int(self._relu_flag()),

@@ -112,22 +112,6 @@ extern "C" int b2c_conv_fprop(const b2c_conv_desc* desc, const void* x, const vo
     return fma_fprop(g, x, w, bias, bn, relu, y, ws, ws_bytes, (cudaStream_t)stream);
 }
 
-extern "C" int b2c_conv_takes_addend(const b2c_conv_desc* desc) {
-    Geo g; if (make_geo(desc, g)) return 0;
-    int e; if (pick_engine(g, B2C_PASS_FPROP, e) || e != B2C_ENGINE_TENSOR) return 0;
-    return tc_takes_addend(g) ? 1 : 0;
-}
-
-extern "C" int b2c_conv_fprop_residual(const b2c_conv_desc* desc, const void* x, const void* w, const void* bias, const b2c_bn_params* bn,
-                                       const void* addend, int relu, void* y, void* ws, size_t ws_bytes, void* stream) {
-    Geo g; int rc = make_geo(desc, g); if (rc) return rc;
-    if (!x || !w || !y || !addend) return B2C_ERR_NULL_POINTER;
-    if (bn && (!bn->mean || !bn->inv_std || !bn->gamma || !bn->beta)) return B2C_ERR_NULL_POINTER;
-    int e; rc = call_engine(g, B2C_PASS_FPROP, x, y, e); if (rc) return rc;
-    if (e != B2C_ENGINE_TENSOR || !tc_takes_addend(g)) return B2C_ERR_UNSUPPORTED;
-    return tc_fprop_residual(g, x, w, bias, bn, addend, relu, y, ws, ws_bytes, (cudaStream_t)stream);
-}
-
 extern "C" size_t b2c_conv_stats_bytes(const b2c_conv_desc* desc) {
     Geo g; if (make_geo(desc, g)) return 0;
     if (g.dtype != B2C_F32) return 0;

@@ -120,9 +120,6 @@ int tc_wait_selftest(long long limit_cycles, cudaStream_t st);
 size_t tc_workspace_bytes(const Geo& g, int pass);
 int tc_fprop(const Geo& g, const void* x, const void* w, const void* bias, const b2c_bn_params* bn, int relu,
              void* y, void* ws, size_t ws_bytes, cudaStream_t st);
-bool tc_takes_addend(const Geo& g);
-int tc_fprop_residual(const Geo& g, const void* x, const void* w, const void* bias, const b2c_bn_params* bn, const void* addend, int relu,
-                      void* y, void* ws, size_t ws_bytes, cudaStream_t st);
 int tc_dgrad(const Geo& g, const void* dy, const void* w, void* dx, void* ws, size_t ws_bytes, cudaStream_t st);
 int tc_wgrad(const Geo& g, const void* x, const void* dy, void* dw, void* db, void* ws, size_t ws_bytes,
              cudaStream_t st);

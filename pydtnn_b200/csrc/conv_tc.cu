@@ -432,6 +432,21 @@ enum { TCB_SPLIT = 0, TCB_RAW_K = 1, TCB_RAW_MN = 2 };
 
 #define TC_CHUNK 8   // k-blocks accumulated in tensor memory before the partial sum is drained
 
+// Division by a launch constant: q = (n * mul) >> 32 >> shift for 0 <= n < 2^31 (round-up reciprocal: with s = ceil(log2 d) and
+// mul = ceil(2^(32 + s - 1) / d) the error stays below 1 / d for 31-bit n).  A role's start-up and each new tile took half a
+// dozen integer divisions, 0.3 us before a launch's first load.
+struct FastDiv {
+    uint32_t d, mul; int shift;
+    FastDiv() = default;
+    __host__ explicit FastDiv(uint32_t d_) : d(d_) {
+        int s = 0;
+        while ((1ull << s) < d_) s++;
+        shift = s - 1;
+        mul = d_ == 1 ? 0 : (uint32_t)(((1ull << (31 + s)) + d_ - 1) / d_);
+    }
+    __device__ __forceinline__ int div(int n) const { return d == 1 ? n : (int)(__umulhi((uint32_t)n, mul) >> shift); }
+};
+
 struct TcParams {
     // FWD: GEMM rows = output pixels, columns = output channels. WGRAD: rows = (tap, ci), columns = co.
     int M, N;
@@ -448,7 +463,6 @@ struct TcParams {
     int splits;                // WGRAD: pixel ranges (1 for FWD)
     // FWD epilogue
     const float *bias, *mean, *inv_std, *gamma, *beta;
-    const float* addend;       // FWD, dense rows: added to the batch-normalised value before the ReLU (a residual sum), or null
     int relu;
     float* out;                // FWD: row m=(n,i,j) at out + n*o_sn + i*o_sh + j*o_sw.  WGRAD: partial [split][M][N]
     int64_t o_sn, o_sh, o_sw;
@@ -489,16 +503,17 @@ struct TcParams {
     // of all its tiles in registers and `stats` is [(grid / nt) * 4][2][N]: one row per CTA group and row quadrant.
     float* stats;
     int stats_cta;
+    FastDiv f_nt, f_mt, f_plane, f_pq, f_q, f_cb, f_s, f_c;      // column tiles, row tiles, their product, P * Q, Q, cblocks, S, C (launch_tc)
 };
 
 // Per-channel epilogue steps of the forward pass, decided once on the host so the drain warps branch on
 // one register instead of testing three pointers per element.
-enum { TC_EPI_BIAS = 1, TC_EPI_BN = 2, TC_EPI_RELU = 4, TC_EPI_VEC = 8, TC_EPI_ADD = 16 };
+enum { TC_EPI_BIAS = 1, TC_EPI_BN = 2, TC_EPI_RELU = 4, TC_EPI_VEC = 8 };
 
 // bias / BN-scale / ReLU on the 32 accumulators a[0..31] of one output row, channels nbase..nbase+31.
 // The per-channel vectors are read at warp-uniform addresses (every lane owns a different row of the
 // same channels); with TC_EPI_VEC (all vectors 16-byte aligned, N a multiple of 4) four channels per load.
-__device__ __forceinline__ void tc_epilogue_math(const TcParams& p, int nbase, float* a, int m)
+__device__ __forceinline__ void tc_epilogue_math(const TcParams& p, int nbase, float* a)
 {
     if (p.epi & TC_EPI_VEC) {
         if (p.epi & TC_EPI_BIAS) {
@@ -539,17 +554,6 @@ __device__ __forceinline__ void tc_epilogue_math(const TcParams& p, int nbase, f
                 }
         }
     }
-    if ((p.epi & TC_EPI_ADD) && m < p.M) {
-        const float* src = p.addend + (int64_t)m * p.o_sw + nbase;       // 16-byte aligned: o_sw and the channel count are multiples of 4
-        float4 q[8];
-#pragma unroll
-        for (int j = 0; j < 8; j++) q[j] = nbase + 4 * j < p.N ? __ldg(reinterpret_cast<const float4*>(src) + j) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            a[4 * j] = __fadd_rn(a[4 * j], q[j].x); a[4 * j + 1] = __fadd_rn(a[4 * j + 1], q[j].y);
-            a[4 * j + 2] = __fadd_rn(a[4 * j + 2], q[j].z); a[4 * j + 3] = __fadd_rn(a[4 * j + 3], q[j].w);
-        }
-    }
     if (p.epi & TC_EPI_RELU) {
 #pragma unroll
         for (int j = 0; j < 32; j++) a[j] = fmaxf(a[j], 0.f);
@@ -584,10 +588,11 @@ struct TcSmem {
 // [total * b / G, total * (b + 1) / G) of CTA b, unit = tile * kblocks + kb.
 struct TileWalk {
     int tile, kb_b, kb_e;
-    int next_tile, total_tiles, kblocks, kper, plane;
+    int next_tile, total_tiles, kblocks, kper;
+    FastDiv plane;
     long long u, u_end;
     __device__ __forceinline__ static long long range_begin(long long total, int cta, int ctas) { return total * cta / ctas; }
-    __device__ __forceinline__ void init(int total_tiles_, int kblocks_, int kper_, int plane_) {
+    __device__ __forceinline__ void init(int total_tiles_, int kblocks_, int kper_, const FastDiv& plane_) {
         total_tiles = total_tiles_; kblocks = kblocks_; kper = kper_; plane = plane_; next_tile = blockIdx.x;
         const long long total = (long long)total_tiles_ * kblocks_;
         u = range_begin(total, blockIdx.x, gridDim.x); u_end = range_begin(total, blockIdx.x + 1, gridDim.x);
@@ -596,7 +601,7 @@ struct TileWalk {
         if (!BALANCED) {
             if (next_tile >= total_tiles) return false;
             tile = next_tile; next_tile += gridDim.x; kb_b = 0; kb_e = kblocks;
-            if (kper) { kb_b = tile / plane * kper; if (kb_b + kper < kblocks) kb_e = kb_b + kper; }
+            if (kper) { kb_b = plane.div(tile) * kper; if (kb_b + kper < kblocks) kb_e = kb_b + kper; }
             return true;
         }
         if (u >= u_end) return false;
@@ -721,12 +726,12 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         if (RESKB) {
             // The grid is a multiple of the column-tile count: this CTA only meets column tile blockIdx.x % nt, whose
             // filter tiles (all k-blocks) are fetched once.
-            const int n0r = (int)(blockIdx.x % nt) * BN;
+            const int n0r = ((int)blockIdx.x - p.f_nt.div((int)blockIdx.x) * nt) * BN;
             {
                 mbar_expect_tx(bres_bar, (uint32_t)(p.kblocks * L::B_BYTES));
                 for (int kb = 0; kb < p.kblocks; kb++) {
-                    const int tap = kb / p.cblocks, cb = kb - tap * p.cblocks;
-                    const int r = tap / p.S, sx = tap - r * p.S;
+                    const int tap = p.f_cb.div(kb), cb = kb - tap * p.cblocks;
+                    const int r = p.f_s.div(tap), sx = tap - r * p.S;
                     const int tap_real = (p.tap_r0 + p.tap_rstep * r) * p.tap_sreal + p.tap_s0 + p.tap_sstep * sx;
                     uint8_t* dst = smem + L::RES_OFFSET + kb * 2 * L::B_BYTES;
                     if (BSRC == TCB_RAW_K) {
@@ -740,18 +745,18 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             }
         }
         TileWalk w;
-        w.init(total_tiles, p.kblocks, MODE == TCM_FWD && !SK && !MULTI && RESKB == 0 ? p.kper : 0, mt * nt);
+        w.init(total_tiles, p.kblocks, MODE == TCM_FWD && !SK && !MULTI && RESKB == 0 ? p.kper : 0, p.f_plane);
         while (ok && w.template next<SK>()) {
             const TileGeo tg = tile_geo(w.tile);
             if (MULTI) w.kb_e = tg.kblocks;
             const int tile = tg.ltile;
-            const int ni = tile % nt, rest = tile / nt, mi = MULTI ? rest : rest % mt, z = MULTI ? 0 : rest / mt;
+            const int rest = p.f_nt.div(tile), ni = tile - rest * nt, z = MULTI ? 0 : p.f_mt.div(rest), mi = rest - z * mt;
             const int m0 = mi * 128, n0 = ni * BN;
             int img = 0, base_w = 0, base_h = 0;
             if (MODE == TCM_FWD) {
-                img = m0 / (tg.P * tg.Q);
+                img = MULTI ? m0 / (tg.P * tg.Q) : p.f_pq.div(m0);
                 const int rem = m0 - img * (tg.P * tg.Q);
-                const int p0 = rem / tg.Q, q0 = rem - p0 * tg.Q;
+                const int p0 = MULTI ? rem / tg.Q : p.f_q.div(rem), q0 = rem - p0 * tg.Q;
                 base_w = q0 * p.str_w + tg.low_w; base_h = p0 * p.str_h + tg.low_h;
             }
             // WGRAD: the tile's boxes are fixed: up to four x boxes (32, 64 or 128 rows of (tap, ci) each: a box stays
@@ -764,9 +769,9 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 for (int j = 0; j < 4; j++) {
                     const int mrow = m0 + a_box * j;
                     if (a_box * j < 128 && mrow < p.M) {
-                        const int tap = mrow / p.C;
+                        const int tap = p.f_c.div(mrow);
                         box_c0[j] = mrow - tap * p.C;
-                        const int r = tap / p.S, sx = tap - r * p.S;
+                        const int r = p.f_s.div(tap), sx = tap - r * p.S;
                         box_offw[j] = sx * p.dil_w; box_offh[j] = r * p.dil_h;
                         tx_bytes += (uint32_t)a_box * 128u;
                     }
@@ -779,18 +784,18 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             int cb = 0, sx = 0, off_w = 0, off_h = 0, tap_real = 0, tap_row = 0, im = 0, p0 = 0, q0 = 0, pix0 = 0;
             int im_step = 0, p_step = 0, q_step = 0;
             if (MODE == TCM_FWD) {
-                const int tap = w.kb_b / p.cblocks;
+                const int tap = p.f_cb.div(w.kb_b);
                 cb = w.kb_b - tap * p.cblocks;
-                const int r = tap / tg.S;
+                const int r = MULTI ? tap / tg.S : p.f_s.div(tap);
                 sx = tap - r * tg.S;
                 off_w = sx * p.dil_w; off_h = r * p.dil_h;
                 tap_row = (tg.r0 + p.tap_rstep * r) * p.tap_sreal + tg.s0; tap_real = tap_row + p.tap_sstep * sx;
             } else {
                 pix0 = (z * p.kblocks + w.kb_b) * 32;
-                im = pix0 / (p.P * p.Q);
+                im = p.f_pq.div(pix0);
                 int rem = pix0 - im * (p.P * p.Q);
-                p0 = rem / p.Q; q0 = rem - p0 * p.Q;
-                im_step = 32 / (p.P * p.Q); rem = 32 - im_step * (p.P * p.Q); p_step = rem / p.Q; q_step = rem - p_step * p.Q;
+                p0 = p.f_q.div(rem); q0 = rem - p0 * p.Q;
+                im_step = p.f_pq.div(32); rem = 32 - im_step * (p.P * p.Q); p_step = p.f_q.div(rem); q_step = rem - p_step * p.Q;
             }
             for (int kb = w.kb_b; kb < w.kb_e; kb++) {
                 const int s = ring.s;
@@ -883,12 +888,12 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             bool ahead = false;                      // the next k-block was seen to be ready
             const uint64_t b_desc0 = make_smem_desc(smem_u32(smem) + (RESKB ? L::RES_OFFSET : L::A_BYTES), LBO, SBO, LAYOUT);
             TileWalk w;
-            w.init(total_tiles, p.kblocks, MODE == TCM_FWD && !SK && !MULTI && RESKB == 0 ? p.kper : 0, mt * nt);
+            w.init(total_tiles, p.kblocks, MODE == TCM_FWD && !SK && !MULTI && RESKB == 0 ? p.kper : 0, p.f_plane);
             while (ok && w.template next<SK>()) {
                 const TileGeo tg = tile_geo(w.tile);
                 if (MULTI) w.kb_e = tg.kblocks;
                 // columns past the last channel are not computed (N of an MMA is a multiple of 16)
-                const int left = p.N - (tg.ltile % nt) * BN;
+                const int left = p.N - (tg.ltile - p.f_nt.div(tg.ltile) * nt) * BN;
                 // and neither are the steps of a last channel block that hold only the zeros past the last channel
                 const uint32_t idesc = make_idesc_tf32(128, left >= BN ? BN : (left + 15) & ~15, 0, B_MN);
                 // The k-blocks of one tile.  WHOLE has operand shape and step count in constants: with them in registers
@@ -987,13 +992,13 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             }
         }
         TileWalk w;
-        w.init(total_tiles, p.kblocks, MODE == TCM_FWD && !SK && !MULTI && RESKB == 0 ? p.kper : 0, mt * nt);
+        w.init(total_tiles, p.kblocks, MODE == TCM_FWD && !SK && !MULTI && RESKB == 0 ? p.kper : 0, p.f_plane);
         while (ok && w.template next<SK>()) {
             if (MULTI) w.kb_e = tile_geo(w.tile).kblocks;
             // WGRAD: the tiles of the first row block also sum their dy tile over the pixels (the bias gradient);
             // a thread meets the same four channels of each 32-channel box in every k-block (see below)
             float4 dbacc[B_VEC / 2 + 1];
-            const bool do_db = MODE == TCM_WGRAD && p.db_partial != nullptr && (w.tile / nt) % mt == 0;
+            const bool do_db = MODE == TCM_WGRAD && p.db_partial != nullptr && (p.f_nt.div(w.tile) - p.f_plane.div(w.tile) * mt) == 0;
 #pragma unroll
             for (int i = 0; i < B_VEC / 2; i++) dbacc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
             for (int kb = w.kb_b; kb < w.kb_e; kb++, ring.next(), slots.next()) {
@@ -1073,7 +1078,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 // chunk ((c >> 1) ^ rr) * 2 + (c & 1) with c = lane & 7, rr = (lane >> 3) & 3: the four lanes that hold
                 // one chunk differ by lane ^ (m << 3 | m << 1), m = 1..3.  After the two exchange steps lanes 0-7
                 // (rr = 0: chunk = c) hold the warp's sums over its 8 pixel rows of every k-block.
-                const int ni = w.tile % nt, z = (w.tile / nt) / mt;
+                const int z = p.f_plane.div(w.tile), ni = w.tile - p.f_nt.div(w.tile) * nt;
 #pragma unroll
                 for (int bx = 0; bx < B_VEC / 2; bx++) {
                     float4 v = dbacc[bx];
@@ -1104,12 +1109,12 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
 #pragma unroll
         for (int i = 0; i < NSLAB; i++) cs0[i] = cs1[i] = 0.f;
         TileWalk w;
-        w.init(total_tiles, p.kblocks, MODE == TCM_FWD && !SK && !MULTI && RESKB == 0 ? p.kper : 0, mt * nt);
+        w.init(total_tiles, p.kblocks, MODE == TCM_FWD && !SK && !MULTI && RESKB == 0 ? p.kper : 0, p.f_plane);
         while (ok && w.template next<SK>()) {
             const TileGeo tg = tile_geo(w.tile);
             if (MULTI) w.kb_e = tg.kblocks;
             const int tile = tg.ltile;
-            const int ni = tile % nt, rest = tile / nt, mi = MULTI ? rest : rest % mt, z = MULTI ? 0 : rest / mt;
+            const int rest = p.f_nt.div(tile), ni = tile - rest * nt, z = MULTI ? 0 : p.f_mt.div(rest), mi = rest - z * mt;
             const int m0 = mi * 128, n0 = ni * BN;
             // One 32-row x 32-column slab of the tile on its way out (dense outputs): epilogue steps, staging in a
             // 128B-swizzled slab (conflict-free float4 writes), TMA store (whole rows, asynchronous, rows >= M and
@@ -1120,7 +1125,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             TC_PROF_T0();
             auto emit_slab = [&](float* a, int cc, int i) {      // slab cc of the tile, number i of this warp's slabs
                 uint8_t* buf = ebuf + (ecount % SLABS) * 4096;
-                if (MODE == TCM_FWD && p.epi) tc_epilogue_math(p, n0 + cc * 32, a, m0 + quad * 32 + lane);
+                if (MODE == TCM_FWD && p.epi) tc_epilogue_math(p, n0 + cc * 32, a);
                 if (threadIdx.x == 192) TC_PROF_ADD(8);     // drain: tensor-memory loads, adds, epilogue arithmetic
                 if (lane == 0) tma_store_wait_read<SLABS - 1>();     // the store that last read this slab is done
                 __syncwarp();
@@ -1300,7 +1305,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             const int m = m0 + quad * 32 + lane;
             int64_t my_off = -1;
             int zmask = 0;                       // zfill: which of the row's three neighbour pixels exist
-            if (m < tg.M) {
+            if (!p.tma_store && m < tg.M) {
                 if (MODE == TCM_FWD) {
                     const int img = m / (tg.P * tg.Q);
                     const int rem = m - img * (tg.P * tg.Q);
@@ -1321,7 +1326,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
 #pragma unroll
                 for (int cc = 0; cc < BN / 32; cc++) {
                     if (n0 + cc * 32 < p.N) {
-                        if (MODE == TCM_FWD && p.epi) tc_epilogue_math(p, n0 + cc * 32, &acc[cc * 32], m);
+                        if (MODE == TCM_FWD && p.epi) tc_epilogue_math(p, n0 + cc * 32, &acc[cc * 32]);
 #pragma unroll
                         for (int j = 0; j < 32; j += 4)
                             *reinterpret_cast<float4*>(stage + lane * 36 + j) =
@@ -1377,7 +1382,7 @@ struct FinishParams {
     const float* partial;
     float* out;
     int64_t o_sn, o_sh, o_sw;
-    const float *bias, *mean, *inv_std, *gamma, *beta, *addend;
+    const float *bias, *mean, *inv_std, *gamma, *beta;
     int relu;
     float* stats;
 };
@@ -1418,10 +1423,6 @@ __global__ void __launch_bounds__(256) tc_split_finish_kernel(FinishParams p)
                     if (p.bias) a[e] += __ldg(p.bias + n0 + e);
                     if (p.mean) { const float t = (a[e] - __ldg(p.mean + n0 + e)) * __ldg(p.inv_std + n0 + e); a[e] = t * __ldg(p.gamma + n0 + e) + __ldg(p.beta + n0 + e); }
                 }
-            if (p.addend) {                    // dense rows, a multiple of four channels
-                const float4 q = __ldg(reinterpret_cast<const float4*>(p.addend + (int64_t)m * p.o_sw + n0));
-                a[0] = __fadd_rn(a[0], q.x); a[1] = __fadd_rn(a[1], q.y); a[2] = __fadd_rn(a[2], q.z); a[3] = __fadd_rn(a[3], q.w);
-            }
             if (p.relu)
 #pragma unroll
                 for (int e = 0; e < 4; e++) a[e] = fmaxf(a[e], 0.f);
@@ -1481,7 +1482,6 @@ __global__ void __launch_bounds__(256) tc_split_finish_deep_kernel(FinishParams 
         if (e < cnt) {
             if (p.bias) a[e] += __ldg(p.bias + n0 + e);
             if (p.mean) { const float t = (a[e] - __ldg(p.mean + n0 + e)) * __ldg(p.inv_std + n0 + e); a[e] = t * __ldg(p.gamma + n0 + e) + __ldg(p.beta + n0 + e); }
-            if (p.addend) a[e] = __fadd_rn(a[e], __ldg(p.addend + (int64_t)m * p.o_sw + n0 + e));
             if (p.relu) a[e] = fmaxf(a[e], 0.f);
             d[e] = a[e];
         }
@@ -1882,6 +1882,9 @@ static int launch_tc(const CUtensorMap& ma, const CUtensorMap& mb0, const CUtens
     if (tiles > 0x7fffffffLL) return B2C_ERR_TOO_LARGE;
     TcParams q = p;
     q.splits = splits;
+    const int nt_ = (p.N + BN - 1) / BN, mt_ = (p.M + 127) / 128;
+    q.f_nt = FastDiv(nt_); q.f_mt = FastDiv(mt_); q.f_plane = FastDiv(nt_ * mt_); q.f_pq = FastDiv(p.P * p.Q); q.f_q = FastDiv(p.Q);
+    q.f_cb = FastDiv(p.cblocks); q.f_s = FastDiv(p.S); q.f_c = FastDiv(p.C);
 #ifdef B2C_TC_DEV
     { const char* e = getenv("B2C_TC_DBG"); q.dbg = e ? atoi(e) : 0; }
 #endif
@@ -2056,7 +2059,7 @@ struct FwdLaunch {
 
 static int run_fwd(const FwdLaunch& f, const void* act, const void* w, PrepParams pp, const void* bias,
                    const b2c_bn_params* bn, int relu, float* out, void* ws, size_t ws_bytes, cudaStream_t st,
-                   bool filters_ready = false, const StatsOut* stats = nullptr, const ZeroFill* zf = nullptr, const float* addend = nullptr)
+                   bool filters_ready = false, const StatsOut* stats = nullptr, const ZeroFill* zf = nullptr)
 {
     if (!load_driver_entry_points()) return B2C_ERR_UNSUPPORTED;
     const int cblocks = (f.C + 31) / 32;
@@ -2118,8 +2121,7 @@ static int run_fwd(const FwdLaunch& f, const void* act, const void* w, PrepParam
     p.bias = (const float*)bias;
     if (bn) { p.mean = (const float*)bn->mean; p.inv_std = (const float*)bn->inv_std; p.gamma = (const float*)bn->gamma; p.beta = (const float*)bn->beta; }
     p.relu = relu;
-    p.addend = addend;
-    p.epi = (addend ? TC_EPI_ADD : 0) | (p.bias ? TC_EPI_BIAS : 0) | (p.mean ? TC_EPI_BN : 0) | (relu ? TC_EPI_RELU : 0);
+    p.epi = (p.bias ? TC_EPI_BIAS : 0) | (p.mean ? TC_EPI_BN : 0) | (relu ? TC_EPI_RELU : 0);
     if (f.N % 4 == 0 && !(((uintptr_t)p.bias | (uintptr_t)p.mean | (uintptr_t)p.inv_std | (uintptr_t)p.gamma | (uintptr_t)p.beta) & 15))
         p.epi |= TC_EPI_VEC;
     p.out = out; p.o_sn = f.o_sn; p.o_sh = f.o_sh; p.o_sw = f.o_sw;
@@ -2135,7 +2137,6 @@ static int run_fwd(const FwdLaunch& f, const void* act, const void* w, PrepParam
         if (!make_map_out(&mo, sk_partial, 0, (uint64_t)(splits * mrows), (uint64_t)round4(f.N), (uint64_t)round4(f.N))) return B2C_ERR_UNSUPPORTED;
         p.tma_store = 1; p.kper = kper; p.epi = 0;
     } else if (dense && make_map_out(&mo, out, 0, (uint64_t)p.M, (uint64_t)f.N, (uint64_t)f.o_sw)) p.tma_store = 1;
-    if (addend && (!dense || f.N % 4 || ((uintptr_t)addend & 15))) return B2C_ERR_UNSUPPORTED;
     if (zf) {
         if (p.tma_store || ((zf->off_w | zf->off_h) & 3)) return B2C_ERR_UNSUPPORTED;
         p.zfill = 1; p.z_W = zf->W; p.z_H = zf->H; p.z_w = zf->off_w; p.z_h = zf->off_h;
@@ -2153,7 +2154,7 @@ static int run_fwd(const FwdLaunch& f, const void* act, const void* w, PrepParam
                  : dispatch_fwd<TCB_SPLIT>(BN, ma, mbh, mbl, mo, p, st);
     if (rc || !kper) return rc;
     FinishParams fp{p.M, p.N, p.P, p.Q, splits, round4(f.N), mrows * round4(f.N), sk_partial, out, f.o_sn, f.o_sh, f.o_sw,
-                    p.bias, p.mean, p.inv_std, p.gamma, p.beta, addend, relu, stats ? stats->sums : nullptr};
+                    p.bias, p.mean, p.inv_std, p.gamma, p.beta, relu, stats ? stats->sums : nullptr};
     const dim3 fgrid((p.N + 127) / 128, stats ? (p.M + 31) / 32 : (p.M + 7) / 8);
     if (stats) launch_pdl(tc_split_finish_kernel<4>, fgrid, 256, 0, st, fp);
     else if (splits >= 8 && (int64_t)p.M * ((p.N + 127) / 128) <= 8 * (int64_t)tc_sm_count())      // the other kernel would not fill the chip
@@ -2194,7 +2195,7 @@ static int launch_lower(const Geo& g, const void* x, float* rows, cudaStream_t s
 }
 
 static int tc_fprop_nhwc(const Geo& g, const void* x, const void* w, const void* bias, const b2c_bn_params* bn, int relu,
-             void* y, void* ws, size_t ws_bytes, cudaStream_t st, const StatsOut* stats = nullptr, const float* addend = nullptr)
+             void* y, void* ws, size_t ws_bytes, cudaStream_t st, const StatsOut* stats = nullptr)
 {
     WStride wsd = w_stride(g.w_layout, g.ci, g.co, g.kh, g.kw);
     const int64_t yp = g.yp;
@@ -2217,13 +2218,13 @@ static int tc_fprop_nhwc(const Geo& g, const void* x, const void* w, const void*
         if (rc) return rc;
         PrepParams none{};
         FwdLaunch f{g.n, g.ho, g.wo, Kp, Kp, g.ho, g.wo, g.co, 1, 1, 0, 0, g.ho, g.wo, 1, 1, 1, 1, g.ho * g.wo * yp, g.wo * yp, yp};
-        return run_fwd(f, rows, nullptr, none, bias, bn, relu, (float*)y, (void*)w_hi, 2 * fbytes + 1024, st, true, stats, nullptr, addend);
+        return run_fwd(f, rows, nullptr, none, bias, bn, relu, (float*)y, (void*)w_hi, 2 * fbytes + 1024, st, true, stats);
     }
     PrepParams pp{g.co, g.ci, g.kh, g.kw, wsd.sk, wsd.sc, wsd.sr, wsd.ss, 0, 1, 0, 1, g.kh, g.kw};
     FwdLaunch f{g.n, g.h, g.w, g.ci, g.xp, g.ho, g.wo, g.co, g.kh, g.kw, -g.vpad, -g.hpad,
                 g.h + 2 * g.vpad - (g.kh - 1) * g.vdil, g.w + 2 * g.hpad - (g.kw - 1) * g.hdil,
                 g.vstr, g.hstr, g.vdil, g.hdil, g.ho * g.wo * yp, g.wo * yp, yp};
-    return run_fwd(f, x, w, pp, bias, bn, relu, (float*)y, ws, ws_bytes, st, false, stats, nullptr, addend);
+    return run_fwd(f, x, w, pp, bias, bn, relu, (float*)y, ws, ws_bytes, st, false, stats);
 }
 
 // Strided data gradient, all parity classes in one launch (MULTI kernel variants): up to four classes, every class
@@ -2730,18 +2731,6 @@ int tc_fprop(const Geo& g, const void* x, const void* w, const void* bias, const
              void* y, void* ws, size_t ws_bytes, cudaStream_t st)
 {
     return tc_fprop_any(g, x, w, bias, bn, relu, y, ws, ws_bytes, st, nullptr);
-}
-
-// y = relu?(bn?(conv + bias) + addend) where the kernels write y itself (no copies) in whole 16-byte pixels.
-bool tc_takes_addend(const Geo& g)
-{
-    const Copies c = tc_copies(g, B2C_PASS_FPROP);
-    return g.layout == B2C_LAYOUT_NHWC && !c.x && !c.y && g.co % 4 == 0;
-}
-int tc_fprop_residual(const Geo& g, const void* x, const void* w, const void* bias, const b2c_bn_params* bn, const void* addend, int relu,
-                      void* y, void* ws, size_t ws_bytes, cudaStream_t st)
-{
-    return tc_fprop_nhwc(g, x, w, bias, bn, relu, y, ws, ws_bytes, st, nullptr, (const float*)addend);
 }
 
 int tc_dgrad(const Geo& g, const void* dy, const void* w, void* dx, void* ws, size_t ws_bytes, cudaStream_t st)
