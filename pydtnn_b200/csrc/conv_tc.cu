@@ -699,12 +699,15 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         if (p.tma_store) tma_prefetch_map(&tmap_out);
         if (MULTI) { if (p.ncls > 1) tma_prefetch_map(&tmap_b1); if (p.ncls > 2) tma_prefetch_map(&tmap_out); if (p.ncls > 3) tma_prefetch_map(&tmap_a3); }
     }
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < STAGES; s++) { mbar_init(&full_bar[s], 1); mbar_init(&afree_bar[s], 4); }
-        for (int s = 0; s < TSLOTS; s++) { mbar_init(&xform_bar[s], 4); mbar_init(&empty_bar[s], 1); }
-        mbar_init(bres_bar, 1);
-        for (int b = 0; b < 2; b++) { mbar_init(&tfull_bar[b], 1); mbar_init(&tempty_bar[b], DW); }
-        *abort_flag = 0;
+    constexpr int NBARS = 2 * STAGES + 2 * TSLOTS + 5;           // they lie one after the other from full_bar on
+    static_assert(NBARS <= 32, "a lane of the first warp for each barrier");
+    if (threadIdx.x < 32) {
+        if (threadIdx.x < NBARS) {
+            const uint64_t* bar = full_bar + threadIdx.x;
+            const bool by_four = (bar >= xform_bar && bar < empty_bar) || (bar >= afree_bar && bar < bres_bar);
+            mbar_init(full_bar + threadIdx.x, by_four ? 4 : bar >= tempty_bar && bar < afree_bar ? DW : 1);
+        }
+        if (threadIdx.x == 0) *abort_flag = 0;
         fence_barrier_init();
         fence_proxy_async();
     }
@@ -900,54 +903,59 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 // (or a branch between the two forms per k-block) a long launch lost 3 to 6 % (2 %).
                 auto issue_tile = [&](auto whole_c) {
                 constexpr bool WHOLE = decltype(whole_c)::value;
-                int ck = 0, cb = WHOLE || MODE == TCM_WGRAD ? 0 : w.kb_b % p.cblocks;
-                for (int kb = w.kb_b; kb < w.kb_e; kb++) {
-                    const int s = ring.s;
-                    const int b = gc & 1;
-                    const bool chunk_start = ck == 0;
-                    const bool chunk_end = ++ck == TC_CHUNK || kb == w.kb_e - 1;
+                int cb = WHOLE || MODE == TCM_WGRAD ? 0 : w.kb_b - p.f_cb.div(w.kb_b) * p.cblocks;
+                for (int kb = w.kb_b; kb < w.kb_e;) {
+                    // one chunk: up to TC_CHUNK k-blocks into one drained tensor-memory buffer (the first two find theirs free)
+                    const int b = gc & 1, chunk = w.kb_e - kb < TC_CHUNK ? w.kb_e - kb : TC_CHUNK;
                     TC_PROF_T0();
-                    // a drained tensor-memory buffer (the first two chunks find theirs free)
-                    if (chunk_start) ok = mbar_wait(&tempty_bar[b], ((gc >> 1) & 1) ^ 1, abort_flag, &g_tc_status, TC_ERR_TEMPTY);
+                    ok = mbar_wait(&tempty_bar[b], ((gc >> 1) & 1) ^ 1, abort_flag, &g_tc_status, TC_ERR_TEMPTY);
                     TC_PROF_ADD(1);    // MMA: waiting for a drained TMEM buffer
-                    // the transform warps arrive only after they have seen the stage's TMA data land
-                    if (ok && !ahead) ok = mbar_wait(&xform_bar[s], ring.phase, abort_flag, &g_tc_status, TC_ERR_XFORM);
-                    TC_PROF_ADD(3);    // MMA: waiting for the transform
-                    if (!ok) break;
-                    tc_fence_after();
-                    const uint64_t b_hi = b_desc0 + (uint64_t)(RESKB ? kb * (2 * L::B_BYTES >> 4) : s * (L::STAGE_BYTES >> 4));
-                    const uint64_t b_lo = b_hi + (L::B_BYTES >> 4);
-                    const uint32_t a_hi = tmem_base + (uint32_t)(L::TMEM_A_COL + s * 64);
-                    const uint32_t a_lo = a_hi + 32;
                     const uint32_t d = tmem_base + (uint32_t)(b * BN);
-                    ring.next();
-                    // small terms first: lo*hi, hi*lo, then hi*hi
-                    auto step = [&](int k, uint32_t id) {
-                        const uint64_t adv = (uint64_t)k * KADV;
+                    uint32_t onto = 0;                               // the chunk's first product overwrites the buffer
+                    for (int i = 0; i < chunk && ok; i++, kb++) {
+                        const int s = ring.s;
+                        TC_PROF_RESET();
+                        // the transform warps arrive only after they have seen the stage's TMA data land
+                        if (!ahead) ok = mbar_wait(&xform_bar[s], ring.phase, abort_flag, &g_tc_status, TC_ERR_XFORM);
+                        TC_PROF_ADD(3);    // MMA: waiting for the transform
+                        if (!ok) break;
+                        tc_fence_after();
+                        const uint64_t b_hi = b_desc0 + (uint64_t)(RESKB ? kb * (2 * L::B_BYTES >> 4) : s * (L::STAGE_BYTES >> 4));
+                        const uint64_t b_lo = b_hi + (L::B_BYTES >> 4);
+                        const uint32_t a_hi = tmem_base + (uint32_t)(L::TMEM_A_COL + s * 64);
+                        const uint32_t a_lo = a_hi + 32;
+                        ring.next();
+                        // small terms first: lo*hi, hi*lo, then hi*hi
+                        auto step = [&](int k, uint32_t id) {
+                            const uint64_t adv = (uint64_t)k * KADV;
 #ifdef B2C_TC_DEV
-                        if (p.dbg & 32) return;
+                            if (p.dbg & 32) return;
 #endif
-                        umma_tf32_ts(d, a_lo + k * 8, b_hi + adv, id, (!chunk_start || k > 0) ? 1u : 0u);
+                            umma_tf32_ts(d, a_lo + k * 8, b_hi + adv, id, k > 0 ? 1u : onto);
 #ifdef B2C_TC_DEV
-                        if (p.dbg & 2) return;
+                            if (p.dbg & 2) return;
 #endif
-                        umma_tf32_ts(d, a_hi + k * 8, b_lo + adv, id, 1u);
-                        umma_tf32_ts(d, a_hi + k * 8, b_hi + adv, id, 1u);
-                    };
-                    if constexpr (WHOLE) {
-                        constexpr uint32_t id = make_idesc_tf32(128, BN, 0, B_MN);
-                        step(0, id); step(1, id); step(2, id);
-                        ahead = mbar_test(&xform_bar[ring.s], ring.phase);
-                        step(3, id);
-                    } else {
-                        const int ks = MODE == TCM_FWD && cb == p.cblocks - 1 ? p.ktail : 4;
-                        for (int k = 0; k < ks; k++) step(k, idesc);
-                        ahead = mbar_test(&xform_bar[ring.s], ring.phase);
+                            umma_tf32_ts(d, a_hi + k * 8, b_lo + adv, id, 1u);
+                            umma_tf32_ts(d, a_hi + k * 8, b_hi + adv, id, 1u);
+                        };
+                        if constexpr (WHOLE) {
+                            constexpr uint32_t id = make_idesc_tf32(128, BN, 0, B_MN);
+                            step(0, id); step(1, id); step(2, id);
+                            ahead = mbar_test(&xform_bar[ring.s], ring.phase);
+                            step(3, id);
+                        } else {
+                            const int ks = MODE == TCM_FWD && cb == p.cblocks - 1 ? p.ktail : 4;
+                            for (int k = 0; k < ks; k++) step(k, idesc);
+                            ahead = mbar_test(&xform_bar[ring.s], ring.phase);
+                            if (++cb == p.cblocks) cb = 0;
+                        }
+                        umma_commit(&empty_bar[s]);
+                        onto = 1;
+                        TC_PROF_ADD(4);    // MMA: issue
                     }
-                    umma_commit(&empty_bar[s]);
-                    if (chunk_end) { umma_commit(&tfull_bar[b]); gc++; ck = 0; }
-                    if (!WHOLE && ++cb == p.cblocks) cb = 0;
-                    TC_PROF_ADD(4);    // MMA: issue
+                    if (!ok) break;
+                    umma_commit(&tfull_bar[b]);
+                    gc++;
                 }
                 };
                 if (left > BN - 16 && (MODE == TCM_WGRAD || p.ktail == 4)) issue_tile(std::true_type{});
