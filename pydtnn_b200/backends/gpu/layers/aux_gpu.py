@@ -277,7 +277,9 @@ class _Pool2DGPU(LayerGPU):
     def forward(self, x):
         m = self.model
         _lib.check(_lib.lib().b2c_pool_forward(self._dt, _lib.LAYOUT_NHWC, self._is_max, *self._geom(),
-                                               self._in(x, "x"), self.y.out, self.idx_max.gpudata if self._is_max else None,
+                                               self._in(x, "x"), self.y.out,
+                                               # the winning taps are for backward only
+                                               self.idx_max.gpudata if self._is_max and m.mode != EVALUATE_MODE else None,
                                                m.stream_handle))
         self.y.written()
         return self.y

@@ -770,38 +770,46 @@ __global__ void pool_bwd_kernel(PoolP p, const T* __restrict__ dy, const int32_t
 }
 
 
-// float32 NHWC pooling with 4 channels per thread (c % 4 == 0).
+// float32 NHWC pooling with 4 channels per thread (c % 4 == 0).  Grid (blocks over a row's positions x channel groups, n x ho):
+// one 32-bit division per thread instead of six 64-bit ones per output, and the window's bounds are clipped once instead of
+// tested at every tap, so the taps' loads are independent (64 x 55 x 55 x 96, 3 x 3 / 2, with the tap numbers: 29.6 us before).
 template <bool IS_MAX>
-__global__ void __launch_bounds__(256) pool_fwd_v4_kernel(PoolP p, const float4* __restrict__ x, float4* __restrict__ y, int4* __restrict__ idx_max)
+__global__ void __launch_bounds__(256) pool_fwd_v4_kernel(PoolP p, const float4* __restrict__ x, float4* __restrict__ y, int4* __restrict__ idx_max, int row0)
 {
     pdl_prologue();
     const int c4 = p.c / 4;
-    const int64_t total = (int64_t)p.n * p.ho * p.wo * c4;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-        const int cg = (int)(i % c4); int64_t r = i / c4;
-        const int yy = (int)(r % p.wo); r /= p.wo;
-        const int xx = (int)(r % p.ho); const int nn = (int)(r / p.ho);
-        float4 best = IS_MAX ? make_float4(-FLT_MAX, -FLT_MAX, -FLT_MAX, -FLT_MAX) : make_float4(0.f, 0.f, 0.f, 0.f);
-        int4 bi = make_int4(0, 0, 0, 0);
-        int items = 0;
-        for (int ii = 0; ii < p.kh; ii++) {
-            const int x_x = p.vstr * xx + p.vdil * ii - p.vpad;
-            if (x_x < 0 || x_x >= p.h) continue;
-            for (int jj = 0; jj < p.kw; jj++) {
-                const int x_y = p.hstr * yy + p.hdil * jj - p.hpad;
-                if (x_y < 0 || x_y >= p.w) continue;
-                const float4 v = x[(((int64_t)nn * p.h + x_x) * p.w + x_y) * c4 + cg];
-                if (IS_MAX) {
-                    const int t = ii * p.kw + jj;
-                    if (v.x > best.x) { best.x = v.x; bi.x = t; }
-                    if (v.y > best.y) { best.y = v.y; bi.y = t; }
-                    if (v.z > best.z) { best.z = v.z; bi.z = t; }
-                    if (v.w > best.w) { best.w = v.w; bi.w = t; }
-                } else { best.x += v.x; best.y += v.y; best.z += v.z; best.w += v.w; items++; }
-            }
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= p.wo * c4) return;
+    const int yy = e / c4, cg = e - yy * c4;
+    const int row = row0 + blockIdx.y, nn = row / p.ho, xx = row - nn * p.ho;
+    const int h0 = p.vstr * xx - p.vpad, w0 = p.hstr * yy - p.hpad;
+    // taps ii0 <= ii < ii1, jj0 <= jj < jj1 lie inside the image
+    const int ii0 = h0 < 0 ? (-h0 + p.vdil - 1) / p.vdil : 0, jj0 = w0 < 0 ? (-w0 + p.hdil - 1) / p.hdil : 0;
+    int ii1 = p.kh, jj1 = p.kw;
+    if (h0 + (p.kh - 1) * p.vdil >= p.h) ii1 = p.h > h0 ? (p.h - h0 + p.vdil - 1) / p.vdil : 0;
+    if (w0 + (p.kw - 1) * p.hdil >= p.w) jj1 = p.w > w0 ? (p.w - w0 + p.hdil - 1) / p.hdil : 0;
+    float4 best = IS_MAX ? make_float4(-FLT_MAX, -FLT_MAX, -FLT_MAX, -FLT_MAX) : make_float4(0.f, 0.f, 0.f, 0.f);
+    int4 bi = make_int4(0, 0, 0, 0);
+    for (int ii = ii0; ii < ii1; ii++) {
+        const float4* src = x + (((int64_t)nn * p.h + h0 + ii * p.vdil) * p.w + w0) * c4 + cg;
+#pragma unroll 4
+        for (int jj = jj0; jj < jj1; jj++) {
+            const float4 v = src[(int64_t)jj * p.hdil * c4];
+            if (IS_MAX) {
+                const int t = ii * p.kw + jj;
+                if (v.x > best.x) { best.x = v.x; bi.x = t; }
+                if (v.y > best.y) { best.y = v.y; bi.y = t; }
+                if (v.z > best.z) { best.z = v.z; bi.z = t; }
+                if (v.w > best.w) { best.w = v.w; bi.w = t; }
+            } else { best.x += v.x; best.y += v.y; best.z += v.z; best.w += v.w; }
         }
-        if (IS_MAX) { y[i] = best; if (idx_max) idx_max[i] = bi; }
-        else { const float inv = (float)items; y[i] = make_float4(best.x / inv, best.y / inv, best.z / inv, best.w / inv); }
+    }
+    const int64_t o = ((int64_t)row * p.wo + yy) * c4 + cg;
+    if (IS_MAX) { y[o] = best; if (idx_max) idx_max[o] = bi; }
+    else {
+        const int items = (ii1 > ii0 ? ii1 - ii0 : 0) * (jj1 > jj0 ? jj1 - jj0 : 0);
+        const float inv = (float)items;
+        y[o] = make_float4(best.x / inv, best.y / inv, best.z / inv, best.w / inv);
     }
 }
 
@@ -1338,9 +1346,15 @@ extern "C" int b2c_pool_forward(int dtype, int layout, int is_max, int n, int h,
     cudaStream_t st = (cudaStream_t)stream;
     int64_t total = (int64_t)n * p.ho * p.wo * c; int nchw = layout == B2C_LAYOUT_NCHW;
     if (dtype == B2C_F32 && !nchw && c % 4 == 0 && (((uintptr_t)x | (uintptr_t)y | (uintptr_t)idx_max) & 15) == 0) {
-        if (is_max) launch_pdl(pool_fwd_v4_kernel<true>, ew_blocks(total / 4), 256, 0, st, p, (const float4*)x, (float4*)y, (int4*)idx_max);
-        else launch_pdl(pool_fwd_v4_kernel<false>, ew_blocks(total / 4), 256, 0, st, p, (const float4*)x, (float4*)y, (int4*)idx_max);
-        return check_launch("pool_forward_v4");
+        const int64_t rows = (int64_t)n * p.ho, per_row = (int64_t)p.wo * (c / 4);
+        if (rows > 0x7fffffffLL || per_row > 0x7fffff00LL) return B2C_ERR_TOO_LARGE;
+        for (int64_t row0 = 0; row0 < rows; row0 += 65535) {          // the rows are a grid axis
+            const dim3 grid((unsigned)((per_row + 255) / 256), (unsigned)(rows - row0 < 65535 ? rows - row0 : 65535));
+            if (is_max) launch_pdl(pool_fwd_v4_kernel<true>, grid, 256, 0, st, p, (const float4*)x, (float4*)y, (int4*)idx_max, (int)row0);
+            else launch_pdl(pool_fwd_v4_kernel<false>, grid, 256, 0, st, p, (const float4*)x, (float4*)y, (int4*)idx_max, (int)row0);
+            const int rc2 = check_launch("pool_forward_v4"); if (rc2) return rc2;
+        }
+        return B2C_OK;
     }
     if (dtype == B2C_F32 && nchw && (int64_t)h * w <= B2C_POOL_TILE && (int64_t)n * c < 0x7fffffffLL) {
         const int planes = n * c;

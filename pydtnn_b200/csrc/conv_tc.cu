@@ -368,18 +368,43 @@ __global__ void tc_lower_rows_kernel(LowerParams p, const float* __restrict__ x,
     extern __shared__ float patch[];                      // [kh][wp][c], column j is input column j - hpad
     const int nn = blockIdx.x / p.ho, oh = blockIdx.x - nn * p.ho;
     const int rowlen = wp * p.c;
-    // one patch pixel per thread and trip (its few channels in an inner loop: no division per element)
-    for (int r = 0; r < p.kh; r++) {
-        const int ih = oh * p.vstr - p.vpad + r * p.vdil;
-        const bool row_in = (unsigned)ih < (unsigned)p.h;
-        const float* src = x + nn * p.sn + ih * p.sh;
-        for (int j = threadIdx.x; j < wp; j += blockDim.x) {
-            const int iw = j - p.hpad;
-            const bool in = row_in && (unsigned)iw < (unsigned)p.w;
-            float* dst = patch + r * rowlen + j * p.c;
-            for (int c = 0; c < p.c; c++) dst[c] = in ? __ldg(src + iw * p.sw + c * p.sc) : 0.f;
+    // Column j of a patch row is input column j - hpad.  A channel-last row is one run of floats, copied as such with four
+    // independent rows in flight; NCHW planes are copied one by one (contiguous along the row as well).
+    auto fill = [&](int r0, auto rows_c) {
+        constexpr int R = decltype(rows_c)::value;
+        const float* src[R];
+        bool in[R];
+#pragma unroll
+        for (int u = 0; u < R; u++) {
+            const int ih = oh * p.vstr - p.vpad + (r0 + u) * p.vdil;
+            in[u] = (unsigned)ih < (unsigned)p.h;
+            src[u] = x + nn * p.sn + (in[u] ? ih : 0) * p.sh;
         }
-    }
+        if (p.sc == 1) {
+            const int lead = p.hpad * p.c, len = p.w * p.c;
+            for (int e = threadIdx.x; e < rowlen; e += blockDim.x) {
+                const bool ok = (unsigned)(e - lead) < (unsigned)len;
+                float v[R];
+#pragma unroll
+                for (int u = 0; u < R; u++) v[u] = ok && in[u] ? __ldg(src[u] + e - lead) : 0.f;
+#pragma unroll
+                for (int u = 0; u < R; u++) patch[(r0 + u) * rowlen + e] = v[u];
+            }
+        } else {
+            for (int c = 0; c < p.c; c++)
+                for (int j = threadIdx.x; j < wp; j += blockDim.x) {
+                    const bool ok = (unsigned)(j - p.hpad) < (unsigned)p.w;
+                    float v[R];
+#pragma unroll
+                    for (int u = 0; u < R; u++) v[u] = ok && in[u] ? __ldg(src[u] + c * p.sc + (j - p.hpad) * p.sw) : 0.f;
+#pragma unroll
+                    for (int u = 0; u < R; u++) patch[(r0 + u) * rowlen + j * p.c + c] = v[u];
+                }
+        }
+    };
+    int r = 0;
+    for (; r + 4 <= p.kh; r += 4) fill(r, std::integral_constant<int, 4>{});
+    for (; r < p.kh; r++) fill(r, std::integral_constant<int, 1>{});
     __syncthreads();
     const int kq = p.Kp / 4;
     const int sub = threadIdx.x / kq, q4 = threadIdx.x - sub * kq, nsub = blockDim.x / kq;
