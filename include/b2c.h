@@ -261,6 +261,13 @@ int b2c_cce_forward_backward(int dtype, int rows, int cols, const void *probs, c
  * pydtnn/model.py:426-438; a data-parallel caller all-reduces the two doubles in place. */
 int b2c_cce_totals(int dtype, int rows, const void *row_loss, const int32_t *hit, double *out2, void *stream);
 
+/* b2c_cce_forward_backward, b2c_cce_totals and the b2c_softmax_backward that follows them in one launch, with the same
+ * results: softmax_dx is the gradient before the softmax whose output is probs.  counter: a DEVICE word, zero before the
+ * first call, left at zero by every call; calls that can overlap need a counter (and outputs) each. */
+int b2c_cce_softmax_backward(int dtype, int rows, int cols, const void *probs, const int32_t *labels, int global_batch,
+                             double eps, void *row_loss, int32_t *hit, void *dx, void *softmax_dx, double *totals,
+                             uint32_t *counter, void *stream);
+
 /* inv_std[i] = 1 / sqrt(running_var[i] + eps), evaluated in double and rounded once: the per-channel factor of the
  * inference-mode batch norm, pydtnn/layers/batch_normalization.py:61 and
  * pydtnn/backends/cpu/layers/batch_normalization_cpu.py:92-94 (computed there on the host). */

@@ -88,6 +88,8 @@ PROTOTYPES = {
     "b2c_softmax_backward": (c_int, [c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p]),
     "b2c_cce_forward_backward": (c_int, [c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_double, c_void_p, c_void_p,
                                          c_void_p, c_void_p]),
+    "b2c_cce_softmax_backward": (c_int, [c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_double, c_void_p, c_void_p, c_void_p, c_void_p,
+                                         c_void_p, c_void_p, c_void_p]),
     "b2c_cce_totals": (c_int, [c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p]),
     "b2c_bn_inv_std": (c_int, [c_int, c_int, c_void_p, c_double, c_void_p, c_void_p]),
     "b2c_probe_fma": (c_int, [c_int, c_int, c_int, c_void_p, POINTER(c_double), c_void_p]),

@@ -176,6 +176,7 @@ class SoftmaxGPU(LayerGPU, Softmax):
         if self.need_dx:
             self.dx = TensorGPU(empty(x.dims, m.dtype), m.tensor_format)
         self._dt = _lib.dtype_code(m.dtype)
+        self.backward_done = False       # the loss of this step has written dx already
         self._rows, self._cols = int(x.dims[0]), int(np.prod(x.dims[1:]))
 
     def forward(self, x):
@@ -184,6 +185,9 @@ class SoftmaxGPU(LayerGPU, Softmax):
         return self.y
 
     def backward(self, dy):
+        if self.backward_done:
+            self.backward_done = False
+            return self.dx
         if self.need_dx:
             _lib.check(_lib.lib().b2c_softmax_backward(self._dt, self._rows, self._cols, dy.ptr, self.y.ptr,
                                                        self.dx.ptr, self.model.stream_handle))

@@ -9,7 +9,7 @@ all-reduce (pydtnn/model.py:426-438): every rank then reports the global numbers
 import numpy as np
 
 from . import _lib
-from .tensor_gpu import TensorGPU, empty
+from .tensor_gpu import TensorGPU, empty, zeros
 
 
 class CategoricalCrossEntropy:
@@ -22,20 +22,30 @@ class CategoricalCrossEntropy:
         self.hit = empty((b,), np.int32)
         self.totals = empty((2,), np.float64)      # [mean loss, accuracy %] of this rank, then of the job
         self.dx = TensorGPU(empty((b, shape[1]), model.dtype), model.tensor_format)
+        self._counter = zeros((1,), np.int32)
         self._work = None
         self._scaled = 1
 
-    def __call__(self, y_pred, labels, global_batch_size):
-        """``labels``: device int32 array (b,). Returns (self, dx): read the numbers with
-        ``loss()`` / ``accuracy()``, which copy two doubles to the host."""
+    def __call__(self, y_pred, labels, global_batch_size, softmax=None):
+        """``labels``: device int32 array (b,). ``softmax``: the layer whose output y_pred is, when its backward
+        follows. Returns (self, dx): read the numbers with ``loss()`` / ``accuracy()``, which copy two doubles
+        to the host."""
         m = self.model
         L = _lib.lib()
-        _lib.check(L.b2c_cce_forward_backward(
-            _lib.dtype_code(m.dtype), m.batch_size, self.shape[1], y_pred.ptr, labels.gpudata,
-            int(global_batch_size), float(self.eps), self.row_loss.gpudata, self.hit.gpudata, self.dx.ptr,
-            m.stream_handle))
-        _lib.check(L.b2c_cce_totals(_lib.dtype_code(m.dtype), m.batch_size, self.row_loss.gpudata, self.hit.gpudata,
-                                    self.totals.gpudata, m.stream_handle))
+        if softmax is not None:
+            # training: the backward of the softmax layer that made y_pred in the same launch
+            _lib.check(L.b2c_cce_softmax_backward(
+                _lib.dtype_code(m.dtype), m.batch_size, self.shape[1], y_pred.ptr, labels.gpudata, int(global_batch_size),
+                float(self.eps), self.row_loss.gpudata, self.hit.gpudata, self.dx.ptr, softmax.dx.ptr, self.totals.gpudata,
+                self._counter.gpudata, m.stream_handle))
+            softmax.backward_done = True
+        else:
+            _lib.check(L.b2c_cce_forward_backward(
+                _lib.dtype_code(m.dtype), m.batch_size, self.shape[1], y_pred.ptr, labels.gpudata,
+                int(global_batch_size), float(self.eps), self.row_loss.gpudata, self.hit.gpudata, self.dx.ptr,
+                m.stream_handle))
+            _lib.check(L.b2c_cce_totals(_lib.dtype_code(m.dtype), m.batch_size, self.row_loss.gpudata, self.hit.gpudata,
+                                        self.totals.gpudata, m.stream_handle))
         self._work, self._scaled = None, 1
         if m.comm is not None:
             import torch.distributed as dist

@@ -272,7 +272,11 @@ class Model:
         for layer in self.layers[1:]:
             with tr.region(layer, tracer.PYDTNN_MDL_FORWARD):
                 x = layer.forward(x)
-        loss, dx = self.loss_func(x, self.y_batch, global_batch_size)
+        last = self.layers[-1]
+        if type(last).__name__ == "SoftmaxGPU" and last.need_dx and type(self.loss_func) is CategoricalCrossEntropy:
+            loss, dx = self.loss_func(x, self.y_batch, global_batch_size, softmax=last)
+        else:
+            loss, dx = self.loss_func(x, self.y_batch, global_batch_size)
         if self.comm is not None:
             self.bucketer.reset()
         for layer in reversed(self.layers[1:]):
