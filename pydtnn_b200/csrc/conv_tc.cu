@@ -29,7 +29,7 @@
 // run on channel-last copies.
 //
 // Warp roles (320 threads; 448 with eight drain warps): warp 0 = TMA producer, warp 1 = TMEM owner + MMA issuer
-// (both stay converged and issue through one elected lane), warps 2-5 = operand transform,
+// (one elected lane of each runs the whole loop), warps 2-5 = operand transform,
 // warps 6-9 (6-13) = drain + epilogue: the tensor core's accumulate step truncates, so sums are kept in
 // tensor memory only for a chunk of 8 k-blocks (two TMEM buffers alternate) and added chunk by
 // chunk into float32 registers with round-to-nearest, then bias / BN-scale / ReLU -> global.
@@ -1735,10 +1735,11 @@ static bool lowered_ok(const Geo& g)
     if (g.K > 1024) return false;
     if ((int64_t)g.M * lowered_kp(g) * 4 > (int64_t)3 << 30) return false;
     if (g.ci % 4) return true;          // the gather needs 16-byte pixels: the other way is a padded copy and one k-block per tap
-    // One k-block per tap read in place (its channels past ci cost loads, not products: about 0.4 us of an SM per 128
-    // rows), or K / 32 full ones (0.6 us) and the matrix written and read once (about 4 TB/s).
+    // One k-block per tap read in place, or K / 32 full ones (0.6 us of an SM per 128 rows) and the matrix written and read once
+    // (about 4 TB/s).  A tap in place took 0.55 to 0.73 us with pixels of 32 or 64 bytes and 0.75 to 0.98 with 16 or 48 (sweep of
+    // 4 to 16 channels, 3x3 to 7x7, 14x14 to 80x80).
     const double tiles = (double)((g.M + 127) / 128) * ((g.co + 127) / 128) / 148.0;
-    const double in_place = tiles * g.kh * g.kw * 0.4e-6;
+    const double in_place = tiles * g.kh * g.kw * (g.ci % 8 ? 0.9e-6 : 0.62e-6);
     const double lowered = tiles * (lowered_kp(g) / 32) * 0.6e-6 + (double)g.M * lowered_kp(g) * 8.0 / 4e12 + 3e-6;
     return lowered < in_place;
 }
@@ -2644,15 +2645,15 @@ __global__ void __launch_bounds__(256) pitch_copy_kernel(const float* __restrict
 static Geo as_nhwc(const Geo& g) { Geo q = g; q.layout = B2C_LAYOUT_NHWC; return q; }
 static size_t act_bytes(int64_t n, int64_t h, int64_t w, int64_t c) { return align_up((size_t)(n * h * w * c) * sizeof(float), 1024); }
 
-// Which activations a pass runs on copies of: NCHW ones, and those whose pixels are no multiple of 16 bytes (a few-channel
-// layer that lowers x reads it as it is, in either layout).  The copies lie at the start of the workspace, channel-last, pixels
+// Which activations a pass runs on copies of: NCHW ones, and those whose pixels are no multiple of 16 bytes (a layer that
+// lowers x reads it as it is, except NCHW with whole 16-byte pixels: copying it, then lowering rows of pixels, is faster).  The copies lie at the start of the workspace, channel-last, pixels
 // round4(channels) floats apart; a forward pass and the weight gradient of a layer agree on the place.
 struct Copies { bool x, y; size_t xb, yb; };
 static Copies tc_copies(const Geo& g, int pass)
 {
     Copies c;
     const bool nchw = g.layout == B2C_LAYOUT_NCHW;
-    c.x = (nchw || g.ci % 4) && (pass == B2C_PASS_DGRAD || !lowered_ok(g));
+    c.x = (nchw || g.ci % 4) && (pass == B2C_PASS_DGRAD || !lowered_ok(g) || (nchw && g.ci % 4 == 0));
     c.y = nchw || g.co % 4;
     c.xb = c.x ? act_bytes(g.n, g.h, g.w, round4(g.ci)) : 0;
     c.yb = c.y ? act_bytes(g.n, g.ho, g.wo, round4(g.co)) : 0;
@@ -2689,12 +2690,13 @@ bool tc_supported(const Geo& g, int pass)
     if (g.dtype != B2C_F32 || g.engine == B2C_ENGINE_FMA) return false;
     if (!tc_supported_nhwc(as_nhwc(g), pass)) return false;
     if (g.engine == B2C_ENGINE_TENSOR) return true;
-    // two tensors are copied there and/or back (read + write each) at about 2.5 TB/s; the FMA engine runs the
-    // pass at about 20 TFLOP/s, this engine at about 130
+    // two tensors are copied there and/or back (read + write each) at about 2.5 TB/s; this engine runs the pass at about
+    // 130 TFLOP/s.  The shapes where the copies weigh have few multiplications per value, and there the FMA engine makes 2 to
+    // 4 (4 channels, 3x3, 56x56 to 80x80: 1.9 to 2.5), not the 20 of a deep layer
     const double flops = 2.0 * (double)g.M * (double)g.K * g.co;
     const double xb = 4.0 * g.n * g.h * g.w * g.ci, yb = 4.0 * (double)g.M * g.co;
     const double moved = 2.0 * (xb + yb);
-    return flops / 130e12 + moved / 2.5e12 < flops / 20e12;
+    return flops / 130e12 + moved / 2.5e12 < flops / 4e12;
 }
 
 // Shapes whose channel counts keep every activation on 16-byte pixels and whole blocks, whatever the pointers: for the
