@@ -7,7 +7,7 @@
 //   dgrad : C[pixel(n,h,w)][ci]   = sum_tap  dy[(pixel + pad - tap) / stride] * w[tap.co][ci][tap.r][tap.s]
 //   wgrad : C[tap(ci,r,s)][co]    = sum_pixel x[pixel + tap] * dy[pixel][co]      (split over pixels)
 //
-// float32 uses FP32 FMA, float64 uses FP64 FMA.  This engine is the one every shape can run on;
+// float32 uses FP32 FMA, float64 the FP64 tensor pipe where the shape allows and FP64 FMA elsewhere.  This engine is the one every shape can run on;
 // the tensor-core engine (conv_tc.cu) takes over the shapes it supports.
 #include "b2c_common.cuh"
 #include <atomic>

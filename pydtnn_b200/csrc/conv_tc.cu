@@ -2692,11 +2692,11 @@ bool tc_supported(const Geo& g, int pass)
     if (g.engine == B2C_ENGINE_TENSOR) return true;
     // two tensors are copied there and/or back (read + write each) at about 2.5 TB/s; this engine runs the pass at about
     // 130 TFLOP/s.  The shapes where the copies weigh have few multiplications per value, and there the FMA engine makes 2 to
-    // 4 (4 channels, 3x3, 56x56 to 80x80: 1.9 to 2.5), not the 20 of a deep layer
-    const double flops = 2.0 * (double)g.M * (double)g.K * g.co;
+    // 4 of its tiles' operations (4 channels, 3x3, 56x56 to 80x80: 1.9 to 2.5 TFLOP/s), not the 20 of a deep layer
+    const double flops = 2.0 * (double)g.M * (double)g.K * g.co, tiles = 2.0 * (double)g.M * (g.K < 32 ? 32 : (double)g.K) * (g.co < 64 ? 64 : g.co);
     const double xb = 4.0 * g.n * g.h * g.w * g.ci, yb = 4.0 * (double)g.M * g.co;
     const double moved = 2.0 * (xb + yb);
-    return flops / 130e12 + moved / 2.5e12 < flops / 4e12;
+    return flops / 130e12 + moved / 2.5e12 < tiles / 4e12;
 }
 
 // Shapes whose channel counts keep every activation on 16-byte pixels and whole blocks, whatever the pointers: for the
