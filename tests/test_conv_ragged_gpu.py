@@ -16,8 +16,8 @@ pytestmark = pytest.mark.gpu
 SHAPES = [(2, 9, 7, 1, 1, 3, 1, 1), (2, 9, 7, 4, 4, 3, 1, 1), (3, 8, 8, 8, 36, 3, 1, 1), (2, 11, 6, 17, 33, 3, 1, 2),
           (2, 12, 12, 20, 12, 5, 2, 1), (1, 10, 9, 30, 31, 3, 1, 1), (2, 7, 9, 33, 130, 1, 0, 1), (3, 15, 11, 40, 72, 3, 1, 1),
           (2, 9, 9, 36, 1, 3, 1, 2), (2, 13, 13, 65, 100, 1, 0, 2), (2, 14, 14, 48, 80, 5, 2, 2), (1, 9, 30, 129, 67, 3, 1, 1),
-          (2, 6, 6, 100, 260, 3, 1, 1), (2, 17, 17, 3, 10, 7, 3, 2), (40, 5, 5, 12, 24, 3, 0, 1), (2, 8, 8, 16, 16, 3, 1, 1)]
-
+          (2, 6, 6, 100, 260, 3, 1, 1), (2, 17, 17, 3, 10, 7, 3, 2), (40, 5, 5, 12, 24, 3, 0, 1), (2, 8, 8, 16, 16, 3, 1, 1),
+          (4, 61, 53, 12, 192, 3, 1, 1), (8, 61, 53, 4, 64, 3, 1, 1)]      # whole 16-byte pixels, large enough to be lowered
 
 @pytest.mark.parametrize("layout,w_layout", [("NHWC", "KRSC"), ("NHWC", "CRSK"), ("NCHW", "KCRS")])
 @pytest.mark.parametrize("shape", SHAPES)
