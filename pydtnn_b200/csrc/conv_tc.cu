@@ -286,6 +286,7 @@ struct PrepParams {
     int r0, rstep, s0, sstep;        // real tap of virtual tap (r, s): (r0 + rstep*r, s0 + sstep*s)
     int Rreal, Sreal;                // extent of the real filter
     int Cp;                          // C up to a multiple of 32 (set by run_fwd)
+    bool round;                      // wherever the filter is split, hi is rounded to nearest (see taps_innermost)
 };
 
 // Also clears `nflags` ints at `flags` (the hand-over flags of the balanced mode of the convolution kernel that
@@ -455,6 +456,23 @@ enum { TCM_FWD = 0, TCM_WGRAD = 1 };
 //  TCB_RAW_MN the same with the channel axis being the GEMM N axis: MN-major boxes as in WGRAD
 enum { TCB_SPLIT = 0, TCB_RAW_K = 1, TCB_RAW_MN = 2 };
 
+// lo of four B values that stay in place as their hi halves: the tensor core reads the upper 19 bits of them.
+__device__ __forceinline__ float4 tc_lo_of_truncated(const float4 q) {
+    return make_float4(q.x - __uint_as_float(__float_as_uint(q.x) & 0xFFFFE000u), q.y - __uint_as_float(__float_as_uint(q.y) & 0xFFFFE000u),
+                       q.z - __uint_as_float(__float_as_uint(q.z) & 0xFFFFE000u), q.w - __uint_as_float(__float_as_uint(q.w) & 0xFFFFE000u));
+}
+// to_tf32_rn in two integer operations: the conversion instruction runs at a fraction of their rate.  (A NaN may leave here
+// as a number; its lo half is still a NaN.)
+__device__ __forceinline__ float tc_rounded_hi(float v) { return __uint_as_float((__float_as_uint(v) + 0x1000u) & 0xFFFFE000u); }
+// The same with hi rounded to nearest: lo takes either sign and is half as large, and so is the
+// dropped product of two lo halves.  q becomes hi, to be written back.
+__device__ __forceinline__ float4 tc_split_rounded(float4& q) {
+    const float4 h = make_float4(tc_rounded_hi(q.x), tc_rounded_hi(q.y), tc_rounded_hi(q.z), tc_rounded_hi(q.w));
+    const float4 l = make_float4(q.x - h.x, q.y - h.y, q.z - h.z, q.w - h.w);
+    q = h;
+    return l;
+}
+
 #define TC_CHUNK 8   // k-blocks accumulated in tensor memory before the partial sum is drained
 
 // Division by a launch constant: q = (n * mul) >> 32 >> shift for 0 <= n < 2^31 (round-up reciprocal: with s = ceil(log2 d) and
@@ -500,6 +518,7 @@ struct TcParams {
     // partial tile in `sk_partial` (slot = CTA index, [BN/4][128 rows][4] floats) and raise `sk_flags` (4 per slot, one per
     // drain warp); the owner adds the partials in CTA order and runs the epilogue.
     int tap_r0, tap_rstep, tap_s0, tap_sstep, tap_sreal;   // raw-filter modes: real tap of virtual tap (r, s)
+    int b_round;               // raw-filter modes: hi halves of the filter rounded to nearest, as in the split copies
     int sk;
     float* sk_partial;
     int* sk_flags;
@@ -1008,17 +1027,13 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             ok = mbar_wait(bres_bar, 0, abort_flag, &g_tc_status, TC_ERR_FULL);
             if (ok) {
                 for (int kb = 0; kb < p.kblocks; kb++) {
-                    const float4* b_hi = (const float4*)(smem + L::RES_OFFSET + kb * 2 * L::B_BYTES);
+                    float4* b_hi = (float4*)(smem + L::RES_OFFSET + kb * 2 * L::B_BYTES);
                     float4* b_lo = (float4*)(smem + L::RES_OFFSET + kb * 2 * L::B_BYTES + L::B_BYTES);
 #pragma unroll
                     for (int i = 0; i < L::B_BYTES / 16 / 128; i++) {
-                        const float4 q = b_hi[t + i * 128];
-                        float4 l;
-                        l.x = q.x - __uint_as_float(__float_as_uint(q.x) & 0xFFFFE000u);
-                        l.y = q.y - __uint_as_float(__float_as_uint(q.y) & 0xFFFFE000u);
-                        l.z = q.z - __uint_as_float(__float_as_uint(q.z) & 0xFFFFE000u);
-                        l.w = q.w - __uint_as_float(__float_as_uint(q.w) & 0xFFFFE000u);
-                        b_lo[t + i * 128] = l;
+                        float4 q = b_hi[t + i * 128];
+                        if (p.b_round) { b_lo[t + i * 128] = tc_split_rounded(q); b_hi[t + i * 128] = q; }
+                        else b_lo[t + i * 128] = tc_lo_of_truncated(q);
                     }
                 }
                 fence_proxy_async();
@@ -1086,16 +1101,17 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 tmem_st_32x32(slot + 32, v);
                 if (SPLIT_B && RESKB == 0) {
                     float4* b_lo = (float4*)(smem + s * L::STAGE_BYTES + L::A_BYTES + L::B_BYTES);
+                    if (MODE == TCM_FWD && p.b_round) {
+                        float4* b_hi = (float4*)(smem + s * L::STAGE_BYTES + L::A_BYTES);
 #pragma unroll
-                    for (int i = 0; i < B_VEC; i++) {
-                        const float4 q = bq[i];
-                        if (do_db) { dbacc[i >> 1].x += q.x; dbacc[i >> 1].y += q.y; dbacc[i >> 1].z += q.z; dbacc[i >> 1].w += q.w; }
-                        float4 l;
-                        l.x = q.x - __uint_as_float(__float_as_uint(q.x) & 0xFFFFE000u);
-                        l.y = q.y - __uint_as_float(__float_as_uint(q.y) & 0xFFFFE000u);
-                        l.z = q.z - __uint_as_float(__float_as_uint(q.z) & 0xFFFFE000u);
-                        l.w = q.w - __uint_as_float(__float_as_uint(q.w) & 0xFFFFE000u);
-                        b_lo[t + i * 128] = l;
+                        for (int i = 0; i < B_VEC; i++) { b_lo[t + i * 128] = tc_split_rounded(bq[i]); b_hi[t + i * 128] = bq[i]; }
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < B_VEC; i++) {
+                            const float4 q = bq[i];
+                            if (do_db) { dbacc[i >> 1].x += q.x; dbacc[i >> 1].y += q.y; dbacc[i >> 1].z += q.z; dbacc[i >> 1].w += q.w; }
+                            b_lo[t + i * 128] = tc_lo_of_truncated(q);
+                        }
                     }
                     fence_proxy_async();
                 }
@@ -2067,6 +2083,10 @@ static int64_t fwd_stats_rows(int64_t M, int N, int64_t kblocks, bool may_balanc
 // Stride-2 data gradient of a 1x1 filter: the launch writes class (0, 0) and the zeros of the other three (TcParams::zfill).
 struct ZeroFill { int W, H; int64_t off_w, off_h; };
 
+// (co, ci, kh, kw) filters are split with hi rounded to nearest, in whichever place the split is made: a truncated hi (what the
+// tensor core reads of a raw tile) has 1.1 to 1.6 times the error against float64 on layers of 128 to 512 channels.
+static bool taps_innermost(const PrepParams& pp) { return pp.s_s == 1; }
+
 // A (co, ci, kh, kw) filter has no contiguous channel axis, so no tensor map can serve it.  Its K-major copy in real tap
 // order, [row][tap][C up to a multiple of 4], is a transpose either way round: (C x taps) per row when the rows are the
 // output channels, (C x rows * taps) when they are the input channels.  Then the strides of `pp` describe the copy.
@@ -2098,6 +2118,7 @@ static int run_fwd(const FwdLaunch& f, const void* act, const void* w, PrepParam
     if (!load_driver_entry_points()) return B2C_ERR_UNSUPPORTED;
     const int cblocks = (f.C + 31) / 32;
     pp.Cp = cblocks * 32;
+    pp.round = pp.round || taps_innermost(pp);
     // the tap strides of a filter with one tap mean nothing: a (co, ci, 1, 1) filter is a (co, 1, 1, ci) one
     if (pp.Rreal * pp.Sreal == 1) pp.s_s = pp.s_r = pp.s_row > pp.s_c ? pp.s_row : pp.s_c;
     const int64_t K = (int64_t)f.kh * f.kw * pp.Cp;
@@ -2160,6 +2181,7 @@ static int run_fwd(const FwdLaunch& f, const void* act, const void* w, PrepParam
         p.epi |= TC_EPI_VEC;
     p.out = out; p.o_sn = f.o_sn; p.o_sh = f.o_sh; p.o_sw = f.o_sw;
     p.tap_r0 = pp.r0; p.tap_rstep = pp.rstep; p.tap_s0 = pp.s0; p.tap_sstep = pp.sstep; p.tap_sreal = pp.Sreal;
+    p.b_round = pp.round;
     p.sk = sk; p.sk_flags = sk_flags; p.sk_partial = sk_partial; p.sk_selfclean = sk_bank ? 1 : 0;
     // dense rows (plain fprop / stride-1 dgrad): rows are a constant pitch apart in (n, i, j) order
     const bool dense = f.o_sw % 4 == 0 && f.o_sh == (int64_t)f.Q * f.o_sw && f.o_sn == (int64_t)f.P * f.Q * f.o_sw;
@@ -2264,7 +2286,7 @@ static int tc_fprop_nhwc(const Geo& g, const void* x, const void* w, const void*
 // Strided data gradient, all parity classes in one launch (MULTI kernel variants): up to four classes, every class
 // with at least one tap, filters read in place.  The tiles of the classes with the most taps come first in the tile
 // list, so the persistent CTAs end with the short ones.  Returns 1 when the shape does not qualify.
-static int tc_dgrad_classes_one_launch(const Geo& g, const WStride& wsd, const void* dy, const void* w, void* dx, cudaStream_t st)
+static int tc_dgrad_classes_one_launch(const Geo& g, const WStride& wsd, bool b_round, const void* dy, const void* w, void* dx, cudaStream_t st)
 {
     if (g.vstr * g.hstr > 4 || !load_driver_entry_points()) return 1;
     struct Cls { AxisClass a, b; int ia, ib; };
@@ -2307,7 +2329,7 @@ static int tc_dgrad_classes_one_launch(const Geo& g, const WStride& wsd, const v
     p.str_h = 1; p.str_w = 1; p.dil_h = 1; p.dil_w = 1;
     p.out = (float*)dx; p.o_sn = (int64_t)g.h * g.w * g.xp; p.o_sh = (int64_t)g.vstr * g.w * g.xp; p.o_sw = (int64_t)g.hstr * g.xp;
     p.tap_rstep = -g.vstr; p.tap_sstep = -g.hstr; p.tap_sreal = g.kw;
-    p.splits = 1; p.ncls = ncls;
+    p.splits = 1; p.ncls = ncls; p.b_round = b_round;
     int64_t tiles = 0;
     for (int i = 0; i < ncls; i++) {
         const AxisClass &ca = cls[i].a, &cb = cls[i].b;
@@ -2345,6 +2367,7 @@ static int tc_dgrad_nhwc(const Geo& g, const void* dy, const void* w, void* dx, 
     }
     // the classes share one K-major copy of a filter that needs one
     PrepParams whole{g.ci, g.co, g.kh, g.kw, wsd.sc, wsd.sk, wsd.sr, wsd.ss, 0, 1, 0, 1, g.kh, g.kw};
+    whole.round = taps_innermost(whole);
     {
         const uintptr_t base = align_up((uintptr_t)ws, 1024);
         const size_t fbytes = filter_split_bytes(g, B2C_PASS_DGRAD);
@@ -2360,7 +2383,7 @@ static int tc_dgrad_nhwc(const Geo& g, const void* dy, const void* w, void* dx, 
     // stride-1 convolution of dy with the sub-filter of the taps that reach it, written to its
     // strided positions of dx. Classes no tap reaches stay zero.
     {
-        int rc = tc_dgrad_classes_one_launch(g, wsd, dy, w, dx, st);
+        int rc = tc_dgrad_classes_one_launch(g, wsd, whole.round, dy, w, dx, st);
         if (rc != 1) return rc;            // 1: not applicable, one launch per class below
     }
     bool any_empty = false;
@@ -2376,7 +2399,7 @@ static int tc_dgrad_nhwc(const Geo& g, const void* dy, const void* w, void* dx, 
         // other classes' zeros next to its own rows, no clearing pass over dx
         AxisClass ca = axis_class(0, g.vstr, g.vpad, g.kh, g.h), cb = axis_class(0, g.hstr, g.hpad, g.kw, g.w);
         if (g.vstr == 2 && g.hstr == 2 && live == 1 && ca.cnt > 0 && cb.cnt > 0 && g.xp % 4 == 0 && ((uintptr_t)dx & 15) == 0) {
-            PrepParams pp{g.ci, g.co, ca.cnt, cb.cnt, wsd.sc, wsd.sk, wsd.sr, wsd.ss, ca.r0, -g.vstr, cb.r0, -g.hstr, g.kh, g.kw};
+            PrepParams pp{g.ci, g.co, ca.cnt, cb.cnt, wsd.sc, wsd.sk, wsd.sr, wsd.ss, ca.r0, -g.vstr, cb.r0, -g.hstr, g.kh, g.kw, 0, whole.round};
             FwdLaunch f{g.n, g.ho, g.wo, g.co, g.yp, ca.out_cnt, cb.out_cnt, g.ci, ca.cnt, cb.cnt, ca.dmin, cb.dmin,
                         ca.out_cnt, cb.out_cnt, 1, 1, 1, 1,
                         (int64_t)g.h * g.w * g.xp, (int64_t)g.vstr * g.w * g.xp, (int64_t)g.hstr * g.xp};
@@ -2393,7 +2416,7 @@ static int tc_dgrad_nhwc(const Geo& g, const void* dy, const void* w, void* dx, 
         for (int b = 0; b < g.hstr; b++) {
             AxisClass ca = axis_class(a, g.vstr, g.vpad, g.kh, g.h), cb = axis_class(b, g.hstr, g.hpad, g.kw, g.w);
             if (ca.out_cnt == 0 || cb.out_cnt == 0 || ca.cnt == 0 || cb.cnt == 0) continue;
-            PrepParams pp{g.ci, g.co, ca.cnt, cb.cnt, wsd.sc, wsd.sk, wsd.sr, wsd.ss, ca.r0, -g.vstr, cb.r0, -g.hstr, g.kh, g.kw};
+            PrepParams pp{g.ci, g.co, ca.cnt, cb.cnt, wsd.sc, wsd.sk, wsd.sr, wsd.ss, ca.r0, -g.vstr, cb.r0, -g.hstr, g.kh, g.kw, 0, whole.round};
             FwdLaunch f{g.n, g.ho, g.wo, g.co, g.yp, ca.out_cnt, cb.out_cnt, g.ci, ca.cnt, cb.cnt, ca.dmin, cb.dmin,
                         ca.out_cnt, cb.out_cnt, 1, 1, 1, 1,
                         (int64_t)g.h * g.w * g.xp, (int64_t)g.vstr * g.w * g.xp, (int64_t)g.hstr * g.xp};
