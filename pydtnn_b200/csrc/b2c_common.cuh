@@ -46,6 +46,7 @@ struct Geo {
     int n, h, w, ci, co, kh, kw, vpad, hpad, vstr, hstr, vdil, hdil;
     int ho, wo;
     int xp, yp;     // elements from one pixel to the next of a channel-last x (dx) and y (dy): ci and co, or more in padded copies
+    bool fine;      // the tensor-core engine sums this call at FMA precision (set by it, see tc_fine_sums)
     bool x_nchw;    // the channel-last pass reads an x that is still NCHW (few-channel layers that lower it)
     int64_t M, K;   // M = n*ho*wo, K = ci*kh*kw
 };
@@ -68,7 +69,7 @@ inline int make_geo(const b2c_conv_desc* d, Geo& g) {
     if (eh < 0 || ew < 0) return B2C_ERR_BAD_GEOMETRY;
     g.ho = eh / d->vstr + 1;
     g.wo = ew / d->hstr + 1;
-    g.xp = g.ci; g.yp = g.co; g.x_nchw = false;
+    g.xp = g.ci; g.yp = g.co; g.x_nchw = g.fine = false;
     g.M = (int64_t)g.n * g.ho * g.wo;
     g.K = (int64_t)g.ci * g.kh * g.kw;
     if (g.M > 0x7fffffffLL || g.K > 0x7fffffffLL || (int64_t)g.n * g.h * g.w > 0x7fffffffLL) return B2C_ERR_TOO_LARGE;
@@ -116,6 +117,7 @@ int channel_sum_v4(int n, int c, int hw, const void* src, void* dst, void* ws, s
 // tensor-core engine (conv_tc.cu)
 bool tc_supported(const Geo& g, int pass);
 bool tc_any_alignment(const Geo& g, int pass);
+bool tc_fine_sums(const Geo& g, int pass);
 int tc_wait_selftest(long long limit_cycles, cudaStream_t st);
 size_t tc_workspace_bytes(const Geo& g, int pass);
 int tc_fprop(const Geo& g, const void* x, const void* w, const void* bias, const b2c_bn_params* bn, int relu,

@@ -685,7 +685,9 @@ constexpr int TC_STREAM8 = 2;
 template <int STREAM> constexpr int tc_drain_warps() { return STREAM == TC_STREAM8 ? 8 : 4; }
 template <int STREAM> constexpr int tc_threads() { return (6 + tc_drain_warps<STREAM>()) * 32; }
 
-template <int MODE, int BN, int STAGES, bool SK, int SLABS, int BSRC, int STREAM, bool MULTI, int RESKB = 0>
+// FINE: sums at the precision of float32 FMAs (see tc_fine_sums): both operands split by rounding, each k-block summed in tensor
+// memory by itself, its small products first.
+template <int MODE, int BN, int STAGES, bool SK, int SLABS, int BSRC, int STREAM, bool MULTI, int RESKB = 0, bool FINE = false>
 __global__ void __launch_bounds__(tc_threads<STREAM>(), 1)
 conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b0,
                const __grid_constant__ CUtensorMap tmap_b1, const __grid_constant__ CUtensorMap tmap_out,
@@ -718,6 +720,8 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     constexpr int DW = tc_drain_warps<STREAM>();
     constexpr int TSLOTS = L::TSLOTS;
     static_assert(RESKB == 0 || (STREAM == TC_STREAM8 && BSRC != TCB_SPLIT), "resident filters: short-K streaming variant on the caller's filter");
+    static_assert(!FINE || (!SK && STREAM == 0 && RESKB == 0), "fine sums: chunked drain, whole tiles or split K loops");
+    constexpr int CHUNK = FINE ? 1 : TC_CHUNK;
     // STREAM variants serve tiles of at most TC_CHUNK k-blocks with dense outputs (see dispatch_fwd)
     static_assert(STREAM == 0 || (MODE == TCM_FWD && !SK), "the streaming epilogue is a whole-tile forward variant");
     extern __shared__ uint8_t smem_raw[];
@@ -1002,7 +1006,32 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                     gc++;
                 }
                 };
-                if (left > BN - 16 && (MODE == TCM_WGRAD || p.ktail == 4)) issue_tile(std::true_type{});
+                if constexpr (FINE) {
+                    // A k-block to a buffer: the twelve products in two runs, the eight small ones (lo*hi, hi*lo) while the sum is
+                    // small and an addition's truncation loses little, then the four large ones.
+                    int cb = MODE == TCM_WGRAD ? 0 : w.kb_b - p.f_cb.div(w.kb_b) * p.cblocks;
+                    for (int kb = w.kb_b; kb < w.kb_e; kb++) {
+                        const int b = gc & 1, s = ring.s;
+                        ok = mbar_wait(&tempty_bar[b], ((gc >> 1) & 1) ^ 1, abort_flag, &g_tc_status, TC_ERR_TEMPTY);
+                        if (ok && !ahead) ok = mbar_wait(&xform_bar[s], ring.phase, abort_flag, &g_tc_status, TC_ERR_XFORM);
+                        if (!ok) break;
+                        tc_fence_after();
+                        const uint64_t b_hi = b_desc0 + (uint64_t)(s * (L::STAGE_BYTES >> 4)), b_lo = b_hi + (L::B_BYTES >> 4);
+                        const uint32_t d = tmem_base + (uint32_t)(b * BN), a_hi = tmem_base + (uint32_t)(L::TMEM_A_COL + s * 64), a_lo = a_hi + 32;
+                        const int ks = MODE == TCM_FWD && cb == p.cblocks - 1 ? p.ktail : 4;
+                        ring.next();
+                        for (int k = 0; k < ks; k++) {
+                            umma_tf32_ts(d, a_lo + k * 8, b_hi + k * KADV, idesc, k > 0);
+                            umma_tf32_ts(d, a_hi + k * 8, b_lo + k * KADV, idesc, 1u);
+                        }
+                        for (int k = 0; k < ks; k++) umma_tf32_ts(d, a_hi + k * 8, b_hi + k * KADV, idesc, 1u);
+                        ahead = mbar_test(&xform_bar[ring.s], ring.phase);
+                        if (++cb == p.cblocks) cb = 0;
+                        umma_commit(&empty_bar[s]);
+                        umma_commit(&tfull_bar[b]);
+                        gc++;
+                    }
+                } else if (left > BN - 16 && (MODE == TCM_WGRAD || p.ktail == 4)) issue_tile(std::true_type{});
                 else issue_tile(std::false_type{});
             }
         }
@@ -1089,6 +1118,13 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                     for (int i = 0; i < B_VEC; i++) bq[i] = b_hi[t + i * 128];
                 }
                 const uint32_t slot = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(L::TMEM_A_COL + ts * 64);
+                uint32_t low[32];
+#pragma unroll
+                for (int j = 0; j < 32; j++) {
+                    const float a = __uint_as_float(v[j]);
+                    if (FINE) { const float h = tc_rounded_hi(a); low[j] = __float_as_uint(a - h); v[j] = __float_as_uint(h); }
+                    else low[j] = __float_as_uint(a - __uint_as_float(v[j] & 0xFFFFE000u));
+                }
                 tmem_st_32x32(slot, v);              // hi: the tensor core reads the upper 19 bits
                 if (RESKB) {
                     // The store above took every lane's values from its registers, so the reads of the stage are done (a load
@@ -1096,12 +1132,10 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&afree_bar[s]);
                 }
-#pragma unroll
-                for (int j = 0; j < 32; j++) v[j] = __float_as_uint(__uint_as_float(v[j]) - __uint_as_float(v[j] & 0xFFFFE000u));
-                tmem_st_32x32(slot + 32, v);
+                tmem_st_32x32(slot + 32, low);
                 if (SPLIT_B && RESKB == 0) {
                     float4* b_lo = (float4*)(smem + s * L::STAGE_BYTES + L::A_BYTES + L::B_BYTES);
-                    if (MODE == TCM_FWD && p.b_round) {
+                    if (FINE || (MODE == TCM_FWD && p.b_round)) {
                         float4* b_hi = (float4*)(smem + s * L::STAGE_BYTES + L::A_BYTES);
 #pragma unroll
                         for (int i = 0; i < B_VEC; i++) { b_lo[t + i * 128] = tc_split_rounded(bq[i]); b_hi[t + i * 128] = bq[i]; }
@@ -1271,7 +1305,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 gc++;
                 store_stats();
             } else {
-            const int nchunks = (w.kb_e - w.kb_b + TC_CHUNK - 1) / TC_CHUNK;
+            const int nchunks = (w.kb_e - w.kb_b + CHUNK - 1) / CHUNK;
             float acc[BN];
             for (int c = 0; c < nchunks && ok; c++, gc++) {
                 const int b = gc & 1;
@@ -1917,14 +1951,14 @@ static size_t tc_workspace_bytes_nhwc(const Geo& g, int pass)
            align_up((size_t)pl.splits * 4 * round4(g.co) * sizeof(float), 1024);
 }
 
-template <int MODE, int BN, int STAGES, bool SK, int SLABS, int BSRC, int STREAM = 0, bool MULTI = false, int RESKB = 0>
+template <int MODE, int BN, int STAGES, bool SK, int SLABS, int BSRC, int STREAM = 0, bool MULTI = false, int RESKB = 0, bool FINE = false>
 static int launch_tc(const CUtensorMap& ma, const CUtensorMap& mb0, const CUtensorMap& mb1, const CUtensorMap& mo, const TcParams& p, int splits, cudaStream_t st,
                      const CUtensorMap* ma3 = nullptr)
 {
     using L = TcSmem<BN, STAGES, SLABS, tc_drain_warps<STREAM>(), RESKB>;
     static PerDeviceOnce attr;
     {
-        cudaError_t e = attr.run([] { return cudaFuncSetAttribute(conv_tc_kernel<MODE, BN, STAGES, SK, SLABS, BSRC, STREAM, MULTI, RESKB>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL); });
+        cudaError_t e = attr.run([] { return cudaFuncSetAttribute(conv_tc_kernel<MODE, BN, STAGES, SK, SLABS, BSRC, STREAM, MULTI, RESKB, FINE>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL); });
         if (e != cudaSuccess) { set_cuda_error(e, "cudaFuncSetAttribute(conv_tc_kernel)"); return B2C_ERR_CUDA; }
     }
     const int sm_count = tc_sm_count();
@@ -1940,13 +1974,18 @@ static int launch_tc(const CUtensorMap& ma, const CUtensorMap& mb0, const CUtens
 #endif
     int grid = q.sk ? sm_count : (int)(tiles < sm_count ? tiles : sm_count);     // one persistent CTA per SM
     if ((q.stats && q.stats_cta) || RESKB) grid -= grid % ((p.N + BN - 1) / BN);    // a CTA keeps its column tile
-    launch_pdl(conv_tc_kernel<MODE, BN, STAGES, SK, SLABS, BSRC, STREAM, MULTI, RESKB>, grid, tc_threads<STREAM>(), L::TOTAL, st, ma, mb0, mb1, mo, ma3 ? *ma3 : ma, q);
+    launch_pdl(conv_tc_kernel<MODE, BN, STAGES, SK, SLABS, BSRC, STREAM, MULTI, RESKB, FINE>, grid, tc_threads<STREAM>(), L::TOTAL, st, ma, mb0, mb1, mo, ma3 ? *ma3 : ma, q);
     return check_launch("conv_tc_kernel");
 }
 
 template <int BSRC>
-static int dispatch_fwd(int bn, const CUtensorMap& ma, const CUtensorMap& mb0, const CUtensorMap& mb1, const CUtensorMap& mo, const TcParams& p, cudaStream_t st)
+static int dispatch_fwd(int bn, bool fine, const CUtensorMap& ma, const CUtensorMap& mb0, const CUtensorMap& mb1, const CUtensorMap& mo, const TcParams& p, cudaStream_t st)
 {
+    if (fine) {
+        const int splits = p.kper ? (p.kblocks + p.kper - 1) / p.kper : 1;
+        if (bn == 64) return launch_tc<TCM_FWD, 64, 6, false, 2, BSRC, 0, false, 0, true>(ma, mb0, mb1, mo, p, splits, st);
+        return launch_tc<TCM_FWD, 128, 4, false, 2, BSRC, 0, false, 0, true>(ma, mb0, mb1, mo, p, splits, st);
+    }
     if (p.sk) {
         if (bn == 64) return launch_tc<TCM_FWD, 64, 6, true, 2, BSRC>(ma, mb0, mb1, mo, p, 1, st);
         return launch_tc<TCM_FWD, 128, 4, true, 2, BSRC>(ma, mb0, mb1, mo, p, 1, st);
@@ -1986,8 +2025,12 @@ static int dispatch_fwd(int bn, const CUtensorMap& ma, const CUtensorMap& mb0, c
     return launch_tc<TCM_FWD, 128, 4, false, 2, BSRC>(ma, mb0, mb1, mo, p, 1, st);
 }
 
-static int dispatch_wgrad(int bn, const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mo, const TcParams& p, int splits, cudaStream_t st)
+static int dispatch_wgrad(int bn, bool fine, const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mo, const TcParams& p, int splits, cudaStream_t st)
 {
+    if (fine) {
+        if (bn == 64) return launch_tc<TCM_WGRAD, 64, 6, false, 2, TCB_SPLIT, 0, false, 0, true>(ma, mb, mb, mo, p, splits, st);
+        return launch_tc<TCM_WGRAD, 128, 4, false, 2, TCB_SPLIT, 0, false, 0, true>(ma, mb, mb, mo, p, splits, st);
+    }
     if (bn == 64) return launch_tc<TCM_WGRAD, 64, 6, false, 2, TCB_SPLIT>(ma, mb, mb, mo, p, splits, st);
     return launch_tc<TCM_WGRAD, 128, 4, false, 2, TCB_SPLIT>(ma, mb, mb, mo, p, splits, st);
 }
@@ -2046,7 +2089,7 @@ struct StatsOut { float* sums; };
 // because tiles x splits is at most one CTA per SM.  Narrow tiles only pay where the wide ones leave the chip idle (single
 // images, late layers of small batches).
 struct FwdPlan { int bn; bool sk; int kper; };
-static FwdPlan fwd_plan(int64_t M, int N, int64_t kblocks, bool may_share)
+static FwdPlan fwd_plan(int64_t M, int N, int64_t kblocks, bool may_share, bool fine = false)
 {
     const int G = tc_sm_count();
     FwdPlan best{128, false, 0};
@@ -2058,7 +2101,7 @@ static FwdPlan fwd_plan(int64_t M, int N, int64_t kblocks, bool may_share)
         offer((double)(rounds * kblocks) * kb + drain, false, 0);
         if (!may_share) continue;
         const double shared = (double)G / (double)tiles;         // CTAs on one tile
-        if (tiles * kblocks >= 4 * (int64_t)G)
+        if (!fine && tiles * kblocks >= 4 * (int64_t)G)
             offer(((double)(tiles * kblocks) / G * kb + 11.0 + (shared > 2.0 ? 4.5 * (shared - 2.0) : 0.0) + drain) / tc_balance_threshold(), true, 0);
         for (int64_t s = 2; s * tiles <= G && s <= kblocks; s++) {
             const int64_t kper = (kblocks + s - 1) / s;
@@ -2109,6 +2152,7 @@ static int kmajor_filter_copy(PrepParams& pp, const void*& w, float* buf, cudaSt
 struct FwdLaunch {
     int n, ah, aw, C, ap, P, Q, N, kh, kw, low_h, low_w, cnt_h, cnt_w, str_h, str_w, dil_h, dil_w;     // ap: pixel pitch of act
     int64_t o_sn, o_sh, o_sw;
+    bool fine;
 };
 
 static int run_fwd(const FwdLaunch& f, const void* act, const void* w, PrepParams pp, const void* bias,
@@ -2134,7 +2178,7 @@ static int run_fwd(const FwdLaunch& f, const void* act, const void* w, PrepParam
     unsigned int* sk_bank = tc_sm_count() * 4 <= TC_SYNC_FLAGS ? tc_sync_bank(st) : nullptr;
     if (sk_bank) sk_flags = (int*)sk_bank;
     const bool room = base + 2 * fbytes + sk_bytes() <= (uintptr_t)ws + ws_bytes;
-    const FwdPlan plan = fwd_plan((int64_t)f.n * f.P * f.Q, f.N, (int64_t)f.kh * f.kw * cblocks, !filters_ready && room && !zf);
+    const FwdPlan plan = fwd_plan((int64_t)f.n * f.P * f.Q, f.N, (int64_t)f.kh * f.kw * cblocks, !filters_ready && room && !zf, f.fine);
     const int BN = plan.bn, sk = plan.sk, kper = plan.kper;
     // The filter itself serves as the B operand when its layout allows a tensor map over it (the channel axis
     // that is contiguous decides K-major or MN-major); otherwise hi/lo copies in the GEMM layout are written first.
@@ -2205,9 +2249,9 @@ static int run_fwd(const FwdLaunch& f, const void* act, const void* w, PrepParam
         fwd_stats_rows(p.M, p.N, p.kblocks, !filters_ready, &by_cta);
         p.stats_cta = by_cta ? 1 : 0;       // by_cta implies whole tiles
     }
-    const int rc = bsrc == TCB_RAW_K ? dispatch_fwd<TCB_RAW_K>(BN, ma, mbh, mbl, mo, p, st)
-                 : bsrc == TCB_RAW_MN ? dispatch_fwd<TCB_RAW_MN>(BN, ma, mbh, mbl, mo, p, st)
-                 : dispatch_fwd<TCB_SPLIT>(BN, ma, mbh, mbl, mo, p, st);
+    const int rc = bsrc == TCB_RAW_K ? dispatch_fwd<TCB_RAW_K>(BN, f.fine, ma, mbh, mbl, mo, p, st)
+                 : bsrc == TCB_RAW_MN ? dispatch_fwd<TCB_RAW_MN>(BN, f.fine, ma, mbh, mbl, mo, p, st)
+                 : dispatch_fwd<TCB_SPLIT>(BN, f.fine, ma, mbh, mbl, mo, p, st);
     if (rc || !kper) return rc;
     FinishParams fp{p.M, p.N, p.P, p.Q, splits, round4(f.N), mrows * round4(f.N), sk_partial, out, f.o_sn, f.o_sh, f.o_sw,
                     p.bias, p.mean, p.inv_std, p.gamma, p.beta, relu, stats ? stats->sums : nullptr};
@@ -2273,13 +2317,13 @@ static int tc_fprop_nhwc(const Geo& g, const void* x, const void* w, const void*
         rc = check_launch("tc_prep_filter_lowered_kernel");
         if (rc) return rc;
         PrepParams none{};
-        FwdLaunch f{g.n, g.ho, g.wo, Kp, Kp, g.ho, g.wo, g.co, 1, 1, 0, 0, g.ho, g.wo, 1, 1, 1, 1, g.ho * g.wo * yp, g.wo * yp, yp};
+        FwdLaunch f{g.n, g.ho, g.wo, Kp, Kp, g.ho, g.wo, g.co, 1, 1, 0, 0, g.ho, g.wo, 1, 1, 1, 1, g.ho * g.wo * yp, g.wo * yp, yp, g.fine};
         return run_fwd(f, rows, nullptr, none, bias, bn, relu, (float*)y, (void*)w_hi, 2 * fbytes + 1024, st, true, stats);
     }
     PrepParams pp{g.co, g.ci, g.kh, g.kw, wsd.sk, wsd.sc, wsd.sr, wsd.ss, 0, 1, 0, 1, g.kh, g.kw};
     FwdLaunch f{g.n, g.h, g.w, g.ci, g.xp, g.ho, g.wo, g.co, g.kh, g.kw, -g.vpad, -g.hpad,
                 g.h + 2 * g.vpad - (g.kh - 1) * g.vdil, g.w + 2 * g.hpad - (g.kw - 1) * g.hdil,
-                g.vstr, g.hstr, g.vdil, g.hdil, g.ho * g.wo * yp, g.wo * yp, yp};
+                g.vstr, g.hstr, g.vdil, g.hdil, g.ho * g.wo * yp, g.wo * yp, yp, g.fine};
     return run_fwd(f, x, w, pp, bias, bn, relu, (float*)y, ws, ws_bytes, st, false, stats);
 }
 
@@ -2346,6 +2390,14 @@ static int tc_dgrad_classes_one_launch(const Geo& g, const WStride& wsd, bool b_
     p.cls_tile0[ncls] = (int)tiles;
     // launch-wide fields the kernel still reads
     p.M = p.cls_M[0]; p.P = p.cls_P[0]; p.Q = p.cls_Q[0]; p.kblocks = p.cls_kblocks[0]; p.S = p.cls_S[0];
+    if (g.fine) {
+        if (bsrc == TCB_RAW_K) {
+            if (BN == 64) return launch_tc<TCM_FWD, 64, 6, false, 2, TCB_RAW_K, 0, true, 0, true>(ma[0], mb, ma[1], ma[2], p, 1, st, &ma[3]);
+            return launch_tc<TCM_FWD, 128, 4, false, 2, TCB_RAW_K, 0, true, 0, true>(ma[0], mb, ma[1], ma[2], p, 1, st, &ma[3]);
+        }
+        if (BN == 64) return launch_tc<TCM_FWD, 64, 6, false, 2, TCB_RAW_MN, 0, true, 0, true>(ma[0], mb, ma[1], ma[2], p, 1, st, &ma[3]);
+        return launch_tc<TCM_FWD, 128, 4, false, 2, TCB_RAW_MN, 0, true, 0, true>(ma[0], mb, ma[1], ma[2], p, 1, st, &ma[3]);
+    }
     if (bsrc == TCB_RAW_K) {
         if (BN == 64) return launch_tc<TCM_FWD, 64, 6, false, 2, TCB_RAW_K, 0, true>(ma[0], mb, ma[1], ma[2], p, 1, st, &ma[3]);
         return launch_tc<TCM_FWD, 128, 4, false, 2, TCB_RAW_K, 0, true>(ma[0], mb, ma[1], ma[2], p, 1, st, &ma[3]);
@@ -2362,7 +2414,7 @@ static int tc_dgrad_nhwc(const Geo& g, const void* dy, const void* w, void* dx, 
         const int pv = (g.kh - 1) * g.vdil - g.vpad, ph = (g.kw - 1) * g.hdil - g.hpad;
         PrepParams pp{g.ci, g.co, g.kh, g.kw, wsd.sc, wsd.sk, wsd.sr, wsd.ss, g.kh - 1, -1, g.kw - 1, -1, g.kh, g.kw};
         FwdLaunch f{g.n, g.ho, g.wo, g.co, g.yp, g.h, g.w, g.ci, g.kh, g.kw, -pv, -ph, g.h, g.w, 1, 1, g.vdil, g.hdil,
-                    (int64_t)g.h * g.w * g.xp, (int64_t)g.w * g.xp, (int64_t)g.xp};
+                    (int64_t)g.h * g.w * g.xp, (int64_t)g.w * g.xp, (int64_t)g.xp, g.fine};
         return run_fwd(f, dy, w, pp, nullptr, nullptr, 0, (float*)dx, ws, ws_bytes, st);
     }
     // the classes share one K-major copy of a filter that needs one
@@ -2402,7 +2454,7 @@ static int tc_dgrad_nhwc(const Geo& g, const void* dy, const void* w, void* dx, 
             PrepParams pp{g.ci, g.co, ca.cnt, cb.cnt, wsd.sc, wsd.sk, wsd.sr, wsd.ss, ca.r0, -g.vstr, cb.r0, -g.hstr, g.kh, g.kw, 0, whole.round};
             FwdLaunch f{g.n, g.ho, g.wo, g.co, g.yp, ca.out_cnt, cb.out_cnt, g.ci, ca.cnt, cb.cnt, ca.dmin, cb.dmin,
                         ca.out_cnt, cb.out_cnt, 1, 1, 1, 1,
-                        (int64_t)g.h * g.w * g.xp, (int64_t)g.vstr * g.w * g.xp, (int64_t)g.hstr * g.xp};
+                        (int64_t)g.h * g.w * g.xp, (int64_t)g.vstr * g.w * g.xp, (int64_t)g.hstr * g.xp, g.fine};
             ZeroFill zf{g.w, g.h, (int64_t)g.xp, (int64_t)g.w * g.xp};
             int rc = run_fwd(f, dy, w, pp, nullptr, nullptr, 0, (float*)dx, ws, ws_bytes, st, false, nullptr, &zf);
             if (rc != B2C_ERR_UNSUPPORTED) return rc;
@@ -2419,7 +2471,7 @@ static int tc_dgrad_nhwc(const Geo& g, const void* dy, const void* w, void* dx, 
             PrepParams pp{g.ci, g.co, ca.cnt, cb.cnt, wsd.sc, wsd.sk, wsd.sr, wsd.ss, ca.r0, -g.vstr, cb.r0, -g.hstr, g.kh, g.kw, 0, whole.round};
             FwdLaunch f{g.n, g.ho, g.wo, g.co, g.yp, ca.out_cnt, cb.out_cnt, g.ci, ca.cnt, cb.cnt, ca.dmin, cb.dmin,
                         ca.out_cnt, cb.out_cnt, 1, 1, 1, 1,
-                        (int64_t)g.h * g.w * g.xp, (int64_t)g.vstr * g.w * g.xp, (int64_t)g.hstr * g.xp};
+                        (int64_t)g.h * g.w * g.xp, (int64_t)g.vstr * g.w * g.xp, (int64_t)g.hstr * g.xp, g.fine};
             float* out = (float*)dx + ((int64_t)a * g.w + b) * g.xp;
             int rc = run_fwd(f, dy, w, pp, nullptr, nullptr, 0, out, ws, ws_bytes, st);
             if (rc) return rc;
@@ -2487,11 +2539,11 @@ static int tc_wgrad_nhwc(const Geo& g, const void* x, const void* dy, void* dw, 
     if (pl.splits == 1 && !low && !exchanged && g.kh * g.kw == 1 && wsd.sk == 1 && wsd.sc % 4 == 0 && ((uintptr_t)dw & 15) == 0 && p.tma_store &&
         make_map_out(&mo, dw, 1, (uint64_t)g.ci, (uint64_t)g.co, (uint64_t)wsd.sc)) {
         p.db_partial = nullptr;
-        const int rc = dispatch_wgrad(pl.bn, ma, mb, mo, p, 1, st);
+        const int rc = dispatch_wgrad(pl.bn, g.fine, ma, mb, mo, p, 1, st);
         if (rc || !db) return rc;
         return channel_sum_pitched(g.M, g.co, g.yp, (const float*)dy, (float*)db, partial, pbytes + cs, st);
     }
-    int rc = dispatch_wgrad(pl.bn, ma, mb, mo, p, pl.splits, st);
+    int rc = dispatch_wgrad(pl.bn, g.fine, ma, mb, mo, p, pl.splits, st);
     if (rc) return rc;
     WgradReduceParams rp{Krows, g.co, low ? g.ci : Cp, g.kw, pl.splits, wsd.sk, wsd.sc, wsd.sr, wsd.ss, low ? (int)g.K : Krows, g.ci, Np, pl.splits * 4};
     const int db_row = db ? 1 : 0;
@@ -2682,9 +2734,31 @@ static Copies tc_copies(const Geo& g, int pass)
     c.yb = c.y ? act_bytes(g.n, g.ho, g.wo, round4(g.co)) : 0;
     return c;
 }
-static Geo copied_geo(const Geo& g, const Copies& c)
+// Which passes sum at the precision of float32 FMAs (the kernel's FINE form): those that the FMA engine would run as well or
+// better if this engine's sums of 256 products in tensor memory, ten times less accurate, were all it had to offer: channel
+// counts that are no whole blocks, fully connected layers of few rows, layers of NCHW networks too small to pay for copies of
+// their activations at 130 against 26 TFLOP/s.  Errors against float64 (2-norms, 100 layers drawn over the sizes of a sweep):
+// FMA engine 1e-7 to 4e-7, 256-product sums 6e-7 to 2.1e-6, this form 0.9e-7 to 2e-7.  It costs 75x43 40->72 3x3 layers 27 us
+// of 77 (the FMA engine: 378), a 64 x 4096 x 1000 fully connected layer 5 of 39 (124).
+bool tc_fine_sums(const Geo& g, int pass)
+{
+    if (g.dtype != B2C_F32) return false;
+    const bool x_blocks = g.ci % 32 == 0 || (g.ci <= 16 && g.K <= 1024 && (int64_t)g.M * lowered_kp(g) * 4 <= (int64_t)3 << 30);
+    const bool blocks = pass == B2C_PASS_FPROP ? x_blocks && g.co % 4 == 0
+                      : pass == B2C_PASS_DGRAD ? g.co % 32 == 0 && g.ci % 4 == 0 : x_blocks && g.co % 32 == 0;
+    if (!blocks) return true;
+    if (g.engine != B2C_ENGINE_AUTO) return false;
+    if (g.h == 1 && g.w == 1 && g.kh == 1 && g.kw == 1 && g.vpad == 0 && g.hpad == 0 && g.n <= 128)
+        return pass == B2C_PASS_WGRAD || (pass == B2C_PASS_FPROP ? g.co : g.ci) <= 1024;
+    if (g.layout == B2C_LAYOUT_NHWC && g.w_layout != B2C_W_KCRS) return false;      // KCRS: a layer of an NCHW network on channel-last activations
+    const double flops = 2.0 * (double)g.M * (double)g.K * g.co, moved = 8.0 * ((double)g.n * g.h * g.w * g.ci + (double)g.M * g.co);
+    return flops / 130e12 + moved / 2.5e12 >= flops / 26e12;
+}
+
+static Geo copied_geo(const Geo& g, const Copies& c, int pass)
 {
     Geo q = as_nhwc(g);
+    q.fine = tc_fine_sums(g, pass);
     if (c.x) q.xp = round4(g.ci);
     else q.x_nchw = g.layout == B2C_LAYOUT_NCHW;
     if (c.y) q.yp = round4(g.co);
@@ -2732,11 +2806,17 @@ bool tc_any_alignment(const Geo& g, int pass)
     return (c.x || g.ci % 32 == 0 || lowered_ok(g)) && g.co % 32 == 0;
 }
 
+static size_t kept_lowered_bytes(const Geo& g) { return lowered_ok(g) ? align_up((size_t)g.M * lowered_kp(g) * sizeof(float), 1024) : 0; }
+
 size_t tc_workspace_bytes(const Geo& g, int pass)
 {
     const Copies c = tc_copies(g, pass);
-    if (!c.x && !c.y) return tc_workspace_bytes_nhwc(g, pass);
-    return c.xb + c.yb + 1024 + tc_workspace_bytes_nhwc(copied_geo(g, c), pass);
+    size_t inner = tc_workspace_bytes_nhwc(copied_geo(g, c, pass), pass);
+    if (pass == B2C_PASS_WGRAD && tc_fine_sums(g, pass)) {
+        const size_t sums = kept_lowered_bytes(g) + 1024 + channel_sum_workspace_bytes(g.n, g.co, g.ho * g.wo);
+        if (sums > inner) inner = sums;
+    }
+    return c.x || c.y ? c.xb + c.yb + 1024 + inner : inner;
 }
 
 // workspace of a call with copies: [x or dx, channel-last][y or dy, channel-last][workspace of the channel-last pass]
@@ -2759,7 +2839,7 @@ static int tc_fprop_any(const Geo& g, const void* x, const void* w, const void* 
     CopyWs t;
     if (!copy_ws(c, ws, ws_bytes, t)) return B2C_ERR_WORKSPACE_TOO_SMALL;
     if (c.x) { const int rc = copy_in(g, x, t.x, g.h * g.w, g.ci, st); if (rc) return rc; }
-    const int rc = tc_fprop_nhwc(copied_geo(g, c), c.x ? t.x : x, w, bias, bn, relu, c.y ? t.y : y, t.inner, t.inner_bytes, st, stats);
+    const int rc = tc_fprop_nhwc(copied_geo(g, c, B2C_PASS_FPROP), c.x ? t.x : x, w, bias, bn, relu, c.y ? t.y : y, t.inner, t.inner_bytes, st, stats);
     if (rc || !c.y) return rc;
     return copy_out(g, t.y, y, g.ho * g.wo, g.co, st);
 }
@@ -2768,7 +2848,7 @@ static int tc_fprop_any(const Geo& g, const void* x, const void* w, const void* 
 // engine only).  Buffer: [rows][2][co] floats, rows as fwd_stats_rows says.
 size_t tc_stats_bytes(const Geo& g)
 {
-    if (g.layout != B2C_LAYOUT_NHWC || !tc_supported_nhwc(g, B2C_PASS_FPROP) || g.co % 4) return 0;
+    if (g.layout != B2C_LAYOUT_NHWC || !tc_supported_nhwc(g, B2C_PASS_FPROP) || tc_fine_sums(g, B2C_PASS_FPROP)) return 0;
     const bool lowered = lowered_ok(g);         // few-channel layers run as a 1x1 convolution over the lowered matrix
     const int64_t kblocks = lowered ? lowered_kp(g) / 32 : (int64_t)g.kh * g.kw * (round32(g.ci) / 32);
     return (size_t)fwd_stats_rows(g.M, g.co, kblocks, !lowered, nullptr) * 2 * g.co * sizeof(float);
@@ -2797,7 +2877,7 @@ int tc_dgrad(const Geo& g, const void* dy, const void* w, void* dx, void* ws, si
     CopyWs t;
     if (!copy_ws(c, ws, ws_bytes, t)) return B2C_ERR_WORKSPACE_TOO_SMALL;
     if (c.y) { const int rc = copy_in(g, dy, t.y, g.ho * g.wo, g.co, st); if (rc) return rc; }
-    const int rc = tc_dgrad_nhwc(copied_geo(g, c), c.y ? t.y : dy, w, c.x ? t.x : dx, t.inner, t.inner_bytes, st);
+    const int rc = tc_dgrad_nhwc(copied_geo(g, c, B2C_PASS_DGRAD), c.y ? t.y : dy, w, c.x ? t.x : dx, t.inner, t.inner_bytes, st);
     if (rc || !c.x) return rc;
     return copy_out(g, t.x, dx, g.h * g.w, g.ci, st);
 }
@@ -2814,7 +2894,14 @@ static int tc_wgrad_any(const Geo& g, const void* x, const void* dy, void* dw, v
     if (!copy_ws(c, ws, ws_bytes, t)) return B2C_ERR_WORKSPACE_TOO_SMALL;
     if (c.x) { const int rc = copy_in(g, x, t.x, g.h * g.w, g.ci, st); if (rc) return rc; }
     if (c.y) { const int rc = copy_in(g, dy, t.y, g.ho * g.wo, g.co, st); if (rc) return rc; }
-    return tc_wgrad_nhwc(copied_geo(g, c), c.x ? t.x : x, c.y ? t.y : dy, dw, db, t.inner, t.inner_bytes, st, lowered_in_ws);
+    const Geo q = copied_geo(g, c, B2C_PASS_WGRAD);
+    // the kernel's own sums of dy are float32 chains; fine passes take the bias gradient from the sums in double, whose
+    // scratch is that of the partial tiles (the lowered matrix in front of them stays)
+    const uintptr_t scratch = align_up((uintptr_t)t.inner, 1024) + kept_lowered_bytes(g), end = (uintptr_t)t.inner + t.inner_bytes;
+    if (q.fine && db && (!t.inner || scratch + channel_sum_workspace_bytes(g.n, g.co, g.ho * g.wo) > end)) return B2C_ERR_WORKSPACE_TOO_SMALL;
+    const int rc = tc_wgrad_nhwc(q, c.x ? t.x : x, c.y ? t.y : dy, dw, q.fine ? nullptr : db, t.inner, t.inner_bytes, st, lowered_in_ws);
+    if (rc || !q.fine || !db) return rc;
+    return channel_sum(B2C_F32, g.layout, g.n, g.co, g.ho * g.wo, dy, db, (void*)scratch, end - scratch, st);
 }
 
 int tc_wgrad_lowered(const Geo& g, const void* x, const void* dy, void* dw, void* db, void* ws, size_t ws_bytes, cudaStream_t st)

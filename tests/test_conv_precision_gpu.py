@@ -39,3 +39,35 @@ def test_filters_with_inner_taps_are_split_by_rounding(shape, layout):
         assert got.size
         # the other operand's lower half loses its last two bits (3 * 2^-23 at most), each of the two sums at most one more
         assert np.abs(got / want - 1).max() <= 5 * 2.0 ** -23, (name, np.abs(got / want - 1).max())
+
+
+def _errors(out, refs):
+    return {k: float(np.linalg.norm(out[k].astype(np.float64).reshape(r.shape) - r) / np.linalg.norm(r)) for k, r in refs.items()}
+
+
+# (layout, n, h, w, ci, co, k, pad, stride): channel counts that are no whole blocks (lowered, one to several blocks, strided: all
+# classes in one launch, one class, a launch per class), whole blocks on NCHW images too small for the copies, one-pixel images
+@pytest.mark.parametrize("shape", [("NHWC", 9, 30, 17, 40, 72, 3, 1, 1), ("NCHW", 3, 16, 16, 3, 20, 3, 1, 1), ("NHWC", 2, 14, 14, 132, 70, 5, 2, 2),
+                                   ("NCHW", 5, 9, 9, 36, 100, 3, 1, 2), ("NHWC", 4, 9, 9, 40, 48, 1, 0, 2), ("NHWC", 4, 11, 11, 50, 24, 2, 0, 3),
+                                   ("NCHW", 1, 14, 14, 256, 256, 1, 0, 2), ("NHWC", 96, 1, 1, 520, 384, 1, 0, 1), ("NHWC", 8, 8, 8, 423, 512, 3, 1, 1),
+                                   ("NCHW", 12, 10, 10, 256, 9, 3, 1, 1), ("NCHW", 6, 28, 28, 1, 16, 3, 1, 1)])
+def test_passes_that_sum_like_the_fma_engine(shape):
+    """Where the tensor-core engine takes over from the FMA engine it is no further from float64.  On top of the FMA engine's own
+    error on the same inputs: one rounding (2^-24) for its shorter chains on the smallest sums."""
+    layout, n, h, w, ci, cout, k, pad, st = shape
+    g = co.Geom(n, h, w, ci, cout, k, k, pad, pad, st, st)
+    rng = np.random.Generator(np.random.PCG64(ci + cout))
+    nchw = layout == "NCHW"
+    x = rng.standard_normal((n, ci, h, w) if nchw else (n, h, w, ci)).astype(np.float32)
+    wt = rng.standard_normal((cout, ci, k, k) if nchw else (ci, k, k, cout)).astype(np.float32)
+    b = rng.standard_normal(cout).astype(np.float32)
+    dy = rng.standard_normal((n, cout, g.ho, g.wo) if nchw else (n, g.ho, g.wo, cout)).astype(np.float32)
+    x64, w64, b64, dy64 = (a.astype(np.float64) for a in (x, wt, b, dy))
+    refs = dict(zip(("y", "dw", "db", "dx"), (co.conv2d_forward(x64, w64, b64, g, layout), *co.conv2d_backward(x64, dy64, w64, g, layout))))
+    w_layout = "KCRS" if nchw else "KRSC"
+    desc = make_desc(g, layout, np.float32, w_layout)
+    assert any(_lib.lib().b2c_conv_engine_for(ctypes.byref(desc), p) == _lib.ENGINE_TENSOR for p in range(3))
+    got = _errors(run_conv(g, layout, np.float32, x, wt, b, dy, w_layout=w_layout), refs)
+    fma = _errors(run_conv(g, layout, np.float32, x, wt, b, dy, w_layout=w_layout, engine=_lib.ENGINE_FMA), refs)
+    for name in refs:
+        assert got[name] <= fma[name] + 2.0 ** -24, (name, got, fma)
