@@ -2320,7 +2320,8 @@ static int tc_fprop_nhwc(const Geo& g, const void* x, const void* w, const void*
         FwdLaunch f{g.n, g.ho, g.wo, Kp, Kp, g.ho, g.wo, g.co, 1, 1, 0, 0, g.ho, g.wo, 1, 1, 1, 1, g.ho * g.wo * yp, g.wo * yp, yp, g.fine};
         return run_fwd(f, rows, nullptr, none, bias, bn, relu, (float*)y, (void*)w_hi, 2 * fbytes + 1024, st, true, stats);
     }
-    PrepParams pp{g.co, g.ci, g.kh, g.kw, wsd.sk, wsd.sc, wsd.sr, wsd.ss, 0, 1, 0, 1, g.kh, g.kw};
+    // few channels read in place: the filter of the lowered form is rounded as well
+    PrepParams pp{g.co, g.ci, g.kh, g.kw, wsd.sk, wsd.sc, wsd.sr, wsd.ss, 0, 1, 0, 1, g.kh, g.kw, 0, g.ci % 32 != 0};
     FwdLaunch f{g.n, g.h, g.w, g.ci, g.xp, g.ho, g.wo, g.co, g.kh, g.kw, -g.vpad, -g.hpad,
                 g.h + 2 * g.vpad - (g.kh - 1) * g.vdil, g.w + 2 * g.hpad - (g.kw - 1) * g.hdil,
                 g.vstr, g.hstr, g.vdil, g.hdil, g.ho * g.wo * yp, g.wo * yp, yp, g.fine};
