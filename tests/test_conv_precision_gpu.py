@@ -75,3 +75,18 @@ def test_passes_that_sum_like_the_fma_engine(shape):
     fma = _errors(run_conv(g, layout, np.float32, x, wt, b, dy, w_layout=w_layout, engine=_lib.ENGINE_FMA), refs)
     for name in refs:
         assert got[name] <= fma[name] + 2.0 ** -24, (name, got, fma)
+
+
+def test_short_ranges_are_not_made_longer():
+    """A launch that balanced ranges cut into 5.4 k-blocks per CTA keeps that advantage (6 of 8 products per sum in tensor memory, and
+    an error in proportion) over one large enough for whole tiles, whose sums are all of 8 k-blocks."""
+    rng = np.random.Generator(np.random.PCG64(7))
+    wt = (rng.standard_normal((256, 5, 5, 128)) / 80).astype(np.float32)
+    err = []
+    for n in (2, 40):
+        g = co.Geom(n, 15, 15, 256, 128, 5, 5, 2, 2, 1, 1)
+        x = rng.standard_normal((n, 15, 15, 256)).astype(np.float32)
+        y = run_conv(g, "NHWC", np.float32, x, wt, None, None, w_layout="KRSC", passes=("fprop",))["y"][:2]
+        ref = co.conv2d_forward(x[:2].astype(np.float64), wt.astype(np.float64), np.zeros(128), co.Geom(2, 15, 15, 256, 128, 5, 5, 2, 2, 1, 1), "NHWC")
+        err.append(np.linalg.norm(y - ref) / np.linalg.norm(ref))
+    assert err[0] <= 0.9 * err[1], err
