@@ -616,6 +616,8 @@ fc_wgrad_kernel(const float* __restrict__ x, const float* __restrict__ dy, float
 // The last layer of a small classifier (128 x 10 and the like): a GEMM kernel's start-up, its second stage and the separate
 // bias sum are all there is to such a layer, so each direction is one launch of plain dot products whose operands stay in L1.
 // Weights up to 16 K elements; with more, re-reading them per batch row costs more than the launches saved.
+// Sums are in double and rounded once: a float32 sum in eight parts is up to 1.3 times further from float64 than one chain of
+// FMAs (5 rows), and the bias gradient of every other route is a sum in double.
 bool fc_tiny(int batch, int in_f, int out_f) { return batch <= 512 && (int64_t)in_f * out_f <= (1 << 14); }
 
 // y[b][o]: block = 32 outputs x 8 parts of the sum over the inputs, one batch row.
@@ -624,20 +626,20 @@ __global__ void __launch_bounds__(256) fc_tiny_forward_kernel(const T* __restric
                                                               T* __restrict__ y, int in_f, int out_f)
 {
     pdl_prologue();
-    __shared__ T part[8][33];
+    __shared__ double part[8][33];
     const int o = blockIdx.x * 32 + threadIdx.x;
     const T* xr = x + (int64_t)blockIdx.y * in_f;
-    T v = T(0);
+    double v = 0.0;
     if (o < out_f) {
 #pragma unroll 8
-        for (int i = threadIdx.y; i < in_f; i += 8) v = fma(__ldg(xr + i), __ldg(w + (int64_t)i * out_f + o), v);
+        for (int i = threadIdx.y; i < in_f; i += 8) v = fma((double)__ldg(xr + i), (double)__ldg(w + (int64_t)i * out_f + o), v);
     }
     part[threadIdx.y][threadIdx.x] = v;
     __syncthreads();
     if (threadIdx.y != 0 || o >= out_f) return;
 #pragma unroll
     for (int k = 1; k < 8; k++) v += part[k][threadIdx.x];
-    y[(int64_t)blockIdx.y * out_f + o] = bias ? v + bias[o] : v;
+    y[(int64_t)blockIdx.y * out_f + o] = (T)(bias ? v + (double)bias[o] : v);
 }
 
 // The first dw_blocks blocks: dw[i][o] and db[o] (the row i = in_f), 32 outputs x 8 parts of the sum over the batch; the
@@ -648,18 +650,18 @@ __global__ void __launch_bounds__(256) fc_tiny_backward_kernel(const T* __restri
                                                                int dw_blocks)
 {
     pdl_prologue();
-    __shared__ T part[8][33];
+    __shared__ double part[8][33];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     if ((int)blockIdx.x < dw_blocks) {
         const int nt = (out_f + 31) / 32, i = blockIdx.x / nt, o = (blockIdx.x - i * nt) * 32 + tx;
-        T v = T(0);
+        double v = 0.0;
         if (o < out_f) {
             if (i < in_f) {
 #pragma unroll 8
-                for (int b = ty; b < batch; b += 8) v = fma(__ldg(x + (int64_t)b * in_f + i), __ldg(dy + (int64_t)b * out_f + o), v);
+                for (int b = ty; b < batch; b += 8) v = fma((double)__ldg(x + (int64_t)b * in_f + i), (double)__ldg(dy + (int64_t)b * out_f + o), v);
             } else {
 #pragma unroll 8
-                for (int b = ty; b < batch; b += 8) v += __ldg(dy + (int64_t)b * out_f + o);
+                for (int b = ty; b < batch; b += 8) v += (double)__ldg(dy + (int64_t)b * out_f + o);
             }
         }
         part[ty][tx] = v;
@@ -667,18 +669,18 @@ __global__ void __launch_bounds__(256) fc_tiny_backward_kernel(const T* __restri
         if (ty != 0 || o >= out_f) return;
 #pragma unroll
         for (int k = 1; k < 8; k++) v += part[k][tx];
-        if (i < in_f) { if (dw) dw[(int64_t)i * out_f + o] = v; }
-        else if (db) db[o] = v;
+        if (i < in_f) { if (dw) dw[(int64_t)i * out_f + o] = (T)v; }
+        else if (db) db[o] = (T)v;
         return;
     }
     const int64_t e = (int64_t)(blockIdx.x - dw_blocks) * 256 + threadIdx.x;
     if (e >= (int64_t)batch * in_f) return;
     const int b = (int)(e / in_f), i = (int)(e - (int64_t)b * in_f);
     const T *d = dy + (int64_t)b * out_f, *wr = w + (int64_t)i * out_f;
-    T v = T(0);
+    double v = 0.0;
 #pragma unroll 8
-    for (int o = 0; o < out_f; o++) v = fma(__ldg(d + o), __ldg(wr + o), v);
-    dx[e] = v;
+    for (int o = 0; o < out_f; o++) v = fma((double)__ldg(d + o), (double)__ldg(wr + o), v);
+    dx[e] = (T)v;
 }
 
 template <typename T>

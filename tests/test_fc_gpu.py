@@ -37,3 +37,20 @@ def test_fc_routes(n, i, o, dtype):
                 assert_parity(u.cpu().numpy(), ref, dtype, str(which))
             else:
                 assert bool(torch.isnan(u).all())
+
+
+@pytest.mark.parametrize("n,i,o", [(5, 151, 11), (42, 163, 59), (64, 128, 10), (512, 4, 4096), (3, 16384, 1)])
+def test_small_layers_round_once(n, i, o):
+    L = _lib.lib()
+    rng = np.random.Generator(np.random.PCG64(n))
+    x, w, b, dy = (rng.standard_normal(s).astype(np.float32) for s in ((n, i), (i, o), (o,), (n, o)))
+    xd, wd, bd, dyd = (dev(a) for a in (x, w, b, dy))
+    y, dw, db, dx = (torch.empty(s, device=DEV) for s in ((n, o), (i, o), (o,), (n, i)))
+    ws = torch.empty(max(256, L.b2c_fc_workspace_bytes(0, n, i, o, 0)), dtype=torch.uint8, device=DEV)
+    _lib.check(L.b2c_fc_forward(0, 0, n, i, o, xd.data_ptr(), wd.data_ptr(), bd.data_ptr(), y.data_ptr(), ws.data_ptr(), ws.numel(), stream()))
+    _lib.check(L.b2c_fc_backward(0, 0, n, i, o, xd.data_ptr(), dyd.data_ptr(), wd.data_ptr(), dw.data_ptr(), db.data_ptr(), dx.data_ptr(),
+                                 ws.data_ptr(), ws.numel(), stream()))
+    X, W, B, D = (a.astype(np.float64) for a in (x, w, b, dy))
+    # one rounding to float32, and what the sums in double leave of 16384 terms at most (2^-53 each of their magnitudes)
+    for got, ref, mag in ((y, X @ W + B, abs(X) @ abs(W) + abs(B)), (dw, X.T @ D, abs(X.T) @ abs(D)), (db, D.sum(0), abs(D).sum(0)), (dx, D @ W.T, abs(D) @ abs(W.T))):
+        assert (abs(got.cpu().numpy() - ref) <= 2.0 ** -24 * abs(ref) + 2.0 ** -38 * mag).all()
