@@ -108,7 +108,6 @@ int fma_index_map(const Geo& g, int64_t* map, cudaStream_t st);
 int channel_sum(int dtype, int layout, int n, int c, int hw, const void* src, void* dst, void* ws, size_t ws_bytes,
                 cudaStream_t st);
 size_t channel_sum_workspace_bytes(int n, int c, int hw);
-int channel_sum_pitched(int64_t rows, int c, int pitch, const float* src, float* dst, void* ws, size_t ws_bytes, cudaStream_t st);
 bool fc_tiny(int batch, int in_f, int out_f);
 int fc_tiny_forward(int dtype, int batch, int in_f, int out_f, const void* x, const void* w, const void* bias, void* y, cudaStream_t st);
 int fc_tiny_backward(int dtype, int batch, int in_f, int out_f, const void* x, const void* dy, const void* w, void* dw, void* db, void* dx, cudaStream_t st);

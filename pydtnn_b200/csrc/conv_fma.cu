@@ -1054,10 +1054,10 @@ __global__ void __launch_bounds__(256) channel_sum_final_kernel(const double* __
 }
 
 // Few rows (a fully connected layer's batch): one launch, block (32 channels, 32 row lanes), a thread adds its rows 32 apart in
-// order, the lanes are added in order.  Rows `pitch` elements apart.
+// order, the lanes are added in order.
 constexpr int CS_FEW_ROWS = 1024;
 template <typename T>
-__global__ void __launch_bounds__(1024) channel_sum_few_kernel(const T* __restrict__ src, T* __restrict__ dst, int rows, int c, int pitch)
+__global__ void __launch_bounds__(1024) channel_sum_few_kernel(const T* __restrict__ src, T* __restrict__ dst, int rows, int c)
 {
     pdl_prologue();
     __shared__ double sm[32][33];
@@ -1065,7 +1065,7 @@ __global__ void __launch_bounds__(1024) channel_sum_few_kernel(const T* __restri
     double acc = 0.0;
     if (ch < c) {
 #pragma unroll 4
-        for (int r = threadIdx.y; r < rows; r += 32) acc += (double)src[(int64_t)r * pitch + ch];
+        for (int r = threadIdx.y; r < rows; r += 32) acc += (double)src[(int64_t)r * c + ch];
     }
     sm[threadIdx.y][threadIdx.x] = acc;
     __syncthreads();
@@ -1075,17 +1075,6 @@ __global__ void __launch_bounds__(1024) channel_sum_few_kernel(const T* __restri
         for (int i = 0; i < 32; i++) s += sm[i][threadIdx.x];
         dst[ch] = (T)s;
     }
-}
-
-// NHWC float32 rows on any pitch (the few-rows kernel up to its limit, else dense rows only through channel_sum).
-int channel_sum_pitched(int64_t rows, int c, int pitch, const float* src, float* dst, void* ws, size_t ws_bytes, cudaStream_t st)
-{
-    if (rows <= CS_FEW_ROWS) {
-        launch_pdl(channel_sum_few_kernel<float>, (c + 31) / 32, dim3(32, 32), 0, st, src, dst, (int)rows, c, pitch);
-        return check_launch("channel_sum_few_kernel");
-    }
-    if (pitch != c) return B2C_ERR_UNSUPPORTED;
-    return channel_sum(B2C_F32, B2C_LAYOUT_NHWC, (int)rows, c, 1, src, dst, ws, ws_bytes, st);
 }
 
 // Enough for the float4 fast path to spread over about four CTAs per SM: two doubles per channel and chunk.
@@ -1104,8 +1093,8 @@ int channel_sum(int dtype, int layout, int n, int c, int hw, const void* src, vo
     if (!src || !dst || !ws) return B2C_ERR_NULL_POINTER;
     if (ws_bytes < (size_t)CS_CHUNKS * c * sizeof(double)) return B2C_ERR_WORKSPACE_TOO_SMALL;
     if ((layout == B2C_LAYOUT_NHWC || hw == 1) && (int64_t)n * hw <= CS_FEW_ROWS) {
-        if (dtype == B2C_F32) launch_pdl(channel_sum_few_kernel<float>, (c + 31) / 32, dim3(32, 32), 0, st, (const float*)src, (float*)dst, n * hw, c, c);
-        else launch_pdl(channel_sum_few_kernel<double>, (c + 31) / 32, dim3(32, 32), 0, st, (const double*)src, (double*)dst, n * hw, c, c);
+        if (dtype == B2C_F32) launch_pdl(channel_sum_few_kernel<float>, (c + 31) / 32, dim3(32, 32), 0, st, (const float*)src, (float*)dst, n * hw, c);
+        else launch_pdl(channel_sum_few_kernel<double>, (c + 31) / 32, dim3(32, 32), 0, st, (const double*)src, (double*)dst, n * hw, c);
         return check_launch("channel_sum_few_kernel");
     }
     if (dtype == B2C_F32 && layout == B2C_LAYOUT_NHWC) {

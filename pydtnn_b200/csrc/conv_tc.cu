@@ -1947,8 +1947,11 @@ static size_t tc_workspace_bytes_nhwc(const Geo& g, int pass)
     if (pass == B2C_PASS_FPROP || pass == B2C_PASS_DGRAD)
         return (pass == B2C_PASS_DGRAD && (g.vstr > 1 || g.hstr > 1) ? 3 : 2) * filter_split_bytes(g, pass) + 2048 + sk_bytes();
     WgradPlan pl = wgrad_plan(g);
-    return lowered + align_up((size_t)pl.splits * wgrad_rows(g) * round4(g.co) * sizeof(float), 1024) + 2048 +
-           align_up((size_t)pl.splits * 4 * round4(g.co) * sizeof(float), 1024);
+    const size_t partials = align_up((size_t)pl.splits * wgrad_rows(g) * round4(g.co) * sizeof(float), 1024) + 2048 +
+                            align_up((size_t)pl.splits * 4 * round4(g.co) * sizeof(float), 1024);
+    // tiles that go straight to dw leave the partials' place to the bias gradient (see tc_wgrad_nhwc)
+    const size_t sums = pl.splits == 1 && g.kh * g.kw == 1 ? channel_sum_workspace_bytes((int)g.M, g.co, 1) + 2048 : 0;
+    return lowered + (sums > partials ? sums : partials);
 }
 
 template <int MODE, int BN, int STAGES, bool SK, int SLABS, int BSRC, int STREAM = 0, bool MULTI = false, int RESKB = 0, bool FINE = false>
@@ -2543,13 +2546,15 @@ static int tc_wgrad_nhwc(const Geo& g, const void* x, const void* dy, void* dw, 
         const int64_t t = wsd.sk; wsd.sk = wsd.sc; wsd.sc = t;
     }
     // One pixel range and a filter layout that is the GEMM's own (rows = input channels, output channels contiguous): the
-    // tiles go straight to dw and only the bias gradient is left for a kernel of its own.
+    // tiles go straight to dw and only the bias gradient is left for a kernel of its own, where the workspace holds its scratch.
+    const size_t rest = (uintptr_t)ws + ws_bytes - (uintptr_t)partial;
     if (pl.splits == 1 && !low && !exchanged && g.kh * g.kw == 1 && wsd.sk == 1 && wsd.sc % 4 == 0 && ((uintptr_t)dw & 15) == 0 && p.tma_store &&
+        (!db || (g.yp == g.co && rest >= channel_sum_workspace_bytes((int)g.M, g.co, 1))) &&
         make_map_out(&mo, dw, 1, (uint64_t)g.ci, (uint64_t)g.co, (uint64_t)wsd.sc)) {
         p.db_partial = nullptr;
         const int rc = dispatch_wgrad(pl.bn, g.fine, ma, mb, mo, p, 1, st);
         if (rc || !db) return rc;
-        return channel_sum_pitched(g.M, g.co, g.yp, (const float*)dy, (float*)db, partial, pbytes + cs, st);
+        return channel_sum(B2C_F32, B2C_LAYOUT_NHWC, (int)g.M, g.co, 1, dy, db, partial, rest, st);
     }
     int rc = dispatch_wgrad(pl.bn, g.fine, ma, mb, mo, p, pl.splits, st);
     if (rc) return rc;

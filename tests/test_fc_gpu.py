@@ -54,3 +54,17 @@ def test_small_layers_round_once(n, i, o):
     # one rounding to float32, and what the sums in double leave of 16384 terms at most (2^-53 each of their magnitudes)
     for got, ref, mag in ((y, X @ W + B, abs(X) @ abs(W) + abs(B)), (dw, X.T @ D, abs(X.T) @ abs(D)), (db, D.sum(0), abs(D).sum(0)), (dx, D @ W.T, abs(D) @ abs(W.T))):
         assert (abs(got.cpu().numpy() - ref) <= 2.0 ** -24 * abs(ref) + 2.0 ** -38 * mag).all()
+
+
+@pytest.mark.parametrize("n,i,o", [(2048, 64, 16384), (1056, 64, 32000), (1025, 32, 16384)])
+def test_bias_gradient_of_wide_layers_with_many_rows(n, i, o):
+    L = _lib.lib()
+    g = torch.Generator(device=DEV).manual_seed(n)
+    x, dy, w = (torch.randn(s, device=DEV, generator=g) for s in ((n, i), (n, o), (i, o)))
+    dw, db, dx = (torch.full(s, float("nan"), device=DEV) for s in ((i, o), (o,), (n, i)))
+    ws = torch.empty(L.b2c_fc_workspace_bytes(0, n, i, o, 0), dtype=torch.uint8, device=DEV)
+    _lib.check(L.b2c_fc_backward(0, 0, n, i, o, x.data_ptr(), dy.data_ptr(), w.data_ptr(), dw.data_ptr(), db.data_ptr(), dx.data_ptr(),
+                                 ws.data_ptr(), ws.numel(), stream()))
+    X, D, W = (a.cpu().numpy().astype(np.float64) for a in (x, dy, w))
+    for got, ref, what in ((dw, X.T @ D, "dw"), (db, D.sum(0), "db"), (dx, D @ W.T, "dx")):
+        assert_parity(got.cpu().numpy(), ref, np.float32, what)
