@@ -38,10 +38,10 @@ static int pick_engine(const Geo& g, int pass, int& engine) {
 }
 
 // The engine of a call: the shape's, except that channel counts which are no whole blocks on 16-byte pixels also run
-// with pointers on any alignment, which only the FMA engine takes.
-static int call_engine(const Geo& g, int pass, const void* a, const void* b, int& engine) {
+// with pointers (x or dx, y or dy) on any alignment, which only the FMA engine takes.
+static int call_engine(const Geo& g, int pass, const void* x, const void* y, int& engine) {
     int rc = pick_engine(g, pass, engine);
-    if (!rc && engine == B2C_ENGINE_TENSOR && g.engine == B2C_ENGINE_AUTO && (((uintptr_t)a | (uintptr_t)b) & 15) && !tc_any_alignment(g, pass))
+    if (!rc && engine == B2C_ENGINE_TENSOR && g.engine == B2C_ENGINE_AUTO && !tc_takes_alignment(g, pass, x, y) && !tc_refuses_unaligned(g, pass))
         engine = B2C_ENGINE_FMA;
     return rc;
 }
@@ -49,7 +49,7 @@ static size_t pass_workspace_bytes(const Geo& g, int pass) {
     int e; if (pick_engine(g, pass, e)) return 0;
     if (e == B2C_ENGINE_FMA) return fma_workspace_bytes(g, pass);
     const size_t t = tc_workspace_bytes(g, pass);
-    if (g.engine != B2C_ENGINE_AUTO || tc_any_alignment(g, pass)) return t;
+    if (g.engine != B2C_ENGINE_AUTO || tc_refuses_unaligned(g, pass)) return t;
     const size_t f = fma_workspace_bytes(g, pass);
     return t > f ? t : f;
 }
@@ -119,7 +119,10 @@ extern "C" int b2c_conv_fprop(const b2c_conv_desc* desc, const void* x, const vo
     if (bn && (!bn->mean || !bn->inv_std || !bn->gamma || !bn->beta)) return B2C_ERR_NULL_POINTER;
     int e; rc = call_engine(g, B2C_PASS_FPROP, x, y, e); if (rc) return rc;
     if (e == B2C_ENGINE_TENSOR) return tc_fprop(g, x, w, bias, bn, relu, y, ws, ws_bytes, (cudaStream_t)stream);
-    return fma_fprop(g, x, w, bias, bn, relu, y, ws, ws_bytes, (cudaStream_t)stream);
+    rc = fma_fprop(g, x, w, bias, bn, relu, y, ws, ws_bytes, (cudaStream_t)stream);
+    // a layer that keeps its lowered input has it in the workspace after every forward pass
+    if (rc || !b2c_conv_keeps_lowered_input(desc)) return rc;
+    return tc_leave_lowered(g, x, ws, ws_bytes, (cudaStream_t)stream);
 }
 
 extern "C" size_t b2c_conv_stats_bytes(const b2c_conv_desc* desc) {
@@ -143,7 +146,7 @@ extern "C" int b2c_conv_dgrad(const b2c_conv_desc* desc, const void* dy, const v
                               void* ws, size_t ws_bytes, void* stream) {
     Geo g; int rc = make_geo(desc, g); if (rc) return rc;
     if (!dy || !w || !dx) return B2C_ERR_NULL_POINTER;
-    int e; rc = call_engine(g, B2C_PASS_DGRAD, dy, dx, e); if (rc) return rc;
+    int e; rc = call_engine(g, B2C_PASS_DGRAD, dx, dy, e); if (rc) return rc;
     if (e == B2C_ENGINE_TENSOR) return tc_dgrad(g, dy, w, dx, ws, ws_bytes, (cudaStream_t)stream);
     return fma_dgrad(g, dy, w, dx, ws, ws_bytes, (cudaStream_t)stream);
 }
@@ -159,6 +162,7 @@ extern "C" int b2c_conv_wgrad_lowered(const b2c_conv_desc* desc, const void* x, 
                                       void* ws, size_t ws_bytes, void* stream) {
     Geo g; int rc = make_geo(desc, g); if (rc) return rc;
     if (!x || !dy || !dw) return B2C_ERR_NULL_POINTER;
+    if (!b2c_conv_keeps_lowered_input(desc)) return B2C_ERR_UNSUPPORTED;
     int e; rc = call_engine(g, B2C_PASS_WGRAD, x, dy, e); if (rc) return rc;
     if (e != B2C_ENGINE_TENSOR) return B2C_ERR_UNSUPPORTED;
     return tc_wgrad_lowered(g, x, dy, dw, db, ws, ws_bytes, (cudaStream_t)stream);
@@ -247,7 +251,7 @@ extern "C" int b2c_fc_backward(int dtype, int engine, int batch, int in_f, int o
     }
     if (dx) {
         if (!w) return B2C_ERR_NULL_POINTER;
-        int e; rc = call_engine(g, B2C_PASS_DGRAD, dy, dx, e); if (rc) return rc;
+        int e; rc = call_engine(g, B2C_PASS_DGRAD, dx, dy, e); if (rc) return rc;
         rc = e == B2C_ENGINE_TENSOR ? tc_dgrad(g, dy, w, dx, ws, ws_bytes, st) : fma_dgrad(g, dy, w, dx, ws, ws_bytes, st);
     }
     return rc;

@@ -115,7 +115,8 @@ int channel_sum_v4(int n, int c, int hw, const void* src, void* dst, void* ws, s
 
 // tensor-core engine (conv_tc.cu)
 bool tc_supported(const Geo& g, int pass);
-bool tc_any_alignment(const Geo& g, int pass);
+bool tc_takes_alignment(const Geo& g, int pass, const void* x, const void* y);
+bool tc_refuses_unaligned(const Geo& g, int pass);
 bool tc_fine_sums(const Geo& g, int pass);
 int tc_wait_selftest(long long limit_cycles, cudaStream_t st);
 size_t tc_workspace_bytes(const Geo& g, int pass);
@@ -126,6 +127,7 @@ int tc_wgrad(const Geo& g, const void* x, const void* dy, void* dw, void* db, vo
              cudaStream_t st);
 int tc_read_status(int* out);
 bool tc_keeps_lowered(const Geo& g);
+int tc_leave_lowered(const Geo& g, const void* x, void* ws, size_t ws_bytes, cudaStream_t st);
 int tc_wgrad_lowered(const Geo& g, const void* x, const void* dy, void* dw, void* db, void* ws, size_t ws_bytes, cudaStream_t st);
 int transpose_images(int dtype, const void* src, void* dst, int n, int rows, int cols, cudaStream_t st);
 bool tc_fc_small_batch(int dtype, int engine, int batch, int in_f, int out_f);

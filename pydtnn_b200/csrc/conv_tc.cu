@@ -2809,9 +2809,18 @@ bool tc_supported(const Geo& g, int pass)
     return flops / 130e12 + moved / 2.5e12 < tiles / 4e12;
 }
 
-// Shapes whose channel counts keep every activation on 16-byte pixels and whole blocks, whatever the pointers: for the
-// others a pointer that is not 16-byte aligned sends the call to the FMA engine (b2c_conv_* with engine AUTO).
-bool tc_any_alignment(const Geo& g, int pass)
+// Whether the engine reads (writes) these activations where they are: those it copies, and an x that is lowered, may lie on any
+// alignment, the others start on 16 bytes.
+bool tc_takes_alignment(const Geo& g, int pass, const void* x, const void* y)
+{
+    const Copies c = tc_copies(g, pass);
+    const bool x_free = c.x || (pass != B2C_PASS_DGRAD && lowered_ok(g));
+    return (x_free || ((uintptr_t)x & 15) == 0) && (c.y || ((uintptr_t)y & 15) == 0);
+}
+
+// Shapes of whole blocks on 16-byte pixels, which this engine alone has always run and refuses on other pointers: for the
+// others such a call goes to the FMA engine (b2c_conv_* with engine AUTO).
+bool tc_refuses_unaligned(const Geo& g, int pass)
 {
     const Copies c = tc_copies(g, pass);
     if (pass == B2C_PASS_FPROP) return g.ci % 32 == 0 && g.co % 4 == 0;
@@ -2899,6 +2908,17 @@ int tc_dgrad(const Geo& g, const void* dy, const void* w, void* dx, void* ws, si
 // pass and again in their weight gradient.  A caller that gives the layer a workspace of its own can say that the forward
 // pass's matrix is still there.
 bool tc_keeps_lowered(const Geo& g) { return g.layout == B2C_LAYOUT_NHWC && lowered_ok(g) && tc_supported_nhwc(g, B2C_PASS_WGRAD) && tc_supported_nhwc(g, B2C_PASS_FPROP); }
+
+// Leaves the matrix where a forward pass on this engine does, for a forward call that the FMA engine ran (an unaligned y).
+int tc_leave_lowered(const Geo& g, const void* x, void* ws, size_t ws_bytes, cudaStream_t st)
+{
+    const Copies c = tc_copies(g, B2C_PASS_FPROP);
+    CopyWs t;
+    if (!copy_ws(c, ws, ws_bytes, t)) return B2C_ERR_WORKSPACE_TOO_SMALL;
+    const uintptr_t rows = align_up((uintptr_t)t.inner, 1024);
+    if (!t.inner || rows + kept_lowered_bytes(g) > (uintptr_t)t.inner + t.inner_bytes) return B2C_ERR_WORKSPACE_TOO_SMALL;
+    return launch_lower(copied_geo(g, c, B2C_PASS_FPROP), x, (float*)rows, st);
+}
 
 static int tc_wgrad_any(const Geo& g, const void* x, const void* dy, void* dw, void* db, void* ws, size_t ws_bytes, cudaStream_t st, bool lowered_in_ws)
 {
