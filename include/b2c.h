@@ -144,7 +144,7 @@ int b2c_conv_wgrad_lowered(const b2c_conv_desc *desc, const void *x, const void 
 int b2c_conv_index_map(const b2c_conv_desc *desc, int64_t *map, void *stream);
 
 /* dst[n][cols][rows] = src[n][rows][cols] (dtype elements, both 16-byte aligned or not): an activation between the
- * NCHW and NHWC orders is n images of (c, h*w) or (h*w, c).  n <= 65535.  Replaces the transposes around the
+ * NCHW and NHWC orders is n images of (c, h*w) or (h*w, c).  Replaces the transposes around the
  * reference's NCHW lowering, pydtnn/backends/cpu/layers/conv_2d_cpu.py:264-291. */
 int b2c_transpose(int dtype, int n, int rows, int cols, const void *src, void *dst, void *stream);
 

@@ -2669,7 +2669,6 @@ __global__ void __launch_bounds__(256) transpose_wide_kernel(const T* __restrict
 template <typename T>
 static int transpose_t(const void* src, void* dst, int n, int rows, int cols, int sp, int dp, cudaStream_t st)
 {
-    if ((rows + 31) / 32 > 65535) return B2C_ERR_TOO_LARGE;
     if (n > 65535) {                                  // the image index is a grid axis: in parts
         const int rc = transpose_t<T>(src, dst, 65535, rows, cols, sp, dp, st);
         return rc ? rc : transpose_t<T>((const T*)src + (size_t)65535 * rows * sp, (T*)dst + (size_t)65535 * cols * dp, n - 65535, rows, cols, sp, dp, st);
@@ -2681,6 +2680,16 @@ static int transpose_t(const void* src, void* dst, int n, int rows, int cols, in
     if (cols <= 8 && rows > 8 && dp == rows) {
         launch_pdl(transpose_thin_kernel<T, false>, dim3((rows + 255) / 256, n), 256, 0, st, (const T*)src, (T*)dst, cols, rows, sp);
         return check_launch("transpose_thin_kernel");
+    }
+    constexpr int MOST_ROWS = 65535 * 32;             // blocks of 32 rows are a grid axis as well: larger images one by one, in parts
+    if (rows > MOST_ROWS) {
+        for (int i = 0; i < n; i++)
+            for (int64_t r = 0; r < rows; r += MOST_ROWS) {
+                const int part = rows - r < MOST_ROWS ? (int)(rows - r) : MOST_ROWS;
+                const int rc = transpose_t<T>((const T*)src + ((int64_t)i * rows + r) * sp, (T*)dst + (int64_t)i * cols * dp + r, 1, part, cols, sp, dp, st);
+                if (rc) return rc;
+            }
+        return B2C_OK;
     }
     const int64_t wide = (int64_t)((cols + 63) / 64) * ((rows + 63) / 64) * n;
     if (rows > 32 && cols > 32 && wide >= tc_sm_count()) {

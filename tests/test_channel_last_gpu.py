@@ -63,3 +63,24 @@ def test_values_written_through_a_look_are_read():
     v = np.random.default_rng(0).standard_normal((2, 4, 5, 7)).astype(np.float32)
     y.ary.set(v)
     assert np.array_equal(m.layers[2].forward(y).ary.get(), np.maximum(v, 0))
+
+
+@pytest.mark.parametrize("n,rows,cols", [(1, 65535 * 32 + 5, 9), (2, 65535 * 32 + 33, 33), (1, 65535 * 32 + 1, 3)])
+def test_transpose_of_many_rows(n, rows, cols):
+    x = torch.randn(n, rows, cols, device=DEV)
+    y = torch.full((n, cols, rows), float("nan"), device=DEV)
+    _lib.check(_lib.lib().b2c_transpose(_lib.F32, n, rows, cols, x.data_ptr(), y.data_ptr(), stream()))
+    assert torch.equal(y, x.transpose(1, 2))
+
+
+def test_large_nchw_images():
+    """Images of more pixels than 32 times a grid axis: the copies of y and dx are cut, or not on that axis at all."""
+    from oracle import conv_oracle as co
+    from tests.gpu_util import rel_l2, run_conv
+    g = co.Geom(1, 1449, 1449, 3, 8, 3, 3, 1, 1, 1, 1)
+    rng = np.random.Generator(np.random.PCG64(4))
+    x, w, dy = (rng.standard_normal(s).astype(np.float32) for s in ((1, 3, 1449, 1449), (8, 3, 3, 3), (1, 8, 1449, 1449)))
+    got = run_conv(g, "NCHW", np.float32, x, w, None, dy)
+    fma = run_conv(g, "NCHW", np.float32, x, w, None, dy, engine=_lib.ENGINE_FMA)
+    for k in ("y", "dw", "dx"):
+        assert rel_l2(got[k], fma[k]) <= 1e-5, k
