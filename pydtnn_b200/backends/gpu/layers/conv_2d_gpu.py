@@ -13,6 +13,16 @@ from .. import memory_allocation as wsp
 from .layer_gpu import LayerGPU
 
 
+class _LayerDesc(_lib.ConvDesc):
+    """A layer's descriptor: a field that is written counts as an edit of the layer (recorded passes depend on it)."""
+    layer = None
+
+    def __setattr__(self, name, value):
+        super().__setattr__(name, value)
+        if self.layer is not None:
+            self.layer.model.layer_edits += 1
+
+
 class Conv2DGPU(LayerGPU, Conv2D):
 
     def __init__(self, *args, **kwargs):
@@ -27,12 +37,14 @@ class Conv2DGPU(LayerGPU, Conv2D):
         m = self.model
         nchw = m.tensor_format == PYDTNN_TENSOR_FORMAT_NCHW
         # activations are channel-last in either format (ChannelLastTensor); the filters keep the format's layout
-        return _lib.ConvDesc(
+        desc = _LayerDesc(
             layout=_lib.LAYOUT_NHWC, dtype=_lib.dtype_code(m.dtype),
             w_layout=_lib.W_KCRS if nchw else _lib.W_KRSC, engine=getattr(m, "conv_engine", self.engine),
             n=m.batch_size, h=self.hi, w=self.wi, ci=self.ci, co=self.co, kh=self.kh, kw=self.kw,
             vpad=self.vpadding, hpad=self.hpadding, vstr=self.vstride, hstr=self.hstride,
             vdil=self.vdilation, hdil=self.hdilation)
+        desc.layer = self
+        return desc
 
     def initialize(self, prev_shape, need_dx, x):
         super().initialize(prev_shape, need_dx, x)

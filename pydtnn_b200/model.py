@@ -36,6 +36,17 @@ def _bn_fast_path(c):
     return 256 % cx == 0 and c4 % cx == 0
 
 
+def _structure(layers):
+    """The layers of a list in order, and after a block the lengths and the layers of its paths."""
+    out = []
+    for layer in layers:
+        out.append(layer)
+        for path in layer.paths:
+            out.append(len(path))
+            out += _structure(path)
+    return out
+
+
 class Model:
     def __init__(self, comm=None, non_blocking_mpi=True, dtype=np.float32, batch_size=64, tensor_format="NHWC",
                  enable_fused_bn_relu=False, enable_fused_conv_relu=False, enable_fused_conv_bn=False,
@@ -216,11 +227,11 @@ class Model:
         return self.record_passes and self.comm is None and not self.tracer.enabled \
             and getattr(self, "conv_profile", None) is None
 
-    def _pass_key(self, *more):
-        """Everything on the host that the launches of a pass depend on, and the shared buffers they use."""
+    def _pass_key(self, layers, *more):
+        """Everything on the host that the launches of a pass over ``layers`` depend on (attributes of layers and fields of
+        their descriptors through ``layer_edits``), and the shared buffers they use."""
         keep = (wsp._buf, wsp._side, wsp._red, wsp._stats)
-        return (self.layer_edits, Storage.moves, len(self.layers), self.overlap_wgrad, self.blocking_mpi, *map(id, keep),
-                *more), keep
+        return (self.layer_edits, Storage.moves, self.overlap_wgrad, self.blocking_mpi, *map(id, keep), *_structure(layers), *more), keep
 
     # -- steps ---------------------------------------------------------------------------------------
     def _ensure_loss(self):
@@ -258,7 +269,7 @@ class Model:
             global_batch_size = self.batch_size * self.nprocs
         if not self._recordable():
             return self._forward_backward(global_batch_size)
-        key, keep = self._pass_key(global_batch_size, id(self.loss_func), getattr(self.loss_func, "eps", None),
+        key, keep = self._pass_key(self.layers, global_batch_size, id(self.loss_func), getattr(self.loss_func, "eps", None),
                                    id(self.y_batch))
         keep += (self.loss_func, self.y_batch)
         recorder = self._train_recorder
@@ -399,7 +410,7 @@ class Model:
         if self._recordable():
             for bn in self._norms:       # refreshed outside the recording: only after a step or a load
                 bn.inference_inv_std()
-            x = self._eval_recorder.run(*self._pass_key(id(self._eval_layers)), self._forward)
+            x = self._eval_recorder.run(*self._pass_key(self._eval_layers), self._forward)
         else:
             x = self._forward()
         x.ary          # the answer is the caller's: in the model's tensor format before this call returns

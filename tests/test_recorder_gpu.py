@@ -97,3 +97,62 @@ def test_a_callers_own_layer_is_never_recorded():
     for _ in range(6):
         m.train_batch(x, y, SGD(0.01))
     assert len(calls) == 6 and m._train_recorder.graph is None
+
+
+def _batch(m):
+    rng = np.random.Generator(np.random.PCG64(3))
+    return rng.standard_normal((4, *m.layers[0].shape)).astype(np.float32), rng.integers(0, 10, 4)
+
+
+@pytest.mark.parametrize("evaluate", [False, True])
+def test_a_changed_descriptor_is_taken_up(evaluate):
+    from pydtnn_b200 import _lib
+    from pydtnn_b200.layers import FC, Conv2D, Flatten, Input
+    from pydtnn_b200.model import Model
+    from pydtnn_b200.optimizers import SGD
+    out = []
+    for record in (True, False):
+        np.random.seed(0)
+        m = Model(batch_size=4)
+        m.record_passes = record
+        for layer in (Input(shape=(9, 9, 32)), Conv2D(nfilters=32, filter_shape=(3, 3)), Conv2D(nfilters=64, filter_shape=(3, 3), activation="relu"),
+                      Flatten(), FC(shape=(10,), activation="softmax")):
+            m.add(layer)
+        x, y = _batch(m)
+        o = SGD(0.0, 0.0)
+        run = (lambda: m.evaluate_batch(x)) if evaluate else (lambda: m.train_batch(x, y, o))
+        for _ in range(5):
+            run()
+        assert ((m._eval_recorder if evaluate else m._train_recorder).graph is not None) == record
+        conv = [l for l in m.get_all_layers() if l.canonical_name == "Conv2D"][1]
+        conv.desc.engine = _lib.ENGINE_FMA
+        run()
+        out.append([conv.dw.ary.t.clone(), m.layers[-1].y.ary.t.clone()])
+    for p, q in zip(*out):
+        assert torch.equal(p, q)
+
+
+@pytest.mark.parametrize("inside", [False, True])
+def test_a_replaced_layer_is_called(inside):
+    from pydtnn_b200.optimizers import SGD
+
+    class Spy:
+        def __init__(self, layer):
+            self.layer, self.calls = layer, 0
+
+        def forward(self, x):
+            self.calls += 1
+            return self.layer.forward(x)
+
+        def __getattr__(self, name):
+            return getattr(self.layer, name)
+    m = _model("NHWC", True)
+    x, y = _batch(m)
+    for _ in range(5):
+        m.train_batch(x, y, SGD(0.01))
+    assert m._train_recorder.graph is not None
+    seq = next(l for l in m.layers if l.paths).paths[0] if inside else m.layers
+    seq[1] = spy = Spy(seq[1])
+    for n in range(4):
+        m.train_batch(x, y, SGD(0.01))
+        assert spy.calls == n + 1
