@@ -69,6 +69,8 @@ class LayerAndActivationBase(ABC):
             m = d.get("model")
             if m is not None:
                 m.layer_edits += 1
+                if hasattr(value, "owned_by"):          # a tensor handle
+                    value.owned_by(m)
         object.__setattr__(self, name, value)
 
     def set_model(self, parent_model):

@@ -25,6 +25,8 @@ class CategoricalCrossEntropy:
         self._counter = zeros((1,), np.int32)
         self._work = None
         self._scaled = 1
+        for handle in (self.row_loss, self.hit, self.totals, self.dx, self._counter):
+            handle.owned_by(model)
 
     def __call__(self, y_pred, labels, global_batch_size, softmax=None):
         """``labels``: device int32 array (b,). ``softmax``: the layer whose output y_pred is, when its backward

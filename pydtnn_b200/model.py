@@ -239,6 +239,7 @@ class Model:
             ncls = int(np.prod(self.layers[-1].shape))
             self.loss_func = CategoricalCrossEntropy((self.batch_size, ncls), self)
             self.y_batch = empty((self.batch_size,), np.int32)
+            self.y_batch.owned_by(self)
 
     @staticmethod
     def _labels(y_batch):

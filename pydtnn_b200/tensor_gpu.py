@@ -17,12 +17,30 @@ _TORCH_DTYPE = {np.dtype(np.float32): torch.float32, np.dtype(np.float64): torch
 
 
 class Storage:
-    #: counts, over the process, the times a tensor handle came to stand for other memory: recorded launches are only
-    #: valid while this has not moved
+    #: counts, over the process, the times a tensor handle that is no model's (or several models') came to stand for other
+    #: memory: recorded launches are only valid while this has not moved.  Handles of one model count as its layers' edits.
     moves = 0
 
 
-class DeviceArray:
+class _Owned:
+    owner = None
+
+    def owned_by(self, model):
+        """Says whose recorded passes read or write this memory; a handle of two models is nobody's."""
+        object.__setattr__(self, "owner", model if self.__dict__.get("owner", model) is model else None)
+
+    def _moved(self):
+        if self.owner is not None:
+            self.owner.layer_edits += 1
+        else:
+            Storage.moves += 1
+
+    def _hand_on(self, other):
+        if "owner" in self.__dict__:
+            other.owned_by(self.owner)
+
+
+class DeviceArray(_Owned):
     """Stands in for ``pycuda.gpuarray.GPUArray`` for the members the layer code touches."""
 
     def __init__(self, tensor: torch.Tensor):
@@ -31,7 +49,7 @@ class DeviceArray:
 
     def __setattr__(self, name, value):
         if name in self.__dict__:
-            Storage.moves += 1
+            self._moved()
         object.__setattr__(self, name, value)
 
     @property
@@ -83,7 +101,7 @@ def to_gpu(host, device=None):
     return a
 
 
-class TensorGPU:
+class TensorGPU(_Owned):
     def __init__(self, gpu_arr: DeviceArray, tensor_format, cudnn_dtype=None, tensor_type="tensor", desc=None,
                  gpudirect=False, cublas=False):
         if len(gpu_arr.shape) == 2:
@@ -100,9 +118,17 @@ class TensorGPU:
         self.desc = desc
 
     def __setattr__(self, name, value):
-        if name == "ary" and "ary" in self.__dict__:
-            Storage.moves += 1
+        if name == "ary":
+            if "ary" in self.__dict__:
+                self._moved()
+            self._hand_on(value)
         object.__setattr__(self, name, value)
+
+    def owned_by(self, model):
+        super().owned_by(model)
+        for array in map(self.__dict__.get, ("ary", "_cl", "_nchw")):
+            if array is not None:
+                array.owned_by(model)
 
     @property
     def ptr(self):
@@ -164,7 +190,8 @@ class ChannelLastTensor(TensorGPU):
         if self._nchw is None:
             n, c, h, w = self._dims
             self._nchw = empty(self._dims, self._cl.dtype, self._cl.t.device)
-            Storage.moves += 1
+            self._hand_on(self._nchw)
+            self._moved()
             transpose_inner(self._cl, self._nchw, n, h * w, c)
         return self._nchw
 

@@ -156,3 +156,27 @@ def test_a_replaced_layer_is_called(inside):
     for n in range(4):
         m.train_batch(x, y, SGD(0.01))
         assert spy.calls == n + 1
+
+
+def test_a_look_into_one_model_leaves_the_others_recordings():
+    from pydtnn_b200.optimizers import SGD
+    a, b = _model("NCHW", True), _model("NCHW", True)
+    x, y = _batch(a)
+    for _ in range(5):
+        a.train_batch(x, y, SGD(0.01)), b.train_batch(x, y, SGD(0.01))
+    ga, gb = a._train_recorder.graph, b._train_recorder.graph
+    assert ga is not None and gb is not None
+    look = b.layers[3].y.ary
+    a.train_batch(x, y, SGD(0.01)), b.train_batch(x, y, SGD(0.01))
+    assert a._train_recorder.graph is ga and b._train_recorder.graph is not gb
+    # memory that both models use is everybody's
+    shared = next(l for l in a.get_all_layers() if l.canonical_name == "Conv2D").weights
+    next(l for l in b.get_all_layers() if l.canonical_name == "Conv2D").weights = shared
+    for _ in range(4):
+        a.train_batch(x, y, SGD(0.0)), b.train_batch(x, y, SGD(0.0))
+    ga, gb = a._train_recorder.graph, b._train_recorder.graph
+    assert ga is not None and gb is not None
+    shared.ary.t = shared.ary.t.clone()
+    a.train_batch(x, y, SGD(0.0)), b.train_batch(x, y, SGD(0.0))
+    assert a._train_recorder.graph is not ga and b._train_recorder.graph is not gb
+    assert look.shape == b.layers[3].y.dims
