@@ -8,6 +8,8 @@ than its kernels run), so after ``WARM`` passes the model records one pass and r
 What a recording depends on is summed up in its key.  A changed key (an attribute of a layer, a flag of the model, a grown
 workspace, a first look at an activation) drops the recording, and the passes that follow are issued one by one until
 the new key has been seen often enough.  Only the model's own pass is recorded; hooks called one by one are not."""
+import warnings
+
 import torch
 
 from . import _lib
@@ -25,11 +27,13 @@ class Recorder:
     def run(self, key, keep, issue):
         """``issue()``, or the replay of an earlier call of it with this key.  ``keep``: tensors the launches read or write
         that nothing else may own for as long as the recording lives."""
+        if torch.cuda.is_current_stream_capturing():         # a caller's own recording takes the launches themselves
+            return issue()
         if self.graph is not None and key == self.key:
             self.graph.replay()
             _lib.lib().b2c_note_launches(self.launches)
             return self.result
-        if self.off or torch.cuda.is_current_stream_capturing():
+        if self.off:
             return issue()
         if key != self.key:
             self.key, self.seen, self.graph, self.result, self.keep = key, 0, None, None, None
@@ -56,9 +60,11 @@ class Recorder:
                     result = issue()
                 finally:
                     graph.capture_end()
-        except RuntimeError:
+        except RuntimeError as e:
             # a pass that cannot be captured (a layer that allocates or synchronises) is issued one by one for good
             self.off = True
+            m._side_pending = None       # an event of the recording that never was
+            warnings.warn(f"passes of this model are not recorded: {e.__context__ or e}", RuntimeWarning, stacklevel=2)
             return issue()
         self.graph, self.result, self.keep, self.launches = graph, result, keep, L.b2c_launch_count() - before
         graph.replay()

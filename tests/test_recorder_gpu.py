@@ -180,3 +180,45 @@ def test_a_look_into_one_model_leaves_the_others_recordings():
     a.train_batch(x, y, SGD(0.0)), b.train_batch(x, y, SGD(0.0))
     assert a._train_recorder.graph is not ga and b._train_recorder.graph is not gb
     assert look.shape == b.layers[3].y.dims
+
+
+def test_a_pass_that_cannot_be_recorded_says_why(monkeypatch):
+    from pydtnn_b200.backends.gpu.layers.fc_gpu import FCGPU
+    from pydtnn_b200.optimizers import SGD
+    backward = FCGPU.backward
+
+    def refuses(self, dy):
+        if torch.cuda.is_current_stream_capturing():
+            raise RuntimeError("looks at the host here")
+        return backward(self, dy)
+    monkeypatch.setattr(FCGPU, "backward", refuses)
+    a, b = _model("NHWC", True), _model("NHWC", False)
+    x, y = _batch(a)
+    with pytest.warns(RuntimeWarning, match="looks at the host here"):
+        for _ in range(5):
+            a.train_batch(x, y, SGD(0.01)), b.train_batch(x, y, SGD(0.01))
+    assert a._train_recorder.graph is None
+    for p, q in zip(_state(a), _state(b)):
+        assert torch.equal(p, q)
+
+
+def test_a_callers_own_recording_takes_the_launches():
+    m = _model("NHWC", True)
+    x, y = _batch(m)
+    from pydtnn_b200.optimizers import SGD
+    for _ in range(5):
+        m.train_batch(x, y, SGD(0.0, 0.0))
+    assert m._train_recorder.graph is not None
+    want = m.arena.chunks[0].dw.clone()
+    g, s = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(s):
+        with torch.cuda.graph(g):
+            m.forward_backward()
+            m.join_side_stream()
+    del m._train_recorder.graph
+    m._train_recorder.graph = None           # the caller's recording does not need the model's
+    m.arena.chunks[0].dw.zero_()
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(m.arena.chunks[0].dw, want)
