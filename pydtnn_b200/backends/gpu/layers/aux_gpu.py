@@ -51,7 +51,6 @@ class BatchNormalizationGPU(LayerGPU, BatchNormalization):
         self.y = self._activation(x.dims)
         if self.need_dx:
             self.dx = self._activation(x.dims)
-        self._x_ptr = None
         self.fuse_relu = False           # set by the model's fusion pass (BN followed by ReLU)
         self.prestats = None             # (buffer, bytes) left by the preceding convolution's forward pass of this step
         self.residual = None             # (other branch, output) while an addition block folds its sum + ReLU in here
@@ -64,7 +63,7 @@ class BatchNormalizationGPU(LayerGPU, BatchNormalization):
         m = self.model
         L = _lib.lib()
         self.x = x
-        x_ptr = self._x_ptr = self._in(x, "x")
+        x_ptr = self._in(x, "x")
         if m.mode == TRAIN_MODE and self.prestats is not None:
             # the convolution that wrote x already summed it per channel: statistics from those sums, one pass over x
             st, nbytes = self.prestats
@@ -121,7 +120,7 @@ class BatchNormalizationGPU(LayerGPU, BatchNormalization):
         m = self.model
         _lib.check(_lib.lib().b2c_bn_train_backward(
             self._dt, _lib.LAYOUT_NHWC, m.batch_size, self.ci, self._hw,
-            self._x_ptr if self._x_ptr is not None else self._in(self.x, "x"), self._in(dy, "dy"),
+            self._in(self.x, "x"), self._in(dy, "dy"),
             self._in(self.y, "y") if self.fuse_relu else None, self.beta.ptr if self.fuse_relu else None, self.gamma.ptr,
             self.save_mean.ptr, self.save_inv_var.ptr,
             self.dgamma.ptr, self.dbeta.ptr, self.dx.out if self.need_dx else None,

@@ -31,7 +31,6 @@ class Conv2DGPU(LayerGPU, Conv2D):
         self.engine = _lib.ENGINE_AUTO
         self.stats_for_bn = None         # set by the model's fusion pass: the BatchNormalization this layer feeds
         self.stats_bytes = 0
-        self._x_ptr = None
 
     def _make_desc(self):
         m = self.model
@@ -108,7 +107,7 @@ class Conv2DGPU(LayerGPU, Conv2D):
 
     def forward(self, x):
         L = _lib.lib()
-        x_ptr = self._x_ptr = self._in(x, "x")
+        x_ptr = self._in(x, "x")
         self.x = x          # backward reads the tensor this call saw (a fused predecessor may hand over its own buffer)
         bn = self.stats_for_bn
         ws_ptr, ws_size = (self._own_ws.data_ptr(), self._own_ws.numel()) if self._own_ws is not None else (wsp.ptr(), wsp.size())
@@ -128,27 +127,27 @@ class Conv2DGPU(LayerGPU, Conv2D):
         self.y.written()
         return self.y
 
-    def _wgrad_call(self, dy_ptr, ws_ptr, ws_size, stream):
+    def _wgrad_call(self, x_ptr, dy_ptr, ws_ptr, ws_size, stream):
         """The weight-gradient call on ``stream``; a layer that still holds its forward pass's lowered input in its own
         workspace uses that instead of lowering x again."""
         L = _lib.lib()
         db = self.db.ptr if self.use_bias else None
-        if self._x_ptr is None:
-            self._x_ptr = self._in(self.x, "x")
         if self._lowered_valid:
             self._lowered_valid = False
             own = self._own_ws
-            return lambda: L.b2c_conv_wgrad_lowered(ctypes.byref(self.desc), self._x_ptr, dy_ptr, self.dw.ptr, db, own.data_ptr(),
+            return lambda: L.b2c_conv_wgrad_lowered(ctypes.byref(self.desc), x_ptr, dy_ptr, self.dw.ptr, db, own.data_ptr(),
                                                     own.numel(), stream)
-        return lambda: L.b2c_conv_wgrad(ctypes.byref(self.desc), self._x_ptr, dy_ptr, self.dw.ptr, db, ws_ptr, ws_size, stream)
+        return lambda: L.b2c_conv_wgrad(ctypes.byref(self.desc), x_ptr, dy_ptr, self.dw.ptr, db, ws_ptr, ws_size, stream)
 
     def backward(self, dy):
         L = _lib.lib()
         m = self.model
         dy_ptr = self._in(dy, "dy")
+        # x as it is now; a kept lowered input stands for it (the address is then only tested)
+        x_ptr = self._own_ws.data_ptr() if self._lowered_valid else self._in(self.x, "x")
         side = m.side_stream_for_wgrad()
         if side is None:
-            self._timed("wgrad", self._wgrad_call(dy_ptr, wsp.ptr(), wsp.size(), m.stream_handle))
+            self._timed("wgrad", self._wgrad_call(x_ptr, dy_ptr, wsp.ptr(), wsp.size(), m.stream_handle))
             if self.need_dx:
                 self._timed("dgrad", lambda: L.b2c_conv_dgrad(
                     ctypes.byref(self.desc), dy_ptr, self.weights.ptr, self.dx.out, wsp.ptr(), wsp.size(), m.stream_handle))
@@ -170,7 +169,7 @@ class Conv2DGPU(LayerGPU, Conv2D):
             self.dx.written()
         side.wait_event(self._dy_ready)
         sw = wsp.side()
-        _lib.check(self._wgrad_call(dy_ptr, sw.data_ptr(), sw.numel(), side.cuda_stream)())
+        _lib.check(self._wgrad_call(x_ptr, dy_ptr, sw.data_ptr(), sw.numel(), side.cuda_stream)())
         self._wgrad_done.record(side)
         m.note_side_work(self._wgrad_done)
         return self.dx if self.need_dx else None

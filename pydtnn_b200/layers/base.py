@@ -60,7 +60,7 @@ class LayerAndActivationBase(ABC):
         self.stream_2 = None
 
     #: attributes a hook hands to the next one; everything else that changes on a layer may change its launches
-    _PASSED_ON = frozenset(("x", "_x_ptr", "prestats", "residual", "updated_running_var", "_inv_std_step", "_lowered_valid",
+    _PASSED_ON = frozenset(("x", "prestats", "residual", "updated_running_var", "_inv_std_step", "_lowered_valid",
                              "backward_done"))
 
     def __setattr__(self, name, value):

@@ -84,3 +84,34 @@ def test_large_nchw_images():
     fma = run_conv(g, "NCHW", np.float32, x, w, None, dy, engine=_lib.ENGINE_FMA)
     for k in ("y", "dw", "dx"):
         assert rel_l2(got[k], fma[k]) <= 1e-5, k
+
+
+@pytest.mark.parametrize("fmt", ["NCHW", "NHWC"])
+@pytest.mark.parametrize("replaced", [False, True])
+def test_backward_reads_x_as_it_is_then(fmt, replaced):
+    from pydtnn_b200.layers import BatchNormalization, Conv2D, Input
+    from pydtnn_b200.model import Model
+    from pydtnn_b200.tensor_gpu import DeviceArray, TensorGPU
+    from tests.gpu_util import rel_l2
+    rng = np.random.default_rng(0)
+    for layer, name in ((Conv2D(nfilters=6, filter_shape=(3, 3), padding=1), "dw"), (BatchNormalization(), "dgamma")):
+        m = Model(batch_size=2, tensor_format=fmt)
+        m.add(Input(shape=(5, 7, 20)))
+        m.add(Conv2D(nfilters=20, filter_shape=(1, 1)))
+        m.add(layer)
+        m.mode = "train"
+        m.overlap_wgrad = False
+        shape, grad = m.layers[1].y.dims, layer.y.dims
+        x0, x1, dy = (torch.from_numpy(rng.standard_normal(s).astype(np.float32)).to(DEV) for s in (shape, shape, grad))
+        x, out = TensorGPU(DeviceArray(x0.clone()), m.tensor_format), []
+        for second in (x0, x1):
+            layer.forward(x)
+            if replaced:
+                x.ary = DeviceArray(second.clone())
+            else:
+                x.ary.t.copy_(second)
+            layer.backward(TensorGPU(DeviceArray(dy.clone()), m.tensor_format))
+            out.append(getattr(layer, name).ary.t.clone())
+            x.ary.t.copy_(x0)
+        # the gradient of the weights (of gamma) is linear in the x that backward reads: x1's is not x0's
+        assert rel_l2(out[1].cpu().numpy(), out[0].cpu().numpy()) > 0.5
