@@ -179,6 +179,7 @@ class SoftmaxGPU(LayerGPU, Softmax):
         self._rows, self._cols = int(x.dims[0]), int(np.prod(x.dims[1:]))
 
     def forward(self, x):
+        self.backward_done = False       # of a step that never reached this layer's backward
         _lib.check(_lib.lib().b2c_softmax_forward(self._dt, self._rows, self._cols, x.ptr, self.y.ptr,
                                                   self.model.stream_handle))
         return self.y

@@ -37,3 +37,23 @@ def test_one_launch_equals_three(rows, cols, dtype):
         for name, u, v in zip(("row loss", "hit", "dx", "softmax dx", "totals"), a, b):
             assert torch.equal(u, v), name
         assert counter.item() == 0
+
+
+def test_a_step_that_was_cut_short_leaves_nothing_for_the_next_backward():
+    from pydtnn_b200.layers import Input, Softmax
+    from pydtnn_b200.losses import CategoricalCrossEntropy
+    from pydtnn_b200.model import Model
+    from pydtnn_b200.tensor_gpu import TensorGPU, to_gpu
+    m = Model(batch_size=4)
+    m.add(Input(shape=(6,)))
+    m.add(Softmax())
+    layer = m.layers[1]
+    layer.need_dx = True
+    rng = np.random.default_rng(0)
+    x, dy = (TensorGPU(to_gpu(rng.standard_normal((4, 6)).astype(np.float32)), m.tensor_format) for _ in "xy")
+    layer.dx = TensorGPU(to_gpu(np.zeros((4, 6), np.float32)), m.tensor_format)
+    y = layer.forward(x)
+    CategoricalCrossEntropy((4, 6), m)(y, to_gpu(np.zeros(4, np.int32)), 4, softmax=layer)
+    p, d = layer.forward(x).ary.get().astype(np.float64), dy.ary.get().astype(np.float64)
+    got = layer.backward(dy).ary.get()
+    assert np.allclose(got, p * (d - (d * p).sum(1, keepdims=True)), atol=1e-6)
