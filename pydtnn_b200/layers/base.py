@@ -41,6 +41,10 @@ class PromoteToBackendMixin:
         return name[:-3] if name.endswith("GPU") else name
 
 
+#: attributes a hook hands to the next one; everything else that changes on a layer may change its launches
+_PASSED_ON = frozenset(("x", "prestats", "residual", "updated_running_var", "_inv_std_step", "_lowered_valid", "backward_done"))
+
+
 class LayerAndActivationBase(ABC):
     """State shared by layers and activations, and the five hooks a back end implements."""
 
@@ -59,13 +63,12 @@ class LayerAndActivationBase(ABC):
         self.reqs_allred = {}
         self.stream_2 = None
 
-    #: attributes a hook hands to the next one; everything else that changes on a layer may change its launches
-    _PASSED_ON = frozenset(("x", "prestats", "residual", "updated_running_var", "_inv_std_step", "_lowered_valid",
-                             "backward_done"))
-
     def __setattr__(self, name, value):
         d = self.__dict__
-        if name not in self._PASSED_ON and d.get(name, d) is not value:
+        if name in _PASSED_ON:
+            d[name] = value
+            return
+        if d.get(name, d) is not value:
             m = d.get("model")
             if m is not None:
                 m.layer_edits += 1

@@ -146,10 +146,12 @@ class TensorGPU(_Owned):
 
     def channel_last(self):
         """Address of the values with the channel axis last, or None where they are stored otherwise."""
-        s = self.ary.shape
-        if self.tensor_format != PYDTNN_TENSOR_FORMAT_NCHW or len(s) != 4 or s[1] == 1 or s[2] * s[3] == 1:
-            return self.ary.gpudata
-        return None
+        t = self.ary.t
+        if self.tensor_format == PYDTNN_TENSOR_FORMAT_NCHW and t.dim() == 4:
+            _, c, h, w = t.shape
+            if c != 1 and h * w != 1:
+                return None
+        return t.data_ptr()
 
     @property
     def out(self):
