@@ -2,11 +2,11 @@
 
     python pydtnn_b200/csrc/build.py [--force] [-v] [--variant profile|switches]
 
-Two development variants of the tensor-core kernel can be built next to the product library (they are never loaded
-by the package; ``role_profile.py`` in this directory loads them by path):
+Two development variants of the tensor-core kernel can be built next to the product library (never loaded by the
+package):
 
 * ``--variant profile``  -> ``pydtnn_b200/libb2c_profile.so`` (``-DB2C_TC_PROFILE``): every warp role of CTA 0 adds up
-  the cycles it spends waiting and working (slots named in ``role_profile.py``), read with ``b2c_debug_prof``.
+  the cycles it spends waiting and working (a slot per ``TC_PROF_ADD``), read with ``b2c_debug_prof``.
 * ``--variant switches`` -> ``pydtnn_b200/libb2c_switches.so`` (``-DB2C_TC_SWITCHES``): the environment variable
   ``B2C_TC_DBG`` switches parts of the kernel off to see what the rest costs (results are then wrong): 2 = one MMA of
   three, 4 = transform warps do no work, 32 = no MMA, 64 = no TMA loads; values add.
