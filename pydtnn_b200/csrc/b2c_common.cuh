@@ -115,6 +115,7 @@ int channel_sum_v4(int n, int c, int hw, const void* src, void* dst, void* ws, s
 
 // tensor-core engine (conv_tc.cu)
 bool tc_supported(const Geo& g, int pass);
+int tc_sm_count();      // of the current device
 bool tc_takes_alignment(const Geo& g, int pass, const void* x, const void* y);
 bool tc_refuses_unaligned(const Geo& g, int pass);
 bool tc_fine_sums(const Geo& g, int pass);

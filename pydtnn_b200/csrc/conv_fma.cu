@@ -7,8 +7,7 @@
 //   dgrad : C[pixel(n,h,w)][ci]   = sum_tap  dy[(pixel + pad - tap) / stride] * w[tap.co][ci][tap.r][tap.s]
 //   wgrad : C[tap(ci,r,s)][co]    = sum_pixel x[pixel + tap] * dy[pixel][co]      (split over pixels)
 //
-// float32 uses FP32 FMA, float64 the FP64 tensor pipe where the shape allows and FP64 FMA elsewhere.  This engine is the one every shape can run on;
-// the tensor-core engine (conv_tc.cu) takes over the shapes it supports.
+// float32 uses FP32 FMA, float64 the FP64 tensor pipe.  This engine is the one every shape can run on; the tensor-core engine (conv_tc.cu) takes over the shapes it supports.
 #include "b2c_common.cuh"
 #include <atomic>
 #include <type_traits>
@@ -768,8 +767,8 @@ static int tile_bn(int N) { return N <= 64 ? 64 : 128; }
 static int choose_splits(const IgemmParams& p, int bk)
 {
     int64_t ctas = (int64_t)((p.M + 127) / 128) * ((p.N + tile_bn(p.N) - 1) / tile_bn(p.N));
-    if (ctas >= 148) return 1;
-    int64_t want = (296 + ctas - 1) / ctas;
+    if (ctas >= tc_sm_count()) return 1;
+    int64_t want = (2 * tc_sm_count() + ctas - 1) / ctas;
     int64_t max_by_k = p.K / (8 * bk);
     if (max_by_k < 1) max_by_k = 1;
     int64_t s = want < max_by_k ? want : max_by_k;
@@ -782,7 +781,7 @@ static int choose_splits(const IgemmParams& p, int bk)
 static int choose_splits_f64(const IgemmParams& p, int bk)
 {
     const int64_t ctas = (int64_t)((p.M + 127) / 128) * ((p.N + tile_bn(p.N) - 1) / tile_bn(p.N));
-    const int64_t room = 148, slices = (p.K + bk - 1) / bk;
+    const int64_t room = tc_sm_count(), slices = (p.K + bk - 1) / bk;
     int64_t best = 1, cost = 0;
     for (int64_t s = 1; s <= 128 && s <= slices && (s == 1 || ctas * s <= 2 * room); s++) {
         const int64_t c = (ctas * s + room - 1) / room * ((slices + s - 1) / s + (s > 1 ? 6 : 3));

@@ -1788,7 +1788,7 @@ static bool lowered_ok(const Geo& g)
     // One k-block per tap read in place, or K / 32 full ones (0.6 us of an SM per 128 rows) and the matrix written and read once
     // (about 4 TB/s).  A tap in place took 0.55 to 0.73 us with pixels of 32 or 64 bytes and 0.75 to 0.98 with 16 or 48 (sweep of
     // 4 to 16 channels, 3x3 to 7x7, 14x14 to 80x80).
-    const double tiles = (double)((g.M + 127) / 128) * ((g.co + 127) / 128) / 148.0;
+    const double tiles = (double)((g.M + 127) / 128) * ((g.co + 127) / 128) / tc_sm_count();
     const double in_place = tiles * g.kh * g.kw * (g.ci % 8 ? 0.9e-6 : 0.62e-6);
     const double lowered = tiles * (lowered_kp(g) / 32) * 0.6e-6 + (double)g.M * lowered_kp(g) * 8.0 / 4e12 + 3e-6;
     return lowered < in_place;
@@ -1831,7 +1831,7 @@ struct PerDeviceOnce {
     }
 };
 
-static int tc_sm_count()
+int tc_sm_count()
 {
     static int sm_count[B2C_MAX_DEVICES] = {};
     static std::mutex m;
@@ -1864,15 +1864,6 @@ static unsigned int* tc_sync_bank(cudaStream_t st)
     if (owners[dev] == TC_SYNC_BANKS) return nullptr;
     owner[dev][owners[dev]] = st;
     return base[dev] + (size_t)(owners[dev]++) * TC_SYNC_WORDS;
-}
-
-// Whole tiles against balanced ranges: balanced mode is taken when its cost estimate is below this share of the plain
-// one (B2C_TC_BALANCE overrides it, for experiments).
-static double tc_balance_threshold()
-{
-    static double v = -1.0;
-    if (v < 0.0) { const char* e = getenv("B2C_TC_BALANCE"); v = e ? atof(e) : 1.0; }
-    return v;
 }
 
 // Balanced mode scratch: 4 flags per CTA (padded to 4 KB) and one 128 x 128 float partial tile per CTA.
@@ -2111,7 +2102,7 @@ static FwdPlan fwd_plan(int64_t M, int N, int64_t kblocks, bool may_share, bool 
         if (!may_share) continue;
         const double shared = (double)G / (double)tiles;         // CTAs on one tile
         if (!fine && tiles * kblocks >= 4 * (int64_t)G)
-            offer(((double)(tiles * kblocks) / G * kb + 11.0 + (shared > 2.0 ? 4.5 * (shared - 2.0) : 0.0) + drain) / tc_balance_threshold(), true, 0);
+            offer((double)(tiles * kblocks) / G * kb + 11.0 + (shared > 2.0 ? 4.5 * (shared - 2.0) : 0.0) + drain, true, 0);
         for (int64_t s = 2; s * tiles <= G && s <= kblocks; s++) {
             const int64_t kper = (kblocks + s - 1) / s;
             if (short_sums && kper * G >= units + G) continue;
@@ -2811,7 +2802,8 @@ bool tc_supported(const Geo& g, int pass)
     if (g.engine == B2C_ENGINE_TENSOR) return true;
     // two tensors are copied there and/or back (read + write each) at about 2.5 TB/s; this engine runs the pass at about
     // 130 TFLOP/s.  The shapes where the copies weigh have few multiplications per value, and there the FMA engine makes 2 to
-    // 4 of its tiles' operations (4 channels, 3x3, 56x56 to 80x80: 1.9 to 2.5 TFLOP/s), not the 20 of a deep layer
+    // 4 of its tiles' operations (4 channels, 3x3, 56x56 to 80x80: 1.9 to 2.5 TFLOP/s).  4 is taken for every shape: a deep layer,
+    // where it makes 20, is this engine's by far either way
     const double flops = 2.0 * (double)g.M * (double)g.K * g.co, tiles = 2.0 * (double)g.M * (g.K < 32 ? 32 : (double)g.K) * (g.co < 64 ? 64 : g.co);
     const double xb = 4.0 * g.n * g.h * g.w * g.ci, yb = 4.0 * (double)g.M * g.co;
     const double moved = 2.0 * (xb + yb);
