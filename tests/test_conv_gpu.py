@@ -395,3 +395,29 @@ def test_weight_gradient_from_the_forward_pass_lowered_input_is_bit_identical():
     assert L.b2c_conv_keeps_lowered_input(ctypes.byref(d2)) == 0
     t = torch.zeros(64, device=DEV)
     assert L.b2c_conv_wgrad_lowered(ctypes.byref(d2), t.data_ptr(), t.data_ptr(), t.data_ptr(), None, t.data_ptr(), 256, stream()) == -6
+
+
+@pytest.mark.parametrize("layout,n,h,ci,cout,k,pad,st", [("NHWC", 16, 56, 64, 256, 1, 0, 1), ("NHWC", 16, 56, 128, 64, 1, 0, 1), ("NCHW", 8, 28, 128, 128, 1, 0, 1),
+                                                         ("NHWC", 8, 28, 256, 128, 1, 0, 1), ("NHWC", 8, 28, 64, 64, 3, 1, 1), ("NHWC", 32, 14, 256, 256, 3, 1, 1),
+                                                         ("NHWC", 1, 14, 256, 256, 3, 1, 1), ("NHWC", 8, 28, 128, 128, 3, 1, 2), ("NHWC", 9, 33, 40, 72, 3, 1, 1)])
+def test_repeats_are_bit_identical(layout, n, h, ci, cout, k, pad, st):
+    """Whatever overlaps whatever inside a launch (resident filters, rings that are refilled early, balanced ranges, split K loops,
+    classes in one launch, fine sums), and between launches, the bits are the same every time."""
+    L = _lib.lib()
+    g = co.Geom(n, h, h, ci, cout, k, k, pad, pad, st, st)
+    w_layout = "KRSC" if layout == "NHWC" else "KCRS"
+    desc = make_desc(g, layout, np.float32, w_layout)
+    gen = torch.Generator(device=DEV).manual_seed(1)
+    act = (lambda s, c: (n, s, s, c)) if layout == "NHWC" else (lambda s, c: (n, c, s, s))
+    x, dy, w = (torch.randn(s, device=DEV, generator=gen) for s in (act(h, ci), act(g.ho, cout), (cout, k, k, ci) if layout == "NHWC" else (cout, ci, k, k)))
+    ws = workspace(desc)
+    first = None
+    for _ in range(40):
+        y, dx, dw, db = (torch.full_like(t, float("nan")) for t in (dy, x, w, torch.empty(cout, device=DEV)))
+        d, p = ctypes.byref(desc), ws.data_ptr()
+        _lib.check(L.b2c_conv_fprop(d, x.data_ptr(), w.data_ptr(), None, None, 0, y.data_ptr(), p, ws.numel(), stream()))
+        _lib.check(L.b2c_conv_dgrad(d, dy.data_ptr(), w.data_ptr(), dx.data_ptr(), p, ws.numel(), stream()))
+        _lib.check(L.b2c_conv_wgrad(d, x.data_ptr(), dy.data_ptr(), dw.data_ptr(), db.data_ptr(), p, ws.numel(), stream()))
+        first = first or (y, dx, dw, db)
+        assert all(torch.equal(a, b) for a, b in zip(first, (y, dx, dw, db)))
+    assert all(bool(torch.isfinite(t).all()) for t in first)
