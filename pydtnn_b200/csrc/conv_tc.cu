@@ -37,6 +37,7 @@
 // status word in global memory, skips its remaining work, frees its tensor memory and returns.
 #include "b2c_common.cuh"
 #include <cuda.h>
+#include <float.h>
 #include <stdlib.h>
 #include <mutex>
 #include <type_traits>
@@ -217,11 +218,18 @@ __device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&r
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-__device__ __forceinline__ float to_tf32_rn(float v) {
-    uint32_t r;
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(v));
-    return __uint_as_float(r);
+// v rounded to nearest tf32 (ties away from zero) in two integer operations: the conversion instruction runs at a fraction of
+// their rate.  A value that is not finite has no hi half and is its own lo half: an infinity then meets the other operand's hi
+// half only, and the product has the sign it should (with hi = inf the lo half would be inf - inf, and inf times the other's
+// lo half has either sign or none).
+__device__ __forceinline__ float tc_rounded(float v) { return __uint_as_float((__float_as_uint(v) + 0x1000u) & 0xFFFFE000u); }
+__device__ __forceinline__ float tc_rounded_hi(float v) {
+    const float h = tc_rounded(v);
+    return fabsf(h) <= FLT_MAX ? h : 0.f;
 }
+// Whether any value of a thread's share with this largest magnitude needs tc_rounded_hi (a NaN does not: its lo half is one
+// whatever its hi half).  Asked once per 32 values it costs 75x43 40->72 3x3 layers 6 us of 105, on every value it cost 16.
+__device__ __forceinline__ bool tc_rounds_to_inf(float largest) { return largest >= __uint_as_float(0x7F7FF000u); }
 
 // Shared-memory matrix descriptor for tiles made of 128-byte rows.
 //  K-major (layout 2 = 128B swizzle): a row is 32 K elements of one M/N row; 8-row groups lie
@@ -304,7 +312,7 @@ __global__ void tc_prep_filter_kernel(PrepParams p, const float* __restrict__ w,
         int c = k % p.Cp; int rs = k / p.Cp; int r = rs / p.S; int s = rs - r * p.S;
         r = p.r0 + p.rstep * r; s = p.s0 + p.sstep * s;
         float v = c < p.C ? w[row * p.s_row + c * p.s_c + r * p.s_r + s * p.s_s] : 0.f;
-        float h = to_tf32_rn(v);
+        const float h = tc_rounded_hi(v);
         hi[i] = h;
         lo[i] = v - h;
     }
@@ -440,7 +448,7 @@ __global__ void tc_prep_filter_lowered_kernel(int rows, int K, int Kp, int C, in
         const int row = (int)(i / Kp), k = (int)(i - (int64_t)row * Kp);
         float v = 0.f;
         if (k < K) { const int c = k % C, rs = k / C, r = rs / S, sx = rs - r * S; v = w[row * s_row + c * s_c + r * s_r + sx * s_s]; }
-        const float h = to_tf32_rn(v);
+        const float h = tc_rounded_hi(v);
         hi[i] = h; lo[i] = v - h;
     }
 }
@@ -461,13 +469,12 @@ __device__ __forceinline__ float4 tc_lo_of_truncated(const float4 q) {
     return make_float4(q.x - __uint_as_float(__float_as_uint(q.x) & 0xFFFFE000u), q.y - __uint_as_float(__float_as_uint(q.y) & 0xFFFFE000u),
                        q.z - __uint_as_float(__float_as_uint(q.z) & 0xFFFFE000u), q.w - __uint_as_float(__float_as_uint(q.w) & 0xFFFFE000u));
 }
-// to_tf32_rn in two integer operations: the conversion instruction runs at a fraction of their rate.  (A NaN may leave here
-// as a number; its lo half is still a NaN.)
-__device__ __forceinline__ float tc_rounded_hi(float v) { return __uint_as_float((__float_as_uint(v) + 0x1000u) & 0xFFFFE000u); }
 // The same with hi rounded to nearest: lo takes either sign and is half as large, and so is the
 // dropped product of two lo halves.  q becomes hi, to be written back.
+template <bool CAREFUL>
 __device__ __forceinline__ float4 tc_split_rounded(float4& q) {
-    const float4 h = make_float4(tc_rounded_hi(q.x), tc_rounded_hi(q.y), tc_rounded_hi(q.z), tc_rounded_hi(q.w));
+    const float4 h = CAREFUL ? make_float4(tc_rounded_hi(q.x), tc_rounded_hi(q.y), tc_rounded_hi(q.z), tc_rounded_hi(q.w))
+                             : make_float4(tc_rounded(q.x), tc_rounded(q.y), tc_rounded(q.z), tc_rounded(q.w));
     const float4 l = make_float4(q.x - h.x, q.y - h.y, q.z - h.z, q.w - h.w);
     q = h;
     return l;
@@ -1061,7 +1068,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
 #pragma unroll
                     for (int i = 0; i < L::B_BYTES / 16 / 128; i++) {
                         float4 q = b_hi[t + i * 128];
-                        if (p.b_round) { b_lo[t + i * 128] = tc_split_rounded(q); b_hi[t + i * 128] = q; }
+                        if (p.b_round) { b_lo[t + i * 128] = tc_split_rounded<true>(q); b_hi[t + i * 128] = q; }
                         else b_lo[t + i * 128] = tc_lo_of_truncated(q);
                     }
                 }
@@ -1119,11 +1126,21 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 }
                 const uint32_t slot = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(L::TMEM_A_COL + ts * 64);
                 uint32_t low[32];
+                float largest = 0.f;
+                if (FINE) {
 #pragma unroll
-                for (int j = 0; j < 32; j++) {
-                    const float a = __uint_as_float(v[j]);
-                    if (FINE) { const float h = tc_rounded_hi(a); low[j] = __float_as_uint(a - h); v[j] = __float_as_uint(h); }
-                    else low[j] = __float_as_uint(a - __uint_as_float(v[j] & 0xFFFFE000u));
+                    for (int j = 0; j < 32; j += 2) largest = fmaxf(largest, fmaxf(fabsf(__uint_as_float(v[j])), fabsf(__uint_as_float(v[j + 1]))));
+                }
+                if (FINE && tc_rounds_to_inf(largest)) {
+#pragma unroll
+                    for (int j = 0; j < 32; j++) { const float a = __uint_as_float(v[j]), h = tc_rounded_hi(a); low[j] = __float_as_uint(a - h); v[j] = __float_as_uint(h); }
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 32; j++) {
+                        const float a = __uint_as_float(v[j]), h = FINE ? tc_rounded(a) : __uint_as_float(v[j] & 0xFFFFE000u);
+                        low[j] = __float_as_uint(a - h);
+                        if (FINE) v[j] = __float_as_uint(h);
+                    }
                 }
                 tmem_st_32x32(slot, v);              // hi: the tensor core reads the upper 19 bits
                 if (RESKB) {
@@ -1137,8 +1154,17 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                     float4* b_lo = (float4*)(smem + s * L::STAGE_BYTES + L::A_BYTES + L::B_BYTES);
                     if (FINE || (MODE == TCM_FWD && p.b_round)) {
                         float4* b_hi = (float4*)(smem + s * L::STAGE_BYTES + L::A_BYTES);
+                        float largest = 0.f;
 #pragma unroll
-                        for (int i = 0; i < B_VEC; i++) { b_lo[t + i * 128] = tc_split_rounded(bq[i]); b_hi[t + i * 128] = bq[i]; }
+                        for (int i = 0; i < B_VEC; i++)
+                            largest = fmaxf(largest, fmaxf(fmaxf(fabsf(bq[i].x), fabsf(bq[i].y)), fmaxf(fabsf(bq[i].z), fabsf(bq[i].w))));
+                        if (!tc_rounds_to_inf(largest)) {
+#pragma unroll
+                            for (int i = 0; i < B_VEC; i++) { b_lo[t + i * 128] = tc_split_rounded<false>(bq[i]); b_hi[t + i * 128] = bq[i]; }
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < B_VEC; i++) { b_lo[t + i * 128] = tc_split_rounded<true>(bq[i]); b_hi[t + i * 128] = bq[i]; }
+                        }
                     } else {
 #pragma unroll
                         for (int i = 0; i < B_VEC; i++) {
@@ -2751,8 +2777,8 @@ static Copies tc_copies(const Geo& g, int pass)
 // better if this engine's sums of 256 products in tensor memory, ten times less accurate, were all it had to offer: channel
 // counts that are no whole blocks, fully connected layers of few rows, layers of NCHW networks too small to pay for copies of
 // their activations at 130 against 26 TFLOP/s.  Errors against float64 (2-norms, 100 layers drawn over the sizes of a sweep):
-// FMA engine 1e-7 to 4e-7, 256-product sums 6e-7 to 2.1e-6, this form 0.9e-7 to 2e-7.  It costs 75x43 40->72 3x3 layers 27 us
-// of 77 (the FMA engine: 378), a 64 x 4096 x 1000 fully connected layer 5 of 39 (124).
+// FMA engine 1e-7 to 4e-7, 256-product sums 6e-7 to 2.1e-6, this form 0.9e-7 to 2e-7.  It costs 75x43 40->72 3x3 layers 34 us
+// on 77 (the FMA engine: 378), a 64 x 4096 x 1000 fully connected layer 5 on 39 (124).
 bool tc_fine_sums(const Geo& g, int pass)
 {
     if (g.dtype != B2C_F32) return false;

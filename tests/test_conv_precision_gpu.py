@@ -90,3 +90,29 @@ def test_short_ranges_are_not_made_longer():
         ref = co.conv2d_forward(x[:2].astype(np.float64), wt.astype(np.float64), np.zeros(128), co.Geom(2, 15, 15, 256, 128, 5, 5, 2, 2, 1, 1), "NHWC")
         err.append(np.linalg.norm(y - ref) / np.linalg.norm(ref))
     assert err[0] <= 0.9 * err[1], err
+
+
+@pytest.mark.parametrize("shape", [("NHWC", 2, 12, 9, 40, 72, 3, 1, 1), ("NCHW", 2, 11, 11, 36, 100, 3, 1, 2), ("NHWC", 64, 1, 1, 520, 384, 1, 0, 1),
+                                   ("NCHW", 2, 16, 16, 3, 21, 5, 2, 1), ("NHWC", 1, 8, 8, 423, 130, 3, 1, 1)])
+@pytest.mark.parametrize("where", ["x", "w", "dy"])
+def test_infinities_come_out_as_from_fmas(shape, where):
+    """Passes that came from the FMA engine answer infinities and NaNs in the same places."""
+    layout, n, h, w, ci, cout, k, pad, st = shape
+    g = co.Geom(n, h, w, ci, cout, k, k, pad, pad, st, st)
+    rng = np.random.Generator(np.random.PCG64(ci))
+    nchw = layout == "NCHW"
+    t = {"x": rng.standard_normal((n, ci, h, w) if nchw else (n, h, w, ci)).astype(np.float32),
+         "w": rng.standard_normal((cout, ci, k, k) if nchw else (ci, k, k, cout)).astype(np.float32),
+         "dy": rng.standard_normal((n, cout, g.ho, g.wo) if nchw else (n, g.ho, g.wo, cout)).astype(np.float32)}
+    # operands that tf32 holds exactly (no lower half), zeros among them, and those that it does not
+    for name in t:
+        t[name].flat[::3] = np.float32(1.5) * np.sign(t[name].flat[::3])
+        t[name].flat[::50] = 0
+    bad = t[where].reshape(-1)
+    bad[bad.size // 3], bad[bad.size // 2 + 1], bad[bad.size - 2] = np.inf, -np.inf, np.nan
+    w_layout = "KCRS" if nchw else "KRSC"
+    a, b = (run_conv(g, layout, np.float32, t["x"], t["w"], None, t["dy"], w_layout=w_layout, engine=e) for e in (_lib.ENGINE_AUTO, _lib.ENGINE_FMA))
+    for name in ("y", "dw", "dx"):
+        assert np.array_equal(np.isnan(a[name]), np.isnan(b[name])), name
+        assert np.array_equal(np.isinf(a[name]), np.isinf(b[name])), name
+        assert np.array_equal(a[name][np.isinf(b[name])], b[name][np.isinf(b[name])]), name
