@@ -120,9 +120,11 @@ extern "C" int b2c_conv_fprop(const b2c_conv_desc* desc, const void* x, const vo
     int e; rc = call_engine(g, B2C_PASS_FPROP, x, y, e); if (rc) return rc;
     if (e == B2C_ENGINE_TENSOR) return tc_fprop(g, x, w, bias, bn, relu, y, ws, ws_bytes, (cudaStream_t)stream);
     rc = fma_fprop(g, x, w, bias, bn, relu, y, ws, ws_bytes, (cudaStream_t)stream);
-    // a layer that keeps its lowered input has it in the workspace after every forward pass
+    // a layer that keeps its lowered input has it in the workspace after every forward pass, if the workspace can hold it: one
+    // that cannot is refused by the weight gradient, which needs more
     if (rc || !b2c_conv_keeps_lowered_input(desc)) return rc;
-    return tc_leave_lowered(g, x, ws, ws_bytes, (cudaStream_t)stream);
+    rc = tc_leave_lowered(g, x, ws, ws_bytes, (cudaStream_t)stream);
+    return rc == B2C_ERR_WORKSPACE_TOO_SMALL ? B2C_OK : rc;
 }
 
 extern "C" size_t b2c_conv_stats_bytes(const b2c_conv_desc* desc) {

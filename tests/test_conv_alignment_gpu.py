@@ -47,6 +47,19 @@ def test_weight_gradient_from_the_lowered_input(cout, off_x, off_y, off_dy):
         assert off_dy and bool(torch.isnan(dw).all())           # dy is the one operand that may be refused
 
 
+def test_forward_on_an_unaligned_y_needs_no_room_for_the_lowered_input():
+    L = _lib.lib()
+    g, desc, x, w, b, dy = _case(64)
+    y, want = _at(torch.zeros_like(dy), 1), torch.empty_like(dy)
+    fma = make_desc(g, "NHWC", np.float32, "KRSC", engine=_lib.ENGINE_FMA)
+    ws = torch.empty(max(256, L.b2c_conv_workspace_bytes(ctypes.byref(fma), _lib.PASS_FPROP)), dtype=torch.uint8, device=DEV)
+    for d, out in ((desc, y), (fma, want)):
+        _lib.check(L.b2c_conv_fprop(ctypes.byref(d), x.data_ptr(), w.data_ptr(), b.data_ptr(), None, 0, out.data_ptr(), ws.data_ptr(), ws.numel(), stream()))
+    assert torch.equal(y, want)
+    dw = torch.empty_like(w)
+    assert L.b2c_conv_wgrad_lowered(ctypes.byref(desc), x.data_ptr(), dy.data_ptr(), dw.data_ptr(), None, ws.data_ptr(), ws.numel(), stream()) != 0
+
+
 def test_forward_with_batch_sums_reads_x_anywhere():
     L = _lib.lib()
     g, desc, x, w, b, dy = _case(64)
