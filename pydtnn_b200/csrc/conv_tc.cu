@@ -28,9 +28,9 @@
 // shared memory for the whole launch; several pixel classes (a strided data gradient) in one launch.  NCHW tensors
 // run on channel-last copies.
 //
-// Warp roles (320 threads; 448 with eight drain warps): warp 0 = TMA producer, warp 1 = TMEM owner + MMA issuer
-// (one elected lane of each runs the whole loop), warps 2-5 = operand transform,
-// warps 6-9 (6-13) = drain + epilogue: the tensor core's accumulate step truncates, so sums are kept in
+// Warp roles: warp 0 = TMA producer, warp 1 = TMEM owner + MMA issuer (one elected lane of each runs the whole loop), four
+// warps that split A, four that split B where a raw B tile is split (tc_b_warps; else the A warps do it), four or
+// eight that drain: the tensor core's accumulate step truncates, so sums are kept in
 // tensor memory only for a chunk of 8 k-blocks (two TMEM buffers alternate) and added chunk by
 // chunk into float32 registers with round-to-nearest, then bias / BN-scale / ReLU -> global.
 // Every mbarrier wait is bounded: when a wait runs out the CTA raises an abort flag, records a
@@ -690,12 +690,32 @@ struct TileGeo {
 // warps per tensor-memory lane quadrant, each taking half of the tile's columns).
 constexpr int TC_STREAM8 = 2;
 template <int STREAM> constexpr int tc_drain_warps() { return STREAM == TC_STREAM8 ? 8 : 4; }
-template <int STREAM> constexpr int tc_threads() { return (6 + tc_drain_warps<STREAM>()) * 32; }
+// Whether the lo half of the B tile is made by four warps of its own.  Four warps that split both tiles were busy for some 870
+// cycles per k-block of 128 columns (768 are products), one k-block after the other: fine sums, whose split is longer, and
+// launches of a few k-blocks waited for them (75x43 40->72 3x3, three passes 111 -> 104 us; a single image through ResNet-50 624 ->
+// 619).  Long launches gain 1 % or nothing: they are bound by shared-memory traffic (128 KB per k-block: 32 in by TMA, 48 for
+// the split, 48 to the tensor core, 1024 cycles at 128 bytes each).  Not with pre-split or resident filters (no B tile to
+// split) and not beside eight drain warps (no registers).
+template <int MODE, int BSRC, int STREAM, int RESKB> constexpr bool tc_b_warps()
+{
+    return (MODE == TCM_WGRAD || BSRC != TCB_SPLIT) && RESKB == 0 && STREAM != TC_STREAM8;
+}
+// Warp roles: 0 producer, 1 MMA issuer, then the transform and the drain warps.  With B warps: 4-7 split A, 8-11 split B, 12-15
+// drain (2 and 3 idle), so that each role is a warpgroup and can take its own share of the registers: the launch has 128 per
+// thread, the roles share out 4 x 128 (issue 64, split 112: the issuing warps spilled).
+constexpr int TC_REGS_ISSUE = 96, TC_REGS_SPLIT = 96, TC_REGS_DRAIN = 224, TC_REGS_LAUNCH = 128;
+static_assert(TC_REGS_ISSUE + 2 * TC_REGS_SPLIT + TC_REGS_DRAIN <= 4 * TC_REGS_LAUNCH, "a larger sum would wait for registers that never come");
+template <int N> __device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> __device__ __forceinline__ void regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int MODE, int BSRC, int STREAM, int RESKB> constexpr int tc_threads()
+{
+    return tc_b_warps<MODE, BSRC, STREAM, RESKB>() ? 512 : (6 + tc_drain_warps<STREAM>()) * 32;
+}
 
 // FINE: sums at the precision of float32 FMAs (see tc_fine_sums): both operands split by rounding, each k-block summed in tensor
 // memory by itself, its small products first.
 template <int MODE, int BN, int STAGES, bool SK, int SLABS, int BSRC, int STREAM, bool MULTI, int RESKB = 0, bool FINE = false>
-__global__ void __launch_bounds__(tc_threads<STREAM>(), 1)
+__global__ void __launch_bounds__(tc_threads<MODE, BSRC, STREAM, RESKB>(), 1)
 conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b0,
                const __grid_constant__ CUtensorMap tmap_b1, const __grid_constant__ CUtensorMap tmap_out,
                const __grid_constant__ CUtensorMap tmap_a3, TcParams p)
@@ -725,6 +745,8 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     // drain warps still store the previous one.
     using L = TcSmem<BN, STAGES, SLABS, tc_drain_warps<STREAM>(), RESKB>;
     constexpr int DW = tc_drain_warps<STREAM>();
+    constexpr bool BW = tc_b_warps<MODE, BSRC, STREAM, RESKB>();
+    constexpr int XWARP = BW ? 4 : 2, DWARP = BW ? 12 : 6;       // first transform and first drain warp
     constexpr int TSLOTS = L::TSLOTS;
     static_assert(RESKB == 0 || (STREAM == TC_STREAM8 && BSRC != TCB_SPLIT), "resident filters: short-K streaming variant on the caller's filter");
     static_assert(!FINE || (!SK && STREAM == 0 && RESKB == 0), "fine sums: chunked drain, whole tiles or split K loops");
@@ -759,8 +781,8 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     if (threadIdx.x < 32) {
         if (threadIdx.x < NBARS) {
             const uint64_t* bar = full_bar + threadIdx.x;
-            const bool by_four = (bar >= xform_bar && bar < empty_bar) || (bar >= afree_bar && bar < bres_bar);
-            mbar_init(full_bar + threadIdx.x, by_four ? 4 : bar >= tempty_bar && bar < afree_bar ? DW : 1);
+            const bool by_four = bar >= afree_bar && bar < bres_bar, by_xform = bar >= xform_bar && bar < empty_bar;
+            mbar_init(full_bar + threadIdx.x, by_xform ? (BW ? 8 : 4) : by_four ? 4 : bar >= tempty_bar && bar < afree_bar ? DW : 1);
         }
         if (threadIdx.x == 0) *abort_flag = 0;
         fence_barrier_init();
@@ -775,6 +797,38 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
+    // The lo half of stage s's B tile, written next to it (the raw tile serves as hi, or is overwritten with the rounded one).
+    // Thread t of 128 takes float4s t, t + 128, ..; with sum it adds each to the bias gradient's sums of its box.
+    auto split_b = [&](int s, int t, bool sum, float4* acc) {
+        constexpr int VEC = L::B_BYTES / 16 / 128;
+        float4* b_hi = (float4*)(smem + s * L::STAGE_BYTES + L::A_BYTES);
+        float4* b_lo = (float4*)(smem + s * L::STAGE_BYTES + L::A_BYTES + L::B_BYTES);
+        float4 q[VEC];
+#pragma unroll
+        for (int i = 0; i < VEC; i++) q[i] = b_hi[t + i * 128];
+        if (FINE || (MODE == TCM_FWD && p.b_round)) {
+            float largest = 0.f;
+#pragma unroll
+            for (int i = 0; i < VEC; i++) largest = fmaxf(largest, fmaxf(fmaxf(fabsf(q[i].x), fabsf(q[i].y)), fmaxf(fabsf(q[i].z), fabsf(q[i].w))));
+            if (!tc_rounds_to_inf(largest)) {
+#pragma unroll
+                for (int i = 0; i < VEC; i++) { b_lo[t + i * 128] = tc_split_rounded<false>(q[i]); b_hi[t + i * 128] = q[i]; }
+            } else {
+#pragma unroll
+                for (int i = 0; i < VEC; i++) { b_lo[t + i * 128] = tc_split_rounded<true>(q[i]); b_hi[t + i * 128] = q[i]; }
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < VEC; i++) {
+                if (MODE == TCM_WGRAD && sum) { acc[i >> 1].x += q[i].x; acc[i >> 1].y += q[i].y; acc[i >> 1].z += q[i].z; acc[i >> 1].w += q[i].w; }
+                b_lo[t + i * 128] = tc_lo_of_truncated(q[i]);
+            }
+        }
+        fence_proxy_async();
+    };
+
+    if (warp < XWARP) {
+    if (BW) regs_dec<TC_REGS_ISSUE>();               // the two issuing warps and the two idle ones that fill their warpgroup
     if (warp == 0) {
         // ---------------- TMA producer ----------------
         // One elected lane runs the whole loop: it arms the barrier and issues the boxes of each k-block.
@@ -1043,18 +1097,18 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             }
         }
         __syncwarp();
-    } else if (warp < 6) {
+    }
+    } else if (warp < (BW ? 8 : DWARP)) {
         // ---------------- operand transform: a = hi + lo ----------------
         // hi = a with the low 13 mantissa bits cleared (what the tensor core reads of a float32 anyway),
         // lo = a - hi (exact).  Each thread owns one row of the A tile: it reads the row's 32 k-values from the
         // shared-memory tile and writes hi and lo into the stage's tensor-memory slot, from where the MMAs take
-        // the A operand, so the A tile costs one shared-memory read in total.  In WGRAD the B tile (dy) is split
-        // in shared memory as well (only lo is written: the raw tile serves as hi).
+        // the A operand, so the A tile costs one shared-memory read in total.
+        if (BW) regs_dec<TC_REGS_SPLIT>();
         const int quad = warp & 3;                   // TMEM lane quadrant this warp may write
         const int row = quad * 32 + lane;            // A-tile row (GEMM M index inside the tile)
-        constexpr bool SPLIT_B = MODE == TCM_WGRAD || BSRC != TCB_SPLIT;    // the lo half of B is made here
-        constexpr int B_VEC = SPLIT_B ? L::B_BYTES / 16 / 128 : 0;
-        const int t = threadIdx.x - 64;              // 0..127
+        constexpr bool SPLIT_B = !BW && RESKB == 0 && (MODE == TCM_WGRAD || BSRC != TCB_SPLIT);      // this role also splits the B tile
+        const int t = threadIdx.x - XWARP * 32;      // 0..127
         Ring<STAGES> ring;
         Ring<TSLOTS> slots;                          // the stages' own A slots, or (resident filters) a separate ring
         bool ok = true;
@@ -1079,12 +1133,6 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         w.init(total_tiles, p.kblocks, MODE == TCM_FWD && !SK && !MULTI && RESKB == 0 ? p.kper : 0, p.f_plane);
         while (ok && w.template next<SK>()) {
             if (MULTI) w.kb_e = tile_geo(w.tile).kblocks;
-            // WGRAD: the tiles of the first row block also sum their dy tile over the pixels (the bias gradient);
-            // a thread meets the same four channels of each 32-channel box in every k-block (see below)
-            float4 dbacc[B_VEC / 2 + 1];
-            const bool do_db = MODE == TCM_WGRAD && p.db_partial != nullptr && (p.f_nt.div(w.tile) - p.f_plane.div(w.tile) * mt) == 0;
-#pragma unroll
-            for (int i = 0; i < B_VEC / 2; i++) dbacc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
             for (int kb = w.kb_b; kb < w.kb_e; kb++, ring.next(), slots.next()) {
                 const int s = ring.s, ts = slots.s;
                 TC_PROF_T0();
@@ -1117,13 +1165,6 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                     else if (p.a_box_log2 == 6) column(std::integral_constant<int, 64>{});
                     else column(std::integral_constant<int, 32>{});
                 }
-                // all reads of the stage first, so that the B tile's latency is under the A tile's
-                float4 bq[SPLIT_B && RESKB == 0 ? B_VEC : 1];
-                if (SPLIT_B && RESKB == 0) {
-                    const float4* b_hi = (const float4*)(st + L::A_BYTES);
-#pragma unroll
-                    for (int i = 0; i < B_VEC; i++) bq[i] = b_hi[t + i * 128];
-                }
                 const uint32_t slot = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(L::TMEM_A_COL + ts * 64);
                 uint32_t low[32];
                 float largest = 0.f;
@@ -1150,36 +1191,40 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                     if (lane == 0) mbar_arrive(&afree_bar[s]);
                 }
                 tmem_st_32x32(slot + 32, low);
-                if (SPLIT_B && RESKB == 0) {
-                    float4* b_lo = (float4*)(smem + s * L::STAGE_BYTES + L::A_BYTES + L::B_BYTES);
-                    if (FINE || (MODE == TCM_FWD && p.b_round)) {
-                        float4* b_hi = (float4*)(smem + s * L::STAGE_BYTES + L::A_BYTES);
-                        float largest = 0.f;
-#pragma unroll
-                        for (int i = 0; i < B_VEC; i++)
-                            largest = fmaxf(largest, fmaxf(fmaxf(fabsf(bq[i].x), fabsf(bq[i].y)), fmaxf(fabsf(bq[i].z), fabsf(bq[i].w))));
-                        if (!tc_rounds_to_inf(largest)) {
-#pragma unroll
-                            for (int i = 0; i < B_VEC; i++) { b_lo[t + i * 128] = tc_split_rounded<false>(bq[i]); b_hi[t + i * 128] = bq[i]; }
-                        } else {
-#pragma unroll
-                            for (int i = 0; i < B_VEC; i++) { b_lo[t + i * 128] = tc_split_rounded<true>(bq[i]); b_hi[t + i * 128] = bq[i]; }
-                        }
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < B_VEC; i++) {
-                            const float4 q = bq[i];
-                            if (do_db) { dbacc[i >> 1].x += q.x; dbacc[i >> 1].y += q.y; dbacc[i >> 1].z += q.z; dbacc[i >> 1].w += q.w; }
-                            b_lo[t + i * 128] = tc_lo_of_truncated(q);
-                        }
-                    }
-                    fence_proxy_async();
-                }
+                if (SPLIT_B) split_b(s, t, false, nullptr);
                 tmem_st_wait();
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&xform_bar[ts]);
                 if (t == 0) TC_PROF_ADD(6);    // transform: work
+            }
+        }
+    } else if (BW && warp < DWARP) {
+        // ---------------- B tile transform ----------------
+        regs_dec<TC_REGS_SPLIT>();
+        const int t = threadIdx.x - 256;             // 0..127
+        constexpr int BOXES = L::B_BYTES / 4096;
+        Ring<STAGES> ring;
+        bool ok = true;
+        TileWalk w;
+        w.init(total_tiles, p.kblocks, MODE == TCM_FWD && !SK && !MULTI ? p.kper : 0, p.f_plane);
+        while (ok && w.template next<SK>()) {
+            if (MULTI) w.kb_e = tile_geo(w.tile).kblocks;
+            // WGRAD: the tiles of the first row block also sum their dy tile over the pixels (the bias gradient);
+            // a thread meets the same four channels of each 32-channel box in every k-block (see below)
+            float4 dbacc[BOXES];
+            const bool do_db = MODE == TCM_WGRAD && p.db_partial != nullptr && (p.f_nt.div(w.tile) - p.f_plane.div(w.tile) * mt) == 0;
+#pragma unroll
+            for (int i = 0; i < BOXES; i++) dbacc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int kb = w.kb_b; kb < w.kb_e; kb++, ring.next()) {
+                const int s = ring.s;
+                if (!mbar_wait(&full_bar[s], ring.phase, abort_flag, &g_tc_status, TC_ERR_FULL)) { ok = false; break; }
+#ifdef B2C_TC_DEV
+                if (!(p.dbg & 4))
+#endif
+                split_b(s, t, do_db, dbacc);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&xform_bar[s]);
             }
             if (MODE == TCM_WGRAD && do_db && ok) {
                 // Float4 number t + 128 i of the B region is box i/2, pixel row t/8 + 16 (i & 1), 16-byte chunk t & 7.
@@ -1189,7 +1234,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 // (rr = 0: chunk = c) hold the warp's sums over its 8 pixel rows of every k-block.
                 const int z = p.f_plane.div(w.tile), ni = w.tile - p.f_nt.div(w.tile) * nt;
 #pragma unroll
-                for (int bx = 0; bx < B_VEC / 2; bx++) {
+                for (int bx = 0; bx < BOXES; bx++) {
                     float4 v = dbacc[bx];
 #pragma unroll
                     for (int m = 1; m <= 2; m <<= 1) {
@@ -1199,7 +1244,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                     }
                     const int n = ni * BN + bx * 32;
                     if (lane < 8 && n + lane * 4 < p.N)
-                        *reinterpret_cast<float4*>(p.db_partial + ((size_t)z * 4 + (warp - 2)) * p.Np + n + lane * 4) = v;
+                        *reinterpret_cast<float4*>(p.db_partial + ((size_t)z * 4 + (warp & 3)) * p.Np + n + lane * 4) = v;
                 }
             }
         }
@@ -1208,12 +1253,13 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         // Each chunk of TC_CHUNK k-blocks is accumulated in tensor memory from zero and added here in
         // float32 round-to-nearest; the tensor core's own accumulate step truncates, and its bias
         // grows with the number of accumulations, so it is kept to one chunk.
+        if (BW) regs_inc<TC_REGS_DRAIN>();
         const int quad = warp & 3;                       // TMEM lane quadrant this warp may read
         bool ok = true;
         int gc = 0, ecount = 0;
         // column slabs of a tile this warp sends out: all BN / 32, or its half of them with eight drain warps
         constexpr int NSLAB = BN / 32 / (DW / 4);
-        const int cbeg = ((warp - 6) >> 2) * NSLAB;
+        const int cbeg = ((warp - DWARP) >> 2) * NSLAB;
         float cs0[NSLAB], cs1[NSLAB];                    // batch statistics summed over this CTA's tiles (stats_cta)
 #pragma unroll
         for (int i = 0; i < NSLAB; i++) cs0[i] = cs1[i] = 0.f;
@@ -1229,16 +1275,16 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             // 128B-swizzled slab (conflict-free float4 writes), TMA store (whole rows, asynchronous, rows >= M and
             // columns >= N clipped; SLABS slabs per warp rotate so the warp never waits on HBM), and the slab's batch
             // statistics when asked for.
-            uint8_t* ebuf = smem + L::EPI_OFFSET + (warp - 6) * (SLABS * 4096);
+            uint8_t* ebuf = smem + L::EPI_OFFSET + (warp - DWARP) * (SLABS * 4096);
             float st0[NSLAB], st1[NSLAB];                               // batch statistics of the tile's slabs
             TC_PROF_T0();
             auto emit_slab = [&](float* a, int cc, int i) {      // slab cc of the tile, number i of this warp's slabs
                 uint8_t* buf = ebuf + (ecount % SLABS) * 4096;
                 if (MODE == TCM_FWD && p.epi) tc_epilogue_math(p, n0 + cc * 32, a);
-                if (threadIdx.x == 192) TC_PROF_ADD(8);     // drain: tensor-memory loads, adds, epilogue arithmetic
+                if (threadIdx.x == DWARP * 32) TC_PROF_ADD(8);     // drain: tensor-memory loads, adds, epilogue arithmetic
                 if (lane == 0) tma_store_wait_read<SLABS - 1>();     // the store that last read this slab is done
                 __syncwarp();
-                if (threadIdx.x == 192) TC_PROF_ADD(10);    // drain: waiting for a free staging slab
+                if (threadIdx.x == DWARP * 32) TC_PROF_ADD(10);    // drain: waiting for a free staging slab
 #pragma unroll
                 for (int j = 0; j < 32; j += 4)
                     *reinterpret_cast<float4*>(buf + lane * 128 + ((((j >> 2) ^ (lane & 7))) << 4)) = make_float4(a[j], a[j + 1], a[j + 2], a[j + 3]);
@@ -1249,7 +1295,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                     else tma_store_3d(&tmap_out, buf, n0 + cc * 32, m0 + quad * 32, z);
                     tma_store_commit();
                 }
-                if (threadIdx.x == 192) TC_PROF_ADD(9);     // drain: staging writes, fence, store issue
+                if (threadIdx.x == DWARP * 32) TC_PROF_ADD(9);     // drain: staging writes, fence, store issue
                 if (MODE == TCM_FWD && p.stats) {
                     // Column sums of the slab over the rows that exist, read back from the staging slab: lane
                     // (rg = lane / 8, c4 = lane % 8) takes columns 4 c4 .. 4 c4 + 3 of rows rg, rg + 4, .. (one float4 each:
@@ -1283,7 +1329,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                     float s0 = odd ? k1 : k0, e0 = odd ? k0 : k1, s1 = odd ? m1s : m0s, e1 = odd ? m0s : m1s;
                     s0 += __shfl_xor_sync(0xffffffffu, e0, 8); s1 += __shfl_xor_sync(0xffffffffu, e1, 8);
                     st0[i] = s0; st1[i] = s1;
-                    if (threadIdx.x == 192) TC_PROF_ADD(11);    // drain: batch statistics
+                    if (threadIdx.x == DWARP * 32) TC_PROF_ADD(11);    // drain: batch statistics
                 }
                 ecount++;
             };
@@ -1309,7 +1355,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 const int b = gc & 1;
                 TC_PROF_RESET();
                 ok = mbar_wait(&tfull_bar[b], (gc >> 1) & 1, abort_flag, &g_tc_status, TC_ERR_TFULL);
-                if (threadIdx.x == 192) TC_PROF_ADD(7);
+                if (threadIdx.x == DWARP * 32) TC_PROF_ADD(7);
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t tsrc = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(b * BN);
@@ -1337,7 +1383,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 const int b = gc & 1;
                 TC_PROF_RESET();
                 ok = mbar_wait(&tfull_bar[b], (gc >> 1) & 1, abort_flag, &g_tc_status, TC_ERR_TFULL);
-                if (threadIdx.x == 192) TC_PROF_ADD(7);    // drain: waiting for a finished chunk
+                if (threadIdx.x == DWARP * 32) TC_PROF_ADD(7);    // drain: waiting for a finished chunk
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t tsrc = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(b * BN);
@@ -1359,7 +1405,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&tempty_bar[b]);
-                if (threadIdx.x == 192) TC_PROF_ADD(8);    // drain: TMEM load + add
+                if (threadIdx.x == DWARP * 32) TC_PROF_ADD(8);    // drain: TMEM load + add
             }
             if (SK && ok) {
                 const int row = quad * 32 + lane;
@@ -1431,7 +1477,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                     if (n0 + cc * 32 < p.N && m0 + quad * 32 < p.M) emit_slab(&acc[cc * 32], cc, cc);     // slabs wholly outside the output are skipped
                 store_stats();
             } else if (ok) {
-                float* stage = (float*)(smem + L::EPI_OFFSET) + (warp - 6) * (SLABS * 4096 / 4);
+                float* stage = (float*)(smem + L::EPI_OFFSET) + (warp - DWARP) * (SLABS * 4096 / 4);
 #pragma unroll
                 for (int cc = 0; cc < BN / 32; cc++) {
                     if (n0 + cc * 32 < p.N) {
@@ -1461,7 +1507,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                     }
                 }
             }
-            if (threadIdx.x == 192) TC_PROF_ADD(9);        // drain: epilogue
+            if (threadIdx.x == DWARP * 32) TC_PROF_ADD(9);        // drain: epilogue
             }   // chunked drain
         }
         if (MODE == TCM_FWD && !SK && !MULTI && p.stats && p.stats_cta && ok) {
@@ -1978,7 +2024,16 @@ static int launch_tc(const CUtensorMap& ma, const CUtensorMap& mb0, const CUtens
     using L = TcSmem<BN, STAGES, SLABS, tc_drain_warps<STREAM>(), RESKB>;
     static PerDeviceOnce attr;
     {
-        cudaError_t e = attr.run([] { return cudaFuncSetAttribute(conv_tc_kernel<MODE, BN, STAGES, SK, SLABS, BSRC, STREAM, MULTI, RESKB, FINE>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL); });
+        cudaError_t e = attr.run([] {
+            const auto kernel = conv_tc_kernel<MODE, BN, STAGES, SK, SLABS, BSRC, STREAM, MULTI, RESKB, FINE>;
+            if (tc_b_warps<MODE, BSRC, STREAM, RESKB>()) {       // the roles' shares must add up to what the launch brings
+                cudaFuncAttributes a;
+                const cudaError_t r = cudaFuncGetAttributes(&a, kernel);
+                if (r != cudaSuccess) return r;
+                if (a.numRegs != TC_REGS_LAUNCH) return cudaErrorLaunchOutOfResources;
+            }
+            return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
+        });
         if (e != cudaSuccess) { set_cuda_error(e, "cudaFuncSetAttribute(conv_tc_kernel)"); return B2C_ERR_CUDA; }
     }
     const int sm_count = tc_sm_count();
@@ -1994,7 +2049,7 @@ static int launch_tc(const CUtensorMap& ma, const CUtensorMap& mb0, const CUtens
 #endif
     int grid = q.sk ? sm_count : (int)(tiles < sm_count ? tiles : sm_count);     // one persistent CTA per SM
     if ((q.stats && q.stats_cta) || RESKB) grid -= grid % ((p.N + BN - 1) / BN);    // a CTA keeps its column tile
-    launch_pdl(conv_tc_kernel<MODE, BN, STAGES, SK, SLABS, BSRC, STREAM, MULTI, RESKB, FINE>, grid, tc_threads<STREAM>(), L::TOTAL, st, ma, mb0, mb1, mo, ma3 ? *ma3 : ma, q);
+    launch_pdl(conv_tc_kernel<MODE, BN, STAGES, SK, SLABS, BSRC, STREAM, MULTI, RESKB, FINE>, grid, tc_threads<MODE, BSRC, STREAM, RESKB>(), L::TOTAL, st, ma, mb0, mb1, mo, ma3 ? *ma3 : ma, q);
     return check_launch("conv_tc_kernel");
 }
 
