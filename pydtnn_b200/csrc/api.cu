@@ -211,9 +211,16 @@ extern "C" int b2c_fc_forward(int dtype, int engine, int batch, int in_f, int ou
     Geo g; int rc = fc_geo(dtype, engine, batch, in_f, out_f, g); if (rc) return rc;
     if (!x || !w || !y) return B2C_ERR_NULL_POINTER;
     if (engine == B2C_ENGINE_AUTO && fc_tiny(batch, in_f, out_f)) return fc_tiny_forward(dtype, batch, in_f, out_f, x, w, bias, y, (cudaStream_t)stream);
+    // The one-launch forms need neither workspace nor alignment; a call with less of either than the other forms ask for is left to them.
+    int e;
+    if (fc_mma_takes(dtype, engine, batch, in_f, out_f, false) && ws && ws_bytes >= pass_workspace_bytes(g, B2C_PASS_FPROP) &&
+        call_engine(g, B2C_PASS_FPROP, x, y, e) == B2C_OK &&
+        !(tc_fc_small_batch(dtype, engine, batch, in_f, out_f) &&
+          ((((uintptr_t)x | (uintptr_t)w | (uintptr_t)y | (uintptr_t)bias) & 15) || ws_bytes < tc_fc_small_batch_bytes(batch, in_f, out_f))))
+        return fc_mma_forward(batch, in_f, out_f, x, w, bias, y, (cudaStream_t)stream);
     if (tc_fc_small_batch(dtype, engine, batch, in_f, out_f))
         return tc_fc_forward_small_batch(batch, in_f, out_f, x, w, bias, y, ws, ws_bytes, (cudaStream_t)stream);
-    int e; rc = call_engine(g, B2C_PASS_FPROP, x, y, e); if (rc) return rc;
+    rc = call_engine(g, B2C_PASS_FPROP, x, y, e); if (rc) return rc;
     if (e == B2C_ENGINE_TENSOR) return tc_fprop(g, x, w, bias, nullptr, 0, y, ws, ws_bytes, (cudaStream_t)stream);
     return fma_fprop(g, x, w, bias, nullptr, 0, y, ws, ws_bytes, (cudaStream_t)stream);
 }
@@ -227,6 +234,13 @@ extern "C" int b2c_fc_backward(int dtype, int engine, int batch, int in_f, int o
         if ((dw && !x) || (dx && !w)) return B2C_ERR_NULL_POINTER;
         return fc_tiny_backward(dtype, batch, in_f, out_f, x, dy, w, dw, db, dx, st);
     }
+    int engine_of;
+    if (fc_mma_takes(dtype, engine, batch, in_f, out_f, true) && (dw || (dx && !db)) && (!dw || x) && (!dx || w) && ws &&
+        (!dw || ws_bytes >= pass_workspace_bytes(g, B2C_PASS_WGRAD)) && (!dx || ws_bytes >= pass_workspace_bytes(g, B2C_PASS_DGRAD)) &&
+        (!dw || call_engine(g, B2C_PASS_WGRAD, x, dy, engine_of) == B2C_OK) && (!dx || call_engine(g, B2C_PASS_DGRAD, dx, dy, engine_of) == B2C_OK) &&
+        !(tc_fc_small_batch(dtype, engine, batch, in_f, out_f) &&
+          ((((uintptr_t)x | (uintptr_t)dy | (uintptr_t)w | (uintptr_t)dw | (uintptr_t)dx) & 15) || ws_bytes < tc_fc_small_batch_bytes(batch, in_f, out_f))))
+        return fc_mma_backward(batch, in_f, out_f, x, dy, w, dw, db, dx, st);
     if (tc_fc_small_batch(dtype, engine, batch, in_f, out_f)) {
         if (dw) {
             if (!x) return B2C_ERR_NULL_POINTER;

@@ -113,6 +113,11 @@ int fc_tiny_forward(int dtype, int batch, int in_f, int out_f, const void* x, co
 int fc_tiny_backward(int dtype, int batch, int in_f, int out_f, const void* x, const void* dy, const void* w, void* dw, void* db, void* dx, cudaStream_t st);
 int channel_sum_v4(int n, int c, int hw, const void* src, void* dst, void* ws, size_t ws_bytes, cudaStream_t st);
 
+// fully connected layers of float32 in one launch a direction (fc_mma.cu)
+bool fc_mma_takes(int dtype, int engine, int batch, int in_f, int out_f, bool backward);
+int fc_mma_forward(int batch, int in_f, int out_f, const void* x, const void* w, const void* bias, void* y, cudaStream_t st);
+int fc_mma_backward(int batch, int in_f, int out_f, const void* x, const void* dy, const void* w, void* dw, void* db, void* dx, cudaStream_t st);
+
 // tensor-core engine (conv_tc.cu)
 bool tc_supported(const Geo& g, int pass);
 int tc_sm_count();      // of the current device

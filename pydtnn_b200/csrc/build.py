@@ -17,7 +17,7 @@ import sys
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 PKG = os.path.dirname(HERE)
-SOURCES = ["api.cu", "conv_fma.cu", "conv_tc.cu", "aux_ops.cu"]
+SOURCES = ["api.cu", "conv_fma.cu", "conv_tc.cu", "fc_mma.cu", "aux_ops.cu"]
 OUT = os.path.join(PKG, "libb2c.so")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",

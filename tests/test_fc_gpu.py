@@ -68,3 +68,38 @@ def test_bias_gradient_of_wide_layers_with_many_rows(n, i, o):
     X, D, W = (a.cpu().numpy().astype(np.float64) for a in (x, dy, w))
     for got, ref, what in ((dw, X.T @ D, "dw"), (db, D.sum(0), "db"), (dx, D @ W.T, "dx")):
         assert_parity(got.cpu().numpy(), ref, np.float32, what)
+
+
+@pytest.mark.parametrize("n,i,o", [(1, 2048, 1000), (16, 256, 257), (17, 65, 260), (32, 1568, 128), (47, 640, 64), (48, 640, 47), (49, 201, 131), (64, 1568, 128),
+                                   (65, 320, 100), (128, 320, 48), (250, 100, 203)])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_passes_in_one_launch(n, i, o, shift):
+    """Edges of the row tiles (16, 32, 64), of the steps of 32 products and of the sums in plain FMAs (47, 48), shares of a K loop
+    without any product, filters on any alignment, an infinity and its row."""
+    L = _lib.lib()
+    g = torch.Generator(device=DEV).manual_seed(n + i + o)
+
+    def buf(s, off):
+        return torch.full((int(np.prod(s)) + off,), float("nan"), device=DEV)[off:].view(s)
+    x, dy, y, dx = (buf(s, 0) for s in ((n, i), (n, o), (n, o), (n, i)))
+    w, b, dw, db = (buf(s, shift) for s in ((i, o), (o,), (i, o), (o,)))
+    for t in (x, w, b, dy):
+        t.copy_(torch.randn(t.shape, device=DEV, generator=g))
+    ws = torch.empty(max(256, L.b2c_fc_workspace_bytes(0, n, i, o, 0)), dtype=torch.uint8, device=DEV)
+
+    def run():
+        _lib.check(L.b2c_fc_forward(0, 0, n, i, o, x.data_ptr(), w.data_ptr(), b.data_ptr(), y.data_ptr(), ws.data_ptr(), ws.numel(), stream()))
+        _lib.check(L.b2c_fc_backward(0, 0, n, i, o, x.data_ptr(), dy.data_ptr(), w.data_ptr(), dw.data_ptr(), db.data_ptr(), dx.data_ptr(),
+                                     ws.data_ptr(), ws.numel(), stream()))
+    run()
+    X, W, B, D = (t.double() for t in (x, w, b, dy))
+    for got, ref in ((y, X @ W + B), (dw, X.T @ D), (db, D.sum(0)), (dx, D @ W.T)):
+        # float32 sums of up to 2048 random terms: 2^-24 each, growing with the root of their number at most
+        assert float((got.double() - ref).norm() / ref.norm()) <= 3e-7
+    first = [t.clone() for t in (y, dw, db, dx)]
+    run()
+    assert all(torch.equal(a, t) for a, t in zip(first, (y, dw, db, dx)))
+    x[0, i - 1] = float("inf")
+    run()
+    assert torch.equal(y[0], torch.where(w[i - 1] > 0, float("inf"), float("-inf")))
+    assert bool(torch.isfinite(y[1:]).all()) and bool(torch.isfinite(dw[: i - 1]).all())
