@@ -36,6 +36,7 @@ struct IgemmParams {
     int64_t c_sn;                 // C(m, n) = Cdst[rowinfo.b_off + n*c_sn]
     int a_lanes_k, b_lanes_k;     // which index runs fastest across lanes when loading A / B
     int k_chunk, splits;
+    int whole, m_whole;           // float64: tiles, and the rows they cover, that take no part in the split
     int relu;
     // Sub-lattices (strided dgrad runs one launch per residue class of the output pixels, each with the taps that
     // reach it): pixel (pp, qq) of the grid is row pix_h0 + pp*pix_hs, column pix_w0 + qq*pix_ws of the tensor;
@@ -325,7 +326,9 @@ __device__ __forceinline__ void bar_arrive(int id, int n) {
 }
 
 // AK, BK_: the tile of A (B) is contiguous along k, else along its other index.  V doubles per copy.  OFF: offsets in A, B, C.
-template <int BN, bool AK, bool BK_, int V, typename OFF>
+// TAIL: only the tiles past whole rounds of the chip are split (split_last_round_f64).  A form of its own: with its index arithmetic
+// in the launches of a few microseconds a small float64 network took 755 us a step for 697.
+template <int BN, bool AK, bool BK_, int V, typename OFF, bool TAIL>
 __global__ void __launch_bounds__(DG_THREADS, 1)
 dgemm_kernel(IgemmParams p, int mode, const double* __restrict__ A, const double* __restrict__ B,
              double* __restrict__ C, double* __restrict__ partial, Epilogue<double> ep)
@@ -340,8 +343,19 @@ dgemm_kernel(IgemmParams p, int mode, const double* __restrict__ A, const double
     DInfo<OFF>* kinfo = reinterpret_cast<DInfo<OFF>*>(dg_smem + DG_STAGES * TILE * sizeof(double));
     DInfo<OFF>* rowinfo = kinfo + DG_STAGES * BK;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
-    const int kbeg = blockIdx.z * p.k_chunk, kend = min(p.K, kbeg + p.k_chunk);
+    int m_tile = blockIdx.x, n_tile = blockIdx.y, z = blockIdx.z;
+    bool split = p.splits > 1;
+    if constexpr (TAIL) {
+        // one row of blocks over the tiles in row order, column tiles fastest: the first p.whole tiles are one block's, of the
+        // others a block takes one of p.splits shares of the K loop
+        const int nt = (p.N + BN - 1) / BN, rest = (p.M + BM - 1) / BM * nt - p.whole;
+        split = m_tile >= p.whole;
+        z = split ? (m_tile - p.whole) / rest : 0;
+        const int tile = m_tile - z * rest;
+        m_tile = tile / nt; n_tile = tile - m_tile * nt;
+    }
+    const int m0 = m_tile * BM, n0 = n_tile * BN;
+    const int kbeg = z * p.k_chunk, kend = TAIL && !split ? p.K : min(p.K, kbeg + p.k_chunk);
     const int nslice = (kend - kbeg + BK - 1) / BK;
     if (tid < BM) rowinfo[tid] = mode == MODE_WGRAD ? dinfo_tap<OFF>(p, mode, m0 + tid, p.M) : dinfo_pix<OFF>(p, mode, m0 + tid, p.M);
     __syncthreads();
@@ -462,7 +476,8 @@ dgemm_kernel(IgemmParams p, int mode, const double* __restrict__ A, const double
                     const int n = n0 + wn + j * 8 + 2 * t + e;
                     if (n >= p.N) continue;
                     const double v = acc[i][j][2 * h + e];
-                    if (p.splits > 1) partial[((int64_t)blockIdx.z * p.M + m) * p.N + n] = v;
+                    if (TAIL && split) partial[((int64_t)z * (p.M - p.m_whole) + m - p.m_whole) * p.N + n] = v;
+                    else if (!TAIL && p.splits > 1) partial[((int64_t)blockIdx.z * p.M + m) * p.N + n] = v;
                     else C[row_off + (int64_t)n * p.c_sn] = apply_epilogue<double>(v, n, ep);
                 }
         }
@@ -477,7 +492,7 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(IgemmParams p, const
     pdl_prologue();
     constexpr int COLS = 256 / ROWS;
     __shared__ T part[ROWS][COLS];
-    const int64_t idx = (int64_t)blockIdx.x * COLS + threadIdx.x, total = (int64_t)p.M * p.N;
+    const int64_t idx = (int64_t)blockIdx.x * COLS + threadIdx.x, total = (int64_t)(p.M - p.m_whole) * p.N;
     T v = T(0);
     if (idx < total) {
         int z = threadIdx.y;
@@ -498,7 +513,7 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(IgemmParams p, const
         for (int y = 1; y < ROWS; y++) v += part[y][threadIdx.x];
     }
     if (idx >= total) return;
-    const int m = (int)(idx / p.N), n = (int)(idx - (int64_t)m * p.N);
+    const int row = (int)(idx / p.N), n = (int)(idx - (int64_t)row * p.N), m = p.m_whole + row;
     const Info ri = (MODE == MODE_WGRAD) ? decode_tap<MODE>(p, m, p.M) : decode_pix<MODE>(p, m, p.M);
     C[ri.b_off + (int64_t)n * p.c_sn] = apply_epilogue<T>(v, n, ep);
 }
@@ -790,6 +805,26 @@ static int choose_splits_f64(const IgemmParams& p, int bk)
     return (int)best;
 }
 
+// More than one round of whole float64 tiles: the 392 of a 28x28 256->256 3x3 layer, batch 32, are 2.65 rounds on 148 SMs that ran as
+// three.  Row tiles that fill whole rounds stay whole, the K loops of the others are split so that they fill the chip too (that
+// layer, three passes: 3168 -> 2987 us).  Where that saves a thirtieth or more; costs as in choose_splits_f64.
+static void split_last_round_f64(IgemmParams& p, int bk)
+{
+    const int64_t nt = (p.N + tile_bn(p.N) - 1) / tile_bn(p.N), ctas = (int64_t)((p.M + 127) / 128) * nt, room = tc_sm_count(), slices = (p.K + bk - 1) / bk;
+    const int64_t rows = ctas / room * room / nt, whole = rows * nt, rest = ctas - whole;         // row tiles that fill whole rounds
+    if (ctas <= room || !rows || !rest) return;
+    const int64_t before = (ctas + room - 1) / room * (slices + 3);
+    int64_t best = 1, cost = before - before / 30;
+    for (int64_t s = 2; s <= 16 && s <= slices; s++) {
+        const int64_t c = (whole + room - 1) / room * (slices + 3) + (rest * s + room - 1) / room * ((slices + s - 1) / s + 6);
+        if (c < cost) { best = s; cost = c; }
+    }
+    if (best == 1) return;
+    p.k_chunk = (int)(((slices + best - 1) / best) * bk);
+    p.splits = (p.K + p.k_chunk - 1) / p.k_chunk;
+    p.whole = (int)whole; p.m_whole = (int)(rows * 128);
+}
+
 static void finish_params(IgemmParams& p, int dtype)
 {
     const int bk = 16;
@@ -800,7 +835,10 @@ static void finish_params(IgemmParams& p, int dtype)
     chunk = (chunk + bk - 1) / bk * bk;
     p.k_chunk = chunk;
     p.splits = (p.K + chunk - 1) / chunk;
+    p.whole = p.m_whole = 0;
+    if (p.splits == 1 && dtype != B2C_F32) split_last_round_f64(p, bk);
 }
+static size_t partial_bytes(const IgemmParams& p, size_t es) { return p.splits > 1 ? (size_t)p.splits * (p.M - p.m_whole) * p.N * es : 0; }
 
 // Strided dgrad: input pixel (h, w) only receives taps with r * vdil = h + vpad, s * hdil = w + hpad (mod the strides).
 // Class (a, b) of those residues is a dense problem over its own pixels and taps; gathering all taps for all pixels instead
@@ -843,19 +881,19 @@ size_t fma_workspace_bytes(const Geo& g, int pass)
                 IgemmParams p = dgrad_class_params(g, a, b);
                 if (p.M == 0) continue;
                 finish_params(p, g.dtype);
-                size_t bytes = p.splits > 1 ? (size_t)p.splits * p.M * p.N * es : 0;
+                size_t bytes = partial_bytes(p, es);
                 if (bytes > most) most = bytes;
             }
         return most;
     }
     IgemmParams p = make_params(g, pass);
     finish_params(p, g.dtype);
-    size_t bytes = p.splits > 1 ? (size_t)p.splits * p.M * p.N * es : 0;
+    size_t bytes = partial_bytes(p, es);
     if (pass == B2C_PASS_WGRAD) bytes = align_up(bytes, 256) + channel_sum_workspace_bytes(g.n, g.co, g.ho * g.wo);
     return bytes;
 }
 
-template <int BN, bool AK, bool BK_, int V, typename OFF>
+template <int BN, bool AK, bool BK_, int V, typename OFF, bool TAIL = false>
 static int launch_dgemm_v(const IgemmParams& p, int mode, dim3 grid, const double* A, const double* B, double* C, double* ws, const Epilogue<double>& ep, cudaStream_t st)
 {
     // once per device: the attribute belongs to the device's copy of the kernel
@@ -863,11 +901,11 @@ static int launch_dgemm_v(const IgemmParams& p, int mode, dim3 grid, const doubl
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev > 63) dev = 63;
     if (dev == 63 || !(done.load() >> dev & 1)) {
-        const cudaError_t e = cudaFuncSetAttribute(dgemm_kernel<BN, AK, BK_, V, OFF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dg_smem_bytes<BN, OFF>());
+        const cudaError_t e = cudaFuncSetAttribute(dgemm_kernel<BN, AK, BK_, V, OFF, TAIL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dg_smem_bytes<BN, OFF>());
         if (e != cudaSuccess) { set_cuda_error(e, "cudaFuncSetAttribute(dgemm_kernel)"); return B2C_ERR_CUDA; }
         done.fetch_or(1ull << dev);
     }
-    launch_pdl(dgemm_kernel<BN, AK, BK_, V, OFF>, grid, DG_THREADS, dg_smem_bytes<BN, OFF>(), st, p, mode, A, B, C, ws, ep);
+    launch_pdl(dgemm_kernel<BN, AK, BK_, V, OFF, TAIL>, grid, DG_THREADS, dg_smem_bytes<BN, OFF>(), st, p, mode, A, B, C, ws, ep);
     return B2C_OK;          // the caller checks the launch
 }
 
@@ -883,12 +921,14 @@ static int launch_dgemm(const IgemmParams& p, int mode, dim3 grid, const double*
     else b_pair = b_pair && p.b_sn == 1 && p.N % 2 == 0 &&
                   ((mode == MODE_WGRAD ? (p.pb_sn | p.pb_sh | p.pb_sw) : (p.tb_sc | p.tb_sr | p.tb_ss)) & 1) == 0;
     const bool pairs = a_pair && b_pair && p.small;         // small: every offset fits 31 bits
-#define B2C_DG(AK, BK_) (pairs ? launch_dgemm_v<BN, AK, BK_, 2, int>(p, mode, grid, A, B, C, ws, ep, st) : launch_dgemm_v<BN, AK, BK_, 1, int64_t>(p, mode, grid, A, B, C, ws, ep, st))
+#define B2C_DG(AK, BK_) (p.whole ? (pairs ? launch_dgemm_v<BN, AK, BK_, 2, int, true>(p, mode, grid, A, B, C, ws, ep, st) : launch_dgemm_v<BN, AK, BK_, 1, int64_t, true>(p, mode, grid, A, B, C, ws, ep, st)) \
+                         : pairs ? launch_dgemm_v<BN, AK, BK_, 2, int>(p, mode, grid, A, B, C, ws, ep, st) : launch_dgemm_v<BN, AK, BK_, 1, int64_t>(p, mode, grid, A, B, C, ws, ep, st))
     if (p.a_lanes_k && p.b_lanes_k) return B2C_DG(true, true);
     if (p.a_lanes_k) return B2C_DG(true, false);
     if (!p.b_lanes_k) return B2C_DG(false, false);
 #undef B2C_DG
-    return launch_dgemm_v<BN, false, true, 1, int64_t>(p, mode, grid, A, B, C, ws, ep, st);
+    return p.whole ? launch_dgemm_v<BN, false, true, 1, int64_t, true>(p, mode, grid, A, B, C, ws, ep, st)
+                   : launch_dgemm_v<BN, false, true, 1, int64_t>(p, mode, grid, A, B, C, ws, ep, st);
 }
 
 template <typename T, int MODE>
@@ -896,12 +936,18 @@ static int launch_igemm(IgemmParams& p, const void* A, const void* B, void* C, v
                         Epilogue<T> ep, cudaStream_t st)
 {
     finish_params(p, sizeof(T) == 4 ? B2C_F32 : B2C_F64);
-    size_t need = p.splits > 1 ? (size_t)p.splits * p.M * p.N * sizeof(T) : 0;
+    size_t need = partial_bytes(p, sizeof(T));
+    if (p.whole && (need > ws_bytes || !ws)) { p.splits = 1; p.k_chunk = (p.K + 15) / 16 * 16; p.whole = p.m_whole = 0; need = 0; }    // whole tiles need none
     if (need > ws_bytes || (need && !ws)) return B2C_ERR_WORKSPACE_TOO_SMALL;
     const int bn = tile_bn(p.N);
     dim3 grid((p.M + 127) / 128, (p.N + bn - 1) / bn, p.splits);
     if (grid.y > 65535 || grid.z > 65535) return B2C_ERR_TOO_LARGE;
     if constexpr (sizeof(T) == 8) {
+        if (p.whole) {
+            const int64_t blocks = p.whole + ((int64_t)grid.x * grid.y - p.whole) * p.splits;
+            if (blocks > 0x7fffffffLL) return B2C_ERR_TOO_LARGE;
+            grid = dim3((unsigned)blocks);
+        }
         const int rc = bn == 64 ? launch_dgemm<64>(p, MODE, grid, (const double*)A, (const double*)B, (double*)C, (double*)ws, ep, st)
                                 : launch_dgemm<128>(p, MODE, grid, (const double*)A, (const double*)B, (double*)C, (double*)ws, ep, st);
         if (rc) return rc;
@@ -912,7 +958,7 @@ static int launch_igemm(IgemmParams& p, const void* A, const void* B, void* C, v
     int rc = check_launch("igemm_kernel");
     if (rc) return rc;
     if (p.splits > 1) {
-        int64_t total = (int64_t)p.M * p.N;
+        int64_t total = (int64_t)(p.M - p.m_whole) * p.N;
         if (p.splits >= 16) launch_pdl(splitk_reduce_kernel<T, MODE, 8>, (unsigned)((total + 31) / 32), dim3(32, 8), 0, st, p, (const T*)ws, (T*)C, ep);
         else launch_pdl(splitk_reduce_kernel<T, MODE, 1>, (unsigned)((total + 255) / 256), dim3(256, 1), 0, st, p, (const T*)ws, (T*)C, ep);
         rc = check_launch("splitk_reduce_kernel");
@@ -973,10 +1019,11 @@ int fma_wgrad(const Geo& g, const void* x, const void* dy, void* dw, void* db, v
     IgemmParams p = make_params(g, MODE_WGRAD);
     finish_params(p, g.dtype);
     size_t es = g.dtype == B2C_F32 ? 4 : 8;
-    size_t part = align_up(p.splits > 1 ? (size_t)p.splits * p.M * p.N * es : 0, 256);
+    size_t part = align_up(partial_bytes(p, es), 256), gemm_bytes = ws_bytes;
+    if (p.whole && ws_bytes < part + (db ? channel_sum_workspace_bytes(g.n, g.co, g.ho * g.wo) : 0)) part = gemm_bytes = 0;      // whole tiles only
     int rc;
-    if (g.dtype == B2C_F32) rc = launch_igemm<float, MODE_WGRAD>(p, x, dy, dw, ws, ws_bytes, Epilogue<float>{}, st);
-    else rc = launch_igemm<double, MODE_WGRAD>(p, x, dy, dw, ws, ws_bytes, Epilogue<double>{}, st);
+    if (g.dtype == B2C_F32) rc = launch_igemm<float, MODE_WGRAD>(p, x, dy, dw, ws, gemm_bytes, Epilogue<float>{}, st);
+    else rc = launch_igemm<double, MODE_WGRAD>(p, x, dy, dw, ws, gemm_bytes, Epilogue<double>{}, st);
     if (rc || !db) return rc;
     size_t cs = channel_sum_workspace_bytes(g.n, g.co, g.ho * g.wo);
     if (!ws || ws_bytes < part + cs) return B2C_ERR_WORKSPACE_TOO_SMALL;

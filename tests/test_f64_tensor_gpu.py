@@ -52,3 +52,25 @@ def test_float64_fc_on_8_byte_pointers(n, i, o):
     xs, wn, bn, dn = (t.cpu().numpy() for t in (x, w, b, dy))
     for got, ref in ((y, xs @ wn + bn), (dw, xs.T @ dn), (db, dn.sum(0)), (dx, dn @ wn.T)):
         assert_parity(got.cpu().numpy(), ref, np.float64)
+
+
+@pytest.mark.parametrize("n,h,w,ci,cout", [(3, 83, 79, 300, 40), (1, 90, 85, 200, 300), (2, 98, 97, 131, 129), (1, 20, 19, 2500, 1030)])
+@pytest.mark.parametrize("room", [True, False])
+def test_float64_last_round_of_tiles_is_split(n, h, w, ci, cout, room):
+    """More tiles than SMs: those past whole rounds share their K loops; without workspace for it they stay whole."""
+    L = _lib.lib()
+    gen = torch.Generator(device=DEV).manual_seed(ci)
+    x, f, b, dy = (torch.randn(s, dtype=torch.float64, device=DEV, generator=gen) for s in ((n * h * w, ci), (ci, cout), (cout,), (n * h * w, cout)))
+    y, df, dx = (torch.full_like(t, float("nan")) for t in (dy, f, x))
+    d = _lib.ConvDesc(_lib.LAYOUT_NHWC, _lib.F64, _lib.W_CRSK, 0, n, h, w, ci, cout, 1, 1, 0, 0, 1, 1, 1, 1)
+    need = [L.b2c_conv_workspace_bytes(d, p) for p in (_lib.PASS_FPROP, _lib.PASS_DGRAD, _lib.PASS_WGRAD)]
+    tiles = [-(-m // 128) * -(-c // (64 if c <= 64 else 128)) for m, c in ((n * h * w, cout), (n * h * w, ci), (ci, cout))]
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert any(t > sms and need[i] > 0 for i, t in enumerate(tiles))
+    ws = torch.empty(max(need), dtype=torch.uint8, device=DEV)
+    size = [ws.numel() if room or tiles[i] <= sms else 0 for i in range(3)]
+    _lib.check(L.b2c_conv_fprop(d, x.data_ptr(), f.data_ptr(), b.data_ptr(), None, 0, y.data_ptr(), ws.data_ptr(), size[0], stream()))
+    _lib.check(L.b2c_conv_dgrad(d, dy.data_ptr(), f.data_ptr(), dx.data_ptr(), ws.data_ptr(), size[1], stream()))
+    _lib.check(L.b2c_conv_wgrad(d, x.data_ptr(), dy.data_ptr(), df.data_ptr(), None, ws.data_ptr(), size[2], stream()))
+    for got, ref in ((y, x @ f + b), (dx, dy @ f.T), (df, x.T @ dy)):
+        assert_parity(got.cpu().numpy(), ref.cpu().numpy(), np.float64)
