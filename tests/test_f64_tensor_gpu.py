@@ -74,3 +74,18 @@ def test_float64_last_round_of_tiles_is_split(n, h, w, ci, cout, room):
     _lib.check(L.b2c_conv_wgrad(d, x.data_ptr(), dy.data_ptr(), df.data_ptr(), None, ws.data_ptr(), size[2], stream()))
     for got, ref in ((y, x @ f + b), (dx, dy @ f.T), (df, x.T @ dy)):
         assert_parity(got.cpu().numpy(), ref.cpu().numpy(), np.float64)
+
+
+@pytest.mark.parametrize("n,h,w,ci,cout,kh,kw,st", [(2, 13, 11, 1, 16, 3, 3, 1), (1, 16, 16, 64, 33, 1, 1, 1), (3, 17, 9, 3, 31, 4, 5, 2), (1, 23, 23, 16, 32, 2, 2, 1), (5, 8, 8, 5, 100, 3, 3, 2)])
+@pytest.mark.parametrize("layout,w_layout", [("NHWC", "KRSC"), ("NHWC", "CRSK"), ("NCHW", "KCRS")])
+def test_float32_forward_of_short_sums(n, h, w, ci, cout, kh, kw, st, layout, w_layout):
+    """Up to 64 products an output: 16, 32 and more channels, rows past the last block, padding and strides, fused ReLU."""
+    g = co.Geom(n, h, w, ci, cout, kh, kw, 1, 1, st, st, 1, 1)
+    rng = np.random.Generator(np.random.PCG64(cout))
+    nchw = layout == "NCHW"
+    x = rng.standard_normal((n, ci, h, w) if nchw else (n, h, w, ci))
+    wt = rng.standard_normal((cout, ci, kh, kw) if nchw else (ci, kh, kw, cout))
+    b = rng.standard_normal(cout)
+    y = co.conv2d_forward(x, wt, b, g, layout)
+    out = run_conv(g, layout, np.float32, x, wt, b, np.zeros(1), w_layout=w_layout, engine=_lib.ENGINE_FMA, passes=("fprop",), relu=True)
+    assert_parity(out["y"].reshape(y.shape), np.maximum(y, 0), np.float32)
