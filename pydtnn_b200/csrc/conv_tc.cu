@@ -1529,7 +1529,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
 
 // Second stage of a forward launch with a split K loop: the partial tiles of a row added in split order, the epilogue
 // steps, the store (row m = (n, i, j) at out + n * o_sn + i * o_sh + j * o_sw) and, when asked for, one row of batch sums
-// per 32 output rows.  A thread takes four channels of ROWS rows; its loads over the splits are independent, so the kernel
+// per 32 output rows.  A thread takes four channels of a row; its loads over the splits are independent, so the kernel
 // costs about one trip to L2 (the partials were just written) behind the launch: 2 to 3 us for the 2 to 10 MB it meets.
 struct FinishParams {
     int M, N, P, Q, splits, pitch;          // pitch: floats per partial row
@@ -1541,62 +1541,70 @@ struct FinishParams {
     int relu;
     float* stats;
 };
-template <int ROWS>
-__global__ void __launch_bounds__(256) tc_split_finish_kernel(FinishParams p)
+// STATS: 32 rows a block, a thread row each (with eight thread rows of four rows each the few blocks of a pass over 256 rows
+// went through one chain of loads after the other: VGG at 32 pixels, eight such launches, 1486 -> 1450 us a step).
+template <bool STATS>
+__global__ void __launch_bounds__(STATS ? 1024 : 256) tc_split_finish_kernel(FinishParams p)
 {
     pdl_prologue();
     const int lane = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const int n0 = blockIdx.x * 128 + lane * 4;
-    float4 t0 = make_float4(0.f, 0.f, 0.f, 0.f), t1 = t0;
-    if (n0 < p.N) {
+    const int n0 = blockIdx.x * 128 + lane * 4, m = blockIdx.y * (STATS ? 32 : 8) + ty;
+    float a[4] = {0.f, 0.f, 0.f, 0.f};
+    if (n0 < p.N && m < p.M) {
         const bool vec = n0 + 4 <= p.N && p.N % 4 == 0 && p.o_sw % 4 == 0;
         const int cnt = p.N - n0 < 4 ? p.N - n0 : 4;
+        const float* src = p.partial + (int64_t)m * p.pitch + n0;
+        // eight sums over every eighth split, then those in order: the order of tc_split_finish_deep_kernel
+        float4 s[8];
 #pragma unroll
-        for (int r = 0; r < ROWS; r++) {
-            const int m = (blockIdx.y * ROWS + r) * 8 + ty;
-            if (m >= p.M) continue;
-            const float* src = p.partial + (int64_t)m * p.pitch + n0;
-            // eight sums over every eighth split, then those in order: the order of tc_split_finish_deep_kernel
-            float4 s[8];
+        for (int u = 0; u < 8; u++) s[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int z = 0; z < p.splits; z += 8) {
 #pragma unroll
-            for (int u = 0; u < 8; u++) s[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int z = 0; z < p.splits; z += 8) {
-#pragma unroll
-                for (int u = 0; u < 8; u++)
-                    if (z + u < p.splits) {
-                        const float4 q = __ldcg(reinterpret_cast<const float4*>(src + (z + u) * p.plane));
-                        s[u].x += q.x; s[u].y += q.y; s[u].z += q.z; s[u].w += q.w;
-                    }
-            }
-            float4 v = s[0];
-#pragma unroll
-            for (int u = 1; u < 8; u++) { v.x += s[u].x; v.y += s[u].y; v.z += s[u].z; v.w += s[u].w; }
-            float a[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-            for (int e = 0; e < 4; e++)
-                if (e < cnt) {
-                    if (p.bias) a[e] += __ldg(p.bias + n0 + e);
-                    if (p.mean) { const float t = (a[e] - __ldg(p.mean + n0 + e)) * __ldg(p.inv_std + n0 + e); a[e] = t * __ldg(p.gamma + n0 + e) + __ldg(p.beta + n0 + e); }
+            for (int u = 0; u < 8; u++)
+                if (z + u < p.splits) {
+                    const float4 q = __ldcg(reinterpret_cast<const float4*>(src + (z + u) * p.plane));
+                    s[u].x += q.x; s[u].y += q.y; s[u].z += q.z; s[u].w += q.w;
                 }
-            if (p.relu)
-#pragma unroll
-                for (int e = 0; e < 4; e++) a[e] = fmaxf(a[e], 0.f);
-            const int img = m / (p.P * p.Q), rem = m - img * (p.P * p.Q), pi = rem / p.Q, qi = rem - pi * p.Q;
-            float* d = p.out + img * p.o_sn + pi * p.o_sh + qi * p.o_sw + n0;
-            if (vec) *reinterpret_cast<float4*>(d) = make_float4(a[0], a[1], a[2], a[3]);
-            else for (int e = 0; e < cnt; e++) d[e] = a[e];
-            t0.x += a[0]; t0.y += a[1]; t0.z += a[2]; t0.w += a[3];
-            t1.x = fmaf(a[0], a[0], t1.x); t1.y = fmaf(a[1], a[1], t1.y); t1.z = fmaf(a[2], a[2], t1.z); t1.w = fmaf(a[3], a[3], t1.w);
         }
+        float4 v = s[0];
+#pragma unroll
+        for (int u = 1; u < 8; u++) { v.x += s[u].x; v.y += s[u].y; v.z += s[u].z; v.w += s[u].w; }
+        a[0] = v.x; a[1] = v.y; a[2] = v.z; a[3] = v.w;
+#pragma unroll
+        for (int e = 0; e < 4; e++)
+            if (e < cnt) {
+                if (p.bias) a[e] += __ldg(p.bias + n0 + e);
+                if (p.mean) { const float t = (a[e] - __ldg(p.mean + n0 + e)) * __ldg(p.inv_std + n0 + e); a[e] = t * __ldg(p.gamma + n0 + e) + __ldg(p.beta + n0 + e); }
+            }
+        if (p.relu)
+#pragma unroll
+            for (int e = 0; e < 4; e++) a[e] = fmaxf(a[e], 0.f);
+        const int img = m / (p.P * p.Q), rem = m - img * (p.P * p.Q), pi = rem / p.Q, qi = rem - pi * p.Q;
+        float* d = p.out + img * p.o_sn + pi * p.o_sh + qi * p.o_sw + n0;
+        if (vec) *reinterpret_cast<float4*>(d) = make_float4(a[0], a[1], a[2], a[3]);
+        else for (int e = 0; e < cnt; e++) d[e] = a[e];
     }
-    if (ROWS == 4 && p.stats) {              // the block's 32 rows: one row of [2][N] sums (N is a multiple of 4 here)
-        __shared__ float4 s0[8][32], s1[8][32];
-        s0[ty][lane] = t0; s1[ty][lane] = t1;
+    if constexpr (STATS) {                   // the block's 32 rows: one row of [2][N] sums (N is a multiple of 4 here)
+        __shared__ float4 val[32][32], s1[8][32];
+        val[ty][lane] = make_float4(a[0], a[1], a[2], a[3]);             // rows past M count as zeros
+        __syncthreads();
+        float4 t0 = make_float4(0.f, 0.f, 0.f, 0.f), t1 = t0;
+        if (ty < 8) {
+#pragma unroll
+            for (int r = 0; r < 4; r++) {
+                const float4 u = val[r * 8 + ty][lane];
+                t0.x += u.x; t0.y += u.y; t0.z += u.z; t0.w += u.w;
+                t1.x = fmaf(u.x, u.x, t1.x); t1.y = fmaf(u.y, u.y, t1.y); t1.z = fmaf(u.z, u.z, t1.z); t1.w = fmaf(u.w, u.w, t1.w);
+            }
+            s1[ty][lane] = t1;
+        }
+        __syncthreads();
+        if (ty < 8) val[ty][lane] = t0;
         __syncthreads();
         if (ty == 0 && n0 < p.N) {
 #pragma unroll
             for (int y = 1; y < 8; y++) {
-                const float4 u = s0[y][lane], w = s1[y][lane];
+                const float4 u = val[y][lane], w = s1[y][lane];
                 t0.x += u.x; t0.y += u.y; t0.z += u.z; t0.w += u.w; t1.x += w.x; t1.y += w.y; t1.z += w.z; t1.w += w.w;
             }
             float* row = p.stats + (size_t)blockIdx.y * 2 * p.N + n0;
@@ -2338,10 +2346,10 @@ static int run_fwd(const FwdLaunch& f, const void* act, const void* w, PrepParam
     FinishParams fp{p.M, p.N, p.P, p.Q, splits, round4(f.N), mrows * round4(f.N), sk_partial, out, f.o_sn, f.o_sh, f.o_sw,
                     p.bias, p.mean, p.inv_std, p.gamma, p.beta, relu, stats ? stats->sums : nullptr};
     const dim3 fgrid((p.N + 127) / 128, stats ? (p.M + 31) / 32 : (p.M + 7) / 8);
-    if (stats) launch_pdl(tc_split_finish_kernel<4>, fgrid, 256, 0, st, fp);
+    if (stats) launch_pdl(tc_split_finish_kernel<true>, fgrid, 1024, 0, st, fp);
     else if (splits >= 8 && (int64_t)p.M * ((p.N + 127) / 128) <= 8 * (int64_t)tc_sm_count())      // the other kernel would not fill the chip
         launch_pdl(tc_split_finish_deep_kernel, dim3((p.N + 127) / 128, p.M), 256, 0, st, fp);
-    else launch_pdl(tc_split_finish_kernel<1>, fgrid, 256, 0, st, fp);
+    else launch_pdl(tc_split_finish_kernel<false>, fgrid, 256, 0, st, fp);
     return check_launch("tc_split_finish_kernel");
 }
 
