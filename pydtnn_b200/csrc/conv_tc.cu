@@ -1743,6 +1743,43 @@ __global__ void __launch_bounds__(256) tc_wgrad_reduce_kernel(WgradReduceParams 
     }
 }
 
+// The same sum for a (co, ci, kh, kw) filter of several taps: a block owns all taps of four channels x 32 output channels, so that
+// what it stores for an output channel is one run of 4 x taps floats.  Tap by tap a warp's stores went to 32 sectors, each
+// sector written by several blocks (ResNet-50 in NCHW, 32 images: nine such launches, 9326 -> 9256 us a step).
+constexpr int RT_C = 4;
+__global__ void __launch_bounds__(256) tc_wgrad_reduce_taps_kernel(WgradReduceParams p, int taps, const float* __restrict__ partial, float* __restrict__ dw,
+                                                                   const float* __restrict__ db_partial, float* __restrict__ db)
+{
+    pdl_prologue();
+    extern __shared__ float tile[];                       // [RT_C * taps][33], at least [8][33]
+    if (db && blockIdx.y == gridDim.y - 1) { tc_wgrad_bias_sums(p, db_partial, db, reinterpret_cast<float (*)[33]>(tile)); return; }
+    const int c0 = blockIdx.y * RT_C, n0 = blockIdx.x * 32, n = n0 + threadIdx.x, rows = RT_C * taps;
+    const int64_t plane = (int64_t)p.M * p.Np;
+    for (int j = threadIdx.y; j < rows; j += 8) {
+        const int c = j / taps, tap = j - c * taps;
+        float v = 0.f;
+        if (n < p.N && c0 + c < p.Creal) {
+            const float* src = partial + (int64_t)(tap * p.C + c0 + c) * p.Np + n;
+            int z = 0;
+            for (; z + 8 <= p.splits; z += 8) {
+                float q[8];
+#pragma unroll
+                for (int u = 0; u < 8; u++) q[u] = __ldcg(src + (int64_t)(z + u) * plane);
+#pragma unroll
+                for (int u = 0; u < 8; u++) v += q[u];
+            }
+            for (; z < p.splits; z++) v += __ldcg(src + (int64_t)z * plane);
+        }
+        tile[j * 33 + threadIdx.x] = v;
+    }
+    __syncthreads();
+    const int left = (p.Creal - c0) * taps, len = left < rows ? left : rows;
+    for (int i = threadIdx.y * 32 + threadIdx.x; i < 32 * rows; i += 256) {
+        const int o = i / rows, j = i - o * rows;
+        if (j < len && n0 + o < p.N) dw[(int64_t)(n0 + o) * p.sk + c0 * p.sc + j] = tile[j * 33 + o];
+    }
+}
+
 // The same sum for small filters cut into very many splits (a 64 x 64 filter summed over 148 pixel ranges): a block
 // owns one row x 32 output channels and its 8 thread rows share the splits (thread row y adds splits y, y + 8, ... in
 // order, then the 8 partial sums are added in thread-row order: a fixed order again).
@@ -2639,8 +2676,11 @@ static int tc_wgrad_nhwc(const Geo& g, const void* x, const void* dy, void* dw, 
     int rc = dispatch_wgrad(pl.bn, g.fine, ma, mb, mo, p, pl.splits, st);
     if (rc) return rc;
     WgradReduceParams rp{Krows, g.co, low ? g.ci : Cp, g.kw, pl.splits, wsd.sk, wsd.sc, wsd.sr, wsd.ss, low ? (int)g.K : Krows, g.ci, Np, pl.splits * 4};
-    const int db_row = db ? 1 : 0;
-    if ((int64_t)((g.co + 31) / 32) * ((Krows + 31) / 32) >= 2 * (int64_t)tc_sm_count())
+    const int db_row = db ? 1 : 0, taps = g.kh * g.kw;
+    const int64_t tap_blocks = (int64_t)((g.co + 31) / 32) * ((g.ci + RT_C - 1) / RT_C);
+    if (!low && taps > 1 && taps <= 64 && wsd.ss == 1 && wsd.sr == g.kw && wsd.sc == taps && tap_blocks >= 2 * (int64_t)tc_sm_count() && g.ci < 4 * 65534)
+        launch_pdl(tc_wgrad_reduce_taps_kernel, dim3((g.co + 31) / 32, (g.ci + RT_C - 1) / RT_C + db_row), dim3(32, 8), (size_t)RT_C * taps * 33 * 4, st, rp, taps, partial, (float*)dw, p.db_partial, (float*)db);
+    else if ((int64_t)((g.co + 31) / 32) * ((Krows + 31) / 32) >= 2 * (int64_t)tc_sm_count())
         launch_pdl(tc_wgrad_reduce_kernel<4>, dim3((g.co + 31) / 32, (Krows + 31) / 32 + db_row), dim3(32, 8), 0, st, rp, partial, (float*)dw, p.db_partial, (float*)db);
     else if ((int64_t)((g.co + 31) / 32) * ((Krows + 7) / 8) >= 2 * (int64_t)tc_sm_count() || pl.splits < 16)
         launch_pdl(tc_wgrad_reduce_kernel<1>, dim3((g.co + 31) / 32, (Krows + 7) / 8 + db_row), dim3(32, 8), 0, st, rp, partial, (float*)dw, p.db_partial, (float*)db);

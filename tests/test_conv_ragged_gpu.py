@@ -44,3 +44,20 @@ def test_ragged_channels(shape, layout, w_layout):
     fused = np.maximum((y - v["running_mean"]) * v["inv_std"] * v["gamma"] + v["beta"], 0)
     got = run_conv(g, layout, np.float32, x, wt, b, None, w_layout=w_layout, engine=_lib.ENGINE_TENSOR, bn=bn, relu=True, passes=("fprop",))
     assert_parity(got["y"], fused, np.float32, f"fused {shape} {layout}")
+
+
+@pytest.mark.parametrize("layout", ["NHWC", "NCHW"])
+@pytest.mark.parametrize("n,h,w,ci,cout,kh,kw", [(1, 7, 6, 203, 190, 3, 2), (2, 6, 5, 64, 600, 1, 3), (1, 9, 9, 130, 300, 5, 5), (1, 9, 8, 33, 1070, 8, 8)])
+def test_weight_gradient_of_wide_kcrs_filters(n, h, w, ci, cout, kh, kw, layout):
+    """(co, ci, kh, kw) filters large enough for the second stage that takes all taps of four channels: 2 to 64 taps, channel
+    counts that end inside its blocks."""
+    g = co.Geom(n, h, w, ci, cout, kh, kw, 1, 1, 1, 1)
+    rng = np.random.Generator(np.random.PCG64(ci))
+    nchw = layout == "NCHW"
+    x = rng.standard_normal((n, ci, h, w) if nchw else (n, h, w, ci)).astype(np.float32)
+    wt = np.zeros((cout, ci, kh, kw) if nchw else (ci, kh, kw, cout), np.float32)
+    dy = rng.standard_normal((n, cout, g.ho, g.wo) if nchw else (n, g.ho, g.wo, cout)).astype(np.float32)
+    dw, db, _ = co.conv2d_backward(x.astype(np.float64), dy.astype(np.float64), wt.astype(np.float64), g, layout)
+    out = run_conv(g, layout, np.float32, x, wt, np.zeros(cout, np.float32), dy, w_layout="KCRS", engine=_lib.ENGINE_TENSOR, passes=("wgrad",))
+    for name, ref in (("dw", dw), ("db", db)):
+        assert_parity(out[name].reshape(ref.shape), ref, np.float32, name)
