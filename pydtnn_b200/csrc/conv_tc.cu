@@ -2202,7 +2202,10 @@ struct StatsOut { float* sums; };
 
 // How a forward launch is cut: column tiles of 128 or 64, whole tiles, balanced k-block ranges (sk), or the K loop of every
 // tile split over several CTAs (kper k-blocks each).  Costs in microseconds, measured: a k-block takes 0.45 (0.33 with 64
-// columns: half the products, the same hand-offs), the last tile's way out 2 (1); whole tiles take rounds x k-blocks.
+// columns: half the products, the same hand-offs), the last tile's way out 2 (1); whole tiles take rounds x k-blocks.  A launch of
+// one round has no other tile under whose products its k-blocks' latency hides: 0.6 (0.42).  With 0.45 (0.33) there too a 512->128
+// 1x1 layer of one 28x28 image ran its 16 k-blocks whole in 14 us, split it takes 9 (single image through ResNet-50 616 -> 550 us;
+// 0.8 and 0.65 gave 543, but 1437 -> 1456 for VGG at 32 pixels, batch 64).
 // Balanced ranges take units / G plus the hand-over of partial tiles, one after the other in the CTA that owns the tile (11 for
 // the first, 4.5 for each further CTA on the same tile: 57 us on 32 tiles of 144 k-blocks that are 20 us of products).  A split
 // takes its k-blocks, the second stage's launch (3) and the partials' way through L2; they fit the balanced mode's scratch
@@ -2221,8 +2224,8 @@ static FwdPlan fwd_plan(int64_t M, int N, int64_t kblocks, bool may_share, bool 
     const bool short_sums = may_share && !fine && units >= 4 * (int64_t)G && units < (int64_t)TC_CHUNK * G &&
                             (double)units / G + 4.0 < 0.85 * (double)((tiles0 + G - 1) / G * kblocks);
     for (int bn = N <= 64 ? 64 : 128; bn >= 64; bn -= 64) {
-        const double kb = bn == 128 ? 0.45 : 0.33, drain = bn == 128 ? 2.0 : 1.0;
         const int64_t tiles = ((M + 127) / 128) * ((N + bn - 1) / bn), rounds = (tiles + G - 1) / G;
+        const double kb = rounds == 1 ? (bn == 128 ? 0.6 : 0.42) : bn == 128 ? 0.45 : 0.33, drain = bn == 128 ? 2.0 : 1.0;
         auto offer = [&](double c, bool sk, int kper) { if (c < 0.95 * cost) { best = FwdPlan{bn, sk, kper}; cost = c; } };
         if (!short_sums) offer((double)(rounds * kblocks) * kb + drain, false, 0);
         if (!may_share) continue;
