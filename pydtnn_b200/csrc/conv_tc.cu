@@ -2208,7 +2208,7 @@ struct StatsOut { float* sums; };
 // 0.8 and 0.65 gave 543, but 1437 -> 1456 for VGG at 32 pixels, batch 64).
 // Balanced ranges take units / G plus the hand-over of partial tiles, one after the other in the CTA that owns the tile (11 for
 // the first, 4.5 for each further CTA on the same tile: 57 us on 32 tiles of 144 k-blocks that are 20 us of products).  A split
-// takes its k-blocks, the second stage's launch (3) and the partials' way through L2; they fit the balanced mode's scratch
+// takes its k-blocks, the second stage's launch (2) and the partials' way through L2 (8 TB/s; with 3 and 4 TB/s the single image took 550 us, 540); they fit the balanced mode's scratch
 // because tiles x splits is at most one CTA per SM.  Narrow tiles only pay where the wide ones leave the chip idle (single
 // images, late layers of small batches).
 struct FwdPlan { int bn; bool sk; int kper; };
@@ -2235,7 +2235,7 @@ static FwdPlan fwd_plan(int64_t M, int N, int64_t kblocks, bool may_share, bool 
         for (int64_t s = 2; s * tiles <= G && s <= kblocks; s++) {
             const int64_t kper = (kblocks + s - 1) / s;
             if (short_sums && kper * G >= units + G) continue;
-            if ((kblocks + kper - 1) / kper == s) offer((double)kper * kb + drain + 3.0 + (double)s * (double)M * N * 8.0 / 4e6, false, (int)kper);
+            if ((kblocks + kper - 1) / kper == s) offer((double)kper * kb + drain + 2.0 + (double)s * (double)M * N * 8.0 / 8e6, false, (int)kper);
         }
     }
     return best;
