@@ -82,8 +82,9 @@ __device__ __forceinline__ void fc_load(uint32_t dst, const float* __restrict__ 
     }
 }
 
-// Sums of fewer than 48 products: 4 columns x BM / 16 rows a thread in float32 FMAs (the split would cost more precision than
-// it is worth there: 2.5e-8 against 8e-8 for one row).  K is at most two steps, the tile is one block's.
+// Sums of fewer than 48 products, in all three kinds: 4 columns x BM / 16 rows a thread in float32 FMAs in the order of k (the
+// split would cost more precision than it is worth there: 2.5e-8 against 8e-8 for one row).  K is at most two steps, the tile is
+// one block's.
 template <int KIND, int BM, bool VEC>
 __device__ void fc_tile_short(const FcProblem& p, int tile, float* smem)
 {
@@ -125,6 +126,9 @@ __device__ void fc_tile_short(const FcProblem& p, int tile, float* smem)
         const int m = m0 + r + i, n = n0 + c;
         if (m >= p.M || n >= p.N) continue;
         float* d = p.c + (int64_t)m * p.N + n;
+        if (KIND == FC_FWD && p.bias)
+#pragma unroll
+            for (int j = 0; j < 4; j++) if (n + j < p.N) acc[i][j] += __ldg(p.bias + n + j);
         if (VEC && p.N % 4 == 0) *reinterpret_cast<float4*>(d) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
         else
 #pragma unroll
@@ -273,7 +277,8 @@ __global__ void __launch_bounds__(FC_THREADS, 2) fc_mma_forward_kernel(FcProblem
 {
     pdl_prologue();
     extern __shared__ __align__(16) float smem[];
-    fc_tile<FC_FWD, BM, VEC>(p, blockIdx.x / p.ks, blockIdx.x % p.ks, smem);
+    if (p.K < FC_SHORT) fc_tile_short<FC_FWD, BM, VEC>(p, blockIdx.x, smem);
+    else fc_tile<FC_FWD, BM, VEC>(p, blockIdx.x / p.ks, blockIdx.x % p.ks, smem);
 }
 // dx tiles first (their K loops are the long ones), then the tiles of dw.
 template <int BM, bool VEC>
@@ -328,7 +333,7 @@ static double fc_step_us(int bm) { return bm == 16 ? 0.43 : bm == 32 ? 0.67 : 1.
 static double fc_chain_us(const FcProblem& p, int bm)
 {
     const int blocks = p.mt * p.nt * p.ks, per_sm = (blocks + tc_sm_count() - 1) / tc_sm_count();
-    return fc_step_us(bm) * (p.kper / FC_BK) * per_sm * (p.ks == 8 && 2 * blocks > tc_sm_count() ? 1.6 : 1.1);
+    return (p.K < FC_SHORT ? 0.6 : fc_step_us(bm)) * (p.kper / FC_BK) * per_sm * (p.ks == 8 && 2 * blocks > tc_sm_count() ? 1.6 : 1.1);
 }
 bool fc_mma_takes(int dtype, int engine, int batch, int in_f, int out_f, bool backward)
 {

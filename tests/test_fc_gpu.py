@@ -103,3 +103,27 @@ def test_passes_in_one_launch(n, i, o, shift):
     run()
     assert torch.equal(y[0], torch.where(w[i - 1] > 0, float("inf"), float("-inf")))
     assert bool(torch.isfinite(y[1:]).all()) and bool(torch.isfinite(dw[: i - 1]).all())
+
+
+@pytest.mark.parametrize("n,i,o", [(3, 1, 17000), (16, 40, 512), (17, 47, 4096), (24, 33, 1000), (64, 16, 2048), (64, 17, 1000), (64, 40, 1000), (200, 47, 400), (250, 33, 515)])
+def test_short_forward_sums_are_fmas(n, i, o):
+    """Fewer than 48 features, more than 16 K weights: one launch, and as precise as FMAs.  Where one product of a sum is not zero
+    an FMA rounds once, so the result is the float32 product (a split product misses it by up to 2^-22)."""
+    L = _lib.lib()
+    g = torch.Generator(device=DEV).manual_seed(n + i + o)
+    w, b, v = (torch.randn(s, device=DEV, generator=g) for s in ((i, o), (o,), (n, i)))
+    one = torch.zeros(n, i, device=DEV)
+    hot = torch.arange(n, device=DEV) % i
+    one[torch.arange(n, device=DEV), hot] = v[:, 0]
+    ws = torch.empty(max(256, L.b2c_fc_workspace_bytes(0, n, i, o, 0)), dtype=torch.uint8, device=DEV)
+
+    def forward(x, bias):
+        y = torch.full((n, o), float("nan"), device=DEV)
+        before = L.b2c_launch_count()
+        _lib.check(L.b2c_fc_forward(0, 0, n, i, o, x.data_ptr(), w.data_ptr(), bias.data_ptr() if bias is not None else None, y.data_ptr(),
+                                    ws.data_ptr(), ws.numel(), stream()))
+        assert L.b2c_launch_count() - before == 1
+        return y
+    assert torch.equal(forward(one, None), v[:, :1] * w[hot])
+    ref = v.double() @ w.double() + b.double()
+    assert float((forward(v, b).double() - ref).norm() / ref.norm()) <= 3e-7       # at most 47 roundings of 2^-24, of either sign
