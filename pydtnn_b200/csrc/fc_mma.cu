@@ -11,7 +11,8 @@
 //
 // Precision: both operands are split by rounding, a = hi + lo.  hi * hi is summed by the tensor core over 32 products at most and
 // then added in float32 (its own additions truncate); the sums of lo * hi and hi * lo are 2^-11 of that and stay there.
-// Against float64 (2-norms) 1.0 to 1.5e-7, as the convolution engine's fine sums; fewer than 48 products are plain FMAs.
+// Against float64 (2-norms) 1.0 to 1.5e-7, as the convolution engine's fine sums; fewer than 48 products are plain FMAs, and so are
+// sums that do not come out finite.
 #include "b2c_common.cuh"
 #include <cooperative_groups.h>
 #include <float.h>
@@ -52,10 +53,10 @@ __device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], 
     asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
-// hi = v rounded to tf32, lo = v - hi.  A value whose hi would not be finite is its own lo half: an infinity comes out as from FMAs.
+// hi = v rounded to tf32, lo = v - hi.  Of an infinity, a NaN, or a value that rounds to an infinity one half is NaN, or they are
+// infinities of either sign: no sum that such a value is part of comes out finite, and such sums are then taken from FMAs.
 __device__ __forceinline__ void split_tf32(float v, uint32_t& hi, uint32_t& lo) {
-    float h = __uint_as_float((__float_as_uint(v) + 0x1000u) & 0xFFFFE000u);
-    h = fabsf(h) <= FLT_MAX ? h : 0.f;
+    const float h = __uint_as_float((__float_as_uint(v) + 0x1000u) & 0xFFFFE000u);
     hi = __float_as_uint(h); lo = __float_as_uint(v - h);
 }
 
@@ -79,6 +80,21 @@ __device__ __forceinline__ void fc_load(uint32_t dst, const float* __restrict__ 
         const bool in = e < ext && k < k_end;
         const float* s = in ? src + (KROWS ? (int64_t)e * ld + k : (int64_t)k * ld + e) : src;
         if (VEC) cp_async16(dst + (uint32_t)(o * P + n) * 4u, s, in); else cp_async4(dst + (uint32_t)(o * P + n) * 4u, s, in);
+    }
+}
+
+// Up to four stored outputs again where they are not finite, as chains of FMAs in the order of k: steps of sa and sb floats, columns
+// `next` apart in b.  hi * lo + lo * hi + hi * hi of an infinity has an infinity times a zero, or two infinities of either sign, where
+// the product itself has one value.  (A call after the store: with the chains in the epilogue passes of 5 us took 0.4 longer.)
+__device__ __noinline__ void fc_redo(const float* a, int64_t sa, const float* b, int64_t sb, int64_t next, int K, const float* bias, float* d, int count)
+{
+#pragma unroll 1
+    for (int e = 0; e < count; e++) {
+        if (fabsf(d[e]) <= FLT_MAX) continue;
+        float acc = 0.f;
+#pragma unroll 4
+        for (int k = 0; k < K; k++) acc = fmaf(__ldg(a + k * sa), __ldg(b + e * next + k * sb), acc);
+        d[e] = bias ? acc + bias[e] : acc;
     }
 }
 
@@ -268,6 +284,9 @@ __device__ void fc_tile(const FcProblem& p, int tile, int rank, float* smem)
         else
 #pragma unroll
             for (int e = 0; e < 4; e++) if (n + e < p.N) d[e] = o[e];
+        if (0.f * o[0] + 0.f * o[1] + 0.f * o[2] + 0.f * o[3] != 0.f)              // NaN where one of them is not finite
+            fc_redo(p.a + (A_KROWS ? (int64_t)m * p.lda : m), A_KROWS ? 1 : p.lda, p.b + (B_KROWS ? (int64_t)n * p.ldb : n), B_KROWS ? 1 : p.ldb,
+                    B_KROWS ? p.ldb : 1, p.K, KIND == FC_FWD && p.bias ? p.bias + n : nullptr, d, p.N - n < 4 ? p.N - n : 4);
     }
     if (p.ks > 1) cluster.sync();                        // nobody leaves while another block reads its sums
 }

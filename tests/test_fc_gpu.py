@@ -127,3 +127,49 @@ def test_short_forward_sums_are_fmas(n, i, o):
     assert torch.equal(forward(one, None), v[:, :1] * w[hot])
     ref = v.double() @ w.double() + b.double()
     assert float((forward(v, b).double() - ref).norm() / ref.norm()) <= 3e-7       # at most 47 roundings of 2^-24, of either sign
+
+
+@pytest.mark.parametrize("n,i,o", [(16, 256, 257), (24, 512, 100), (64, 777, 333), (64, 256, 256), (100, 300, 203), (48, 512, 130)])
+def test_values_that_are_not_finite_come_out_as_from_fmas(n, i, o):
+    """Infinities times infinities, tiny values and zeros, NaN, sums with infinities of both signs, values next to the largest one:
+    forward, dw (48 to 100 rows, out no multiple of 4 among them) and dx."""
+    L = _lib.lib()
+    rng = np.random.Generator(np.random.PCG64(n + i + o))
+    x, w, dy = (rng.standard_normal(s).astype(np.float32) for s in ((n, i), (i, o), (n, o)))
+    inf, big, tiny = np.float32(np.inf), np.finfo(np.float32).max, np.float32(1e-42)
+    # x and w meet in y (over i), x and dy in dw (over n), dy and w in dx (over o): planted at indices of their own in each
+    x[0, 5] = inf
+    x[1, 7], x[1, 9], x[2, 9], x[3, 11] = inf, -inf, np.nan, big * np.float32(2.0) ** -60
+    def small(count):
+        return np.ldexp(rng.standard_normal(count), -100).astype(np.float32)
+    x[4, 13], w[13, :], dy[4, :] = big, small(o), small(o)
+    dy[0, 6], dy[5, 8], dy[6, 4], dy[7, 4], dy[8, 10] = inf, -inf, inf, -inf, np.nan
+    dy[9, 12], w[:, 12], x[9, :] = -big, small(i), small(i)
+    w[5, :4] = inf, -inf, tiny, 0.0
+    X, W, D, B = (dev(a) for a in (x, w, dy, np.zeros(o, np.float32)))
+    y, dw, db, dx = (torch.full(s, 3.0, device=DEV) for s in ((n, o), (i, o), (o,), (n, i)))
+    ws = torch.empty(max(256, L.b2c_fc_workspace_bytes(0, n, i, o, 0)), dtype=torch.uint8, device=DEV)
+    count = [L.b2c_launch_count()]
+    _lib.check(L.b2c_fc_forward(0, 0, n, i, o, X.data_ptr(), W.data_ptr(), B.data_ptr(), y.data_ptr(), ws.data_ptr(), ws.numel(), stream()))
+    count.append(L.b2c_launch_count())
+    _lib.check(L.b2c_fc_backward(0, 0, n, i, o, X.data_ptr(), D.data_ptr(), W.data_ptr(), dw.data_ptr(), db.data_ptr(), dx.data_ptr(), ws.data_ptr(),
+                                 ws.numel(), stream()))
+    count.append(L.b2c_launch_count())
+    assert count[2] - count[1] == 1
+    passes = [(dw, x.T, dy, "dw"), (dx, dy, w.T, "dx")]
+    if i < 777:                                     # a wide forward pass is the convolution engine's, where infinities meet as NaN
+        assert count[1] - count[0] == 1
+        passes.append((y, x, w, "y"))
+    with np.errstate(all="ignore"):
+        for got, a, b, what in passes:
+            products = [a[r].astype(np.float64)[:, None] * b.astype(np.float64) for r in range(len(a))]      # exact, or not finite
+            ref, size = (np.stack([f(p) for p in products]) for f in (lambda p: p.sum(0), lambda p: np.abs(p).sum(0)))
+            got = got.cpu().numpy()
+            assert np.array_equal(np.isnan(got), np.isnan(ref)), what
+            assert np.array_equal(np.isinf(got), np.isinf(ref)) and np.array_equal(got[np.isinf(ref)], ref[np.isinf(ref)].astype(np.float32)), what
+            ok = np.isfinite(ref)
+            assert ok.sum() > 0.5 * ok.size and size[ok].max() < big, what
+            # lo * lo and the bits of either lo past tf32 are 2^-22 of a product each, the tensor core's four truncating sums of a step
+            # 2^-23, the float32 sums of up to 25 steps 2^-24 each: 2.7e-6 together; a product of tiny values may vanish below 2^-126, in
+            # each of its three parts, up to 777 times
+            assert np.all(np.abs(got[ok] - ref[ok]) <= 2.0 ** -18 * size[ok] + 2.0 ** -114), what
