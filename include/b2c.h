@@ -149,7 +149,8 @@ int b2c_conv_index_map(const b2c_conv_desc *desc, int64_t *map, void *stream);
 int b2c_transpose(int dtype, int n, int rows, int cols, const void *src, void *dst, void *stream);
 
 /* FC layer, row-major: y(b,out) = x(b,in) @ w(in,out) + bias; dw = x^T dy; db = sum_b dy;
- * dx = dy @ w^T.  Any of dw, db, dx may be NULL to skip it.
+ * dx = dy @ w^T.  Any of dw, db, dx may be NULL to skip it.  Outputs must not overlap inputs, nor each other; layers of
+ * more than 16384 weights also take dx on the buffer of x (dw is then finished before dx is written).
  * Replaces cublasSgemm/Dgemm + cudnnAddTensor + cublas gemv, pydtnn/backends/gpu/layers/fc_gpu.py:105-181. */
 size_t b2c_fc_workspace_bytes(int dtype, int batch, int in_features, int out_features, int engine);
 int b2c_fc_forward(int dtype, int engine, int batch, int in_features, int out_features,

@@ -206,14 +206,21 @@ extern "C" size_t b2c_fc_workspace_bytes(int dtype, int batch, int in_f, int out
     return m;
 }
 
+static bool overlap(const void* a, size_t a_floats, const void* b, size_t b_floats) {
+    const uintptr_t p = (uintptr_t)a, q = (uintptr_t)b;
+    return a && b && p < q + b_floats * 4 && q < p + a_floats * 4;
+}
+
 extern "C" int b2c_fc_forward(int dtype, int engine, int batch, int in_f, int out_f, const void* x, const void* w,
                               const void* bias, void* y, void* ws, size_t ws_bytes, void* stream) {
     Geo g; int rc = fc_geo(dtype, engine, batch, in_f, out_f, g); if (rc) return rc;
     if (!x || !w || !y) return B2C_ERR_NULL_POINTER;
     if (engine == B2C_ENGINE_AUTO && fc_tiny(batch, in_f, out_f)) return fc_tiny_forward(dtype, batch, in_f, out_f, x, w, bias, y, (cudaStream_t)stream);
     // The one-launch forms need neither workspace nor alignment; a call with less of either than the other forms ask for is left to them.
+    // So is one with an output on an input's memory: there are blocks that read while others store.
+    const size_t xs = (size_t)batch * in_f, ys = (size_t)batch * out_f, wts = (size_t)in_f * out_f;
     int e;
-    if (fc_mma_takes(dtype, engine, batch, in_f, out_f, false) && ws && ws_bytes >= pass_workspace_bytes(g, B2C_PASS_FPROP) &&
+    if (fc_mma_takes(dtype, engine, batch, in_f, out_f, false) && !overlap(y, ys, x, xs) && !overlap(y, ys, w, wts) && !overlap(y, ys, bias, out_f) && ws && ws_bytes >= pass_workspace_bytes(g, B2C_PASS_FPROP) &&
         call_engine(g, B2C_PASS_FPROP, x, y, e) == B2C_OK &&
         !(tc_fc_small_batch(dtype, engine, batch, in_f, out_f) &&
           ((((uintptr_t)x | (uintptr_t)w | (uintptr_t)y | (uintptr_t)bias) & 15) || ws_bytes < tc_fc_small_batch_bytes(batch, in_f, out_f))))
@@ -234,8 +241,10 @@ extern "C" int b2c_fc_backward(int dtype, int engine, int batch, int in_f, int o
         if ((dw && !x) || (dx && !w)) return B2C_ERR_NULL_POINTER;
         return fc_tiny_backward(dtype, batch, in_f, out_f, x, dy, w, dw, db, dx, st);
     }
+    const size_t xs = (size_t)batch * in_f, ys = (size_t)batch * out_f, wts = (size_t)in_f * out_f;
+    auto on_input = [&](const void* out, size_t floats) { return overlap(out, floats, x, xs) || overlap(out, floats, dy, ys) || overlap(out, floats, w, wts); };
     int engine_of;
-    if (fc_mma_takes(dtype, engine, batch, in_f, out_f, true) && (dw || (dx && !db)) && (!dw || x) && (!dx || w) && ws &&
+    if (fc_mma_takes(dtype, engine, batch, in_f, out_f, true) && !on_input(dx, xs) && !on_input(dw, wts) && !on_input(db, out_f) && (dw || (dx && !db)) && (!dw || x) && (!dx || w) && ws &&
         (!dw || ws_bytes >= pass_workspace_bytes(g, B2C_PASS_WGRAD)) && (!dx || ws_bytes >= pass_workspace_bytes(g, B2C_PASS_DGRAD)) &&
         (!dw || call_engine(g, B2C_PASS_WGRAD, x, dy, engine_of) == B2C_OK) && (!dx || call_engine(g, B2C_PASS_DGRAD, dx, dy, engine_of) == B2C_OK) &&
         !(tc_fc_small_batch(dtype, engine, batch, in_f, out_f) &&

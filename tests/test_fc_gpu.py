@@ -173,3 +173,23 @@ def test_values_that_are_not_finite_come_out_as_from_fmas(n, i, o):
             # 2^-23, the float32 sums of up to 25 steps 2^-24 each: 2.7e-6 together; a product of tiny values may vanish below 2^-126, in
             # each of its three parts, up to 777 times
             assert np.all(np.abs(got[ok] - ref[ok]) <= 2.0 ** -18 * size[ok] + 2.0 ** -114), what
+
+
+@pytest.mark.parametrize("n,i,o", [(16, 256, 257), (64, 256, 256), (64, 777, 333), (8, 1024, 40)])
+def test_input_gradient_on_the_buffer_of_the_input(n, i, o):
+    """dw is finished before dx is written over x: not in the launch that makes both; the same where dx only reaches into x."""
+    L = _lib.lib()
+    g = torch.Generator(device=DEV).manual_seed(i)
+    w, dy, x = (torch.randn(s, device=DEV, generator=g) for s in ((i, o), (n, o), (n, i)))
+    X, W, D = (t.double() for t in (x, w, dy))
+    ws = torch.empty(max(256, L.b2c_fc_workspace_bytes(0, n, i, o, 0)), dtype=torch.uint8, device=DEV)
+    for shift, at_once in ((0, False), (4 * (n * i // 8), False), (n * i, True)):
+        both = torch.zeros(2 * n * i, device=DEV)
+        both[:n * i] = x.flatten()
+        dx, dw, db = both[shift:shift + n * i], torch.full_like(w, float("nan")), torch.full((o,), float("nan"), device=DEV)
+        before = L.b2c_launch_count()
+        _lib.check(L.b2c_fc_backward(0, 0, n, i, o, both.data_ptr(), dy.data_ptr(), w.data_ptr(), dw.data_ptr(), db.data_ptr(), dx.data_ptr(),
+                                     ws.data_ptr(), ws.numel(), stream()))
+        assert (L.b2c_launch_count() - before == 1) == at_once
+        for got, ref in ((dw, X.T @ D), (db, D.sum(0)), (dx.view(n, i), D @ W.T)):
+            assert float((got.double() - ref).norm() / ref.norm()) <= 2e-6      # the bar of sums of 256 products
