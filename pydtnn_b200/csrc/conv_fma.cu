@@ -252,8 +252,8 @@ igemm_kernel(IgemmParams p, const float* __restrict__ A, const float* __restrict
 
 // Forward pass of sums so short that gathering them is the work (a 3x3 filter on one channel): a thread owns a pixel and NC output
 // channels, its operands come through L1 and the filter from shared memory.  The products of an output are added in the order of
-// igemm_kernel, whose 128 x 64 tiles spend a slice of 16 on nine products and several block barriers: the step of a digit classifier
-// whose first layer this is (64 images of 28x28, 1 -> 16 channels) 133 -> 124 us.
+// igemm_kernel, whose 128 x 64 tiles spend a slice of 16 on nine products and several block barriers: the first layer of a digit
+// classifier (64 images of 28x28, 1 -> 16 channels) 13.0 -> 5.5 us.  Taken where short_fprop_pays.
 constexpr int SHORT_K = 64;
 template <int NC>
 __global__ void __launch_bounds__(256)
@@ -979,6 +979,29 @@ static int launch_dgemm(const IgemmParams& p, int mode, dim3 grid, const double*
                    : launch_dgemm_v<BN, false, true, 1, int64_t>(p, mode, grid, A, B, C, ws, ep, st);
 }
 
+// Which of the two kernels takes a forward pass of at most SHORT_K products an output, in microseconds.  Both are fits (7 to 10 %) to
+// 1728 layers: 784 to 100 352 pixels, 8 to 512 outputs, 8 to 64 products, both layouts.  A tile costs igemm_kernel by slices of 16; a
+// thread of short_fprop_kernel pays for each product in latency (more where a product is a channel of one tap, and so a line
+// of its own), gathers its pixel again for every 32 outputs and is slow to store outputs that are no float4 runs.  16x28x28 40->512 1x1
+// 39 us in tiles, 46 by threads (NHWC); 44->47 10 / 18; 1->16 3x3 13 / 6; 17->64 1x1 of 56x56, 32 images, 39 / 25 (NCHW).  Lines of a warp's
+// pixels 192 bytes and more apart do not stay in L1 until their last channel: 64->512 29 / 53.  In place (1x1) is for the tiles, which
+// read a whole row before they store it.
+static bool short_fprop_pays(const IgemmParams& p, bool vec, bool in_place)
+{
+    const bool nhwc = p.c_sn == 1;
+    if (in_place || (nhwc && p.C >= 48)) return false;
+    const int slices = (p.K + 15) / 16, narrow = p.N <= 16;
+    auto rounds_past_one = [](int64_t blocks) { const double r = (double)blocks / tc_sm_count() - 1.0; return r > 0.0 ? r : 0.0; };
+    const double t = rounds_past_one((int64_t)((p.M + 127) / 128) * ((p.N + tile_bn(p.N) - 1) / tile_bn(p.N)));
+    const double b = rounds_past_one((int64_t)((p.M + 255) / 256) * (narrow ? 1 : (p.N + 31) / 32));
+    const double tiles_us = tile_bn(p.N) == 64 ? 5.1 + 1.9 * slices + t * (2.3 + 1.5 * slices)
+                          : nhwc ? 9.4 + 2.8 * slices + t * (5.0 + 2.2 * slices) : 12.8 + 2.8 * slices + t * (8.0 + 2.2 * slices);
+    const double latency = (p.R * p.S == 1 && p.K >= 24 ? 0.22 : 0.15) * p.K;
+    const double threads_us = narrow ? 3.6 + latency + b * (1.3 + 0.12 * p.K)
+                            : nhwc && !vec ? 11.0 + latency + b * (4.5 + 0.107 * p.K) : 6.5 + latency + b * ((nhwc ? 2.5 : 1.5) + 0.105 * p.K);
+    return 1.05 * threads_us < tiles_us;
+}
+
 template <typename T, int MODE>
 static int launch_igemm(IgemmParams& p, const void* A, const void* B, void* C, void* ws, size_t ws_bytes,
                         Epilogue<T> ep, cudaStream_t st)
@@ -988,6 +1011,7 @@ static int launch_igemm(IgemmParams& p, const void* A, const void* B, void* C, v
     if (p.whole && (need > ws_bytes || !ws)) { p.splits = 1; p.k_chunk = (p.K + 15) / 16 * 16; p.whole = p.m_whole = 0; need = 0; }    // whole tiles need none
     if (need > ws_bytes || (need && !ws)) return B2C_ERR_WORKSPACE_TOO_SMALL;
     const int bn = tile_bn(p.N);
+    const bool vec = p.c_sn == 1 && p.N % 4 == 0 && ((p.pb_sn | p.pb_sh | p.pb_sw) & 3) == 0 && ((uintptr_t)C & 15) == 0;
     dim3 grid((p.M + 127) / 128, (p.N + bn - 1) / bn, p.splits);
     if (grid.y > 65535 || grid.z > 65535) return B2C_ERR_TOO_LARGE;
     if constexpr (sizeof(T) == 8) {
@@ -999,8 +1023,7 @@ static int launch_igemm(IgemmParams& p, const void* A, const void* B, void* C, v
         const int rc = bn == 64 ? launch_dgemm<64>(p, MODE, grid, (const double*)A, (const double*)B, (double*)C, (double*)ws, ep, st)
                                 : launch_dgemm<128>(p, MODE, grid, (const double*)A, (const double*)B, (double*)C, (double*)ws, ep, st);
         if (rc) return rc;
-    } else if (MODE == MODE_FPROP && p.K <= SHORT_K && p.splits == 1 && (p.N + 31) / 32 <= 65535) {
-        const bool vec = p.c_sn == 1 && p.N % 4 == 0 && ((p.pb_sn | p.pb_sh | p.pb_sw) & 3) == 0 && ((uintptr_t)C & 15) == 0;
+    } else if (MODE == MODE_FPROP && p.K <= SHORT_K && p.splits == 1 && (p.N + 31) / 32 <= 65535 && short_fprop_pays(p, vec, A == C)) {
         if (p.N <= 16) launch_pdl(short_fprop_kernel<16>, dim3((p.M + 255) / 256), 256, 0, st, p, (const float*)A, (const float*)B, (float*)C, ep, vec);
         else launch_pdl(short_fprop_kernel<32>, dim3((p.M + 255) / 256, (p.N + 31) / 32), 256, 0, st, p, (const float*)A, (const float*)B, (float*)C, ep, vec);
     } else if (bn == 64)

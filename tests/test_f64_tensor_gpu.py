@@ -89,3 +89,35 @@ def test_float32_forward_of_short_sums(n, h, w, ci, cout, kh, kw, st, layout, w_
     y = co.conv2d_forward(x, wt, b, g, layout)
     out = run_conv(g, layout, np.float32, x, wt, b, np.zeros(1), w_layout=w_layout, engine=_lib.ENGINE_FMA, passes=("fprop",), relu=True)
     assert_parity(out["y"].reshape(y.shape), np.maximum(y, 0), np.float32)
+
+
+@pytest.mark.parametrize("n,hw,ci,cout", [(4, 28, 17, 64), (16, 28, 44, 47), (16, 28, 17, 96), (64, 28, 8, 16), (64, 28, 44, 512), (8, 28, 64, 96), (3, 29, 33, 130)])
+@pytest.mark.parametrize("layout", ["NHWC", "NCHW"])
+def test_float32_forward_of_short_sums_by_threads_and_by_tiles(n, hw, ci, cout, layout):
+    """1x1 layers on both sides of the rule, at sizes where it is decided by rounds of the chip."""
+    L = _lib.lib()
+    gen = torch.Generator(device=DEV).manual_seed(ci)
+    nhwc = layout == "NHWC"
+    x, f, b = (torch.randn(s, device=DEV, generator=gen) for s in ((n, hw * hw, ci), (cout, ci), (cout,)))
+    ref = x.double() @ f.double().T + b.double()
+    xin = x if nhwc else x.transpose(1, 2).contiguous()
+    y = torch.full((n, hw * hw, cout) if nhwc else (n, cout, hw * hw), float("nan"), device=DEV)
+    d = _lib.ConvDesc(_lib.LAYOUT_NHWC if nhwc else _lib.LAYOUT_NCHW, _lib.F32, _lib.W_KRSC if nhwc else _lib.W_KCRS, _lib.ENGINE_FMA,
+                      n, hw, hw, ci, cout, 1, 1, 0, 0, 1, 1, 1, 1)
+    ws = torch.empty(max(256, L.b2c_conv_workspace_bytes(d, _lib.PASS_FPROP)), dtype=torch.uint8, device=DEV)
+    _lib.check(L.b2c_conv_fprop(d, xin.data_ptr(), f.data_ptr(), b.data_ptr(), None, 0, y.data_ptr(), ws.data_ptr(), ws.numel(), stream()))
+    got = (y if nhwc else y.transpose(1, 2)).double()
+    assert float((got - ref).abs().max()) <= (ci + 1) * 2.0 ** -24 * float((x.abs().double() @ f.abs().double().T + b.abs().double()).max())
+
+
+@pytest.mark.parametrize("c", [20, 40, 60])
+def test_float32_forward_in_place(c):
+    """A 1x1 layer that writes y over x: every output of a pixel is stored after its inputs have been read."""
+    L = _lib.lib()
+    gen = torch.Generator(device=DEV).manual_seed(c)
+    x, f = (torch.randn(s, device=DEV, generator=gen) for s in ((16 * 28 * 28, c), (c, c)))
+    ref = x.double() @ f.double().T
+    d = _lib.ConvDesc(_lib.LAYOUT_NHWC, _lib.F32, _lib.W_KRSC, _lib.ENGINE_FMA, 16, 28, 28, c, c, 1, 1, 0, 0, 1, 1, 1, 1)
+    ws = torch.empty(max(256, L.b2c_conv_workspace_bytes(d, _lib.PASS_FPROP)), dtype=torch.uint8, device=DEV)
+    _lib.check(L.b2c_conv_fprop(d, x.data_ptr(), f.data_ptr(), None, None, 0, x.data_ptr(), ws.data_ptr(), ws.numel(), stream()))
+    assert_parity(x.cpu().numpy(), ref.cpu().numpy(), np.float32)
