@@ -855,16 +855,21 @@ static int choose_splits_f64(const IgemmParams& p, int bk)
 
 // More than one round of whole float64 tiles: the 392 of a 28x28 256->256 3x3 layer, batch 32, are 2.65 rounds on 148 SMs that ran as
 // three.  Row tiles that fill whole rounds stay whole, the K loops of the others are split so that they fill the chip too (that
-// layer, three passes: 3168 -> 2987 us).  Where that saves a thirtieth or more; costs as in choose_splits_f64.
+// layer, three passes: 3168 -> 2987 us).  Costs in slices of 128 columns (2.1 us) as in choose_splits_f64; a whole tile takes a
+// twentieth longer in the form with a tail, and a MB of partial sums 0.2 (0.4 of the narrow tiles' slices).  Without these two a tail saved
+// nothing where K loops are short: 1x1 512->128 of 7040 pixels 66 us whole, 76 with a tail.  By this rule 1716 of 1979 passes
+// measured (5 to 300 slices) have one, 1.27 times as fast on average; 48 of them are slower than whole by more than 1 %.
 static void split_last_round_f64(IgemmParams& p, int bk)
 {
     const int64_t nt = (p.N + tile_bn(p.N) - 1) / tile_bn(p.N), ctas = (int64_t)((p.M + 127) / 128) * nt, room = tc_sm_count(), slices = (p.K + bk - 1) / bk;
     const int64_t rows = ctas / room * room / nt, whole = rows * nt, rest = ctas - whole;         // row tiles that fill whole rounds
     if (ctas <= room || !rows || !rest) return;
-    const int64_t before = (ctas + room - 1) / room * (slices + 3);
-    int64_t best = 1, cost = before - before / 30;
+    int64_t best = 1;
+    double cost = (double)((ctas + room - 1) / room * (slices + 3));
+    const double split_mb = (double)(p.M - rows * 128) * p.N * 8e-6 * (tile_bn(p.N) == 64 ? 0.4 : 0.2);
     for (int64_t s = 2; s <= 16 && s <= slices; s++) {
-        const int64_t c = (whole + room - 1) / room * (slices + 3) + (rest * s + room - 1) / room * ((slices + s - 1) / s + 6);
+        const double c = (double)((whole + room - 1) / room) * (1.05 * (double)slices + 3.0) +
+                         (double)((rest * s + room - 1) / room * ((slices + s - 1) / s + 6)) + (double)s * split_mb;
         if (c < cost) { best = s; cost = c; }
     }
     if (best == 1) return;

@@ -76,6 +76,18 @@ def test_float64_last_round_of_tiles_is_split(n, h, w, ci, cout, room):
         assert_parity(got.cpu().numpy(), ref.cpu().numpy(), np.float64)
 
 
+def test_float64_tails_are_split_where_that_pays():
+    """Partial sums are asked for where the K loops past whole rounds are long, not where a tail costs more than it saves."""
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("sizes chosen for 148 SMs")
+    L = _lib.lib()
+    for n, h, w, ci, cout, k, which, split in ((1, 88, 80, 512, 128, 1, _lib.PASS_DGRAD, False), (13, 72, 70, 3, 128, 7, _lib.PASS_FPROP, False),
+                                               (14, 48, 48, 256, 256, 1, _lib.PASS_FPROP, False), (32, 28, 28, 256, 256, 3, _lib.PASS_FPROP, True),
+                                               (32, 28, 28, 256, 256, 3, _lib.PASS_DGRAD, True), (1, 90, 85, 200, 300, 3, _lib.PASS_FPROP, True)):
+        d = _lib.ConvDesc(_lib.LAYOUT_NHWC, _lib.F64, _lib.W_KRSC, 0, n, h, w, ci, cout, k, k, k // 2, k // 2, 1, 1, 1, 1)
+        assert (L.b2c_conv_workspace_bytes(d, which) > 0) == split, (n, h, w, ci, cout, k)
+
+
 @pytest.mark.parametrize("n,h,w,ci,cout,kh,kw,st", [(2, 13, 11, 1, 16, 3, 3, 1), (1, 16, 16, 64, 33, 1, 1, 1), (3, 17, 9, 3, 31, 4, 5, 2), (1, 23, 23, 16, 32, 2, 2, 1), (5, 8, 8, 5, 100, 3, 3, 2)])
 @pytest.mark.parametrize("layout,w_layout", [("NHWC", "KRSC"), ("NHWC", "CRSK"), ("NCHW", "KCRS")])
 def test_float32_forward_of_short_sums(n, h, w, ci, cout, kh, kw, st, layout, w_layout):
