@@ -347,7 +347,7 @@ static void fc_split(FcProblem& p, int bm)
 // A pass is taken where it costs less than as convolutions, in microseconds.  One step of 32 products takes an SM 0.43, 0.67 or 1.05
 // with tiles of 16, 32 or 64 rows, 0.6 in FMAs, and 2.5 come before the first and after the last.  Many clusters of eight leave SMs
 // idle (a GPU part of 16 SMs and a few more holds two of them): 1.6 times.  The convolutions' side is a fit to nine layers of 41 000 to
-// 38 million weights at 1 to 256 rows: forward 7 to 14, gradients 10 to 36.
+// 38 million weights at 1 to 256 rows: forward 7 to 14, gradients 10 to 36; looked at again on 28 layers at 14 batch sizes.
 static double fc_step_us(int bm) { return bm == 16 ? 0.43 : bm == 32 ? 0.67 : 1.05; }
 static double fc_chain_us(const FcProblem& p, int bm)
 {
@@ -371,6 +371,19 @@ bool fc_mma_takes(int dtype, int engine, int batch, int in_f, int out_f, bool ba
     const int steps_x = (out_f + FC_BK - 1) / FC_BK, steps_w = (batch + FC_BK - 1) / FC_BK;
     const double dx = (double)p.mt * p.nt * steps_x * (out_f < FC_SHORT ? 0.6 : fc_step_us(bm));
     const double dw = (double)((in_f + 63) / 64) * ((out_f + FC_BN - 1) / FC_BN) * steps_w * (batch < FC_SHORT ? 0.6 : fc_step_us(64));
+    if (batch > 128) {
+        // More rows than a weight gradient's blocks get through quickly: 1.3 a step (1.35 to 1.5 times that where two blocks share an SM),
+        // and the blocks past two an SM wait for most of the dx blocks.  The convolutions no longer use fine sums where in and out are whole blocks of 32:
+        // 256 x 512 x 512 21 us against 22 here, 256 x 1024 x 256 18 / 21, 256 x 100 x 4000 25 / 29; 256 x 256 x 256 15.5 / 13.0, 192 x 512 x 512 19 / 13.
+        const int blocks = p.mt * p.nt * p.ks + (in_f + 63) / 64 * ((out_f + FC_BN - 1) / FC_BN);
+        const double share = blocks > 2 * tc_sm_count() ? 1.5 : blocks > tc_sm_count() ? 1.35 : 1.0;
+        const double x = 1.1 * (out_f < FC_SHORT ? 0.6 : fc_step_us(bm)) * (p.kper / FC_BK) * share, w = 1.3 * steps_w * share;
+        const double here = 2.5 + (blocks > 2 * tc_sm_count() ? 0.8 * x + w : x > w ? x : w);
+        const double work = 1.25 * (dx + dw) / tc_sm_count() + 2.5;
+        const double there = in_f % 32 == 0 && out_f % 32 == 0 ? (out_f > 64 ? 12.5 : 10.3) + 14.0 * (weights < 1.0 ? weights : 1.0) + 0.012 * (batch - 128)
+                                                               : 10.0 + 3.5 * limb + 0.05 * batch;
+        if ((here > work ? here : work) >= there) return false;
+    }
     double t = 1.25 * (dx + dw) / tc_sm_count();
     const double chain_x = fc_chain_us(p, bm), chain_w = 2.1 * steps_w;        // the blocks that also sum the bias gradient take twice as long
     t = t > chain_x ? t : chain_x;

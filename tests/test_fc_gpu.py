@@ -193,3 +193,22 @@ def test_input_gradient_on_the_buffer_of_the_input(n, i, o):
         assert (L.b2c_launch_count() - before == 1) == at_once
         for got, ref in ((dw, X.T @ D), (db, D.sum(0)), (dx.view(n, i), D @ W.T)):
             assert float((got.double() - ref).norm() / ref.norm()) <= 2e-6      # the bar of sums of 256 products
+
+
+@pytest.mark.parametrize("n,i,o,one", [(256, 512, 512, False), (256, 1024, 256, False), (256, 100, 4000, False), (256, 256, 256, True), (192, 512, 512, True),
+                                       (129, 333, 777, True)])
+def test_gradients_of_more_than_128_rows(n, i, o, one):
+    """One launch only where it is the faster route; the same results either way."""
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("sizes chosen for 148 SMs")
+    L = _lib.lib()
+    g = torch.Generator(device=DEV).manual_seed(n + i + o)
+    x, w, dy = (torch.randn(s, device=DEV, generator=g) for s in ((n, i), (i, o), (n, o)))
+    dx, dw, db = torch.full_like(x, float("nan")), torch.full_like(w, float("nan")), torch.full((o,), float("nan"), device=DEV)
+    ws = torch.empty(max(256, L.b2c_fc_workspace_bytes(0, n, i, o, 0)), dtype=torch.uint8, device=DEV)
+    before = L.b2c_launch_count()
+    _lib.check(L.b2c_fc_backward(0, 0, n, i, o, x.data_ptr(), dy.data_ptr(), w.data_ptr(), dw.data_ptr(), db.data_ptr(), dx.data_ptr(),
+                                 ws.data_ptr(), ws.numel(), stream()))
+    assert (L.b2c_launch_count() - before == 1) == one
+    for got, ref in ((dw, x.T.double() @ dy.double()), (db, dy.double().sum(0)), (dx, dy.double() @ w.T.double())):
+        assert_parity(got.cpu().numpy(), ref.cpu().numpy(), np.float32)
