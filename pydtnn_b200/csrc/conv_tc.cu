@@ -2201,14 +2201,17 @@ static int transpose_t(const void* src, void* dst, int n, int rows, int cols, in
 struct StatsOut { float* sums; };
 
 // How a forward launch is cut: column tiles of 128 or 64, whole tiles, balanced k-block ranges (sk), or the K loop of every
-// tile split over several CTAs (kper k-blocks each).  Costs in microseconds, measured: a k-block takes 0.45 (0.33 with 64
-// columns: half the products, the same hand-offs), the last tile's way out 2 (1); whole tiles take rounds x k-blocks.  A launch of
-// one round has no other tile under whose products its k-blocks' latency hides: 0.6 (0.42).  With 0.45 (0.33) there too a 512->128
-// 1x1 layer of one 28x28 image ran its 16 k-blocks whole in 14 us, split it takes 9 (single image through ResNet-50 616 -> 550 us;
-// 0.8 and 0.65 gave 543, but 1437 -> 1456 for VGG at 32 pixels, batch 64).
+// tile split over several CTAs (kper k-blocks each).  Costs in microseconds, measured, without the 4.7 that every launch takes.
+// Several rounds: a k-block 0.45 (0.33 with 64 columns: half the products, the same hand-offs), the last tile's way out 2 (1).
+// Launches of one round, 420 layers of 49 to 12 544 pixels, 64 to 2048 channels and 2 to 144 k-blocks with up to nine ways to cut
+// each: whole tiles 2.8 + 0.5 a k-block (1 + 0.36), a split 3.5 (2.7) with its second stage + 0.5 (0.36) a k-block of its share +
+// 0.16 per MB of partial sums, out and back.  What these pick takes 0.4 % longer than the fastest cut on average (of 377 where a choice
+// is free).  Figures on which a k-block of such a launch took 0.6 (0.42) and partial sums 0.125 split loops of 16 to 36 k-blocks
+// on half a chip's tiles: 3x3/2 128->128 of 33 images of 29x29 18.8 us whole, 20.8 split; 0.45 (0.33) and a second stage of 3 left them
+// whole where one image has few tiles: 1x1 512->128 of 28x28 10.5 whole, 6.7 split.
 // Balanced ranges take units / G plus the hand-over of partial tiles, one after the other in the CTA that owns the tile (11 for
-// the first, 4.5 for each further CTA on the same tile: 57 us on 32 tiles of 144 k-blocks that are 20 us of products).  A split
-// takes its k-blocks, the second stage's launch (2) and the partials' way through L2 (8 TB/s; with 3 and 4 TB/s the single image took 550 us, 540); they fit the balanced mode's scratch
+// the first, 4.5 for each further CTA on the same tile: 57 us on 32 tiles of 144 k-blocks that are 20 us of products).  Splits fit the
+// balanced mode's scratch
 // because tiles x splits is at most one CTA per SM.  Narrow tiles only pay where the wide ones leave the chip idle (single
 // images, late layers of small batches).
 struct FwdPlan { int bn; bool sk; int kper; };
@@ -2225,9 +2228,10 @@ static FwdPlan fwd_plan(int64_t M, int N, int64_t kblocks, bool may_share, bool 
                             (double)units / G + 4.0 < 0.85 * (double)((tiles0 + G - 1) / G * kblocks);
     for (int bn = N <= 64 ? 64 : 128; bn >= 64; bn -= 64) {
         const int64_t tiles = ((M + 127) / 128) * ((N + bn - 1) / bn), rounds = (tiles + G - 1) / G;
-        const double kb = rounds == 1 ? (bn == 128 ? 0.6 : 0.42) : bn == 128 ? 0.45 : 0.33, drain = bn == 128 ? 2.0 : 1.0;
-        auto offer = [&](double c, bool sk, int kper) { if (c < 0.95 * cost) { best = FwdPlan{bn, sk, kper}; cost = c; } };
-        if (!short_sums) offer((double)(rounds * kblocks) * kb + drain, false, 0);
+        const bool one = rounds == 1;
+        const double kb = bn == 128 ? (one ? 0.5 : 0.45) : one ? 0.36 : 0.33, drain = bn == 128 ? 2.0 : 1.0;
+        auto offer = [&](double c, bool sk, int kper) { if (c < (one ? 0.98 : 0.95) * cost) { best = FwdPlan{bn, sk, kper}; cost = c; } };
+        if (!short_sums) offer((double)(rounds * kblocks) * kb + (one && bn == 128 ? 2.8 : drain), false, 0);
         if (!may_share) continue;
         const double shared = (double)G / (double)tiles;         // CTAs on one tile
         if (!fine && tiles * kblocks >= 4 * (int64_t)G)
@@ -2235,7 +2239,7 @@ static FwdPlan fwd_plan(int64_t M, int N, int64_t kblocks, bool may_share, bool 
         for (int64_t s = 2; s * tiles <= G && s <= kblocks; s++) {
             const int64_t kper = (kblocks + s - 1) / s;
             if (short_sums && kper * G >= units + G) continue;
-            if ((kblocks + kper - 1) / kper == s) offer((double)kper * kb + drain + 2.0 + (double)s * (double)M * N * 8.0 / 8e6, false, (int)kper);
+            if ((kblocks + kper - 1) / kper == s) offer((double)kper * kb + (bn == 128 ? 3.5 : 2.7) + (double)s * (double)M * N * 8e-6 * 0.16, false, (int)kper);
         }
     }
     return best;

@@ -69,3 +69,23 @@ def test_batch_sums_of_split_launches(shape):
     for got, ref, mag in ((stats[:, 0], v, v.abs()), (stats[:, 1], v * v, v * v)):
         err = (got.double().sum(0) - ref.sum(0)).abs()
         assert bool((err <= 34 * 2.0 ** -24 * mag.sum(0)).all())
+
+
+@pytest.mark.parametrize("n,hw,ci,cout,k,st,launches", [(33, 29, 128, 128, 3, 2, 1), (12, 28, 64, 64, 3, 1, 1), (2, 28, 128, 512, 3, 1, 1), (33, 15, 1024, 96, 1, 1, 1),
+                                                        (1, 28, 512, 128, 1, 1, 2), (1, 7, 512, 2048, 1, 1, 2), (1, 56, 64, 64, 3, 1, 2)])
+def test_k_loops_are_split_where_that_pays(n, hw, ci, cout, k, st, launches):
+    """Tiles on half of the chip or more with K loops of 18 to 36 k-blocks stay whole (one launch); the few tiles of one image are split."""
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("sizes chosen for 148 SMs")
+    L = _lib.lib()
+    g = co.Geom(n, hw, hw, ci, cout, k, k, k // 2, k // 2, st, st)
+    desc = make_desc(g, "NHWC", np.float32, "KRSC")
+    gen = torch.Generator(device=DEV).manual_seed(ci)
+    x, wt, b = (torch.randn(s, device=DEV, generator=gen) for s in ((n, hw, hw, ci), (cout, k, k, ci), (cout,)))
+    y = torch.full((n, g.ho, g.wo, cout), float("nan"), device=DEV)
+    ws = workspace(desc)
+    before = L.b2c_launch_count()
+    _lib.check(L.b2c_conv_fprop(ctypes.byref(desc), x.data_ptr(), wt.data_ptr(), b.data_ptr(), None, 0, y.data_ptr(), ws.data_ptr(), ws.numel(), stream()))
+    assert L.b2c_launch_count() - before == launches
+    ref = torch.nn.functional.conv2d(x.permute(0, 3, 1, 2).double(), wt.permute(0, 3, 1, 2).double(), b.double(), stride=st, padding=k // 2).permute(0, 2, 3, 1)
+    assert_parity(y.cpu().numpy(), ref.cpu().numpy(), np.float32)
