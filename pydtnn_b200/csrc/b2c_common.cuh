@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <stdio.h>
+#include <mutex>
 #include "../../include/b2c.h"
 
 namespace b2c {
@@ -39,6 +40,30 @@ inline int check_launch(const char* where) {
     if (e != cudaSuccess) { set_cuda_error(e, where); return B2C_ERR_CUDA; }
     return B2C_OK;
 }
+
+// ---- per device ---------------------------------------------------------------------------
+// Function attributes and the SM count belong to a device, not to the process: both are kept per device ordinal
+// (the device current at the call), so a process that drives several GPUs sets each one up.
+#define B2C_MAX_DEVICES 64
+inline int current_device()
+{
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= B2C_MAX_DEVICES) dev = 0;
+    return dev;
+}
+struct PerDeviceOnce {
+    std::mutex m;
+    bool done[B2C_MAX_DEVICES] = {};
+    // Runs fn() the first time it is called with a given device current; returns fn's error (and retries next time).
+    template <typename Fn> cudaError_t run(Fn fn) {
+        const int dev = current_device();
+        std::lock_guard<std::mutex> lock(m);
+        if (done[dev]) return cudaSuccess;
+        cudaError_t e = fn();
+        if (e == cudaSuccess) done[dev] = true;
+        return e;
+    }
+};
 
 // ---- geometry -----------------------------------------------------------------------------
 struct Geo {

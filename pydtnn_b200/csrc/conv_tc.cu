@@ -39,7 +39,6 @@
 #include <cuda.h>
 #include <float.h>
 #include <stdlib.h>
-#include <mutex>
 #include <type_traits>
 
 namespace b2c {
@@ -1924,29 +1923,6 @@ static bool tc_supported_nhwc(const Geo& g, int pass)
     }
     return true;
 }
-
-// Function attributes and the SM count belong to a device, not to the process: both are kept per device ordinal
-// (the device current at the call), so a process that drives several GPUs sets each one up.
-#define B2C_MAX_DEVICES 64
-static int current_device()
-{
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= B2C_MAX_DEVICES) dev = 0;
-    return dev;
-}
-struct PerDeviceOnce {
-    std::mutex m;
-    bool done[B2C_MAX_DEVICES] = {};
-    // Runs fn() the first time it is called with a given device current; returns fn's error (and retries next time).
-    template <typename Fn> cudaError_t run(Fn fn) {
-        const int dev = current_device();
-        std::lock_guard<std::mutex> lock(m);
-        if (done[dev]) return cudaSuccess;
-        cudaError_t e = fn();
-        if (e == cudaSuccess) done[dev] = true;
-        return e;
-    }
-};
 
 int tc_sm_count()
 {

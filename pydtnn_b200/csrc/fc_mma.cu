@@ -315,10 +315,11 @@ __global__ void __launch_bounds__(FC_THREADS, 2) fc_mma_backward_kernel(FcProble
     }
 }
 
-template <typename... KArgs, typename... Args>
-static int launch_cluster(const char* what, void (*kernel)(KArgs...), int blocks, int ks, size_t smem, cudaStream_t st, Args&&... args)
+template <auto KERNEL, typename... Args>
+static int launch_cluster(const char* what, int blocks, int ks, size_t smem, cudaStream_t st, const Args&... args)
 {
-    cudaError_t e = cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    static PerDeviceOnce attr_set;             // a kernel's shared memory is the same at every launch
+    const cudaError_t e = attr_set.run([smem] { return cudaFuncSetAttribute((const void*)KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); });
     if (e != cudaSuccess) { set_cuda_error(e, what); return B2C_ERR_CUDA; }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = blocks; cfg.blockDim = FC_THREADS; cfg.dynamicSmemBytes = smem; cfg.stream = st;
@@ -328,7 +329,7 @@ static int launch_cluster(const char* what, void (*kernel)(KArgs...), int blocks
     attr[1].id = cudaLaunchAttributeClusterDimension;
     attr[1].val.clusterDim.x = ks; attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr; cfg.numAttrs = 2;
-    cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+    cudaLaunchKernelEx(&cfg, KERNEL, args...);
     return check_launch(what);
 }
 
@@ -391,19 +392,31 @@ bool fc_mma_takes(int dtype, int engine, int batch, int in_f, int out_f, bool ba
     return 1.1 * (2.5 + t) < 10.0 + 3.5 * limb + 0.05 * batch;
 }
 
+template <int BM>
+static int forward(const FcProblem& p, bool vec, cudaStream_t st)
+{
+    constexpr size_t smem = fc_smem_bytes<FC_FWD, BM>();
+    const int blocks = p.mt * p.nt * p.ks;
+    return vec ? launch_cluster<fc_mma_forward_kernel<BM, true>>("fc_mma_forward_kernel", blocks, p.ks, smem, st, p)
+               : launch_cluster<fc_mma_forward_kernel<BM, false>>("fc_mma_forward_kernel", blocks, p.ks, smem, st, p);
+}
 int fc_mma_forward(int batch, int in_f, int out_f, const void* x, const void* w, const void* bias, void* y, cudaStream_t st)
 {
     FcProblem p{(const float*)x, (const float*)w, (const float*)bias, (float*)y, nullptr, batch, out_f, in_f, in_f, out_f};
     const int bm = fc_bm(batch);
     fc_split(p, bm);
     const bool vec = in_f % 4 == 0 && out_f % 4 == 0 && !(((uintptr_t)x | (uintptr_t)w | (uintptr_t)y) & 15);
-    const int blocks = p.mt * p.nt * p.ks;
-    auto go = [&](auto kernel, size_t smem) { return launch_cluster("fc_mma_forward_kernel", kernel, blocks, p.ks, smem, st, p); };
-    if (bm == 16) return vec ? go(fc_mma_forward_kernel<16, true>, fc_smem_bytes<FC_FWD, 16>()) : go(fc_mma_forward_kernel<16, false>, fc_smem_bytes<FC_FWD, 16>());
-    if (bm == 32) return vec ? go(fc_mma_forward_kernel<32, true>, fc_smem_bytes<FC_FWD, 32>()) : go(fc_mma_forward_kernel<32, false>, fc_smem_bytes<FC_FWD, 32>());
-    return vec ? go(fc_mma_forward_kernel<64, true>, fc_smem_bytes<FC_FWD, 64>()) : go(fc_mma_forward_kernel<64, false>, fc_smem_bytes<FC_FWD, 64>());
+    return bm == 16 ? forward<16>(p, vec, st) : bm == 32 ? forward<32>(p, vec, st) : forward<64>(p, vec, st);
 }
 
+template <int BM>
+static int backward(const FcProblem& px, const FcProblem& pw, bool vec, cudaStream_t st)
+{
+    constexpr size_t smem_w = fc_smem_bytes<FC_DW, 64>(), smem_x = fc_smem_bytes<FC_DX, 64>(), smem = smem_w > smem_x ? smem_w : smem_x;
+    const int dx_blocks = px.mt * px.nt * px.ks, blocks = dx_blocks + (pw.mt * pw.nt + px.ks - 1) / px.ks * px.ks;      // whole clusters
+    return vec ? launch_cluster<fc_mma_backward_kernel<BM, true>>("fc_mma_backward_kernel", blocks, px.ks, smem, st, px, pw, dx_blocks)
+               : launch_cluster<fc_mma_backward_kernel<BM, false>>("fc_mma_backward_kernel", blocks, px.ks, smem, st, px, pw, dx_blocks);
+}
 // dw with db, or dx, or all three (db alone is a column sum of dy and not for this).
 int fc_mma_backward(int batch, int in_f, int out_f, const void* x, const void* dy, const void* w, void* dw, void* db, void* dx, cudaStream_t st)
 {
@@ -414,13 +427,7 @@ int fc_mma_backward(int batch, int in_f, int out_f, const void* x, const void* d
     if (dx) fc_split(px, bm); else px.mt = px.nt = 0;
     pw.mt = dw ? (in_f + 63) / 64 : 0; pw.nt = (out_f + FC_BN - 1) / FC_BN; pw.ks = 1; pw.kper = (batch + FC_BK - 1) / FC_BK * FC_BK;
     const bool vec = in_f % 4 == 0 && out_f % 4 == 0 && !(((uintptr_t)x | (uintptr_t)dy | (uintptr_t)w | (uintptr_t)dw | (uintptr_t)dx) & 15);
-    const int dx_blocks = px.mt * px.nt * px.ks, blocks = dx_blocks + (pw.mt * pw.nt + px.ks - 1) / px.ks * px.ks;      // whole clusters
-    constexpr size_t smem_w = fc_smem_bytes<FC_DW, 64>(), smem_x = fc_smem_bytes<FC_DX, 64>();
-    const size_t smem = smem_w > smem_x ? smem_w : smem_x;
-    auto go = [&](auto kernel) { return launch_cluster("fc_mma_backward_kernel", kernel, blocks, px.ks, smem, st, px, pw, dx_blocks); };
-    if (bm == 16) return vec ? go(fc_mma_backward_kernel<16, true>) : go(fc_mma_backward_kernel<16, false>);
-    if (bm == 32) return vec ? go(fc_mma_backward_kernel<32, true>) : go(fc_mma_backward_kernel<32, false>);
-    return vec ? go(fc_mma_backward_kernel<64, true>) : go(fc_mma_backward_kernel<64, false>);
+    return bm == 16 ? backward<16>(px, pw, vec, st) : bm == 32 ? backward<32>(px, pw, vec, st) : backward<64>(px, pw, vec, st);
 }
 
 }  // namespace b2c
