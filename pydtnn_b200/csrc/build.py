@@ -12,6 +12,7 @@ package):
   three, 4 = transform warps do no work, 32 = no MMA, 64 = no TMA loads; values add.
 """
 import os
+import re
 import subprocess
 import sys
 
@@ -25,6 +26,24 @@ FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std
 VARIANTS = {None: ("", [], OUT),
             "profile": (".profile", ["-DB2C_TC_PROFILE"], os.path.join(PKG, "libb2c_profile.so")),
             "switches": (".switches", ["-DB2C_TC_SWITCHES"], os.path.join(PKG, "libb2c_switches.so"))}
+
+# conv_tc_kernel<MODE, BN, STAGES, SK, SLABS, BSRC, STREAM, MULTI, RESKB, FINE> in a symbol
+_TC_KERNEL = re.compile(r"Compiling entry function '\w*conv_tc_kernelI" + "".join(f"L[ib](?P<{a}>\\d+)E" for a in
+                        ("mode", "bn", "stages", "sk", "slabs", "bsrc", "stream", "multi", "reskb", "fine")) + r"E.*?Used (?P<regs>\d+) registers", re.S)
+LAUNCH_REGISTERS = 128
+
+
+def check_role_registers(ptxas_output):
+    """The warp roles of the kernels with warps of their own for the B tile (``tc_b_warps``) share out 4 x 128 registers: a variant
+    that was compiled to fewer would wait for registers that never come, so it must not be linked (its launch is refused)."""
+    found = 0
+    for m in _TC_KERNEL.finditer(ptxas_output):
+        v = {k: int(x) for k, x in m.groupdict().items()}
+        if (v["mode"] == 1 or v["bsrc"] != 0) and v["reskb"] == 0 and v["stream"] != 2:
+            found += 1
+            if v["regs"] != LAUNCH_REGISTERS:
+                raise RuntimeError(f"conv_tc_kernel with {LAUNCH_REGISTERS} registers a thread to share out was compiled to {v['regs']}: {v}")
+    return found
 
 
 def build(force=False, verbose=False, variant=None):
@@ -48,6 +67,8 @@ def build(force=False, verbose=False, variant=None):
             sys.stderr.write(text)
         if p.returncode:
             failed = True
+        elif os.path.basename(s) == "conv_tc.cu" and not check_role_registers(text):
+            raise RuntimeError("no conv_tc_kernel found in what ptxas says")
     if failed:
         raise RuntimeError("nvcc failed")
     subprocess.run([NVCC, "-shared", "-o", out, *objs, "-gencode", "arch=compute_100a,code=sm_100a"], check=True)
