@@ -76,6 +76,63 @@ def test_float64_last_round_of_tiles_is_split(n, h, w, ci, cout, room):
         assert_parity(got.cpu().numpy(), ref.cpu().numpy(), np.float64)
 
 
+@pytest.mark.parametrize("n,h,w,ci,cout", [(1, 20, 19, 2500, 1030)])
+def test_float64_weight_and_bias_gradient_share_the_workspace(n, h, w, ci, cout):
+    """The partial sums of a weight gradient's tail lie before the bias gradient's; with room for the latter only, tiles stay whole."""
+    L = _lib.lib()
+    gen = torch.Generator(device=DEV).manual_seed(ci)
+    x, dy = (torch.randn(s, dtype=torch.float64, device=DEV, generator=gen) for s in ((n * h * w, ci), (n * h * w, cout)))
+    d = _lib.ConvDesc(_lib.LAYOUT_NHWC, _lib.F64, _lib.W_CRSK, 0, n, h, w, ci, cout, 1, 1, 0, 0, 1, 1, 1, 1)
+    full = L.b2c_conv_workspace_bytes(d, _lib.PASS_WGRAD)
+    ws = torch.empty(full, dtype=torch.uint8, device=DEV)
+
+    def run(size):
+        df, db = torch.full((ci, cout), float("nan"), dtype=torch.float64, device=DEV), torch.full((cout,), float("nan"), dtype=torch.float64, device=DEV)
+        ws.fill_(255)
+        return L.b2c_conv_wgrad(d, x.data_ptr(), dy.data_ptr(), df.data_ptr(), db.data_ptr(), ws.data_ptr(), size, stream()), df, db
+    least, most = 0, full
+    while least < most:
+        mid = (least + most) // 2
+        least, most = (least, mid) if run(mid)[0] == 0 else (mid + 1, most)
+    assert least < full // 4                                  # what the bias gradient alone asks for
+    for size in (full, full - 1, least):
+        rc, df, db = run(size)
+        assert rc == 0
+        assert_parity(df.cpu().numpy(), (x.T @ dy).cpu().numpy(), np.float64)
+        assert_parity(db.cpu().numpy(), dy.sum(0).cpu().numpy(), np.float64)
+
+
+@pytest.mark.parametrize("layout", ["NHWC", "NCHW"])
+@pytest.mark.parametrize("n,h,w,ci,cout,k,st,which", [(1, 90, 85, 24, 300, 3, 1, _lib.PASS_FPROP), (1, 90, 85, 300, 24, 3, 1, _lib.PASS_DGRAD),
+                                                      (1, 176, 176, 300, 60, 3, 2, _lib.PASS_DGRAD)])
+def test_float64_tails_of_filters_with_taps(n, h, w, ci, cout, k, st, which, layout):
+    """Padding, several taps, pixel classes of a strided input gradient; both orders of the gathered operand."""
+    L = _lib.lib()
+    nhwc = layout == "NHWC"
+    gen = torch.Generator(device=DEV).manual_seed(ci)
+    x, f, b = (torch.randn(s, dtype=torch.float64, device=DEV, generator=gen) for s in ((n, ci, h, w), (cout, ci, k, k), (cout,)))
+    x.requires_grad_(True)
+    y = torch.nn.functional.conv2d(x, f, b, stride=st, padding=k // 2)
+    dy = torch.randn(y.shape, dtype=torch.float64, device=DEV, generator=gen)
+    y.backward(dy)
+    order = (lambda t: t.detach().permute(0, 2, 3, 1).contiguous()) if nhwc else (lambda t: t.detach().contiguous())
+    d = _lib.ConvDesc(_lib.LAYOUT_NHWC if nhwc else _lib.LAYOUT_NCHW, _lib.F64, _lib.W_KRSC if nhwc else _lib.W_KCRS, 0,
+                      n, h, w, ci, cout, k, k, k // 2, k // 2, st, st, 1, 1)
+    need = L.b2c_conv_workspace_bytes(d, which)
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert need > 0                                       # a tail
+    xs, ds, fs = order(x), order(dy), order(f)
+    for size in (need, 0):
+        ws = torch.empty(max(size, 256), dtype=torch.uint8, device=DEV)
+        if which == _lib.PASS_FPROP:
+            out, ref = torch.full_like(ds, float("nan")), order(y)
+            _lib.check(L.b2c_conv_fprop(d, xs.data_ptr(), fs.data_ptr(), b.data_ptr(), None, 0, out.data_ptr(), ws.data_ptr(), size, stream()))
+        else:
+            out, ref = torch.full_like(xs, float("nan")), order(x.grad)
+            _lib.check(L.b2c_conv_dgrad(d, ds.data_ptr(), fs.data_ptr(), out.data_ptr(), ws.data_ptr(), size, stream()))
+        assert_parity(out.cpu().numpy(), ref.cpu().numpy(), np.float64)
+
+
 def test_float64_tails_are_split_where_that_pays():
     """Partial sums are asked for where the K loops past whole rounds are long, not where a tail costs more than it saves."""
     if torch.cuda.get_device_properties(0).multi_processor_count != 148:

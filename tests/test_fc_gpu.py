@@ -212,3 +212,26 @@ def test_gradients_of_more_than_128_rows(n, i, o, one):
     assert (L.b2c_launch_count() - before == 1) == one
     for got, ref in ((dw, x.T.double() @ dy.double()), (db, dy.double().sum(0)), (dx, dy.double() @ w.T.double())):
         assert_parity(got.cpu().numpy(), ref.cpu().numpy(), np.float32)
+
+
+@pytest.mark.parametrize("n,i,o", [(8, 1024, 40), (16, 516, 100), (15, 513, 101), (24, 1024, 33), (24, 1024, 36), (32, 512, 100), (20, 515, 131), (64, 256, 256),
+                                   (64, 131, 203), (48, 512, 44), (40, 300, 203)])
+def test_every_form_of_the_one_launch_kernels(n, i, o):
+    """Row tiles of 16, 32 and 64, float4 and scalar loads, sums over out in FMAs and in products: one launch a direction, so it is
+    these kernels that ran."""
+    L = _lib.lib()
+    g = torch.Generator(device=DEV).manual_seed(n + i + o)
+    x, w, b, dy = (torch.randn(s, device=DEV, generator=g) for s in ((n, i), (i, o), (o,), (n, o)))
+    y, dx, dw, db = (torch.full_like(t, float("nan")) for t in (dy, x, w, b))
+    ws = torch.empty(max(256, L.b2c_fc_workspace_bytes(0, n, i, o, 0)), dtype=torch.uint8, device=DEV)
+    count = [L.b2c_launch_count()]
+    _lib.check(L.b2c_fc_forward(0, 0, n, i, o, x.data_ptr(), w.data_ptr(), b.data_ptr(), y.data_ptr(), ws.data_ptr(), ws.numel(), stream()))
+    count.append(L.b2c_launch_count())
+    _lib.check(L.b2c_fc_backward(0, 0, n, i, o, x.data_ptr(), dy.data_ptr(), w.data_ptr(), dw.data_ptr(), db.data_ptr(), dx.data_ptr(),
+                                 ws.data_ptr(), ws.numel(), stream()))
+    count.append(L.b2c_launch_count())
+    assert [count[1] - count[0], count[2] - count[1]] == [1, 1]
+    X, W, B, D = (t.double() for t in (x, w, b, dy))
+    for got, ref in ((y, X @ W + B), (dw, X.T @ D), (db, D.sum(0)), (dx, D @ W.T)):
+        # float32 sums of up to 1024 random terms: 2^-24 each, growing with the root of their number at most
+        assert float((got.double() - ref).norm() / ref.norm()) <= 3e-7
