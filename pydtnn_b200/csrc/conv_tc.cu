@@ -691,8 +691,8 @@ constexpr int TC_STREAM8 = 2;
 template <int STREAM> constexpr int tc_drain_warps() { return STREAM == TC_STREAM8 ? 8 : 4; }
 // Whether the lo half of the B tile is made by four warps of its own.  Four warps that split both tiles were busy for some 870
 // cycles per k-block of 128 columns (768 are products), one k-block after the other: fine sums, whose split is longer, and
-// launches of a few k-blocks waited for them (75x43 40->72 3x3, three passes 111 -> 104 us; a single image through ResNet-50 624 ->
-// 619).  Long launches gain 1 % or nothing: they are bound by shared-memory traffic (128 KB per k-block: 32 in by TMA, 48 for
+// launches of a few k-blocks waited for them (75x43 40->72 3x3, three passes 112.3 -> 105.6 us; a single image through ResNet-50 626 ->
+// 623).  Long launches gain 1 % or nothing: they are bound by shared-memory traffic (128 KB per k-block: 32 in by TMA, 48 for
 // the split, 48 to the tensor core, 1024 cycles at 128 bytes each).  Not with pre-split or resident filters (no B tile to
 // split) and not beside eight drain warps (no registers).
 template <int MODE, int BSRC, int STREAM, int RESKB> constexpr bool tc_b_warps()

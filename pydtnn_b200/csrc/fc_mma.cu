@@ -4,10 +4,11 @@
 // Such a pass as a split 1x1 convolution is a few microseconds of products between 7 of set-up (tensor memory, barriers, tensor
 // maps) and a second stage that adds the splits.  Here a block multiplies a 64-column tile with warp-level tf32 products out of a
 // cp.async ring; the blocks of a cluster share the K loop of a tile and add their sums through distributed shared memory, so no
-// partial sum touches global memory.  Forward / both gradients in us, before -> now: 64 x 256 x 256 8.5 / 16.2 -> 5.0 / 5.1;
-// 64 x 777 x 333 (pixels of no 16 bytes) 13.5 / 36.5 -> 13.5 / 8.1; 1 x 2048 x 1000 10.7 / 16.1 -> 8.0 / 8.8; gradients of
-// 64 x 4096 x 10 26.4 -> 5.7.  Bound by instructions: 460 a warp for a step of 64 x 64 x 32, a third of them the split, 2100
-// cycles of which the products take 770; what the convolution engine does faster is left to it (fc_mma_takes).
+// partial sum touches global memory.  Forward / both gradients in us, before -> now: 64 x 256 x 256 8.8 / 16.5 -> 5.1 / 5.2;
+// 64 x 333 x 777 (pixels of no 16 bytes) 17.3 / 35.4 -> 7.5 / 9.6; 1 x 2048 x 1000 11.0 / 16.2 -> 7.8 / 8.8; gradients of
+// 64 x 4096 x 10 25.4 -> 6.1; forward 32 x 40 x 512 (FMAs) 12.5 -> 3.4.  Bound by instructions: 387 a warp for a step of
+// 64 x 64 x 32 (460 while the split looked at each hi half), 0.8 us of which the products take 0.4; what the
+// convolution engine does faster is left to it (fc_mma_takes).
 //
 // Precision: both operands are split by rounding, a = hi + lo.  hi * hi is summed by the tensor core over 32 products at most and
 // then added in float32 (its own additions truncate); the sums of lo * hi and hi * lo are 2^-11 of that and stay there.
