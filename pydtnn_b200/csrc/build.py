@@ -39,7 +39,7 @@ def check_role_registers(ptxas_output):
     found = 0
     for m in _TC_KERNEL.finditer(ptxas_output):
         v = {k: int(x) for k, x in m.groupdict().items()}
-        if (v["mode"] == 1 or v["bsrc"] != 0) and v["reskb"] == 0 and v["stream"] != 2:
+        if (v["mode"] == 1 or v["bsrc"] != 0) and v["reskb"] == 0 and v["stream"] != 2 and not (v["fine"] and v["multi"] and v["bn"] == 64):
             found += 1
             if v["regs"] != LAUNCH_REGISTERS:
                 raise RuntimeError(f"conv_tc_kernel with {LAUNCH_REGISTERS} registers a thread to share out was compiled to {v['regs']}: {v}")

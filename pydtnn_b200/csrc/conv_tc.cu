@@ -694,10 +694,12 @@ template <int STREAM> constexpr int tc_drain_warps() { return STREAM == TC_STREA
 // launches of a few k-blocks waited for them (75x43 40->72 3x3, three passes 112.3 -> 105.6 us; a single image through ResNet-50 626 ->
 // 623).  Long launches gain 1 % or nothing: they are bound by shared-memory traffic (128 KB per k-block: 32 in by TMA, 48 for
 // the split, 48 to the tensor core, 1024 cycles at 128 bytes each).  Not with pre-split or resident filters (no B tile to
-// split) and not beside eight drain warps (no registers).
-template <int MODE, int BSRC, int STREAM, int RESKB> constexpr bool tc_b_warps()
+// split) and not beside eight drain warps (no registers).  Not in strided input gradients of 64 columns with fine sums either: there
+// both tiles split by four warps were 1 to 8 % faster (33x104x104 64->65 5x5/2 232 -> 219 us, 8x112x112 32->48 3x3/2 24.7 -> 22.7; with 128
+// columns the other way round, 16x56x56 128->65 3x3/2 33.2 against 35.8).
+template <int MODE, int BN, int BSRC, int STREAM, bool MULTI, int RESKB, bool FINE> constexpr bool tc_b_warps()
 {
-    return (MODE == TCM_WGRAD || BSRC != TCB_SPLIT) && RESKB == 0 && STREAM != TC_STREAM8;
+    return !(FINE && MULTI && BN == 64) && (MODE == TCM_WGRAD || BSRC != TCB_SPLIT) && RESKB == 0 && STREAM != TC_STREAM8;
 }
 // Warp roles: 0 producer, 1 MMA issuer, then the transform and the drain warps.  With B warps: 4-7 split A, 8-11 split B, 12-15
 // drain (2 and 3 idle), so that each role is a warpgroup and can take its own share of the registers: the launch has 128 per
@@ -706,15 +708,15 @@ constexpr int TC_REGS_ISSUE = 96, TC_REGS_SPLIT = 96, TC_REGS_DRAIN = 224, TC_RE
 static_assert(TC_REGS_ISSUE + 2 * TC_REGS_SPLIT + TC_REGS_DRAIN <= 4 * TC_REGS_LAUNCH, "a larger sum would wait for registers that never come");
 template <int N> __device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N> __device__ __forceinline__ void regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
-template <int MODE, int BSRC, int STREAM, int RESKB> constexpr int tc_threads()
+template <int MODE, int BN, int BSRC, int STREAM, bool MULTI, int RESKB, bool FINE> constexpr int tc_threads()
 {
-    return tc_b_warps<MODE, BSRC, STREAM, RESKB>() ? 512 : (6 + tc_drain_warps<STREAM>()) * 32;
+    return tc_b_warps<MODE, BN, BSRC, STREAM, MULTI, RESKB, FINE>() ? 512 : (6 + tc_drain_warps<STREAM>()) * 32;
 }
 
 // FINE: sums at the precision of float32 FMAs (see tc_fine_sums): both operands split by rounding, each k-block summed in tensor
 // memory by itself, its small products first.
 template <int MODE, int BN, int STAGES, bool SK, int SLABS, int BSRC, int STREAM, bool MULTI, int RESKB = 0, bool FINE = false>
-__global__ void __launch_bounds__(tc_threads<MODE, BSRC, STREAM, RESKB>(), 1)
+__global__ void __launch_bounds__(tc_threads<MODE, BN, BSRC, STREAM, MULTI, RESKB, FINE>(), 1)
 conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b0,
                const __grid_constant__ CUtensorMap tmap_b1, const __grid_constant__ CUtensorMap tmap_out,
                const __grid_constant__ CUtensorMap tmap_a3, TcParams p)
@@ -744,7 +746,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     // drain warps still store the previous one.
     using L = TcSmem<BN, STAGES, SLABS, tc_drain_warps<STREAM>(), RESKB>;
     constexpr int DW = tc_drain_warps<STREAM>();
-    constexpr bool BW = tc_b_warps<MODE, BSRC, STREAM, RESKB>();
+    constexpr bool BW = tc_b_warps<MODE, BN, BSRC, STREAM, MULTI, RESKB, FINE>();
     constexpr int XWARP = BW ? 4 : 2, DWARP = BW ? 12 : 6;       // first transform and first drain warp
     constexpr int TSLOTS = L::TSLOTS;
     static_assert(RESKB == 0 || (STREAM == TC_STREAM8 && BSRC != TCB_SPLIT), "resident filters: short-K streaming variant on the caller's filter");
@@ -798,13 +800,15 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
 
     // The lo half of stage s's B tile, written next to it (the raw tile serves as hi, or is overwritten with the rounded one).
     // Thread t of 128 takes float4s t, t + 128, ..; with sum it adds each to the bias gradient's sums of its box.
-    auto split_b = [&](int s, int t, bool sum, float4* acc) {
-        constexpr int VEC = L::B_BYTES / 16 / 128;
-        float4* b_hi = (float4*)(smem + s * L::STAGE_BYTES + L::A_BYTES);
-        float4* b_lo = (float4*)(smem + s * L::STAGE_BYTES + L::A_BYTES + L::B_BYTES);
-        float4 q[VEC];
+    constexpr int VEC = L::B_BYTES / 16 / 128;
+    auto read_b = [&](int s, int t, float4 (&q)[VEC]) {
+        const float4* b_hi = (const float4*)(smem + s * L::STAGE_BYTES + L::A_BYTES);
 #pragma unroll
         for (int i = 0; i < VEC; i++) q[i] = b_hi[t + i * 128];
+    };
+    auto split_b = [&](int s, int t, float4 (&q)[VEC], bool sum, float4* acc) {
+        float4* b_hi = (float4*)(smem + s * L::STAGE_BYTES + L::A_BYTES);
+        float4* b_lo = (float4*)(smem + s * L::STAGE_BYTES + L::A_BYTES + L::B_BYTES);
         if (FINE || (MODE == TCM_FWD && p.b_round)) {
             float largest = 0.f;
 #pragma unroll
@@ -1164,6 +1168,8 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                     else if (p.a_box_log2 == 6) column(std::integral_constant<int, 64>{});
                     else column(std::integral_constant<int, 32>{});
                 }
+                float4 bq[VEC];
+                if (SPLIT_B) read_b(s, t, bq);       // all reads of the stage first, so that the B tile's latency is under the A tile's
                 const uint32_t slot = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(L::TMEM_A_COL + ts * 64);
                 uint32_t low[32];
                 float largest = 0.f;
@@ -1190,7 +1196,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                     if (lane == 0) mbar_arrive(&afree_bar[s]);
                 }
                 tmem_st_32x32(slot + 32, low);
-                if (SPLIT_B) split_b(s, t, false, nullptr);
+                if (SPLIT_B) split_b(s, t, bq, false, nullptr);
                 tmem_st_wait();
                 tc_fence_before();
                 __syncwarp();
@@ -1221,7 +1227,11 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
 #ifdef B2C_TC_DEV
                 if (!(p.dbg & 4))
 #endif
-                split_b(s, t, do_db, dbacc);
+                {
+                    float4 bq[VEC];
+                    read_b(s, t, bq);
+                    split_b(s, t, bq, do_db, dbacc);
+                }
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&xform_bar[s]);
             }
@@ -2047,7 +2057,7 @@ static int launch_tc(const CUtensorMap& ma, const CUtensorMap& mb0, const CUtens
     {
         cudaError_t e = attr.run([] {
             const auto kernel = conv_tc_kernel<MODE, BN, STAGES, SK, SLABS, BSRC, STREAM, MULTI, RESKB, FINE>;
-            if (tc_b_warps<MODE, BSRC, STREAM, RESKB>()) {       // the roles' shares must add up to what the launch brings
+            if (tc_b_warps<MODE, BN, BSRC, STREAM, MULTI, RESKB, FINE>()) {       // the roles' shares must add up to what the launch brings
                 cudaFuncAttributes a;
                 const cudaError_t r = cudaFuncGetAttributes(&a, kernel);
                 if (r != cudaSuccess) return r;
@@ -2070,7 +2080,7 @@ static int launch_tc(const CUtensorMap& ma, const CUtensorMap& mb0, const CUtens
 #endif
     int grid = q.sk ? sm_count : (int)(tiles < sm_count ? tiles : sm_count);     // one persistent CTA per SM
     if ((q.stats && q.stats_cta) || RESKB) grid -= grid % ((p.N + BN - 1) / BN);    // a CTA keeps its column tile
-    launch_pdl(conv_tc_kernel<MODE, BN, STAGES, SK, SLABS, BSRC, STREAM, MULTI, RESKB, FINE>, grid, tc_threads<MODE, BSRC, STREAM, RESKB>(), L::TOTAL, st, ma, mb0, mb1, mo, ma3 ? *ma3 : ma, q);
+    launch_pdl(conv_tc_kernel<MODE, BN, STAGES, SK, SLABS, BSRC, STREAM, MULTI, RESKB, FINE>, grid, tc_threads<MODE, BN, BSRC, STREAM, MULTI, RESKB, FINE>(), L::TOTAL, st, ma, mb0, mb1, mo, ma3 ? *ma3 : ma, q);
     return check_launch("conv_tc_kernel");
 }
 
