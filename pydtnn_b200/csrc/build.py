@@ -27,9 +27,9 @@ VARIANTS = {None: ("", [], OUT),
             "profile": (".profile", ["-DB2C_TC_PROFILE"], os.path.join(PKG, "libb2c_profile.so")),
             "switches": (".switches", ["-DB2C_TC_SWITCHES"], os.path.join(PKG, "libb2c_switches.so"))}
 
-# conv_tc_kernel<MODE, BN, STAGES, SK, SLABS, BSRC, STREAM, MULTI, RESKB, FINE> in a symbol
+# conv_tc_kernel<MODE, BN, STAGES, SK, SLABS, BSRC, STREAM, MULTI, RESKB, FINE, BOTH> in a symbol
 _TC_KERNEL = re.compile(r"Compiling entry function '\w*conv_tc_kernelI" + "".join(f"L[ib](?P<{a}>\\d+)E" for a in
-                        ("mode", "bn", "stages", "sk", "slabs", "bsrc", "stream", "multi", "reskb", "fine")) + r"E.*?Used (?P<regs>\d+) registers", re.S)
+                        ("mode", "bn", "stages", "sk", "slabs", "bsrc", "stream", "multi", "reskb", "fine", "both")) + r"E.*?Used (?P<regs>\d+) registers", re.S)
 LAUNCH_REGISTERS = 128
 
 
@@ -39,7 +39,7 @@ def check_role_registers(ptxas_output):
     found = 0
     for m in _TC_KERNEL.finditer(ptxas_output):
         v = {k: int(x) for k, x in m.groupdict().items()}
-        if (v["mode"] == 1 or v["bsrc"] != 0) and v["reskb"] == 0 and v["stream"] != 2 and not (v["fine"] and v["multi"] and v["bn"] == 64):
+        if (v["mode"] == 1 or v["bsrc"] != 0) and v["reskb"] == 0 and v["stream"] != 2 and not v["both"]:
             found += 1
             if v["regs"] != LAUNCH_REGISTERS:
                 raise RuntimeError(f"conv_tc_kernel with {LAUNCH_REGISTERS} registers a thread to share out was compiled to {v['regs']}: {v}")

@@ -694,12 +694,13 @@ template <int STREAM> constexpr int tc_drain_warps() { return STREAM == TC_STREA
 // launches of a few k-blocks waited for them (75x43 40->72 3x3, three passes 112.3 -> 105.6 us; a single image through ResNet-50 626 ->
 // 623).  Long launches gain 1 % or nothing: they are bound by shared-memory traffic (128 KB per k-block: 32 in by TMA, 48 for
 // the split, 48 to the tensor core, 1024 cycles at 128 bytes each).  Not with pre-split or resident filters (no B tile to
-// split) and not beside eight drain warps (no registers).  Not in strided input gradients of 64 columns with fine sums either: there
-// both tiles split by four warps were 1 to 8 % faster (33x104x104 64->65 5x5/2 232 -> 219 us, 8x112x112 32->48 3x3/2 24.7 -> 22.7; with 128
-// columns the other way round, 16x56x56 128->65 3x3/2 33.2 against 35.8).
-template <int MODE, int BN, int BSRC, int STREAM, bool MULTI, int RESKB, bool FINE> constexpr bool tc_b_warps()
+// split), not beside eight drain warps (no registers), and not where BOTH says so: strided input gradients of 64 columns with fine sums
+// more than a round and a quarter of tiles and at most 32 k-blocks a tile, which were 2 to 8 % faster with both tiles split by four warps
+// (33x104x104 64->65 5x5/2 233 -> 220 us, 8x112x112 32->48 3x3/2 24.7 -> 22.6).  With fewer tiles, longer K loops or 128 columns
+// it is the other way round: 21x11x13 351->512 7x7/2 161 against 169, 3x112x112 32->300 7x7/2 144 / 162, 16x56x56 128->65 3x3/2 33.2 / 35.8.
+template <int MODE, int BSRC, int STREAM, int RESKB, bool BOTH> constexpr bool tc_b_warps()
 {
-    return !(FINE && MULTI && BN == 64) && (MODE == TCM_WGRAD || BSRC != TCB_SPLIT) && RESKB == 0 && STREAM != TC_STREAM8;
+    return !BOTH && (MODE == TCM_WGRAD || BSRC != TCB_SPLIT) && RESKB == 0 && STREAM != TC_STREAM8;
 }
 // Warp roles: 0 producer, 1 MMA issuer, then the transform and the drain warps.  With B warps: 4-7 split A, 8-11 split B, 12-15
 // drain (2 and 3 idle), so that each role is a warpgroup and can take its own share of the registers: the launch has 128 per
@@ -708,15 +709,15 @@ constexpr int TC_REGS_ISSUE = 96, TC_REGS_SPLIT = 96, TC_REGS_DRAIN = 224, TC_RE
 static_assert(TC_REGS_ISSUE + 2 * TC_REGS_SPLIT + TC_REGS_DRAIN <= 4 * TC_REGS_LAUNCH, "a larger sum would wait for registers that never come");
 template <int N> __device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N> __device__ __forceinline__ void regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
-template <int MODE, int BN, int BSRC, int STREAM, bool MULTI, int RESKB, bool FINE> constexpr int tc_threads()
+template <int MODE, int BSRC, int STREAM, int RESKB, bool BOTH> constexpr int tc_threads()
 {
-    return tc_b_warps<MODE, BN, BSRC, STREAM, MULTI, RESKB, FINE>() ? 512 : (6 + tc_drain_warps<STREAM>()) * 32;
+    return tc_b_warps<MODE, BSRC, STREAM, RESKB, BOTH>() ? 512 : (6 + tc_drain_warps<STREAM>()) * 32;
 }
 
 // FINE: sums at the precision of float32 FMAs (see tc_fine_sums): both operands split by rounding, each k-block summed in tensor
-// memory by itself, its small products first.
-template <int MODE, int BN, int STAGES, bool SK, int SLABS, int BSRC, int STREAM, bool MULTI, int RESKB = 0, bool FINE = false>
-__global__ void __launch_bounds__(tc_threads<MODE, BN, BSRC, STREAM, MULTI, RESKB, FINE>(), 1)
+// memory by itself, its small products first.  BOTH: the warps that split A split B too (see tc_b_warps).
+template <int MODE, int BN, int STAGES, bool SK, int SLABS, int BSRC, int STREAM, bool MULTI, int RESKB = 0, bool FINE = false, bool BOTH = false>
+__global__ void __launch_bounds__(tc_threads<MODE, BSRC, STREAM, RESKB, BOTH>(), 1)
 conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b0,
                const __grid_constant__ CUtensorMap tmap_b1, const __grid_constant__ CUtensorMap tmap_out,
                const __grid_constant__ CUtensorMap tmap_a3, TcParams p)
@@ -746,7 +747,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     // drain warps still store the previous one.
     using L = TcSmem<BN, STAGES, SLABS, tc_drain_warps<STREAM>(), RESKB>;
     constexpr int DW = tc_drain_warps<STREAM>();
-    constexpr bool BW = tc_b_warps<MODE, BN, BSRC, STREAM, MULTI, RESKB, FINE>();
+    constexpr bool BW = tc_b_warps<MODE, BSRC, STREAM, RESKB, BOTH>();
     constexpr int XWARP = BW ? 4 : 2, DWARP = BW ? 12 : 6;       // first transform and first drain warp
     constexpr int TSLOTS = L::TSLOTS;
     static_assert(RESKB == 0 || (STREAM == TC_STREAM8 && BSRC != TCB_SPLIT), "resident filters: short-K streaming variant on the caller's filter");
@@ -2048,7 +2049,7 @@ static size_t tc_workspace_bytes_nhwc(const Geo& g, int pass)
     return lowered + (sums > partials ? sums : partials);
 }
 
-template <int MODE, int BN, int STAGES, bool SK, int SLABS, int BSRC, int STREAM = 0, bool MULTI = false, int RESKB = 0, bool FINE = false>
+template <int MODE, int BN, int STAGES, bool SK, int SLABS, int BSRC, int STREAM = 0, bool MULTI = false, int RESKB = 0, bool FINE = false, bool BOTH = false>
 static int launch_tc(const CUtensorMap& ma, const CUtensorMap& mb0, const CUtensorMap& mb1, const CUtensorMap& mo, const TcParams& p, int splits, cudaStream_t st,
                      const CUtensorMap* ma3 = nullptr)
 {
@@ -2056,8 +2057,8 @@ static int launch_tc(const CUtensorMap& ma, const CUtensorMap& mb0, const CUtens
     static PerDeviceOnce attr;
     {
         cudaError_t e = attr.run([] {
-            const auto kernel = conv_tc_kernel<MODE, BN, STAGES, SK, SLABS, BSRC, STREAM, MULTI, RESKB, FINE>;
-            if (tc_b_warps<MODE, BN, BSRC, STREAM, MULTI, RESKB, FINE>()) {       // the roles' shares must add up to what the launch brings
+            const auto kernel = conv_tc_kernel<MODE, BN, STAGES, SK, SLABS, BSRC, STREAM, MULTI, RESKB, FINE, BOTH>;
+            if (tc_b_warps<MODE, BSRC, STREAM, RESKB, BOTH>()) {       // the roles' shares must add up to what the launch brings
                 cudaFuncAttributes a;
                 const cudaError_t r = cudaFuncGetAttributes(&a, kernel);
                 if (r != cudaSuccess) return r;
@@ -2080,7 +2081,7 @@ static int launch_tc(const CUtensorMap& ma, const CUtensorMap& mb0, const CUtens
 #endif
     int grid = q.sk ? sm_count : (int)(tiles < sm_count ? tiles : sm_count);     // one persistent CTA per SM
     if ((q.stats && q.stats_cta) || RESKB) grid -= grid % ((p.N + BN - 1) / BN);    // a CTA keeps its column tile
-    launch_pdl(conv_tc_kernel<MODE, BN, STAGES, SK, SLABS, BSRC, STREAM, MULTI, RESKB, FINE>, grid, tc_threads<MODE, BN, BSRC, STREAM, MULTI, RESKB, FINE>(), L::TOTAL, st, ma, mb0, mb1, mo, ma3 ? *ma3 : ma, q);
+    launch_pdl(conv_tc_kernel<MODE, BN, STAGES, SK, SLABS, BSRC, STREAM, MULTI, RESKB, FINE, BOTH>, grid, tc_threads<MODE, BSRC, STREAM, RESKB, BOTH>(), L::TOTAL, st, ma, mb0, mb1, mo, ma3 ? *ma3 : ma, q);
     return check_launch("conv_tc_kernel");
 }
 
@@ -2511,6 +2512,10 @@ static int tc_dgrad_classes_one_launch(const Geo& g, const WStride& wsd, bool b_
     p.cls_tile0[ncls] = (int)tiles;
     // launch-wide fields the kernel still reads
     p.M = p.cls_M[0]; p.P = p.cls_P[0]; p.Q = p.cls_Q[0]; p.kblocks = p.cls_kblocks[0]; p.S = p.cls_S[0];
+    if (g.fine && BN == 64 && p.kblocks <= 32 && tiles * 4 > (int64_t)tc_sm_count() * 5) {
+        if (bsrc == TCB_RAW_K) return launch_tc<TCM_FWD, 64, 6, false, 2, TCB_RAW_K, 0, true, 0, true, true>(ma[0], mb, ma[1], ma[2], p, 1, st, &ma[3]);
+        return launch_tc<TCM_FWD, 64, 6, false, 2, TCB_RAW_MN, 0, true, 0, true, true>(ma[0], mb, ma[1], ma[2], p, 1, st, &ma[3]);
+    }
     if (g.fine) {
         if (bsrc == TCB_RAW_K) {
             if (BN == 64) return launch_tc<TCM_FWD, 64, 6, false, 2, TCB_RAW_K, 0, true, 0, true>(ma[0], mb, ma[1], ma[2], p, 1, st, &ma[3]);
