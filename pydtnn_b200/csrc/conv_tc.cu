@@ -2190,12 +2190,14 @@ struct StatsOut { float* sums; };
 // How a forward launch is cut: column tiles of 128 or 64, whole tiles, balanced k-block ranges (sk), or the K loop of every
 // tile split over several CTAs (kper k-blocks each).  Costs in microseconds, measured, without the 4.7 that every launch takes.
 // Several rounds: a k-block 0.45 (0.33 with 64 columns: half the products, the same hand-offs), the last tile's way out 2 (1).
-// Launches of one round, 420 layers of 49 to 12 544 pixels, 64 to 2048 channels and 2 to 144 k-blocks with up to nine ways to cut
+// Launches of one round, 1240 layers of 49 to 12 544 pixels, 8 to 2048 channels and 2 to 144 k-blocks with up to nine ways to cut
 // each: whole tiles 2.8 + 0.5 a k-block (1 + 0.36), a split 3.5 (2.7) with its second stage + 0.5 (0.36) a k-block of its share +
-// 0.16 per MB of partial sums, out and back.  What these pick takes 0.4 % longer than the fastest cut on average (of 377 where a choice
-// is free).  Figures on which a k-block of such a launch took 0.6 (0.42) and partial sums 0.125 split loops of 16 to 36 k-blocks
+// 0.16 per MB of partial sums, out and back (fewer than 64 columns cost what 64 do: the second stage's warps take 128).  What these pick
+// takes 0.5 % longer than the fastest cut on average (1188 layers where a choice is free, 8 columns and fine sums among them).  Figures on which a k-block of such a launch took 0.6 (0.42) and partial sums 0.125 split loops of 16 to 36 k-blocks
 // on half a chip's tiles: 3x3/2 128->128 of 33 images of 29x29 18.8 us whole, 20.8 split; 0.45 (0.33) and a second stage of 3 left them
 // whole where one image has few tiles: 1x1 512->128 of 28x28 10.5 whole, 6.7 split.
+// Fine sums drain every k-block: 0.6 (0.45) in one round, 0.42 with 64 columns in several (with the others' figures 1.3 % slower than the
+// fastest cut, 0.6 with these: 1x1 200->89 of five 50x50 images in two rounds of 64 columns 18.7 us, in one of 128 16.4).
 // Balanced ranges take units / G plus the hand-over of partial tiles, one after the other in the CTA that owns the tile (11 for
 // the first, 4.5 for each further CTA on the same tile: 57 us on 32 tiles of 144 k-blocks that are 20 us of products).  Splits fit the
 // balanced mode's scratch
@@ -2216,7 +2218,7 @@ static FwdPlan fwd_plan(int64_t M, int N, int64_t kblocks, bool may_share, bool 
     for (int bn = N <= 64 ? 64 : 128; bn >= 64; bn -= 64) {
         const int64_t tiles = ((M + 127) / 128) * ((N + bn - 1) / bn), rounds = (tiles + G - 1) / G;
         const bool one = rounds == 1;
-        const double kb = bn == 128 ? (one ? 0.5 : 0.45) : one ? 0.36 : 0.33, drain = bn == 128 ? 2.0 : 1.0;
+        const double kb = bn == 128 ? (one ? (fine ? 0.6 : 0.5) : 0.45) : one ? (fine ? 0.45 : 0.36) : fine ? 0.42 : 0.33, drain = bn == 128 ? 2.0 : 1.0;
         auto offer = [&](double c, bool sk, int kper) { if (c < (one ? 0.98 : 0.95) * cost) { best = FwdPlan{bn, sk, kper}; cost = c; } };
         if (!short_sums) offer((double)(rounds * kblocks) * kb + (one && bn == 128 ? 2.8 : drain), false, 0);
         if (!may_share) continue;
@@ -2226,7 +2228,7 @@ static FwdPlan fwd_plan(int64_t M, int N, int64_t kblocks, bool may_share, bool 
         for (int64_t s = 2; s * tiles <= G && s <= kblocks; s++) {
             const int64_t kper = (kblocks + s - 1) / s;
             if (short_sums && kper * G >= units + G) continue;
-            if ((kblocks + kper - 1) / kper == s) offer((double)kper * kb + (bn == 128 ? 3.5 : 2.7) + (double)s * (double)M * N * 8e-6 * 0.16, false, (int)kper);
+            if ((kblocks + kper - 1) / kper == s) offer((double)kper * kb + (bn == 128 ? 3.5 : 2.7) + (double)s * (double)M * (N > 64 ? N : 64) * 8e-6 * 0.16, false, (int)kper);
         }
     }
     return best;

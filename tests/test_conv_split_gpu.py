@@ -72,7 +72,8 @@ def test_batch_sums_of_split_launches(shape):
 
 
 @pytest.mark.parametrize("n,hw,ci,cout,k,st,launches", [(33, 29, 128, 128, 3, 2, 1), (12, 28, 64, 64, 3, 1, 1), (2, 28, 128, 512, 3, 1, 1), (33, 15, 1024, 96, 1, 1, 1),
-                                                        (1, 28, 512, 128, 1, 1, 2), (1, 7, 512, 2048, 1, 1, 2), (1, 56, 64, 64, 3, 1, 2)])
+                                                        (1, 28, 512, 128, 1, 1, 2), (1, 7, 512, 2048, 1, 1, 2), (1, 56, 64, 64, 3, 1, 2),
+                                                        (6, 28, 40, 128, 3, 1, 2), (12, 28, 100, 100, 3, 1, 2)])
 def test_k_loops_are_split_where_that_pays(n, hw, ci, cout, k, st, launches):
     """Tiles on half of the chip or more with K loops of 18 to 36 k-blocks stay whole (one launch); the few tiles of one image are split."""
     if torch.cuda.get_device_properties(0).multi_processor_count != 148:
