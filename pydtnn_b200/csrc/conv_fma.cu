@@ -984,7 +984,7 @@ static int launch_dgemm(const IgemmParams& p, int mode, dim3 grid, const double*
                    : launch_dgemm_v<BN, false, true, 1, int64_t>(p, mode, grid, A, B, C, ws, ep, st);
 }
 
-// Which of the two kernels takes a forward pass of at most SHORT_K products an output, in microseconds.  Both are fits (7 to 10 %) to
+// Which of the two kernels takes a forward pass of at most SHORT_K products an output, in microseconds.  Both are fits (7 to 12 %) to
 // 1728 layers: 784 to 100 352 pixels, 8 to 512 outputs, 8 to 64 products, both layouts.  A tile costs igemm_kernel by slices of 16; a
 // thread of short_fprop_kernel pays for each product in latency (more where a product is a channel of one tap, and so a line
 // of its own), gathers its pixel again for every 32 outputs and is slow to store outputs that are no float4 runs.  16x28x28 40->512 1x1
