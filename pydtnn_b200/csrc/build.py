@@ -27,9 +27,9 @@ VARIANTS = {None: ("", [], OUT),
             "profile": (".profile", ["-DB2C_TC_PROFILE"], os.path.join(PKG, "libb2c_profile.so")),
             "switches": (".switches", ["-DB2C_TC_SWITCHES"], os.path.join(PKG, "libb2c_switches.so"))}
 
-# conv_tc_kernel<MODE, BN, STAGES, SK, SLABS, BSRC, STREAM, MULTI, RESKB, FINE, BOTH> in a symbol
+# conv_tc_kernel<MODE, BN, STAGES, SK, SLABS, BSRC, STREAM, MULTI, RESKB, FINE, BOTH, PAIR> in a symbol
 _TC_KERNEL = re.compile(r"Compiling entry function '\w*conv_tc_kernelI" + "".join(f"L[ib](?P<{a}>\\d+)E" for a in
-                        ("mode", "bn", "stages", "sk", "slabs", "bsrc", "stream", "multi", "reskb", "fine", "both")) + r"E.*?Used (?P<regs>\d+) registers", re.S)
+                        ("mode", "bn", "stages", "sk", "slabs", "bsrc", "stream", "multi", "reskb", "fine", "both")) + r"(?:Lb\d+E)?E.*?Used (?P<regs>\d+) registers", re.S)
 LAUNCH_REGISTERS = 128
 
 

@@ -71,6 +71,20 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
     return ok != 0;
 }
 
+// Arrival on the barrier at the same place in the first CTA of a pair.  What the arrival vouches for is read by the tensor core
+// only, each CTA's half of it from that CTA's own shared and tensor memory, and is ordered by fence.proxy.async and
+// tcgen05.wait in front of the arrival; no thread of the other CTA reads it, so neither the arrival nor the wait asks for
+// cluster scope (with .release.cluster and .acquire.cluster every k-block waited for a fence: 218 -> 440 us on 16x56x56 256->256 3x3).
+__device__ __forceinline__ void mbar_arrive_first(uint64_t* bar) {
+    uint32_t remote;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(remote) : "r"(smem_u32(bar)));
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(remote) : "memory");
+}
+__device__ __forceinline__ uint32_t cluster_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 // One lane of the (converged) warp is chosen; the compiler knows that exactly one thread runs the guarded
 // code, which lets it keep descriptors, coordinates and barrier addresses in uniform registers, the form
 // the TMA and tensor-core instructions take their operands in.
@@ -155,30 +169,42 @@ __device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk
 // Wait until at most N of this thread's committed store groups still read their shared-memory source.
 template <int N> __device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
 
-__device__ __forceinline__ void tmem_alloc(uint32_t* dst_smem, uint32_t ncols) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst_smem)), "r"(ncols) : "memory");
+// PAIR: a warp of each of the two CTAs takes part, as all tensor-core instructions of such a kernel are the pair's.
+template <bool PAIR> __device__ __forceinline__ void tmem_alloc(uint32_t* dst_smem, uint32_t ncols) {
+    if constexpr (PAIR) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst_smem)), "r"(ncols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst_smem)), "r"(ncols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
 }
-__device__ __forceinline__ void tmem_relinquish() { asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+template <bool PAIR> __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
+    if constexpr (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+    else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 
-// D[tmem] (+)= A[smem] * B[smem], tf32 inputs, f32 accumulate.
-__device__ __forceinline__ void umma_tf32(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
-                 ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
 // D[tmem] (+)= A[tmem] * B[smem]: the A tile sits in tensor memory (row m in lane m, one tf32 element per
 // 32-bit column, K-major), so only B is fetched from shared memory.
+// PAIR: rows 0-127 of A and D lie in the first CTA's tensor memory, rows 128-255 in the second's, at the same columns; either
+// CTA's shared memory holds half of B's columns, at the descriptor's place.
+template <bool PAIR>
 __device__ __forceinline__ void umma_tf32_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}"
-                 ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+    if constexpr (PAIR)
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                     "tcgen05.mma.cta_group::2.kind::tf32 [%0], [%1], %2, %3, p;\n\t}"
+                     ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+    else
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                     "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}"
+                     ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
-// Arrive on an mbarrier once every MMA issued so far by this thread has completed.
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+// Arrive on an mbarrier once every MMA issued so far by this thread has completed; PAIR: on those of both CTAs.
+template <bool PAIR> __device__ __forceinline__ void umma_commit(uint64_t* bar) {
+    if constexpr (PAIR)
+        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)), "h"((uint16_t)3) : "memory");
+    else
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
 __device__ __forceinline__ void tmem_ld_32x32(uint32_t taddr, uint32_t (&r)[32]) {
@@ -616,14 +642,15 @@ __device__ __forceinline__ void tc_epilogue_math(const TcParams& p, int nbase, f
 // RESKB > 0 (resident filters): the B tiles of all k-blocks (at most RESKB) stay in shared memory for the whole launch,
 // a stage holds the A tile only, and the A slots in tensor memory (TSLOTS of them) cycle separately from the STAGES
 // shared-memory stages.
-template <int BN, int STAGES, int SLABS, int DRAIN_WARPS = 4, int RESKB = 0>
+template <int BN, int STAGES, int SLABS, int DRAIN_WARPS = 4, int RESKB = 0, bool PAIR = false>
 struct TcSmem {
     static constexpr int A_BYTES = 128 * 128;   // 128 rows x 32 floats (FWD) or 32 pixels x 128 rows (WGRAD)
-    static constexpr int B_BYTES = BN * 128;
+    static constexpr int B_BYTES = (PAIR ? BN / 2 : BN) * 128;
     static constexpr int STAGE_BYTES = RESKB ? A_BYTES : A_BYTES + 2 * B_BYTES;
     static constexpr int RES_OFFSET = STAGES * STAGE_BYTES;         // resident B tiles: per k-block the raw tile, then its lo half
     static constexpr int BAR_OFFSET = RES_OFFSET + RESKB * 2 * B_BYTES;
-    static constexpr int TSLOTS = RESKB ? (512 - 2 * BN) / 64 : STAGES;
+    static constexpr int TSLOTS = RESKB || PAIR ? (512 - 2 * BN) / 64 : STAGES;
+    static constexpr int XBARS = RESKB ? TSLOTS : STAGES;         // a k-block's hand-over: by A slot or by stage
     static constexpr int EPI_OFFSET = BAR_OFFSET + 1024;          // barriers and flags live in the first 512 bytes
     static constexpr int EPI_BYTES = DRAIN_WARPS * SLABS * 4096;  // per drain warp: SLABS 32 x 32 float staging slabs
     static constexpr int TOTAL = EPI_OFFSET + EPI_BYTES + 1024;   // + alignment slack
@@ -636,21 +663,24 @@ struct TcSmem {
 // The sequence of (tile, k-block range) segments one CTA works through; every warp role walks the same sequence.
 // Plain mode: whole tiles blockIdx.x, blockIdx.x + gridDim.x, ...  Balanced mode: the contiguous unit range
 // [total * b / G, total * (b + 1) / G) of CTA b, unit = tile * kblocks + kb.
-struct TileWalk {
+template <int CL> struct TileWalk {
+    // CTAs, or pairs of them (CL = 2), are counted in place: kept in registers their number and count cost the roles spills
+    __device__ __forceinline__ static int cta() { return CL == 2 ? (int)blockIdx.x >> 1 : (int)blockIdx.x; }
+    __device__ __forceinline__ static int ctas() { return CL == 2 ? (int)gridDim.x >> 1 : (int)gridDim.x; }
     int tile, kb_b, kb_e;
     int next_tile, total_tiles, kblocks, kper;
     FastDiv plane;
     long long u, u_end;
     __device__ __forceinline__ static long long range_begin(long long total, int cta, int ctas) { return total * cta / ctas; }
     __device__ __forceinline__ void init(int total_tiles_, int kblocks_, int kper_, const FastDiv& plane_) {
-        total_tiles = total_tiles_; kblocks = kblocks_; kper = kper_; plane = plane_; next_tile = blockIdx.x;
+        total_tiles = total_tiles_; kblocks = kblocks_; kper = kper_; plane = plane_; next_tile = cta();
         const long long total = (long long)total_tiles_ * kblocks_;
-        u = range_begin(total, blockIdx.x, gridDim.x); u_end = range_begin(total, blockIdx.x + 1, gridDim.x);
+        u = range_begin(total, cta(), ctas()); u_end = range_begin(total, cta() + 1, ctas());
     }
     template <bool BALANCED> __device__ __forceinline__ bool next() {
         if (!BALANCED) {
             if (next_tile >= total_tiles) return false;
-            tile = next_tile; next_tile += gridDim.x; kb_b = 0; kb_e = kblocks;
+            tile = next_tile; next_tile += ctas(); kb_b = 0; kb_e = kblocks;
             if (kper) { kb_b = plane.div(tile) * kper; if (kb_b + kper < kblocks) kb_e = kb_b + kper; }
             return true;
         }
@@ -714,9 +744,15 @@ template <int MODE, int BSRC, int STREAM, int RESKB, bool BOTH> constexpr int tc
     return tc_b_warps<MODE, BSRC, STREAM, RESKB, BOTH>() ? 512 : (6 + tc_drain_warps<STREAM>()) * 32;
 }
 
+// PAIR: the CTAs of a cluster of two work on 256 rows of a column tile (tcgen05 cta_group::2), each on its own 128 with its own A
+// tiles and drained sums; either loads and splits half of the B tile's columns, and the first CTA's issuing lane runs the
+// products of both.  A k-block of 128 columns then moves 80 KB through an SM's shared memory instead of 128 (24 in by TMA, 32 for
+// the split, 24 to the tensor core) and 24 KB instead of 32 from L2, a stage is 32 KB instead of 48 (six stages, whose A halves
+// go through the four slots of tensor memory).  Long launches: 16x56x56 256->256 3x3 from 242 to 209 us forward, from 272 to 240 weight gradient.
+// With 64 columns (24 KB of 20 + 36) the hand-offs bound a k-block and pairs were 2 % slower. Sums are the same bit for bit.
 // FINE: sums at the precision of float32 FMAs (see tc_fine_sums): both operands split by rounding, each k-block summed in tensor
 // memory by itself, its small products first.  BOTH: the warps that split A split B too (see tc_b_warps).
-template <int MODE, int BN, int STAGES, bool SK, int SLABS, int BSRC, int STREAM, bool MULTI, int RESKB = 0, bool FINE = false, bool BOTH = false>
+template <int MODE, int BN, int STAGES, bool SK, int SLABS, int BSRC, int STREAM, bool MULTI, int RESKB = 0, bool FINE = false, bool BOTH = false, bool PAIR = false>
 __global__ void __launch_bounds__(tc_threads<MODE, BSRC, STREAM, RESKB, BOTH>(), 1)
 conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b0,
                const __grid_constant__ CUtensorMap tmap_b1, const __grid_constant__ CUtensorMap tmap_out,
@@ -745,7 +781,12 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     // CTAs running at the same time share activation rows in L2).  The smem pipeline and the two TMEM
     // buffers keep running across tile boundaries: the producer prefetches the next tile while the
     // drain warps still store the previous one.
-    using L = TcSmem<BN, STAGES, SLABS, tc_drain_warps<STREAM>(), RESKB>;
+    using L = TcSmem<BN, STAGES, SLABS, tc_drain_warps<STREAM>(), RESKB, PAIR>;
+    static_assert(!PAIR || (STREAM == 0 && RESKB == 0 && !FINE && !BOTH), "pairs of CTAs: chunked drain, sums of whole chunks");
+    // PAIR: two CTAs (a cluster) work on 256 rows of one column tile, each on its 128 rows; Walk::cta() of Walk::ctas() counts pairs.
+    constexpr int CL = PAIR ? 2 : 1, ROWS = 128 * CL, BNL = BN / CL;
+    using Walk = TileWalk<CL>;
+    const int rank = PAIR ? (int)cluster_rank() : 0;
     constexpr int DW = tc_drain_warps<STREAM>();
     constexpr bool BW = tc_b_warps<MODE, BSRC, STREAM, RESKB, BOTH>();
     constexpr int XWARP = BW ? 4 : 2, DWARP = BW ? 12 : 6;       // first transform and first drain warp
@@ -759,17 +800,17 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint64_t* full_bar = (uint64_t*)(smem + L::BAR_OFFSET);
     uint64_t* xform_bar = full_bar + STAGES;
-    uint64_t* empty_bar = xform_bar + TSLOTS;
-    uint64_t* tfull_bar = empty_bar + TSLOTS;
+    uint64_t* empty_bar = xform_bar + L::XBARS;
+    uint64_t* tfull_bar = empty_bar + L::XBARS;
     uint64_t* tempty_bar = tfull_bar + 2;
     uint64_t* afree_bar = tempty_bar + 2;              // RESKB: the transform warps have read the stage's A tile
-    uint64_t* bres_bar = afree_bar + STAGES;           // RESKB: the resident B tiles have landed
+    uint64_t* bres_bar = afree_bar + (RESKB ? STAGES : 0);           // RESKB: the resident B tiles have landed
     uint32_t* tmem_slot = (uint32_t*)(bres_bar + 1);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     TC_PROF_DECL();
-    const int mt = (p.M + 127) / 128, nt = (p.N + BN - 1) / BN;
+    const int mt = (p.M + ROWS - 1) / ROWS, nt = (p.N + BN - 1) / BN;
     const int total_tiles = MULTI ? p.cls_tile0[p.ncls] : mt * nt * p.splits;
 
     if (threadIdx.x == 32) {      // the tensor maps are kernel parameters: their fetch can start before anything else
@@ -778,26 +819,28 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         if (p.tma_store) tma_prefetch_map(&tmap_out);
         if (MULTI) { if (p.ncls > 1) tma_prefetch_map(&tmap_b1); if (p.ncls > 2) tma_prefetch_map(&tmap_out); if (p.ncls > 3) tma_prefetch_map(&tmap_a3); }
     }
-    constexpr int NBARS = 2 * STAGES + 2 * TSLOTS + 5;           // they lie one after the other from full_bar on
+    constexpr int NBARS = (RESKB ? 2 : 1) * STAGES + 2 * L::XBARS + 5;           // they lie one after the other from full_bar on
     static_assert(NBARS <= 32, "a lane of the first warp for each barrier");
     if (threadIdx.x < 32) {
         if (threadIdx.x < NBARS) {
             const uint64_t* bar = full_bar + threadIdx.x;
             const bool by_four = bar >= afree_bar && bar < bres_bar, by_xform = bar >= xform_bar && bar < empty_bar;
-            mbar_init(full_bar + threadIdx.x, by_xform ? (BW ? 8 : 4) : by_four ? 4 : bar >= tempty_bar && bar < afree_bar ? DW : 1);
+            mbar_init(full_bar + threadIdx.x, by_xform ? (BW ? 8 : 4) * CL : by_four ? 4 : bar >= tempty_bar && bar < afree_bar ? DW * CL : 1);
         }
         if (threadIdx.x == 0) *abort_flag = 0;
         fence_barrier_init();
         fence_proxy_async();
     }
-    if (warp == 1) { tmem_alloc(tmem_slot, L::TMEM_COLS); tmem_relinquish(); }
+    if (warp == 1) tmem_alloc<PAIR>(tmem_slot, L::TMEM_COLS);
     // barriers, tensor memory and the abort flag are on-chip state, set up while the kernel before this one in the
     // stream may still be draining; global memory is first touched below, after that kernel has completed
     pdl_wait();
     tc_fence_before();
-    __syncthreads();
+    if constexpr (PAIR) cluster_sync();          // the other CTA's barriers are set up as well
+    else __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    auto arrive_mma = [&](uint64_t* bar) { if constexpr (PAIR) mbar_arrive_first(bar); else mbar_arrive(bar); };      // on the issuer's side
 
     // The lo half of stage s's B tile, written next to it (the raw tile serves as hi, or is overwritten with the rounded one).
     // Thread t of 128 takes float4s t, t + 128, ..; with sum it adds each to the bias gradient's sums of its box.
@@ -860,14 +903,14 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 }
             }
         }
-        TileWalk w;
+        Walk w;
         w.init(total_tiles, p.kblocks, MODE == TCM_FWD && !SK && !MULTI && RESKB == 0 ? p.kper : 0, p.f_plane);
         while (ok && w.template next<SK>()) {
             const TileGeo tg = tile_geo(w.tile);
             if (MULTI) w.kb_e = tg.kblocks;
             const int tile = tg.ltile;
             const int rest = p.f_nt.div(tile), ni = tile - rest * nt, z = MULTI ? 0 : p.f_mt.div(rest), mi = rest - z * mt;
-            const int m0 = mi * 128, n0 = ni * BN;
+            const int m0 = mi * ROWS + rank * 128, n0 = ni * BN + rank * BNL;        // rows and columns that this CTA loads
             int img = 0, base_w = 0, base_h = 0;
             if (MODE == TCM_FWD) {
                 img = MULTI ? m0 / (tg.P * tg.Q) : p.f_pq.div(m0);
@@ -893,7 +936,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                     }
                 }
 #pragma unroll
-                for (int j = 0; j < BN / 32; j++) if (n0 + 32 * j < p.N) tx_bytes += 4096u;
+                for (int j = 0; j < BNL / 32; j++) if (n0 + 32 * j < p.N) tx_bytes += 4096u;
             }
             // FWD: channel block and tap of the k-block, the tap's pixel offset and its place in the caller's filter.
             // WGRAD: the first pixel of the k-block (32 pixels further each time: im_step images, p_step rows, q_step columns).
@@ -942,7 +985,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                                     tma_load_3d(st + L::A_BYTES, &tmap_b0, &full_bar[s], cb * 32, tap_real, n0);
                                 } else {
 #pragma unroll
-                                    for (int j = 0; j < BN / 32; j++)       // boxes past N are zero-filled by the TMA unit
+                                    for (int j = 0; j < BNL / 32; j++)      // boxes past N are zero-filled by the TMA unit
                                         tma_load_3d(st + L::A_BYTES + j * 4096, &tmap_b0, &full_bar[s], n0 + 32 * j, tap_real, cb * 32);
                                 }
                             }
@@ -967,7 +1010,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                                 tma_load_im2col_4d(st + j * (a_box * 128), &tmap_a, &full_bar[s], box_c0[j], cw, chh, im,
                                                    (uint16_t)box_offw[j], (uint16_t)box_offh[j]);
 #pragma unroll
-                        for (int j = 0; j < BN / 32; j++)
+                        for (int j = 0; j < BNL / 32; j++)
                             if (n0 + 32 * j < p.N)
                                 tma_load_2d(st + L::A_BYTES + j * 4096, &tmap_b0, &full_bar[s], n0 + 32 * j, pix0);
                         }
@@ -989,7 +1032,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         // 100 cycles between groups of twelve are free with 128 columns, 400 cost 330), so whatever this lane does between
         // the last MMA of a k-block and the first of the next is time the pipe stands still: the next k-block's barrier is
         // looked at under the last MMAs, and votes, elections and divisions are out of the loop.
-        if (elect_one_sync()) {
+        if ((!PAIR || rank == 0) && elect_one_sync()) {
             constexpr bool B_MN = MODE == TCM_WGRAD || BSRC == TCB_RAW_MN;
             // B tiles, K-major (FWD): rows of 128 B, 8-row groups 1024 B apart, K advances 32 B inside the row.
             // B tiles, MN-major (WGRAD): 32-row (K) boxes of 4096 B per 32 N elements, 4-row swizzle atoms of
@@ -999,11 +1042,12 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             constexpr uint32_t LAYOUT = B_MN ? 1 : 2;
             constexpr uint64_t KADV = B_MN ? (1024 >> 4) : (32 >> 4);
             bool ok = true;
-            Ring<TSLOTS> ring;                       // A slots in tensor memory (= the stages, unless the filters are resident)
+            Ring<L::XBARS> ring;                     // stages (A slots in tensor memory where the filters are resident)
+            Ring<TSLOTS> slots;                      // PAIR: A slots, fewer than the stages
             int gc = 0;
             bool ahead = false;                      // the next k-block was seen to be ready
             const uint64_t b_desc0 = make_smem_desc(smem_u32(smem) + (RESKB ? L::RES_OFFSET : L::A_BYTES), LBO, SBO, LAYOUT);
-            TileWalk w;
+            Walk w;
             w.init(total_tiles, p.kblocks, MODE == TCM_FWD && !SK && !MULTI && RESKB == 0 ? p.kper : 0, p.f_plane);
             while (ok && w.template next<SK>()) {
                 const TileGeo tg = tile_geo(w.tile);
@@ -1011,7 +1055,8 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 // columns past the last channel are not computed (N of an MMA is a multiple of 16)
                 const int left = p.N - (tg.ltile - p.f_nt.div(tg.ltile) * nt) * BN;
                 // and neither are the steps of a last channel block that hold only the zeros past the last channel
-                const uint32_t idesc = make_idesc_tf32(128, left >= BN ? BN : (left + 15) & ~15, 0, B_MN);
+                // (a pair's CTAs hold half of the tile's columns each, wherever the last channel lies)
+                const uint32_t idesc = make_idesc_tf32(ROWS, PAIR || left >= BN ? BN : (left + 15) & ~15, 0, B_MN);
                 // The k-blocks of one tile.  WHOLE has operand shape and step count in constants: with them in registers
                 // (or a branch between the two forms per k-block) a long launch lost 3 to 6 % (2 %).
                 auto issue_tile = [&](auto whole_c) {
@@ -1035,24 +1080,25 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                         tc_fence_after();
                         const uint64_t b_hi = b_desc0 + (uint64_t)(RESKB ? kb * (2 * L::B_BYTES >> 4) : s * (L::STAGE_BYTES >> 4));
                         const uint64_t b_lo = b_hi + (L::B_BYTES >> 4);
-                        const uint32_t a_hi = tmem_base + (uint32_t)(L::TMEM_A_COL + s * 64);
+                        const uint32_t a_hi = tmem_base + (uint32_t)(L::TMEM_A_COL + (PAIR ? slots.s : s) * 64);
                         const uint32_t a_lo = a_hi + 32;
                         ring.next();
+                        if (PAIR) slots.next();
                         // small terms first: lo*hi, hi*lo, then hi*hi
                         auto step = [&](int k, uint32_t id) {
                             const uint64_t adv = (uint64_t)k * KADV;
 #ifdef B2C_TC_DEV
                             if (p.dbg & 32) return;
 #endif
-                            umma_tf32_ts(d, a_lo + k * 8, b_hi + adv, id, k > 0 ? 1u : onto);
+                            umma_tf32_ts<PAIR>(d, a_lo + k * 8, b_hi + adv, id, k > 0 ? 1u : onto);
 #ifdef B2C_TC_DEV
                             if (p.dbg & 2) return;
 #endif
-                            umma_tf32_ts(d, a_hi + k * 8, b_lo + adv, id, 1u);
-                            umma_tf32_ts(d, a_hi + k * 8, b_hi + adv, id, 1u);
+                            umma_tf32_ts<PAIR>(d, a_hi + k * 8, b_lo + adv, id, 1u);
+                            umma_tf32_ts<PAIR>(d, a_hi + k * 8, b_hi + adv, id, 1u);
                         };
                         if constexpr (WHOLE) {
-                            constexpr uint32_t id = make_idesc_tf32(128, BN, 0, B_MN);
+                            constexpr uint32_t id = make_idesc_tf32(ROWS, BN, 0, B_MN);
                             step(0, id); step(1, id); step(2, id);
                             ahead = mbar_test(&xform_bar[ring.s], ring.phase);
                             step(3, id);
@@ -1062,12 +1108,12 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                             ahead = mbar_test(&xform_bar[ring.s], ring.phase);
                             if (++cb == p.cblocks) cb = 0;
                         }
-                        umma_commit(&empty_bar[s]);
+                        umma_commit<PAIR>(&empty_bar[s]);
                         onto = 1;
                         TC_PROF_ADD(4);    // MMA: issue
                     }
                     if (!ok) break;
-                    umma_commit(&tfull_bar[b]);
+                    umma_commit<PAIR>(&tfull_bar[b]);
                     gc++;
                 }
                 };
@@ -1086,14 +1132,14 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                         const int ks = MODE == TCM_FWD && cb == p.cblocks - 1 ? p.ktail : 4;
                         ring.next();
                         for (int k = 0; k < ks; k++) {
-                            umma_tf32_ts(d, a_lo + k * 8, b_hi + k * KADV, idesc, k > 0);
-                            umma_tf32_ts(d, a_hi + k * 8, b_lo + k * KADV, idesc, 1u);
+                            umma_tf32_ts<false>(d, a_lo + k * 8, b_hi + k * KADV, idesc, k > 0);
+                            umma_tf32_ts<false>(d, a_hi + k * 8, b_lo + k * KADV, idesc, 1u);
                         }
-                        for (int k = 0; k < ks; k++) umma_tf32_ts(d, a_hi + k * 8, b_hi + k * KADV, idesc, 1u);
+                        for (int k = 0; k < ks; k++) umma_tf32_ts<false>(d, a_hi + k * 8, b_hi + k * KADV, idesc, 1u);
                         ahead = mbar_test(&xform_bar[ring.s], ring.phase);
                         if (++cb == p.cblocks) cb = 0;
-                        umma_commit(&empty_bar[s]);
-                        umma_commit(&tfull_bar[b]);
+                        umma_commit<false>(&empty_bar[s]);
+                        umma_commit<false>(&tfull_bar[b]);
                         gc++;
                     }
                 } else if (left > BN - 16 && (MODE == TCM_WGRAD || p.ktail == 4)) issue_tile(std::true_type{});
@@ -1114,7 +1160,9 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         constexpr bool SPLIT_B = !BW && RESKB == 0 && (MODE == TCM_WGRAD || BSRC != TCB_SPLIT);      // this role also splits the B tile
         const int t = threadIdx.x - XWARP * 32;      // 0..127
         Ring<STAGES> ring;
-        Ring<TSLOTS> slots;                          // the stages' own A slots, or (resident filters) a separate ring
+        Ring<TSLOTS> slots;                          // the stages' own A slots, or (resident filters, PAIR) a separate ring
+        Ring<STAGES> freed;                          // PAIR: the stage of the k-block TSLOTS before this one, which had its slot
+        int filled = 0;
         bool ok = true;
         if (RESKB) {
             // the lo halves of the resident filter tiles, once per launch
@@ -1133,7 +1181,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 fence_proxy_async();
             }
         }
-        TileWalk w;
+        Walk w;
         w.init(total_tiles, p.kblocks, MODE == TCM_FWD && !SK && !MULTI && RESKB == 0 ? p.kper : 0, p.f_plane);
         while (ok && w.template next<SK>()) {
             if (MULTI) w.kb_e = tile_geo(w.tile).kblocks;
@@ -1144,9 +1192,16 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 if (t == 0) TC_PROF_ADD(5);    // transform: waiting for TMA data
                 const uint8_t* st = smem + s * L::STAGE_BYTES;
                 // a slot of a separate ring is free once the MMAs that read it have completed
+                if (PAIR) {
+                    if (filled < TSLOTS) filled++;
+                    else {
+                        if (!mbar_wait(&empty_bar[freed.s], freed.phase, abort_flag, &g_tc_status, TC_ERR_EMPTY)) { ok = false; break; }
+                        freed.next();
+                    }
+                }
                 if (RESKB && !mbar_wait(&empty_bar[ts], slots.phase ^ 1, abort_flag, &g_tc_status, TC_ERR_EMPTY)) { ok = false; break; }
 #ifdef B2C_TC_DEV
-                if (p.dbg & 4) { tc_fence_before(); __syncwarp(); if (lane == 0) { if (RESKB) mbar_arrive(&afree_bar[s]); mbar_arrive(&xform_bar[ts]); } continue; }
+                if (p.dbg & 4) { tc_fence_before(); __syncwarp(); if (lane == 0) { if (RESKB) mbar_arrive(&afree_bar[s]); arrive_mma(&xform_bar[RESKB ? ts : s]); } continue; }
 #endif
                 uint32_t v[32];
                 if (MODE == TCM_FWD) {
@@ -1201,7 +1256,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 tmem_st_wait();
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&xform_bar[ts]);
+                if (lane == 0) arrive_mma(&xform_bar[RESKB ? ts : s]);
                 if (t == 0) TC_PROF_ADD(6);    // transform: work
             }
         }
@@ -1212,7 +1267,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         constexpr int BOXES = L::B_BYTES / 4096;
         Ring<STAGES> ring;
         bool ok = true;
-        TileWalk w;
+        Walk w;
         w.init(total_tiles, p.kblocks, MODE == TCM_FWD && !SK && !MULTI ? p.kper : 0, p.f_plane);
         while (ok && w.template next<SK>()) {
             if (MULTI) w.kb_e = tile_geo(w.tile).kblocks;
@@ -1234,7 +1289,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                     split_b(s, t, bq, do_db, dbacc);
                 }
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&xform_bar[s]);
+                if (lane == 0) arrive_mma(&xform_bar[s]);
             }
             if (MODE == TCM_WGRAD && do_db && ok) {
                 // Float4 number t + 128 i of the B region is box i/2, pixel row t/8 + 16 (i & 1), 16-byte chunk t & 7.
@@ -1252,7 +1307,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                         v.x += __shfl_xor_sync(0xffffffffu, v.x, mask); v.y += __shfl_xor_sync(0xffffffffu, v.y, mask);
                         v.z += __shfl_xor_sync(0xffffffffu, v.z, mask); v.w += __shfl_xor_sync(0xffffffffu, v.w, mask);
                     }
-                    const int n = ni * BN + bx * 32;
+                    const int n = ni * BN + rank * BNL + bx * 32;
                     if (lane < 8 && n + lane * 4 < p.N)
                         *reinterpret_cast<float4*>(p.db_partial + ((size_t)z * 4 + (warp & 3)) * p.Np + n + lane * 4) = v;
                 }
@@ -1273,14 +1328,14 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         float cs0[NSLAB], cs1[NSLAB];                    // batch statistics summed over this CTA's tiles (stats_cta)
 #pragma unroll
         for (int i = 0; i < NSLAB; i++) cs0[i] = cs1[i] = 0.f;
-        TileWalk w;
+        Walk w;
         w.init(total_tiles, p.kblocks, MODE == TCM_FWD && !SK && !MULTI && RESKB == 0 ? p.kper : 0, p.f_plane);
         while (ok && w.template next<SK>()) {
             const TileGeo tg = tile_geo(w.tile);
             if (MULTI) w.kb_e = tg.kblocks;
             const int tile = tg.ltile;
             const int rest = p.f_nt.div(tile), ni = tile - rest * nt, z = MULTI ? 0 : p.f_mt.div(rest), mi = rest - z * mt;
-            const int m0 = mi * 128, n0 = ni * BN;
+            const int m0 = mi * ROWS + rank * 128, n0 = ni * BN;
             // One 32-row x 32-column slab of the tile on its way out (dense outputs): epilogue steps, staging in a
             // 128B-swizzled slab (conflict-free float4 writes), TMA store (whole rows, asynchronous, rows >= M and
             // columns >= N clipped; SLABS slabs per warp rotate so the warp never waits on HBM), and the slab's batch
@@ -1301,7 +1356,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 fence_proxy_async();
                 __syncwarp();
                 if (lane == 0) {
-                    if (MODE == TCM_FWD) tma_store_2d(&tmap_out, buf, n0 + cc * 32, (p.kper ? z * mt * 128 : 0) + m0 + quad * 32);
+                    if (MODE == TCM_FWD) tma_store_2d(&tmap_out, buf, n0 + cc * 32, (p.kper ? z * mt * ROWS : 0) + m0 + quad * 32);
                     else tma_store_3d(&tmap_out, buf, n0 + cc * 32, m0 + quad * 32, z);
                     tma_store_commit();
                 }
@@ -1414,7 +1469,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 }
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&tempty_bar[b]);
+                if (lane == 0) arrive_mma(&tempty_bar[b]);
                 if (threadIdx.x == DWARP * 32) TC_PROF_ADD(8);    // drain: TMEM load + add
             }
             if (SK && ok) {
@@ -1433,8 +1488,9 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                     // this CTA started the tile and its range ended inside it: the following CTAs hold the rest
                     const long long total = (long long)total_tiles * p.kblocks;
                     const long long tile_end = (long long)(tile + 1) * p.kblocks;
-                    for (int c2 = blockIdx.x + 1; c2 < (int)gridDim.x && ok; c2++) {
-                        if (TileWalk::range_begin(total, c2, gridDim.x) >= tile_end) break;
+                    for (int p2 = Walk::cta() + 1; p2 < Walk::ctas() && ok; p2++) {
+                        if (Walk::range_begin(total, p2, Walk::ctas()) >= tile_end) break;
+                        const int c2 = p2 * CL + rank;
                         int got = 1;
                         if (lane == 0) {
                             const int* flag = &p.sk_flags[c2 * 4 + quad];
@@ -1521,20 +1577,23 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             }   // chunked drain
         }
         if (MODE == TCM_FWD && !SK && !MULTI && p.stats && p.stats_cta && ok) {
-            // One row of sums per (group of nt CTAs, row quadrant): the nt CTAs of a group hold the nt column tiles.
-            const int n0 = (int)(blockIdx.x % nt) * BN;
+            // One row of sums per (group of nt CTAs, row quadrant): the nt CTAs of a group hold the nt column tiles.  (The second CTA of
+            // a launch's last pair may have no rows at all: nobody expects a row of its.)
+            const int n0 = (int)((unsigned)Walk::cta() % (unsigned)nt) * BN;
             const int col = tc_stats_col(lane);
-            float* srow = p.stats + ((size_t)((blockIdx.x / nt) * 4 + quad) * 2) * p.N + n0 + cbeg * 32 + col;
+            float* srow = p.stats + ((size_t)(((unsigned)Walk::cta() / (unsigned)nt * CL + rank) * 4 + quad) * 2) * p.N + n0 + cbeg * 32 + col;
 #pragma unroll
             for (int i = 0; i < NSLAB; i++)
-                if (n0 + (cbeg + i) * 32 + col < p.N) { __stcg(srow + i * 32, cs0[i]); __stcg(srow + i * 32 + p.N, cs1[i]); }
+                if (n0 + (cbeg + i) * 32 + col < p.N && (!PAIR || (int)((unsigned)Walk::cta() / (unsigned)nt * CL + rank) * 128 < p.M)) { __stcg(srow + i * 32, cs0[i]); __stcg(srow + i * 32 + p.N, cs1[i]); }
         }
         if (p.tma_store && lane == 0) tma_store_wait_read<0>();   // the slabs stay allocated until the last store has read them
     }
     TC_PROF_FLUSH();
     tc_fence_before();
-    __syncthreads();
-    if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem_base, L::TMEM_COLS); }
+    __syncwarp();
+    if constexpr (PAIR) cluster_sync();          // nothing arrives at, or reads, a CTA that has left
+    else __syncthreads();
+    if (warp == 1) { tc_fence_after(); tmem_dealloc<PAIR>(tmem_base, L::TMEM_COLS); }
 }
 
 // Second stage of a forward launch with a split K loop: the partial tiles of a row added in split order, the epilogue
@@ -1984,29 +2043,32 @@ static size_t filter_split_bytes(const Geo& g, int pass)
 // GEMM rows of a weight gradient: (tap, channel up to a multiple of 32), or the columns of the lowered matrix.
 static int64_t wgrad_rows(const Geo& g) { return lowered_ok(g) ? lowered_kp(g) : (int64_t)g.kh * g.kw * round32(g.ci); }
 
-struct WgradPlan { int splits, kblocks, bn; };
+struct WgradPlan { int splits, kblocks, bn; bool pair; };
 // The pixel axis is cut into `splits` ranges of `kblocks` 32-pixel blocks; tiles x splits work items run on one
 // persistent CTA per SM.  The split count minimises a cost in k-block units: rounds of the CTA grid x (k-blocks per
 // item + a fixed per-item cost for pipeline fill, drain and the partial-tile store) + the second-stage reduce, whose
-// traffic grows with the split count.
+// traffic grows with the split count.  Pairs of CTAs (256 rows) take 0.88 of the time a k-block and 1.5 k-blocks more an item, and are taken
+// where that is 2 % less: 64x14x14 256->256 3x3 60.5 -> 56.0 us, 32x56x56 128->256 5x5/2 (NCHW) 232 -> 196; with nine row
+// tiles, ten in pairs, 64x28x28 128->128 3x3 62.5 / 64.4 us.
 static WgradPlan wgrad_plan(const Geo& g)
 {
     WgradPlan pl;
     pl.bn = g.co <= 64 ? 64 : 128;
     const int64_t Krows = wgrad_rows(g);
-    const int64_t tiles = ((Krows + 127) / 128) * ((g.co + pl.bn - 1) / pl.bn);
     const int64_t blocks = (g.M + 31) / 32;
     const double reduce_per_split = (double)Krows * g.co * 4.0 / 5e12 / 0.6e-6;   // k-block units (0.6 us each)
-    double best = 0.0;
-    const int64_t G = tc_sm_count();
-    pl.splits = 1; pl.kblocks = (int)blocks;
-    for (int64_t s = 1; s <= 512 && s <= blocks; s++) {
-        const int64_t kb = (blocks + s - 1) / s;
-        if ((blocks + kb - 1) / kb != s) continue;       // same k-blocks per split as a smaller count
-        if (kb < 4 && s > 1) break;
-        const int64_t rounds = (tiles * s + G - 1) / G;
-        const double cost = (double)rounds * (double)(kb + 6) + (double)s * reduce_per_split;
-        if (s == 1 || cost < best) { best = cost; pl.splits = (int)s; pl.kblocks = (int)kb; }
+    double best = 1e30;
+    pl.splits = 1; pl.kblocks = (int)blocks; pl.pair = false;
+    for (int cl = 1; cl <= (g.fine || pl.bn == 64 || Krows <= 128 ? 1 : 2); cl++) {
+        const int64_t G = tc_sm_count() / cl, tiles = ((Krows + 128 * cl - 1) / (128 * cl)) * ((g.co + pl.bn - 1) / pl.bn);
+        for (int64_t s = 1; s <= 512 && s <= blocks; s++) {
+            const int64_t kb = (blocks + s - 1) / s;
+            if ((blocks + kb - 1) / kb != s) continue;       // same k-blocks per split as a smaller count
+            if (kb < 4 && s > 1) break;
+            const int64_t rounds = (tiles * s + G - 1) / G;
+            const double cost = (double)rounds * (cl == 2 ? 0.88 * (double)kb + 7.5 : (double)kb + 6) + (double)s * reduce_per_split;
+            if (cost < (cl == 2 && !pl.pair ? 0.98 : 1.0) * best) { best = cost; pl.splits = (int)s; pl.kblocks = (int)kb; pl.pair = cl == 2; }
+        }
     }
     return pl;
 }
@@ -2049,15 +2111,16 @@ static size_t tc_workspace_bytes_nhwc(const Geo& g, int pass)
     return lowered + (sums > partials ? sums : partials);
 }
 
-template <int MODE, int BN, int STAGES, bool SK, int SLABS, int BSRC, int STREAM = 0, bool MULTI = false, int RESKB = 0, bool FINE = false, bool BOTH = false>
+template <int MODE, int BN, int STAGES, bool SK, int SLABS, int BSRC, int STREAM = 0, bool MULTI = false, int RESKB = 0, bool FINE = false, bool BOTH = false, bool PAIR = false>
 static int launch_tc(const CUtensorMap& ma, const CUtensorMap& mb0, const CUtensorMap& mb1, const CUtensorMap& mo, const TcParams& p, int splits, cudaStream_t st,
                      const CUtensorMap* ma3 = nullptr)
 {
-    using L = TcSmem<BN, STAGES, SLABS, tc_drain_warps<STREAM>(), RESKB>;
+    using L = TcSmem<BN, STAGES, SLABS, tc_drain_warps<STREAM>(), RESKB, PAIR>;
+    constexpr int CL = PAIR ? 2 : 1, ROWS = 128 * CL;
     static PerDeviceOnce attr;
     {
         cudaError_t e = attr.run([] {
-            const auto kernel = conv_tc_kernel<MODE, BN, STAGES, SK, SLABS, BSRC, STREAM, MULTI, RESKB, FINE, BOTH>;
+            const auto kernel = conv_tc_kernel<MODE, BN, STAGES, SK, SLABS, BSRC, STREAM, MULTI, RESKB, FINE, BOTH, PAIR>;
             if (tc_b_warps<MODE, BSRC, STREAM, RESKB, BOTH>()) {       // the roles' shares must add up to what the launch brings
                 cudaFuncAttributes a;
                 const cudaError_t r = cudaFuncGetAttributes(&a, kernel);
@@ -2069,29 +2132,36 @@ static int launch_tc(const CUtensorMap& ma, const CUtensorMap& mb0, const CUtens
         if (e != cudaSuccess) { set_cuda_error(e, "cudaFuncSetAttribute(conv_tc_kernel)"); return B2C_ERR_CUDA; }
     }
     const int sm_count = tc_sm_count();
-    int64_t tiles = MULTI ? p.cls_tile0[p.ncls] : (int64_t)((p.M + 127) / 128) * ((p.N + BN - 1) / BN) * splits;
+    int64_t tiles = MULTI ? p.cls_tile0[p.ncls] : (int64_t)((p.M + ROWS - 1) / ROWS) * ((p.N + BN - 1) / BN) * splits;
     if (tiles > 0x7fffffffLL) return B2C_ERR_TOO_LARGE;
     TcParams q = p;
     q.splits = splits;
-    const int nt_ = (p.N + BN - 1) / BN, mt_ = (p.M + 127) / 128;
+    const int nt_ = (p.N + BN - 1) / BN, mt_ = (p.M + ROWS - 1) / ROWS;
     q.f_nt = FastDiv(nt_); q.f_mt = FastDiv(mt_); q.f_plane = FastDiv(nt_ * mt_); q.f_pq = FastDiv(p.P * p.Q); q.f_q = FastDiv(p.Q);
     q.f_cb = FastDiv(p.cblocks); q.f_s = FastDiv(p.S); q.f_c = FastDiv(p.C);
 #ifdef B2C_TC_DEV
     { const char* e = getenv("B2C_TC_DBG"); q.dbg = e ? atoi(e) : 0; }
 #endif
-    int grid = q.sk ? sm_count : (int)(tiles < sm_count ? tiles : sm_count);     // one persistent CTA per SM
+    const int most = sm_count / CL;
+    int grid = q.sk ? most : (int)(tiles < most ? tiles : most);                    // one persistent CTA per SM
     if ((q.stats && q.stats_cta) || RESKB) grid -= grid % ((p.N + BN - 1) / BN);    // a CTA keeps its column tile
-    launch_pdl(conv_tc_kernel<MODE, BN, STAGES, SK, SLABS, BSRC, STREAM, MULTI, RESKB, FINE, BOTH>, grid, tc_threads<MODE, BSRC, STREAM, RESKB, BOTH>(), L::TOTAL, st, ma, mb0, mb1, mo, ma3 ? *ma3 : ma, q);
+    grid *= CL;
+    launch_pdl_cluster(CL, conv_tc_kernel<MODE, BN, STAGES, SK, SLABS, BSRC, STREAM, MULTI, RESKB, FINE, BOTH, PAIR>, grid, tc_threads<MODE, BSRC, STREAM, RESKB, BOTH>(), L::TOTAL, st, ma, mb0, mb1, mo, ma3 ? *ma3 : ma, q);
     return check_launch("conv_tc_kernel");
 }
 
 template <int BSRC>
-static int dispatch_fwd(int bn, bool fine, const CUtensorMap& ma, const CUtensorMap& mb0, const CUtensorMap& mb1, const CUtensorMap& mo, const TcParams& p, cudaStream_t st)
+static int dispatch_fwd(int bn, bool fine, bool pair, const CUtensorMap& ma, const CUtensorMap& mb0, const CUtensorMap& mb1, const CUtensorMap& mo, const TcParams& p, cudaStream_t st)
 {
     if (fine) {
         const int splits = p.kper ? (p.kblocks + p.kper - 1) / p.kper : 1;
         if (bn == 64) return launch_tc<TCM_FWD, 64, 6, false, 2, BSRC, 0, false, 0, true>(ma, mb0, mb1, mo, p, splits, st);
         return launch_tc<TCM_FWD, 128, 4, false, 2, BSRC, 0, false, 0, true>(ma, mb0, mb1, mo, p, splits, st);
+    }
+    if (pair) {
+        const int splits = p.kper ? (p.kblocks + p.kper - 1) / p.kper : 1;
+        if (p.sk) return launch_tc<TCM_FWD, 128, 6, true, 2, BSRC, 0, false, 0, false, false, true>(ma, mb0, mb1, mo, p, 1, st);
+        return launch_tc<TCM_FWD, 128, 6, false, 2, BSRC, 0, false, 0, false, false, true>(ma, mb0, mb1, mo, p, splits, st);
     }
     if (p.sk) {
         if (bn == 64) return launch_tc<TCM_FWD, 64, 6, true, 2, BSRC>(ma, mb0, mb1, mo, p, 1, st);
@@ -2132,12 +2202,13 @@ static int dispatch_fwd(int bn, bool fine, const CUtensorMap& ma, const CUtensor
     return launch_tc<TCM_FWD, 128, 4, false, 2, BSRC>(ma, mb0, mb1, mo, p, 1, st);
 }
 
-static int dispatch_wgrad(int bn, bool fine, const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mo, const TcParams& p, int splits, cudaStream_t st)
+static int dispatch_wgrad(int bn, bool fine, bool pair, const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mo, const TcParams& p, int splits, cudaStream_t st)
 {
     if (fine) {
         if (bn == 64) return launch_tc<TCM_WGRAD, 64, 6, false, 2, TCB_SPLIT, 0, false, 0, true>(ma, mb, mb, mo, p, splits, st);
         return launch_tc<TCM_WGRAD, 128, 4, false, 2, TCB_SPLIT, 0, false, 0, true>(ma, mb, mb, mo, p, splits, st);
     }
+    if (pair) return launch_tc<TCM_WGRAD, 128, 6, false, 2, TCB_SPLIT, 0, false, 0, false, false, true>(ma, mb, mb, mo, p, splits, st);
     if (bn == 64) return launch_tc<TCM_WGRAD, 64, 6, false, 2, TCB_SPLIT>(ma, mb, mb, mo, p, splits, st);
     return launch_tc<TCM_WGRAD, 128, 4, false, 2, TCB_SPLIT>(ma, mb, mb, mo, p, splits, st);
 }
@@ -2203,11 +2274,11 @@ struct StatsOut { float* sums; };
 // balanced mode's scratch
 // because tiles x splits is at most one CTA per SM.  Narrow tiles only pay where the wide ones leave the chip idle (single
 // images, late layers of small batches).
-struct FwdPlan { int bn; bool sk; int kper; };
-static FwdPlan fwd_plan(int64_t M, int N, int64_t kblocks, bool may_share, bool fine = false)
+struct FwdPlan { int bn; bool sk; int kper; bool pair; };
+static FwdPlan fwd_plan(int64_t M, int N, int64_t kblocks, bool may_share, bool may_pair, bool fine = false)
 {
     const int G = tc_sm_count();
-    FwdPlan best{128, false, 0};
+    FwdPlan best{128, false, 0, false};
     double cost = 1e30;
     // A range shorter than a chunk is a shorter sum in tensor memory, and a more accurate one (1.1 against 1.4e-6 at 5 and 8
     // k-blocks of a 256-channel 5x5 layer): launches that balanced ranges would cut into less than a chunk per CTA are
@@ -2219,7 +2290,7 @@ static FwdPlan fwd_plan(int64_t M, int N, int64_t kblocks, bool may_share, bool 
         const int64_t tiles = ((M + 127) / 128) * ((N + bn - 1) / bn), rounds = (tiles + G - 1) / G;
         const bool one = rounds == 1;
         const double kb = bn == 128 ? (one ? (fine ? 0.6 : 0.5) : 0.45) : one ? (fine ? 0.45 : 0.36) : fine ? 0.42 : 0.33, drain = bn == 128 ? 2.0 : 1.0;
-        auto offer = [&](double c, bool sk, int kper) { if (c < (one ? 0.98 : 0.95) * cost) { best = FwdPlan{bn, sk, kper}; cost = c; } };
+        auto offer = [&](double c, bool sk, int kper) { if (c < (one ? 0.98 : 0.95) * cost) { best = FwdPlan{bn, sk, kper, false}; cost = c; } };
         if (!short_sums) offer((double)(rounds * kblocks) * kb + (one && bn == 128 ? 2.8 : drain), false, 0);
         if (!may_share) continue;
         const double shared = (double)G / (double)tiles;         // CTAs on one tile
@@ -2231,6 +2302,21 @@ static FwdPlan fwd_plan(int64_t M, int N, int64_t kblocks, bool may_share, bool 
             if ((kblocks + kper - 1) / kper == s) offer((double)kper * kb + (bn == 128 ? 3.5 : 2.7) + (double)s * (double)M * (N > 64 ? N : 64) * 8e-6 * 0.16, false, (int)kper);
         }
     }
+    // The same cut for pairs of CTAs.  What they gain is contention (see PAIR at conv_tc_kernel): 0.06 us a k-block with every SM at
+    // work, in proportion less in a launch that leaves SMs idle; the clusters' start and end cost 0.6 us (1.2 where a layer runs again
+    // and again on operands that L2 holds; with 1.2 a step of ResNet-50, 32 images, NCHW, and of VGG at 32 pixels took 0.8 and 1 % longer),
+    // and the rows that fill up a column's last pair what any others do.  64x28x28 512->256 1x1 (6 rounds of 16 k-blocks) 65.8 us by single CTAs, 57.2 by pairs;
+    // 64x28x28 128->128 3x3 (3 of 36) 63.4 / 57.0; 64x14x14 256->256 3x3 (balanced) 67.8 / 63.7; 64x16x16 128->128 3x3 (1 of 36) 27.1 / 26.1;
+    // on few SMs 3x26x45 128->128 3x3 (28 tiles) 21.4 / 22.2.  Filters as hi and lo copies (lowered inputs) gain nothing: 35x47x47 6->512
+    // 7x7/2 72.4 / 74.0.
+    if (may_pair && best.bn == 128 && !fine && M > 128 && (best.kper ? best.kper : kblocks) >= 12) {
+        const int64_t nt = (N + 127) / 128, splits = best.kper ? (kblocks + best.kper - 1) / best.kper : 1;
+        const int64_t tiles = (M + 127) / 128 * nt * splits, pairs = (M + 255) / 256 * nt * splits, len = best.kper ? best.kper : kblocks;
+        const double kb = tiles <= G ? 0.5 : 0.45, busy = tiles < G && !best.sk ? (double)tiles / G : 1.0;
+        const double whole = best.sk ? (double)(tiles * len) / G : (double)((tiles + G - 1) / G * len);
+        const double paired = best.sk ? (double)(pairs * len) / (G / 2) : (double)((pairs + G / 2 - 1) / (G / 2) * len);
+        best.pair = (!best.kper || pairs <= G / 2) && paired * (kb - 0.06 * busy) + 0.6 < whole * kb;
+    }
     return best;
 }
 
@@ -2239,12 +2325,14 @@ static FwdPlan fwd_plan(int64_t M, int N, int64_t kblocks, bool may_share, bool 
 static int64_t fwd_stats_rows(int64_t M, int N, int64_t kblocks, bool may_balance, bool* by_cta)
 {
     const int G = tc_sm_count();
-    const FwdPlan plan = fwd_plan(M, N, kblocks, may_balance);
-    const int64_t nt = (N + plan.bn - 1) / plan.bn, tiles = ((M + 127) / 128) * nt;
-    const int64_t grid = tiles < G ? tiles : G;
+    const FwdPlan plan = fwd_plan(M, N, kblocks, may_balance, may_balance);
+    const int64_t cl = plan.pair ? 2 : 1, most = G / cl;
+    const int64_t nt = (N + plan.bn - 1) / plan.bn, tiles = ((M + 128 * cl - 1) / (128 * cl)) * nt;
+    const int64_t grid = tiles < most ? tiles : most;
     const bool cta = nt <= grid && !plan.sk && !plan.kper;
     if (by_cta) *by_cta = cta;
-    return cta ? (grid / nt) * 4 : (M + 31) / 32;
+    const int64_t rows = (grid / nt) * cl, most_rows = (M + 127) / 128;
+    return cta ? (rows < most_rows ? rows : most_rows) * 4 : (M + 31) / 32;
 }
 // Stride-2 data gradient of a 1x1 filter: the launch writes class (0, 0) and the zeros of the other three (TcParams::zfill).
 struct ZeroFill { int W, H; int64_t off_w, off_h; };
@@ -2301,23 +2389,26 @@ static int run_fwd(const FwdLaunch& f, const void* act, const void* w, PrepParam
     unsigned int* sk_bank = tc_sm_count() * 4 <= TC_SYNC_FLAGS ? tc_sync_bank(st) : nullptr;
     if (sk_bank) sk_flags = (int*)sk_bank;
     const bool room = base + 2 * fbytes + sk_bytes() <= (uintptr_t)ws + ws_bytes;
-    const FwdPlan plan = fwd_plan((int64_t)f.n * f.P * f.Q, f.N, (int64_t)f.kh * f.kw * cblocks, !filters_ready && room && !zf, f.fine);
-    const int BN = plan.bn, sk = plan.sk, kper = plan.kper;
+    const FwdPlan plan = fwd_plan((int64_t)f.n * f.P * f.Q, f.N, (int64_t)f.kh * f.kw * cblocks, !filters_ready && room && !zf, !filters_ready, f.fine);
+    const int BN = plan.bn, sk = plan.sk, kper = plan.kper, BNL = plan.pair ? BN / 2 : BN;
     // The filter itself serves as the B operand when its layout allows a tensor map over it (the channel axis
     // that is contiguous decides K-major or MN-major); otherwise hi/lo copies in the GEMM layout are written first.
     // Splitting the B tile in shared memory costs a long launch about 4 % (measured on a 0.9 ms layer), the split
-    // kernel about 5 us: the copies win beyond roughly 125 us of work (0.6 us per k-block on 148 SMs).
+    // kernel about 5 us: the copies win beyond roughly 125 us of work (0.6 us per k-block on 148 SMs).  Not where CTAs work in pairs
+    // and split half of the tile each (16x56x56 256->256 3x3 210 us, with copies 236), with the filter rounded as in the copies.
     int bsrc = TCB_SPLIT;
     CUtensorMap ma, mbh, mbl;
     const bool long_launch = (((int64_t)f.n * f.P * f.Q + 127) / 128) * ((f.N + BN - 1) / BN) * f.kh * f.kw * cblocks > 30000;
-    if (!filters_ready && !long_launch) {
+    const bool copies = long_launch && !plan.pair;
+    pp.round = pp.round || long_launch;
+    if (!filters_ready && !copies) {
         const int rc = kmajor_filter_copy(pp, w, w_hi, st);
         if (rc < 0) return rc;
     }
-    if (!filters_ready && !long_launch && ((uintptr_t)w & 15) == 0 && pp.s_r == (int64_t)pp.Sreal * pp.s_s && (pp.s_s * 4) % 16 == 0) {
+    if (!filters_ready && !copies && ((uintptr_t)w & 15) == 0 && pp.s_r == (int64_t)pp.Sreal * pp.s_s && (pp.s_s * 4) % 16 == 0) {
         const uint64_t taps = (uint64_t)pp.Rreal * pp.Sreal;
         if (pp.s_c == 1 && (pp.s_row * 4) % 16 == 0 &&
-            make_map_filter(&mbh, w, (uint64_t)pp.C, taps, (uint64_t)pp.rows, (uint64_t)pp.s_s * 4, (uint64_t)pp.s_row * 4, BN, CU_TENSOR_MAP_SWIZZLE_128B))
+            make_map_filter(&mbh, w, (uint64_t)pp.C, taps, (uint64_t)pp.rows, (uint64_t)pp.s_s * 4, (uint64_t)pp.s_row * 4, BNL, CU_TENSOR_MAP_SWIZZLE_128B))
             bsrc = TCB_RAW_K;
         else if (pp.s_row == 1 && (pp.s_c * 4) % 16 == 0 &&
                  make_map_filter(&mbh, w, (uint64_t)pp.rows, taps, (uint64_t)pp.C, (uint64_t)pp.s_s * 4, (uint64_t)pp.s_c * 4, 32, CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B))
@@ -2335,7 +2426,7 @@ static int run_fwd(const FwdLaunch& f, const void* act, const void* w, PrepParam
         if (e != cudaSuccess) { set_cuda_error(e, "cudaMemsetAsync(balanced-mode flags)"); return B2C_ERR_CUDA; }
     }
     if (!make_map_im2col(&ma, act, f.n, f.ah, f.aw, f.C, f.ap, f.low_h, f.low_w, f.cnt_h, f.cnt_w, f.str_h, f.str_w, 128)) return B2C_ERR_UNSUPPORTED;
-    if (bsrc == TCB_SPLIT && (!make_map_2d(&mbh, w_hi, f.N, K, K, BN) || !make_map_2d(&mbl, w_lo, f.N, K, K, BN))) return B2C_ERR_UNSUPPORTED;
+    if (bsrc == TCB_SPLIT && (!make_map_2d(&mbh, w_hi, f.N, K, K, BNL) || !make_map_2d(&mbl, w_lo, f.N, K, K, BNL))) return B2C_ERR_UNSUPPORTED;
     TcParams p{};
     p.M = f.n * f.P * f.Q; p.N = f.N; p.P = f.P; p.Q = f.Q;
     p.C = f.C; p.cblocks = cblocks; p.ktail = (f.C - (cblocks - 1) * 32 + 7) / 8; p.kblocks = f.kh * f.kw * p.cblocks; p.S = f.kw;
@@ -2355,7 +2446,7 @@ static int run_fwd(const FwdLaunch& f, const void* act, const void* w, PrepParam
     CUtensorMap mo = mbh;
     p.tma_store = 0;
     const int splits = kper ? (p.kblocks + kper - 1) / kper : 1;
-    const int64_t mrows = (int64_t)((p.M + 127) / 128) * 128;
+    const int64_t trows = plan.pair ? 256 : 128, mrows = (p.M + trows - 1) / trows * trows;
     if (kper) {
         if (!make_map_out(&mo, sk_partial, 0, (uint64_t)(splits * mrows), (uint64_t)round4(f.N), (uint64_t)round4(f.N))) return B2C_ERR_UNSUPPORTED;
         p.tma_store = 1; p.kper = kper; p.epi = 0;
@@ -2372,9 +2463,9 @@ static int run_fwd(const FwdLaunch& f, const void* act, const void* w, PrepParam
         fwd_stats_rows(p.M, p.N, p.kblocks, !filters_ready, &by_cta);
         p.stats_cta = by_cta ? 1 : 0;       // by_cta implies whole tiles
     }
-    const int rc = bsrc == TCB_RAW_K ? dispatch_fwd<TCB_RAW_K>(BN, f.fine, ma, mbh, mbl, mo, p, st)
-                 : bsrc == TCB_RAW_MN ? dispatch_fwd<TCB_RAW_MN>(BN, f.fine, ma, mbh, mbl, mo, p, st)
-                 : dispatch_fwd<TCB_SPLIT>(BN, f.fine, ma, mbh, mbl, mo, p, st);
+    const int rc = bsrc == TCB_RAW_K ? dispatch_fwd<TCB_RAW_K>(BN, f.fine, plan.pair, ma, mbh, mbl, mo, p, st)
+                 : bsrc == TCB_RAW_MN ? dispatch_fwd<TCB_RAW_MN>(BN, f.fine, plan.pair, ma, mbh, mbl, mo, p, st)
+                 : dispatch_fwd<TCB_SPLIT>(BN, f.fine, plan.pair, ma, mbh, mbl, mo, p, st);
     if (rc || !kper) return rc;
     FinishParams fp{p.M, p.N, p.P, p.Q, splits, round4(f.N), mrows * round4(f.N), sk_partial, out, f.o_sn, f.o_sh, f.o_sw,
                     p.bias, p.mean, p.inv_std, p.gamma, p.beta, relu, stats ? stats->sums : nullptr};
@@ -2480,11 +2571,20 @@ static int tc_dgrad_classes_one_launch(const Geo& g, const WStride& wsd, bool b_
     if (s_r != (int64_t)g.kw * s_s || (s_s * 4) % 16) return 1;
     // narrow tiles where the wide ones would leave half of the chip idle (see fwd_plan)
     const int BN = g.ci <= 64 || ((int64_t)g.n * g.h * g.w + 127) / 128 * ((g.ci + 127) / 128) * 2 <= tc_sm_count() ? 64 : 128;
+    // Pairs of CTAs take 0.87 of the time: unless the rows that fill up the classes' last pairs are more than that (56x56 128->128 3x3/2 of
+    // 64 images 92 -> 82 us, 32x56x56 128->256 5x5/2 246 -> 200).
+    int64_t whole[2] = {};                    // row tiles of all classes in 128 rows and in pairs of 256
+    for (int i = 0; i < ncls; i++) {
+        const int64_t m = (int64_t)g.n * cls[i].a.out_cnt * cls[i].b.out_cnt;
+        whole[0] += (m + 127) / 128; whole[1] += (m + 255) / 256 * 2;
+    }
+    const bool pair = !g.fine && BN == 128 && (double)whole[1] * 0.87 < (double)whole[0];
+    const int BNL = pair ? BN / 2 : BN, rows = pair ? 256 : 128;
     const uint64_t taps = (uint64_t)g.kh * g.kw;
     CUtensorMap mb;
     int bsrc;
     if (s_c == 1 && (s_row * 4) % 16 == 0 &&
-        make_map_filter(&mb, w, (uint64_t)g.co, taps, (uint64_t)g.ci, (uint64_t)s_s * 4, (uint64_t)s_row * 4, BN, CU_TENSOR_MAP_SWIZZLE_128B))
+        make_map_filter(&mb, w, (uint64_t)g.co, taps, (uint64_t)g.ci, (uint64_t)s_s * 4, (uint64_t)s_row * 4, BNL, CU_TENSOR_MAP_SWIZZLE_128B))
         bsrc = TCB_RAW_K;
     else if (s_row == 1 && (s_c * 4) % 16 == 0 &&
              make_map_filter(&mb, w, (uint64_t)g.ci, taps, (uint64_t)g.co, (uint64_t)s_s * 4, (uint64_t)s_c * 4, 32, CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B))
@@ -2507,7 +2607,7 @@ static int tc_dgrad_classes_one_launch(const Geo& g, const WStride& wsd, bool b_
         p.cls_kblocks[i] = ca.cnt * cb.cnt * p.cblocks; p.cls_S[i] = cb.cnt;
         p.cls_low_h[i] = ca.dmin; p.cls_low_w[i] = cb.dmin; p.cls_r0[i] = ca.r0; p.cls_s0[i] = cb.r0;
         p.cls_out[i] = ((int64_t)cls[i].ia * g.w + cls[i].ib) * g.xp;
-        tiles += (int64_t)((p.cls_M[i] + 127) / 128) * nt;
+        tiles += (int64_t)((p.cls_M[i] + rows - 1) / rows) * nt;
         if (tiles > 0x7fffffffLL) return 1;
     }
     for (int i = ncls; i < 4; i++) ma[i] = ma[0];
@@ -2525,6 +2625,10 @@ static int tc_dgrad_classes_one_launch(const Geo& g, const WStride& wsd, bool b_
         }
         if (BN == 64) return launch_tc<TCM_FWD, 64, 6, false, 2, TCB_RAW_MN, 0, true, 0, true>(ma[0], mb, ma[1], ma[2], p, 1, st, &ma[3]);
         return launch_tc<TCM_FWD, 128, 4, false, 2, TCB_RAW_MN, 0, true, 0, true>(ma[0], mb, ma[1], ma[2], p, 1, st, &ma[3]);
+    }
+    if (pair) {
+        if (bsrc == TCB_RAW_K) return launch_tc<TCM_FWD, 128, 6, false, 2, TCB_RAW_K, 0, true, 0, false, false, true>(ma[0], mb, ma[1], ma[2], p, 1, st, &ma[3]);
+        return launch_tc<TCM_FWD, 128, 6, false, 2, TCB_RAW_MN, 0, true, 0, false, false, true>(ma[0], mb, ma[1], ma[2], p, 1, st, &ma[3]);
     }
     if (bsrc == TCB_RAW_K) {
         if (BN == 64) return launch_tc<TCM_FWD, 64, 6, false, 2, TCB_RAW_K, 0, true>(ma[0], mb, ma[1], ma[2], p, 1, st, &ma[3]);
@@ -2669,11 +2773,11 @@ static int tc_wgrad_nhwc(const Geo& g, const void* x, const void* dy, void* dw, 
         (!db || (g.yp == g.co && rest >= channel_sum_workspace_bytes((int)g.M, g.co, 1))) &&
         make_map_out(&mo, dw, 1, (uint64_t)g.ci, (uint64_t)g.co, (uint64_t)wsd.sc)) {
         p.db_partial = nullptr;
-        const int rc = dispatch_wgrad(pl.bn, g.fine, ma, mb, mo, p, 1, st);
+        const int rc = dispatch_wgrad(pl.bn, g.fine, pl.pair, ma, mb, mo, p, 1, st);
         if (rc || !db) return rc;
         return channel_sum(B2C_F32, B2C_LAYOUT_NHWC, (int)g.M, g.co, 1, dy, db, partial, rest, st);
     }
-    int rc = dispatch_wgrad(pl.bn, g.fine, ma, mb, mo, p, pl.splits, st);
+    int rc = dispatch_wgrad(pl.bn, g.fine, pl.pair, ma, mb, mo, p, pl.splits, st);
     if (rc) return rc;
     WgradReduceParams rp{Krows, g.co, low ? g.ci : Cp, g.kw, pl.splits, wsd.sk, wsd.sc, wsd.sr, wsd.ss, low ? (int)g.K : Krows, g.ci, Np, pl.splits * 4};
     const int db_row = db ? 1 : 0, taps = g.kh * g.kw;

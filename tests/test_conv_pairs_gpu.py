@@ -1,0 +1,94 @@
+"""Launches whose CTAs work in pairs on 256 rows (conv_tc_kernel, PAIR): row tiles that do not fill the last pair, a last column
+tile of few columns, every filter layout, whole tiles, balanced ranges, split K loops, the classes of a strided input gradient,
+the weight gradient, batch sums. GPU."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+from oracle import conv_oracle as co
+from pydtnn_b200 import _lib
+from tests.gpu_util import DEV, assert_parity, make_desc, stream, workspace
+
+pytestmark = pytest.mark.gpu
+
+# (n, h, w, ci, co, k, stride): what the forward pass (input gradient) is cut into on 148 SMs, row tiles of 128
+SHAPES = [
+    (13, 41, 41, 128, 200, 3, 1),       # whole tiles in several rounds, 171 row tiles (the last pair has one), second column tile of 72
+    (55, 17, 17, 128, 128, 3, 1),       # whole tiles in one round, 125 row tiles
+    (63, 14, 14, 256, 256, 3, 1),       # balanced ranges, 97 row tiles
+    (50, 4, 4, 512, 512, 3, 1),         # split K loops, 7 row tiles (the last of 32 rows)
+    (5, 56, 56, 128, 256, 5, 2),        # input gradient: four classes of 31 row tiles
+    (20, 27, 27, 96, 200, 5, 1),        # weight gradient: 19 row tiles of (tap, channel), ranges of the pixels, second column tile of 72
+    (3, 45, 33, 256, 384, 1, 1),        # weight gradient of a 1x1 layer, two pairs
+]
+
+
+def _layer(shape, layout, w_layout):
+    n, h, w, ci, cout, k, st = shape
+    g = co.Geom(n, h, w, ci, cout, k, k, k // 2, k // 2, st, st)
+    desc = make_desc(g, layout, np.float32, w_layout)
+    gen = torch.Generator(device=DEV).manual_seed(ci + cout)
+    rnd = lambda *s: torch.randn(s, device=DEV, generator=gen)
+    x, dy, b = rnd(n, ci, h, w), rnd(n, cout, g.ho, g.wo), rnd(cout)
+    wt = rnd(cout, ci, k, k) * float(np.sqrt(2.0 / (ci * k * k)))
+    act = (lambda t: t.permute(0, 2, 3, 1).contiguous()) if layout == "NHWC" else (lambda t: t)
+    order = {"KCRS": (0, 1, 2, 3), "KRSC": (0, 2, 3, 1), "CRSK": (1, 2, 3, 0)}[w_layout]
+    return g, desc, (x, dy, wt, b), (act(x), act(dy), wt.permute(*order).contiguous()), act, order
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("layout,w_layout", [("NHWC", "KRSC"), ("NHWC", "CRSK"), ("NCHW", "KCRS")])
+def test_pairs_of_ctas(shape, layout, w_layout):
+    n, h, w, ci, cout, k, st = shape
+    L = _lib.lib()
+    g, desc, (x, dy, wt, b), (xd, dyd, wd), act, order = _layer(shape, layout, w_layout)
+    ws = workspace(desc)
+    d = ctypes.byref(desc)
+
+    def passes():
+        out = [torch.full_like(t, float("nan")) for t in (dyd, wd, b, xd)]
+        y, dw, db, dx = out
+        _lib.check(L.b2c_conv_fprop(d, xd.data_ptr(), wd.data_ptr(), b.data_ptr(), None, 1, y.data_ptr(), ws.data_ptr(), ws.numel(), stream()))
+        _lib.check(L.b2c_conv_wgrad(d, xd.data_ptr(), dyd.data_ptr(), dw.data_ptr(), db.data_ptr(), ws.data_ptr(), ws.numel(), stream()))
+        _lib.check(L.b2c_conv_dgrad(d, dyd.data_ptr(), wd.data_ptr(), dx.data_ptr(), ws.data_ptr(), ws.numel(), stream()))
+        return out
+
+    y, dw, db, dx = passes()
+    x64, w64, dy64 = (t.double() for t in (x, wt, dy))
+    x64.requires_grad_(), w64.requires_grad_()
+    y64 = torch.nn.functional.conv2d(x64, w64, b.double(), stride=st, padding=k // 2)
+    y64.backward(dy64)
+    refs = (act(torch.relu(y64.detach())), w64.grad.permute(*order), dy64.sum((0, 2, 3)), act(x64.grad))
+    for name, got, ref in zip(("y", "dw", "db", "dx"), (y, dw, db, dx), refs):
+        assert_parity(got.cpu().numpy(), ref.cpu().numpy(), np.float32, f"{name} {shape} {layout} {w_layout}")
+    for _ in range(5):
+        for first, again in zip((y, dw, db, dx), passes()):
+            assert torch.equal(first, again)
+    status = ctypes.c_int()
+    _lib.check(L.b2c_check_device_status(ctypes.byref(status)))
+    assert status.value == 0
+
+
+@pytest.mark.parametrize("shape", [(55, 17, 17, 128, 128, 3, 1), (13, 41, 41, 128, 200, 3, 1), (63, 14, 14, 256, 256, 3, 1)])
+def test_batch_sums_of_pairs(shape):
+    """The sums a pair leaves for a batch norm, and that the last pair of an odd count of row tiles leaves none for rows there are not."""
+    L = _lib.lib()
+    g, desc, _, (xd, dyd, wd), _, _ = _layer(shape, "NHWC", "KRSC")
+    cout = shape[4]
+    nbytes = L.b2c_conv_stats_bytes(ctypes.byref(desc))
+    rows, pixels = nbytes // (8 * cout), g.n * g.ho * g.wo
+    assert nbytes and rows <= (pixels + 127) // 128 * 4
+    stats = torch.full((rows + 8, 2, cout), float("nan"), device=DEV)
+    y = torch.full_like(dyd, float("nan"))
+    ws = workspace(desc)
+    _lib.check(L.b2c_conv_fprop_stats(ctypes.byref(desc), xd.data_ptr(), wd.data_ptr(), None, y.data_ptr(), stats.data_ptr(), nbytes,
+                                      ws.data_ptr(), ws.numel(), stream()))
+    assert bool(torch.isnan(stats[rows:]).all())
+    v = y.double().view(-1, cout)
+    # a row holds the sums of at most pixels / rows values and a tile's 32 more, one float32 addition each
+    adds = pixels // rows + 64
+    for got, ref, mag in ((stats[:rows, 0], v, v.abs()), (stats[:rows, 1], v * v, v * v)):
+        err = (got.double().sum(0) - ref.sum(0)).abs()
+        assert bool((err <= adds * 2.0 ** -24 * mag.sum(0)).all())
