@@ -40,6 +40,20 @@ inline void launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t s
 {
     launch_pdl_cluster(1, kernel, grid, block, smem, st, static_cast<Args&&>(args)...);
 }
+// Division by a launch constant: q = (n * mul) >> 32 >> shift for 0 <= n < 2^31 (round-up reciprocal: with s = ceil(log2 d) and
+// mul = ceil(2^(32 + s - 1) / d) the error stays below 1 / d for 31-bit n).  A role's start-up and each new tile of the tensor-core
+// convolution took half a dozen integer divisions, 0.3 us before a launch's first load.
+struct FastDiv {
+    uint32_t d, mul; int shift;
+    FastDiv() = default;
+    __host__ explicit FastDiv(uint32_t d_) : d(d_) {
+        int s = 0;
+        while ((1ull << s) < d_) s++;
+        shift = s - 1;
+        mul = d_ == 1 ? 0 : (uint32_t)(((1ull << (31 + s)) + d_ - 1) / d_);
+    }
+    __device__ __forceinline__ int div(int n) const { return d == 1 ? n : (int)(__umulhi((uint32_t)n, mul) >> shift); }
+};
 #endif
 
 inline int check_launch(const char* where) {

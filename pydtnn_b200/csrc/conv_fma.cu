@@ -35,7 +35,7 @@ struct IgemmParams {
     int64_t b_sn;                 // B(k, n) = Bsrc[kinfo.b_off + n*b_sn]
     int64_t c_sn;                 // C(m, n) = Cdst[rowinfo.b_off + n*c_sn]
     int a_lanes_k, b_lanes_k;     // which index runs fastest across lanes when loading A / B
-    int k_chunk, splits;
+    int k_chunk, splits, bn;      // bn: columns of a tile
     int whole, m_whole;           // float64: tiles, and the rows they cover, that take no part in the split
     int relu;
     // Sub-lattices (strided dgrad runs one launch per residue class of the output pixels, each with the taps that
@@ -45,9 +45,24 @@ struct IgemmParams {
     int tap_r0, tap_rs, tap_s0, tap_ss;
     bool small;                   // x (dx), y (dy) with a window's overhang and the filter have fewer than 2^31 elements each
     int lin_h, lin_w;             // dgrad: how far one tap of the (R, S) grid moves the gathered row and column
+    FastDiv f_pq, f_q, f_c, f_s, f_rs;       // float64 kernel (launch_igemm): PQ, Q, C, S, R * S
 };
 
 template <typename T> struct Epilogue { const T *bias, *mean, *inv_std, *gamma, *beta; int relu; };
+// The same of one output channel, whose values are loaded once.
+template <typename T> struct ChannelEpilogue {
+    T bias, mean, inv_std, gamma, beta;
+    bool has_bias, has_bn, relu;
+    __device__ __forceinline__ ChannelEpilogue(const Epilogue<T>& ep, int n)
+        : bias(ep.bias ? ep.bias[n] : T(0)), mean(ep.mean ? ep.mean[n] : T(0)), inv_std(ep.mean ? ep.inv_std[n] : T(0)),
+          gamma(ep.mean ? ep.gamma[n] : T(0)), beta(ep.mean ? ep.beta[n] : T(0)), has_bias(ep.bias), has_bn(ep.mean), relu(ep.relu) {}
+    __device__ __forceinline__ T operator()(T v) const {
+        if (has_bias) v += bias;
+        if (has_bn) { T t = (v - mean) * inv_std; v = t * gamma + beta; }
+        if (relu) v = v > T(0) ? v : T(0);
+        return v;
+    }
+};
 
 template <int MODE> __device__ __forceinline__ Info decode_pix(const IgemmParams& p, int idx, int limit) {
     Info f;
@@ -302,7 +317,7 @@ short_fprop_kernel(IgemmParams p, const float* __restrict__ A, const float* __re
 // mma.m16n8k8 keeps the full FP64 rate (measured 37.0 TFLOP/s on register-resident chains, 35 with the fragment reads of
 // this kernel; the FMA pipe reaches 33) with a sixteenth of the operand reads of 8 x 8 register blocks, which is what held
 // the FMA form of this kernel to 14 TFLOP/s.  One CTA per SM = a 128 x BN tile: eight warps of 64 x 32 (BN = 128) or
-// 32 x 32 (BN = 64) only read fragments and multiply, four more gather k-slices of 16 into a ring of three stages with cp.async,
+// 32 x 32 (BN = 64) only read fragments and multiply, four more gather k-slices of 16 into a ring of stages with cp.async,
 // zero-filled where a tap or an index is out of range.  The roles are separate because a warp issues in order: with the
 // gather's address arithmetic between the products of the same warps the pipe stood idle 30 to 40 % of the time.
 // An address is the sum of a row's and a k's offset, a bound check the sum of their coordinates (DInfo), and pairs of
@@ -312,7 +327,7 @@ short_fprop_kernel(IgemmParams p, const float* __restrict__ A, const float* __re
 // source is contiguous: a row pitch of 4 modulo 16 doubles makes the fragments' (8 x 4) reads conflict-free either way.
 // Consecutive warps lie along M so that a narrow N (whose unused 8-column steps are skipped) still feeds all four
 // sub-partitions.
-constexpr int DG_BK = 16, DG_STAGES = 3, DG_KP = DG_BK + 4, DG_MMA = 256, DG_GATHER = 128, DG_THREADS = DG_MMA + DG_GATHER;
+constexpr int DG_BK = 16, DG_KP = DG_BK + 4, DG_MMA = 256, DG_GATHER = 128, DG_THREADS = DG_MMA + DG_GATHER;
 
 // A GEMM row or a k index: element (row, k) of A lies at off + off and is inside the tensor when the summed coordinates
 // are; boff is a k's offset in B or a row's in C.  With 32-bit offsets it is one 16-byte read.
@@ -321,8 +336,19 @@ template <typename OFF> struct __align__(16) DInfo { OFF off; int d0, d1; OFF bo
 template <int BN> constexpr int dg_tile_doubles() {
     return (128 * DG_KP > DG_BK * 132 ? 128 * DG_KP : DG_BK * 132) + (BN * DG_KP > DG_BK * (BN + 4) ? BN * DG_KP : DG_BK * (BN + 4));
 }
+// Stages of the ring: one is multiplied, one has landed, the others are on their way.  More than these leave less of the SM's memory to
+// the L1 that copies of single doubles want (64 columns, six stages: 7x25x25 512->64 3x3 108 -> 112 us).
+template <int BN> constexpr int dg_stages() { return BN == 128 ? 5 : 4; }
+// The k's of DG_AHEAD slices are decoded at once, one by each gathering thread (slice by slice, by 16 of them with the others waiting, that
+// was half of the 1.3 us a slice of a small launch took), into one of two places in turn.
+constexpr int DG_AHEAD = DG_GATHER / DG_BK;
+// The ring of slices, whose place the output tile takes on its way out: [row][32] of each warp's 32 columns, rows of DG_OUT doubles.
+constexpr int DG_OUT = 34;
+template <int BN> constexpr int dg_ring_doubles() {
+    return dg_stages<BN>() * dg_tile_doubles<BN>() > 128 * (BN / 32) * DG_OUT ? dg_stages<BN>() * dg_tile_doubles<BN>() : 128 * (BN / 32) * DG_OUT;
+}
 template <int BN, typename OFF> constexpr size_t dg_smem_bytes() {
-    return DG_STAGES * (dg_tile_doubles<BN>() * sizeof(double) + DG_BK * sizeof(DInfo<OFF>)) + 128 * sizeof(DInfo<OFF>);
+    return dg_ring_doubles<BN>() * sizeof(double) + (2 * DG_GATHER + 128) * sizeof(DInfo<OFF>);
 }
 template <int N> __device__ __forceinline__ void cp_async_doubles(uint32_t d, const double* src, bool ok) {
     if (N == 2) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(ok ? 16 : 0) : "memory");
@@ -339,8 +365,8 @@ template <typename OFF>
 __device__ __forceinline__ DInfo<OFF> dinfo_pix(const IgemmParams& p, int mode, int idx, int limit) {
     DInfo<OFF> f{0, -B2C_SENTINEL, 0, 0};
     if (idx >= limit) return f;
-    const int n = idx / p.PQ, rem = idx - n * p.PQ;
-    int pp = rem / p.Q, qq = rem - pp * p.Q;
+    const int n = p.f_pq.div(idx), rem = idx - n * p.PQ;
+    int pp = p.f_q.div(rem), qq = rem - pp * p.Q;
     pp = p.pix_h0 + pp * p.pix_hs; qq = p.pix_w0 + qq * p.pix_ws;
     if (mode == MODE_DGRAD) { f.d0 = (pp + p.vpad - p.tap_r0 * p.vdil) / p.vstr; f.d1 = (qq + p.hpad - p.tap_s0 * p.hdil) / p.hstr; }
     else { f.d0 = pp * p.vstr - p.vpad; f.d1 = qq * p.hstr - p.hpad; }
@@ -353,8 +379,10 @@ __device__ __forceinline__ DInfo<OFF> dinfo_tap(const IgemmParams& p, int mode, 
     DInfo<OFF> f{0, -B2C_SENTINEL, 0, 0};
     if (idx >= limit) return f;
     int c, r, s;
-    if (p.tap_c_fast) { c = idx % p.C; const int rs = idx / p.C; r = rs / p.S; s = rs - r * p.S; }
-    else { const int RS = p.R * p.S; c = idx / RS; const int rs = idx - c * RS; r = rs / p.S; s = rs - r * p.S; }
+    int rs;
+    if (p.tap_c_fast) { rs = p.f_c.div(idx); c = idx - rs * p.C; }
+    else { c = p.f_rs.div(idx); rs = idx - c * (p.R * p.S); }
+    r = p.f_s.div(rs); s = rs - r * p.S;
     if (mode == MODE_DGRAD) { f.d0 = -r * p.lin_h; f.d1 = -s * p.lin_w; }
     else { f.d0 = r * p.vdil; f.d1 = s * p.hdil; }
     f.off = (OFF)(c * p.a_sc + f.d0 * p.a_sh + f.d1 * p.a_sw);
@@ -362,10 +390,13 @@ __device__ __forceinline__ DInfo<OFF> dinfo_tap(const IgemmParams& p, int mode, 
     return f;
 }
 
-// Named barriers: DG_FULL + stage (slice landed), DG_EMPTY + stage (slice read), DG_KS (among the gathering warps).  The
-// gathering warps wait for DG_EMPTY of slice s - 3 before they refill its stage and report slice s - 1 only after that;
-// the multiplying warps need slices up to s - 3 for it, all of them reported one round before: no cycle.
-enum { DG_FULL = 1, DG_EMPTY = 4, DG_KS = 7 };
+// Named barriers: DG_FULL + stage (slice landed), DG_EMPTY + stage (slice read), DG_KS (among the gathering warps), DG_DONE (among
+// the multiplying warps, behind the last slice).  The
+// gathering warps wait for DG_EMPTY of slice s - stages before they refill its stage and report slice s - LAG = s - stages + 2 only
+// after that; the multiplying warps need slices up to s - stages for it, all of them reported before: no cycle.  They have slice
+// s - stages + 1 to multiply meanwhile (with the report one slice later they stood while slice s was issued: 28x28 256->256 3x3
+// 1005 -> 1422 us forward).
+enum { DG_FULL = 1, DG_EMPTY = 7, DG_KS = 13, DG_DONE = 14 };
 __device__ __forceinline__ void bar_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 // what this thread wrote or read before it is done when the barrier completes
 __device__ __forceinline__ void bar_arrive(int id, int n) {
@@ -382,14 +413,15 @@ dgemm_kernel(IgemmParams p, int mode, const double* __restrict__ A, const double
              double* __restrict__ C, double* __restrict__ partial, Epilogue<double> ep)
 {
     pdl_prologue();
-    constexpr int BM = 128, BK = DG_BK, KP = DG_KP, NP = DG_GATHER;
+    constexpr int BM = 128, BK = DG_BK, KP = DG_KP, NP = DG_GATHER, DG_STAGES = dg_stages<BN>(), LAG = DG_STAGES - 2;
+    static_assert(LAG >= 1 && LAG <= 3 && DG_STAGES <= DG_EMPTY - DG_FULL && DG_STAGES <= DG_KS - DG_EMPTY, "a named barrier each way for every stage");
     constexpr int A_SIZE = 128 * KP > BK * 132 ? 128 * KP : BK * 132, TILE = dg_tile_doubles<BN>();
     constexpr int WM = BN == 128 ? 64 : 32, MI = WM / 16, WARPS_M = BM / WM;     // warp tile WM x 32
     constexpr int A_SI = AK ? KP : 1, A_SK = AK ? 1 : 132, B_SI = BK_ ? KP : 1, B_SK = BK_ ? 1 : BN + 4;   // strides of (index, k)
     extern __shared__ __align__(16) uint8_t dg_smem[];
     double* tiles = reinterpret_cast<double*>(dg_smem);
-    DInfo<OFF>* kinfo = reinterpret_cast<DInfo<OFF>*>(dg_smem + DG_STAGES * TILE * sizeof(double));
-    DInfo<OFF>* rowinfo = kinfo + DG_STAGES * BK;
+    DInfo<OFF>* kinfo = reinterpret_cast<DInfo<OFF>*>(dg_smem + dg_ring_doubles<BN>() * sizeof(double));
+    DInfo<OFF>* rowinfo = kinfo + 2 * DG_GATHER;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     int m_tile = blockIdx.x, n_tile = blockIdx.y, z = blockIdx.z;
     bool split = p.splits > 1;
@@ -412,20 +444,20 @@ dgemm_kernel(IgemmParams p, int mode, const double* __restrict__ A, const double
         // ---------------- gather ----------------
         const int t = tid - DG_MMA;
         const int H = p.H, W = p.W, N = p.N;
-        auto decode_k = [&](int slice, int st) {           // by threads 0 .. BK-1
-            const int k = kbeg + slice * BK + t;
-            kinfo[st * BK + t] = mode == MODE_WGRAD ? dinfo_pix<OFF>(p, mode, k, kend) : dinfo_tap<OFF>(p, mode, k, kend);
-        };
         // copy e of a tile: V doubles from index (e % FAST) * V along memory, at index e / FAST of the other axis
         constexpr int A_FAST = (AK ? BK : BM) / V, A_CNT = BM * BK / V / NP, B_FAST = (BK_ ? BK : BN) / V, B_CNT = BN * BK / V / NP;
         const uint32_t tiles_s = (uint32_t)__cvta_generic_to_shared(tiles);
-        if (t < BK) decode_k(0, 0);
         int st = 0;
 #pragma unroll 1
         for (int s = 0; s < nslice; s++) {
+            DInfo<OFF>* block = kinfo + (s / DG_AHEAD & 1) * DG_GATHER;
+            if (s % DG_AHEAD == 0) {                      // every thread is past the k's that lie there: it has met the barrier since
+                const int k = kbeg + s * BK + t;
+                block[t] = mode == MODE_WGRAD ? dinfo_pix<OFF>(p, mode, k, kend) : dinfo_tap<OFF>(p, mode, k, kend);
+                bar_sync(DG_KS, NP);
+            }
             if (s >= DG_STAGES) bar_sync(DG_EMPTY + st, DG_THREADS);
-            bar_sync(DG_KS, NP);                          // the k's of slice s are decoded
-            const DInfo<OFF>* kis = kinfo + st * BK;
+            const DInfo<OFF>* kis = block + s % DG_AHEAD * BK;
             const uint32_t as = tiles_s + st * TILE * 8, bs = as + A_SIZE * 8;
 #pragma unroll 8
             for (int i = 0; i < A_CNT; i++) {
@@ -442,19 +474,24 @@ dgemm_kernel(IgemmParams p, int mode, const double* __restrict__ A, const double
                 cp_async_doubles<V>(bs + 8 * (x * (BK_ ? KP : BN + 4) + f), B + (ok ? ki.boff + n * (OFF)p.b_sn : 0), ok);
             }
             asm volatile("cp.async.commit_group;" ::: "memory");
-            const int nxt = st + 1 == DG_STAGES ? 0 : st + 1, prev = st == 0 ? DG_STAGES - 1 : st - 1;
-            // the k's of slice s + 1 go where those of slice s - 2 were read: every gathering thread is past them (DG_KS)
-            if (t < BK) decode_k(s + 1, nxt);
-            if (s > 0) {
-                asm volatile("cp.async.wait_group 1;" ::: "memory");
-                bar_arrive(DG_FULL + prev, DG_THREADS);
+            const int nxt = st + 1 == DG_STAGES ? 0 : st + 1, landed = st + 2 >= DG_STAGES ? st + 2 - DG_STAGES : st + 2;      // stage of slice s - LAG
+            if (s >= LAG) {
+                asm volatile("cp.async.wait_group %0;" ::"n"(LAG) : "memory");
+                bar_arrive(DG_FULL + landed, DG_THREADS);
             }
             st = nxt;
         }
-        if (nslice > 0) {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-            bar_arrive(DG_FULL + (st == 0 ? DG_STAGES - 1 : st - 1), DG_THREADS);
-        }
+        // the last LAG slices one by one; st is the stage of the slice behind the last one
+        auto rest = [&](auto left_c) {
+            constexpr int left = decltype(left_c)::value;          // slices behind this one
+            if (nslice > left) {
+                asm volatile("cp.async.wait_group %0;" ::"n"(left) : "memory");
+                int at = st - 1 - left;
+                if (at < 0) at += DG_STAGES;
+                bar_arrive(DG_FULL + at, DG_THREADS);
+            }
+        };
+        if (LAG > 2) rest(std::integral_constant<int, 2>{}); rest(std::integral_constant<int, 1>{}); rest(std::integral_constant<int, 0>{});
         return;
     }
 
@@ -510,25 +547,42 @@ dgemm_kernel(IgemmParams p, int mode, const double* __restrict__ A, const double
         st = st + 1 == DG_STAGES ? 0 : st + 1;
     }
 
+    // The way out: the tile goes through shared memory to a loop of few instructions.  Written from the registers, 64 values a
+    // thread with the epilogue's steps beside each, it was 30 KB of code that a launch runs through once, and a small one waited
+    // for instructions most of its time (32x4x4 32->128 1x1: 18.7 us, of which 4.2 are products).  A store's lanes lie along
+    // whichever of rows and columns is contiguous.
+    bar_sync(DG_DONE, DG_MMA);                   // nobody reads the ring any more
+    double* out = tiles + warp * (WM * DG_OUT);
 #pragma unroll
     for (int i = 0; i < MI; i++)
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const int rl = wm + i * 16 + h * 8 + g, m = m0 + rl;
-            if (m >= p.M) continue;
-            const OFF row_off = rowinfo[rl].boff;
+        for (int h = 0; h < 2; h++)
 #pragma unroll
             for (int j = 0; j < 4; j++)
-#pragma unroll
-                for (int e = 0; e < 2; e++) {
-                    const int n = n0 + wn + j * 8 + 2 * t + e;
-                    if (n >= p.N) continue;
-                    const double v = acc[i][j][2 * h + e];
-                    if (TAIL && split) partial[((int64_t)z * (p.M - p.m_whole) + m - p.m_whole) * p.N + n] = v;
-                    else if (!TAIL && p.splits > 1) partial[((int64_t)blockIdx.z * p.M + m) * p.N + n] = v;
-                    else C[row_off + (int64_t)n * p.c_sn] = apply_epilogue<double>(v, n, ep);
-                }
+                *reinterpret_cast<double2*>(out + (i * 16 + h * 8 + g) * DG_OUT + j * 8 + 2 * t) = make_double2(acc[i][j][2 * h], acc[i][j][2 * h + 1]);
+    __syncwarp();
+    const bool part = TAIL ? split : p.splits > 1;
+    const int n_end = min(32, p.N - n0 - wn), m_end = min(WM, p.M - m0 - wm);       // what the warp has of columns and rows
+    const DInfo<OFF>* rows = rowinfo + wm;
+    if (part || p.c_sn == 1) {
+        if (lane >= n_end) return;
+        const int n = n0 + wn + lane;
+        if (part) {
+            double* d = partial + ((TAIL ? (int64_t)z * (p.M - p.m_whole) - p.m_whole : (int64_t)z * p.M) + m0 + wm) * p.N + n;
+#pragma unroll 8
+            for (int r = 0; r < m_end; r++) d[(int64_t)r * p.N] = out[r * DG_OUT + lane];
+        } else {
+            const ChannelEpilogue<double> own(ep, n);
+#pragma unroll 8
+            for (int r = 0; r < m_end; r++) C[rows[r].boff + n] = own(out[r * DG_OUT + lane]);
         }
+    } else {
+        for (int r = lane; r < m_end; r += 32) {
+            double* d = C + rows[r].boff + (int64_t)(n0 + wn) * p.c_sn;
+#pragma unroll 4
+            for (int c = 0; c < n_end; c++) d[c * p.c_sn] = apply_epilogue<double>(out[r * DG_OUT + c], n0 + wn + c, ep);
+        }
+    }
 }
 
 // Second stage of split-K: fixed-order sum over the splits, epilogue, scatter to the output.  Block (32, ROWS): the thread
@@ -839,23 +893,31 @@ static int choose_splits(const IgemmParams& p, int bk)
     return (int)s;
 }
 
-// The float64 tensor kernel holds one CTA per SM: the split count that needs the fewest rounds of the chip x (slices of a
-// split + about six for its start, its drain and its share of the second stage).
-static int choose_splits_f64(const IgemmParams& p, int bk)
+// The float64 tensor kernel holds one CTA per SM: the split count that needs the least time by rounds of the chip x (slices of a
+// split + about three for its start and its drain, six with its share of the second stage).  Tiles of 128 columns that leave half of the
+// chip idle may be two of 64, whose slices take two thirds of the time (1.4 us of 2.1, 1.8 where doubles are copied one by one; the starts half as long): 32x4x4 32->128
+// 1x1 15.6 -> 8.4 us, while 5x7x48 256->512 3x3, 144 slices, is 166 us by 128 columns and 210 by 64.
+struct F64Plan { int bn, splits; };
+static F64Plan plan_f64(const IgemmParams& p, int bk)
 {
-    const int64_t ctas = (int64_t)((p.M + 127) / 128) * ((p.N + tile_bn(p.N) - 1) / tile_bn(p.N));
+    F64Plan best{};
+    double cost = 0.0;
     const int64_t room = tc_sm_count(), slices = (p.K + bk - 1) / bk;
-    int64_t best = 1, cost = 0;
-    for (int64_t s = 1; s <= 128 && s <= slices && (s == 1 || ctas * s <= 2 * room); s++) {
-        const int64_t c = (ctas * s + room - 1) / room * ((slices + s - 1) / s + (s > 1 ? 6 : 3));
-        if (s == 1 || c < cost) { best = s; cost = c; }
+    for (int bn = p.N <= 64 ? 64 : 128; bn >= 64; bn -= 64) {
+        const int64_t ctas = (int64_t)((p.M + 127) / 128) * ((p.N + bn - 1) / bn);
+        if (best.bn && ctas > room) break;
+        const double slice = bn == 128 || !best.bn ? 1.0 : p.tap_c_fast && p.C % 2 == 0 ? 0.67 : 0.85, start = best.bn ? 0.5 : 1.0;
+        for (int64_t s = 1; s <= 128 && s <= slices && (s == 1 || ctas * s <= 2 * room); s++) {
+            const double c = (double)((ctas * s + room - 1) / room) * ((double)((slices + s - 1) / s) * slice + (s > 1 ? 6.0 : 3.0) * start);
+            if (!best.bn || c < (bn == best.bn ? 1.0 : 0.95) * cost) { best = F64Plan{bn, (int)s}; cost = c; }
+        }
     }
-    return (int)best;
+    return best;
 }
 
 // More than one round of whole float64 tiles: the 392 of a 28x28 256->256 3x3 layer, batch 32, are 2.65 rounds on 148 SMs that ran as
 // three.  Row tiles that fill whole rounds stay whole, the K loops of the others are split so that they fill the chip too (that
-// layer, three passes: 3168 -> 2987 us).  Costs in slices of 128 columns (2.1 us) as in choose_splits_f64; a whole tile takes a
+// layer, three passes: 3168 -> 2987 us).  Costs in slices of 128 columns (2.1 us) as in plan_f64; a whole tile takes a
 // twentieth longer in the form with a tail, and a MB of partial sums 0.2 (0.4 of the narrow tiles' slices).  Without these two a tail saved
 // nothing where K loops are short: 1x1 512->128 of 7040 pixels 66 us whole, 76 with a tail.  By this rule 1716 of 1979 passes
 // measured (5 to 300 slices) have one, 1.27 times as fast on average; 48 of them are slower than whole by more than 1 %.
@@ -882,14 +944,16 @@ static void finish_params(IgemmParams& p, int dtype)
 {
     const int bk = 16;
     static_assert(FMA_BK == 16 && DG_BK == 16, "k-chunks are whole slices of either kernel");
+    p.bn = tile_bn(p.N);
     if (p.K <= 0) { p.splits = 1; p.k_chunk = bk; return; }        // no taps reach these pixels: the launch writes zeros
-    p.splits = dtype == B2C_F32 ? choose_splits(p, bk) : choose_splits_f64(p, bk);
+    if (dtype == B2C_F32) p.splits = choose_splits(p, bk);
+    else { const F64Plan plan = plan_f64(p, bk); p.splits = plan.splits; p.bn = plan.bn; }
     int chunk = (p.K + p.splits - 1) / p.splits;
     chunk = (chunk + bk - 1) / bk * bk;
     p.k_chunk = chunk;
     p.splits = (p.K + chunk - 1) / chunk;
     p.whole = p.m_whole = 0;
-    if (p.splits == 1 && dtype != B2C_F32) split_last_round_f64(p, bk);
+    if (p.splits == 1 && dtype != B2C_F32 && p.bn == tile_bn(p.N)) split_last_round_f64(p, bk);
 }
 static size_t partial_bytes(const IgemmParams& p, size_t es) { return p.splits > 1 ? (size_t)p.splits * (p.M - p.m_whole) * p.N * es : 0; }
 
@@ -1015,11 +1079,13 @@ static int launch_igemm(IgemmParams& p, const void* A, const void* B, void* C, v
     size_t need = partial_bytes(p, sizeof(T));
     if (p.whole && (need > ws_bytes || !ws)) { p.splits = 1; p.k_chunk = (p.K + 15) / 16 * 16; p.whole = p.m_whole = 0; need = 0; }    // whole tiles need none
     if (need > ws_bytes || (need && !ws)) return B2C_ERR_WORKSPACE_TOO_SMALL;
-    const int bn = tile_bn(p.N);
+    const int bn = p.bn;
     const bool vec = p.c_sn == 1 && p.N % 4 == 0 && ((p.pb_sn | p.pb_sh | p.pb_sw) & 3) == 0 && ((uintptr_t)C & 15) == 0;
     dim3 grid((p.M + 127) / 128, (p.N + bn - 1) / bn, p.splits);
     if (grid.y > 65535 || grid.z > 65535) return B2C_ERR_TOO_LARGE;
     if constexpr (sizeof(T) == 8) {
+        p.f_pq = FastDiv(p.PQ); p.f_q = FastDiv(p.Q);
+        if (p.K > 0) { p.f_c = FastDiv(p.C); p.f_s = FastDiv(p.S); p.f_rs = FastDiv(p.R * p.S); }
         if (p.whole) {
             const int64_t blocks = p.whole + ((int64_t)grid.x * grid.y - p.whole) * p.splits;
             if (blocks > 0x7fffffffLL) return B2C_ERR_TOO_LARGE;

@@ -507,21 +507,6 @@ __device__ __forceinline__ float4 tc_split_rounded(float4& q) {
 
 #define TC_CHUNK 8   // k-blocks accumulated in tensor memory before the partial sum is drained
 
-// Division by a launch constant: q = (n * mul) >> 32 >> shift for 0 <= n < 2^31 (round-up reciprocal: with s = ceil(log2 d) and
-// mul = ceil(2^(32 + s - 1) / d) the error stays below 1 / d for 31-bit n).  A role's start-up and each new tile took half a
-// dozen integer divisions, 0.3 us before a launch's first load.
-struct FastDiv {
-    uint32_t d, mul; int shift;
-    FastDiv() = default;
-    __host__ explicit FastDiv(uint32_t d_) : d(d_) {
-        int s = 0;
-        while ((1ull << s) < d_) s++;
-        shift = s - 1;
-        mul = d_ == 1 ? 0 : (uint32_t)(((1ull << (31 + s)) + d_ - 1) / d_);
-    }
-    __device__ __forceinline__ int div(int n) const { return d == 1 ? n : (int)(__umulhi((uint32_t)n, mul) >> shift); }
-};
-
 struct TcParams {
     // FWD: GEMM rows = output pixels, columns = output channels. WGRAD: rows = (tap, ci), columns = co.
     int M, N;

@@ -190,3 +190,27 @@ def test_float32_forward_in_place(c):
     ws = torch.empty(max(256, L.b2c_conv_workspace_bytes(d, _lib.PASS_FPROP)), dtype=torch.uint8, device=DEV)
     _lib.check(L.b2c_conv_fprop(d, x.data_ptr(), f.data_ptr(), None, None, 0, x.data_ptr(), ws.data_ptr(), ws.numel(), stream()))
     assert_parity(x.cpu().numpy(), ref.cpu().numpy(), np.float32)
+
+
+# Sums of 1 to 33 slices of 16 (the ring's stages, the eight slices that are decoded at once, and one more and less of each), an odd channel
+# count (single doubles are copied), outputs of one and of several tiles of 64 or 128 columns that end inside them, rows that end inside 32
+@pytest.mark.parametrize("ci,cout,n", [(16, 65, 3), (48, 130, 5), (64, 128, 2), (80, 30, 7), (128, 96, 4), (129, 257, 1), (144, 64, 9), (271, 192, 2), (528, 140, 40)])
+@pytest.mark.parametrize("layout,w_layout", [("NHWC", "KRSC"), ("NHWC", "CRSK"), ("NCHW", "KCRS")])
+def test_float64_tiles_slices_and_stores(ci, cout, n, layout, w_layout):
+    g = co.Geom(n, 7, 9, ci, cout, 1, 1, 0, 0, 1, 1)
+    rng = np.random.Generator(np.random.PCG64(ci + cout))
+    nchw = layout == "NCHW"
+    x = rng.standard_normal((n, ci, 7, 9) if nchw else (n, 7, 9, ci))
+    wt = rng.standard_normal((cout, ci, 1, 1) if nchw else (ci, 1, 1, cout)) / np.sqrt(ci)
+    b = rng.standard_normal(cout)
+    dy = rng.standard_normal((n, cout, 7, 9) if nchw else (n, 7, 9, cout))
+    y = co.conv2d_forward(x, wt, b, g, layout)
+    dw, db, dx = co.conv2d_backward(x, dy, wt, g, layout)
+    out = run_conv(g, layout, np.float64, x, wt, b, dy, w_layout=w_layout)
+    for name, ref in (("y", y), ("dw", dw), ("db", db), ("dx", dx)):
+        assert_parity(out[name].reshape(ref.shape), ref, np.float64, f"{name} {layout} {w_layout}")
+    bn = {k: rng.uniform(0.5, 1.5, cout) for k in ("running_mean", "inv_std", "gamma", "beta")}
+    v = {k: a.reshape((1, cout, 1, 1) if nchw else (1, 1, 1, cout)) for k, a in bn.items()}
+    fused = np.maximum((y - v["running_mean"]) * v["inv_std"] * v["gamma"] + v["beta"], 0)
+    got = run_conv(g, layout, np.float64, x, wt, b, None, w_layout=w_layout, bn=bn, relu=True, passes=("fprop",))
+    assert_parity(got["y"], fused, np.float64, f"fused {layout}")
