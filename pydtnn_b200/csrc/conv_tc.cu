@@ -817,9 +817,9 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         fence_proxy_async();
     }
     if (warp == 1) tmem_alloc<PAIR>(tmem_slot, L::TMEM_COLS);
-    // barriers, tensor memory and the abort flag are on-chip state, set up while the kernel before this one in the
-    // stream may still be draining; global memory is first touched below, after that kernel has completed
-    pdl_wait();
+    // Barriers, tensor memory and the abort flag are on-chip state, set up while the kernel before this one in the stream may
+    // still be draining, and so is where each role starts: the roles that touch global memory (the producer, the drain warps, the B
+    // warps with their bias sums) wait for that kernel themselves, with their first tile's arithmetic done and their code fetched.
     tc_fence_before();
     if constexpr (PAIR) cluster_sync();          // the other CTA's barriers are set up as well
     else __syncthreads();
@@ -866,8 +866,9 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         // One elected lane runs the whole loop: it arms the barrier and issues the boxes of each k-block.
         if (elect_one_sync()) {
         Ring<STAGES> ring;
-        bool ok = true;
+        bool ok = true, first = true;
         if (RESKB) {
+            pdl_wait();
             // The grid is a multiple of the column-tile count: this CTA only meets column tile blockIdx.x % nt, whose
             // filter tiles (all k-blocks) are fetched once.
             const int n0r = ((int)blockIdx.x - p.f_nt.div((int)blockIdx.x) * nt) * BN;
@@ -941,6 +942,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 p0 = p.f_q.div(rem); q0 = rem - p0 * p.Q;
                 im_step = p.f_pq.div(32); rem = 32 - im_step * (p.P * p.Q); p_step = p.f_q.div(rem); q_step = rem - p_step * p.Q;
             }
+            if (!RESKB && first) { pdl_wait(); first = false; }
             for (int kb = w.kb_b; kb < w.kb_e; kb++) {
                 const int s = ring.s;
                 TC_PROF_T0();
@@ -1277,6 +1279,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 if (lane == 0) arrive_mma(&xform_bar[s]);
             }
             if (MODE == TCM_WGRAD && do_db && ok) {
+                pdl_wait();
                 // Float4 number t + 128 i of the B region is box i/2, pixel row t/8 + 16 (i & 1), 16-byte chunk t & 7.
                 // The box layout XORs the 32-byte atom index (chunk >> 1) with (row & 3), so the lane's channels are
                 // chunk ((c >> 1) ^ rr) * 2 + (c & 1) with c = lane & 7, rr = (lane >> 3) & 3: the four lanes that hold
@@ -1304,6 +1307,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         // float32 round-to-nearest; the tensor core's own accumulate step truncates, and its bias
         // grows with the number of accumulations, so it is kept to one chunk.
         if (BW) regs_inc<TC_REGS_DRAIN>();
+        pdl_wait();
         const int quad = warp & 3;                       // TMEM lane quadrant this warp may read
         bool ok = true;
         int gc = 0, ecount = 0;
