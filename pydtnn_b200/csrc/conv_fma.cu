@@ -412,7 +412,6 @@ __global__ void __launch_bounds__(DG_THREADS, 1)
 dgemm_kernel(IgemmParams p, int mode, const double* __restrict__ A, const double* __restrict__ B,
              double* __restrict__ C, double* __restrict__ partial, Epilogue<double> ep)
 {
-    pdl_prologue();
     constexpr int BM = 128, BK = DG_BK, KP = DG_KP, NP = DG_GATHER, DG_STAGES = dg_stages<BN>(), LAG = DG_STAGES - 2;
     static_assert(LAG >= 1 && LAG <= 3 && DG_STAGES <= DG_EMPTY - DG_FULL && DG_STAGES <= DG_KS - DG_EMPTY, "a named barrier each way for every stage");
     constexpr int A_SIZE = 128 * KP > BK * 132 ? 128 * KP : BK * 132, TILE = dg_tile_doubles<BN>();
@@ -448,6 +447,7 @@ dgemm_kernel(IgemmParams p, int mode, const double* __restrict__ A, const double
         constexpr int A_FAST = (AK ? BK : BM) / V, A_CNT = BM * BK / V / NP, B_FAST = (BK_ ? BK : BN) / V, B_CNT = BN * BK / V / NP;
         const uint32_t tiles_s = (uint32_t)__cvta_generic_to_shared(tiles);
         int st = 0;
+        bool first = true;
 #pragma unroll 1
         for (int s = 0; s < nslice; s++) {
             DInfo<OFF>* block = kinfo + (s / DG_AHEAD & 1) * DG_GATHER;
@@ -456,6 +456,7 @@ dgemm_kernel(IgemmParams p, int mode, const double* __restrict__ A, const double
                 block[t] = mode == MODE_WGRAD ? dinfo_pix<OFF>(p, mode, k, kend) : dinfo_tap<OFF>(p, mode, k, kend);
                 bar_sync(DG_KS, NP);
             }
+            if (first) { pdl_prologue(); first = false; }      // rows and k's are decoded while the kernel in front ends
             if (s >= DG_STAGES) bar_sync(DG_EMPTY + st, DG_THREADS);
             const DInfo<OFF>* kis = block + s % DG_AHEAD * BK;
             const uint32_t as = tiles_s + st * TILE * 8, bs = as + A_SIZE * 8;
@@ -496,6 +497,7 @@ dgemm_kernel(IgemmParams p, int mode, const double* __restrict__ A, const double
     }
 
     // ---------------- products ----------------
+    pdl_prologue();
     const int wm = (warp % WARPS_M) * WM, wn = (warp / WARPS_M) * 32;
     const int g = lane >> 2, t = lane & 3;
     int nj = (p.N - n0 - wn + 7) / 8;            // 8-column steps of this warp that hold columns of the output
@@ -591,10 +593,19 @@ dgemm_kernel(IgemmParams p, int mode, const double* __restrict__ A, const double
 template <typename T, int MODE, int ROWS>
 __global__ void __launch_bounds__(256) splitk_reduce_kernel(IgemmParams p, const T* __restrict__ partial, T* __restrict__ C, Epilogue<T> ep)
 {
-    pdl_prologue();
     constexpr int COLS = 256 / ROWS;
     __shared__ T part[ROWS][COLS];
     const int64_t idx = (int64_t)blockIdx.x * COLS + threadIdx.x, total = (int64_t)(p.M - p.m_whole) * p.N;
+    // where the sum goes is worked out while the kernel in front ends
+    int64_t to = 0;
+    int n = 0;
+    if (idx < total && threadIdx.y == 0) {
+        const int row = (int)(idx / p.N), m = p.m_whole + row;
+        n = (int)(idx - (int64_t)row * p.N);
+        const Info ri = (MODE == MODE_WGRAD) ? decode_tap<MODE>(p, m, p.M) : decode_pix<MODE>(p, m, p.M);
+        to = ri.b_off + (int64_t)n * p.c_sn;
+    }
+    pdl_prologue();
     T v = T(0);
     if (idx < total) {
         int z = threadIdx.y;
@@ -615,9 +626,7 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(IgemmParams p, const
         for (int y = 1; y < ROWS; y++) v += part[y][threadIdx.x];
     }
     if (idx >= total) return;
-    const int row = (int)(idx / p.N), n = (int)(idx - (int64_t)row * p.N), m = p.m_whole + row;
-    const Info ri = (MODE == MODE_WGRAD) ? decode_tap<MODE>(p, m, p.M) : decode_pix<MODE>(p, m, p.M);
-    C[ri.b_off + (int64_t)n * p.c_sn] = apply_epilogue<T>(v, n, ep);
+    C[to] = apply_epilogue<T>(v, n, ep);
 }
 
 // Index map of the lowering, numbered as the reference numbers rows and columns.
