@@ -773,7 +773,9 @@ __global__ void pool_bwd_kernel(PoolP p, const T* __restrict__ dy, const int32_t
 // float32 NHWC pooling with 4 channels per thread (c % 4 == 0).  Grid (blocks over a row's positions x channel groups, n x ho):
 // one 32-bit division per thread instead of six 64-bit ones per output, and the window's bounds are clipped once instead of
 // tested at every tap, so the taps' loads are independent (64 x 55 x 55 x 96, 3 x 3 / 2, with the tap numbers: 29.6 us before).
-template <bool IS_MAX>
+// K: the window where it is K x K without dilation.  A window inside the image then has all its loads in flight at once instead of a
+// row's (K = 0): the kernel waits for memory, not for its bandwidth.
+template <bool IS_MAX, int K>
 __global__ void __launch_bounds__(256) pool_fwd_v4_kernel(PoolP p, const float4* __restrict__ x, float4* __restrict__ y, int4* __restrict__ idx_max, int row0)
 {
     pdl_prologue();
@@ -790,18 +792,26 @@ __global__ void __launch_bounds__(256) pool_fwd_v4_kernel(PoolP p, const float4*
     if (w0 + (p.kw - 1) * p.hdil >= p.w) jj1 = p.w > w0 ? (p.w - w0 + p.hdil - 1) / p.hdil : 0;
     float4 best = IS_MAX ? make_float4(-FLT_MAX, -FLT_MAX, -FLT_MAX, -FLT_MAX) : make_float4(0.f, 0.f, 0.f, 0.f);
     int4 bi = make_int4(0, 0, 0, 0);
-    for (int ii = ii0; ii < ii1; ii++) {
+    auto take = [&](const float4& v, int t) {
+        if (IS_MAX) {
+            if (v.x > best.x) { best.x = v.x; bi.x = t; }
+            if (v.y > best.y) { best.y = v.y; bi.y = t; }
+            if (v.z > best.z) { best.z = v.z; bi.z = t; }
+            if (v.w > best.w) { best.w = v.w; bi.w = t; }
+        } else { best.x += v.x; best.y += v.y; best.z += v.z; best.w += v.w; }
+    };
+    if (K && ii0 == 0 && ii1 == K && jj0 == 0 && jj1 == K) {
+        float4 v[K ? K * K : 1];
+        const float4* src = x + (((int64_t)nn * p.h + h0) * p.w + w0) * c4 + cg;
+#pragma unroll
+        for (int t = 0; t < K * K; t++) v[t] = src[((int64_t)(t / (K ? K : 1)) * p.w + t % (K ? K : 1)) * c4];
+#pragma unroll
+        for (int t = 0; t < K * K; t++) take(v[t], t);
+    } else for (int ii = ii0; ii < ii1; ii++) {
         const float4* src = x + (((int64_t)nn * p.h + h0 + ii * p.vdil) * p.w + w0) * c4 + cg;
 #pragma unroll 4
         for (int jj = jj0; jj < jj1; jj++) {
-            const float4 v = src[(int64_t)jj * p.hdil * c4];
-            if (IS_MAX) {
-                const int t = ii * p.kw + jj;
-                if (v.x > best.x) { best.x = v.x; bi.x = t; }
-                if (v.y > best.y) { best.y = v.y; bi.y = t; }
-                if (v.z > best.z) { best.z = v.z; bi.z = t; }
-                if (v.w > best.w) { best.w = v.w; bi.w = t; }
-            } else { best.x += v.x; best.y += v.y; best.z += v.z; best.w += v.w; }
+            take(src[(int64_t)jj * p.hdil * c4], ii * p.kw + jj);
         }
     }
     const int64_t o = ((int64_t)row * p.wo + yy) * c4 + cg;
@@ -851,10 +861,17 @@ __global__ void __launch_bounds__(256) pool_bwd_v4_kernel(PoolP p, const float4*
                     if (id.z == tap) acc.z += g.z;
                     if (id.w == tap) acc.w += g.w;
                 } else {
-                    int items = 0;
-                    for (int a = 0; a < p.kh; a++) { int q = p.vstr * xx + p.vdil * a - p.vpad; if (q < 0 || q >= p.h) continue;
-                        for (int b = 0; b < p.kw; b++) { int r2 = p.hstr * yy + p.hdil * b - p.hpad; if (r2 >= 0 && r2 < p.w) items++; } }
-                    const float inv = (float)items;
+                    // the window's taps inside the image, rows times columns (counted tap by tap, a 7x7 window's 49 for every element were
+                    // 42 us of a ResNet-50 step)
+                    int rows = 0, cols = 0;
+                    if (UNIT_DIL) {
+                        const int q = p.vstr * xx - p.vpad, u = p.hstr * yy - p.hpad;
+                        rows = min(p.kh, p.h - q) - max(0, -q); cols = min(p.kw, p.w - u) - max(0, -u);
+                    } else {
+                        for (int a = 0; a < p.kh; a++) { const int q = p.vstr * xx + p.vdil * a - p.vpad; if (q >= 0 && q < p.h) rows++; }
+                        for (int b = 0; b < p.kw; b++) { const int q = p.hstr * yy + p.hdil * b - p.hpad; if (q >= 0 && q < p.w) cols++; }
+                    }
+                    const float inv = (float)(rows * cols);
                     acc.x += g.x / inv; acc.y += g.y / inv; acc.z += g.z / inv; acc.w += g.w / inv;
                 }
             }
@@ -1401,8 +1418,11 @@ extern "C" int b2c_pool_forward(int dtype, int layout, int is_max, int n, int h,
         if (rows > 0x7fffffffLL || per_row > 0x7fffff00LL) return B2C_ERR_TOO_LARGE;
         for (int64_t row0 = 0; row0 < rows; row0 += 65535) {          // the rows are a grid axis
             const dim3 grid((unsigned)((per_row + 255) / 256), (unsigned)(rows - row0 < 65535 ? rows - row0 : 65535));
-            if (is_max) launch_pdl(pool_fwd_v4_kernel<true>, grid, 256, 0, st, p, (const float4*)x, (float4*)y, (int4*)idx_max, (int)row0);
-            else launch_pdl(pool_fwd_v4_kernel<false>, grid, 256, 0, st, p, (const float4*)x, (float4*)y, (int4*)idx_max, (int)row0);
+            const int k = p.kh == p.kw && p.vdil == 1 && p.hdil == 1 ? p.kh : 0;
+            auto* kernel = k == 3 ? (is_max ? pool_fwd_v4_kernel<true, 3> : pool_fwd_v4_kernel<false, 3>)
+                         : k == 2 ? (is_max ? pool_fwd_v4_kernel<true, 2> : pool_fwd_v4_kernel<false, 2>)
+                                  : (is_max ? pool_fwd_v4_kernel<true, 0> : pool_fwd_v4_kernel<false, 0>);
+            launch_pdl(kernel, grid, 256, 0, st, p, (const float4*)x, (float4*)y, (int4*)idx_max, (int)row0);
             const int rc2 = check_launch("pool_forward_v4"); if (rc2) return rc2;
         }
         return B2C_OK;
