@@ -25,8 +25,8 @@
 // tiles between consecutive CTAs; the filter from split copies or read in place (K-major or MN-major); a chunked
 // drain, or for tiles of one chunk a streaming epilogue (32 columns at a time straight from tensor memory) with four
 // or eight drain warps; for tiles of at most four k-blocks the filter tiles of the CTA's column tile resident in
-// shared memory for the whole launch; several pixel classes (a strided data gradient) in one launch.  NCHW tensors
-// run on channel-last copies.
+// shared memory for the whole launch; several pixel classes (a strided data gradient) in one launch; two CTAs that share
+// a B tile (PAIR).  NCHW tensors run on channel-last copies.
 //
 // Warp roles: warp 0 = TMA producer, warp 1 = TMEM owner + MMA issuer (one elected lane of each runs the whole loop), four
 // warps that split A, four that split B where a raw B tile is split (tc_b_warps; else the A warps do it), four or
