@@ -77,7 +77,10 @@ static int launch_reduce2(F f, double* partial, int layout, int n, int c, int hw
 
 static size_t reduce2_bytes(int c) { return (size_t)RED_CHUNKS * 2 * c * sizeof(double); }
 
-__device__ __forceinline__ int channel_of(int64_t idx, int c, int hw, int nchw)
+// IDX = int where the element count plus one grid stride (ew_blocks) fits 31 bits: the kernels below that divide an element's index
+// do so in 32 bits then (small float64 ResNet step, 31 such launches: 503 -> 500 us).
+static bool fits_int(int64_t total) { return total < 0x7fffffffLL - 148LL * 16 * 256; }
+template <typename IDX> __device__ __forceinline__ int channel_of(IDX idx, int c, int hw, int nchw)
 {
     return nchw ? (int)((idx / hw) % c) : (int)(idx % c);
 }
@@ -89,15 +92,15 @@ template <typename T> struct StatF {
     __device__ void operator()(int64_t i, int, double& v0, double& v1) const { double v = (double)x[i]; v0 = v; v1 = v * v; }
 };
 
-template <typename T>
+template <typename T, typename IDX>
 __global__ void bn_apply_kernel(const T* __restrict__ x, T* __restrict__ y, const T* __restrict__ mean,
                                 const T* __restrict__ inv_std, const T* __restrict__ gamma, const T* __restrict__ beta,
                                 int64_t total, int c, int hw, int nchw, int relu, int ref_order, const T* __restrict__ addend)
 {
     pdl_prologue();
-    int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-        int ch = channel_of(i, c, hw, nchw);
+    const IDX count = (IDX)total, stride = (IDX)gridDim.x * blockDim.x;
+    for (IDX i = (IDX)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += stride) {
+        int ch = channel_of<IDX>(i, c, hw, nchw);
         T xn = (x[i] - mean[ch]) * inv_std[ch];
         T v = ref_order ? (xn * gamma[ch] + beta[ch]) : (gamma[ch] * xn + beta[ch]);
         if (addend) v = v + addend[i];        // residual sum: the rounded BN output plus the other branch
@@ -117,16 +120,16 @@ template <typename T> struct BnBwdF {
 };
 
 // dx = (gamma / (std*n)) * (n*dy - xn*dgamma - dbeta)   (pydtnn/cython_modules/bn_training_cython.pyx:227)
-template <typename T>
+template <typename T, typename IDX>
 __global__ void bn_bwd_dx_kernel(const T* __restrict__ x, const T* __restrict__ dy, const T* __restrict__ y,
                                  const T* __restrict__ gamma, const T* __restrict__ mean, const T* __restrict__ inv_std,
                                  const T* __restrict__ dgamma, const T* __restrict__ dbeta, T* __restrict__ dx,
                                  int64_t total, int c, int hw, int nchw, int relu, T count)
 {
     pdl_prologue();
-    int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-        int ch = channel_of(i, c, hw, nchw);
+    const IDX all = (IDX)total, stride = (IDX)gridDim.x * blockDim.x;
+    for (IDX i = (IDX)blockIdx.x * blockDim.x + threadIdx.x; i < all; i += stride) {
+        int ch = channel_of<IDX>(i, c, hw, nchw);
         T g = dy[i];
         if (relu && !(y[i] > T(0))) g = T(0);
         T xn = (x[i] - mean[ch]) * inv_std[ch];
@@ -523,7 +526,7 @@ static int bn_train_forward_t(int layout, int n, int c, int hw, const T* x, cons
     if (rc) return rc;
     rc = final_warp<T>(scratch, chunks, c, 0, (double)n * hw, momentum, eps, sm, si, rm, rv, st); if (rc) return rc;
     int64_t total = (int64_t)n * c * hw;
-    launch_pdl(bn_apply_kernel<T>, ew_blocks(total), 256, 0, st, x, y, sm, si, gamma, beta, total, c, hw, layout == B2C_LAYOUT_NCHW, relu, 0, addend);
+    launch_pdl(fits_int(total) ? bn_apply_kernel<T, int> : bn_apply_kernel<T, int64_t>, ew_blocks(total), 256, 0, st, x, y, sm, si, gamma, beta, total, c, hw, layout == B2C_LAYOUT_NCHW, relu, 0, addend);
     return check_launch("bn_apply");
 }
 
@@ -556,7 +559,7 @@ static int bn_train_backward_t(int layout, int n, int c, int hw, const T* x, con
     rc = final_warp<T>(scratch, chunks, c, 1, 1.0, 0.0, 0.0, dgamma, dbeta, (T*)nullptr, (T*)nullptr, st); if (rc) return rc;
     if (!dx) return B2C_OK;
     int64_t total = (int64_t)n * c * hw;
-    launch_pdl(bn_bwd_dx_kernel<T>, ew_blocks(total), 256, 0, st, x, dy, y, gamma, sm, si, dgamma, dbeta, dx, total, c, hw,
+    launch_pdl(fits_int(total) ? bn_bwd_dx_kernel<T, int> : bn_bwd_dx_kernel<T, int64_t>, ew_blocks(total), 256, 0, st, x, dy, y, gamma, sm, si, dgamma, dbeta, dx, total, c, hw,
                                                           layout == B2C_LAYOUT_NCHW, relu, (T)((double)n * hw));
     return check_launch("bn_bwd_dx");
 }
@@ -734,16 +737,15 @@ __global__ void __launch_bounds__(256) pool_fwd_nchw_planes_kernel(PoolP p, cons
 }
 
 // Backward as a gather over the windows that contain each input element (fixed summation order).
-template <typename T, bool IS_MAX>
+template <typename T, bool IS_MAX, typename IDX>
 __global__ void pool_bwd_kernel(PoolP p, const T* __restrict__ dy, const int32_t* __restrict__ idx_max, T* __restrict__ dx, int nchw)
 {
     pdl_prologue();
-    int64_t total = (int64_t)p.n * p.h * p.w * p.c;
-    int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
+    const IDX total = (IDX)p.n * p.h * p.w * p.c, stride = (IDX)gridDim.x * blockDim.x;
+    for (IDX i = (IDX)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
         int cc, iw, ih, nn;
-        if (nchw) { iw = (int)(i % p.w); int64_t r = i / p.w; ih = (int)(r % p.h); r /= p.h; cc = (int)(r % p.c); nn = (int)(r / p.c); }
-        else { cc = (int)(i % p.c); int64_t r = i / p.c; iw = (int)(r % p.w); r /= p.w; ih = (int)(r % p.h); nn = (int)(r / p.h); }
+        if (nchw) { iw = (int)(i % p.w); IDX r = i / p.w; ih = (int)(r % p.h); r /= p.h; cc = (int)(r % p.c); nn = (int)(r / p.c); }
+        else { cc = (int)(i % p.c); IDX r = i / p.c; iw = (int)(r % p.w); r /= p.w; ih = (int)(r % p.h); nn = (int)(r / p.h); }
         T acc = T(0);
         for (int ii = 0; ii < p.kh; ii++) {
             int t = ih + p.vpad - p.vdil * ii;
@@ -758,10 +760,10 @@ __global__ void pool_bwd_kernel(PoolP p, const T* __restrict__ dy, const int32_t
                 int64_t o = nn * p.ysn + xx * p.ysh + yy * p.ysw + cc * p.ysc;
                 if (IS_MAX) { if (idx_max[o] == ii * p.kw + jj) acc += dy[o]; }
                 else {
-                    int items = 0;
-                    for (int a = 0; a < p.kh; a++) { int q = p.vstr * xx + p.vdil * a - p.vpad; if (q < 0 || q >= p.h) continue;
-                        for (int b = 0; b < p.kw; b++) { int r2 = p.hstr * yy + p.hdil * b - p.hpad; if (r2 >= 0 && r2 < p.w) items++; } }
-                    acc += dy[o] / (T)items;
+                    int rows = 0, cols = 0;
+                    for (int a = 0; a < p.kh; a++) { const int q = p.vstr * xx + p.vdil * a - p.vpad; if (q >= 0 && q < p.h) rows++; }
+                    for (int b = 0; b < p.kw; b++) { const int q = p.hstr * yy + p.hdil * b - p.hpad; if (q >= 0 && q < p.w) cols++; }
+                    acc += dy[o] / (T)(rows * cols);
                 }
             }
         }
@@ -1311,10 +1313,10 @@ extern "C" int b2c_bn_inference(int dtype, int layout, int n, int c, int hw, con
         return check_launch("bn_inference_v4");
     }
     if (dtype == B2C_F32)
-        launch_pdl(bn_apply_kernel<float>, ew_blocks(total), 256, 0, st, (const float*)x, (float*)y, (const float*)mean, (const float*)inv_std,
+        launch_pdl(fits_int(total) ? bn_apply_kernel<float, int> : bn_apply_kernel<float, int64_t>, ew_blocks(total), 256, 0, st, (const float*)x, (float*)y, (const float*)mean, (const float*)inv_std,
                                                                 (const float*)gamma, (const float*)beta, total, c, hw, layout == B2C_LAYOUT_NCHW, relu, 1, (const float*)nullptr);
     else
-        launch_pdl(bn_apply_kernel<double>, ew_blocks(total), 256, 0, st, (const double*)x, (double*)y, (const double*)mean, (const double*)inv_std,
+        launch_pdl(fits_int(total) ? bn_apply_kernel<double, int> : bn_apply_kernel<double, int64_t>, ew_blocks(total), 256, 0, st, (const double*)x, (double*)y, (const double*)mean, (const double*)inv_std,
                                                                  (const double*)gamma, (const double*)beta, total, c, hw, layout == B2C_LAYOUT_NCHW, relu, 1, (const double*)nullptr);
     return check_launch("bn_inference");
 }
@@ -1480,11 +1482,11 @@ extern "C" int b2c_pool_backward(int dtype, int layout, int is_max, int n, int h
         return check_launch("pool_backward_v4");
     }
     if (dtype == B2C_F32) {
-        if (is_max) launch_pdl(pool_bwd_kernel<float, true>, ew_blocks(total), 256, 0, st, p, (const float*)dy, idx_max, (float*)dx, nchw);
-        else launch_pdl(pool_bwd_kernel<float, false>, ew_blocks(total), 256, 0, st, p, (const float*)dy, idx_max, (float*)dx, nchw);
+        if (is_max) launch_pdl(fits_int(total) ? pool_bwd_kernel<float, true, int> : pool_bwd_kernel<float, true, int64_t>, ew_blocks(total), 256, 0, st, p, (const float*)dy, idx_max, (float*)dx, nchw);
+        else launch_pdl(fits_int(total) ? pool_bwd_kernel<float, false, int> : pool_bwd_kernel<float, false, int64_t>, ew_blocks(total), 256, 0, st, p, (const float*)dy, idx_max, (float*)dx, nchw);
     } else {
-        if (is_max) launch_pdl(pool_bwd_kernel<double, true>, ew_blocks(total), 256, 0, st, p, (const double*)dy, idx_max, (double*)dx, nchw);
-        else launch_pdl(pool_bwd_kernel<double, false>, ew_blocks(total), 256, 0, st, p, (const double*)dy, idx_max, (double*)dx, nchw);
+        if (is_max) launch_pdl(fits_int(total) ? pool_bwd_kernel<double, true, int> : pool_bwd_kernel<double, true, int64_t>, ew_blocks(total), 256, 0, st, p, (const double*)dy, idx_max, (double*)dx, nchw);
+        else launch_pdl(fits_int(total) ? pool_bwd_kernel<double, false, int> : pool_bwd_kernel<double, false, int64_t>, ew_blocks(total), 256, 0, st, p, (const double*)dy, idx_max, (double*)dx, nchw);
     }
     return check_launch("pool_backward");
 }
