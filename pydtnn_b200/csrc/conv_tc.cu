@@ -2267,7 +2267,7 @@ struct StatsOut { float* sums; };
 // because tiles x splits is at most one CTA per SM.  Narrow tiles only pay where the wide ones leave the chip idle (single
 // images, late layers of small batches).
 struct FwdPlan { int bn; bool sk; int kper; bool pair; };
-static FwdPlan fwd_plan(int64_t M, int N, int64_t kblocks, bool may_share, bool may_pair, bool fine = false)
+static FwdPlan fwd_plan(int64_t M, int N, int64_t kblocks, bool may_share, bool may_pair, bool sums, bool fine = false)
 {
     const int G = tc_sm_count();
     FwdPlan best{128, false, 0, false};
@@ -2300,13 +2300,19 @@ static FwdPlan fwd_plan(int64_t M, int N, int64_t kblocks, bool may_share, bool 
     // and the rows that fill up a column's last pair what any others do.  64x28x28 512->256 1x1 (6 rounds of 16 k-blocks) 65.8 us by single CTAs, 57.2 by pairs;
     // 64x28x28 128->128 3x3 (3 of 36) 63.4 / 57.0; 64x14x14 256->256 3x3 (balanced) 67.8 / 63.7; 64x16x16 128->128 3x3 (1 of 36) 27.1 / 26.1;
     // on few SMs 3x26x45 128->128 3x3 (28 tiles) 21.4 / 22.2.  Filters as hi and lo copies (lowered inputs) gain nothing: 35x47x47 6->512
-    // 7x7/2 72.4 / 74.0.
+    // 7x7/2 72.4 / 74.0.  A launch that keeps batch sums by CTA (`sums`) runs on whole groups of column tiles (launch_tc): with 16 of
+    // them on 144 CTAs but on 64 pairs, four rounds instead of three: 64x7x7 512->2048 1x1 35.1 us by single CTAs, 38.8 by pairs (without
+    // sums 36.3 / 33.2).
     if (may_pair && best.bn == 128 && !fine && M > 128 && (best.kper ? best.kper : kblocks) >= 12) {
         const int64_t nt = (N + 127) / 128, splits = best.kper ? (kblocks + best.kper - 1) / best.kper : 1;
         const int64_t tiles = (M + 127) / 128 * nt * splits, pairs = (M + 255) / 256 * nt * splits, len = best.kper ? best.kper : kblocks;
         const double kb = tiles <= G ? 0.5 : 0.45, busy = tiles < G && !best.sk ? (double)tiles / G : 1.0;
-        const double whole = best.sk ? (double)(tiles * len) / G : (double)((tiles + G - 1) / G * len);
-        const double paired = best.sk ? (double)(pairs * len) / (G / 2) : (double)((pairs + G / 2 - 1) / (G / 2) * len);
+        auto rounds = [&](int64_t items, int64_t most) {
+            const int64_t grid = items < most ? items : most, used = sums && !best.kper && nt <= grid ? grid - grid % nt : most;
+            return (items + used - 1) / used;
+        };
+        const double whole = best.sk ? (double)(tiles * len) / G : (double)(rounds(tiles, G) * len);
+        const double paired = best.sk ? (double)(pairs * len) / (G / 2) : (double)(rounds(pairs, G / 2) * len);
         best.pair = (!best.kper || pairs <= G / 2) && paired * (kb - 0.06 * busy) + 0.6 < whole * kb;
     }
     return best;
@@ -2317,7 +2323,7 @@ static FwdPlan fwd_plan(int64_t M, int N, int64_t kblocks, bool may_share, bool 
 static int64_t fwd_stats_rows(int64_t M, int N, int64_t kblocks, bool may_balance, bool* by_cta)
 {
     const int G = tc_sm_count();
-    const FwdPlan plan = fwd_plan(M, N, kblocks, may_balance, may_balance);
+    const FwdPlan plan = fwd_plan(M, N, kblocks, may_balance, may_balance, true);
     const int64_t cl = plan.pair ? 2 : 1, most = G / cl;
     const int64_t nt = (N + plan.bn - 1) / plan.bn, tiles = ((M + 128 * cl - 1) / (128 * cl)) * nt;
     const int64_t grid = tiles < most ? tiles : most;
@@ -2381,7 +2387,7 @@ static int run_fwd(const FwdLaunch& f, const void* act, const void* w, PrepParam
     unsigned int* sk_bank = tc_sm_count() * 4 <= TC_SYNC_FLAGS ? tc_sync_bank(st) : nullptr;
     if (sk_bank) sk_flags = (int*)sk_bank;
     const bool room = base + 2 * fbytes + sk_bytes() <= (uintptr_t)ws + ws_bytes;
-    const FwdPlan plan = fwd_plan((int64_t)f.n * f.P * f.Q, f.N, (int64_t)f.kh * f.kw * cblocks, !filters_ready && room && !zf, !filters_ready, f.fine);
+    const FwdPlan plan = fwd_plan((int64_t)f.n * f.P * f.Q, f.N, (int64_t)f.kh * f.kw * cblocks, !filters_ready && room && !zf, !filters_ready, stats != nullptr, f.fine);
     const int BN = plan.bn, sk = plan.sk, kper = plan.kper, BNL = plan.pair ? BN / 2 : BN;
     // The filter itself serves as the B operand when its layout allows a tensor map over it (the channel axis
     // that is contiguous decides K-major or MN-major); otherwise hi/lo copies in the GEMM layout are written first.

@@ -2,6 +2,7 @@
 tile of few columns, every filter layout, whole tiles, balanced ranges, split K loops, the classes of a strided input gradient,
 the weight gradient, batch sums. GPU."""
 import ctypes
+import re
 
 import numpy as np
 import pytest
@@ -23,6 +24,17 @@ SHAPES = [
     (20, 27, 27, 96, 200, 5, 1),        # weight gradient: 19 row tiles of (tap, channel), ranges of the pixels, second column tile of 72
     (3, 45, 33, 256, 384, 1, 1),        # weight gradient of a 1x1 layer, two pairs
 ]
+
+
+def _pairs(launch):
+    """Whether the tensor-core kernel that `launch` runs is the form for pairs of CTAs (its last template argument)."""
+    torch.cuda.synchronize()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        launch()
+        torch.cuda.synchronize()
+    forms = [re.search(r"conv_tc_kernel<(.*?)>", e.name).group(1).split(", ") for e in prof.events() if "conv_tc_kernel" in e.name]
+    assert len(forms) == 1 and len(forms[0]) == 12, forms
+    return forms[0][-1].strip("()bool") in ("true", "1")
 
 
 def _layer(shape, layout, w_layout):
@@ -92,3 +104,20 @@ def test_batch_sums_of_pairs(shape):
     for got, ref, mag in ((stats[:rows, 0], v, v.abs()), (stats[:rows, 1], v * v, v * v)):
         err = (got.double().sum(0) - ref.sum(0)).abs()
         assert bool((err <= adds * 2.0 ** -24 * mag.sum(0)).all())
+
+
+@pytest.mark.parametrize("shape", [(64, 7, 7, 512, 2048, 1, 1), (64, 14, 14, 1024, 2048, 1, 2)])
+def test_no_pairs_where_batch_sums_leave_them_too_few_ctas(shape):
+    """16 column tiles: 144 of 148 CTAs hold whole groups of them, but only 64 of 74 pairs: four rounds of pairs instead of three."""
+    L = _lib.lib()
+    _, desc, _, (xd, dyd, wd), _, _ = _layer(shape, "NHWC", "KRSC")
+    d, ws, y = ctypes.byref(desc), workspace(desc), torch.empty_like(dyd)
+    nbytes = L.b2c_conv_stats_bytes(d)
+    stats = torch.empty(nbytes, dtype=torch.uint8, device=DEV)
+    args = (ws.data_ptr(), ws.numel(), stream())
+    with_sums = lambda: _lib.check(L.b2c_conv_fprop_stats(d, xd.data_ptr(), wd.data_ptr(), None, y.data_ptr(), stats.data_ptr(), nbytes, *args))
+    without = lambda: _lib.check(L.b2c_conv_fprop(d, xd.data_ptr(), wd.data_ptr(), None, None, 0, y.data_ptr(), *args))
+    assert not _pairs(with_sums)
+    first = y.clone()
+    assert _pairs(without)
+    assert torch.equal(first, y)
