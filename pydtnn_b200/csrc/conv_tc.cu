@@ -2302,7 +2302,10 @@ static FwdPlan fwd_plan(int64_t M, int N, int64_t kblocks, bool may_share, bool 
     // on few SMs 3x26x45 128->128 3x3 (28 tiles) 21.4 / 22.2.  Filters as hi and lo copies (lowered inputs) gain nothing: 35x47x47 6->512
     // 7x7/2 72.4 / 74.0.  A launch that keeps batch sums by CTA (`sums`) runs on whole groups of column tiles (launch_tc): with 16 of
     // them on 144 CTAs but on 64 pairs, four rounds instead of three: 64x7x7 512->2048 1x1 35.1 us by single CTAs, 38.8 by pairs (without
-    // sums 36.3 / 33.2).
+    // sums 36.3 / 33.2).  A single CTA does not multiply past the last channel, so a k-block of a last column tile takes it 0.6 + 0.3 of
+    // the columns' share of what a whole one takes; a pair always multiplies 128.  In balanced ranges the CTA with the most whole
+    // tiles counts (of whole tiles and splits that is one with whole ones only): 32x36x36 256->132 3x3 146 / 150 us, 34x41x41 256->172 5x5
+    // 640 / 652; 53x25x25 512->188 3x3 285 / 277.
     if (may_pair && best.bn == 128 && !fine && M > 128 && (best.kper ? best.kper : kblocks) >= 12) {
         const int64_t nt = (N + 127) / 128, splits = best.kper ? (kblocks + best.kper - 1) / best.kper : 1;
         const int64_t tiles = (M + 127) / 128 * nt * splits, pairs = (M + 255) / 256 * nt * splits, len = best.kper ? best.kper : kblocks;
@@ -2311,7 +2314,14 @@ static FwdPlan fwd_plan(int64_t M, int N, int64_t kblocks, bool may_share, bool 
             const int64_t grid = items < most ? items : most, used = sums && !best.kper && nt <= grid ? grid - grid % nt : most;
             return (items + used - 1) / used;
         };
-        const double whole = best.sk ? (double)(tiles * len) / G : (double)(rounds(tiles, G) * len);
+        double whole = best.sk ? (double)(tiles * len) / G : (double)(rounds(tiles, G) * len);
+        const int left = N - (int)(nt - 1) * 128;
+        if (best.sk && left <= 112) {
+            const double span = (double)tiles / G;                // tiles of a CTA, one after the other
+            const int64_t turns = (int64_t)(span / nt);
+            const double rest = span - (double)(turns * nt), full = (double)(turns * (nt - 1)) + (rest < nt - 1 ? rest : (double)(nt - 1));
+            whole *= (full + (0.6 + 0.3 * ((left + 15) & ~15) / 128) * (span - full)) / span;
+        }
         const double paired = best.sk ? (double)(pairs * len) / (G / 2) : (double)(rounds(pairs, G / 2) * len);
         best.pair = (!best.kper || pairs <= G / 2) && paired * (kb - 0.06 * busy) + 0.6 < whole * kb;
     }
