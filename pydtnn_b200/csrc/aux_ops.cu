@@ -77,9 +77,12 @@ static int launch_reduce2(F f, double* partial, int layout, int n, int c, int hw
 
 static size_t reduce2_bytes(int c) { return (size_t)RED_CHUNKS * 2 * c * sizeof(double); }
 
-// IDX = int where the element count plus one grid stride (ew_blocks) fits 31 bits: the kernels below that divide an element's index
+// Blocks of an elementwise launch, at most EW_BLOCKS, of 256 threads that step by the whole grid.
+constexpr int64_t EW_BLOCKS = 148 * 16;
+static unsigned ew_blocks(int64_t total) { int64_t b = (total + 255) / 256; return (unsigned)(b > EW_BLOCKS ? EW_BLOCKS : (b < 1 ? 1 : b)); }
+// IDX = int where the element count plus one such step fits 31 bits: the kernels below that divide an element's index
 // do so in 32 bits then (small float64 ResNet step, 31 such launches: 503 -> 500 us).
-static bool fits_int(int64_t total) { return total < 0x7fffffffLL - 148LL * 16 * 256; }
+static bool fits_int(int64_t total) { return total < 0x7fffffffLL - EW_BLOCKS * 256; }
 template <typename IDX> __device__ __forceinline__ int channel_of(IDX idx, int c, int hw, int nchw)
 {
     return nchw ? (int)((idx / hw) % c) : (int)(idx % c);
@@ -499,8 +502,6 @@ int channel_sum_v4(int n, int c, int hw, const void* src, void* dst, void* ws, s
     int rc = check_launch("reduce2_v4(sum)"); if (rc) return rc;
     return final_warp((const double*)ws, g.chunks, c, 2, 1.0, 0.0, 0.0, (float*)dst, (float*)nullptr, (float*)nullptr, (float*)nullptr, st);
 }
-
-static unsigned ew_blocks(int64_t total) { int64_t b = (total + 255) / 256; return (unsigned)(b > 148 * 16 ? 148 * 16 : (b < 1 ? 1 : b)); }
 
 template <typename T>
 static int bn_train_forward_t(int layout, int n, int c, int hw, const T* x, const T* gamma, const T* beta,
