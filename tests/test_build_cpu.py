@@ -23,3 +23,10 @@ def test_kernels_whose_roles_share_registers_have_them_all():
     for few in (_ptxas(1, 0, 0, 0, 126), _ptxas(0, 2, 1, 0, 120)):
         with pytest.raises(RuntimeError, match="registers"):
             build.check_role_registers(other + few)
+
+
+def test_the_check_knows_the_form_for_pairs_of_ctas():
+    name = lambda text: text.replace("EEEv14CUtensorMap", "ELb1EEEv14CUtensorMap")            # its last template argument
+    assert build.check_role_registers(name(_ptxas(0, 1, 0, 0, 128) + _ptxas(1, 0, 0, 0, 128))) == 2
+    with pytest.raises(RuntimeError, match="registers"):
+        build.check_role_registers(name(_ptxas(1, 0, 0, 0, 126)))
