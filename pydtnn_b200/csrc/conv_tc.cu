@@ -1012,6 +1012,10 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 TC_PROF_ADD(14);   // producer: TMA issue
             }
         }
+        // A pair's stages are released by arrivals that the first CTA's tensor core sends to both: all of them are in before either
+        // CTA may leave (nobody else waits for the last ones, and one that came later would find another block's shared memory).
+        if (PAIR)
+            for (int i = 0; i < STAGES && ok; i++, ring.next()) ok = mbar_wait(&empty_bar[ring.s], ring.phase ^ 1, abort_flag, &g_tc_status, TC_ERR_EMPTY);
         }
         __syncwarp();
     } else if (warp == 1) {
