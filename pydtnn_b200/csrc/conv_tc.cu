@@ -2309,7 +2309,8 @@ static FwdPlan fwd_plan(int64_t M, int N, int64_t kblocks, bool may_share, bool 
     // sums 36.3 / 33.2).  A single CTA does not multiply past the last channel, so a k-block of a last column tile takes it 0.6 + 0.3 of
     // the columns' share of what a whole one takes; a pair always multiplies 128.  In balanced ranges the CTA with the most whole
     // tiles counts (of whole tiles and splits that is one with whole ones only): 32x36x36 256->132 3x3 146 / 150 us, 34x41x41 256->172 5x5
-    // 640 / 652; 53x25x25 512->188 3x3 285 / 277.
+    // 640 / 652; 53x25x25 512->188 3x3 285 / 277.  A column tile that is the only one costs nearly what a whole one does: 7x79x51 512->112
+    // 3x3 133 / 116, 4x76x40 128->88 5x5 49.1 / 46.9.
     if (may_pair && best.bn == 128 && !fine && M > 128 && (best.kper ? best.kper : kblocks) >= 12) {
         const int64_t nt = (N + 127) / 128, splits = best.kper ? (kblocks + best.kper - 1) / best.kper : 1;
         const int64_t tiles = (M + 127) / 128 * nt * splits, pairs = (M + 255) / 256 * nt * splits, len = best.kper ? best.kper : kblocks;
@@ -2320,7 +2321,7 @@ static FwdPlan fwd_plan(int64_t M, int N, int64_t kblocks, bool may_share, bool 
         };
         double whole = best.sk ? (double)(tiles * len) / G : (double)(rounds(tiles, G) * len);
         const int left = N - (int)(nt - 1) * 128;
-        if (best.sk && left <= 112) {
+        if (best.sk && nt > 1 && left <= 112) {
             const double span = (double)tiles / G;                // tiles of a CTA, one after the other
             const int64_t turns = (int64_t)(span / nt);
             const double rest = span - (double)(turns * nt), full = (double)(turns * (nt - 1)) + (rest < nt - 1 ? rest : (double)(nt - 1));

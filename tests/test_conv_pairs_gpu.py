@@ -168,9 +168,11 @@ def test_no_pairs_where_batch_sums_leave_them_too_few_ctas(shape):
     assert torch.equal(first, y)
 
 
-@pytest.mark.parametrize("shape,pairs", [((32, 36, 36, 256, 132, 3, 1), False), ((34, 41, 41, 256, 172, 5, 1), False), ((53, 25, 25, 512, 188, 3, 1), True)])
+@pytest.mark.parametrize("shape,pairs", [((32, 36, 36, 256, 132, 3, 1), False), ((34, 41, 41, 256, 172, 5, 1), False), ((53, 25, 25, 512, 188, 3, 1), True),
+                                         ((7, 79, 51, 512, 112, 3, 1), True), ((4, 76, 40, 128, 88, 5, 1), True)])
 def test_no_pairs_where_the_last_column_tile_is_narrow(shape, pairs):
-    """Balanced ranges of many tiles with a last column tile of 4, 44 and 60 channels: a single CTA does not multiply past them, a pair does."""
+    """Balanced ranges of many tiles with a last column tile of 4, 44 and 60 channels: a single CTA does not multiply past them, a pair does.
+    (An only column tile costs nearly what a whole one does.)"""
     L = _lib.lib()
     _, desc, _, (xd, dyd, wd), _, _ = _layer(shape, "NHWC", "KRSC")
     ws, y = workspace(desc), torch.empty_like(dyd)
