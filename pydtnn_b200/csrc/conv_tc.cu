@@ -556,12 +556,15 @@ struct TcParams {
     int cls_M[4], cls_P[4], cls_Q[4], cls_kblocks[4], cls_S[4], cls_low_h[4], cls_low_w[4], cls_r0[4], cls_s0[4];
     int64_t cls_out[4];
     // FWD with the K loop split over CTAs (a launch with few tiles): CTA (tile, z) takes k-blocks [z * kper, (z + 1) * kper)
-    // and stores its partial tile to row block z of [splits][row tiles * 128][N]; tc_split_finish_kernel adds them.  0: off.
+    // and stores its partial tile to row block z of [splits][row tiles * 128][N] (of pairs of CTAs: row tiles * 256);
+    // tc_split_finish_kernel adds them.  0: off.
     int kper;
     // FWD with batch statistics: for every block of 32 output rows, row (m / 32) of `stats` ([ceil(M/32)][2][N] floats)
     // receives the per-channel sum and sum of squares of the stored values (rows past M left out).  Null: off.
     // stats_cta: the grid is a multiple of the column-tile count nt, so a CTA keeps one column tile; it adds the sums
-    // of all its tiles in registers and `stats` is [(grid / nt) * 4][2][N]: one row per CTA group and row quadrant.
+    // of all its tiles in registers and `stats` is [(grid / nt) * 4][2][N]: one row per CTA group and row quadrant.  Pairs of
+    // CTAs are groups of nt pairs, each CTA of a pair with rows of its own: [(pairs / nt) * 8][2][N], without the rows of a CTA
+    // whose 128 output rows all lie past M (fwd_stats_rows).
     float* stats;
     int stats_cta;
     FastDiv f_nt, f_mt, f_plane, f_pq, f_q, f_cb, f_s, f_c;      // column tiles, row tiles, their product, P * Q, Q, cblocks, S, C (launch_tc)
@@ -734,7 +737,8 @@ template <int MODE, int BSRC, int STREAM, int RESKB, bool BOTH> constexpr int tc
 // products of both.  A k-block of 128 columns then moves 80 KB through an SM's shared memory instead of 128 (24 in by TMA, 32 for
 // the split, 24 to the tensor core) and 24 KB instead of 32 from L2, a stage is 32 KB instead of 48 (six stages, whose A halves
 // go through the four slots of tensor memory).  Long launches: 16x56x56 256->256 3x3 from 242 to 209 us forward, from 272 to 240 weight gradient.
-// With 64 columns (24 KB of 20 + 36) the hand-offs bound a k-block and pairs were 2 % slower. Sums are the same bit for bit.
+// With 64 columns (24 KB of 20 + 36) the hand-offs bound a k-block and pairs were 2 % slower. Sums are the
+// same bit for bit where the K loop is cut at the same k-blocks: whole tiles and splits are, balanced ranges are counted in pairs.
 // FINE: sums at the precision of float32 FMAs (see tc_fine_sums): both operands split by rounding, each k-block summed in tensor
 // memory by itself, its small products first.  BOTH: the warps that split A split B too (see tc_b_warps).
 template <int MODE, int BN, int STAGES, bool SK, int SLABS, int BSRC, int STREAM, bool MULTI, int RESKB = 0, bool FINE = false, bool BOTH = false, bool PAIR = false>
@@ -2045,7 +2049,8 @@ struct WgradPlan { int splits, kblocks, bn; bool pair; };
 // item + a fixed per-item cost for pipeline fill, drain and the partial-tile store) + the second-stage reduce, whose
 // traffic grows with the split count.  Pairs of CTAs (256 rows) take 0.88 of the time a k-block and 1.5 k-blocks more an item, and are taken
 // where that is 2 % less: 64x14x14 256->256 3x3 60.5 -> 56.0 us, 32x56x56 128->256 5x5/2 (NCHW) 232 -> 196; with nine row
-// tiles, ten in pairs, 64x28x28 128->128 3x3 62.5 / 64.4 us.
+// tiles, ten in pairs, 64x28x28 128->128 3x3 62.5 / 64.4 us.  A narrow last column tile is charged as a whole one for both: of 34 layers
+// of 96 to 288 columns one lost by it (26x30x9 256->96 3x3 23.2 / 23.8 us).
 static WgradPlan wgrad_plan(const Geo& g)
 {
     WgradPlan pl;
@@ -2585,7 +2590,9 @@ static int tc_dgrad_classes_one_launch(const Geo& g, const WStride& wsd, bool b_
     // narrow tiles where the wide ones would leave half of the chip idle (see fwd_plan)
     const int BN = g.ci <= 64 || ((int64_t)g.n * g.h * g.w + 127) / 128 * ((g.ci + 127) / 128) * 2 <= tc_sm_count() ? 64 : 128;
     // Pairs of CTAs take 0.87 of the time: unless the rows that fill up the classes' last pairs are more than that (56x56 128->128 3x3/2 of
-    // 64 images 92 -> 82 us, 32x56x56 128->256 5x5/2 246 -> 200).
+    // 64 images 92 -> 82 us, 32x56x56 128->256 5x5/2 246 -> 200).  Neither the length of the classes' K loops nor a narrow last column
+    // tile asks for more of a rule: 80 layers with classes of 2 to 72 k-blocks and 128 to 256 columns 0.84 to 1.005 of the time (32x14x14
+    // 256->64 3x3/2, 2 to 8 k-blocks, 13.6 / 13.6 us; 64x28x28 128->64 3x3/2 21.7 / 21.5; 23x57x57 132->96 5x5/2 102 / 89).
     int64_t whole[2] = {};                    // row tiles of all classes in 128 rows and in pairs of 256
     for (int i = 0; i < ncls; i++) {
         const int64_t m = (int64_t)g.n * cls[i].a.out_cnt * cls[i].b.out_cnt;
