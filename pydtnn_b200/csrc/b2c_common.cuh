@@ -14,7 +14,7 @@ void count_launch();
 // Programmatic dependent launch.  pdl_prologue() waits until the kernel before it in the stream has completed and its writes
 // are visible, then lets the kernel after it be scheduled early.  Most kernels of the library begin with it; those with set-up
 // worth hiding (tensor-core and float64 convolutions, second stages of splits) do that first, and every one of their threads that
-// touches global memory or a wait with a limit comes to a pdl_wait() before it.  launch_pdl() marks the launch as allowed to start while its predecessor drains, so launch
+// touches global memory, or starts the clock of a wait with a limit, comes to a pdl_wait() before it.  launch_pdl() marks the launch as allowed to start while its predecessor drains, so launch
 // latency and the start-up of the next kernel's blocks overlap with the tail of the running one; data is only
 // touched after the wait, so the stream's ordering is unchanged.
 #ifdef __CUDACC__

@@ -100,7 +100,9 @@ __device__ __forceinline__ bool elect_one_sync() {
 // Bounded wait. Returns false when the wait ran out or another role already gave up.
 // mbarrier.try_wait suspends the thread in hardware for a short while, so the loop is not hot; the abort
 // flag and the clock are looked at only every 32 failed tries to keep waiting warps off the LSU and the
-// issue ports the working warps need.
+// issue ports the working warps need.  The clock starts when the kernel in front in the stream has ended: a role that works on
+// chip only may wait while that kernel still runs, which is not this launch's time (a kernel that lets its dependents start and
+// runs longer than the limit made all waits run out).
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status, int code,
                                           long long limit_cycles = TC_WAIT_CYCLES) {
     if (mbar_try_wait(bar, parity)) return true;
@@ -110,9 +112,8 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
         if (mbar_try_wait(bar, parity)) return true;
         if ((++tries & 31u) == 0) {
             if (*abort_flag) return false;
-            const long long now = clock64();
-            if (t0 == 0) t0 = now;
-            else if (now - t0 > limit_cycles) {
+            if (t0 == 0) { pdl_wait(); t0 = clock64(); }
+            else if (clock64() - t0 > limit_cycles) {
                 *abort_flag = 1;
                 atomicCAS(status, 0, code);
                 return false;
@@ -822,9 +823,9 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     }
     if (warp == 1) tmem_alloc<PAIR>(tmem_slot, L::TMEM_COLS);
     // Barriers, tensor memory and the abort flag are on-chip state, set up while the kernel before this one in the stream may
-    // still be draining, and so is where each role starts: every role waits for that kernel itself, with its first tile's arithmetic
-    // done and its code fetched, before it touches global memory and before its first bounded wait, whose limit is then for what
-    // this launch does (a kernel in front that lets its dependents start and runs longer than the limit made all waits run out).
+    // still be draining, and so is where each role starts: the roles that touch global memory (the producer, the drain warps, the B
+    // warps with their bias sums) wait for that kernel themselves, with their first tile's arithmetic done and their code fetched.
+    // The others wait for what those bring; no wait's limit counts the time before that kernel has ended (mbar_wait).
     tc_fence_before();
     if constexpr (PAIR) cluster_sync();          // the other CTA's barriers are set up as well
     else __syncthreads();
@@ -1045,7 +1046,6 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             const uint64_t b_desc0 = make_smem_desc(smem_u32(smem) + (RESKB ? L::RES_OFFSET : L::A_BYTES), LBO, SBO, LAYOUT);
             Walk w;
             w.init(total_tiles, p.kblocks, MODE == TCM_FWD && !SK && !MULTI && RESKB == 0 ? p.kper : 0, p.f_plane);
-            pdl_wait();
             while (ok && w.template next<SK>()) {
                 const TileGeo tg = tile_geo(w.tile);
                 if (MULTI) w.kb_e = tg.kblocks;
@@ -1161,7 +1161,6 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         Ring<STAGES> freed;                          // PAIR: the stage of the k-block TSLOTS before this one, which had its slot
         int filled = 0;
         bool ok = true;
-        pdl_wait();
         if (RESKB) {
             // the lo halves of the resident filter tiles, once per launch
             ok = mbar_wait(bres_bar, 0, abort_flag, &g_tc_status, TC_ERR_FULL);
@@ -1267,7 +1266,6 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         bool ok = true;
         Walk w;
         w.init(total_tiles, p.kblocks, MODE == TCM_FWD && !SK && !MULTI ? p.kper : 0, p.f_plane);
-        pdl_wait();
         while (ok && w.template next<SK>()) {
             if (MULTI) w.kb_e = tile_geo(w.tile).kblocks;
             // WGRAD: the tiles of the first row block also sum their dy tile over the pixels (the bias gradient);
@@ -1291,6 +1289,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 if (lane == 0) arrive_mma(&xform_bar[s]);
             }
             if (MODE == TCM_WGRAD && do_db && ok) {
+                pdl_wait();
                 // Float4 number t + 128 i of the B region is box i/2, pixel row t/8 + 16 (i & 1), 16-byte chunk t & 7.
                 // The box layout XORs the 32-byte atom index (chunk >> 1) with (row & 3), so the lane's channels are
                 // chunk ((c >> 1) ^ rr) * 2 + (c & 1) with c = lane & 7, rr = (lane >> 3) & 3: the four lanes that hold
